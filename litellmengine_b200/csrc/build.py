@@ -45,6 +45,7 @@ FAMILIES: Dict[str, List[str]] = {
     "sampling": ["sampling.cu"],
     "gemm_skinny": ["gemm_skinny.cu"],
     "gemm_pair_tcgen05": ["gemm_pair_tcgen05.cu"],
+    "gemm_f32": ["gemm_f32.cu"],
     "host_core": ["host_core.cpp"],            # the host side's bookkeeping: plain C++, no device code
 }
 HOST_FAMILIES = {"host_core"}

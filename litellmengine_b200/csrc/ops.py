@@ -1835,6 +1835,25 @@ def linear_silu_mul(x: torch.Tensor, w_gate_up: torch.Tensor, out_dtype: torch.d
     return silu_and_mul(linear(x, w_gate_up, out_dtype=out_dtype, partials_ok=True), activation=activation, limit=limit)
 
 
+STREAM_F32_MAX_ROWS = 16     # rows up to which a float32 product takes the engine's own kernel (17 and more: the arithmetic bounds it)
+
+
+def linear_f32(x: torch.Tensor, weight: torch.Tensor) -> torch.Tensor:
+    """x [M, K] @ weight[N, K]^T, all float32, with the engine's own weight-streaming kernel (multiply-adds in float32,
+    nothing rounded below it).  K must be a multiple of 4 and both operands 16-byte aligned."""
+    _dev(x, weight)
+    if x.dtype != torch.float32 or weight.dtype != torch.float32:
+        raise KernelError("the float32 product takes float32 operands")
+    M, K = x.shape
+    N = weight.shape[0]
+    if weight.shape[1] != K:
+        raise KernelError("x and weight disagree on K")
+    out = torch.empty((M, N), dtype=torch.float32, device=x.device)
+    f = _fn("gemm_f32", "llm_linear_f32", [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p])
+    _check(f(_ptr(x), _ptr(weight), _ptr(out), M, N, K, 0, _stream()), "linear_f32")
+    return out
+
+
 def linear(x: torch.Tensor, weight: torch.Tensor, out_dtype: Optional[torch.dtype] = None,
            partials_ok: bool = False):
     """x [T, K] @ weight[N, K]^T.  Up to 16 bfloat16 rows (decode steps; up to 32 for the small products
@@ -1846,7 +1865,7 @@ def linear(x: torch.Tensor, weight: torch.Tensor, out_dtype: Optional[torch.dtyp
     goes through the library matrix product (under `LLM_PAIR=all`, prompt portions take the paired tcgen05
     product `linear_pair`; by default only the gate/up product does, through `linear_silu_mul`) (the reference uses cuBLAS for all its products,
     src/layers/linear.cu:169-215).  bfloat16 operands accumulate in float32; a float32 weight
-    keeps its product in true float32 (no TF32), whatever x is."""
+    keeps its product in true float32 (no TF32), whatever x is: up to 16 rows in the engine's own streaming kernel."""
     _dev(x, weight)
     rows = x.shape[0]
     if (x.dtype == torch.bfloat16 and weight.dtype == torch.bfloat16 and x.shape[1] % 8 == 0 and weight.data_ptr() % 16 == 0
@@ -1857,8 +1876,13 @@ def linear(x: torch.Tensor, weight: torch.Tensor, out_dtype: Optional[torch.dtyp
             x, weight, weight.shape[0], "plain"):
         return linear_pair(x, weight, out_dtype or x.dtype)
     if weight.dtype == torch.float32:
-        y = torch.mm(x if x.dtype == torch.float32 else x.float(), weight.t())
         want = out_dtype or x.dtype
+        x = x if x.dtype == torch.float32 else x.float()
+        if (1 <= rows <= STREAM_F32_MAX_ROWS and 0 < weight.shape[0] <= 1 << 20 and x.shape[1] % 4 == 0 and x.shape[1] > 0
+                and x.data_ptr() % 16 == 0 and weight.data_ptr() % 16 == 0):
+            y = linear_f32(x, weight)
+        else:
+            y = torch.mm(x, weight.t())
         return y if want == torch.float32 else y.to(want)
     if x.dtype != weight.dtype:
         x = x.to(weight.dtype)
