@@ -31,6 +31,7 @@ FAMILIES: Dict[str, List[str]] = {
     "activation": ["activation.cu"],
     "rope_cache": ["rope_cache.cu"],
     "attention_generic": ["attention_generic.cu"],
+    "attention_f32": ["attention_f32.cu"],
     "attention_prepare": ["attention_prepare.cu"],
     "linear_attention": ["linear_attention.cu"],
     "delta_rule": ["delta_rule.cu"],

@@ -522,6 +522,62 @@ def paged_attention_generic(q: torch.Tensor, cache: torch.Tensor, positions, tok
     return out
 
 
+def attention_f32_supported(d: int, group: int) -> bool:
+    """Whether the float32 kernels for single tokens and for portions take this head size and group."""
+    if d % 64 != 0:          # head sizes 64 and 128: do not compile them just to hear "no"
+        return False
+    return bool(_fn("attention_f32", "llm_attention_f32_decode_supported", [c_int, c_int])(d, group)) and bool(
+        _fn("attention_f32", "llm_attention_f32_prefill_supported", [c_int])(d))
+
+
+def _f32_operands(q, out, cache, nq: int, nkv: int, d: int, page_size: int) -> None:
+    if q.dtype != torch.float32 or cache.dtype != torch.float32 or out.dtype != torch.float32:
+        raise KernelError("the float32 attention kernels take float32 only")
+    if q.shape[1] != nq * d or out.shape != q.shape or tuple(cache.shape[1:]) != (2, nkv, page_size, d):
+        raise KernelError("q and out must be [T, heads*head_dim] and cache [pages, 2, kv_heads, page_size, head_dim]")
+
+
+def attention_f32_decode(q: torch.Tensor, out: torch.Tensor, cache: torch.Tensor, rows: Optional[torch.Tensor], n_rows: int,
+                         positions, token_entry, entry_slot, block_table: torch.Tensor, nq: int, nkv: int, d: int,
+                         page_size: int, window: Optional[int], scale: float, splits: int, status: torch.Tensor) -> torch.Tensor:
+    """`paged_attention_decode` for float32 queries and pages, everything in float32.  The splits' scratch is allocated per
+    call (steps of the 32-bit mode may run on several streams at once)."""
+    _dev(q, out, cache, rows, positions, token_entry, entry_slot, block_table, status)
+    for t, n in ((positions, "positions"), (token_entry, "token_entry"), (entry_slot, "entry_slot"), (block_table, "block_table")):
+        _i32(t, n)
+    _i32(rows, "rows")
+    _f32_operands(q, out, cache, nq, nkv, d, page_size)
+    scratch = torch.empty(n_rows * nq * splits * (d + 2), dtype=torch.float32, device=q.device) if splits > 1 else None
+    f = _fn("attention_f32", "llm_attention_f32_decode",
+            [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int,
+             c_int, c_int, c_float, c_int, c_int, c_void_p, c_void_p, c_void_p])
+    _check(f(_ptr(q), _ptr(out), _ptr(cache), _ptr(rows), n_rows, _ptr(positions), _ptr(token_entry), _ptr(entry_slot),
+             _ptr(block_table), block_table.shape[1], nq, nkv, d, page_size, int(window) if window else 0, float(scale),
+             cache.shape[0], splits, _ptr(scratch), _ptr(status), _stream()), "attention_f32_decode")
+    if splits > 1:
+        global launch_count
+        launch_count += 1                         # the merge kernel
+    return out
+
+
+def attention_f32_prefill(q: torch.Tensor, out: torch.Tensor, cache: torch.Tensor, tiles: torch.Tensor, n_tiles: int, entry_slot,
+                          entry_q_start, entry_q_len, entry_kv_len, block_table: torch.Tensor, nq: int, nkv: int, d: int,
+                          page_size: int, window: Optional[int], scale: float, status: torch.Tensor) -> torch.Tensor:
+    """`paged_attention_prefill` for float32 queries and pages, everything in float32."""
+    _dev(q, out, cache, tiles, entry_slot, entry_q_start, entry_q_len, entry_kv_len, block_table, status)
+    for t, n in ((tiles, "tiles"), (entry_slot, "entry_slot"), (entry_q_start, "entry_q_start"), (entry_q_len, "entry_q_len"),
+                 (entry_kv_len, "entry_kv_len"), (block_table, "block_table")):
+        _i32(t, n)
+    _f32_operands(q, out, cache, nq, nkv, d, page_size)
+    f = _fn("attention_f32", "llm_attention_f32_prefill",
+            [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int,
+             c_int, c_int, c_int, c_int, c_float, c_int, c_void_p, c_void_p])
+    _check(f(_ptr(q), _ptr(out), _ptr(cache), _ptr(tiles), n_tiles, PREFILL_TILE_ROWS, _ptr(entry_slot), _ptr(entry_q_start),
+             _ptr(entry_q_len), _ptr(entry_kv_len), _ptr(block_table), block_table.shape[1], nq, nkv, d, page_size,
+             int(window) if window else 0, float(scale), cache.shape[0], _ptr(status), _stream()), "attention_f32_prefill")
+    return out
+
+
 NORM_SCOPES = {None: 0, "none": 0, "head": 1, "projection": 2}
 
 

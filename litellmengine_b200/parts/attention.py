@@ -559,8 +559,9 @@ def attention_over_pages(q: torch.Tensor, ctx: StageContext, nq: int, nkv: int, 
     """Pick the attention kernels for this batch.  Every choice reads the same pages and gives
     the same result up to rounding.  bfloat16 with a head size and group the tuned kernels
     take: single tokens go to the split-key decode kernel, longer portions to the tensor-core
-    prefill kernel (a mixed batch launches both, each over its own rows).  Everything else,
-    float32 included, goes through the generic kernel.  `span`: see `key_span`.  `out`: where the result goes, if the
+    prefill kernel (a mixed batch launches both, each over its own rows).  float32 with a head size
+    of 64 or 128 and a group of 1, 2, 4 or 8 takes two float32 kernels in the same way.  Everything
+    else goes through the generic kernel.  `span`: see `key_span`.  `out`: where the result goes, if the
     tuned kernels take the step (bfloat16 [T, heads * head_dim], contiguous)."""
     b = ctx.batch
     cache = ctx.cache
@@ -585,6 +586,22 @@ def attention_over_pages(q: torch.Tensor, ctx: StageContext, nq: int, nkv: int, 
             kernel(q, out, cache, work.padded_tiles if padded else work.prefill_tiles, n_tiles, b.entry_slot,
                    b.entry_q_start, b.entry_q_len, b.entry_kv_len, ctx.block_table, nq, nkv, d, ctx.page_size, span,
                    scale, ctx.status)
+        return out
+    if (work is not None and q.dtype == torch.float32 and cache.dtype == torch.float32
+            and ops.attention_f32_supported(d, nq // nkv)):
+        out = torch.empty_like(q)
+        padded = getattr(b, "any_division", False)
+        n_dec = work.padded_rows.shape[0] if padded else work.num_decode
+        n_tiles = work.padded_tiles.shape[0] if padded else work.num_prefill_tiles
+        if n_dec:
+            splits = decode_key_splits(q.device, n_dec, nkv, decode_reach(b, span))
+            rows = work.padded_rows if padded else (None if n_dec == b.num_tokens else work.decode_rows)
+            ops.attention_f32_decode(q, out, cache, rows, n_dec, b.positions, b.token_entry, b.entry_slot,
+                                     ctx.block_table, nq, nkv, d, ctx.page_size, span, scale, splits, ctx.status)
+        if n_tiles:
+            ops.attention_f32_prefill(q, out, cache, work.padded_tiles if padded else work.prefill_tiles, n_tiles,
+                                      b.entry_slot, b.entry_q_start, b.entry_q_len, b.entry_kv_len, ctx.block_table,
+                                      nq, nkv, d, ctx.page_size, span, scale, ctx.status)
         return out
     return ops.paged_attention_generic(q, cache, b.positions, b.token_entry, b.entry_slot,
                                        ctx.block_table, nq, nkv, d, ctx.page_size, span, scale, ctx.status)

@@ -31,3 +31,77 @@ def test_streaming_product(M, N, K):
         w[N // 2, K - 1] = float("inf")                       # what a lane past the row's end must not multiply by zero
         bad = ops().linear(x, w)
         assert bool(torch.isinf(bad[:, N // 2]).all()) and bool(torch.isfinite(bad).sum() == M * (N - 1))
+
+
+def pages_of(lens, nkv, d, page, g):
+    width = max(-(-n // page) for n in lens)
+    perm = torch.randperm(len(lens) * width + 2, generator=g)
+    cache = torch.full((len(perm), 2, nkv, page, d), 33.0)
+    table = torch.stack([perm[b * width:(b + 1) * width] for b in range(len(lens))]).to(torch.int32)
+    ks, vs = [], []
+    for b, n in enumerate(lens):
+        k, v = torch.randn(n, nkv, d, generator=g), torch.randn(n, nkv, d, generator=g)
+        j = torch.arange(n)
+        cache[table[b, j // page].long(), 0, :, j % page] = k
+        cache[table[b, j // page].long(), 1, :, j % page] = v
+        ks.append(k), vs.append(v)
+    return cache.to(DEV), table.to(DEV), ks, vs
+
+
+def plain(q, k, v, pos, span, scale):
+    """q [H, d] at `pos` over k, v [S, G, d] in float64; span as the kernels take it."""
+    lo = max(0, pos - span + 1) if span and span > 0 else pos - pos % -span if span else 0
+    rep = q.shape[0] // k.shape[1]
+    kk, vv = (t[lo:pos + 1].double().repeat_interleave(rep, dim=1) for t in (k, v))
+    p = torch.softmax(torch.einsum("hd,shd->hs", q.double(), kk) * scale, -1)
+    return torch.einsum("hs,shd->hd", p, vv)
+
+
+def tolerance(d, keys, scale_of_scores):
+    """Rounding of a score (d products, then its exponential's argument) and of the sums over the keys."""
+    return U * (8 * d ** 0.5 + 4 * scale_of_scores + 4 * math.sqrt(keys)) * 4
+
+
+@pytest.mark.parametrize("nq,nkv,d,page", [(4, 4, 64, 16), (4, 2, 128, 16), (8, 2, 128, 5), (8, 1, 128, 16), (16, 2, 64, 64), (2, 2, 128, 1)])
+@pytest.mark.parametrize("span", [None, 1, 37, -50])
+@pytest.mark.parametrize("splits", [1, 3])
+def test_single_tokens(nq, nkv, d, page, span, splits):
+    g = torch.Generator().manual_seed(nq * 100 + d + page)
+    lens = [1, 7, 8, 9, 63, 64, 65, 200, 313]
+    cache, table, ks, vs = pages_of(lens, nkv, d, page, g)
+    B, i32 = len(lens), lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)
+    q = torch.randn(B + 1, nq * d, generator=g).to(DEV)
+    out, status = torch.zeros_like(q), i32([0, 0])
+    # the rows in another order, with padding; one row belongs to nobody
+    order = [r for r in range(B)][::-1]
+    rows = i32([-1] + [r + 1 for r in order] + [-1])
+    ops().attention_f32_decode(q, out, cache, rows, B + 2, i32([0] + [n - 1 for n in lens]), i32([0] + list(range(B))), i32(list(range(B))),
+                               table, nq, nkv, d, page, span, d ** -0.5, splits, status)
+    for b, n in enumerate(lens):
+        ref = plain(q[b + 1].view(nq, d).cpu(), ks[b], vs[b], n - 1, span, d ** -0.5)
+        err = float((out[b + 1].view(nq, d).double().cpu() - ref).abs().max())
+        assert err <= tolerance(d, n, 6.0) * float(vs[b].abs().max()), (n, err)
+    assert status.tolist() == [0, 0] and float(out[0].abs().max()) == 0.0
+
+
+@pytest.mark.parametrize("nq,nkv,d,page", [(4, 4, 64, 16), (8, 2, 128, 16), (3, 1, 128, 5), (4, 2, 64, 1)])
+@pytest.mark.parametrize("span", [None, 1, 70, -100])
+def test_portions(nq, nkv, d, page, span):
+    """(keys cached after the step, query rows at their end), around the edges of 64 and 128 rows and of 64 keys."""
+    g = torch.Generator().manual_seed(nq * 100 + d + page)
+    reqs = [(2, 2), (64, 64), (65, 65), (130, 129), (200, 3), (300, 127), (257, 257)]
+    cache, table, ks, vs = pages_of([n for n, _ in reqs], nkv, d, page, g)
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)
+    T = sum(t for _, t in reqs)
+    q = torch.randn(T, nq * d, generator=g).to(DEV)
+    out, status, R = torch.zeros_like(q), i32([0, 0]), ops().PREFILL_TILE_ROWS
+    starts = [sum(t for _, t in reqs[:i]) for i in range(len(reqs))]
+    tiles = [(e, r) for e, (_, t) in enumerate(reqs) for r in range(0, t, R)][::-1] + [(-1, -1)]
+    ops().attention_f32_prefill(q, out, cache, i32(tiles), len(tiles), i32(list(range(len(reqs)))), i32(starts), i32([t for _, t in reqs]),
+                                i32([n for n, _ in reqs]), table, nq, nkv, d, page, span, d ** -0.5, status)
+    for e, (n, t) in enumerate(reqs):
+        for r in {0, 1, t // 2, min(63, t - 1), min(64, t - 1), t - 1}:
+            ref = plain(q[starts[e] + r].view(nq, d).cpu(), ks[e], vs[e], n - t + r, span, d ** -0.5)
+            err = float((out[starts[e] + r].view(nq, d).double().cpu() - ref).abs().max())
+            assert err <= tolerance(d, n, 6.0) * float(vs[e].abs().max()), (n, t, r, err)
+    assert status.tolist() == [0, 0]
