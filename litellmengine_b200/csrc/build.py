@@ -38,6 +38,7 @@ FAMILIES: Dict[str, List[str]] = {
     "streams": ["streams.cu"],
     "conv_norm": ["conv_norm.cu"],
     "latent_attention": ["latent_attention.cu"],
+    "latent_prefill_tcgen05": ["latent_prefill_tcgen05.cu"],
     "moe": ["moe.cu"],
     "attention_decode": ["attention_decode.cu"],
     "attention_prefill": ["attention_prefill.cu"],
@@ -50,7 +51,7 @@ FAMILIES: Dict[str, List[str]] = {
     "host_core": ["host_core.cpp"],            # the host side's bookkeeping: plain C++, no device code
 }
 HOST_FAMILIES = {"host_core"}
-HEADERS = ["common.cuh", "mma_tiles.cuh", "attention_decode_noalloc.h", "attention_decode_tma.cuh"]
+HEADERS = ["common.cuh", "mma_tiles.cuh", "tcgen05_attention.cuh", "attention_decode_noalloc.h", "attention_decode_tma.cuh"]
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-lineinfo", "-std=c++17",

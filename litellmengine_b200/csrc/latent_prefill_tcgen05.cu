@@ -1,0 +1,442 @@
+// Prompt portions of latent attention on the 5th-generation tensor cores, bfloat16: heads of 128 key entries and 64 rotated
+// ones, values of 128.
+//
+// The kernels in latent_attention.cu attend over the cached rows [c | kr] themselves, which is right for a few queries: per
+// query, key and head that costs 2 (2 R + P) flops (2,176 at R 512, P 64).  A portion of many queries meets every row with
+// every query, so here the rows are mapped ONCE to per-head keys and values, [k | v][h] = W_ukv[h] c, and attention costs
+// 2 (128 + 64 + 128) = 640.  The map is 2 R 256 flops a row and head, i.e. as much as 170 queries save.  Steps:
+//   latent_gather    the rows of every portion, from their pages, to consecutive rows of one tensor, each request's padded
+//                    with zero rows to whole tiles (so that a tile never shows another request's rows)
+//   (a product)      [k | v] of all rows and heads
+//   latent_q_pack    the queries [qn | rotated qr] per head in bfloat16
+//   attention        below
+// Measured, 32 heads over rows of 512 + 64, a prompt of 2,000 tokens: attention over the cached rows 1,275 us; here rows 5,
+// map 18, queries 12, attention 81 us (0.54 PFLOP/s of what it cannot do without, 43 GFLOP).  The layer 1,480 -> 273 us.
+//
+// Attention.  The structure of the one-pass kernel in attention_prefill_tcgen05.cu (a reference maximum that trails the
+// running one, two rows of work in turns on the tensor pipe, P over S in TMEM, two softmax threads a row), with two changes.
+// Every head has keys of its own, so the two pieces of work that share a key/value tile are two tiles of 128 QUERY rows of
+// one head.  And a tile is 96 keys: queries are 2 x 128 x 192 (96 KB), a tile of 128 keys with its values 80 KB, and two of
+// those would not fit beside them; two of 96 keys (60 KB each) do, and a product of N 96 is as efficient as one of 128.
+// The rotated key part is the same for all heads and comes straight from the gathered rows.
+#include "tcgen05_attention.cuh"
+#include <math_constants.h>
+
+#define LP_BM 128
+#define LP_BN 96
+#define LP_QB (LP_BM * 64)                   // elements of one 64-column block of a query tile
+#define LP_KB (LP_BN * 64)                   // and of a key or value tile
+#define LP_DK 192
+#define LP_DV 128
+#define LP_STAGES 2
+#define LP_JUMP 8.0f
+#define LP_THREADS (64 + 2 * 256)
+
+__device__ __forceinline__ void lp_ld16(unsigned taddr, unsigned (&r)[48], int at) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];\n"
+                 : "=r"(r[at]), "=r"(r[at + 1]), "=r"(r[at + 2]), "=r"(r[at + 3]), "=r"(r[at + 4]), "=r"(r[at + 5]), "=r"(r[at + 6]),
+                   "=r"(r[at + 7]), "=r"(r[at + 8]), "=r"(r[at + 9]), "=r"(r[at + 10]), "=r"(r[at + 11]), "=r"(r[at + 12]),
+                   "=r"(r[at + 13]), "=r"(r[at + 14]), "=r"(r[at + 15])
+                 : "r"(taddr) : "memory");
+}
+__device__ __forceinline__ void lp_st8(unsigned taddr, const unsigned (&r)[24], int at) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};\n" ::
+                     "r"(taddr), "r"(r[at]), "r"(r[at + 1]), "r"(r[at + 2]), "r"(r[at + 3]), "r"(r[at + 4]), "r"(r[at + 5]),
+                 "r"(r[at + 6]), "r"(r[at + 7]) : "memory");
+}
+
+// grid (H, work items).  tiles: int32 [n][2] = (segment, first query row inside the portion), 256 rows each, longest walk
+// first; segs: int32 [segments][4] = (entry, first position gathered, first gathered row, rows).
+__global__ void __launch_bounds__(LP_THREADS, 1) latent_prefill_tcgen05_kernel(
+    const __grid_constant__ CUtensorMap q_map, const __grid_constant__ CUtensorMap kv_map, const __grid_constant__ CUtensorMap r_map,
+    bf16* __restrict__ out, const int32_t* __restrict__ tiles, const int32_t* __restrict__ segs,
+    const int32_t* __restrict__ entry_q_start, const int32_t* __restrict__ entry_q_len, const int32_t* __restrict__ entry_kv_len,
+    int H, int R, int window, float scale_log2e, const float* __restrict__ gate, long long gate_stride, int32_t* __restrict__ status) {
+    pdl_begin();
+    extern __shared__ unsigned char smem_dyn[];
+    unsigned char* smem_al = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_dyn) + 1023) & ~uintptr_t(1023));
+    bf16* q_s = reinterpret_cast<bf16*>(smem_al);                 // [2 query tiles][3 blocks][128][64]
+    bf16* k_s = q_s + 2 * 3 * LP_QB;                              // [stages][3][96][64]
+    bf16* v_s = k_s + LP_STAGES * 3 * LP_KB;                      // [stages][2][96][64]
+    __shared__ __align__(8) unsigned long long q_full, k_full[LP_STAGES], k_empty[LP_STAGES], v_full[LP_STAGES], v_empty[LP_STAGES],
+        s_full[2], p_full[2], pv_done[2];
+    __shared__ unsigned tmem_base_s;
+    __shared__ int abort_flag;
+    __shared__ float x_max[2][2][2][128];                         // [tile parity][query tile][column half][row]
+    __shared__ float x_sum[2][2][128];
+
+    const int h = blockIdx.x;
+    const int seg = tiles[2 * blockIdx.y], q0 = tiles[2 * blockIdx.y + 1];
+    const int e = segs[4 * seg], first_pos = segs[4 * seg + 1], kv_row0 = segs[4 * seg + 2];
+    const int q_len = entry_q_len[e];
+    const int past = entry_kv_len[e] - q_len - first_pos;         // positions are counted from the first gathered row
+    const int row_base = entry_q_start[e] + q0;
+    const int rows_all = min(2 * LP_BM, q_len - q0);
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    auto rows_of = [&](int g) { return max(0, min(LP_BM, rows_all - g * LP_BM)); };
+    const int k_lo = first_visible(past + q0, window) / LP_BN * LP_BN;      // the earliest key of the earliest row
+    auto tiles_of = [&](int g) {                                  // key tiles that query tile g walks, all from k_lo
+        const int rows = rows_of(g);
+        return rows > 0 ? (past + q0 + g * LP_BM + rows - 1 - k_lo) / LP_BN + 1 : 0;
+    };
+    const int n0 = tiles_of(0), n1 = tiles_of(1), n_tiles = max(n0, n1);
+
+    if (tid == 0) {
+        abort_flag = 0;
+        t5_mbar_init(&q_full, 1);
+        for (int s = 0; s < LP_STAGES; ++s) {
+            t5_mbar_init(&k_full[s], 1); t5_mbar_init(&k_empty[s], 1);
+            t5_mbar_init(&v_full[s], 1); t5_mbar_init(&v_empty[s], 1);
+        }
+        for (int g = 0; g < 2; ++g) {
+            t5_mbar_init(&s_full[g], 1);
+            t5_mbar_init(&p_full[g], 256);
+            t5_mbar_init(&pv_done[g], 1);
+        }
+        asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+    }
+    if (warp == 1) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(t5_smem(&tmem_base_s)), "r"(512u) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
+    }
+    t5_fence_before();
+    __syncthreads();
+    t5_fence_after();
+    const unsigned tmem = tmem_base_s;
+    auto s_col = [](int g) { return static_cast<unsigned>(g * 128); };           // 96 columns used
+    auto o_col = [](int g) { return static_cast<unsigned>(256 + g * 128); };
+
+    if (warp == 0) {
+        // ---- producer: one thread, eleven boxes at most a tile ----
+        if (lane == 0) {
+            t5_expect_tx(&q_full, 2 * 3 * LP_QB * sizeof(bf16));
+#pragma unroll
+            for (int g = 0; g < 2; ++g)
+#pragma unroll
+                for (int b = 0; b < 3; ++b)
+                    t5_tma_2d(q_s + (g * 3 + b) * LP_QB, &q_map, h * LP_DK + 64 * b, row_base + g * LP_BM, &q_full);
+            int issued = 0;
+            bool ok = true;
+            for (int j = 0; j < n_tiles; ++j) {
+                const int st = j % LP_STAGES, y = kv_row0 + k_lo + j * LP_BN;
+                if (j >= LP_STAGES && !t5_wait(&k_empty[st], ((j / LP_STAGES) - 1) & 1, &abort_flag, status, row_base)) { ok = false; break; }
+                t5_expect_tx(&k_full[st], 3 * LP_KB * sizeof(bf16));
+                bf16* kd = k_s + st * 3 * LP_KB;
+                t5_tma_2d(kd, &kv_map, h * 256, y, &k_full[st]);
+                t5_tma_2d(kd + LP_KB, &kv_map, h * 256 + 64, y, &k_full[st]);
+                t5_tma_2d(kd + 2 * LP_KB, &r_map, R, y, &k_full[st]);
+                issued = 2 * j + 1;
+                if (j >= LP_STAGES && !t5_wait(&v_empty[st], ((j / LP_STAGES) - 1) & 1, &abort_flag, status, row_base)) { ok = false; break; }
+                t5_expect_tx(&v_full[st], 2 * LP_KB * sizeof(bf16));
+                bf16* vd = v_s + st * 2 * LP_KB;
+                t5_tma_2d(vd, &kv_map, h * 256 + 128, y, &v_full[st]);
+                t5_tma_2d(vd + LP_KB, &kv_map, h * 256 + 192, y, &v_full[st]);
+                issued = 2 * j + 2;
+            }
+            if (!ok || abort_flag) {                              // let what is in flight land before the CTA goes away
+                for (int i = 0; i < T5_WAIT_LIMIT && !t5_try_wait(&q_full, 0); ++i) {}
+                const int nk = (issued + 1) / 2, nv = issued / 2;
+                for (int j = max(0, nk - LP_STAGES); j < nk; ++j)
+                    for (int i = 0; i < T5_WAIT_LIMIT && !t5_try_wait(&k_full[j % LP_STAGES], (j / LP_STAGES) & 1); ++i) {}
+                for (int j = max(0, nv - LP_STAGES); j < nv; ++j)
+                    for (int i = 0; i < T5_WAIT_LIMIT && !t5_try_wait(&v_full[j % LP_STAGES], (j / LP_STAGES) & 1); ++i) {}
+            }
+        }
+    } else if (warp == 1) {
+        // ---- MMA issuer: S0(j), O1 += P1 V(j-1), S1(j), O0 += P0 V(j); a query tile takes part while it has keys ----
+        if (lane == 0) {
+            constexpr unsigned IDESC_QK = t5_idesc(LP_BM, LP_BN, 0);
+            constexpr unsigned IDESC_PV = t5_idesc(LP_BM, LP_DV, 1);
+            const unsigned long long qd0 = t5_desc(q_s, 16, 1024), kd0 = t5_desc(k_s, 16, 1024);
+            const unsigned long long vd0 = t5_desc(v_s, LP_KB * sizeof(bf16), 1024);
+            constexpr unsigned long long K_STEP = (3 * LP_KB * sizeof(bf16)) >> 4, V_STEP = (2 * LP_KB * sizeof(bf16)) >> 4;
+            auto qk = [&](int g, int st) {                        // g, st: constants where this is inlined
+#pragma unroll
+                for (int k = 0; k < 12; ++k)
+                    t5_mma_ss(tmem + s_col(g), qd0 + (((g * 3 + (k >> 2)) * LP_QB + (k & 3) * 16) * sizeof(bf16) >> 4),
+                              kd0 + st * K_STEP + (((k >> 2) * LP_KB + (k & 3) * 16) * sizeof(bf16) >> 4), IDESC_QK, k > 0);
+                t5_commit(&s_full[g]);
+            };
+            auto pv = [&](int g, int st, bool first) {
+#pragma unroll
+                for (int k = 0; k < 6; ++k)                       // P of keys 48 .. 95 lies over S column 48
+                    t5_mma_ts(tmem + o_col(g), tmem + s_col(g) + (k / 3) * 48 + (k % 3) * 8, vd0 + st * V_STEP + ((k * 16 * 64) * sizeof(bf16) >> 4),
+                              IDESC_PV, (!first || k > 0) ? 1u : 0u);
+                t5_commit(&pv_done[g]);
+            };
+            bool ok = t5_wait(&q_full, 0, &abort_flag, status, row_base);
+            auto one_tile = [&](int j, int st) -> bool {          // st = j % 2, a constant where this is inlined
+                if (!t5_wait(&k_full[st], (j >> 1) & 1, &abort_flag, status, row_base)) return false;
+                t5_fence_after();
+                if (j < n0) qk(0, st);
+                if (j > 0) {
+                    if (j - 1 < n1) {
+                        if (!t5_wait(&p_full[1], (j - 1) & 1, &abort_flag, status, row_base)) return false;
+                        t5_fence_after();
+                        pv(1, 1 - st, j == 1);
+                    }
+                    t5_commit(&v_empty[1 - st]);                  // the last reader of the values of tile j - 1
+                }
+                if (j < n1) qk(1, st);
+                t5_commit(&k_empty[st]);
+                if (!t5_wait(&v_full[st], (j >> 1) & 1, &abort_flag, status, row_base)) return false;
+                if (j < n0) {
+                    if (!t5_wait(&p_full[0], j & 1, &abort_flag, status, row_base)) return false;
+                    t5_fence_after();
+                    pv(0, st, j == 0);
+                }
+                return true;
+            };
+            static_assert(LP_STAGES == 2, "the issue loop is unrolled by the number of stages");
+            for (int j = 0; ok && j < n_tiles; j += 2) {
+                ok = one_tile(j, 0);
+                if (ok && j + 1 < n_tiles) ok = one_tile(j + 1, 1);
+            }
+            if (ok && n1 == n_tiles && t5_wait(&p_full[1], (n1 - 1) & 1, &abort_flag, status, row_base)) {
+                t5_fence_after();
+                if ((n1 - 1) & 1) pv(1, 1, n1 == 1); else pv(1, 0, n1 == 1);
+            }
+        }
+    } else {
+        // ---- softmax: two threads share a query row, 48 columns of S each ----
+        const int wl = warp - 2;
+        const int g = wl >> 3;                                    // warps 2..9: the first query tile, 10..17: the second
+        const int half = (wl >> 2) & 1;                           // columns 48 * half .. + 47 of every tile
+        const int quarter = warp & 3;
+        const int row = quarter * 32 + lane;
+        const unsigned lane_addr = static_cast<unsigned>(quarter * 32) << 16;
+        const unsigned my_s = tmem + lane_addr + s_col(g) + half * 48;
+        const unsigned my_o = tmem + lane_addr + o_col(g) + half * 64;
+        const int rows_here = rows_of(g), mine = g ? n1 : n0;
+        const int pos_first = past + q0 + g * LP_BM;
+        const int pos = row < rows_here ? pos_first + row : -1;
+        const int lo = first_visible(pos, window), lo_last = first_visible(pos_first + rows_here - 1, window);
+        float m = -CUDART_INF_F, l = 0.0f;                        // m: the reference maximum, in units of log2
+        bool ok = true;
+        for (int j = 0; j < mine; ++j) {
+            const int kt = k_lo + j * LP_BN + half * 48;          // this thread's first key of the tile
+            // After a wait has run out (ok false) a thread still passes every barrier below, as often as the others.
+            if (ok && !t5_wait(&s_full[g], j & 1, &abort_flag, status, row_base)) ok = false;
+            t5_fence_after();
+            const bool full_tile = (kt + 47 <= pos_first) && (kt >= lo_last) && (rows_here == LP_BM);
+            unsigned r[48];
+            float mx = -CUDART_INF_F;
+            auto fetch = [&] {
+                lp_ld16(my_s, r, 0);
+                lp_ld16(my_s + 16, r, 16);
+                lp_ld16(my_s + 32, r, 32);
+                t5_wait_ld();
+            };
+            if (ok) {
+                fetch();
+                if (full_tile) {
+#pragma unroll
+                    for (int i = 0; i < 48; ++i) mx = fmaxf(mx, __uint_as_float(r[i]));
+                } else {
+#pragma unroll
+                    for (int i = 0; i < 48; ++i)
+                        if (kt + i <= pos && kt + i >= lo) mx = fmaxf(mx, __uint_as_float(r[i]));
+                }
+                x_max[j & 1][g][half][row] = mx;
+            }
+            asm volatile("bar.sync %0, 256;\n" ::"r"(1 + g) : "memory");      // the 8 softmax warps of this query tile
+            if (!ok) continue;
+            mx = fmaxf(mx, x_max[j & 1][g][half ^ 1][row]) * scale_log2e;     // scale > 0; -inf stays -inf
+            const bool adopt = (m == -CUDART_INF_F) && (mx > m);
+            const bool jump = (m != -CUDART_INF_F) && (mx > m + LP_JUMP);
+            if (__any_sync(0xffffffffu, jump)) {
+                // O still receives the previous tile's product: wait for it, then scale this thread's half of its row
+                if (!t5_wait(&pv_done[g], (j - 1) & 1, &abort_flag, status, row_base)) { ok = false; continue; }
+                t5_fence_after();
+                const float alpha = jump ? t5_ex2(m - mx) : 1.0f;
+                l *= alpha;
+#pragma unroll 1
+                for (int c = 0; c < 64; c += 32) {
+                    unsigned o[32];
+                    t5_ld32(my_o + c, o);
+                    t5_wait_ld();
+#pragma unroll
+                    for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
+                    t5_st32(my_o + c, o);
+                }
+                t5_wait_st();
+                fetch();
+            }
+            if (adopt || jump) m = mx;
+            const float msub = (m == -CUDART_INF_F) ? 0.0f : m;
+            unsigned pk[24];                                      // the weights, rounded to bfloat16, over the first half of this thread's S
+#pragma unroll
+            for (int i = 0; i < 48; i += 2) {
+                float p0 = t5_ex2(fmaf(__uint_as_float(r[i]), scale_log2e, -msub));
+                float p1 = t5_ex2(fmaf(__uint_as_float(r[i + 1]), scale_log2e, -msub));
+                if (!full_tile) {
+                    const int key = kt + i;
+                    p0 = (key <= pos && key >= lo) ? p0 : 0.0f;
+                    p1 = (key + 1 <= pos && key + 1 >= lo) ? p1 : 0.0f;
+                }
+                l += p0 + p1;
+                pk[i >> 1] = t5_pack(p0, p1);
+            }
+            lp_st8(my_s, pk, 0);
+            lp_st8(my_s + 8, pk, 8);
+            lp_st8(my_s + 16, pk, 16);
+            t5_wait_st();
+            t5_fence_before();
+            t5_arrive(&p_full[g]);
+        }
+        x_sum[g][half][row] = l;                                  // the row sum is the two halves' sums
+        asm volatile("bar.sync %0, 256;\n" ::"r"(1 + g) : "memory");
+        l += x_sum[g][half ^ 1][row];
+        if (ok && mine > 0 && t5_wait(&pv_done[g], (mine - 1) & 1, &abort_flag, status, row_base)) {
+            t5_fence_after();
+            float inv = (l > 0.0f) ? 1.0f / l : 0.0f;
+            if (gate && row < rows_here)                          // a sigmoid gate per token and head, on the result as it leaves
+                inv /= 1.0f + expf(-gate[static_cast<size_t>(row_base + g * LP_BM + row) * gate_stride + h]);
+            bf16* orow = out + (static_cast<size_t>(row_base + g * LP_BM + row) * H + h) * LP_DV + half * 64;
+#pragma unroll 1
+            for (int c = 0; c < 64; c += 32) {
+                unsigned o[32];
+                t5_ld32(my_o + c, o);
+                t5_wait_ld();
+                if (row < rows_here) {
+#pragma unroll
+                    for (int i = 0; i < 32; i += 8) {
+                        uint4 w;
+                        w.x = t5_pack(__uint_as_float(o[i]) * inv, __uint_as_float(o[i + 1]) * inv);
+                        w.y = t5_pack(__uint_as_float(o[i + 2]) * inv, __uint_as_float(o[i + 3]) * inv);
+                        w.z = t5_pack(__uint_as_float(o[i + 4]) * inv, __uint_as_float(o[i + 5]) * inv);
+                        w.w = t5_pack(__uint_as_float(o[i + 6]) * inv, __uint_as_float(o[i + 7]) * inv);
+                        *reinterpret_cast<uint4*>(orow + c + i) = w;
+                    }
+                }
+            }
+        }
+    }
+    t5_fence_before();
+    __syncthreads();
+    if (warp == 1) {
+        t5_fence_after();
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(512u) : "memory");
+    }
+}
+
+// ---- the rows of the portions, and the queries --------------------------------------------------------------------
+// grid (row groups of 8, segments), a warp a row: position first + i of the segment's request, zeros beyond its last one.
+__global__ void latent_gather_kernel(const bf16* __restrict__ rows_cache, long long page_stride, bf16* __restrict__ out,
+                                     const int32_t* __restrict__ segs, const int32_t* __restrict__ entry_slot,
+                                     const int32_t* __restrict__ entry_kv_len, const int32_t* __restrict__ block_table,
+                                     int table_stride, int DK, int page_size, int num_pages, int32_t* __restrict__ status) {
+    pdl_begin();
+    const int* s = segs + 4 * blockIdx.y;
+    const int i = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (i >= s[3]) return;
+    const int e = s[0], pos = s[1] + i;
+    const bf16* src = nullptr;
+    if (pos < entry_kv_len[e]) {
+        const int logical = pos / page_size;
+        const int page = logical < table_stride ? block_table[static_cast<size_t>(entry_slot[e]) * table_stride + logical] : -1;
+        if (page < 0 || page >= num_pages) {
+            if (lane == 0 && atomicCAS(status, 0, 4) == 0) status[1] = s[2] + i;
+        } else {
+            src = rows_cache + static_cast<long long>(page) * page_stride + static_cast<size_t>(pos - logical * page_size) * DK;
+        }
+    }
+    bf16* dst = out + static_cast<size_t>(s[2] + i) * DK;
+    for (int c = lane; c < DK / 8; c += 32)
+        *reinterpret_cast<uint4*>(dst + 8 * c) = src ? *reinterpret_cast<const uint4*>(src + 8 * c) : make_uint4(0u, 0u, 0u, 0u);
+}
+
+// One block a token: q float32 [T, H * (D + P)] -> bfloat16 of the same layout, the first `dims` entries of every head's
+// P-part rotated (pairs as in latent_attention.cu).  The angles of a token are made once for all heads.
+__global__ void latent_q_pack_kernel(const float* __restrict__ q, bf16* __restrict__ out, const int32_t* __restrict__ positions,
+                                     const float* __restrict__ inv_freq, int H, int D, int P, int dims, int rot_pairs, float rot_mag) {
+    pdl_begin();
+    extern __shared__ float2 turn[];                              // (cos, sin) of the token's angles, times the magnitude
+    const int t = blockIdx.x, half = dims / 2, W = D + P;
+    const float pos = static_cast<float>(positions[t]);
+    for (int f = threadIdx.x; f < half; f += blockDim.x) {
+        float sn, cs;
+        sincosf(pos * inv_freq[f], &sn, &cs);
+        turn[f] = make_float2(cs * rot_mag, sn * rot_mag);
+    }
+    __syncthreads();
+    const float* src = q + static_cast<size_t>(t) * H * W;
+    bf16* dst = out + static_cast<size_t>(t) * H * W;
+    for (int i = threadIdx.x; i < H * (W / 8); i += blockDim.x) {
+        const int h = i / (W / 8), c = (i - h * (W / 8)) * 8;
+        const float* hd = src + h * W;
+        float v[8];
+        load8(hd + c, v);
+        if (c >= D) {
+#pragma unroll
+            for (int u = 0; u < 8; ++u) {
+                const int k = c - D + u;
+                if (k < dims) {
+                    const bool first = rot_pairs ? (k & 1) == 0 : k < half;
+                    const int f = rot_pairs ? k >> 1 : (first ? k : k - half);
+                    const float other = hd[D + (rot_pairs ? k ^ 1 : (first ? k + half : k - half))];
+                    const float2 cs = turn[f];
+                    v[u] = first ? v[u] * cs.x - other * cs.y : v[u] * cs.x + other * cs.y;
+                }
+            }
+        }
+        store8(dst + h * W + c, v);
+    }
+}
+
+extern "C" int llm_latent_prefill_supported(int D, int V, int R, int P) {
+    return D == 128 && V == LP_DV && P == 64 && R > 0 && R % 8 == 0;
+}
+extern "C" int llm_latent_prefill_tile_rows() { return 2 * LP_BM; }
+extern "C" int llm_latent_prefill_tile_keys() { return LP_BN; }
+
+// rows_cache: bfloat16 [pages, 1, page, DK] with `page_stride`; out: bfloat16 [total rows, DK]; segs as above, every first
+// gathered row and row count a multiple of the key tile; most_rows: the largest count.
+extern "C" int llm_latent_gather(const void* rows_cache, long long page_stride, void* out, const int32_t* segs, int n_segs,
+                                 int most_rows, const int32_t* entry_slot, const int32_t* entry_kv_len,
+                                 const int32_t* block_table, int table_stride, int DK, int page_size, int num_pages,
+                                 int32_t* status, uintptr_t stream) {
+    if (n_segs <= 0 || most_rows <= 0) return LLM_OK;
+    if (n_segs > 65535 || DK <= 0 || DK % 8 || page_size <= 0) return LLM_REFUSED_SIZE;
+    if (!aligned16(rows_cache) || !aligned16(out) || page_stride % 8) return LLM_REFUSED_ALIGN;
+    launch_pdl(latent_gather_kernel, dim3((most_rows + 7) / 8, n_segs), dim3(256), 0, reinterpret_cast<cudaStream_t>(stream),
+               static_cast<const bf16*>(rows_cache), page_stride, static_cast<bf16*>(out), segs, entry_slot, entry_kv_len,
+               block_table, table_stride, DK, page_size, num_pages, status);
+    return launch_status();
+}
+
+extern "C" int llm_latent_q_pack(const float* q, void* out, const int32_t* positions, const float* inv_freq, int num_tokens, int H,
+                                 int D, int P, int dims, int rot_pairs, float rot_mag, uintptr_t stream) {
+    if (num_tokens <= 0) return LLM_OK;
+    if (H <= 0 || D <= 0 || P < 0 || D % 8 || P % 8 || dims < 0 || dims > P || dims % 2 || (dims > 0 && !inv_freq)) return LLM_REFUSED_SIZE;
+    if (!aligned16(q) || !aligned16(out)) return LLM_REFUSED_ALIGN;
+    launch_pdl(latent_q_pack_kernel, dim3(num_tokens), dim3(256), sizeof(float2) * (dims / 2), reinterpret_cast<cudaStream_t>(stream),
+               q, static_cast<bf16*>(out), positions, inv_freq, H, D, P, dims, rot_pairs, rot_mag);
+    return launch_status();
+}
+
+// q: bfloat16 [num_tokens, H * 192]; kv: bfloat16 [rows, H * 256] = per head [k | v]; gathered: bfloat16 [rows, R + 64];
+// out: bfloat16 [num_tokens, H * 128]; gate: null, or float32, token t's and head h's at t * gate_stride + h, the result is
+// multiplied by its sigmoid.
+extern "C" int llm_latent_prefill(const void* q, const void* kv, const void* gathered, void* out, int num_tokens, int rows,
+                                  const int32_t* tiles, int n_tiles, const int32_t* segs, const int32_t* entry_q_start,
+                                  const int32_t* entry_q_len, const int32_t* entry_kv_len, int H, int R, int window, float scale,
+                                  const float* gate, long long gate_stride, int32_t* status, uintptr_t stream) {
+    if (n_tiles <= 0) return LLM_OK;
+    if (H <= 0 || n_tiles > 65535 || !llm_latent_prefill_supported(128, LP_DV, R, 64) || rows <= 0 || rows % LP_BN || !(scale > 0.0f) ||
+        window < 0)
+        return LLM_REFUSED_SIZE;
+    if (!aligned16(q) || !aligned16(kv) || !aligned16(gathered) || !aligned16(out)) return LLM_REFUSED_ALIGN;
+    CUtensorMap q_map, kv_map, r_map;
+    if (!t5_encode_2d(&q_map, q, static_cast<long long>(H) * LP_DK, num_tokens, 64, LP_BM) ||
+        !t5_encode_2d(&kv_map, kv, static_cast<long long>(H) * 256, rows, 64, LP_BN) ||
+        !t5_encode_2d(&r_map, gathered, R + 64, rows, 64, LP_BN))
+        return LLM_REFUSED_SIZE;
+    const size_t smem = static_cast<size_t>(2 * 3 * LP_QB + LP_STAGES * 5 * LP_KB) * sizeof(bf16) + 1024;
+    const cudaError_t e = cudaFuncSetAttribute(latent_prefill_tcgen05_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+    if (e != cudaSuccess) return static_cast<int>(e);
+    launch_pdl(latent_prefill_tcgen05_kernel, dim3(H, n_tiles), dim3(LP_THREADS), smem, reinterpret_cast<cudaStream_t>(stream), q_map,
+               kv_map, r_map, static_cast<bf16*>(out), tiles, segs, entry_q_start, entry_q_len, entry_kv_len, H, R, window,
+               scale * 1.4426950408889634f, gate, gate_stride, status);
+    return launch_status();
+}

@@ -884,6 +884,75 @@ def latent_attention(q: torch.Tensor, rows_cache: torch.Tensor, positions, token
 GLA_FULL, GLA_LOCAL, GLA_OUT = 0, 1, 2
 
 
+def latent_prefill_supported(D: int, V: int, R: int, P: int) -> bool:
+    """Whether the tcgen05 kernel for prompt portions of latent attention (rows mapped to per-head keys and values first)
+    takes heads of D + P key and V value entries over latents of R."""
+    if D != 128 or V != 128 or P != 64:      # do not compile it just to hear "no"
+        return False
+    return bool(_fn("latent_prefill_tcgen05", "llm_latent_prefill_supported", [c_int, c_int, c_int, c_int])(D, V, R, P))
+
+
+LATENT_TILE_ROWS, LATENT_TILE_KEYS = 256, 96        # query rows of a work item, and what a request's gathered rows are padded to
+
+
+def latent_gather(rows_cache: torch.Tensor, segs: torch.Tensor, n_segs: int, total_rows: int, most_rows: int, entry_slot,
+                  entry_kv_len, block_table: torch.Tensor, page_size: int, status: torch.Tensor) -> torch.Tensor:
+    """The cached rows [pages, 1, page, n] of `n_segs` requests as one bfloat16 [total_rows, n].  segs int32 [n_segs, 4] =
+    (entry, first position, first row, rows); rows beyond a request's last position are zero."""
+    _dev(segs, entry_slot, entry_kv_len, block_table, status)
+    if rows_cache.dtype != torch.bfloat16 or rows_cache.dim() != 4 or rows_cache[0].stride() != (
+            page_size * rows_cache.shape[3], rows_cache.shape[3], 1):
+        raise KernelError("rows_cache must be bfloat16 [pages, 1, page, n] with dense pages")
+    DK = rows_cache.shape[3]
+    out = torch.empty((total_rows, DK), dtype=torch.bfloat16, device=rows_cache.device)
+    f = _fn("latent_prefill_tcgen05", "llm_latent_gather",
+            [c_void_p, c_longlong, c_void_p, c_void_p, c_int, c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int,
+             c_void_p, c_void_p])
+    _check(f(_ptr(rows_cache), rows_cache.stride(0), _ptr(out), _ptr(segs), n_segs, most_rows, _ptr(entry_slot), _ptr(entry_kv_len),
+             _ptr(block_table), block_table.shape[1], DK, page_size, rows_cache.shape[0], _ptr(status), _stream()), "latent_gather")
+    return out
+
+
+def latent_q_pack(q: torch.Tensor, positions: torch.Tensor, inv_freq: Optional[torch.Tensor], H: int, D: int, P: int, dims: int,
+                  rot_pairs: bool = False, rot_mag: float = 1.0) -> torch.Tensor:
+    """float32 [T, H * (D + P)] -> bfloat16 of the same layout, the first `dims` entries of each head's P-part rotated."""
+    _dev(q, positions, inv_freq)
+    T = q.shape[0]
+    if q.dtype != torch.float32 or tuple(q.shape) != (T, H * (D + P)):
+        raise KernelError("q must be float32 [T, heads * (unrotated + rotated)]")
+    out = torch.empty((T, H * (D + P)), dtype=torch.bfloat16, device=q.device)
+    f = _fn("latent_prefill_tcgen05", "llm_latent_q_pack",
+            [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_void_p])
+    _check(f(_ptr(q), _ptr(out), _ptr(positions), _ptr(inv_freq), T, H, D, P, dims, 1 if rot_pairs else 0, float(rot_mag), _stream()),
+           "latent_q_pack")
+    return out
+
+
+def latent_prefill(q: torch.Tensor, kv: torch.Tensor, gathered: torch.Tensor, out: torch.Tensor, tiles: torch.Tensor, n_tiles: int,
+                   segs: torch.Tensor, entry_q_start, entry_q_len, entry_kv_len, H: int, R: int, window: Optional[int], scale: float,
+                   status: torch.Tensor, gate: Optional[torch.Tensor] = None, gate_off: int = 0) -> torch.Tensor:
+    """Causal attention of prompt portions over per-head keys and values: q bfloat16 [T, H * 192], kv bfloat16 [rows, H * 256]
+    (per head keys of 128, then values of 128), gathered bfloat16 [rows, R + 64] (its last 64 columns: the key part that all
+    heads share), out bfloat16 [T, H * 128].  tiles int32 [n, 2] = (segment, first query row), 256 rows each.  With `gate`
+    (float32 [T, m]) a head's result is multiplied by the sigmoid of column gate_off + head."""
+    _dev(q, kv, gathered, out, tiles, segs, entry_q_start, entry_q_len, entry_kv_len, status)
+    T, rows = q.shape[0], gathered.shape[0]
+    if (tuple(q.shape) != (T, H * 192) or tuple(kv.shape) != (rows, H * 256) or gathered.shape[1] != R + 64
+            or tuple(out.shape) != (T, H * 128) or any(t.dtype != torch.bfloat16 for t in (q, kv, gathered, out))):
+        raise KernelError("latent_prefill: shapes or types disagree")
+    if gate is not None and (gate.dtype != torch.float32 or gate.dim() != 2 or gate.shape[0] != T or gate.stride(1) != 1
+                             or not gate.is_cuda or gate_off < 0 or gate_off + H > gate.shape[1]):
+        raise KernelError("the gate must be float32 [T, m] with unit stride along its rows and hold the heads' columns")
+    f = _fn("latent_prefill_tcgen05", "llm_latent_prefill",
+            [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_int,
+             c_int, c_int, c_float, c_void_p, c_longlong, c_void_p, c_void_p])
+    _check(f(_ptr(q), _ptr(kv), _ptr(gathered), _ptr(out), T, rows, _ptr(tiles), n_tiles, _ptr(segs), _ptr(entry_q_start),
+             _ptr(entry_q_len), _ptr(entry_kv_len), H, R, int(window) if window else 0, float(scale),
+             gate.data_ptr() + 4 * gate_off if gate is not None else None, gate.stride(0) if gate is not None else 0, _ptr(status),
+             _stream()), "latent_prefill")
+    return out
+
+
 def gla_supported(d: int, v: int) -> bool:
     return bool(_fn("linear_attention", "llm_gla_supported", [c_int, c_int])(d, v))
 

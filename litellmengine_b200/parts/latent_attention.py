@@ -2,16 +2,68 @@
 from __future__ import annotations
 
 import math
+from dataclasses import dataclass
 from typing import Dict, Optional
 
+import numpy as np
 import torch
 
 from ..cache import PagedNeed
 from ..config.specs import MixerSpec
 from ..csrc import ops
 from ..weights.loader import ParamSpec
-from .context import StageContext
+from .context import StageContext, StepPrelude
 from .registry import lookup, register_mixer
+
+
+class LatentWork(StepPrelude):
+    """How a long prompt step of latent attention is cut: the requests that bring several tokens as segments (entry, first
+    position some query of it sees, first gathered row, rows padded to whole key tiles) and tiles of 256 query rows of them,
+    longest walk first; the rows of the others, which bring one.  Filled only for steps of at least `FROM` tokens."""
+    # Shorter steps are replayed as captured graphs that serve any division of their tokens among requests, and what is
+    # allocated here depends on how many rows the requests have cached.  (At 1,024 tokens of one request the cached-row
+    # kernel takes 340 us, the expanded path about 90.)
+    FROM = 1025
+
+    @dataclass
+    class Views:
+        tiles: torch.Tensor              # int32 [n, 2]
+        segs: torch.Tensor               # int32 [n, 4]
+        rows: torch.Tensor               # int32 [n] rows of the batch that are single tokens
+        num_tiles: int
+        num_segs: int
+        num_single: int
+        gathered: int                    # rows of all segments
+        longest: int                     # and of the longest
+
+    def __init__(self, window: Optional[int]):
+        self.window = window
+        self.name = f"latent_work:{window or 0}"
+
+    def sections(self, max_tokens: int, max_entries: int):
+        return {"tiles": 2 * (max_tokens // ops.LATENT_TILE_ROWS + max_entries + 1), "segs": 4 * max_entries, "rows": max_entries}
+
+    def fill(self, facts, out):
+        if facts.num_tokens < self.FROM:
+            return 0, 0, 0, 0, 0
+        several = np.nonzero(facts.q_len > 1)[0]
+        single = facts.q_start[facts.q_len == 1]
+        out["rows"][:len(single)] = single
+        past, n = facts.past[several], facts.q_len[several]
+        first = np.maximum(past - self.window + 1, 0) if self.window else np.zeros_like(past)
+        K, R = ops.LATENT_TILE_KEYS, ops.LATENT_TILE_ROWS
+        rows = -(-(past + n - first) // K) * K
+        start = np.cumsum(rows) - rows
+        out["segs"][:4 * len(several)] = np.stack([several, first, start, rows], axis=1).reshape(-1)
+        tiles = [(i, q0) for i in range(len(several)) for q0 in range(0, int(n[i]), R)]
+        tiles.sort(key=lambda t: -(int(past[t[0]] - first[t[0]]) + t[1]))
+        out["tiles"][:2 * len(tiles)] = np.asarray(tiles, dtype=np.int64).reshape(-1)
+        return len(tiles), len(several), len(single), int(rows.sum()), int(rows.max()) if len(rows) else 0
+
+    def views(self, dev, filled):
+        n, segs, single, gathered, longest = filled
+        return LatentWork.Views(dev["tiles"][:2 * n].view(n, 2), dev["segs"][:4 * segs].view(segs, 4), dev["rows"][:single], n, segs,
+                                single, gathered, longest)
 
 
 @register_mixer("latent_attention")
@@ -35,7 +87,10 @@ class LatentAttentionMixer:
     One product yields [dq | dkv | g] per token in float32; `latent_prepare` norms both latents, rotates kr and
     writes the page row; W_uq; `latent_q_split` rotates qr and lays qn out head-major; a batched product with
     W_uk^T fills q_abs; attention (bfloat16: the tensor-core kernel in which all heads of a token share each staged
-    tile of rows; float32: the general kernel); a batched product with W_uv^T; the gate; W_o."""
+    tile of rows; float32: the general kernel); a batched product with W_uv^T; the gate; W_o.
+
+    Long prompt steps (bfloat16, heads of 128 + 64 and 128) turn that around: where many queries meet every row it is
+    cheaper to map the rows to per-head keys and values once, and attend to those (`_expanded`)."""
 
     graph_safe = True           # kernels and library products on the current stream only
     any_division_safe = True    # nothing is shaped by the number of entries
@@ -80,6 +135,8 @@ class LatentAttentionMixer:
         # bfloat16 on the tensor-core kernel over the cached rows; float32 (and other latent sizes) on the general kernel
         self.tensor_core = (compute_dtype == torch.bfloat16 and self.device.type == "cuda"
                             and ops.latent_attention_supported(self.R, self.P))
+        self.expands = (self.tensor_core and self.scale > 0 and ops.latent_prefill_supported(self.D, self.V, self.R, self.P))
+        self._expand = None         # (W_ukv [H * (D + V), R],): per head the key map, then the value map, for long prompt steps
         self.w_in = self.w_uq = self.w_uk_t = self.w_uv_t = self.w_o = None
         self.wq_norm = self.wkv_norm = None
 
@@ -106,6 +163,8 @@ class LatentAttentionMixer:
         # per head: [D, R] (q_abs = qn W_uk) and [R, V] (value = latent sum times W_uv^T), the batched products' right sides
         self.w_uk_t = t[n["uk"]].view(self.H, self.D, self.R).contiguous()
         self.w_uv_t = t[n["uv"]].view(self.H, self.V, self.R).transpose(1, 2).contiguous()
+        if self.expands and t[n["uk"]].dtype == t[n["uv"]].dtype == torch.bfloat16:
+            self._expand = (torch.cat([self.w_uk_t, t[n["uv"]].view(self.H, self.V, self.R)], dim=1).view(-1, self.R),)
         self.wq_norm = t[n["dq_norm"]].float().contiguous()
         if s.has_kv:
             self.wkv_norm = t[n["dkv_norm"]].float().contiguous()
@@ -117,6 +176,65 @@ class LatentAttentionMixer:
             return None
         return PagedNeed(1, self.R + self.P, self.keep_window, 0)       # keys only: the values are part of the key rows
 
+    # Keys and values of all rows of a step that are made at once at most: a step whose requests have cached more (over
+    # 65,536 rows at 32 heads) stays on the cached-row kernel, which needs nothing per row.
+    EXPANDED_BYTES = 1 << 30
+
+    @property
+    def _work_name(self):
+        return f"latent_work:{self.spec.window or 0}"
+
+    def step_prelude(self):
+        return LatentWork(self.spec.window) if self.expands else None
+
+    def _absorbed(self, q: torch.Tensor, positions: torch.Tensor, token_entry: torch.Tensor, ctx: StageContext) -> torch.Tensor:
+        """Attention over the cached rows themselves: q float32 [n, H * (D + P)] of n tokens -> [n, H * V]."""
+        b, s = ctx.batch, self.spec
+        H, D, P, R, V, T = self.H, self.D, self.P, self.R, self.V, q.shape[0]
+        qn, packed = ops.latent_q_split(q, positions, self.inv_freq, H, D, P, R, self.rot_dims, self.dtype,
+                                        rot_pairs=self.rot_pairs, rot_mag=self.rot_mag)
+        # q_abs[h] = qn[h] W_uk[h], written into the first R columns of head h of the packed query
+        torch.bmm(qn, self.w_uk_t if self.w_uk_t.dtype == qn.dtype else self.w_uk_t.to(qn.dtype),
+                  out=packed.view(T, H, R + P)[:, :, :R].permute(1, 0, 2))
+        lat = torch.empty((T, H * R), dtype=self.dtype, device=q.device)
+        if self.tensor_core:
+            ops.latent_attention(packed, ctx.cache_keys, positions, token_entry, b.entry_slot, ctx.block_table, H, R, P,
+                                 ctx.page_size, s.window, self.scale, ctx.status, lat)
+        else:
+            ops.paged_attention_generic_kv(packed, ctx.cache_keys, None, positions, token_entry, b.entry_slot,
+                                           ctx.block_table, H, 1, R + P, R, ctx.page_size, s.window, self.scale, ctx.status,
+                                           lat, values_in_keys=True)
+        heads = torch.empty((T, H * V), dtype=self.dtype, device=q.device)
+        torch.bmm(lat.view(T, H, R).permute(1, 0, 2), self.w_uv_t if self.w_uv_t.dtype == lat.dtype else self.w_uv_t.to(lat.dtype),
+                  out=heads.view(T, H, V).permute(1, 0, 2))
+        return heads
+
+    def _gated(self, heads: torch.Tensor, proj: torch.Tensor) -> torch.Tensor:
+        if self.spec.output_gate:
+            ops.gate_mul(heads, proj, self.g_off, heads, 0, self.spec.output_gate, per_head=self.V if self.gate_per_head else 0)
+        return heads
+
+    def _expanded(self, q: torch.Tensor, proj: torch.Tensor, work: LatentWork.Views, ctx: StageContext) -> torch.Tensor:
+        """Portions of several tokens over per-head keys and values made from their requests' rows (a gate per head is applied
+        as the kernel stores); single tokens of the same step over the rows themselves."""
+        b, s = ctx.batch, self.spec
+        H, D, P, R, V, T = self.H, self.D, self.P, self.R, self.V, q.shape[0]
+        rows = ops.latent_gather(ctx.cache_keys, work.segs, work.num_segs, work.gathered, work.longest, b.entry_slot, b.entry_kv_len,
+                                 ctx.block_table, ctx.page_size, ctx.status)
+        kv = torch.mm(rows[:, :R], self._expand[0].t())
+        packed = ops.latent_q_pack(q, b.positions, self.inv_freq, H, D, P, self.rot_dims, rot_pairs=self.rot_pairs, rot_mag=self.rot_mag)
+        heads = torch.empty((T, H * V), dtype=self.dtype, device=q.device)
+        ops.latent_prefill(packed, kv, rows, heads, work.tiles, work.num_tiles, work.segs, b.entry_q_start, b.entry_q_len,
+                           b.entry_kv_len, H, R, s.window, self.scale, ctx.status, gate=proj if self.gate_per_head else None,
+                           gate_off=self.g_off)
+        if not self.gate_per_head:
+            heads = self._gated(heads, proj)
+        if work.num_single:
+            pick = work.rows.long()
+            one = self._absorbed(q.index_select(0, pick), b.positions.index_select(0, pick), b.token_entry.index_select(0, pick), ctx)
+            heads.index_copy_(0, pick, self._gated(one, proj.index_select(0, pick)))
+        return heads
+
     def forward(self, x: torch.Tensor, ctx: StageContext):
         b, s = ctx.batch, self.spec
         if s.has_kv != ctx.writes_cache:
@@ -127,22 +245,9 @@ class LatentAttentionMixer:
                                 self.eps, self.inv_freq, ctx.cache_keys if s.has_kv else None, b, ctx.block_table,
                                 ctx.page_size, ctx.status, self.dtype, rot_pairs=self.rot_pairs, rot_mag=self.rot_mag)
         q = ops.as_tensor(ops.linear(cq, self.w_uq, out_dtype=torch.float32))
-        qn, packed = ops.latent_q_split(q, b.positions, self.inv_freq, H, D, P, R, self.rot_dims, self.dtype,
-                                        rot_pairs=self.rot_pairs, rot_mag=self.rot_mag)
-        # q_abs[h] = qn[h] W_uk[h], written into the first R columns of head h of the packed query
-        torch.bmm(qn, self.w_uk_t if self.w_uk_t.dtype == qn.dtype else self.w_uk_t.to(qn.dtype),
-                  out=packed.view(T, H, R + P)[:, :, :R].permute(1, 0, 2))
-        lat = torch.empty((T, H * R), dtype=self.dtype, device=x.device)
-        if self.tensor_core:
-            ops.latent_attention(packed, ctx.cache_keys, b.positions, b.token_entry, b.entry_slot, ctx.block_table, H, R, P,
-                                 ctx.page_size, s.window, self.scale, ctx.status, lat)
+        work = b.preludes.get(self._work_name) if self._expand is not None else None
+        if work is not None and work.num_tiles and 2 * work.gathered * H * (D + V) <= self.EXPANDED_BYTES:
+            heads = self._expanded(q, proj, work, ctx)
         else:
-            ops.paged_attention_generic_kv(packed, ctx.cache_keys, None, b.positions, b.token_entry, b.entry_slot,
-                                           ctx.block_table, H, 1, R + P, R, ctx.page_size, s.window, self.scale, ctx.status,
-                                           lat, values_in_keys=True)
-        heads = torch.empty((T, H * V), dtype=self.dtype, device=x.device)
-        torch.bmm(lat.view(T, H, R).permute(1, 0, 2), self.w_uv_t if self.w_uv_t.dtype == lat.dtype else self.w_uv_t.to(lat.dtype),
-                  out=heads.view(T, H, V).permute(1, 0, 2))
-        if s.output_gate:
-            ops.gate_mul(heads, proj, self.g_off, heads, 0, s.output_gate, per_head=V if self.gate_per_head else 0)
+            heads = self._gated(self._absorbed(q, b.positions, b.token_entry, ctx), proj)
         return ops.linear(heads, self.w_o, out_dtype=torch.float32, partials_ok=getattr(ctx, "partials_ok", False))

@@ -1,0 +1,119 @@
+"""Long prompt steps of latent attention: the path that maps the cached rows to per-head keys and values against the
+path over the rows themselves, and its kernels against float64."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+F64 = torch.float64
+
+
+def ops():
+    from litellmengine_b200.csrc import ops as o
+    return o
+
+
+@pytest.mark.parametrize("H,R,window", [(1, 64, None), (3, 128, None), (2, 512, 100), (2, 512, 1), (3, 256, 300)])
+def test_kernels(H, R, window):
+    """(cached after the step, queries at the end) around the edges of 96 keys and of 128 and 256 query rows."""
+    o = ops()
+    g = torch.Generator(device=DEV).manual_seed(H * 100 + R)
+    reqs = [(2, 2), (96, 96), (97, 97), (130, 129), (256, 256), (400, 257), (500, 3), (900, 300)]
+    page, DK, K = 16, R + 64, o.LATENT_TILE_KEYS
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)
+    width = max(-(-n // page) for n, _ in reqs)
+    order = torch.randperm(len(reqs) * width, generator=g, device=DEV).to(torch.int32)
+    table = order.view(len(reqs), width).contiguous()
+    cache = torch.full((len(reqs) * width, 1, page, DK), float("nan"), device=DEV, dtype=torch.bfloat16)
+    rows = [torch.randn(n, DK, generator=g, device=DEV).to(torch.bfloat16) for n, _ in reqs]
+    for b, r in enumerate(rows):
+        j = torch.arange(len(r), device=DEV)
+        cache[table[b, j // page].long(), 0, j % page] = r
+    T = sum(t for _, t in reqs)
+    starts = [sum(t for _, t in reqs[:b]) for b in range(len(reqs))]
+    first = [max(0, n - t - window + 1) if window else 0 for n, t in reqs]
+    count = [-(-(n - f) // K) * K for (n, _), f in zip(reqs, first)]
+    at = [sum(count[:b]) for b in range(len(reqs))]
+    segs, status = i32([list(x) for x in zip(range(len(reqs)), first, at, count)]), i32([0, 0])
+    slots, q_len, kv_len = i32(list(range(len(reqs)))), i32([t for _, t in reqs]), i32([n for n, _ in reqs])
+    gathered = o.latent_gather(cache, segs, len(reqs), sum(count), max(count), slots, kv_len, table, page, status)
+    want = torch.zeros(sum(count), DK, device=DEV, dtype=torch.bfloat16)
+    for (n, _), f, a, r in zip(reqs, first, at, rows):
+        want[a:a + n - f] = r[f:]
+    assert torch.equal(gathered, want)
+    w = (torch.randn(H * 256, R, generator=g, device=DEV) * R ** -0.5).to(torch.bfloat16)
+    kv = torch.mm(gathered[:, :R], w.t())
+    q32 = torch.randn(T, H * 192, generator=g, device=DEV)
+    pos = i32([p for n, t in reqs for p in range(n - t, n)])
+    inv = torch.rand(32, generator=g, device=DEV)
+    for pairs in (False, True):
+        qp = o.latent_q_pack(q32, pos, inv, H, 128, 64, 64, rot_pairs=pairs, rot_mag=1.25)
+        qn, packed = o.latent_q_split(q32, pos, inv, H, 128, 64, R, 64, torch.bfloat16, rot_pairs=pairs, rot_mag=1.25)
+        assert torch.equal(qp.view(T, H, 192)[..., :128].permute(1, 0, 2), qn)
+        assert torch.allclose(qp.view(T, H, 192)[..., 128:].float(), packed.view(T, H, DK)[..., R:].float(), rtol=2 ** -7, atol=1e-6)
+    R2 = o.LATENT_TILE_ROWS
+    tiles = i32([(b, r) for b, (_, t) in enumerate(reqs) for r in range(0, t, R2)])
+    out = torch.full((T, H * 128), 7.0, device=DEV, dtype=torch.bfloat16)
+    scale = 192 ** -0.5
+    gate = torch.randn(T, H + 5, generator=g, device=DEV) if R == 512 else None
+    o.latent_prefill(qp, kv, gathered, out, tiles, len(tiles), segs, i32(starts), q_len, kv_len, H, R, window, scale, status,
+                     gate=gate, gate_off=3)
+    assert status.tolist() == [0, 0]
+    share = torch.sigmoid(gate[:, 3:3 + H].to(F64)) if gate is not None else torch.ones(T, H, device=DEV, dtype=F64)
+    for b, (n, t) in enumerate(reqs):
+        a, f = at[b], first[b]
+        kh = kv[a:a + n - f].view(n - f, H, 256).to(F64)
+        k = torch.cat([kh[..., :128], gathered[a:a + n - f, None, R:].to(F64).expand(n - f, H, 64)], -1)
+        qq = qp[starts[b]:starts[b] + t].view(t, H, 192).to(F64)
+        s = torch.einsum("thd,shd->hts", qq, k) * scale
+        i, j = torch.arange(n - t, n, device=DEV)[:, None], torch.arange(f, n, device=DEV)[None, :]
+        see = (j <= i) & ((i - j < window) if window else True)
+        p = torch.softmax(s.masked_fill(~see, float("-inf")), -1)
+        ref = torch.einsum("hts,shd->thd", p, kh[..., 128:])
+        share_b = share[starts[b]:starts[b] + t, :, None]
+        ref = ref * share_b
+        got = out[starts[b]:starts[b] + t].view(t, H, 128).to(F64)
+        # weights and result rounded to bfloat16 (2^-9 each), the weights' errors weighted by the values they meet
+        bound = 2 ** -8 * (ref.abs() + share_b * torch.einsum("hts,shd->thd", p, kh[..., 128:].abs())) + 1e-3
+        assert bool(((got - ref).abs() <= bound).all()), (n, t, float(((got - ref).abs() / bound).max()))
+
+
+@pytest.mark.parametrize("window", [None, 200])
+def test_long_step_of_every_kind_of_entry(window):
+    """Portions with and without earlier tokens beside single tokens, in one step, over both paths."""
+    from litellmengine_b200.config import config_from_dict
+    from litellmengine_b200.engine import ModelRunner, StepEntry
+    m = {"heads": 3, "dim": 128, "rot_dim": 64, "vdim": 128, "q_rank": 96, "kv_rank": 128, "scale": 192 ** -0.5,
+         "rot": {"base": 10000.0, "dims": 64}}
+    if window:
+        m["mask"] = {"size": window}
+    cfg = {"architecture": "Vugedra", "vocab": 64, "width": 256, "norm": {"eps": 1e-5},
+           "layers": [{"type": "latent_attention", "mixer": m, "mlp": None}]}
+    runner = ModelRunner.from_config(config_from_dict(cfg), seed=3, device=DEV, max_total_tokens=8192, max_requests=8, max_tokens_per_step=2048)
+    mixer = runner.model.blocks[0].mixer
+    past, new = [0, 130, 500, 77, 400, 0], [700, 1, 260, 129, 1, 2]
+    g = torch.Generator(device=DEV).manual_seed(1)
+    slots = [runner.admit() for _ in past]
+    x = lambda n: torch.randn(n, 256, generator=g, device=DEV).to(torch.bfloat16)
+    for s, p in zip(slots, past):
+        if p:
+            b = runner.prepare([StepEntry(s, [0] * p)])
+            mixer.forward(x(p), runner.model.stage_context(0, b, runner.cache))
+            runner.finish(b)
+    b = runner.prepare([StepEntry(s, [0] * n) for s, n in zip(slots, new)])
+    ctx, xs = runner.model.stage_context(0, b, runner.cache), x(sum(new))
+    assert sum(new) >= 1025 and mixer._expand is not None
+    before = ops().launch_count
+    got = mixer.forward(xs, ctx)
+    launched = ops().launch_count - before
+    held, mixer._expand = mixer._expand, None
+    ref = mixer.forward(xs, ctx)
+    mixer._expand = held
+    # both paths round queries, keys (or folded queries) and sums to bfloat16 a handful of times, 2^-9 each
+    err = (got - ref).double().norm(dim=1) / ref.double().norm(dim=1)
+    assert float(err.max()) < 6 * 2 ** -8, float(err.max())
+    assert launched > 5
+    runner.check_status()
+    limit, mixer.EXPANDED_BYTES = mixer.EXPANDED_BYTES, 1000          # more rows than may be expanded at once: the other path
+    assert torch.equal(mixer.forward(xs, ctx), ref)
+    mixer.EXPANDED_BYTES = limit
