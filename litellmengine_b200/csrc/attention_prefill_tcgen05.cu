@@ -338,14 +338,31 @@ __global__ void __launch_bounds__(64 + 128 * HEADS, 1) paged_prefill_attention_t
 // before the barrier that they all pass once a tile.  Three tables take turns: a thread that is late with tile j
 // may still read table j after that barrier (when it has to fetch its scores a second time) while an early one
 // already writes the table of tile j + 2.
-template <bool BIAS>
+// EXT: a window that keeps the sequence's first `keep_first` keys (the tiles that hold them and lie wholly below the
+// window's first tile are walked first; kept keys inside the window's tiles are a matter of the mask), one more term
+// exp(sinks[head]) in the softmax's denominator, a sigmoid gate per head (column gate_off + head of a float32 row per
+// token), a factor, and a result that is a column range of a wider buffer.  Measured, 32 heads over 8, window 1,024, four
+// kept keys, learned sinks, 2,500 tokens: 219 us on mma.sync (attention_prefill.cu), 80 us here.
+struct T5Ext {
+    int keep_first;
+    const float* sinks;
+    const float* gate;
+    long long gate_stride;
+    int gate_off;
+    float out_scale;
+    long long out_stride;
+    int out_off;
+};
+enum { T5_PLAIN, T5_BIAS, T5_EXT };
+template <int MODE>
 __global__ void __launch_bounds__(T5O_THREADS, 1) paged_prefill_attention_tcgen05_online_kernel(
     const __grid_constant__ CUtensorMap q_map, const __grid_constant__ CUtensorMap kv_map, bf16* __restrict__ out,
     const int32_t* __restrict__ tiles, const int32_t* __restrict__ entry_slot, const int32_t* __restrict__ entry_q_start,
     const int32_t* __restrict__ entry_q_len, const int32_t* __restrict__ entry_kv_len,
     const int32_t* __restrict__ block_table, int table_stride, int nq, int nkv, int page_size, int window,
-    float scale_log2e, int num_pages, int32_t* __restrict__ status, const float* __restrict__ head_bias) {
+    float scale_log2e, int num_pages, int32_t* __restrict__ status, const float* __restrict__ head_bias, const T5Ext ext) {
     pdl_begin();
+    constexpr bool BIAS = MODE == T5_BIAS, EXT = MODE == T5_EXT;
     constexpr int STAGES = T5O_STAGES;
     constexpr unsigned TMEM_COLS = 512;                           // S0 S1 O0 O1, 128 columns each
     extern __shared__ unsigned char smem_dyn[];
@@ -376,7 +393,10 @@ __global__ void __launch_bounds__(T5O_THREADS, 1) paged_prefill_attention_tcgen0
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int pos_first = past + q0, pos_last = past + q0 + rows_here - 1;
     const int k_lo = first_visible(pos_first, window) / T5O_BN * T5O_BN;
-    const int n_tiles = (pos_last - k_lo) / T5O_BN + 1;
+    const int keep = EXT && window > 0 ? ext.keep_first : 0;
+    const int head_tiles = EXT ? min((keep + T5O_BN - 1) / T5O_BN, k_lo / T5O_BN) : 0;
+    const int n_tiles = head_tiles + (pos_last - k_lo) / T5O_BN + 1;
+    auto tile_key = [&](int j) { return EXT && j < head_tiles ? j * T5O_BN : k_lo + (j - head_tiles) * T5O_BN; };
 
     if (tid == 0) {
         abort_flag = 0;
@@ -420,7 +440,11 @@ __global__ void __launch_bounds__(T5O_THREADS, 1) paged_prefill_attention_tcgen0
         const int last_logical = pos_last / page_size;
         auto page_of = [&](int j) {                               // lane b: the page of box b of tile j (checked)
             if (j >= n_tiles || lane >= boxes) return 0;
-            const int logical = min((k_lo + j * T5O_BN) / page_size + lane, last_logical);
+            int logical = min(tile_key(j) / page_size + lane, last_logical);
+            if (EXT) {                                            // pages that hold no key anybody sees may be gone: read a held one
+                if (j < head_tiles) logical = min(logical, (keep - 1) / page_size);
+                else if (logical * page_size >= keep) logical = max(logical, first_visible(pos_first, window) / page_size);
+            }
             int page = logical < table_stride ? __ldg(table + logical) : -1;
             if (page < 0 || page >= num_pages) {
                 if (atomicCAS(status, 0, 4) == 0) status[1] = row_base;
@@ -561,7 +585,7 @@ __global__ void __launch_bounds__(T5O_THREADS, 1) paged_prefill_attention_tcgen0
             asm volatile("bar.sync %0, 256;\n" ::"r"(1 + g) : "memory");
         }
         for (int j = 0; j < n_tiles; ++j) {
-            const int kt = k_lo + j * T5O_BN + half * 64;         // this thread's first key of the tile
+            const int kt = tile_key(j) + half * 64;               // this thread's first key of the tile
             const int tb_next = tb_cur == 2 ? 0 : tb_cur + 1;
             if constexpr (BIAS) {
                 if (j + 1 < n_tiles) fill_table(j + 1, tb_next);
@@ -576,7 +600,8 @@ __global__ void __launch_bounds__(T5O_THREADS, 1) paged_prefill_attention_tcgen0
             // number of times as the others, and touches nothing else.
             if (ok && !t5_wait(&s_full[g], j & 1, &abort_flag, status, row_base)) ok = false;
             t5_fence_after();
-            const bool full_tile = (kt + 63 <= pos_first) && (kt >= lo_last) && (rows_here == T5_BM);
+            const bool full_tile = (kt + 63 <= pos_first) && (kt >= lo_last || (EXT && kt + 63 < keep)) && (rows_here == T5_BM);
+            auto seen = [&](int key) { return key <= pos && (key >= lo || (EXT && key < keep)); };
             unsigned ra[32], rb[32];
             float mx = -CUDART_INF_F;
             if (ok) {
@@ -590,8 +615,8 @@ __global__ void __launch_bounds__(T5O_THREADS, 1) paged_prefill_attention_tcgen0
                 } else {
 #pragma unroll
                     for (int i = 0; i < 32; ++i) {
-                        if (kt + i <= pos && kt + i >= lo) mx = fmaxf(mx, __uint_as_float(ra[i]));
-                        if (kt + 32 + i <= pos && kt + 32 + i >= lo) mx = fmaxf(mx, __uint_as_float(rb[i]));
+                        if (seen(kt + i)) mx = fmaxf(mx, __uint_as_float(ra[i]));
+                        if (seen(kt + 32 + i)) mx = fmaxf(mx, __uint_as_float(rb[i]));
                     }
                 }
                 x_max[j & 1][g][half][row] = mx;
@@ -646,8 +671,8 @@ __global__ void __launch_bounds__(T5O_THREADS, 1) paged_prefill_attention_tcgen0
 #pragma unroll
                     for (int i = 0; i < 32; i += 2) {
                         const int key = kt + c + i;
-                        const float p0 = (key <= pos && key >= lo) ? t5_ex2(fmaf(__uint_as_float(r[i]), eff, -msub)) : 0.0f;
-                        const float p1 = (key + 1 <= pos && key + 1 >= lo) ? t5_ex2(fmaf(__uint_as_float(r[i + 1]), eff, -msub)) : 0.0f;
+                        const float p0 = seen(key) ? t5_ex2(fmaf(__uint_as_float(r[i]), eff, -msub)) : 0.0f;
+                        const float p1 = seen(key + 1) ? t5_ex2(fmaf(__uint_as_float(r[i + 1]), eff, -msub)) : 0.0f;
                         l += p0 + p1;
                         pk[i >> 1] = t5_pack(p0, p1);
                     }
@@ -666,8 +691,15 @@ __global__ void __launch_bounds__(T5O_THREADS, 1) paged_prefill_attention_tcgen0
         l += x_sum[g][half ^ 1][row];
         if (ok && t5_wait(&pv_done[g], (n_tiles - 1) & 1, &abort_flag, status, row_base)) {
             t5_fence_after();
-            const float inv = (l > 0.0f) ? 1.0f / l : 0.0f;
+            if (EXT && ext.sinks) l += t5_ex2(fmaf(ext.sinks[h0 + g], 1.4426950408889634f, -m));   // a term without a value
+            float inv = (l > 0.0f) ? 1.0f / l : 0.0f;
             bf16* orow = out + (static_cast<size_t>(row_base + row) * nq + h0 + g) * T5_D + half * 64;
+            if constexpr (EXT) {
+                orow = out + static_cast<size_t>(row_base + row) * ext.out_stride + ext.out_off + (h0 + g) * T5_D + half * 64;
+                inv *= ext.out_scale;
+                if (ext.gate && row < rows_here)
+                    inv /= 1.0f + expf(-ext.gate[static_cast<size_t>(row_base + row) * ext.gate_stride + ext.gate_off + h0 + g]);
+            }
 #pragma unroll 1
             for (int c = 0; c < 64; c += 32) {
                 unsigned r[32];
@@ -714,7 +746,7 @@ static int t5_launch(
     const void* q, void* out, const void* cache, int num_tokens, const int32_t* tiles, int n_tiles,
     const int32_t* entry_slot, const int32_t* entry_q_start, const int32_t* entry_q_len, const int32_t* entry_kv_len,
     const int32_t* block_table, int table_stride, int nq, int nkv, int d, int page_size, int window, float scale,
-    int num_pages, int32_t* status, const float* head_bias, uintptr_t stream) {
+    int num_pages, int32_t* status, const float* head_bias, const T5Ext* ext, uintptr_t stream) {
     if (n_tiles <= 0) return LLM_OK;
     if (nq <= 0 || nkv <= 0 || nq % nkv != 0 || !llm_paged_prefill_tcgen05_supported(d, page_size) || nq > 65535 ||
         n_tiles > 65535)
@@ -727,7 +759,7 @@ static int t5_launch(
     cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
     const float sl2 = scale * 1.4426950408889634f;
     const int group = nq / nkv;
-    if (head_bias && group % 2 != 0) return LLM_REFUSED_SIZE;
+    if ((head_bias || ext) && (group % 2 != 0 || (head_bias && ext))) return LLM_REFUSED_SIZE;
 #define T5_GO(HEADS, STAGES)                                                                                         \
     {                                                                                                                \
         const size_t smem = static_cast<size_t>(HEADS * 2 * T5_QHALF + 2 * STAGES * T5_TILE) * sizeof(bf16) + 1024;  \
@@ -741,13 +773,14 @@ static int t5_launch(
     }
     if (group % 2 == 0) {                                           // two heads of a group share a CTA: the one-pass kernel
         const size_t smem = static_cast<size_t>(2 * 2 * T5_QHALF + 2 * T5O_STAGES * T5O_TILE) * sizeof(bf16) + 1024;
-        auto kern = head_bias ? paged_prefill_attention_tcgen05_online_kernel<true>
-                              : paged_prefill_attention_tcgen05_online_kernel<false>;
+        auto kern = head_bias ? paged_prefill_attention_tcgen05_online_kernel<T5_BIAS>
+                    : ext     ? paged_prefill_attention_tcgen05_online_kernel<T5_EXT>
+                              : paged_prefill_attention_tcgen05_online_kernel<T5_PLAIN>;
         const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
         if (e != cudaSuccess) return static_cast<int>(e);
         launch_pdl(kern, dim3(nq / 2, n_tiles), dim3(T5O_THREADS), smem, s, q_map, kv_map, static_cast<bf16*>(out), tiles,
                    entry_slot, entry_q_start, entry_q_len, entry_kv_len, block_table, table_stride, nq, nkv, page_size,
-                   window, sl2, num_pages, status, head_bias);
+                   window, sl2, num_pages, status, head_bias, ext ? *ext : T5Ext{});
         return launch_status();
     }
     T5_GO(1, 4)                                                     // odd groups: the two-pass kernel, one head per CTA
@@ -761,7 +794,7 @@ extern "C" int llm_paged_attention_prefill_tcgen05(
     const int32_t* block_table, int table_stride, int nq, int nkv, int d, int page_size, int window, float scale,
     int num_pages, int32_t* status, uintptr_t stream) {
     return t5_launch(q, out, cache, num_tokens, tiles, n_tiles, entry_slot, entry_q_start, entry_q_len, entry_kv_len,
-                     block_table, table_stride, nq, nkv, d, page_size, window, scale, num_pages, status, nullptr, stream);
+                     block_table, table_stride, nq, nkv, d, page_size, window, scale, num_pages, status, nullptr, nullptr, stream);
 }
 
 extern "C" int llm_paged_attention_prefill_tcgen05_biased(
@@ -771,5 +804,20 @@ extern "C" int llm_paged_attention_prefill_tcgen05_biased(
     int num_pages, int32_t* status, const float* head_bias, uintptr_t stream) {
     if (!head_bias) return LLM_REFUSED_SIZE;
     return t5_launch(q, out, cache, num_tokens, tiles, n_tiles, entry_slot, entry_q_start, entry_q_len, entry_kv_len,
-                     block_table, table_stride, nq, nkv, d, page_size, window, scale, num_pages, status, head_bias, stream);
+                     block_table, table_stride, nq, nkv, d, page_size, window, scale, num_pages, status, head_bias, nullptr, stream);
+}
+
+// out: bfloat16, row t and head h at t * out_stride + out_off + h * 128.  keep_first: with a window, the first so many keys stay
+// visible; sinks: null, or float32 [nq]; gate: null, or float32 rows of gate_stride with one value a head from gate_off on.
+extern "C" int llm_paged_attention_prefill_tcgen05_ext(
+    const void* q, void* out, const void* cache, int num_tokens, const int32_t* tiles, int n_tiles,
+    const int32_t* entry_slot, const int32_t* entry_q_start, const int32_t* entry_q_len, const int32_t* entry_kv_len,
+    const int32_t* block_table, int table_stride, int nq, int nkv, int d, int page_size, int window, float scale,
+    int num_pages, int32_t* status, int keep_first, const float* sinks, const float* gate, long long gate_stride, int gate_off,
+    float out_scale, long long out_stride, int out_off, uintptr_t stream) {
+    if (keep_first < 0 || !(scale > 0.0f)) return LLM_REFUSED_SIZE;
+    if (out_stride % 8 || out_off % 8) return LLM_REFUSED_ALIGN;
+    const T5Ext ext = {keep_first, sinks, gate, gate_stride, gate_off, out_scale, out_stride, out_off};
+    return t5_launch(q, out, cache, num_tokens, tiles, n_tiles, entry_slot, entry_q_start, entry_q_len, entry_kv_len,
+                     block_table, table_stride, nq, nkv, d, page_size, window, scale, num_pages, status, nullptr, &ext, stream);
 }

@@ -1672,6 +1672,39 @@ def paged_attention_prefill_tcgen05_biased(q: torch.Tensor, out: torch.Tensor, c
     return out
 
 
+def paged_attention_prefill_tcgen05_ext(q: torch.Tensor, out: torch.Tensor, out_off: int, cache: torch.Tensor, tiles: torch.Tensor,
+                                        n_tiles: int, entry_slot, entry_q_start, entry_q_len, entry_kv_len,
+                                        block_table: torch.Tensor, nq: int, nkv: int, d: int, page_size: int,
+                                        window: Optional[int], scale: float, status: torch.Tensor,
+                                        head_gate: Optional[torch.Tensor] = None, gate_off: int = 0, out_scale: float = 1.0,
+                                        keep_first: int = 0, sink=None) -> torch.Tensor:
+    """`paged_attention_prefill_biased` without a bias by distance, on the tcgen05 kernel (even groups, see
+    `prefill_tcgen05_biased_supported`; a positive scale; out_off and out's row stride multiples of 8)."""
+    _dev(q, cache, tiles, entry_slot, entry_q_start, entry_q_len, entry_kv_len, block_table, status)
+    T = q.shape[0]
+    if q.dtype != torch.bfloat16 or cache.dtype != torch.bfloat16 or out.dtype != torch.bfloat16 or not out.is_cuda:
+        raise KernelError("the tcgen05 prefill attention kernel is bfloat16 only")
+    if q.shape[1] != nq * d or tuple(cache.shape[1:]) != (2, nkv, page_size, d):
+        raise KernelError("q must be [T, heads*head_dim] and cache [pages, 2, kv_heads, page_size, head_dim]")
+    if out.dim() != 2 or out.shape[0] != T or out.stride(1) != 1 or out_off < 0 or out_off + nq * d > out.shape[1]:
+        raise KernelError("out must be [T, n] with unit stride along its rows and hold the heads' columns")
+    if head_gate is not None and (head_gate.dtype != torch.float32 or head_gate.dim() != 2 or head_gate.shape[0] != T
+                                  or head_gate.stride(1) != 1 or not head_gate.is_cuda or gate_off < 0
+                                  or gate_off + nq > head_gate.shape[1]):
+        raise KernelError("head_gate must be float32 [T, m] with unit stride along its rows and hold the heads' columns")
+    f = _fn("attention_prefill_tcgen05", "llm_paged_attention_prefill_tcgen05_ext",
+            [c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
+             c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_int, c_void_p, c_int, c_void_p, c_void_p, c_longlong, c_int,
+             c_float, c_longlong, c_int, c_void_p])
+    sinks = _sinks(sink, nq, q.device)
+    _check(f(_ptr(q), _ptr(out), _ptr(cache), T, _ptr(tiles), n_tiles, _ptr(entry_slot), _ptr(entry_q_start),
+             _ptr(entry_q_len), _ptr(entry_kv_len), _ptr(block_table), block_table.shape[1], nq, nkv, d, page_size,
+             int(window) if window else 0, float(scale), cache.shape[0], _ptr(status), int(keep_first) if window else 0, _ptr(sinks),
+             _ptr(head_gate), head_gate.stride(0) if head_gate is not None else 0, gate_off, float(out_scale), out.stride(0), out_off,
+             _stream()), "paged_attention_prefill_tcgen05_ext")
+    return out
+
+
 def argmax_rows(logits: torch.Tensor, out: Optional[torch.Tensor] = None) -> torch.Tensor:
     _dev(logits, out)
     if logits.dtype != torch.float32 or logits.dim() != 2:

@@ -431,6 +431,14 @@ class GatedAttentionMixer(BranchMixer):
                     q, out, ctx.cache, work.padded_tiles if padded else work.prefill_tiles, n_tiles, b.entry_slot,
                     b.entry_q_start, b.entry_q_len, b.entry_kv_len, ctx.block_table, self.nq, self.nkv, self.d,
                     ctx.page_size, self.span, self.scale, ctx.status, self.dist_table_t)
+            elif (n_tiles and self.dist_table_t is None and self.scale > 0 and out_col0 % 8 == 0 and out.stride(0) % 8 == 0
+                  and ops.prefill_tcgen05_biased_supported(self.d, ctx.page_size, self.nq // self.nkv)):
+                # kept first keys, a sink and a gate per head over plain scores: in the tcgen05 kernel too
+                ops.paged_attention_prefill_tcgen05_ext(
+                    q, out, out_col0, ctx.cache, work.padded_tiles if padded else work.prefill_tiles, n_tiles, b.entry_slot,
+                    b.entry_q_start, b.entry_q_len, b.entry_kv_len, ctx.block_table, self.nq, self.nkv, self.d, ctx.page_size,
+                    self.span, self.scale, ctx.status, head_gate=gate, gate_off=col0 + self.g_off, out_scale=out_scale,
+                    keep_first=self.keep_first, sink=self.sink)
             elif n_tiles:
                 ops.paged_attention_prefill_biased(
                     q, out, out_col0, ctx.cache, work.padded_tiles if padded else work.prefill_tiles, n_tiles, b.entry_slot,
