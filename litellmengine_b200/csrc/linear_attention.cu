@@ -100,6 +100,60 @@ __global__ void gla_decay_kernel(const float* __restrict__ proj, long long strid
         }
 }
 
+// The same where channels come in fours: a thread makes 4 channels x 8 tokens, so that a weight load and two loads of four
+// inputs (kept token-minor in shared memory) feed 32 multiply-adds; one thread a channel needed a shared load for every
+// multiply-add.  The sums run over the rank in the same order.  2,048 tokens x 2,048 channels of rank 64: 71 -> 36 us.
+__global__ void __launch_bounds__(128) gla_decay_tiled_kernel(const float* __restrict__ proj, long long stride, int a_off, int rank,
+                                                              const float* __restrict__ w2t, const float* __restrict__ b2,
+                                                              float inv_tau, float* __restrict__ la, int channels, int num_tokens) {
+    pdl_begin();
+    extern __shared__ __align__(16) float a[];      // [rank][GLA_DECAY_TOKENS]
+    const int t0 = blockIdx.x * GLA_DECAY_TOKENS;
+    const int nt = min(GLA_DECAY_TOKENS, num_tokens - t0);
+    for (int idx = threadIdx.x; idx < GLA_DECAY_TOKENS * rank; idx += blockDim.x) {
+        const int t = idx / rank, j = idx - t * rank;
+        a[j * GLA_DECAY_TOKENS + t] = t < nt ? proj[static_cast<size_t>(t0 + t) * stride + a_off + j] : 0.0f;
+    }
+    __syncthreads();
+    const int c = blockIdx.y * GLA_DECAY_CHANNELS + (threadIdx.x & 31) * 4, tg = (threadIdx.x >> 5) * 8;
+    if (c >= channels) return;
+    float z[8][4];
+    const float4 bias = b2 ? *reinterpret_cast<const float4*>(b2 + c) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll
+    for (int t = 0; t < 8; ++t) { z[t][0] = bias.x; z[t][1] = bias.y; z[t][2] = bias.z; z[t][3] = bias.w; }
+    auto add = [&](const float4 w, int j) {
+        float x[8];
+        load8(a + j * GLA_DECAY_TOKENS + tg, x);
+#pragma unroll
+        for (int t = 0; t < 8; ++t) {
+            z[t][0] += w.x * x[t];
+            z[t][1] += w.y * x[t];
+            z[t][2] += w.z * x[t];
+            z[t][3] += w.w * x[t];
+        }
+    };
+    int j = 0;
+    for (; j + 8 <= rank; j += 8) {
+        float4 w[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) w[u] = *reinterpret_cast<const float4*>(w2t + static_cast<size_t>(j + u) * channels + c);
+#pragma unroll
+        for (int u = 0; u < 8; ++u) add(w[u], j + u);
+    }
+    for (; j < rank; ++j) add(*reinterpret_cast<const float4*>(w2t + static_cast<size_t>(j) * channels + c), j);
+#pragma unroll
+    for (int t = 0; t < 8; ++t)
+        if (tg + t < nt) {
+            float r[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const float ls = z[t][i] < 0.0f ? z[t][i] - log1pf(expf(z[t][i])) : -log1pf(expf(-z[t][i]));
+                r[i] = expf(ls * inv_tau);
+            }
+            *reinterpret_cast<float4*>(la + static_cast<size_t>(t0 + tg + t) * channels + c) = make_float4(r[0], r[1], r[2], r[3]);
+        }
+}
+
 extern "C" int llm_gla_decay(const float* proj, long long stride, int a_off, int rank, const float* w2t, const float* b2,
                              float tau, float* la, int num_tokens, int channels, uintptr_t stream) {
     if (num_tokens <= 0) return LLM_OK;
@@ -107,6 +161,12 @@ extern "C" int llm_gla_decay(const float* proj, long long stride, int a_off, int
     const dim3 grid((num_tokens + GLA_DECAY_TOKENS - 1) / GLA_DECAY_TOKENS,
                     (channels + GLA_DECAY_CHANNELS - 1) / GLA_DECAY_CHANNELS);
     if (grid.y > 65535) return LLM_REFUSED_SIZE;
+    // from a few rows on (a handful of tokens leaves most of a thread's eight idle), and while the inputs fit 48 KB
+    if (num_tokens >= 8 && channels % 4 == 0 && rank <= 384 && aligned16(w2t) && aligned16(la) && (!b2 || aligned16(b2))) {
+        launch_pdl(gla_decay_tiled_kernel, grid, dim3(128), GLA_DECAY_TOKENS * rank * sizeof(float), reinterpret_cast<cudaStream_t>(stream),
+                   proj, stride, a_off, rank, w2t, b2, 1.0f / tau, la, channels, num_tokens);
+        return launch_status();
+    }
     launch_pdl(gla_decay_kernel, grid, dim3(GLA_DECAY_CHANNELS), GLA_DECAY_TOKENS * rank * sizeof(float),
                reinterpret_cast<cudaStream_t>(stream), proj, stride, a_off, rank, w2t, b2, 1.0f / tau, la, channels,
                num_tokens);
@@ -378,6 +438,214 @@ __global__ void __launch_bounds__(MAX_THREADS) gla_scan_kernel(
     }
 }
 
+// ---- the per-channel scan for states of 64 or 128 rows, register-tiled --------------------------------------------
+// In the kernel above a thread owns one column, so every product of the recurrence needs its share of a 16-byte shared load
+// of decays, keys and queries that serves that column only: 24 loads (96 clocks of the 128-byte shared-memory path) for 96
+// multiply-adds a token and thread at R = 32.  Here a thread owns RR rows x 8 columns: one load of four decays, keys or
+// queries serves eight columns, 3 RR / 4 + 2 loads for 24 RR multiply-adds, and packed two-wide arithmetic (two rows an
+// instruction) halves what has to be issued.  Sixteen lanes hold the rows of a column (a lane's rows are 4 rg .. + 3 and, at
+// 128 rows, 64 + 4 rg .. + 3, so that a quarter-warp's loads are contiguous); their shares of o are added by halving
+// exchanges, eight shuffles for eight columns, and one lane of two leaves a column's sum in shared memory.  A block is 2 V
+// threads, two blocks an SM.  Same modes, staging and epilogue as above; every state element is updated by the same
+// operations in the same order (k v, then decay times state plus that), only o's sum runs over the rows in another order.
+// 2,048 tokens, 16 heads of 128 x 128: local pass and output pass 193 us each -> 67 and 161 us.
+typedef unsigned long long gla_pair;
+__device__ __forceinline__ gla_pair gla_mul2(gla_pair a, gla_pair b) {
+    gla_pair r;
+    asm("mul.rn.f32x2 %0, %1, %2;\n" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ gla_pair gla_fma2(gla_pair a, gla_pair b, gla_pair c) {
+    gla_pair r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;\n" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ gla_pair gla_both(float lo, float hi) {
+    gla_pair r;
+    asm("mov.b64 %0, {%1, %2};\n" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ float2 gla_split(gla_pair a) {
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;\n" : "=f"(r.x), "=f"(r.y) : "l"(a));
+    return r;
+}
+
+template <int RR, int MODE, typename TO>
+__global__ void __launch_bounds__(256, 2) gla_scan_tiled_kernel(
+    const float* __restrict__ proj, long long stride, int q_off, int k_off, int v_off, int g_off,
+    const float* __restrict__ alpha, const float* __restrict__ norm_w, float eps, float q_scale, float out_scale,
+    TO* __restrict__ out, long long out_stride, int out_off, float* __restrict__ state,
+    const int32_t* __restrict__ entry_slot, const int32_t* __restrict__ entry_q_start,
+    const int32_t* __restrict__ entry_q_len, const int32_t* __restrict__ items,
+    float* __restrict__ scratch_s, float* __restrict__ scratch_a, int H, int V) {
+    pdl_begin();
+    constexpr int D = 16 * RR, Q4 = RR / 4;          // Q4: groups of four rows a lane holds
+    constexpr bool OUTPUTS = MODE != GLA_LOCAL;
+    extern __shared__ __align__(16) float smem[];
+    const int h = blockIdx.y;
+    int entry, row0, count, sidx;
+    if (items) {
+        entry = items[4 * blockIdx.x];
+        if (entry < 0) return;                       // padding of a work list
+        row0 = items[4 * blockIdx.x + 1];
+        count = items[4 * blockIdx.x + 2];
+        sidx = items[4 * blockIdx.x + 3];
+    } else {
+        entry = blockIdx.x;
+        row0 = entry_q_start[entry];
+        count = entry_q_len[entry];
+        sidx = entry;
+    }
+    const int tid = threadIdx.x, nthreads = blockDim.x, warp = tid >> 5, lane = tid & 31;
+    const int rg = lane & 15, col0 = (tid >> 4) * 8;
+    const int buf_floats = GLA_TB * (3 * D + V);
+    float* part = smem + 2 * buf_floats;             // [TB][V]
+    const size_t HD = static_cast<size_t>(H) * D, per = static_cast<size_t>(D) * V;
+    float* slot_state = state + (static_cast<size_t>(entry_slot[entry]) * H + h) * per;
+    const float* s_in = MODE == GLA_FULL ? slot_state : MODE == GLA_OUT ? scratch_s + (static_cast<size_t>(sidx) * H + h) * per : nullptr;
+    gla_pair S[RR / 2][8], A[RR / 2];
+    auto row_of = [&](int p) { return 64 * (p >> 1) + 4 * rg + 2 * (p & 1); };       // the first of a pair's two rows
+#pragma unroll
+    for (int p = 0; p < RR / 2; ++p) {
+        A[p] = gla_both(1.0f, 1.0f);
+        float lo[8], hi[8];
+        if (MODE == GLA_LOCAL) {
+#pragma unroll
+            for (int c = 0; c < 8; ++c) lo[c] = hi[c] = 0.0f;
+        } else {
+            load8(s_in + static_cast<size_t>(row_of(p)) * V + col0, lo);
+            load8(s_in + static_cast<size_t>(row_of(p) + 1) * V + col0, hi);
+        }
+#pragma unroll
+        for (int c = 0; c < 8; ++c) S[p][c] = gla_both(lo[c], hi[c]);
+    }
+    auto stage = [&](int done, int buf) {
+        const int nb = min(GLA_TB, count - done);
+        const size_t base = static_cast<size_t>(row0 + done);
+        float* bq = smem + buf * buf_floats;
+        float* bk = bq + GLA_TB * D;
+        float* ba = bk + GLA_TB * D;
+        float* bv = ba + GLA_TB * D;
+        for (int idx = tid; idx < nb * (D / 4); idx += nthreads) {
+            const int tok = idx / (D / 4), c = (idx % (D / 4)) << 2;
+            const float* pr = proj + (base + tok) * stride + h * D + c;
+            gla_cp16(bk + tok * D + c, pr + k_off);
+            gla_cp16(ba + tok * D + c, alpha + (base + tok) * HD + h * D + c);
+            if (OUTPUTS) gla_cp16(bq + tok * D + c, pr + q_off);
+        }
+        const int v4 = V >> 2;
+        for (int idx = tid; idx < nb * v4; idx += nthreads) {
+            const int tok = idx / v4, c = (idx - tok * v4) << 2;
+            gla_cp16(bv + tok * V + c, proj + (base + tok) * stride + v_off + h * V + c);
+        }
+        asm volatile("cp.async.commit_group;\n" ::);
+    };
+    stage(0, 0);
+    for (int done = 0, b = 0; done < count; done += GLA_TB, ++b) {
+        const int nb = min(GLA_TB, count - done);
+        const size_t base = static_cast<size_t>(row0 + done);
+        if (done + GLA_TB < count) {
+            stage(done + GLA_TB, (b + 1) & 1);
+            asm volatile("cp.async.wait_group 1;\n" ::: "memory");
+        } else {
+            asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+        }
+        __syncthreads();
+        const float* sq = smem + (b & 1) * buf_floats;
+        const float* sk = sq + GLA_TB * D;
+        const float* sa = sk + GLA_TB * D;
+        const float* sv = sa + GLA_TB * D;
+        for (int tok = 0; tok < nb; ++tok) {
+            gla_pair k[RR / 2], a[RR / 2], q[RR / 2];
+#pragma unroll
+            for (int g = 0; g < Q4; ++g) {
+                const ulonglong2 kk = *reinterpret_cast<const ulonglong2*>(sk + tok * D + 64 * g + 4 * rg);
+                const ulonglong2 aa = *reinterpret_cast<const ulonglong2*>(sa + tok * D + 64 * g + 4 * rg);
+                k[2 * g] = kk.x; k[2 * g + 1] = kk.y;
+                a[2 * g] = aa.x; a[2 * g + 1] = aa.y;
+                if (OUTPUTS) {
+                    const ulonglong2 qq = *reinterpret_cast<const ulonglong2*>(sq + tok * D + 64 * g + 4 * rg);
+                    q[2 * g] = qq.x; q[2 * g + 1] = qq.y;
+                }
+            }
+            float v[8], o[8];
+            load8(sv + tok * V + col0, v);
+#pragma unroll
+            for (int c = 0; c < 8; ++c) {
+                const gla_pair vv = gla_both(v[c], v[c]);
+                gla_pair share = 0;
+#pragma unroll
+                for (int p = 0; p < RR / 2; ++p) {
+                    S[p][c] = gla_fma2(a[p], S[p][c], gla_mul2(k[p], vv));
+                    if (OUTPUTS) share = p == 0 ? gla_mul2(S[p][c], q[p]) : gla_fma2(S[p][c], q[p], share);
+                }
+                if (OUTPUTS) {
+                    const float2 t = gla_split(share);
+                    o[c] = t.x + t.y;
+                }
+            }
+            if (MODE == GLA_LOCAL) {                 // the chunk's total decay per key channel
+#pragma unroll
+                for (int p = 0; p < RR / 2; ++p) A[p] = gla_mul2(A[p], a[p]);
+            }
+            if (OUTPUTS) {
+#pragma unroll
+                for (int off = 8, n = 4; n >= 1; off >>= 1, n >>= 1)
+#pragma unroll
+                    for (int i = 0; i < 4; ++i)
+                        if (i < n) {
+                            const bool up = (lane & off) != 0;
+                            const float send = up ? o[i] : o[i + n], keep = up ? o[i + n] : o[i];
+                            o[i] = keep + __shfl_xor_sync(0xffffffffu, send, off);
+                        }
+                o[0] += __shfl_xor_sync(0xffffffffu, o[0], 1);
+                if ((lane & 1) == 0) part[tok * V + col0 + (rg >> 1)] = o[0];
+            }
+        }
+        __syncthreads();
+        if (OUTPUTS) {                               // a warp per token: norm over V, weight, gate, scale
+            for (int tok = warp; tok < nb; tok += nthreads >> 5) {
+                float* o = part + tok * V;
+                float ss = 0.0f;
+                for (int c = lane; c < V; c += 32) {
+                    const float x = o[c] * q_scale;
+                    ss += x * x;
+                }
+                const float inv = q_scale / sqrtf(warp_sum(ss) / static_cast<float>(V) + eps) * out_scale;
+                const float* gr = proj + (base + tok) * stride + g_off + h * V;
+                TO* orow = out + (base + tok) * out_stride + out_off + h * V;
+                for (int c = lane; c < V; c += 32) orow[c] = from_f32<TO>(o[c] * inv * norm_w[c] * recur_gate(gr[c], 2));
+            }
+            // the next batch's shares are written after its first barrier, this buffer is filled again two batches on
+        }
+    }
+    if (MODE == GLA_OUT) return;
+    float* s_out = MODE == GLA_FULL ? slot_state : scratch_s + (static_cast<size_t>(sidx) * H + h) * per;
+#pragma unroll
+    for (int p = 0; p < RR / 2; ++p) {
+        float lo[8], hi[8];
+#pragma unroll
+        for (int c = 0; c < 8; ++c) {
+            const float2 t = gla_split(S[p][c]);
+            lo[c] = t.x; hi[c] = t.y;
+        }
+        store8(s_out + static_cast<size_t>(row_of(p)) * V + col0, lo);
+        store8(s_out + static_cast<size_t>(row_of(p) + 1) * V + col0, hi);
+        if (MODE == GLA_LOCAL && col0 == 0) {
+            const float2 t = gla_split(A[p]);
+            float* to = scratch_a + (static_cast<size_t>(sidx) * H + h) * D + row_of(p);
+            to[0] = t.x; to[1] = t.y;
+        }
+    }
+}
+
+static bool gla_tiled_takes(int D, int V) {
+    static int rows_forced = -1;                   // LLM_GLA_ROWS asks for the kernel above
+    if (rows_forced < 0) rows_forced = getenv("LLM_GLA_ROWS") != nullptr;
+    return !rows_forced && (D == 64 || D == 128) && (V == 32 || V == 64 || V == 128);
+}
+
 // Rows of a state column that one thread keeps (R), the row groups DG = ceil(D / R), and the block size the
 // kernel is compiled for: 16, else 32, else 64, else 8 rows, whichever block of V * DG threads fits first
 // within 512 threads (64 x 64 a head: 110 us with 16 rows, 134 with 8, 173 with 32 for 2,048 tokens of 16
@@ -464,6 +732,30 @@ extern "C" int llm_recur_scan(
     const int vec = D % 4 == 0 && V % 4 == 0 && stride % 4 == 0 && q_off % 4 == 0 && k_off % 4 == 0 && v_off % 4 == 0 &&
                     aligned16(proj) && (decay_kind || aligned16(la));
     if (smem > 220 * 1024) return LLM_REFUSED_SIZE;
+    if (out_dtype != LLM_DT_F32 && out_dtype != LLM_DT_BF16) return LLM_REFUSED_DTYPE;
+    if (decay_kind == 0 && vec && gla_tiled_takes(D, V) && aligned16(state) && (mode == GLA_FULL || aligned16(scratch_s))) {
+        const size_t need = static_cast<size_t>(GLA_TB) * (2 * (3 * D + V) + V) * sizeof(float);
+#define TILED(RR, MODE, TO)                                                                                          \
+        do {                                                                                                          \
+            auto kern = gla_scan_tiled_kernel<RR, MODE, TO>;                                                          \
+            if (need > 48 * 1024) {                                                                                   \
+                const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,         \
+                                                           static_cast<int>(need));                                   \
+                if (e != cudaSuccess) return static_cast<int>(e);                                                     \
+            }                                                                                                         \
+            launch_pdl(kern, dim3(num_items, H), dim3(2 * V), need, reinterpret_cast<cudaStream_t>(stream), proj,     \
+                       stride, q_off, k_off, v_off, g_off, la, norm_w, eps, q_scale, out_scale,                       \
+                       static_cast<TO*>(out), out_stride, out_off, state, entry_slot, entry_q_start, entry_q_len,     \
+                       items, scratch_s, scratch_a, H, V);                                                            \
+            return launch_status();                                                                                   \
+        } while (0)
+#define TILED_MODES(RR, TO)                                                                                           \
+        do { if (mode == GLA_FULL) TILED(RR, GLA_FULL, TO); else if (mode == GLA_LOCAL) TILED(RR, GLA_LOCAL, TO); else TILED(RR, GLA_OUT, TO); } while (0)
+        if (D == 128) { if (out_dtype == LLM_DT_F32) TILED_MODES(8, float); else TILED_MODES(8, bf16); }
+        else { if (out_dtype == LLM_DT_F32) TILED_MODES(4, float); else TILED_MODES(4, bf16); }
+#undef TILED_MODES
+#undef TILED
+    }
     const RecurOpts opt = {a_tok, a_head, kscale, nfloor, norm_stride, gate_kind, state_head_stride, state_slot_stride};
     cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
     const dim3 grid(num_items, H), block((VC * DG + 31) / 32 * 32);
@@ -490,7 +782,6 @@ extern "C" int llm_recur_scan(
             else LAUNCH(64, 1024, TO, SC);                                                                        \
             break;                                                                                                \
     }
-    if (out_dtype != LLM_DT_F32 && out_dtype != LLM_DT_BF16) return LLM_REFUSED_DTYPE;
     if (R == 32 && MT == 544) {
         if (out_dtype == LLM_DT_F32) LAUNCH(32, 544, float, true);
         else LAUNCH(32, 544, bf16, true);
