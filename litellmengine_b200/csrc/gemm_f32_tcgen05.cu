@@ -1,0 +1,366 @@
+// y[M, N] = x[M, K] . W[N, K]^T for float32 operands and more rows than a decode step, on the 5th-generation tensor cores.
+//
+// A float32 value is exactly the sum of three bfloat16 values, h + m + l, each the next eight bits of its significand
+// (truncated, so that nothing overflows and each remainder is exact).  A product is then hh + (hm + mh) + (mm + hl + lh) plus
+// three terms below 2^-23 of it, which are left out; six bfloat16 products with float32 accumulation take the place of one
+// float32 product, at 6 / 31 of the tensor cores' time against the multiply-add units' (4,096 against 128 products a clock and SM).
+//
+// What makes the sums as good as float32's: the tensor cores cut, rather than round, what they add to an accumulator, and
+// 256 steps in a row along K = 4096 would show that.  So an accumulator lives for 64 k-values only, smallest terms first,
+// and is then added, rounded, to sums kept in registers by the warps that drain it.  Error against 64 bits (relative, 2-norm,
+// K = 4096): 1.5e-7 to 1.9e-7; the library's float32 product 1.1e-6.
+// A result that is not finite is computed again with plain multiply-adds (a split infinity times zero is NaN), so infinities
+// and NaN come out as a float32 product has them.
+//
+// A CTA makes 128 weight rows x NT tokens (the MMA's M side is the weights, so that 17 tokens cost a tile of 32).  Roles: warp
+// 0 feeds the copy engine: 128 x 64 weights as float32, and NT x 64 of the three planes of x, which a small kernel has
+// split; warps 2 to 9 split the weights in shared memory, half a row a thread (11 instructions for two values; storing the split
+// weights instead would double their memory and their bytes); one lane of warp 1 issues 6 x 4 products a block of 64;
+// warps 10 to 17 drain.  Planes are double-buffered (96 KB of weights' planes, 96 KB of x at NT 128).
+// The weights' planes go to tensor memory, from where the tensor cores take their left operand: kept in shared memory, their
+// stores and the operand reads of 24 products a block (8 KB each) filled the shared-memory path (500 tokens of 4096 x 12288:
+// 323 us, now 291).  What bounds it now is the tensor pipe: 24 products of 128 x NT x 16 a block take 2,500 to 2,900 clocks.
+// Tiles that fill the SMs badly are cut along K (`splits`), the parts added in order by a second kernel.
+//
+// Measured (us; the library's float32 product in brackets):
+//   N x K              17 rows        64 rows        128 rows       500 rows       2,048 rows
+//   6144 x 4096        39 (102)       43 (124)       66 (167)       203 (541)      679 (1,772)
+//   4096 x 4096        31 (101)       34 (102)       55 (121)       117 (309)      455 (1,131)
+//   24576 x 4096       146 (198)      153 (282)      241 (548)      665 (1,775)    2,336 (6,606)
+//   4096 x 12288       74 (242)       77 (305)       103 (359)      293 (911)      1,196 (3,350)
+//   2048 x 2048        18 (51)        21 (51)
+// Matrices of fewer than 2^21 values stay with the library (1024 x 1024: 17 against 14 at 17 rows, 31 against 30 at 512).
+#include "tcgen05_attention.cuh"
+#include <math_constants.h>
+
+#define LT_ROWS 128                              // weight rows of a tile
+#define LT_K 64                                  // k-values of a block: a 128-byte row of bfloat16
+#define LT_SPLITTERS 256                          // threads that split the weights
+#define LT_THREADS (18 * 32)
+#define LT_BOX (LT_ROWS * 32 * 4)                // bytes of a box of float32 weights: 32 k-values, half a block
+#define LT_STATUS 9
+
+__device__ __forceinline__ bool lt_wait(unsigned long long* bar, unsigned parity, volatile int* abort_flag, int32_t* status) {
+    for (int i = 0; i < T5_WAIT_LIMIT; ++i) {
+        if (t5_try_wait(bar, parity)) return true;
+        if (*abort_flag) return false;
+    }
+    *abort_flag = 1;
+    if (atomicCAS(status, 0, LT_STATUS) == 0) status[1] = blockIdx.y;
+    return false;
+}
+
+// The same for a whole warp, which goes on or stops together (tensor-memory accesses are a warp's).
+__device__ __forceinline__ bool lt_wait_warp(unsigned long long* bar, unsigned parity, volatile int* abort_flag, int32_t* status) {
+    return __all_sync(0xffffffffu, lt_wait(bar, parity, abort_flag, status));
+}
+
+// The high halves of two floats as a pair of bfloat16 (a in the lower half).
+__device__ __forceinline__ unsigned lt_tops(float a, float b) { return __byte_perm(__float_as_uint(a), __float_as_uint(b), 0x7632); }
+__device__ __forceinline__ float lt_rest(float a) { return a - __uint_as_float(__float_as_uint(a) & 0xffff0000u); }
+// Eight floats as three planes of eight bfloat16.
+__device__ __forceinline__ void lt_split8(const float4 a, const float4 b, unsigned* h, unsigned* m, unsigned* l) {
+    const float v[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const float r0 = lt_rest(v[2 * i]), r1 = lt_rest(v[2 * i + 1]);
+        h[i] = lt_tops(v[2 * i], v[2 * i + 1]);
+        m[i] = lt_tops(r0, r1);
+        l[i] = lt_tops(lt_rest(r0), lt_rest(r1));
+    }
+}
+
+__device__ __forceinline__ void lt_st8(unsigned taddr, const unsigned (&r)[8]) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};\n" ::
+                     "r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]) : "memory");
+}
+__device__ __forceinline__ void lt_ld16(unsigned taddr, unsigned (&r)[16]) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];\n"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+                   "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+                 : "r"(taddr) : "memory");
+}
+
+__global__ void linear_f32_split_kernel(const float* __restrict__ x, uint4* __restrict__ planes, long long pieces) {
+    pdl_begin();
+    const long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
+    if (i >= pieces) return;
+    const float4* p = reinterpret_cast<const float4*>(x) + 2 * i;
+    unsigned h[4], m[4], l[4];
+    lt_split8(p[0], p[1], h, m, l);
+    planes[i] = make_uint4(h[0], h[1], h[2], h[3]);
+    planes[pieces + i] = make_uint4(m[0], m[1], m[2], m[3]);
+    planes[2 * pieces + i] = make_uint4(l[0], l[1], l[2], l[3]);
+}
+
+// grid (token tiles, row tiles, splits of K): tiles that share weights are neighbours.  NT: tokens of a tile (32, 64 or 128);
+// WB: boxes of float32 weights in flight; XS: blocks of x;
+// PS: blocks of the weights' planes (2 or 4; as many as fit beside the accumulators).  y: [M, N], or [splits, M, N] parts.
+template <int NT, int WB, int XS, int PS>
+__global__ void __launch_bounds__(LT_THREADS, 1) linear_f32_tcgen05_kernel(
+    const __grid_constant__ CUtensorMap w_map, const __grid_constant__ CUtensorMap x_map, const float* __restrict__ x,
+    const float* __restrict__ w, float* __restrict__ y, int M, int N, int K, int blocks_per_split, int32_t* __restrict__ status) {
+    pdl_invite();
+    constexpr int X_PLANE = NT * LT_K, DRAIN = NT >= 64 ? 256 : 128, COLS = NT >= 64 ? NT / 2 : NT;
+    // tensor memory: two accumulators of NT columns, then PS stages of three planes of 32 columns (64 k-values as pairs)
+    constexpr unsigned TMEM_COLS = 512, PLANE_COL = 2 * NT;
+    static_assert(2 * NT + PS * 96 <= 512, "tensor memory");
+    extern __shared__ unsigned char smem_dyn[];
+    unsigned char* smem_al = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_dyn) + 1023) & ~uintptr_t(1023));
+    unsigned char* w_s = smem_al;                                 // [WB][128 rows][32 floats], 128-byte swizzle
+    bf16* x_s = reinterpret_cast<bf16*>(w_s + WB * LT_BOX);       // [XS][3 planes][NT][64]
+    __shared__ __align__(8) unsigned long long w_full[WB], w_empty[WB], p_full[PS], p_empty[PS], x_full[XS], x_empty[XS],
+        acc_full[2], acc_empty[2];
+    __shared__ unsigned tmem_base_s;
+    __shared__ int abort_flag;
+
+    const int m0 = blockIdx.x * NT, n0 = blockIdx.y * LT_ROWS;
+    const int kb0 = blockIdx.z * blocks_per_split, kb_all = (K + LT_K - 1) / LT_K;
+    const int kbs = min(blocks_per_split, kb_all - kb0);          // at least one: the host sees to that
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    if (tid == 0) {
+        abort_flag = 0;
+        for (int s = 0; s < WB; ++s) { t5_mbar_init(&w_full[s], 1); t5_mbar_init(&w_empty[s], LT_SPLITTERS); }
+        for (int s = 0; s < XS; ++s) { t5_mbar_init(&x_full[s], 1); t5_mbar_init(&x_empty[s], 1); }
+        for (int s = 0; s < PS; ++s) {
+            t5_mbar_init(&p_full[s], LT_SPLITTERS);               // every splitting thread has written its part of a row
+            t5_mbar_init(&p_empty[s], 1);                         // the products that read these planes have finished
+        }
+        for (int s = 0; s < 2; ++s) { t5_mbar_init(&acc_full[s], 1); t5_mbar_init(&acc_empty[s], DRAIN); }
+        asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+    }
+    if (warp == 1) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(t5_smem(&tmem_base_s)), "r"(TMEM_COLS) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
+    }
+    t5_fence_before();
+    __syncthreads();
+    t5_fence_after();
+    const unsigned tmem = tmem_base_s;
+
+    if (warp == 0) {
+        if (lane == 0) {
+            int nw = 0, nx = 0;
+            bool ok = true;
+            const int boxes = 2 * kbs;
+            auto fetch_w = [&]() {                                // the next box
+                const int st = nw % WB;
+                if (nw >= WB && !lt_wait(&w_empty[st], ((nw / WB) - 1) & 1, &abort_flag, status)) return false;
+                t5_expect_tx(&w_full[st], LT_BOX);
+                t5_tma_2d(w_s + st * LT_BOX, &w_map, kb0 * LT_K + nw * 32, n0, &w_full[st]);
+                ++nw;
+                return true;
+            };
+            while (ok && nw < min(WB, boxes)) ok = fetch_w();     // weights: before the wait for the kernel in front
+            pdl_wait();
+            auto fetch_x = [&]() {                                // the next block
+                const int st = nx % XS;
+                if (nx >= XS && !lt_wait(&x_empty[st], ((nx / XS) - 1) & 1, &abort_flag, status)) return false;
+                t5_expect_tx(&x_full[st], 3 * X_PLANE * sizeof(bf16));
+#pragma unroll
+                for (int p = 0; p < 3; ++p)
+                    t5_tma_2d(x_s + (st * 3 + p) * X_PLANE, &x_map, (kb0 + nx) * LT_K, p * M + m0, &x_full[st]);
+                ++nx;
+                return true;
+            };
+            // x runs a block ahead of the weights: its stage is free when the one of the planes being written is
+            if (ok) ok = fetch_x();
+            for (int kb = 0; ok && kb < kbs; ++kb) {
+                if (nx < kbs) ok = fetch_x();
+                while (ok && nw < min(boxes, 2 * kb + 2 + WB)) ok = fetch_w();
+            }
+            if (!ok || abort_flag) {                              // let what is in flight land before the CTA goes away
+                for (int n = max(0, nw - WB); n < nw; ++n)
+                    for (int i = 0; i < T5_WAIT_LIMIT && !t5_try_wait(&w_full[n % WB], (n / WB) & 1); ++i) {}
+                for (int kb = max(0, nx - XS); kb < nx; ++kb)
+                    for (int i = 0; i < T5_WAIT_LIMIT && !t5_try_wait(&x_full[kb % XS], (kb / XS) & 1); ++i) {}
+            }
+        }
+    } else if (warp == 1) {
+        if (lane == 0) {
+            constexpr unsigned IDESC = t5_idesc(LT_ROWS, NT, 0);
+            const unsigned long long xd = t5_desc(x_s, 16, 1024);
+            constexpr unsigned long long X_STEP = X_PLANE * sizeof(bf16) >> 4;
+            // the smallest terms first: l h, h l, m m, m h, h m, h h
+            constexpr int WP[6] = {2, 0, 1, 1, 0, 0}, XP[6] = {0, 2, 1, 0, 1, 0};
+            auto block = [&](int kb, int st) -> bool {            // st = kb % 2, a constant where this is inlined
+                if (kb >= 2 && !lt_wait(&acc_empty[st], ((kb >> 1) - 1) & 1, &abort_flag, status)) return false;
+                const int xs = kb % XS;
+                if (!lt_wait(&x_full[xs], (kb / XS) & 1, &abort_flag, status)) return false;
+                const int ps = kb % PS;
+                if (!lt_wait(&p_full[ps], (kb / PS) & 1, &abort_flag, status)) return false;
+                t5_fence_after();
+                const unsigned long long xb = xd + xs * 3 * X_STEP;
+                const unsigned pl = tmem + PLANE_COL + ps * 96;
+#pragma unroll
+                for (int t = 0; t < 6; ++t)
+#pragma unroll
+                    for (int k = 0; k < 4; ++k)
+                        t5_mma_ts(tmem + st * NT, pl + WP[t] * 32 + k * 8, xb + XP[t] * X_STEP + 2 * k, IDESC,
+                                  t > 0 || k > 0);
+                t5_commit(&p_empty[ps]);
+                t5_commit(&x_empty[xs]);
+                t5_commit(&acc_full[st]);
+                return true;
+            };
+            bool ok = true;
+            for (int kb = 0; ok && kb < kbs; kb += 2) {
+                ok = block(kb, 0);
+                if (ok && kb + 1 < kbs) ok = block(kb + 1, 1);
+            }
+        }
+    } else if (warp < 10) {
+        // ---- split the weights: two threads a row, each 16 k-values of every box ----
+        const int quarter = warp & 3, part = (warp - 2) >> 2, r = quarter * 32 + lane, sw = r & 7;
+        const unsigned planes = tmem + (static_cast<unsigned>(quarter * 32) << 16) + PLANE_COL + 8 * part;
+        bool ok = true;
+        for (int kb = 0; ok && kb < kbs; ++kb) {
+            const int st = kb % PS;
+            if (kb >= PS && !lt_wait_warp(&p_empty[st], ((kb / PS) - 1) & 1, &abort_flag, status)) break;
+            t5_fence_after();
+#pragma unroll
+            for (int half = 0; half < 2; ++half) {
+                const int box = 2 * kb + half, ws = box % WB;
+                if (!lt_wait_warp(&w_full[ws], (box / WB) & 1, &abort_flag, status)) { ok = false; break; }
+                const unsigned char* src = w_s + ws * LT_BOX + r * 128;
+                float4 a[4];
+#pragma unroll
+                for (int i = 0; i < 4; ++i) a[i] = *reinterpret_cast<const float4*>(src + ((4 * part + i) ^ sw) * 16);
+                unsigned h[8], m[8], l[8];
+                lt_split8(a[0], a[1], h, m, l);
+                lt_split8(a[2], a[3], h + 4, m + 4, l + 4);
+                lt_st8(planes + st * 96 + 16 * half, h);
+                lt_st8(planes + st * 96 + 32 + 16 * half, m);
+                lt_st8(planes + st * 96 + 64 + 16 * half, l);
+                t5_arrive(&w_empty[ws]);
+            }
+            if (!ok) break;
+            t5_wait_st();
+            t5_fence_before();
+            t5_arrive(&p_full[st]);
+        }
+    } else if (NT >= 64 || warp < 14) {
+        // ---- drain: a thread owns weight row n0 + its TMEM lane, COLS tokens ----
+        pdl_wait();
+        const int quarter = warp & 3, part = (warp - 10) >> 2;
+        const unsigned addr = tmem + (static_cast<unsigned>(quarter * 32) << 16) + part * COLS;
+        float acc[COLS];
+#pragma unroll
+        for (int i = 0; i < COLS; ++i) acc[i] = 0.0f;
+        bool ok = true;
+        for (int kb = 0; kb < kbs; ++kb) {
+            const int st = kb & 1;
+            if (!lt_wait_warp(&acc_full[st], (kb >> 1) & 1, &abort_flag, status)) { ok = false; break; }
+            t5_fence_after();
+#pragma unroll
+            for (int c = 0; c < COLS; c += 16) {
+                unsigned r[16];
+                lt_ld16(addr + st * NT + c, r);
+                t5_wait_ld();
+#pragma unroll
+                for (int i = 0; i < 16; ++i) acc[c + i] += __uint_as_float(r[i]);
+            }
+            t5_fence_before();
+            t5_arrive(&acc_empty[st]);
+        }
+        const int n = n0 + quarter * 32 + lane;
+        if (ok && n < N) {
+            float* out = y + static_cast<size_t>(blockIdx.z) * M * N;
+            const int k_from = kb0 * LT_K, k_to = min(K, (kb0 + kbs) * LT_K);
+#pragma unroll
+            for (int i = 0; i < COLS; ++i) {
+                const int m = m0 + part * COLS + i;
+                if (m >= M) continue;
+                float v = acc[i];
+                if (!(fabsf(v) <= 3.402823466e38f)) {             // infinite or NaN: what plain multiply-adds make of it
+                    v = 0.0f;
+                    for (int k = k_from; k < k_to; ++k) v = fmaf(x[static_cast<size_t>(m) * K + k], w[static_cast<size_t>(n) * K + k], v);
+                }
+                out[static_cast<size_t>(m) * N + n] = v;
+            }
+        }
+    }
+    t5_fence_before();
+    __syncthreads();
+    if (warp == 1) {
+        t5_fence_after();
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(TMEM_COLS) : "memory");
+    }
+}
+
+__global__ void linear_f32_sum_kernel(const float* __restrict__ parts, float* __restrict__ y, long long n, int splits) {
+    pdl_begin();
+    const long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    float v = parts[i];
+    for (int s = 1; s < splits; ++s) v += parts[s * n + i];
+    y[i] = v;
+}
+
+static bool lt_encode_f32(CUtensorMap* map, const void* base, long long cols, long long rows, int box_rows) {
+    CUtensorMap probe;
+    if (g_t5_state == 0 && !t5_encode_2d(&probe, base, 64, 128, 64, 8)) return false;      // looks the encoder up
+    if (g_t5_state < 0 || rows >= (1LL << 31)) return false;
+    const cuuint64_t dims[2] = {static_cast<cuuint64_t>(cols), static_cast<cuuint64_t>(rows)};
+    const cuuint64_t strides[1] = {static_cast<cuuint64_t>(cols) * sizeof(float)};
+    const cuuint32_t box[2] = {32u, static_cast<cuuint32_t>(box_rows)};
+    const cuuint32_t estr[2] = {1u, 1u};
+    return g_t5_encode(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<void*>(base), dims, strides, box, estr,
+                       CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                       CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+static int lt_tile(int M) { return M <= 32 ? 32 : M <= 64 ? 64 : 128; }
+
+// Into how many parts K is cut: the least of waves of 148 CTAs x (blocks of 64 x BLK + 4 us) + the parts' way through memory,
+// with the measured time of a block (1.5 us at 128 tokens, 1.0 below).  500 tokens: 6144 x 4096 takes 2 (221 -> 201 us), 4096
+// x 4096 stays whole (117; in eight parts 214); 17 tokens of 4096 x 12288: 4 (256 -> 75).
+extern "C" int llm_linear_f32_tcgen05_splits(int M, int N, int K) {
+    if (M <= 0 || N <= 0 || K <= 0) return 1;
+    const int nt = lt_tile(M);
+    const long long tiles = static_cast<long long>((M + nt - 1) / nt) * ((N + LT_ROWS - 1) / LT_ROWS);
+    const int kb = (K + LT_K - 1) / LT_K;
+    const double block = nt == 128 ? 1.5 : 1.0;
+    int best = 1;
+    double least = 0.0;
+    for (int s = 1; s <= 8 && (s == 1 || kb / s >= 8); ++s) {        // a part is at least eight blocks
+        const int per = (kb + s - 1) / s;
+        if (s > 1 && ((kb + per - 1) / per != s || 4LL * s * M * N > (64 << 20))) continue;
+        const double us = static_cast<double>((tiles * s + 147) / 148) * (per * block + 4.0) + (s > 1 ? 3.0 + 8e-6 * s * M * N / 4.0 : 0.0);
+        if (s == 1 || us < least) { least = us; best = s; }
+    }
+    return best;
+}
+
+// x: float32 [M, K]; w: float32 [N, K]; y: float32 [M, N]; planes: room for 3 * M * K bfloat16; parts: room for splits * M * N
+// floats when splits > 1.  K a multiple of 8.
+extern "C" int llm_linear_f32_tcgen05(const float* x, const float* w, float* y, void* planes, float* parts, int splits, int M, int N,
+                                      int K, int32_t* status, uintptr_t stream) {
+    if (M <= 0 || N <= 0) return LLM_OK;
+    if (K <= 0 || (K & 7) || splits < 1 || (splits > 1 && !parts) || 3LL * M >= (1LL << 31)) return LLM_REFUSED_SIZE;
+    if (!aligned16(x) || !aligned16(w) || !aligned16(planes)) return LLM_REFUSED_ALIGN;
+    const int nt = lt_tile(M), kb = (K + LT_K - 1) / LT_K, per = (kb + splits - 1) / splits;
+    if ((kb + per - 1) / per != splits || (N + LT_ROWS - 1) / LT_ROWS > 65535) return LLM_REFUSED_SIZE;
+    CUtensorMap w_map, x_map;
+    if (!lt_encode_f32(&w_map, w, K, N, LT_ROWS) || !t5_encode_2d(&x_map, planes, K, 3LL * M, LT_K, nt)) return LLM_REFUSED_SIZE;
+    cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
+    const long long pieces = static_cast<long long>(M) * K / 8;
+    launch_pdl(linear_f32_split_kernel, dim3(static_cast<unsigned>((pieces + 255) / 256)), dim3(256), 0, s, x, static_cast<uint4*>(planes), pieces);
+    const dim3 grid((M + nt - 1) / nt, (N + LT_ROWS - 1) / LT_ROWS, splits);
+    float* to = splits > 1 ? parts : y;
+#define GO(NT, WB, XS, PS)                                                                                                    \
+    {                                                                                                                   \
+        auto kern = linear_f32_tcgen05_kernel<NT, WB, XS, PS>;                                                                 \
+        const size_t smem = WB * LT_BOX + XS * 3 * NT * LT_K * sizeof(bf16) + 1024;                    \
+        const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)); \
+        if (e != cudaSuccess) return static_cast<int>(e);                                                               \
+        launch_pdl(kern, grid, dim3(LT_THREADS), smem, s, w_map, x_map, x, w, to, M, N, K, per, status);                \
+    }
+    if (nt == 32) GO(32, 8, 5, 4) else if (nt == 64) GO(64, 6, 5, 4) else GO(128, 4, 3, 2)
+#undef GO
+    if (splits > 1) {
+        const long long n = static_cast<long long>(M) * N;
+        launch_pdl(linear_f32_sum_kernel, dim3(static_cast<unsigned>((n + 255) / 256)), dim3(256), 0, s, static_cast<const float*>(parts), y, n, splits);
+    }
+    return launch_status();
+}

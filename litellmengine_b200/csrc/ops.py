@@ -1893,7 +1893,7 @@ _stream_status: Dict[str, torch.Tensor] = {}
 
 def stream_status(device) -> torch.Tensor:
     """The status word of the engine's matrix products (code 8: a bounded wait of the weight-streaming
-    product ran out; 9: of the paired product)."""
+    product ran out; 9: of the paired or the float32 tcgen05 product)."""
     key = str(device)
     t = _stream_status.get(key)
     if t is None:
@@ -2012,6 +2012,37 @@ def linear_f32(x: torch.Tensor, weight: torch.Tensor) -> torch.Tensor:
     return out
 
 
+F32_TENSOR_MIN_WEIGHTS = 1 << 21    # values of a weight matrix from which the tensor-core form beats the library's product
+F32_TENSOR_ROWS = 2048              # rows at a time: the split of x takes six bytes a value of scratch
+
+
+def linear_f32_tcgen05(x: torch.Tensor, weight: torch.Tensor) -> torch.Tensor:
+    """x [M, K] @ weight[N, K]^T, all float32, on the tensor cores: both operands as exact sums of three bfloat16 values, six
+    products of them accumulated in float32 (see csrc/gemm_f32_tcgen05.cu; its error is below that of a float32 product added
+    in order).  K must be a multiple of 8 and both operands 16-byte aligned."""
+    _dev(x, weight)
+    if x.dtype != torch.float32 or weight.dtype != torch.float32:
+        raise KernelError("the float32 product takes float32 operands")
+    M, K = x.shape
+    N = weight.shape[0]
+    if weight.shape[1] != K:
+        raise KernelError("x and weight disagree on K")
+    out = torch.empty((M, N), dtype=torch.float32, device=x.device)
+    f = _fn("gemm_f32_tcgen05", "llm_linear_f32_tcgen05",
+            [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_void_p])
+    splits_of = _fn("gemm_f32_tcgen05", "llm_linear_f32_tcgen05_splits", [c_int, c_int, c_int])
+    global launch_count
+    for at in range(0, M, F32_TENSOR_ROWS):
+        m = min(M - at, F32_TENSOR_ROWS)
+        planes = torch.empty(3 * m * K, dtype=torch.bfloat16, device=x.device)
+        splits = splits_of(m, N, K)
+        parts = torch.empty(splits * m * N, dtype=torch.float32, device=x.device) if splits > 1 else None
+        _check(f(x.data_ptr() + 4 * at * K, _ptr(weight), out.data_ptr() + 4 * at * N, _ptr(planes), _ptr(parts), splits, m, N, K,
+                 _ptr(stream_status(x.device)), _stream()), "linear_f32_tcgen05")
+        launch_count += 2 if splits > 1 else 1            # the split of x and the sum of the parts
+    return out
+
+
 def linear(x: torch.Tensor, weight: torch.Tensor, out_dtype: Optional[torch.dtype] = None,
            partials_ok: bool = False):
     """x [T, K] @ weight[N, K]^T.  Up to 16 bfloat16 rows (decode steps; up to 32 for the small products
@@ -2023,7 +2054,8 @@ def linear(x: torch.Tensor, weight: torch.Tensor, out_dtype: Optional[torch.dtyp
     goes through the library matrix product (under `LLM_PAIR=all`, prompt portions take the paired tcgen05
     product `linear_pair`; by default only the gate/up product does, through `linear_silu_mul`) (the reference uses cuBLAS for all its products,
     src/layers/linear.cu:169-215).  bfloat16 operands accumulate in float32; a float32 weight
-    keeps its product in true float32 (no TF32), whatever x is: up to 16 rows in the engine's own streaming kernel."""
+    keeps its product in true float32 (no TF32), whatever x is: up to 16 rows in the engine's own streaming kernel, more rows of large matrices
+    on the tensor cores as exact sums of bfloat16 values."""
     _dev(x, weight)
     rows = x.shape[0]
     if (x.dtype == torch.bfloat16 and weight.dtype == torch.bfloat16 and x.shape[1] % 8 == 0 and weight.data_ptr() % 16 == 0
@@ -2039,6 +2071,9 @@ def linear(x: torch.Tensor, weight: torch.Tensor, out_dtype: Optional[torch.dtyp
         if (1 <= rows <= STREAM_F32_MAX_ROWS and 0 < weight.shape[0] <= 1 << 20 and x.shape[1] % 4 == 0 and x.shape[1] > 0
                 and x.data_ptr() % 16 == 0 and weight.data_ptr() % 16 == 0):
             y = linear_f32(x, weight)
+        elif (rows > STREAM_F32_MAX_ROWS and weight.numel() >= F32_TENSOR_MIN_WEIGHTS and weight.shape[0] <= 1 << 22
+              and x.shape[1] % 8 == 0 and x.shape[1] >= 64 and x.data_ptr() % 16 == 0 and weight.data_ptr() % 16 == 0):
+            y = linear_f32_tcgen05(x, weight)
         else:
             y = torch.mm(x, weight.t())
         return y if want == torch.float32 else y.to(want)

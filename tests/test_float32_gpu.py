@@ -33,6 +33,43 @@ def test_streaming_product(M, N, K):
         assert bool(torch.isinf(bad[:, N // 2]).all()) and bool(torch.isfinite(bad).sum() == M * (N - 1))
 
 
+@pytest.mark.parametrize("M,N,K", [(1, 1, 64), (17, 130, 72), (32, 128, 128), (33, 1000, 136), (64, 257, 520), (65, 300, 1000),
+                                   (128, 4096, 512), (129, 31, 4096), (500, 1024, 2048), (2050, 160, 64)])
+def test_tensor_core_product(M, N, K):
+    """Tiles of 32, 64 and 128 tokens and 128 weight rows, blocks of 64 along K, whole and in parts."""
+    torch.manual_seed(M * 1000 + N)
+    x, w = torch.randn(M, K, device=DEV), torch.randn(N, K, device=DEV)
+    x[0, :8] *= 1e18                                          # a wide range of exponents in one sum
+    w[0, :8] *= 1e-18
+    ref = x.double() @ w.double().T
+    got = ops().linear_f32_tcgen05(x, w)
+    # three terms of 2^-23 of a product are left out, a block's 24 additions are cut at the last place, the blocks' sums rounded
+    bound = (3 * 2 * U + 24 * 2 * U + -(-K // 64) * U) * (x.double().abs() @ w.double().abs().T)
+    assert bool(((got.double() - ref).abs() <= bound).all())
+    assert float((got - ref).norm() / ref.norm()) < 4e-7
+    assert ops().stream_status(DEV).tolist() == [0, 0]
+    if K >= 128 and M > 1 and N > 3:                           # infinities and NaN as plain multiply-adds give them
+        x[1, 5], w[2, 70], w[3, 9] = float("inf"), float("-inf"), float("nan")
+        x[0] = w[1] = 1e30
+        lib, got = torch.mm(x, w.t()), ops().linear_f32_tcgen05(x, w)
+        assert torch.equal(torch.isnan(got), torch.isnan(lib)) and torch.equal(torch.isinf(got), torch.isinf(lib))
+        assert torch.equal(got[torch.isinf(got)], lib[torch.isinf(lib)])
+        assert ops().stream_status(DEV).tolist() == [0, 0]
+
+
+def test_the_product_of_each_size_takes_its_path():
+    o = ops()
+    w = torch.randn(4096, 512, device=DEV)
+    for rows, k in ((16, 512), (17, 512), (300, 512), (17, 508), (40, 256)):
+        x, ww = torch.randn(rows, k, device=DEV), w[:, :k].contiguous()
+        before = o.launch_count
+        y = o.linear(x, ww)
+        own = o.launch_count - before
+        assert (own > 0) == (rows <= 16 or (k % 8 == 0 and ww.numel() >= o.F32_TENSOR_MIN_WEIGHTS)), (rows, k, own)
+        ref = x.double() @ ww.double().t()
+        assert float((y - ref).norm() / ref.norm()) < 2e-6
+
+
 def pages_of(lens, nkv, d, page, g):
     width = max(-(-n // page) for n in lens)
     perm = torch.randperm(len(lens) * width + 2, generator=g)
