@@ -8,9 +8,9 @@
 //            is one row.  The 8 x group partial scores of a lane are added across lanes by halving exchanges (31 shuffles
 //            for 32 sums instead of 160), which leaves lane i with the score of (key i / group, head i % group).
 //   prefill  portions of several tokens.  What bounds it: multiply-adds.  A block takes 64 query rows of one head, tiles of
-//            64 keys; a thread makes 8 x 4 scores and 8 rows x 8 output columns, 10.7 and 16 multiply-adds per shared
+//            64 keys; a thread makes 4 x 4 scores and 4 rows x 8 output columns, 8 and 10.7 multiply-adds per shared
 //            16-byte load, where the general kernel made one dot product a lane and one value column a load.
-// Measured, 32 query heads over 8 of 128, against the general kernel: a prompt of 500 tokens 888 -> 167 us; 8 single tokens
+// Measured, 32 query heads over 8 of 128, against the general kernel: a prompt of 500 tokens 888 -> 129 us (167 with 8 rows a thread in blocks of 128 threads and the tile list outermost); 8 single tokens
 // at contexts of 1,125 to 1,500 190 -> 29 us (85 MB of keys and values: 2.9 TB/s; the exchanges, not the bytes, are what is
 // left).
 #include "common.cuh"
@@ -234,7 +234,8 @@ extern "C" int llm_attention_f32_decode(
 // ---- portions of several tokens ---------------------------------------------------------------------------------
 #define FP_ROWS 64
 #define FP_KEYS 64
-#define FP_THREADS 128
+#define FP_THREADS 256
+#define FP_RPT (FP_ROWS * 16 / FP_THREADS)      // query rows a thread takes
 
 template <int D>
 __global__ void __launch_bounds__(FP_THREADS, 2) attention_f32_prefill_kernel(
@@ -250,11 +251,11 @@ __global__ void __launch_bounds__(FP_THREADS, 2) attention_f32_prefill_kernel(
     float* vs = ks + FP_KEYS * KLD;                          // [64][D]
     float* ps = ks;
     const int h = blockIdx.x, kvh = h / (nq / nkv);
-    const int e = tiles[2 * blockIdx.y];
+    const int e = tiles[2 * blockIdx.z], part = gridDim.y - 1 - blockIdx.y;      // the part that walks more keys first
     if (e < 0) return;                                       // a padding entry of the tile list
-    const int q0 = tiles[2 * blockIdx.y + 1] + FP_ROWS * blockIdx.z;
+    const int q0 = tiles[2 * blockIdx.z + 1] + FP_ROWS * part;
     const int q_len = entry_q_len[e], past = entry_kv_len[e] - q_len;
-    const int rows_here = min(min(FP_ROWS, tile_rows - FP_ROWS * static_cast<int>(blockIdx.z)), q_len - q0);
+    const int rows_here = min(min(FP_ROWS, tile_rows - FP_ROWS * part), q_len - q0);
     if (rows_here <= 0) return;
     const int row_base = entry_q_start[e] + q0;
     const int32_t* table = block_table + static_cast<size_t>(entry_slot[e]) * table_stride;
@@ -268,9 +269,9 @@ __global__ void __launch_bounds__(FP_THREADS, 2) attention_f32_prefill_kernel(
         v.x *= scale; v.y *= scale; v.z *= scale; v.w *= scale;
         *reinterpret_cast<float4*>(qs + r * D + 4 * c) = v;
     }
-    float o[8][4 * OC], m[8], l[8];
+    float o[FP_RPT][4 * OC], m[FP_RPT], l[FP_RPT];
 #pragma unroll
-    for (int r = 0; r < 8; ++r) {
+    for (int r = 0; r < FP_RPT; ++r) {
         m[r] = -CUDART_INF_F; l[r] = 0.0f;
 #pragma unroll
         for (int c = 0; c < 4 * OC; ++c) o[r][c] = 0.0f;
@@ -305,17 +306,17 @@ __global__ void __launch_bounds__(FP_THREADS, 2) attention_f32_prefill_kernel(
         stage(vs, D, kt, nkv * khead);
         asm volatile("cp.async.wait_group 1;\n" ::: "memory");
         __syncthreads();                                     // the keys (and at first the queries) are in place
-        float s[8][4];
+        float s[FP_RPT][4];
 #pragma unroll
-        for (int r = 0; r < 8; ++r) s[r][0] = s[r][1] = s[r][2] = s[r][3] = 0.0f;
+        for (int r = 0; r < FP_RPT; ++r) s[r][0] = s[r][1] = s[r][2] = s[r][3] = 0.0f;
 #pragma unroll 2
         for (int k = 0; k < D; k += 4) {
             float4 kb[4];
 #pragma unroll
             for (int c = 0; c < 4; ++c) kb[c] = *reinterpret_cast<const float4*>(ks + (tx + 16 * c) * KLD + k);
 #pragma unroll
-            for (int r = 0; r < 8; ++r) {
-                const float4 a = *reinterpret_cast<const float4*>(qs + (ty * 8 + r) * D + k);
+            for (int r = 0; r < FP_RPT; ++r) {
+                const float4 a = *reinterpret_cast<const float4*>(qs + (ty * FP_RPT + r) * D + k);
 #pragma unroll
                 for (int c = 0; c < 4; ++c) {
                     s[r][c] = fmaf(a.x, kb[c].x, s[r][c]);
@@ -327,8 +328,8 @@ __global__ void __launch_bounds__(FP_THREADS, 2) attention_f32_prefill_kernel(
         }
         __syncthreads();                                     // the keys are read: the weights may take their place
 #pragma unroll
-        for (int r = 0; r < 8; ++r) {
-            const int pos = pos_first + ty * 8 + r, lo = first_visible(pos, window);
+        for (int r = 0; r < FP_RPT; ++r) {
+            const int pos = pos_first + ty * FP_RPT + r, lo = first_visible(pos, window);
             float top = -CUDART_INF_F;
 #pragma unroll
             for (int c = 0; c < 4; ++c) {
@@ -345,7 +346,7 @@ __global__ void __launch_bounds__(FP_THREADS, 2) attention_f32_prefill_kernel(
 #pragma unroll
             for (int c = 0; c < 4; ++c) {
                 const float p = expf(s[r][c] - base);
-                ps[(ty * 8 + r) * PLD + tx + 16 * c] = p;
+                ps[(ty * FP_RPT + r) * PLD + tx + 16 * c] = p;
                 sum += p;
             }
             l[r] = l[r] * alpha + sum;
@@ -357,16 +358,16 @@ __global__ void __launch_bounds__(FP_THREADS, 2) attention_f32_prefill_kernel(
         __syncthreads();                                     // weights and values are in place
 #pragma unroll 1
         for (int k = 0; k < FP_KEYS; k += 4) {
-            float4 p[8];
+            float4 p[FP_RPT];
 #pragma unroll
-            for (int r = 0; r < 8; ++r) p[r] = *reinterpret_cast<const float4*>(ps + (ty * 8 + r) * PLD + k);
+            for (int r = 0; r < FP_RPT; ++r) p[r] = *reinterpret_cast<const float4*>(ps + (ty * FP_RPT + r) * PLD + k);
 #pragma unroll
             for (int u = 0; u < 4; ++u)
 #pragma unroll
                 for (int c = 0; c < OC; ++c) {
                     const float4 v = *reinterpret_cast<const float4*>(vs + (k + u) * D + c * 64 + tx * 4);
 #pragma unroll
-                    for (int r = 0; r < 8; ++r) {
+                    for (int r = 0; r < FP_RPT; ++r) {
                         const float w = u == 0 ? p[r].x : u == 1 ? p[r].y : u == 2 ? p[r].z : p[r].w;
                         o[r][4 * c] = fmaf(w, v.x, o[r][4 * c]);
                         o[r][4 * c + 1] = fmaf(w, v.y, o[r][4 * c + 1]);
@@ -378,12 +379,12 @@ __global__ void __launch_bounds__(FP_THREADS, 2) attention_f32_prefill_kernel(
         __syncthreads();                                     // before the next tile overwrites them
     }
 #pragma unroll
-    for (int r = 0; r < 8; ++r) {
+    for (int r = 0; r < FP_RPT; ++r) {
 #pragma unroll
         for (int off = 1; off < 16; off <<= 1) l[r] += __shfl_xor_sync(0xffffffffu, l[r], off);
-        if (ty * 8 + r >= rows_here) continue;
+        if (ty * FP_RPT + r >= rows_here) continue;
         const float inv = 1.0f / l[r];
-        float* orow = out + (static_cast<size_t>(row_base + ty * 8 + r) * nq + h) * D;
+        float* orow = out + (static_cast<size_t>(row_base + ty * FP_RPT + r) * nq + h) * D;
 #pragma unroll
         for (int c = 0; c < OC; ++c)
             *reinterpret_cast<float4*>(orow + c * 64 + tx * 4) =
@@ -407,7 +408,8 @@ extern "C" int llm_attention_f32_prefill(
     if (!aligned16(q) || !aligned16(out) || !aligned16(cache)) return LLM_REFUSED_ALIGN;
     cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
     const size_t smem = static_cast<size_t>(FP_ROWS * d + FP_KEYS * (d + 4) + FP_KEYS * d) * sizeof(float);
-    const dim3 grid(nq, n_tiles, (tile_rows + FP_ROWS - 1) / FP_ROWS);
+    // blocks start in this order: tiles come longest walk first, and the heads of one before the next
+    const dim3 grid(nq, (tile_rows + FP_ROWS - 1) / FP_ROWS, n_tiles);
 #define GO(D)                                                                                                              \
     {                                                                                                                      \
         const cudaError_t e = cudaFuncSetAttribute(attention_f32_prefill_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, \
