@@ -74,13 +74,6 @@ __device__ __forceinline__ void lt_st8(unsigned taddr, const unsigned (&r)[8]) {
     asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};\n" ::
                      "r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]) : "memory");
 }
-__device__ __forceinline__ void lt_ld16(unsigned taddr, unsigned (&r)[16]) {
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];\n"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-                   "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-                 : "r"(taddr) : "memory");
-}
-
 __global__ void linear_f32_split_kernel(const float* __restrict__ x, uint4* __restrict__ planes, long long pieces) {
     pdl_begin();
     const long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
@@ -177,6 +170,7 @@ __global__ void __launch_bounds__(LT_THREADS, 1) linear_f32_tcgen05_kernel(
             }
         }
     } else if (warp == 1) {
+        pdl_wait();                                               // before any bounded wait: the kernel in front may take its time
         if (lane == 0) {
             constexpr unsigned IDESC = t5_idesc(LT_ROWS, NT, 0);
             const unsigned long long xd = t5_desc(x_s, 16, 1024);
@@ -211,6 +205,7 @@ __global__ void __launch_bounds__(LT_THREADS, 1) linear_f32_tcgen05_kernel(
         }
     } else if (warp < 10) {
         // ---- split the weights: two threads a row, each 16 k-values of every box ----
+        pdl_wait();
         const int quarter = warp & 3, part = (warp - 2) >> 2, r = quarter * 32 + lane, sw = r & 7;
         const unsigned planes = tmem + (static_cast<unsigned>(quarter * 32) << 16) + PLANE_COL + 8 * part;
         bool ok = true;
@@ -255,7 +250,7 @@ __global__ void __launch_bounds__(LT_THREADS, 1) linear_f32_tcgen05_kernel(
 #pragma unroll
             for (int c = 0; c < COLS; c += 16) {
                 unsigned r[16];
-                lt_ld16(addr + st * NT + c, r);
+                t5_ld16(addr + st * NT + c, r);
                 t5_wait_ld();
 #pragma unroll
                 for (int i = 0; i < 16; ++i) acc[c + i] += __uint_as_float(r[i]);

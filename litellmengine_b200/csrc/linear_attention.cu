@@ -445,10 +445,11 @@ __global__ void __launch_bounds__(MAX_THREADS) gla_scan_kernel(
 // queries serves eight columns, 3 RR / 4 + 2 loads for 24 RR multiply-adds, and packed two-wide arithmetic (two rows an
 // instruction) halves what has to be issued.  Sixteen lanes hold the rows of a column (a lane's rows are 4 rg .. + 3 and, at
 // 128 rows, 64 + 4 rg .. + 3, so that a quarter-warp's loads are contiguous); their shares of o are added by halving
-// exchanges, eight shuffles for eight columns, and one lane of two leaves a column's sum in shared memory.  A block is 2 V
+// exchanges, two tokens at a time: fifteen shuffles for sixteen sums, one of which each lane leaves in shared memory.  A block is 2 V
 // threads, two blocks an SM.  Same modes, staging and epilogue as above; every state element is updated by the same
 // operations in the same order (k v, then decay times state plus that), only o's sum runs over the rows in another order.
-// 2,048 tokens, 16 heads of 128 x 128: local pass and output pass 193 us each -> 67 and 161 us.
+// 2,048 tokens, 16 heads of 128 x 128: local pass and output pass 193 us each -> 66 and 113 us
+// (161 with one token's sums at a time and the gates read from global memory in the epilogue).
 typedef unsigned long long gla_pair;
 __device__ __forceinline__ gla_pair gla_mul2(gla_pair a, gla_pair b) {
     gla_pair r;
@@ -499,7 +500,7 @@ __global__ void __launch_bounds__(256, 2) gla_scan_tiled_kernel(
     }
     const int tid = threadIdx.x, nthreads = blockDim.x, warp = tid >> 5, lane = tid & 31;
     const int rg = lane & 15, col0 = (tid >> 4) * 8;
-    const int buf_floats = GLA_TB * (3 * D + V);
+    const int buf_floats = GLA_TB * (3 * D + 2 * V);
     float* part = smem + 2 * buf_floats;             // [TB][V]
     const size_t HD = static_cast<size_t>(H) * D, per = static_cast<size_t>(D) * V;
     float* slot_state = state + (static_cast<size_t>(entry_slot[entry]) * H + h) * per;
@@ -538,6 +539,7 @@ __global__ void __launch_bounds__(256, 2) gla_scan_tiled_kernel(
         for (int idx = tid; idx < nb * v4; idx += nthreads) {
             const int tok = idx / v4, c = (idx - tok * v4) << 2;
             gla_cp16(bv + tok * V + c, proj + (base + tok) * stride + v_off + h * V + c);
+            if (OUTPUTS) gla_cp16(bv + (GLA_TB + tok) * V + c, proj + (base + tok) * stride + g_off + h * V + c);      // the gates
         }
         asm volatile("cp.async.commit_group;\n" ::);
     };
@@ -556,51 +558,62 @@ __global__ void __launch_bounds__(256, 2) gla_scan_tiled_kernel(
         const float* sk = sq + GLA_TB * D;
         const float* sa = sk + GLA_TB * D;
         const float* sv = sa + GLA_TB * D;
-        for (int tok = 0; tok < nb; ++tok) {
-            gla_pair k[RR / 2], a[RR / 2], q[RR / 2];
+        // two tokens at a time: their sixteen sums over the rows go through one chain of exchanges
+        for (int tok0 = 0; tok0 < nb; tok0 += 2) {
+            float o[16];
 #pragma unroll
-            for (int g = 0; g < Q4; ++g) {
-                const ulonglong2 kk = *reinterpret_cast<const ulonglong2*>(sk + tok * D + 64 * g + 4 * rg);
-                const ulonglong2 aa = *reinterpret_cast<const ulonglong2*>(sa + tok * D + 64 * g + 4 * rg);
-                k[2 * g] = kk.x; k[2 * g + 1] = kk.y;
-                a[2 * g] = aa.x; a[2 * g + 1] = aa.y;
-                if (OUTPUTS) {
-                    const ulonglong2 qq = *reinterpret_cast<const ulonglong2*>(sq + tok * D + 64 * g + 4 * rg);
-                    q[2 * g] = qq.x; q[2 * g + 1] = qq.y;
+            for (int u = 0; u < 2; ++u) {
+                const int tok = tok0 + u;
+                if (u == 1 && tok >= nb) {
+#pragma unroll
+                    for (int c = 0; c < 8; ++c) o[8 + c] = 0.0f;
+                    break;
                 }
-            }
-            float v[8], o[8];
-            load8(sv + tok * V + col0, v);
+                gla_pair k[RR / 2], a[RR / 2], q[RR / 2];
 #pragma unroll
-            for (int c = 0; c < 8; ++c) {
-                const gla_pair vv = gla_both(v[c], v[c]);
-                gla_pair share = 0;
-#pragma unroll
-                for (int p = 0; p < RR / 2; ++p) {
-                    S[p][c] = gla_fma2(a[p], S[p][c], gla_mul2(k[p], vv));
-                    if (OUTPUTS) share = p == 0 ? gla_mul2(S[p][c], q[p]) : gla_fma2(S[p][c], q[p], share);
+                for (int g = 0; g < Q4; ++g) {
+                    const ulonglong2 kk = *reinterpret_cast<const ulonglong2*>(sk + tok * D + 64 * g + 4 * rg);
+                    const ulonglong2 aa = *reinterpret_cast<const ulonglong2*>(sa + tok * D + 64 * g + 4 * rg);
+                    k[2 * g] = kk.x; k[2 * g + 1] = kk.y;
+                    a[2 * g] = aa.x; a[2 * g + 1] = aa.y;
+                    if (OUTPUTS) {
+                        const ulonglong2 qq = *reinterpret_cast<const ulonglong2*>(sq + tok * D + 64 * g + 4 * rg);
+                        q[2 * g] = qq.x; q[2 * g + 1] = qq.y;
+                    }
                 }
-                if (OUTPUTS) {
-                    const float2 t = gla_split(share);
-                    o[c] = t.x + t.y;
-                }
-            }
-            if (MODE == GLA_LOCAL) {                 // the chunk's total decay per key channel
+                float v[8];
+                load8(sv + tok * V + col0, v);
 #pragma unroll
-                for (int p = 0; p < RR / 2; ++p) A[p] = gla_mul2(A[p], a[p]);
+                for (int c = 0; c < 8; ++c) {
+                    const gla_pair vv = gla_both(v[c], v[c]);
+                    gla_pair share = 0;
+#pragma unroll
+                    for (int p = 0; p < RR / 2; ++p) {
+                        S[p][c] = gla_fma2(a[p], S[p][c], gla_mul2(k[p], vv));
+                        if (OUTPUTS) share = p == 0 ? gla_mul2(S[p][c], q[p]) : gla_fma2(S[p][c], q[p], share);
+                    }
+                    if (OUTPUTS) {
+                        const float2 t = gla_split(share);
+                        o[8 * u + c] = t.x + t.y;
+                    }
+                }
+                if (MODE == GLA_LOCAL) {             // the chunk's total decay per key channel
+#pragma unroll
+                    for (int p = 0; p < RR / 2; ++p) A[p] = gla_mul2(A[p], a[p]);
+                }
             }
             if (OUTPUTS) {
 #pragma unroll
-                for (int off = 8, n = 4; n >= 1; off >>= 1, n >>= 1)
+                for (int off = 8, n = 8; n >= 1; off >>= 1, n >>= 1)
 #pragma unroll
-                    for (int i = 0; i < 4; ++i)
+                    for (int i = 0; i < 8; ++i)
                         if (i < n) {
                             const bool up = (lane & off) != 0;
                             const float send = up ? o[i] : o[i + n], keep = up ? o[i + n] : o[i];
                             o[i] = keep + __shfl_xor_sync(0xffffffffu, send, off);
                         }
-                o[0] += __shfl_xor_sync(0xffffffffu, o[0], 1);
-                if ((lane & 1) == 0) part[tok * V + col0 + (rg >> 1)] = o[0];
+                const int tok = tok0 + (rg >> 3);     // lane rg holds column rg % 8 of token rg / 8
+                if (tok < nb) part[tok * V + col0 + (rg & 7)] = o[0];
             }
         }
         __syncthreads();
@@ -613,11 +626,13 @@ __global__ void __launch_bounds__(256, 2) gla_scan_tiled_kernel(
                     ss += x * x;
                 }
                 const float inv = q_scale / sqrtf(warp_sum(ss) / static_cast<float>(V) + eps) * out_scale;
-                const float* gr = proj + (base + tok) * stride + g_off + h * V;
+                const float* gr = sv + (GLA_TB + tok) * V;
                 TO* orow = out + (base + tok) * out_stride + out_off + h * V;
                 for (int c = lane; c < V; c += 32) orow[c] = from_f32<TO>(o[c] * inv * norm_w[c] * recur_gate(gr[c], 2));
             }
-            // the next batch's shares are written after its first barrier, this buffer is filled again two batches on
+            // the next batch's shares are written after its first barrier; this buffer, whose gates were just read, is filled
+            // again by the next batch's staging: every warp must be done with it
+            __syncthreads();
         }
     }
     if (MODE == GLA_OUT) return;
@@ -733,8 +748,8 @@ extern "C" int llm_recur_scan(
                     aligned16(proj) && (decay_kind || aligned16(la));
     if (smem > 220 * 1024) return LLM_REFUSED_SIZE;
     if (out_dtype != LLM_DT_F32 && out_dtype != LLM_DT_BF16) return LLM_REFUSED_DTYPE;
-    if (decay_kind == 0 && vec && gla_tiled_takes(D, V) && aligned16(state) && (mode == GLA_FULL || aligned16(scratch_s))) {
-        const size_t need = static_cast<size_t>(GLA_TB) * (2 * (3 * D + V) + V) * sizeof(float);
+    if (decay_kind == 0 && vec && g_off % 4 == 0 && gla_tiled_takes(D, V) && aligned16(state) && (mode == GLA_FULL || aligned16(scratch_s))) {
+        const size_t need = static_cast<size_t>(GLA_TB) * (2 * (3 * D + 2 * V) + V) * sizeof(float);
 #define TILED(RR, MODE, TO)                                                                                          \
         do {                                                                                                          \
             auto kern = gla_scan_tiled_kernel<RR, MODE, TO>;                                                          \

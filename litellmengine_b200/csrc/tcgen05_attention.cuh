@@ -1,4 +1,4 @@
-// What the tcgen05 attention kernels share: mbarriers with bounded waits, tensor-map copies, the tensor-memory
+// What the tcgen05 kernels of attention and of the matrix products share: mbarriers with bounded waits, tensor-map copies, the tensor-memory
 // instructions (cta_group::1, bfloat16 operands, float32 accumulators) and the tensor maps' encoding.
 #pragma once
 
@@ -69,6 +69,13 @@ __device__ __forceinline__ void t5_ld32(unsigned taddr, unsigned (&r)[32]) {
           "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]),
           "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
         : "r"(taddr) : "memory");
+}
+// 16 of them
+__device__ __forceinline__ void t5_ld16(unsigned taddr, unsigned (&r)[16]) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];\n"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+                   "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+                 : "r"(taddr) : "memory");
 }
 __device__ __forceinline__ void t5_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory"); }
 __device__ __forceinline__ void t5_st16(unsigned taddr, const unsigned (&r)[16]) {
