@@ -10,21 +10,24 @@
 //
 // The columns of S do not touch one another: column v needs k, q, g of the head and its own v_t.  So blocks take any
 // number of columns of any head, and a long prompt of one request spreads over as many SMs as it has columns without
-// being cut in time.  C columns (1, 2 or 4) are L lanes of a warp, each holding R = DP / L rows of all of them (rows 4 l +
-// 4 L j .. + 3 of lane l), so that a vector read from shared memory serves C columns.  Along time four tokens go together.  With p_i the product of the decays of the chunk's tokens up
+// being cut in time.  C columns (1, 2 or 4) are L lanes of a warp, each holding R = DP / L rows of all of them (rows
+// 4 l + 4 L j .. + 3 of lane l), so that a vector read from shared memory serves C columns.  Along time eight tokens go
+// together: a chunk's chain of loads, products, exchanges and dependent u is what a long portion waits for (2,048 tokens
+// of one request, 16 heads of 128 x 128, 361 us with four tokens a chunk, 272 with eight).  With p_i the product of the
+// decays of the chunk's tokens up
 // to i, s_j that of the tokens behind j, and S the state that enters the chunk,
 //
-//     r_i = S^T (p_i k_i)     x_i = S^T (p_i q_i)                            eight products with S, one exchange of sums
+//     r_i = S^T (p_i k_i)     x_i = S^T (p_i q_i)                            sixteen products with S, one exchange of sums
 //     u_i = beta_i (v_i - r_i - sum_{j<i} A_ij u_j)                           A_ij = sum_d k_i k_j (decays from j to i)
 //     o_i = x_i + sum_{j<=i} B_ij u_j                                         B_ij = sum_d q_i k_j (decays from j to i)
-//     S  <- p_3 S + sum_j (s_j k_j) u_j
+//     S  <- p_7 S + sum_j (s_j k_j) u_j
 //
 // which is the recurrence with its sums regrouped: every factor is a product of decays, none is divided by one.  The
 // vectors p k, p q, s k and the numbers A, B are the same for all columns of a head.
 //
 //   delta_prepare_kernel   a warp per (four tokens, head of q, k or v): convolution, silu, unit norm of q and k; beta
 //   delta_lowrank_kernel   the second halves of both low-rank projections: decays and gates
-//   delta_chunk_kernel     a warp per (four tokens, head): p k, p q, s k, p_3, A and B
+//   delta_chunk_kernel     a warp per (eight tokens, head): p k, p q, s k, p_7, A and B
 //   delta_scan_kernel      one block per (entry, head, columns): the recurrence over the entry's tokens, staged sixteen
 //                          at a time with cp.async into two buffers; o in 32-bit; keeps the convolutions' last inputs
 //   delta_output_kernel    a warp per (token, head): norm, weight, gate, scale, store in the compute dtype
@@ -40,7 +43,7 @@
 #include "common.cuh"
 
 #define DR_TB 16            // tokens staged at a time
-#define DR_CHUNK 4          // tokens that go through the state together
+#define DR_CHUNK 8          // tokens that go through the state together
 #define DR_LANES 8          // lanes a column of the state is spread over in the decode kernel
 
 __device__ __forceinline__ void dr_cp16(float* smem_dst, const float* src) {
@@ -316,14 +319,14 @@ __device__ __forceinline__ void dr_sums(float (&v)[NV], int lane, int l, float* 
     }
 }
 
-#define DR_NUM 24                             // numbers a chunk: A (six, two unused), then B as [4][4], zero above its diagonal
+#define DR_NUM (2 * DR_CHUNK * DR_CHUNK)      // numbers a chunk: A [8][8], zero from its diagonal on, then B [8][8], zero above it
 
-// Where a chunk's shared vectors and numbers are: chunks start at every fourth row of an entry, so row / 4 + entry is a
+// Where a chunk's shared vectors and numbers are: chunks start at every eighth row of an entry, so row / 8 + entry is a
 // number of its own for each of them.
 __device__ __forceinline__ long long dr_chunk_place(long long row, int entry) { return row / DR_CHUNK + entry; }
 
-// What a chunk's four tokens share over all columns of a head: a warp per (first token of a chunk, head); tokens that
-// begin no chunk have no work.  pk = p k, pq = p q, and in place of the decays s k; total = p_3; num = A and B.
+// What a chunk's eight tokens share over all columns of a head: a warp per (first token of a chunk, head); tokens that
+// begin no chunk have no work.  pk = p k, pq = p q, and in place of the decays s k; total = p_7; num = A and B.
 #define DC_WARPS 4
 template <int DP>
 __global__ void __launch_bounds__(DC_WARPS * 32) delta_chunk_kernel(
@@ -342,13 +345,16 @@ __global__ void __launch_bounds__(DC_WARPS * 32) delta_chunk_kernel(
     const int nt = static_cast<int>(min(static_cast<long long>(DR_CHUNK), row0 + entry_q_len[entry] - t));
     const int kvh = h / (s.H / s.G);
     const size_t place = static_cast<size_t>(dr_chunk_place(t, entry)) * s.H + h;
-    float acc[16];                            // A10 A20 A21 A30 A31 A32, then B00 B10 B11 B20 B21 B22 B30 B31 B32 B33
+    constexpr int CH = DR_CHUNK, NA = CH * (CH - 1) / 2;                    // A's pairs (i, j < i), then B's (i, j <= i)
+    __shared__ float nums[DC_WARPS][DR_NUM];
+    float* mine = nums[threadIdx.x >> 5];
+    float acc[CH * CH];
 #pragma unroll
-    for (int n = 0; n < 16; ++n) acc[n] = 0.0f;
+    for (int n = 0; n < CH * CH; ++n) acc[n] = 0.0f;
     for (int x = lane * 4; x < DP; x += 128) {
-        float kk[4][4], qq[4][4], gg[4][4];
+        float kk[CH][4], qq[CH][4], gg[CH][4];
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
+        for (int i = 0; i < CH; ++i) {
             float4 a = make_float4(0, 0, 0, 0), b = a, c = make_float4(1, 1, 1, 1);      // a missing token
             if (i < nt) {
                 const size_t at = (static_cast<size_t>(t + i) * s.G + kvh) * DP + x;
@@ -360,69 +366,80 @@ __global__ void __launch_bounds__(DC_WARPS * 32) delta_chunk_kernel(
             qq[i][0] = b.x; qq[i][1] = b.y; qq[i][2] = b.z; qq[i][3] = b.w;
             gg[i][0] = c.x; gg[i][1] = c.y; gg[i][2] = c.z; gg[i][3] = c.w;
         }
-        float sk[4][4], p[4] = {1.0f, 1.0f, 1.0f, 1.0f};
+        float p[4] = {1.0f, 1.0f, 1.0f, 1.0f};
 #pragma unroll
-        for (int e = 0; e < 4; ++e)
+        for (int j = 0; j < CH; ++j) {
+            float w[4];
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                float w = kk[j][e];
-                acc[6 + j * (j + 1) / 2 + j] += qq[j][e] * w;
+            for (int e = 0; e < 4; ++e) {
+                w[e] = kk[j][e];
+                acc[NA + j * (j + 1) / 2 + j] += qq[j][e] * w[e];
 #pragma unroll
-                for (int i = j + 1; i < 4; ++i) {
-                    w *= gg[i][e];
-                    acc[i * (i - 1) / 2 + j] += kk[i][e] * w;
-                    acc[6 + i * (i + 1) / 2 + j] += qq[i][e] * w;
+                for (int i = j + 1; i < CH; ++i) {
+                    w[e] *= gg[i][e];
+                    acc[i * (i - 1) / 2 + j] += kk[i][e] * w[e];
+                    acc[NA + i * (i + 1) / 2 + j] += qq[i][e] * w[e];
                 }
-                sk[j][e] = w;
+                p[e] *= gg[j][e];
             }
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-#pragma unroll
-            for (int e = 0; e < 4; ++e) p[e] *= gg[i][e];
-            if (i < nt) {
-                const size_t at = (static_cast<size_t>(t + i) * s.H + h) * DP + x;
-                *reinterpret_cast<float4*>(pk + at) = make_float4(p[0] * kk[i][0], p[1] * kk[i][1], p[2] * kk[i][2], p[3] * kk[i][3]);
-                *reinterpret_cast<float4*>(pq + at) = make_float4(p[0] * qq[i][0], p[1] * qq[i][1], p[2] * qq[i][2], p[3] * qq[i][3]);
-                *reinterpret_cast<float4*>(decay + at) = make_float4(sk[i][0], sk[i][1], sk[i][2], sk[i][3]);
+            if (j < nt) {
+                const size_t at = (static_cast<size_t>(t + j) * s.H + h) * DP + x;
+                *reinterpret_cast<float4*>(pk + at) = make_float4(p[0] * kk[j][0], p[1] * kk[j][1], p[2] * kk[j][2], p[3] * kk[j][3]);
+                *reinterpret_cast<float4*>(pq + at) = make_float4(p[0] * qq[j][0], p[1] * qq[j][1], p[2] * qq[j][2], p[3] * qq[j][3]);
+                *reinterpret_cast<float4*>(decay + at) = make_float4(w[0], w[1], w[2], w[3]);
             }
         }
         *reinterpret_cast<float4*>(total + place * DP + x) = make_float4(p[0], p[1], p[2], p[3]);
     }
-    dr_deal<16, 16>(acc, lane);
-    dr_deal<8, 8>(acc, lane);
-    dr_deal<4, 4>(acc, lane);
-    dr_deal<2, 2>(acc, lane);
-    const float sum = acc[0] + __shfl_xor_sync(0xffffffffu, acc[0], 1);
-    const int n = lane >> 1;                  // the value this pair of lanes holds
+    dr_deal<64, 16>(acc, lane);
+    dr_deal<32, 8>(acc, lane);
+    dr_deal<16, 4>(acc, lane);
+    dr_deal<8, 2>(acc, lane);
+    dr_deal<4, 1>(acc, lane);                 // lane l holds values 2 l and 2 l + 1
+    for (int n = lane; n < DR_NUM; n += 32) mine[n] = 0.0f;
+    __syncwarp();
+#pragma unroll
+    for (int n = 0; n < 2; ++n) {
+        const int v = 2 * lane + n;
+        const bool is_a = v < NA;
+        const int m = is_a ? v : v - NA;
+        int i = is_a ? 1 : 0, at = 0;         // row i of the triangle starts at value `at` and has i (A) or i + 1 (B) of them
+        while (at + (is_a ? i : i + 1) <= m) { at += is_a ? i : i + 1; ++i; }
+        mine[(is_a ? 0 : CH * CH) + CH * i + (m - at)] = acc[n];
+    }
+    __syncwarp();
     float* out = num + place * DR_NUM;
-    if (lane & 1) {                           // the odd lanes clear what is above B's diagonal
-        if (n < 4)
-            for (int j = n + 1; j < 4; ++j) out[8 + 4 * n + j] = 0.0f;
-    } else if (n < 6) {
-        out[n] = sum;
+    *reinterpret_cast<float4*>(out + 4 * lane) = *reinterpret_cast<const float4*>(mine + 4 * lane);
+}
+
+// C neighbouring floats from shared memory.
+template <int C> __device__ __forceinline__ void dr_row(float (&v)[C], const float* p) {
+    if constexpr (C == 4) {
+        const float4 x = *reinterpret_cast<const float4*>(p);
+        v[0] = x.x; v[1] = x.y; v[2] = x.z; v[3] = x.w;
     } else {
-        const int m = n - 6, i = m < 1 ? 0 : m < 3 ? 1 : m < 6 ? 2 : 3;
-        out[8 + 4 * i + (m - i * (i + 1) / 2)] = sum;
+#pragma unroll
+        for (int m = 0; m < C; ++m) v[m] = p[m];
     }
 }
 
 // grid (entries, H, column tiles): WARPS warps a block, each 32 / L groups of C columns.
-template <int DP, int C, int WARPS>
+template <int DP, int C, int WARPS, int L>
 __global__ void __launch_bounds__(WARPS * 32) delta_scan_kernel(
     const DeltaShape s, const float* __restrict__ proj, const float* __restrict__ pq, const float* __restrict__ pk,
     const float* __restrict__ vn, const float* __restrict__ beta, const float* __restrict__ sk, const float* __restrict__ total,
     const float* __restrict__ num, float* __restrict__ o, float* __restrict__ state, const int32_t* __restrict__ positions,
     const int32_t* __restrict__ entry_slot, const int32_t* __restrict__ entry_q_start, const int32_t* __restrict__ entry_q_len) {
     pdl_begin();
-    constexpr int L = DP >= 128 ? 32 : DP / 4, R = DP / L, THREADS = WARPS * 32, CHUNKS = DR_TB / DR_CHUNK;
-    constexpr int COLS = WARPS * (32 / L) * C, NV = 8 * C;
-    // a buffer: q, k, s k, v of a batch of tokens, then beta; then p_3 and the numbers of its chunks
+    constexpr int R = DP / L, THREADS = WARPS * 32, CH = DR_CHUNK, CHUNKS = DR_TB / CH;
+    constexpr int COLS = WARPS * (32 / L) * C, NV = 2 * CH * C;
+    // a buffer: q, k, s k, v of a batch of tokens, then beta; then p_7 and the numbers of its chunks
     constexpr int BUF = DR_TB * (3 * DP + COLS + 1) + CHUNKS * (DP + DR_NUM);
     extern __shared__ __align__(16) float smem[];
     const int entry = blockIdx.x, h = blockIdx.y, tid = threadIdx.x, lane = tid & 31;
     const int c0 = blockIdx.z * COLS;
     const int l = lane & (L - 1), group = tid / L, cb = group * C;          // the group's first column in the block
-    float* sums = smem + 2 * BUF + group * NV;                  // [8][C]: the group's sums, by value and column
+    float* sums = smem + 2 * BUF + group * NV;                  // [16][C]: the group's sums, by value and column
     const long long row0 = entry_q_start[entry];
     const int count = entry_q_len[entry];
     float* slot = state + entry_slot[entry] * s.slot_stride;
@@ -497,70 +514,86 @@ __global__ void __launch_bounds__(WARPS * 32) delta_scan_kernel(
         const float* bn = bt + CHUNKS * DP;
         const int chunks = (nb + DR_CHUNK - 1) / DR_CHUNK;
         for (int ch = 0; ch < chunks; ++ch) {
-            const float* k = bk + ch * 4 * DP + 4 * l;
-            const float* q = bq + ch * 4 * DP + 4 * l;
-            const float* w = bs + ch * 4 * DP + 4 * l;
-            float v[NV];                      // value n of column m at n C + m: r_0 .. r_3, x_0 .. x_3
+            const float* k = bk + ch * CH * DP + 4 * l;
+            const float* q = bq + ch * CH * DP + 4 * l;
+            const float* w = bs + ch * CH * DP + 4 * l;
+            float v[NV];                      // value n of column m at n C + m: r_0 .. r_7, x_0 .. x_7
 #pragma unroll
             for (int n = 0; n < NV; ++n) v[n] = 0.0f;
 #pragma unroll
             for (int j = 0; j < R / 4; ++j)
 #pragma unroll
-                for (int i = 0; i < 4; ++i) {
+                for (int i = 0; i < CH; ++i) {
                     const float4 a = *reinterpret_cast<const float4*>(k + i * DP + 4 * L * j);
                     const float4 e = *reinterpret_cast<const float4*>(q + i * DP + 4 * L * j);
 #pragma unroll
                     for (int m = 0; m < C; ++m) {
                         v[i * C + m] += S[m][4 * j] * a.x;
-                        v[(4 + i) * C + m] += S[m][4 * j] * e.x;
+                        v[(CH + i) * C + m] += S[m][4 * j] * e.x;
                         v[i * C + m] += S[m][4 * j + 1] * a.y;
-                        v[(4 + i) * C + m] += S[m][4 * j + 1] * e.y;
+                        v[(CH + i) * C + m] += S[m][4 * j + 1] * e.y;
                         v[i * C + m] += S[m][4 * j + 2] * a.z;
-                        v[(4 + i) * C + m] += S[m][4 * j + 2] * e.z;
+                        v[(CH + i) * C + m] += S[m][4 * j + 2] * e.z;
                         v[i * C + m] += S[m][4 * j + 3] * a.w;
-                        v[(4 + i) * C + m] += S[m][4 * j + 3] * e.w;
+                        v[(CH + i) * C + m] += S[m][4 * j + 3] * e.w;
                     }
                 }
             dr_sums<NV, L>(v, lane, l, sums);
             __syncwarp();
             const float* nu = bn + ch * DR_NUM;
-            const float4 a0 = *reinterpret_cast<const float4*>(nu), be = *reinterpret_cast<const float4*>(bb + ch * 4);
-            const float2 a1 = *reinterpret_cast<const float2*>(nu + 4);
-            const int left = nb - ch * DR_CHUNK;               // tokens of the chunk; the missing ones write nothing
-            float u[4][C];
+            const int left = nb - ch * CH;                     // tokens of the chunk; the missing ones write nothing
+            float u[CH][C];
 #pragma unroll
-            for (int m = 0; m < C; ++m) {
-                const float* vt = bv + ch * 4 * COLS + cb + m;
-                u[0][m] = be.x * (vt[0] - sums[m]);
-                u[1][m] = left > 1 ? be.y * (vt[COLS] - sums[C + m] - a0.x * u[0][m]) : 0.0f;
-                u[2][m] = left > 2 ? be.z * (vt[2 * COLS] - sums[2 * C + m] - a0.y * u[0][m] - a0.z * u[1][m]) : 0.0f;
-                u[3][m] = left > 3 ? be.w * (vt[3 * COLS] - sums[3 * C + m] - a0.w * u[0][m] - a1.x * u[1][m] - a1.y * u[2][m]) : 0.0f;
+            for (int i = 0; i < CH; ++i) {
+                const float be = bb[ch * CH + i];
+                const float4 a0 = *reinterpret_cast<const float4*>(nu + CH * i), a1 = *reinterpret_cast<const float4*>(nu + CH * i + 4);
+                const float a[CH] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
+                float vt[C], r[C];
+                dr_row<C>(vt, bv + (ch * CH + i) * COLS + cb);
+                dr_row<C>(r, sums + i * C);
+#pragma unroll
+                for (int m = 0; m < C; ++m) {
+                    float x = vt[m] - r[m];
+#pragma unroll
+                    for (int j = 0; j < i; ++j) x -= a[j] * u[j][m];
+                    u[i][m] = i < left ? be * x : 0.0f;
+                }
             }
 #pragma unroll
-            for (int n = l; n < 4 * C; n += L) {                // token n / C of column n % C
+            for (int n = l; n < CH * C; n += L) {               // token n / C of column n % C
                 const int i = n / C, m = n % C;
-                const float4 bi = *reinterpret_cast<const float4*>(nu + 8 + 4 * i);
-                float um[4];
+                const float4 b0 = *reinterpret_cast<const float4*>(nu + CH * CH + CH * i), b1 = *reinterpret_cast<const float4*>(nu + CH * CH + CH * i + 4);
+                const float bi[CH] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
+                float out = sums[(CH + i) * C + m];
 #pragma unroll
-                for (int t = 0; t < 4; ++t)
-                    um[t] = C == 1 ? u[t][0] : C == 2 ? ((m & 1) ? u[t][C - 1] : u[t][0])
-                                             : (m & 2) ? ((m & 1) ? u[t][C - 1] : u[t][C >= 4 ? 2 : 0]) : ((m & 1) ? u[t][C >= 2 ? 1 : 0] : u[t][0]);
-                const float out = sums[(4 + i) * C + m] + bi.x * um[0] + bi.y * um[1] + bi.z * um[2] + bi.w * um[3];
+                for (int t = 0; t < CH; ++t) {
+                    const float um = C == 1 ? u[t][0] : C == 2 ? ((m & 1) ? u[t][C - 1] : u[t][0])
+                                            : (m & 2) ? ((m & 1) ? u[t][C - 1] : u[t][C >= 4 ? 2 : 0]) : ((m & 1) ? u[t][C >= 2 ? 1 : 0] : u[t][0]);
+                    out += bi[t] * um;
+                }
                 if (i < left && m < cols_here)
-                    o[(static_cast<size_t>(row0 + done + ch * DR_CHUNK + i) * s.H + h) * s.V + c0 + cb + m] = out;
+                    o[(static_cast<size_t>(row0 + done + ch * CH + i) * s.H + h) * s.V + c0 + cb + m] = out;
             }
 #pragma unroll
             for (int j = 0; j < R / 4; ++j) {
                 const float4 p = *reinterpret_cast<const float4*>(bt + ch * DP + 4 * l + 4 * L * j);
-                const float4 w0 = *reinterpret_cast<const float4*>(w + 4 * L * j), w1 = *reinterpret_cast<const float4*>(w + DP + 4 * L * j),
-                             w2 = *reinterpret_cast<const float4*>(w + 2 * DP + 4 * L * j),
-                             w3 = *reinterpret_cast<const float4*>(w + 3 * DP + 4 * L * j);
 #pragma unroll
                 for (int m = 0; m < C; ++m) {
-                    S[m][4 * j] = p.x * S[m][4 * j] + w0.x * u[0][m] + w1.x * u[1][m] + w2.x * u[2][m] + w3.x * u[3][m];
-                    S[m][4 * j + 1] = p.y * S[m][4 * j + 1] + w0.y * u[0][m] + w1.y * u[1][m] + w2.y * u[2][m] + w3.y * u[3][m];
-                    S[m][4 * j + 2] = p.z * S[m][4 * j + 2] + w0.z * u[0][m] + w1.z * u[1][m] + w2.z * u[2][m] + w3.z * u[3][m];
-                    S[m][4 * j + 3] = p.w * S[m][4 * j + 3] + w0.w * u[0][m] + w1.w * u[1][m] + w2.w * u[2][m] + w3.w * u[3][m];
+                    S[m][4 * j] *= p.x;
+                    S[m][4 * j + 1] *= p.y;
+                    S[m][4 * j + 2] *= p.z;
+                    S[m][4 * j + 3] *= p.w;
+                }
+#pragma unroll
+                for (int t = 0; t < CH; ++t) {
+                    const float4 x = *reinterpret_cast<const float4*>(w + t * DP + 4 * L * j);
+#pragma unroll
+                    for (int m = 0; m < C; ++m) {
+                        S[m][4 * j] += x.x * u[t][m];
+                        S[m][4 * j + 1] += x.y * u[t][m];
+                        S[m][4 * j + 2] += x.z * u[t][m];
+                        S[m][4 * j + 3] += x.w * u[t][m];
+                    }
                 }
             }
             __syncwarp();                                       // `sums` is written again
@@ -817,7 +850,7 @@ static int delta_shape(DeltaShape& s, int H, int G, int D, int V, int taps, int 
 
 // Everything of a step that is not all single tokens.  Scratch (float32): qn, kn [T, G, DP], vn [T, H, VP], beta [T, H],
 // decay [T, H, DP] (whose places from D on must be finite), gate and o [T, H, V], pk and pq [T, H, DP], and for P =
-// T / 4 + entries + 1 chunks total [P, H, DP] and num [P, H, 24].
+// T / 8 + entries + 1 chunks total [P, H, DP] and num [P, H, 128].
 // `conv_w` [C, taps]: the rows of q, k and v one after another.
 extern "C" int llm_delta_scan(
     const float* proj, long long stride, int q_off, int b_off, int a_off, int ra, int g_off, int rg, const float* conv_w, int taps,
@@ -876,11 +909,11 @@ extern "C" int llm_delta_scan(
         default: CHUNKS_OF(256); break;
     }
 #undef CHUNKS_OF
-#define SCAN(DP, C, WARPS)                                                                                            \
+#define SCAN(DP, C, WARPS, L)                                                                                         \
     do {                                                                                                              \
-        auto kern = delta_scan_kernel<DP, C, WARPS>;                                                                  \
-        constexpr int K = DP >= 128 ? 1 : 128 / DP, COLS = WARPS * K * C, CH = DR_TB / DR_CHUNK;                      \
-        const size_t smem = (2 * (static_cast<size_t>(DR_TB) * (3 * DP + COLS + 1) + CH * (DP + DR_NUM)) + COLS * 8) * sizeof(float); \
+        auto kern = delta_scan_kernel<DP, C, WARPS, L>;                                                                  \
+        constexpr int K = 32 / L, COLS = WARPS * K * C, CH = DR_TB / DR_CHUNK;                      \
+        const size_t smem = (2 * (static_cast<size_t>(DR_TB) * (3 * DP + COLS + 1) + CH * (DP + DR_NUM)) + COLS * 2 * DR_CHUNK) * sizeof(float); \
         if (smem > 48 * 1024) {                                                                                       \
             const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,             \
                                                        static_cast<int>(smem));                                       \
@@ -889,21 +922,23 @@ extern "C" int llm_delta_scan(
         launch_pdl(kern, dim3(num_entries, H, (V + COLS - 1) / COLS), dim3(WARPS * 32), smem, st, s, proj, pq, pk, vn, \
                    beta, decay, total, num, o, state, positions, entry_slot, entry_q_start, entry_q_len);             \
     } while (0)
-    // few columns: fewer a warp, so that more schedulers have one; many: more a warp, which costs fewer instructions a column
+    // few columns: fewer a warp, so that more schedulers have one; many: more a warp, which costs fewer instructions a column.
+    // Measured at 128 rows (us; one, two, four columns on 32 lanes, four on 16): 512 columns (1,000 tokens) 106 111 133 177,
+    // 1,024: 141 112 134 181, 2,048: 213 159 136 182, 4,096 (1,500 tokens of 4 requests): 203 154 131 113.
     const long long columns = static_cast<long long>(num_entries) * H * V;
     const int plan = columns <= 640 ? 0 : columns <= 1300 ? 1 : columns <= 3000 ? 2 : 3;
     switch (s.DP) {
-        case 32: SCAN(32, 2, 2); break;
-        case 64: SCAN(64, 2, 4); break;
+        case 32: SCAN(32, 2, 2, 8); break;
+        case 64: SCAN(64, 2, 4, 16); break;
         case 128:
-            if (plan == 0) SCAN(128, 1, 4);
-            else if (plan == 1) SCAN(128, 2, 4);
-            else if (plan == 2) SCAN(128, 2, 8);
-            else SCAN(128, 4, 4);
+            if (plan == 0) SCAN(128, 1, 4, 32);
+            else if (plan == 1) SCAN(128, 2, 4, 32);
+            else if (plan == 2) SCAN(128, 4, 4, 32);
+            else SCAN(128, 4, 4, 16);
             break;
         default:
-            if (plan == 0) SCAN(256, 1, 4);
-            else SCAN(256, 2, 4);
+            if (plan == 0) SCAN(256, 1, 4, 32);
+            else SCAN(256, 2, 4, 32);
             break;
     }
 #undef SCAN

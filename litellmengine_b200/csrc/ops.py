@@ -1186,8 +1186,8 @@ def delta_rule(proj: torch.Tensor, offs, ranks, conv_w: torch.Tensor, w_decay: t
         _check(f(*args, _ptr(batch.entry_slot), _ptr(batch.entry_q_start), batch.num_entries, H, G, D, V, _stream()), "delta_step")
         return
     DP, VP = delta_padded(D), (V + 3) // 4 * 4
-    chunks = T // 4 + batch.num_entries + 1                 # places for what the four tokens of a chunk share
-    sizes = (T * H * DP,) + 2 * (T * G * DP,) + (T * H * VP, T * H, T * H * V, T * H * V) + 2 * (T * H * DP,) + (chunks * H * DP, chunks * H * 24)
+    chunks = T // 8 + batch.num_entries + 1                 # places for what the eight tokens of a chunk share
+    sizes = (T * H * DP,) + 2 * (T * G * DP,) + (T * H * VP, T * H, T * H * V, T * H * V) + 2 * (T * H * DP,) + (chunks * H * DP, chunks * H * 128)
     starts = [0]
     for n in sizes:
         starts.append(starts[-1] + (n + 3) // 4 * 4)
