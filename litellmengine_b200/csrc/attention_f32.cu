@@ -10,9 +10,9 @@
 //   prefill  portions of several tokens.  What bounds it: multiply-adds.  A block takes 64 query rows of one head, tiles of
 //            64 keys; a thread makes 4 x 4 scores and 4 rows x 8 output columns, 8 and 10.7 multiply-adds per shared
 //            16-byte load, where the general kernel made one dot product a lane and one value column a load.
-// Measured, 32 query heads over 8 of 128, against the general kernel: a prompt of 500 tokens 888 -> 129 us (167 with 8 rows a thread in blocks of 128 threads and the tile list outermost); 8 single tokens
-// at contexts of 1,125 to 1,500 190 -> 29 us (85 MB of keys and values: 2.9 TB/s; the exchanges, not the bytes, are what is
-// left).
+// Measured, 32 query heads over 8 of 128, against the general kernel: a prompt of 500 tokens 888 -> 129 us (167 with 8 rows a
+// thread in blocks of 128 threads and the list of tiles outermost in the grid); 8 single tokens at contexts of 1,125 to 1,500
+// 190 -> 29 us (85 MB of keys and values: 2.9 TB/s; the exchanges, not the bytes, are what is left).
 #include "common.cuh"
 #include <math_constants.h>
 

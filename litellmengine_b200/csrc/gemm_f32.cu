@@ -20,7 +20,7 @@
 // i.e. 0.9 to 1.0 of the measured copy bandwidth at a row, 0.65 to 0.86 at 8, where the token rows' loads from the
 // first-level cache (4 KB per 2 KB of weights) are what is left.  Its error against 64 bits is 1.1e-7 (relative, 2-norm)
 // at K = 4096 where the library's is 1.4e-7 to 1.1e-6.  From 17 rows on the arithmetic bounds it (N = 152000, 24 rows:
-// 277 against 243), and the library product stays.
+// 277 against the library's 243): large matrices go to the tensor cores (gemm_f32_tcgen05.cu), small ones to the library.
 #include "common.cuh"
 
 #define LF_ROWS 4

@@ -48,3 +48,34 @@ def test_portions_end_anywhere(H, D, V, lens):
         assert float(err) < 1e-4, (n, float(err))
         got = state[e, :H * V * DP].view(H, V, DP)[..., :D].transpose(1, 2).to(F64)
         assert float((got - S).abs().max()) < 2e-5 * max(1.0, float(S.abs().max())), n
+
+
+@pytest.mark.parametrize("T,H,D,V,ra,rg", [(1 + 2, 1, 128, 128, 64, 33), (63, 2, 64, 24, 33, 80), (64, 3, 32, 20, 48, 64), (65, 1, 128, 64, 130, 1),
+                                           (129, 5, 128, 33, 64, 64)])
+def test_low_rank_products_on_the_tensor_cores(T, H, D, V, ra, rg):
+    """bfloat16 weights (the split product) against the same weights as float32 (plain multiply-adds): edges of 64 tokens, 128
+    channels, 64 and 16 ranks, widths with and without sixteen-byte rows, a token with an infinity and one with a NaN."""
+    from litellmengine_b200.csrc import ops
+    g = torch.Generator(device=DEV).manual_seed(T)
+    taps, C = 2, 2 * H * D + H * V
+    rnd = lambda *s: torch.randn(*s, generator=g, device=DEV)
+    proj, conv = rnd(T, C + H + ra + rg), rnd(C, taps)
+    proj[-1, C + H] = float("inf")
+    proj[-2, C + H + ra] = float("nan")
+    wa, wg = (rnd(ra, H * D) * 0.2).bfloat16(), (rnd(rg, H * V) * 0.2).bfloat16()
+    dt, al, nw = rnd(H * D), rnd(H) * 0.5, torch.ones(V, device=DEV)
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)
+    b = types.SimpleNamespace(positions=i32(list(range(T))), token_entry=i32([0] * T), entry_slot=i32([0]), entry_q_start=i32([0]),
+                              entry_q_len=i32([T]), num_entries=1)
+    got = []
+    for kind in (torch.bfloat16, torch.float32):
+        state = torch.zeros(1, (H * V * ops.delta_padded(D) + taps * C + 3) // 4 * 4, device=DEV)
+        out = torch.zeros(T, H * V, device=DEV)
+        ops.delta_rule(proj, (0, C, C + H, C + H + ra), (ra, rg), conv, wa.to(kind), wg.to(kind), dt, al, nw, 1e-5, 1.0, out, 0, state, b,
+                       H, H, D, V, single=False)
+        got.append((out, state[:, :H * V * ops.delta_padded(D)].clone()))
+    (a, sa), (w, sw) = got
+    assert torch.equal(torch.isnan(a), torch.isnan(w)) and torch.isnan(w[-2]).all()
+    # rank products of 32-bit rounding a number, through a logistic function or a decay; the norm divides by the outputs' size
+    assert torch.allclose(a, w, rtol=2e-4, atol=2e-5, equal_nan=True)
+    assert torch.allclose(sa, sw, rtol=1e-4, atol=2e-5, equal_nan=True)
