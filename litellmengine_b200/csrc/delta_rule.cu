@@ -544,21 +544,32 @@ template <int C> __device__ __forceinline__ void dr_row(float (&v)[C], const flo
     }
 }
 
-// grid (entries, H, column tiles): WARPS warps a block, each 32 / L groups of C columns.
+// grid: entries (longest portion first) x H x column tiles, the tiles fastest: WARPS warps a block, each 32 / L groups of C columns.
 template <int DP, int C, int WARPS, int L>
 __global__ void __launch_bounds__(WARPS * 32) delta_scan_kernel(
     const DeltaShape s, const float* __restrict__ proj, const float* __restrict__ pq, const float* __restrict__ pk,
     const float* __restrict__ vn, const float* __restrict__ beta, const float* __restrict__ sk, const float* __restrict__ total,
     const float* __restrict__ num, float* __restrict__ o, float* __restrict__ state, const int32_t* __restrict__ positions,
-    const int32_t* __restrict__ entry_slot, const int32_t* __restrict__ entry_q_start, const int32_t* __restrict__ entry_q_len) {
+    const int32_t* __restrict__ entry_slot, const int32_t* __restrict__ entry_q_start, const int32_t* __restrict__ entry_q_len,
+    int num_entries, int tiles) {
     pdl_begin();
     constexpr int R = DP / L, THREADS = WARPS * 32, CH = DR_CHUNK, CHUNKS = DR_TB / CH;
     constexpr int COLS = WARPS * (32 / L) * C, NV = 2 * CH * C;
     // a buffer: q, k, s k, v of a batch of tokens, then beta; then p_7 and the numbers of its chunks
     constexpr int BUF = DR_TB * (3 * DP + COLS + 1) + CHUNKS * (DP + DR_NUM);
     extern __shared__ __align__(16) float smem[];
-    const int entry = blockIdx.x, h = blockIdx.y, tid = threadIdx.x, lane = tid & 31;
-    const int c0 = blockIdx.z * COLS;
+    const int tid = threadIdx.x, lane = tid & 31, tile = blockIdx.x % tiles, c0 = tile * COLS;
+    const int h = blockIdx.x / tiles % s.H;
+    int entry = blockIdx.x / (tiles * s.H);
+    if (num_entries <= 32) {                                    // longest portions first: the entry with `entry` ones before it
+        const int mine = lane < num_entries ? entry_q_len[lane] : -1;
+        int before = 0;
+        for (int e = 0; e < num_entries; ++e) {
+            const int len = __shfl_sync(0xffffffffu, mine, e);
+            before += len > mine || (len == mine && e < lane);
+        }
+        entry = __ffs(__ballot_sync(0xffffffffu, before == entry && lane < num_entries)) - 1;
+    }
     const int l = lane & (L - 1), group = tid / L, cb = group * C;          // the group's first column in the block
     float* sums = smem + 2 * BUF + group * NV;                  // [16][C]: the group's sums, by value and column
     const long long row0 = entry_q_start[entry];
@@ -730,7 +741,7 @@ __global__ void __launch_bounds__(WARPS * 32) delta_scan_kernel(
     // the convolutions' inputs of the portion's last tokens (the kernels before this one have read the ring)
     const int channels = 2 * s.G * s.D + s.H * s.V, keep = min(count, s.taps - 1), kvh = h / (s.H / s.G);
     float* ring = slot + s.ring_off;
-    const bool with_qk = blockIdx.z == 0 && h % (s.H / s.G) == 0;
+    const bool with_qk = tile == 0 && h % (s.H / s.G) == 0;
     for (int i = 0; i < keep; ++i) {
         const long long t = row0 + count - keep + i;
         float* dst = ring + static_cast<long long>(positions[t] % s.taps) * channels;
@@ -1036,18 +1047,28 @@ extern "C" int llm_delta_scan(
         default: CHUNKS_OF(256); break;
     }
 #undef CHUNKS_OF
+// A portion is as long as its blocks' walk, and a block beside another on its SM walks at half the pace (two fill the
+// multiply-add pipe).  So portions start longest first, and up to two blocks an SM of the device the blocks ask for more than
+// half of an SM's shared memory: each has an SM of its own, and the last ones begin where short portions have ended.  Measured
+// (us; portions of 284, 567 and 849 tokens, 192 blocks): as the hardware deals them 241, longest first 188, and alone 160;
+// eight of 55 to 445 tokens, 256 blocks: longest first 106, and alone 89; 512 blocks: side by side 179, alone 208.
+#define DR_ALONE_BLOCKS (2 * 148)
+#define DR_ALONE_SMEM (116 * 1024)
 #define SCAN(DP, C, WARPS, L)                                                                                         \
     do {                                                                                                              \
-        auto kern = delta_scan_kernel<DP, C, WARPS, L>;                                                                  \
-        constexpr int K = 32 / L, COLS = WARPS * K * C, CH = DR_TB / DR_CHUNK;                      \
-        const size_t smem = (2 * (static_cast<size_t>(DR_TB) * (3 * DP + COLS + 1) + CH * (DP + DR_NUM)) + COLS * 2 * DR_CHUNK) * sizeof(float); \
-        if (smem > 48 * 1024) {                                                                                       \
-            const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,             \
-                                                       static_cast<int>(smem));                                       \
-            if (e != cudaSuccess) return static_cast<int>(e);                                                         \
-        }                                                                                                             \
-        launch_pdl(kern, dim3(num_entries, H, (V + COLS - 1) / COLS), dim3(WARPS * 32), smem, st, s, proj, pq, pk, vn, \
-                   beta, decay, total, num, o, state, positions, entry_slot, entry_q_start, entry_q_len);             \
+        auto kern = delta_scan_kernel<DP, C, WARPS, L>;                                                               \
+        constexpr int COLS = WARPS * (32 / L) * C, CH = DR_TB / DR_CHUNK;                                             \
+        constexpr size_t need = (2 * (DR_TB * (3 * DP + COLS + 1) + CH * (DP + DR_NUM)) + COLS * 2 * DR_CHUNK) * sizeof(float); \
+        constexpr size_t most = need > DR_ALONE_SMEM ? need : DR_ALONE_SMEM;                                          \
+        const int tiles = (V + COLS - 1) / COLS;                                                                      \
+        const long long blocks = static_cast<long long>(num_entries) * H * tiles;                                     \
+        if (blocks > 0x7fffffffLL) return LLM_REFUSED_SIZE;                                                           \
+        const size_t smem = blocks <= DR_ALONE_BLOCKS ? most : need;                                                  \
+        /* the limit is the same for every launch: another thread may be between the two calls */                     \
+        const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(most)); \
+        if (e != cudaSuccess) return static_cast<int>(e);                                                             \
+        launch_pdl(kern, dim3(static_cast<unsigned>(blocks)), dim3(WARPS * 32), smem, st, s, proj, pq, pk, vn, beta, decay, \
+                   total, num, o, state, positions, entry_slot, entry_q_start, entry_q_len, num_entries, tiles);      \
     } while (0)
     // few columns: fewer a warp, so that more schedulers have one; many: more a warp, which costs fewer instructions a column.
     // Measured at 128 rows (us; one, two, four columns on 32 lanes, four on 16): 512 columns (1,000 tokens) 106 111 133 177,

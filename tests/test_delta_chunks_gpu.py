@@ -1,5 +1,5 @@
 """The delta rule's scan, eight tokens a chunk, against the token-by-token recurrence in 64 bits: portions that end anywhere in
-a chunk and in a batch of sixteen, alone and beside others, for every layout of columns that the sizes choose."""
+a chunk and in a batch of sixteen, alone and beside others, for every layout of columns that the sizes choose, up to 32 entries (walked longest first) and more."""
 import types
 
 import pytest
@@ -10,7 +10,7 @@ DEV = "cuda:0"
 F64 = torch.float64
 
 
-@pytest.mark.parametrize("H,D,V,lens", [(2, 128, 128, [2, 3, 7, 8, 9]), (4, 128, 128, [15, 16]), (8, 128, 128, [17, 33]), (16, 128, 128, [40, 24, 9]),
+@pytest.mark.parametrize("H,D,V,lens", [(2, 128, 128, [2, 3, 7, 8, 9]), (4, 128, 128, [15, 16]), (8, 128, 128, [17, 33]), (2, 128, 128, [1 + i % 19 for i in range(32)]), (1, 64, 16, [1 + i % 5 for i in range(40)]), (16, 128, 128, [40, 24, 9]),
                                         (3, 64, 20, [5, 23]), (2, 32, 33, [8, 31]), (2, 256, 64, [12, 18])])
 def test_portions_end_anywhere(H, D, V, lens):
     from litellmengine_b200.csrc import ops
