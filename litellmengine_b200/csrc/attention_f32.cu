@@ -15,6 +15,7 @@
 // 190 -> 29 us (85 MB of keys and values: 2.9 TB/s; the exchanges, not the bytes, are what is left).
 #include "common.cuh"
 #include <math_constants.h>
+#include <type_traits>
 
 #define FA_WARPS 8
 
@@ -260,7 +261,7 @@ __global__ void __launch_bounds__(FP_THREADS, 2) attention_f32_prefill_kernel(
     const int row_base = entry_q_start[e] + q0;
     const int32_t* table = block_table + static_cast<size_t>(entry_slot[e]) * table_stride;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, tx = tid & 15, ty = tid >> 4;
-    const int pos_first = past + q0, pos_last = pos_first + rows_here - 1;
+    const int pos_first = past + q0, pos_last = pos_first + rows_here - 1, lo_last = first_visible(pos_last, window);
     const size_t khead = static_cast<size_t>(page_size) * D, kpage = 2 * static_cast<size_t>(nkv) * khead;
     for (int i = tid; i < FP_ROWS * C4; i += FP_THREADS) {
         const int r = i / C4, c = i - r * C4;
@@ -346,7 +347,8 @@ __global__ void __launch_bounds__(FP_THREADS, 2) attention_f32_prefill_kernel(
 #pragma unroll
             for (int c = 0; c < 4; ++c) {
                 const float p = expf(s[r][c] - base);
-                ps[(ty * FP_RPT + r) * PLD + tx + 16 * c] = p;
+                const int j = kt + tx + 16 * c;
+                ps[(ty * FP_RPT + r) * PLD + tx + 16 * c] = (j > pos || j < lo) ? -1.0f : p;
                 sum += p;
             }
             l[r] = l[r] * alpha + sum;
@@ -356,26 +358,33 @@ __global__ void __launch_bounds__(FP_THREADS, 2) attention_f32_prefill_kernel(
         }
         asm volatile("cp.async.wait_group 0;\n" ::: "memory");
         __syncthreads();                                     // weights and values are in place
+        // Zero times a value that is not finite is NaN: where some row of the block does not see some key of the tile, each product
+        // is made only for the rows that see its key (weight -1: it does not).
+        auto values = [&](auto hidden) {
 #pragma unroll 1
-        for (int k = 0; k < FP_KEYS; k += 4) {
-            float4 p[FP_RPT];
+            for (int k = 0; k < FP_KEYS; k += 4) {
+                float4 p[FP_RPT];
 #pragma unroll
-            for (int r = 0; r < FP_RPT; ++r) p[r] = *reinterpret_cast<const float4*>(ps + (ty * FP_RPT + r) * PLD + k);
+                for (int r = 0; r < FP_RPT; ++r) p[r] = *reinterpret_cast<const float4*>(ps + (ty * FP_RPT + r) * PLD + k);
 #pragma unroll
-            for (int u = 0; u < 4; ++u)
+                for (int u = 0; u < 4; ++u)
 #pragma unroll
-                for (int c = 0; c < OC; ++c) {
-                    const float4 v = *reinterpret_cast<const float4*>(vs + (k + u) * D + c * 64 + tx * 4);
+                    for (int c = 0; c < OC; ++c) {
+                        const float4 v = *reinterpret_cast<const float4*>(vs + (k + u) * D + c * 64 + tx * 4);
 #pragma unroll
-                    for (int r = 0; r < FP_RPT; ++r) {
-                        const float w = u == 0 ? p[r].x : u == 1 ? p[r].y : u == 2 ? p[r].z : p[r].w;
-                        o[r][4 * c] = fmaf(w, v.x, o[r][4 * c]);
-                        o[r][4 * c + 1] = fmaf(w, v.y, o[r][4 * c + 1]);
-                        o[r][4 * c + 2] = fmaf(w, v.z, o[r][4 * c + 2]);
-                        o[r][4 * c + 3] = fmaf(w, v.w, o[r][4 * c + 3]);
+                        for (int r = 0; r < FP_RPT; ++r) {
+                            const float w = u == 0 ? p[r].x : u == 1 ? p[r].y : u == 2 ? p[r].z : p[r].w;
+                            if (decltype(hidden)::value && w < 0.0f) continue;
+                            o[r][4 * c] = fmaf(w, v.x, o[r][4 * c]);
+                            o[r][4 * c + 1] = fmaf(w, v.y, o[r][4 * c + 1]);
+                            o[r][4 * c + 2] = fmaf(w, v.z, o[r][4 * c + 2]);
+                            o[r][4 * c + 3] = fmaf(w, v.w, o[r][4 * c + 3]);
+                        }
                     }
-                }
-        }
+            }
+        };
+        if (kt + FP_KEYS - 1 > pos_first || kt < lo_last) values(std::true_type());
+        else values(std::false_type());
         __syncthreads();                                     // before the next tile overwrites them
     }
 #pragma unroll

@@ -142,3 +142,28 @@ def test_portions(nq, nkv, d, page, span):
             err = float((out[starts[e] + r].view(nq, d).double().cpu() - ref).abs().max())
             assert err <= tolerance(d, n, 6.0) * float(vs[e].abs().max()), (n, t, r, err)
     assert status.tolist() == [0, 0]
+
+
+@pytest.mark.parametrize("span", [None, 70, -100])
+def test_a_value_that_is_not_finite_reaches_only_who_sees_it(span):
+    """Infinities and NaN among the values of a portion: rows before them, or with their window behind them, stay finite."""
+    g = torch.Generator().manual_seed(5)
+    nq, nkv, d, page, n, t = 4, 2, 128, 16, 300, 250
+    cache, table, ks, vs = pages_of([n], nkv, d, page, g)
+    bad = {60: float("nan"), 200: float("inf"), 281: float("-inf")}
+    for j, x in bad.items():
+        cache[table[0, j // page].long(), 1, :, j % page] = x
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)
+    q = torch.randn(t, nq * d, generator=g).to(DEV)
+    out, status, R = torch.zeros_like(q), i32([0, 0]), ops().PREFILL_TILE_ROWS
+    tiles = [(0, r) for r in range(0, t, R)][::-1]
+    ops().attention_f32_prefill(q, out, cache, i32(tiles), len(tiles), i32([0]), i32([0]), i32([t]), i32([n]), table, nq, nkv, d, page, span,
+                                d ** -0.5, status)
+    for r in range(t):
+        pos = n - t + r
+        lo = max(0, pos - span + 1) if span and span > 0 else pos - pos % -span if span else 0
+        seen = any(lo <= j <= pos for j in bad)
+        assert bool(torch.isfinite(out[r]).all()) != seen, pos
+        if not seen:
+            ref = plain(q[r].view(nq, d).cpu(), ks[0], vs[0], pos, span, d ** -0.5)
+            assert float((out[r].view(nq, d).double().cpu() - ref).abs().max()) <= tolerance(d, n, 6.0) * float(vs[0].abs().max()), pos
