@@ -119,7 +119,8 @@ __global__ void __launch_bounds__(FA_WARPS * 32, 2) attention_f32_decode_kernel(
         for (int off = G << SHIFT; off < 32; off <<= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, off));
         const float m_new = fmaxf(m, top);
         const float alpha = (m == -CUDART_INF_F) ? 0.0f : expf(m - m_new);
-        const float p = seen ? expf(score - m_new) : 0.0f;
+        const float base = m_new == -CUDART_INF_F ? 0.0f : m_new;         // only scores of minus infinity so far: weights of zero
+        const float p = seen ? expf(score - base) : 0.0f;
         l = l * alpha + p;
         if (__any_sync(0xffffffffu, m_new != m)) {
 #pragma unroll

@@ -167,3 +167,27 @@ def test_a_value_that_is_not_finite_reaches_only_who_sees_it(span):
         if not seen:
             ref = plain(q[r].view(nq, d).cpu(), ks[0], vs[0], pos, span, d ** -0.5)
             assert float((out[r].view(nq, d).double().cpu() - ref).abs().max()) <= tolerance(d, n, 6.0) * float(vs[0].abs().max()), pos
+
+
+@pytest.mark.parametrize("splits", [1, 2])
+def test_single_tokens_with_scores_of_minus_infinity(splits):
+    """Keys whose product with the query overflows downwards weigh nothing, also where a warp meets nothing else at first."""
+    g = torch.Generator().manual_seed(6)
+    nq, nkv, d, page, n = 8, 2, 128, 16, 200
+    cache, table, ks, vs = pages_of([n], nkv, d, page, g)
+    far = [j for j in range(n) if j % 64 < 16 or j >= 184]
+    for j in far:
+        ks[0][j] = 0.0
+        ks[0][j, :, 0] = -1e30
+        cache[table[0, j // page].long(), 0, :, j % page] = ks[0][j].to(DEV)
+    q = torch.randn(1, nq * d, generator=g)
+    q.view(nq, d)[:, 0] = 1e10
+    for j in set(range(n)) - set(far):
+        ks[0][j, :, 0] = 0.0
+        cache[table[0, j // page].long(), 0, :, j % page] = ks[0][j].to(DEV)
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)
+    out, status = torch.zeros(1, nq * d, device=DEV), i32([0, 0])
+    ops().attention_f32_decode(q.to(DEV), out, cache, None, 1, i32([n - 1]), i32([0]), i32([0]), table, nq, nkv, d, page, None, d ** -0.5,
+                               splits, status)
+    ref = plain(q[0].view(nq, d), ks[0], vs[0], n - 1, None, d ** -0.5)
+    assert float((out.view(nq, d).double().cpu() - ref).abs().max()) <= tolerance(d, n, 6.0) * float(vs[0].abs().max())
