@@ -1,16 +1,19 @@
 // y[M, N] = x[M, K] . W[N, K]^T for float32 operands and more rows than a decode step, on the 5th-generation tensor cores.
 //
-// A float32 value is exactly the sum of three bfloat16 values, h + m + l, each the next eight bits of its significand
-// (truncated, so that nothing overflows and each remainder is exact).  A product is then hh + (hm + mh) + (mm + hl + lh) plus
-// three terms below 2^-23 of it, which are left out; six bfloat16 products with float32 accumulation take the place of one
-// float32 product, at 6 / 31 of the tensor cores' time against the multiply-add units' (4,096 against 128 products a clock and SM).
+// A float32 value is the sum of three bfloat16 values, h + m + l: h and m are what is left, rounded to nearest, so every
+// remainder is exact and signed, |m| <= 2^-8 and |l| <= 2^-17 of the value, and l takes the rest exactly (down to bfloat16's
+// smallest numbers: values below 2^-110 lose their last bits).  A product is then hh + (hm + mh) + (mm + hl + lh) plus ml + lm
+// + ll, which are left out: at most 2^-24 of the product, what rounding it once may cost, and of either sign (pieces that are
+// cut instead of rounded all have the value's sign, and what they leave out reaches 2^-21, always towards zero).  Six bfloat16
+// products with float32 accumulation take the place of one float32 product, at 6 / 31 of the tensor cores' time against the
+// multiply-add units' (4,096 against 128 products a clock and SM).
 //
 // What makes the sums as good as float32's: the tensor cores cut, rather than round, what they add to an accumulator, and
 // 256 steps in a row along K = 4096 would show that.  So an accumulator lives for 64 k-values only, smallest terms first,
 // and is then added, rounded, to sums kept in registers by the warps that drain it.  Error against 64 bits (relative, 2-norm,
 // K = 4096): 1.5e-7 to 1.9e-7; the library's float32 product 1.1e-6.
-// A result that is not finite is computed again with plain multiply-adds (a split infinity times zero is NaN), so infinities
-// and NaN come out as a float32 product has them.
+// A result that is not finite is computed again with plain multiply-adds (a split infinity times zero is NaN, and a value
+// above bfloat16's largest rounds to infinity), so infinities and NaN come out as a float32 product has them.
 //
 // A CTA makes 128 weight rows x NT tokens (the MMA's M side is the weights, so that 17 tokens cost a tile of 32).  Roles: warp
 // 0 feeds the copy engine: 128 x 64 weights as float32, and NT x 64 of the three planes of x, which a small kernel has
@@ -55,18 +58,22 @@ __device__ __forceinline__ bool lt_wait_warp(unsigned long long* bar, unsigned p
     return __all_sync(0xffffffffu, lt_wait(bar, parity, abort_flag, status));
 }
 
-// The high halves of two floats as a pair of bfloat16 (a in the lower half).
-__device__ __forceinline__ unsigned lt_tops(float a, float b) { return __byte_perm(__float_as_uint(a), __float_as_uint(b), 0x7632); }
-__device__ __forceinline__ float lt_rest(float a) { return a - __uint_as_float(__float_as_uint(a) & 0xffff0000u); }
+// Two floats as a pair of bfloat16 (a in the lower half), rounded to nearest; a and b become what is left of them.
+__device__ __forceinline__ unsigned lt_piece(float& a, float& b) {
+    unsigned r;
+    asm("cvt.rn.bf16x2.f32 %0, %1, %2;\n" : "=r"(r) : "f"(b), "f"(a));
+    a -= __uint_as_float(r << 16);
+    b -= __uint_as_float(r & 0xffff0000u);
+    return r;
+}
 // Eight floats as three planes of eight bfloat16.
 __device__ __forceinline__ void lt_split8(const float4 a, const float4 b, unsigned* h, unsigned* m, unsigned* l) {
-    const float v[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+    float v[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-        const float r0 = lt_rest(v[2 * i]), r1 = lt_rest(v[2 * i + 1]);
-        h[i] = lt_tops(v[2 * i], v[2 * i + 1]);
-        m[i] = lt_tops(r0, r1);
-        l[i] = lt_tops(lt_rest(r0), lt_rest(r1));
+        h[i] = lt_piece(v[2 * i], v[2 * i + 1]);
+        m[i] = lt_piece(v[2 * i], v[2 * i + 1]);
+        l[i] = lt_piece(v[2 * i], v[2 * i + 1]);
     }
 }
 

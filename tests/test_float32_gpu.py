@@ -43,8 +43,8 @@ def test_tensor_core_product(M, N, K):
     w[0, :8] *= 1e-18
     ref = x.double() @ w.double().T
     got = ops().linear_f32_tcgen05(x, w)
-    # three terms of 2^-23 of a product are left out, a block's 24 additions are cut at the last place, the blocks' sums rounded
-    bound = (3 * 2 * U + 24 * 2 * U + -(-K // 64) * U) * (x.double().abs() @ w.double().abs().T)
+    # what is left out of a product is at most 2^-24 of it, a block's 24 additions are cut at the last place, the blocks' sums rounded
+    bound = (1.01 * U + 24 * 2 * U + -(-K // 64) * U) * (x.double().abs() @ w.double().abs().T)
     assert bool(((got.double() - ref).abs() <= bound).all())
     assert float((got - ref).norm() / ref.norm()) < 4e-7
     assert ops().stream_status(DEV).tolist() == [0, 0]
@@ -55,6 +55,32 @@ def test_tensor_core_product(M, N, K):
         assert torch.equal(torch.isnan(got), torch.isnan(lib)) and torch.equal(torch.isinf(got), torch.isinf(lib))
         assert torch.equal(got[torch.isinf(got)], lib[torch.isinf(lib)])
         assert ops().stream_status(DEV).tolist() == [0, 0]
+
+
+@pytest.mark.parametrize("M,N,K", [(17, 512, 64), (32, 130, 4096), (33, 257, 1024), (64, 300, 12288), (65, 512, 4096), (128, 512, 12288),
+                                   (300, 9472, 512), (500, 1024, 4096)])
+@pytest.mark.parametrize("kind", ["signed", "same", "cut"])
+def test_tensor_core_product_is_as_near_as_float32_sums(M, N, K, kind):
+    """Every row against 64 bits, for values of either sign, of one sign, and for values whose pieces, if they were cut instead of
+    rounded, would leave out 2^-21 of every product.  A block's last additions are cut at the place of their sum, its smaller
+    terms matter little, and the blocks' sums are rounded: 1 to 3 units of 2^-24 together.  A product without the third pieces is 2^-17 off."""
+    g = torch.Generator(device=DEV).manual_seed(M * 1000 + K)
+    x, w = torch.randn(M, K, generator=g, device=DEV), torch.randn(N, K, generator=g, device=DEV)
+    if kind == "same":
+        x, w = x.abs(), w.abs()
+    elif kind == "cut":
+        x, w = torch.full_like(x, 1 + 2.0 ** -7 - 2.0 ** -23), torch.full_like(w, 1 + 2.0 ** -7 - 2.0 ** -23)
+    ref = x.double() @ w.double().T
+    error = lambda got: float(((got - ref).norm(dim=1) / ref.norm(dim=1)).max())
+    assert error(ops().linear_f32_tcgen05(x, w)) < 5 * U
+    # the largest numbers round to an infinity of bfloat16: those sums are made again, without the split
+    x[1, 0], w[:, 0] = 3.4028234e38, 2.0 ** -120
+    ref = x.double() @ w.double().T
+    got = ops().linear_f32_tcgen05(x, w)
+    assert float(((got[1] - ref[1]).abs() / ref[1].abs()).max()) < K * U and bool(torch.isfinite(got).all())
+    others = [m for m in range(M) if m != 1]
+    assert float(((got - ref)[others].norm(dim=1) / ref[others].norm(dim=1)).max()) < 5 * U
+    assert ops().stream_status(DEV).tolist() == [0, 0]
 
 
 def test_the_product_of_each_size_takes_its_path():
