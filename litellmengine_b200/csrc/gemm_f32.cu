@@ -65,9 +65,9 @@ __global__ void __launch_bounds__(LF_WARPS * 32, MT <= 4 ? 3 : 2) linear_f32_str
     };
     int c = slice * 32 + lane;
     float4 b0[LF_ROWS], b1[LF_ROWS];
-    fetch(b0, c);                                       // weights are nobody's output: they may be read before the wait
+    pdl_wait();                                         // before the weights too: the kernel in front may have made them
+    fetch(b0, c);
     fetch(b1, c + STEP);
-    pdl_wait();
     auto multiply = [&](const float4 (&b)[LF_ROWS], int at) {
         const float* xp = x + 4 * at;
 #pragma unroll

@@ -151,8 +151,8 @@ __global__ void __launch_bounds__(LT_THREADS, 1) linear_f32_tcgen05_kernel(
                 ++nw;
                 return true;
             };
-            while (ok && nw < min(WB, boxes)) ok = fetch_w();     // weights: before the wait for the kernel in front
-            pdl_wait();
+            pdl_wait();                                           // before the weights too: the kernel in front may have made them
+            while (ok && nw < min(WB, boxes)) ok = fetch_w();
             auto fetch_x = [&]() {                                // the next block
                 const int st = nx % XS;
                 if (nx >= XS && !lt_wait(&x_empty[st], ((nx / XS) - 1) & 1, &abort_flag, status)) return false;

@@ -31,10 +31,10 @@
 
 // TOKENS a block takes: four in prompt portions, whose router's matrix is then read once for all of them; one in steps of few
 // tokens, where a block's latency is all there is: a warp an expert (up to sixteen warps), the first 1,024 columns of its
-// row fetched before the wait for the kernel in front.  The choice is a warp's: every lane looks at its experts, the
+// row fetched beside the token's.  The choice is a warp's: every lane looks at its experts, the
 // largest wins by exchanges (one thread walking all experts `top` times took a third of the kernel).  24 tokens of width
 // 2,048, eight experts and a shared gate: 16.6 -> 7.3 us.
-#define MOE_ROUTE_AHEAD 8         // loads of a lane before the wait
+#define MOE_ROUTE_AHEAD 8         // loads of a lane before the block waits for the token's row
 
 template <typename TX, int MOE_ROUTE_TOKENS>
 __global__ void __launch_bounds__(512) moe_route_kernel(const TX* __restrict__ x, const float* __restrict__ wr, float* __restrict__ dense,
@@ -43,7 +43,7 @@ __global__ void __launch_bounds__(512) moe_route_kernel(const TX* __restrict__ x
                                  const float* __restrict__ correction, int identity, float* __restrict__ idw,
                                  const float* __restrict__ bias, const float* __restrict__ shared_w, float* __restrict__ share,
                                  int normalize) {
-    pdl_invite();
+    pdl_begin();
     extern __shared__ float smem[];
     const int G = groups > 0 ? groups : 1;
     float* xs = smem;                                   // [TOKENS][W]
@@ -55,13 +55,12 @@ __global__ void __launch_bounds__(512) moe_route_kernel(const TX* __restrict__ x
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, warps = blockDim.x >> 5;
     const int rows = E + (shared_w ? 1 : 0);
     auto row_of = [&](int e) { return e < E ? wr + static_cast<size_t>(e) * W : shared_w; };
-    float4 ahead[MOE_ROUTE_AHEAD];                      // weights are nobody's output: they may be read before the wait
+    float4 ahead[MOE_ROUTE_AHEAD];                      // beside the loads of the token's row
     if (MOE_ROUTE_TOKENS == 1 && vec && warp < rows) {
 #pragma unroll
         for (int u = 0; u < MOE_ROUTE_AHEAD; ++u)
             if (lane * 4 + 128 * u < W) ahead[u] = *reinterpret_cast<const float4*>(row_of(warp) + lane * 4 + 128 * u);
     }
-    pdl_wait();
     if (vec) {                                          // sixteen-byte loads of the tokens' rows
         for (int i = tid * 8; i < nt * W; i += blockDim.x * 8) {
             float v[8];
