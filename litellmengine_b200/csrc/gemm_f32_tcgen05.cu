@@ -276,7 +276,12 @@ __global__ void __launch_bounds__(LT_THREADS, 1) linear_f32_tcgen05_kernel(
                 float v = acc[i];
                 if (!(fabsf(v) <= 3.402823466e38f)) {             // infinite or NaN: what plain multiply-adds make of it
                     v = 0.0f;
-                    for (int k = k_from; k < k_to; ++k) v = fmaf(x[static_cast<size_t>(m) * K + k], w[static_cast<size_t>(n) * K + k], v);
+                    const float *xr = x + static_cast<size_t>(m) * K, *wr = w + static_cast<size_t>(n) * K;
+#pragma unroll 1
+                    for (int k = k_from; k < k_to && v == v; k += 4) {      // a sum that is NaN stays it
+                        const float4 a = *reinterpret_cast<const float4*>(xr + k), b = *reinterpret_cast<const float4*>(wr + k);
+                        v = fmaf(a.w, b.w, fmaf(a.z, b.z, fmaf(a.y, b.y, fmaf(a.x, b.x, v))));
+                    }
                 }
                 out[static_cast<size_t>(m) * N + n] = v;
             }
