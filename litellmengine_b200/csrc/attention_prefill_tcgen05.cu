@@ -629,7 +629,7 @@ __global__ void __launch_bounds__(T5O_THREADS, 1) paged_prefill_attention_tcgen0
             // move the reference up only when the maximum has run away from it (both threads of a row
             // see the same numbers and decide alike)
             const bool adopt = (m == -CUDART_INF_F) && (mx > m);  // nothing accumulated under the old reference
-            const bool jump = (m != -CUDART_INF_F) && (mx > m + T5O_JUMP);
+            const bool jump = (m != -CUDART_INF_F) && (mx > m + (EXT ? 0.0f : T5O_JUMP));
             if (__any_sync(0xffffffffu, jump)) {
                 // O still receives the previous tile's product: wait for it, then scale this thread's half of its row
                 if (!t5_wait(&pv_done[g], (j - 1) & 1, &abort_flag, status, row_base)) { ok = false; continue; }
@@ -655,7 +655,10 @@ __global__ void __launch_bounds__(T5O_THREADS, 1) paged_prefill_attention_tcgen0
             }
             if (adopt || jump) m = mx;
             const float msub = (m == -CUDART_INF_F) ? 0.0f : m;
-            // the weights, rounded to bfloat16: 32 columns of P over the first half of this thread's 64 of S
+            // the weights, rounded to bfloat16: 32 columns of P over the first half of this thread's 64 of S; EXT sums them as rounded
+            auto sum_of = [](float p0, float p1, unsigned packed) {
+                return EXT ? __uint_as_float(packed << 16) + __uint_as_float(packed & 0xffff0000u) : p0 + p1;
+            };
             auto weights = [&](const unsigned (&r)[32], int c) {
                 unsigned pk[16];
                 if (full_tile) {
@@ -664,8 +667,8 @@ __global__ void __launch_bounds__(T5O_THREADS, 1) paged_prefill_attention_tcgen0
                         const float x0 = fmaf(__uint_as_float(r[i]), eff, -msub);
                         const float x1 = fmaf(__uint_as_float(r[i + 1]), eff, -msub);
                         const float p0 = t5_ex2(x0), p1 = t5_ex2(x1);     // (a cubic on the FMA pipe for a share of them: measured slower)
-                        l += p0 + p1;
                         pk[i >> 1] = t5_pack(p0, p1);
+                        l += sum_of(p0, p1, pk[i >> 1]);
                     }
                 } else {
 #pragma unroll
@@ -673,8 +676,8 @@ __global__ void __launch_bounds__(T5O_THREADS, 1) paged_prefill_attention_tcgen0
                         const int key = kt + c + i;
                         const float p0 = seen(key) ? t5_ex2(fmaf(__uint_as_float(r[i]), eff, -msub)) : 0.0f;
                         const float p1 = seen(key + 1) ? t5_ex2(fmaf(__uint_as_float(r[i + 1]), eff, -msub)) : 0.0f;
-                        l += p0 + p1;
                         pk[i >> 1] = t5_pack(p0, p1);
+                        l += sum_of(p0, p1, pk[i >> 1]);
                     }
                 }
                 t5_st16(my_s + (c >> 1), pk);
