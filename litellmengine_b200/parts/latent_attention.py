@@ -21,7 +21,8 @@ class LatentWork(StepPrelude):
     position some query of it sees, first gathered row, rows padded to whole key tiles) and tiles of 256 query rows of them,
     longest walk first; the rows of the others, which bring one.  Filled only for steps of at least `FROM` tokens."""
     # Shorter steps are replayed as captured graphs that serve any division of their tokens among requests, and what is
-    # allocated here depends on how many rows the requests have cached.  (At 1,024 tokens of one request the cached-row
+    # allocated here depends on how many rows the requests have cached (a step that is being captured never takes the lists).
+    # (At 1,024 tokens of one request the cached-row
     # kernel takes 340 us, the expanded path about 90.)
     FROM = 1025
 
@@ -245,7 +246,7 @@ class LatentAttentionMixer:
                                 self.eps, self.inv_freq, ctx.cache_keys if s.has_kv else None, b, ctx.block_table,
                                 ctx.page_size, ctx.status, self.dtype, rot_pairs=self.rot_pairs, rot_mag=self.rot_mag)
         q = ops.as_tensor(ops.linear(cq, self.w_uq, out_dtype=torch.float32))
-        work = b.preludes.get(self._work_name) if self._expand is not None else None
+        work = b.preludes.get(self._work_name) if self._expand is not None and not getattr(b, "any_division", False) else None
         if work is not None and work.num_tiles and 2 * work.gathered * H * (D + V) <= self.EXPANDED_BYTES:
             heads = self._expanded(q, proj, work, ctx)
         else:

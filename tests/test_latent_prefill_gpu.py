@@ -117,3 +117,37 @@ def test_long_step_of_every_kind_of_entry(window):
     limit, mixer.EXPANDED_BYTES = mixer.EXPANDED_BYTES, 1000          # more rows than may be expanded at once: the other path
     assert torch.equal(mixer.forward(xs, ctx), ref)
     mixer.EXPANDED_BYTES = limit
+
+
+def long_step(window=None, seed=3):
+    """A mixer, a step of 1,100 tokens (a prompt, short and long portions, a single token) and its inputs."""
+    from litellmengine_b200.config import config_from_dict
+    from litellmengine_b200.engine import ModelRunner, StepEntry
+    m = {"heads": 3, "dim": 128, "rot_dim": 64, "vdim": 128, "q_rank": 96, "kv_rank": 128, "scale": 192 ** -0.5,
+         "rot": {"base": 10000.0, "dims": 64}}
+    cfg = {"architecture": "Vugedra", "vocab": 64, "width": 256, "norm": {"eps": 1e-5},
+           "layers": [{"type": "latent_attention", "mixer": m, "mlp": None}]}
+    runner = ModelRunner.from_config(config_from_dict(cfg), seed=seed, device=DEV, max_total_tokens=4096, max_requests=8, max_tokens_per_step=2048)
+    mixer, g = runner.model.blocks[0].mixer, torch.Generator(device=DEV).manual_seed(1)
+    x = lambda n: torch.randn(n, 256, generator=g, device=DEV).to(torch.bfloat16)
+    past, new = [0, 130, 500, 77], [800, 1, 296, 3]
+    slots = [runner.admit() for _ in past]
+    for s, p in zip(slots, past):
+        if p:
+            b = runner.prepare([StepEntry(s, [0] * p)])
+            mixer.forward(x(p), runner.model.stage_context(0, b, runner.cache))
+            runner.finish(b)
+    b = runner.prepare([StepEntry(s, [0] * n) for s, n in zip(slots, new)])
+    ctx, xs = runner.model.stage_context(0, b, runner.cache), x(sum(new))
+    held, mixer._expand = mixer._expand, None
+    rows = mixer.forward(xs, ctx)                              # the path over the cached rows
+    mixer._expand = held
+    return runner, mixer, ctx, xs, rows
+
+
+def test_a_step_that_is_being_captured_keeps_to_the_cached_rows():
+    """A graph that serves any division of its tokens must not hold one step's segments, however many tokens it has."""
+    _, mixer, ctx, xs, rows = long_step()
+    assert not torch.equal(mixer.forward(xs, ctx), rows)       # by itself the step is expanded
+    ctx.batch.any_division = True
+    assert torch.equal(mixer.forward(xs, ctx), rows)
