@@ -387,8 +387,6 @@ __global__ void latent_q_pack_kernel(const float* __restrict__ q, bf16* __restri
 extern "C" int llm_latent_prefill_supported(int D, int V, int R, int P) {
     return D == 128 && V == LP_DV && P == 64 && R > 0 && R % 8 == 0;
 }
-extern "C" int llm_latent_prefill_tile_rows() { return 2 * LP_BM; }
-extern "C" int llm_latent_prefill_tile_keys() { return LP_BN; }
 
 // rows_cache: bfloat16 [pages, 1, page, DK] with `page_stride`; out: bfloat16 [total rows, DK]; segs as above, every first
 // gathered row and row count a multiple of the key tile; most_rows: the largest count.
@@ -416,15 +414,16 @@ extern "C" int llm_latent_q_pack(const float* q, void* out, const int32_t* posit
 }
 
 // q: bfloat16 [num_tokens, H * 192]; kv: bfloat16 [rows, H * 256] = per head [k | v]; gathered: bfloat16 [rows, R + 64];
-// out: bfloat16 [num_tokens, H * 128]; gate: null, or float32, token t's and head h's at t * gate_stride + h, the result is
+// out: bfloat16 [num_tokens, H * 128]; tile_rows, tile_keys: what the caller cut its tiles to and padded its segments to,
+// which have to be this kernel's; gate: null, or float32, token t's and head h's at t * gate_stride + h, the result is
 // multiplied by its sigmoid.
 extern "C" int llm_latent_prefill(const void* q, const void* kv, const void* gathered, void* out, int num_tokens, int rows,
-                                  const int32_t* tiles, int n_tiles, const int32_t* segs, const int32_t* entry_q_start,
-                                  const int32_t* entry_q_len, const int32_t* entry_kv_len, int H, int R, int window, float scale,
-                                  const float* gate, long long gate_stride, int32_t* status, uintptr_t stream) {
+                                  const int32_t* tiles, int n_tiles, int tile_rows, int tile_keys, const int32_t* segs,
+                                  const int32_t* entry_q_start, const int32_t* entry_q_len, const int32_t* entry_kv_len, int H, int R,
+                                  int window, float scale, const float* gate, long long gate_stride, int32_t* status, uintptr_t stream) {
     if (n_tiles <= 0) return LLM_OK;
-    if (H <= 0 || n_tiles > 65535 || !llm_latent_prefill_supported(128, LP_DV, R, 64) || rows <= 0 || rows % LP_BN || !(scale > 0.0f) ||
-        window < 0)
+    if (H <= 0 || n_tiles > 65535 || tile_rows != 2 * LP_BM || tile_keys != LP_BN || !llm_latent_prefill_supported(128, LP_DV, R, 64) ||
+        rows <= 0 || rows % LP_BN || !(scale > 0.0f) || window < 0)
         return LLM_REFUSED_SIZE;
     if (!aligned16(q) || !aligned16(kv) || !aligned16(gathered) || !aligned16(out)) return LLM_REFUSED_ALIGN;
     CUtensorMap q_map, kv_map, r_map;

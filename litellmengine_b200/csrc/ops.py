@@ -944,10 +944,10 @@ def latent_prefill(q: torch.Tensor, kv: torch.Tensor, gathered: torch.Tensor, ou
                              or not gate.is_cuda or gate_off < 0 or gate_off + H > gate.shape[1]):
         raise KernelError("the gate must be float32 [T, m] with unit stride along its rows and hold the heads' columns")
     f = _fn("latent_prefill_tcgen05", "llm_latent_prefill",
-            [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_int,
-             c_int, c_int, c_float, c_void_p, c_longlong, c_void_p, c_void_p])
-    _check(f(_ptr(q), _ptr(kv), _ptr(gathered), _ptr(out), T, rows, _ptr(tiles), n_tiles, _ptr(segs), _ptr(entry_q_start),
-             _ptr(entry_q_len), _ptr(entry_kv_len), H, R, int(window) if window else 0, float(scale),
+            [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_void_p, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p,
+             c_void_p, c_int, c_int, c_int, c_float, c_void_p, c_longlong, c_void_p, c_void_p])
+    _check(f(_ptr(q), _ptr(kv), _ptr(gathered), _ptr(out), T, rows, _ptr(tiles), n_tiles, LATENT_TILE_ROWS, LATENT_TILE_KEYS,
+             _ptr(segs), _ptr(entry_q_start), _ptr(entry_q_len), _ptr(entry_kv_len), H, R, int(window) if window else 0, float(scale),
              gate.data_ptr() + 4 * gate_off if gate is not None else None, gate.stride(0) if gate is not None else 0, _ptr(status),
              _stream()), "latent_prefill")
     return out

@@ -151,3 +151,12 @@ def test_a_step_that_is_being_captured_keeps_to_the_cached_rows():
     assert not torch.equal(mixer.forward(xs, ctx), rows)       # by itself the step is expanded
     ctx.batch.any_division = True
     assert torch.equal(mixer.forward(xs, ctx), rows)
+
+
+def test_tile_sizes_are_the_kernels(monkeypatch):
+    _, mixer, ctx, xs, _ = long_step()
+    for name, other in (("LATENT_TILE_ROWS", 128), ("LATENT_TILE_KEYS", 48)):      # the lists were made with the right ones
+        with monkeypatch.context() as m:
+            m.setattr(ops(), name, other)
+            with pytest.raises(ops().KernelError):
+                mixer.forward(xs, ctx)
