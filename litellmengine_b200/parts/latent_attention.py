@@ -17,54 +17,70 @@ from .registry import lookup, register_mixer
 
 
 class LatentWork(StepPrelude):
-    """How a long prompt step of latent attention is cut: the requests that bring several tokens as segments (entry, first
-    position some query of it sees, first gathered row, rows padded to whole key tiles) and tiles of 256 query rows of them,
-    longest walk first; the rows of the others, which bring one.  Filled only for steps of at least `FROM` tokens."""
+    """How a long prompt step of latent attention is cut: the portions that are worth it as segments (entry, first position
+    some query of it sees, first gathered row, rows padded to whole key tiles) and tiles of 256 query rows of them, longest
+    walk first; the rows of all other entries.  Filled only for steps of at least `FROM` tokens."""
     # Shorter steps are replayed as captured graphs that serve any division of their tokens among requests, and what is
     # allocated here depends on how many rows the requests have cached (a step that is being captured never takes the lists).
-    # (At 1,024 tokens of one request the cached-row
-    # kernel takes 340 us, the expanded path about 90.)
+    # (At 1,024 tokens of one request the cached-row kernel takes 340 us, the expanded path about 90.)
     FROM = 1025
+    # Queries a portion needs: mapping a row costs the same for two queries as for two thousand.  Four portions beside a prompt
+    # of 1,100 tokens, the layer at 32 heads (us, expanded and on the cached rows): 4,000 cached rows each, 8 queries 377, 275; 16:
+    # 379, 390; 32: 387, 542; 128: 393, 1,595; 500 rows, 16 queries: 191, 226; 8 heads, 4,000 rows, 8 queries 206, 187; 16: 207, 300.
+    LEAST = 16
+    # With fewer, a portion is expanded only where that leaves no token to the other path, whose launches cost about 50 us, and
+    # these have few rows together (of portions as above, 8 queries each: no cached rows 152, 195; 500 each 185, 210).
+    FEW_ROWS = 3072
 
     @dataclass
     class Views:
         tiles: torch.Tensor              # int32 [n, 2]
         segs: torch.Tensor               # int32 [n, 4]
-        rows: torch.Tensor               # int32 [n] rows of the batch that are single tokens
+        rows: torch.Tensor               # int32 [n] rows of the batch that belong to no segment
         num_tiles: int
         num_segs: int
-        num_single: int
+        num_rest: int
         gathered: int                    # rows of all segments
         longest: int                     # and of the longest
 
-    def __init__(self, window: Optional[int]):
-        self.window = window
-        self.name = f"latent_work:{window or 0}"
+    def __init__(self, window: Optional[int], most_rows: int):
+        """`most_rows`: gathered rows of a step that may be expanded at once."""
+        self.window, self.most_rows = window, most_rows
+        self.name = f"latent_work:{window or 0}:{most_rows}"
 
     def sections(self, max_tokens: int, max_entries: int):
-        return {"tiles": 2 * (max_tokens // ops.LATENT_TILE_ROWS + max_entries + 1), "segs": 4 * max_entries, "rows": max_entries}
+        return {"tiles": 2 * (max_tokens // ops.LATENT_TILE_ROWS + max_entries + 1), "segs": 4 * max_entries, "rows": max_tokens}
 
     def fill(self, facts, out):
         if facts.num_tokens < self.FROM:
             return 0, 0, 0, 0, 0
-        several = np.nonzero(facts.q_len > 1)[0]
-        single = facts.q_start[facts.q_len == 1]
-        out["rows"][:len(single)] = single
-        past, n = facts.past[several], facts.q_len[several]
-        first = np.maximum(past - self.window + 1, 0) if self.window else np.zeros_like(past)
         K, R = ops.LATENT_TILE_KEYS, ops.LATENT_TILE_ROWS
-        rows = -(-(past + n - first) // K) * K
+        first = np.maximum(facts.past - self.window + 1, 0) if self.window else np.zeros_like(facts.past)
+        rows = -(-(facts.past + facts.q_len - first) // K) * K
+        chosen = facts.q_len >= self.LEAST
+        if not chosen.all() and (facts.q_len > 1).all() and rows[~chosen].sum() <= self.FEW_ROWS:
+            chosen[:] = True
+        # those with the fewest rows a query first, while there is room: one request with a long past leaves the others alone
+        long = np.nonzero(chosen)[0]
+        long = long[np.argsort(rows[long] / facts.q_len[long], kind="stable")]
+        long = np.sort(long[np.cumsum(rows[long]) <= self.most_rows])
+        rest = np.ones(len(facts.q_len), dtype=bool)
+        rest[long] = False
+        token_rest = np.repeat(rest, facts.q_len)
+        num_rest = int(token_rest.sum())
+        out["rows"][:num_rest] = np.nonzero(token_rest)[0]
+        past, n, first, rows = facts.past[long], facts.q_len[long], first[long], rows[long]
         start = np.cumsum(rows) - rows
-        out["segs"][:4 * len(several)] = np.stack([several, first, start, rows], axis=1).reshape(-1)
-        tiles = [(i, q0) for i in range(len(several)) for q0 in range(0, int(n[i]), R)]
+        out["segs"][:4 * len(long)] = np.stack([long, first, start, rows], axis=1).reshape(-1)
+        tiles = [(i, q0) for i in range(len(long)) for q0 in range(0, int(n[i]), R)]
         tiles.sort(key=lambda t: -(int(past[t[0]] - first[t[0]]) + t[1]))
         out["tiles"][:2 * len(tiles)] = np.asarray(tiles, dtype=np.int64).reshape(-1)
-        return len(tiles), len(several), len(single), int(rows.sum()), int(rows.max()) if len(rows) else 0
+        return len(tiles), len(long), num_rest, int(rows.sum()), int(rows.max()) if len(rows) else 0
 
     def views(self, dev, filled):
-        n, segs, single, gathered, longest = filled
-        return LatentWork.Views(dev["tiles"][:2 * n].view(n, 2), dev["segs"][:4 * segs].view(segs, 4), dev["rows"][:single], n, segs,
-                                single, gathered, longest)
+        n, segs, rest, gathered, longest = filled
+        return LatentWork.Views(dev["tiles"][:2 * n].view(n, 2), dev["segs"][:4 * segs].view(segs, 4), dev["rows"][:rest], n, segs,
+                                rest, gathered, longest)
 
 
 @register_mixer("latent_attention")
@@ -137,6 +153,7 @@ class LatentAttentionMixer:
         self.tensor_core = (compute_dtype == torch.bfloat16 and self.device.type == "cuda"
                             and ops.latent_attention_supported(self.R, self.P))
         self.expands = (self.tensor_core and self.scale > 0 and ops.latent_prefill_supported(self.D, self.V, self.R, self.P))
+        self._work = LatentWork(spec.window, self.EXPANDED_BYTES // (2 * self.H * (self.D + self.V))) if self.expands else None
         self._expand = None         # (W_ukv [H * (D + V), R],): per head the key map, then the value map, for long prompt steps
         self.w_in = self.w_uq = self.w_uk_t = self.w_uv_t = self.w_o = None
         self.wq_norm = self.wkv_norm = None
@@ -177,16 +194,12 @@ class LatentAttentionMixer:
             return None
         return PagedNeed(1, self.R + self.P, self.keep_window, 0)       # keys only: the values are part of the key rows
 
-    # Keys and values of all rows of a step that are made at once at most: a step whose requests have cached more (over
-    # 65,536 rows at 32 heads) stays on the cached-row kernel, which needs nothing per row.
+    # Keys and values of all rows of a step that are made at once at most (65,536 rows at 32 heads); portions beyond that stay
+    # on the cached-row kernel, which needs nothing per row.
     EXPANDED_BYTES = 1 << 30
 
-    @property
-    def _work_name(self):
-        return f"latent_work:{self.spec.window or 0}"
-
     def step_prelude(self):
-        return LatentWork(self.spec.window) if self.expands else None
+        return self._work
 
     def _absorbed(self, q: torch.Tensor, positions: torch.Tensor, token_entry: torch.Tensor, ctx: StageContext) -> torch.Tensor:
         """Attention over the cached rows themselves: q float32 [n, H * (D + P)] of n tokens -> [n, H * V]."""
@@ -210,30 +223,36 @@ class LatentAttentionMixer:
                   out=heads.view(T, H, V).permute(1, 0, 2))
         return heads
 
-    def _gated(self, heads: torch.Tensor, proj: torch.Tensor) -> torch.Tensor:
+    def _gated(self, heads: torch.Tensor, gates: torch.Tensor, off: int) -> torch.Tensor:
         if self.spec.output_gate:
-            ops.gate_mul(heads, proj, self.g_off, heads, 0, self.spec.output_gate, per_head=self.V if self.gate_per_head else 0)
+            ops.gate_mul(heads, gates, off, heads, 0, self.spec.output_gate, per_head=self.V if self.gate_per_head else 0)
         return heads
 
-    def _expanded(self, q: torch.Tensor, proj: torch.Tensor, work: LatentWork.Views, ctx: StageContext) -> torch.Tensor:
-        """Portions of several tokens over per-head keys and values made from their requests' rows (a gate per head is applied
-        as the kernel stores); single tokens of the same step over the rows themselves."""
+    def _portions(self, q: torch.Tensor, proj: torch.Tensor, work: LatentWork.Views, ctx: StageContext) -> torch.Tensor:
+        """[T, H * V] whose rows that belong to segments hold their attention over per-head keys and values (a gate per head is
+        applied as the kernel stores)."""
         b, s = ctx.batch, self.spec
         H, D, P, R, V, T = self.H, self.D, self.P, self.R, self.V, q.shape[0]
+        heads = torch.empty((T, H * V), dtype=self.dtype, device=q.device)
         rows = ops.latent_gather(ctx.cache_keys, work.segs, work.num_segs, work.gathered, work.longest, b.entry_slot, b.entry_kv_len,
                                  ctx.block_table, ctx.page_size, ctx.status)
         kv = torch.mm(rows[:, :R], self._expand[0].t())
         packed = ops.latent_q_pack(q, b.positions, self.inv_freq, H, D, P, self.rot_dims, rot_pairs=self.rot_pairs, rot_mag=self.rot_mag)
-        heads = torch.empty((T, H * V), dtype=self.dtype, device=q.device)
         ops.latent_prefill(packed, kv, rows, heads, work.tiles, work.num_tiles, work.segs, b.entry_q_start, b.entry_q_len,
                            b.entry_kv_len, H, R, s.window, self.scale, ctx.status, gate=proj if self.gate_per_head else None,
                            gate_off=self.g_off)
-        if not self.gate_per_head:
-            heads = self._gated(heads, proj)
-        if work.num_single:
+        return heads if self.gate_per_head else self._gated(heads, proj, self.g_off)
+
+    def _expanded(self, q: torch.Tensor, proj: torch.Tensor, work: LatentWork.Views, ctx: StageContext) -> torch.Tensor:
+        """Long portions over per-head keys and values made from their requests' rows; the other tokens of the same step over
+        the rows themselves."""
+        b = ctx.batch
+        heads = self._portions(q, proj, work, ctx)
+        if work.num_rest:
             pick = work.rows.long()
             one = self._absorbed(q.index_select(0, pick), b.positions.index_select(0, pick), b.token_entry.index_select(0, pick), ctx)
-            heads.index_copy_(0, pick, self._gated(one, proj.index_select(0, pick)))
+            gate = proj.narrow(1, self.g_off, self.gate_width).index_select(0, pick)
+            heads.index_copy_(0, pick, self._gated(one, gate, 0))
         return heads
 
     def forward(self, x: torch.Tensor, ctx: StageContext):
@@ -246,9 +265,10 @@ class LatentAttentionMixer:
                                 self.eps, self.inv_freq, ctx.cache_keys if s.has_kv else None, b, ctx.block_table,
                                 ctx.page_size, ctx.status, self.dtype, rot_pairs=self.rot_pairs, rot_mag=self.rot_mag)
         q = ops.as_tensor(ops.linear(cq, self.w_uq, out_dtype=torch.float32))
-        work = b.preludes.get(self._work_name) if self._expand is not None and not getattr(b, "any_division", False) else None
+        work = b.preludes.get(self._work.name) if self._expand is not None and not getattr(b, "any_division", False) else None
+        heads = None
         if work is not None and work.num_tiles and 2 * work.gathered * H * (D + V) <= self.EXPANDED_BYTES:
             heads = self._expanded(q, proj, work, ctx)
-        else:
-            heads = self._gated(self._absorbed(q, b.positions, b.token_entry, ctx), proj)
+        if heads is None:
+            heads = self._gated(self._absorbed(q, b.positions, b.token_entry, ctx), proj, self.g_off)
         return ops.linear(heads, self.w_o, out_dtype=torch.float32, partials_ok=getattr(ctx, "partials_ok", False))
