@@ -182,7 +182,9 @@ class LatentAttentionMixer:
         self.w_uk_t = t[n["uk"]].view(self.H, self.D, self.R).contiguous()
         self.w_uv_t = t[n["uv"]].view(self.H, self.V, self.R).transpose(1, 2).contiguous()
         if self.expands and t[n["uk"]].dtype == t[n["uv"]].dtype == torch.bfloat16:
-            self._expand = (torch.cat([self.w_uk_t, t[n["uv"]].view(self.H, self.V, self.R)], dim=1).view(-1, self.R),)
+            both = torch.cat([self.w_uk_t, t[n["uv"]].view(self.H, self.V, self.R)], dim=1)
+            self._expand = (both.view(-1, self.R),)
+            self.w_uk_t = both[:, :self.D]              # the key map is kept once
         self.wq_norm = t[n["dq_norm"]].float().contiguous()
         if s.has_kv:
             self.wkv_norm = t[n["dkv_norm"]].float().contiguous()
@@ -268,7 +270,10 @@ class LatentAttentionMixer:
         work = b.preludes.get(self._work.name) if self._expand is not None and not getattr(b, "any_division", False) else None
         heads = None
         if work is not None and work.num_tiles and 2 * work.gathered * H * (D + V) <= self.EXPANDED_BYTES:
-            heads = self._expanded(q, proj, work, ctx)
+            try:
+                heads = self._expanded(q, proj, work, ctx)
+            except torch.cuda.OutOfMemoryError:
+                pass                                  # what it holds grows with the cached rows; the other path's does not
         if heads is None:
             heads = self._gated(self._absorbed(q, b.positions, b.token_entry, ctx), proj, self.g_off)
         return ops.linear(heads, self.w_o, out_dtype=torch.float32, partials_ok=getattr(ctx, "partials_ok", False))

@@ -160,3 +160,11 @@ def test_tile_sizes_are_the_kernels(monkeypatch):
             m.setattr(ops(), name, other)
             with pytest.raises(ops().KernelError):
                 mixer.forward(xs, ctx)
+
+
+def test_out_of_memory_in_the_expanded_path_takes_the_other(monkeypatch):
+    _, mixer, ctx, xs, rows = long_step()
+    def full(*a, **k):
+        raise torch.cuda.OutOfMemoryError("no room for keys and values")
+    monkeypatch.setattr(ops(), "latent_q_pack", full)
+    assert torch.equal(mixer.forward(xs, ctx), rows)
