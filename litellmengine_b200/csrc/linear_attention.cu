@@ -655,10 +655,15 @@ __global__ void __launch_bounds__(256, 2) gla_scan_tiled_kernel(
     }
 }
 
-static bool gla_tiled_takes(int D, int V) {
+// A block is then alone on its SM while there are no more of them than SMs: two walk side by side at half the pace, and the
+// hardware doubles them up where blocks of the kernel in front still sit on the others.
+#define GLA_ALONE_BLOCKS 148
+#define GLA_ALONE_SMEM (116 * 1024)
+static bool gla_tiled_takes(int D, int V, int mode) {
     static int rows_forced = -1;                   // LLM_GLA_ROWS asks for the kernel above
     if (rows_forced < 0) rows_forced = getenv("LLM_GLA_ROWS") != nullptr;
-    return !rows_forced && (D == 64 || D == 128) && (V == 32 || V == 64 || V == 128);
+    if (rows_forced || (D != 64 && D != 128)) return false;
+    return V == 64 || V == 128 || (V == 32 && (mode == GLA_LOCAL || (mode == GLA_OUT && D == 64)));
 }
 
 // Rows of a state column that one thread keeps (R), the row groups DG = ceil(D / R), and the block size the
@@ -748,17 +753,16 @@ extern "C" int llm_recur_scan(
                     aligned16(proj) && (decay_kind || aligned16(la));
     if (smem > 220 * 1024) return LLM_REFUSED_SIZE;
     if (out_dtype != LLM_DT_F32 && out_dtype != LLM_DT_BF16) return LLM_REFUSED_DTYPE;
-    if (decay_kind == 0 && vec && g_off % 4 == 0 && gla_tiled_takes(D, V) && aligned16(state) && (mode == GLA_FULL || aligned16(scratch_s))) {
-        const size_t need = static_cast<size_t>(GLA_TB) * (2 * (3 * D + 2 * V) + V) * sizeof(float);
+    if (decay_kind == 0 && vec && g_off % 4 == 0 && gla_tiled_takes(D, V, mode) && aligned16(state) && (mode == GLA_FULL || aligned16(scratch_s))) {
+        const size_t need = static_cast<size_t>(GLA_TB) * (2 * (3 * D + 2 * V) + V) * sizeof(float);      // 88 KB at most
+        const size_t bytes = static_cast<long long>(num_items) * H <= GLA_ALONE_BLOCKS ? GLA_ALONE_SMEM : need;
 #define TILED(RR, MODE, TO)                                                                                          \
         do {                                                                                                          \
             auto kern = gla_scan_tiled_kernel<RR, MODE, TO>;                                                          \
-            if (need > 48 * 1024) {                                                                                   \
-                const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,         \
-                                                           static_cast<int>(need));                                   \
-                if (e != cudaSuccess) return static_cast<int>(e);                                                     \
-            }                                                                                                         \
-            launch_pdl(kern, dim3(num_items, H), dim3(2 * V), need, reinterpret_cast<cudaStream_t>(stream), proj,     \
+            /* the limit is the same for every launch: another thread may be between the two calls */                 \
+            const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, GLA_ALONE_SMEM); \
+            if (e != cudaSuccess) return static_cast<int>(e);                                                         \
+            launch_pdl(kern, dim3(num_items, H), dim3(2 * V), bytes, reinterpret_cast<cudaStream_t>(stream), proj,     \
                        stride, q_off, k_off, v_off, g_off, la, norm_w, eps, q_scale, out_scale,                       \
                        static_cast<TO*>(out), out_stride, out_off, state, entry_slot, entry_q_start, entry_q_len,     \
                        items, scratch_s, scratch_a, H, V);                                                            \

@@ -1,5 +1,5 @@
 """The register-tiled scan of gated linear attention and the tiled decay kernel against float64, over every state size they
-take, at the edges of their batches of 16 tokens and chunks of 64, in each mode."""
+take, at the edges of their batches of 16 tokens and chunks of 64, in each mode, with a block an SM and with several."""
 import pytest
 import torch
 
@@ -8,12 +8,12 @@ DEV = "cuda:0"
 F64 = torch.float64
 
 
-@pytest.mark.parametrize("D,V", [(64, 32), (64, 128), (128, 32), (128, 64), (128, 128)])
+@pytest.mark.parametrize("D,V,H", [(64, 32, 3), (64, 128, 3), (128, 32, 3), (128, 64, 3), (128, 128, 3), (64, 64, 20), (128, 128, 20)])
 @pytest.mark.parametrize("out_dtype", [torch.float32, torch.bfloat16])
-def test_scan_in_one_pass_and_over_chunks(D, V, out_dtype):
+def test_scan_in_one_pass_and_over_chunks(D, V, H, out_dtype):
     from litellmengine_b200.csrc import ops
     g = torch.Generator(device=DEV).manual_seed(D + V)
-    H, rank, eps, C = 3, 20, 1e-5, 64
+    rank, eps, C = 20, 1e-5, 64
     lens, tau = [1, 15, 16, 17, 63, 64, 65, 130], 4.0
     T = sum(lens)
     W = 2 * H * D + 2 * H * V + rank
