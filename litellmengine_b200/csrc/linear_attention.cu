@@ -161,8 +161,10 @@ extern "C" int llm_gla_decay(const float* proj, long long stride, int a_off, int
     const dim3 grid((num_tokens + GLA_DECAY_TOKENS - 1) / GLA_DECAY_TOKENS,
                     (channels + GLA_DECAY_CHANNELS - 1) / GLA_DECAY_CHANNELS);
     if (grid.y > 65535) return LLM_REFUSED_SIZE;
-    // from a few rows on (a handful of tokens leaves most of a thread's eight idle), and while the inputs fit 48 KB
-    if (num_tokens >= 8 && channels % 4 == 0 && rank <= 384 && aligned16(w2t) && aligned16(la) && (!b2 || aligned16(b2))) {
+    // From 16 rows on (fewer leave most of a thread's eight idle), and while the inputs fit 48 KB.  Both (us, this one first), at
+    // 2,048 channels of rank 64: 8 tokens 15.0, 14.3; 16: 15.3, 16.2; 32: 16.6, 21.1; 256: 17.5, 23.1; 2,048: 39.6, 64.6; at 512
+    // channels 14.7, 13.7; 15.1, 16.0; 16.4, 20.8; 16.7, 21.2; 20.0, 33.9.
+    if (num_tokens >= 16 && channels % 4 == 0 && rank <= 384 && aligned16(w2t) && aligned16(la) && (!b2 || aligned16(b2))) {
         launch_pdl(gla_decay_tiled_kernel, grid, dim3(128), GLA_DECAY_TOKENS * rank * sizeof(float), reinterpret_cast<cudaStream_t>(stream),
                    proj, stride, a_off, rank, w2t, b2, 1.0f / tau, la, channels, num_tokens);
         return launch_status();
