@@ -983,14 +983,14 @@ static int delta_shape(DeltaShape& s, int H, int G, int D, int V, int taps, int 
 // Everything of a step that is not all single tokens.  Scratch (float32): qn, kn [T, G, DP], vn [T, H, VP], beta [T, H],
 // decay [T, H, DP] (whose places from D on must be finite), gate and o [T, H, V], pk and pq [T, H, DP], and for P =
 // T / 8 + entries + 1 chunks total [P, H, DP] and num [P, H, 128].
-// `conv_w` [C, taps]: the rows of q, k and v one after another.
+// `conv_w` [C, taps]: the rows of q, k and v one after another.  max_len: tokens of the longest entry, 0: not known.
 extern "C" int llm_delta_scan(
     const float* proj, long long stride, int q_off, int b_off, int a_off, int ra, int g_off, int rg, const float* conv_w, int taps,
     const void* wa, const void* wg, int w_dtype, const float* dt_bias, const float* a_log, const float* norm_w, float eps,
     float out_scale, void* out, int out_dtype, long long out_stride, int out_off, float* state, long long slot_stride,
     const int32_t* positions, const int32_t* token_entry, const int32_t* entry_slot, const int32_t* entry_q_start,
-    const int32_t* entry_q_len, int num_tokens, int num_entries, int H, int G, int D, int V, float* qn, float* kn, float* vn,
-    float* beta, float* decay, float* gate, float* o, float* pk, float* pq, float* total, float* num, uintptr_t stream) {
+    const int32_t* entry_q_len, int num_tokens, int num_entries, int max_len, int H, int G, int D, int V, float* qn, float* kn,
+    float* vn, float* beta, float* decay, float* gate, float* o, float* pk, float* pq, float* total, float* num, uintptr_t stream) {
     if (num_tokens <= 0 || num_entries <= 0) return LLM_OK;
     DeltaShape s;
     const int rc = delta_shape(s, H, G, D, V, taps, q_off, b_off, a_off, ra, g_off, rg, stride, slot_stride);
@@ -1047,12 +1047,14 @@ extern "C" int llm_delta_scan(
         default: CHUNKS_OF(256); break;
     }
 #undef CHUNKS_OF
-// A portion is as long as its blocks' walk, and a block beside another on its SM walks at half the pace (two fill the
-// multiply-add pipe).  So portions start longest first, and up to two blocks an SM of the device the blocks ask for more than
-// half of an SM's shared memory: each has an SM of its own, and the last ones begin where short portions have ended.  Measured
-// (us; portions of 284, 567 and 849 tokens, 192 blocks): as the hardware deals them 241, longest first 188, and alone 160;
-// eight of 55 to 445 tokens, 256 blocks: longest first 106, and alone 89; 512 blocks: side by side 179, alone 208.
-#define DR_ALONE_BLOCKS (2 * 148)
+// A portion is as long as its blocks' walk, and a block beside another on its SM walks at a little over half the pace.  So
+// portions start longest first, and the blocks ask for more than half of an SM's shared memory, each to have an SM of its own,
+// while the device's SMs can do all walks in the time of the longest one: the last blocks begin where short portions have ended.
+// Up to two blocks an SM, and by the longest portion (`max_len`; not known, 0: while no SM gets two).  Measured (us; portions
+// of 284, 567 and 849 tokens, 192 blocks): as the hardware deals them 241, longest first 188, and alone 160; eight of 55 to 445
+// tokens, 256 blocks: longest first 106, and alone 89; 512 blocks: side by side 179, alone 208.  Equal portions of 256 tokens, the
+// whole layer's kernels: 156 blocks side by side 128, alone 148; 192: 138, 157; 256: 151, 172; 288: 154, 176.
+#define DR_SMS 148
 #define DR_ALONE_SMEM (116 * 1024)
 #define SCAN(DP, C, WARPS, L)                                                                                         \
     do {                                                                                                              \
@@ -1063,7 +1065,8 @@ extern "C" int llm_delta_scan(
         const int tiles = (V + COLS - 1) / COLS;                                                                      \
         const long long blocks = static_cast<long long>(num_entries) * H * tiles;                                     \
         if (blocks > 0x7fffffffLL) return LLM_REFUSED_SIZE;                                                           \
-        const size_t smem = blocks <= DR_ALONE_BLOCKS ? most : need;                                                  \
+        const bool alone = blocks <= DR_SMS || (blocks <= 2 * DR_SMS && walks * tiles <= static_cast<long long>(DR_SMS) * max_len); \
+        const size_t smem = alone ? most : need;                                                                      \
         /* the limit is the same for every launch: another thread may be between the two calls */                     \
         const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(most)); \
         if (e != cudaSuccess) return static_cast<int>(e);                                                             \
@@ -1073,7 +1076,7 @@ extern "C" int llm_delta_scan(
     // few columns: fewer a warp, so that more schedulers have one; many: more a warp, which costs fewer instructions a column.
     // Measured at 128 rows (us; one, two, four columns on 32 lanes, four on 16): 512 columns (1,000 tokens) 106 111 133 177,
     // 1,024: 141 112 134 181, 2,048: 213 159 136 182, 4,096 (1,500 tokens of 4 requests): 203 154 131 113.
-    const long long columns = static_cast<long long>(num_entries) * H * V;
+    const long long columns = static_cast<long long>(num_entries) * H * V, walks = static_cast<long long>(num_tokens) * H;
     const int plan = columns <= 640 ? 0 : columns <= 1300 ? 1 : columns <= 3000 ? 2 : 3;
     switch (s.DP) {
         case 32: SCAN(32, 2, 2, 8); break;

@@ -1196,9 +1196,11 @@ def delta_rule(proj: torch.Tensor, offs, ranks, conv_w: torch.Tensor, w_decay: t
         room[:sizes[0]].zero_()                             # decays behind a head's key width must be finite
     decay, qn, kn, vn, beta, gate, o, pk, pq, total, num = (room.data_ptr() + 4 * n for n in starts[:-1])
     f = _fn("delta_rule", "llm_delta_scan",
-            head + [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int] + [c_void_p] * 12)
+            head + [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int] + [c_void_p] * 12)
+    # a graph that is being captured serves other divisions of its tokens too
+    longest = 0 if getattr(batch, "any_division", False) else getattr(batch, "max_q_len", 0)
     _check(f(*args, _ptr(batch.token_entry), _ptr(batch.entry_slot), _ptr(batch.entry_q_start), _ptr(batch.entry_q_len), T,
-             batch.num_entries, H, G, D, V, qn, kn, vn, beta, decay, gate, o, pk, pq, total, num, _stream()), "delta_scan")
+             batch.num_entries, longest, H, G, D, V, qn, kn, vn, beta, decay, gate, o, pk, pq, total, num, _stream()), "delta_scan")
     global launch_count
     launch_count += 4                          # five kernels in one call
 

@@ -23,7 +23,7 @@ def test_portions_end_anywhere(H, D, V, lens):
     i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)
     starts = [sum(lens[:i]) for i in range(len(lens))]
     b = types.SimpleNamespace(positions=i32([p for n in lens for p in range(n)]), token_entry=i32([e for e, n in enumerate(lens) for _ in range(n)]),
-                              entry_slot=i32(list(range(len(lens)))), entry_q_start=i32(starts), entry_q_len=i32(lens), num_entries=len(lens))
+                              entry_slot=i32(list(range(len(lens)))), entry_q_start=i32(starts), entry_q_len=i32(lens), num_entries=len(lens), max_q_len=max(lens))
     DP = ops.delta_padded(D)
     state = torch.zeros(len(lens), (H * V * DP + taps * C + 3) // 4 * 4, device=DEV)
     out = torch.zeros(T, H * V, device=DEV)
