@@ -79,3 +79,38 @@ def test_low_rank_products_on_the_tensor_cores(T, H, D, V, ra, rg):
     # rank products of 32-bit rounding a number, through a logistic function or a decay; the norm divides by the outputs' size
     assert torch.allclose(a, w, rtol=2e-4, atol=2e-5, equal_nan=True)
     assert torch.allclose(sa, sw, rtol=1e-4, atol=2e-5, equal_nan=True)
+
+
+@pytest.mark.parametrize("T,H,D,V,ra,rg", [(3, 1, 128, 128, 64, 33), (64, 2, 64, 24, 33, 80), (65, 5, 128, 33, 200, 64)])
+def test_decays_and_gates_of_the_low_rank_products(T, H, D, V, ra, rg):
+    """Each number alone against 64 bits: T requests of one token that write nothing (beta zero) leave the decay times the state they
+    found, and two runs that differ in the gate's weights only have outputs whose ratio is the gate."""
+    from litellmengine_b200.csrc import ops
+    g = torch.Generator(device=DEV).manual_seed(T)
+    taps, C = 2, 2 * H * D + H * V
+    rnd = lambda *s: torch.randn(*s, generator=g, device=DEV)
+    proj, conv = rnd(T, C + H + ra + rg), rnd(C, taps)
+    proj[:, C:C + H] = -200.0
+    wa, wg = (rnd(ra, H * D) * 0.2).bfloat16(), (rnd(rg, H * V) * 0.2).bfloat16()
+    dt, al, nw = rnd(H * D), rnd(H) * 0.5 - 2, torch.ones(V, device=DEV)
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)
+    b = types.SimpleNamespace(positions=i32([0] * T), token_entry=i32(list(range(T))), entry_slot=i32(list(range(T))),
+                              entry_q_start=i32(list(range(T))), entry_q_len=i32([1] * T), num_entries=T)
+    DP, outs = ops.delta_padded(D), []
+    for w in (wg, torch.zeros_like(wg)):
+        state = torch.zeros(T, (H * V * DP + taps * C + 3) // 4 * 4, device=DEV)
+        state[:, :H * V * DP] = 1.0
+        out = torch.zeros(T, H * V, device=DEV)
+        ops.delta_rule(proj, (0, C, C + H, C + H + ra), (ra, rg), conv, wa, w, dt, al, nw, 1e-5, 1.0, out, 0, state, b, H, H, D, V,
+                       single=False)
+        outs.append(out.to(F64))
+    x = proj.to(F64)
+    gate = torch.sigmoid(x[:, C + H + ra:] @ wg.to(F64))
+    z = x[:, C + H:C + H + ra] @ wa.to(F64) + dt.to(F64)
+    decay = torch.exp(-torch.exp(al.to(F64))[None, :, None] * torch.nn.functional.softplus(z).view(T, H, D))
+    got = state[:, :H * V * DP].view(T, H, V, DP)[..., :D].to(F64)
+    rms = lambda e: float(e.pow(2).mean().sqrt())
+    # A few roundings of 2^-24 and the error of a sum of up to 200 exact products: 1e-7 to 2e-7.  Without the third part of the
+    # inputs' split it is 2^-17 of the sum, above 5e-6 of a gate or a decay.
+    assert rms(0.5 * outs[0] / outs[1] / gate - 1) < 1e-6
+    assert rms(got / decay[:, :, None, :] - 1) < 1e-6
