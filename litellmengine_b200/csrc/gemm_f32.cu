@@ -151,18 +151,17 @@ static double lf_fill(long long groups, long long tokens, int ks, int mt) {
     return static_cast<double>(blocks) / static_cast<double>((blocks + slots - 1) / slots * slots);
 }
 
-// x: float32 [M, K]; w: float32 [N, K]; y: float32 [M, N].  K a multiple of 4.  ks: 0, or 1, 2, 4, 8 by force.
-extern "C" int llm_linear_f32(const float* x, const float* w, float* y, int M, int N, int K, int ks, uintptr_t stream) {
+// x: float32 [M, K]; w: float32 [N, K]; y: float32 [M, N].  K a multiple of 4.
+extern "C" int llm_linear_f32(const float* x, const float* w, float* y, int M, int N, int K, uintptr_t stream) {
     if (M <= 0 || N <= 0) return LLM_OK;
     if (K <= 0 || (K & 3)) return LLM_REFUSED_SIZE;
     if (!aligned16(x) || !aligned16(w)) return LLM_REFUSED_ALIGN;
     const int mt = M == 1 ? 1 : M == 2 ? 2 : M <= 4 ? 4 : 8;
     const int groups = (N + LF_ROWS - 1) / LF_ROWS, tokens = (M + mt - 1) / mt;
-    if (ks == 0) {                                      // the fewest slices that fill the last wave about as well as any
-        double best = 0.0;
-        for (int c = 1; c <= 8; c *= 2) best = lf_fill(groups, tokens, c, mt) > best ? lf_fill(groups, tokens, c, mt) : best;
-        for (ks = 1; ks < 8 && lf_fill(groups, tokens, ks, mt) < best - 0.07; ks *= 2) {}
-    }
+    double best = 0.0;                                  // the fewest slices that fill the last wave about as well as any
+    for (int c = 1; c <= 8; c *= 2) best = lf_fill(groups, tokens, c, mt) > best ? lf_fill(groups, tokens, c, mt) : best;
+    int ks = 1;
+    while (ks < 8 && lf_fill(groups, tokens, ks, mt) < best - 0.07) ks *= 2;
     while (ks > 1 && groups / (LF_WARPS / ks) >= 65535) ks /= 2;
     cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
     const int per_block = LF_WARPS / ks;

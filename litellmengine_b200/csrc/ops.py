@@ -2009,8 +2009,8 @@ def linear_f32(x: torch.Tensor, weight: torch.Tensor) -> torch.Tensor:
     if weight.shape[1] != K:
         raise KernelError("x and weight disagree on K")
     out = torch.empty((M, N), dtype=torch.float32, device=x.device)
-    f = _fn("gemm_f32", "llm_linear_f32", [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p])
-    _check(f(_ptr(x), _ptr(weight), _ptr(out), M, N, K, 0, _stream()), "linear_f32")
+    f = _fn("gemm_f32", "llm_linear_f32", [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p])
+    _check(f(_ptr(x), _ptr(weight), _ptr(out), M, N, K, _stream()), "linear_f32")
     return out
 
 
