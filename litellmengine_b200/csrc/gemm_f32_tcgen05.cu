@@ -11,7 +11,8 @@
 // What makes the sums as good as float32's: the tensor cores cut, rather than round, what they add to an accumulator, and
 // 256 steps in a row along K = 4096 would show that.  So an accumulator lives for 64 k-values only, smallest terms first,
 // and is then added, rounded, to sums kept in registers by the warps that drain it.  Error against 64 bits (relative, 2-norm,
-// K = 4096): 1.5e-7 to 1.9e-7; the library's float32 product 1.1e-6.
+// K = 4096, values of either sign and of one): 1.1e-7 and 1.0e-7; the library's float32 product 4.3e-7 to 1.2e-6 and 1.5e-7 to
+// 9.9e-7.
 // A result that is not finite is computed again with plain multiply-adds (a split infinity times zero is NaN, and a value
 // above bfloat16's largest rounds to infinity), so infinities and NaN come out as a float32 product has them.
 //
@@ -22,17 +23,21 @@
 // warps 10 to 17 drain.  Planes are double-buffered (96 KB of weights' planes, 96 KB of x at NT 128).
 // The weights' planes go to tensor memory, from where the tensor cores take their left operand: kept in shared memory, their
 // stores and the operand reads of 24 products a block (8 KB each) filled the shared-memory path (500 tokens of 4096 x 12288:
-// 323 us, now 291).  What bounds it now is the tensor pipe: 24 products of 128 x NT x 16 a block take 2,500 to 2,900 clocks.
+// 323 us, 291 in tensor memory).  What bounds it is the chain of small products: 24 of 128 x NT x 16 a block take 2,500 to 2,900
+// clocks, the tensor pipe is busy for 43 % of the time (q/k/v and output product of a prompt of 500 tokens, width 4,096).
+// The loop that makes sums again which are not finite stays rolled: unrolled into each of a drain thread's sums it cost
+// finite ones up to 20 % (500 tokens of 6144 x 4096: 209 us, now 167).
 // Tiles that fill the SMs badly are cut along K (`splits`), the parts added in order by a second kernel.
 //
 // Measured (us; the library's float32 product in brackets):
 //   N x K              17 rows        64 rows        128 rows       500 rows       2,048 rows
-//   6144 x 4096        39 (102)       43 (124)       66 (167)       203 (541)      679 (1,772)
-//   4096 x 4096        31 (101)       34 (102)       55 (121)       117 (309)      455 (1,131)
-//   24576 x 4096       146 (198)      153 (282)      241 (548)      665 (1,775)    2,336 (6,606)
-//   4096 x 12288       74 (242)       77 (305)       103 (359)      293 (911)      1,196 (3,350)
-//   2048 x 2048        18 (51)        21 (51)
-// Matrices of fewer than 2^21 values stay with the library (1024 x 1024: 17 against 14 at 17 rows, 31 against 30 at 512).
+//   6144 x 4096        41 (106)       42 (129)       49 (170)       167 (542)      577 (1,773)
+//   4096 x 4096        33 (105)       34 (106)       38 (126)       101 (311)      390 (1,132)
+//   24576 x 4096       143 (199)      148 (283)      169 (551)      576 (1,779)    2,028 (6,686)
+//   4096 x 12288       77 (250)       81 (321)       87 (373)       283 (925)      1,063 (3,353)
+//   2048 x 2048        23 (54)        23 (53)        25 (52)        37 (87)        109 (308)
+// Matrices of fewer than 2^21 values stay with the library: of 1024 x 1024, 17 rows take 23 us against 18 (and 64 to 2,048 rows 23
+// to 34 against 29 to 86: for many rows the line could lie lower).
 #include "tcgen05_attention.cuh"
 #include <math_constants.h>
 
@@ -320,8 +325,9 @@ static bool lt_encode_f32(CUtensorMap* map, const void* base, long long cols, lo
 static int lt_tile(int M) { return M <= 32 ? 32 : M <= 64 ? 64 : 128; }
 
 // Into how many parts K is cut: the least of waves of 148 CTAs x (blocks of 64 x BLK + 4 us) + the parts' way through memory,
-// with the measured time of a block (1.5 us at 128 tokens, 1.0 below).  500 tokens: 6144 x 4096 takes 2 (221 -> 201 us), 4096
-// x 4096 stays whole (117; in eight parts 214); 17 tokens of 4096 x 12288: 4 (256 -> 75).
+// with a block's time (1.5 us at 128 tokens, 1.0 below).  In 1, 2, 3, 4, 6, 8 parts (us): 500 tokens of 6144 x 4096 195, 169, 167,
+// 200, 203, 238 (takes 3), of 4096 x 4096 101, 115, 124, 134, 148, 155 (1), of 4096 x 12288 278, 297, 307, 315, 328, 313 (1); 17
+// tokens of 4096 x 12288 259, 137, 96, 77, 101, 83 (4), of 24576 x 4096 182, 149, 142, 163, 161, 177 (3).
 extern "C" int llm_linear_f32_tcgen05_splits(int M, int N, int K) {
     if (M <= 0 || N <= 0 || K <= 0) return 1;
     const int nt = lt_tile(M);

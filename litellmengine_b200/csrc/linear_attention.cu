@@ -450,8 +450,14 @@ __global__ void __launch_bounds__(MAX_THREADS) gla_scan_kernel(
 // exchanges, two tokens at a time: fifteen shuffles for sixteen sums, one of which each lane leaves in shared memory.  A block is 2 V
 // threads, two blocks an SM.  Same modes, staging and epilogue as above; every state element is updated by the same
 // operations in the same order (k v, then decay times state plus that), only o's sum runs over the rows in another order.
-// 2,048 tokens, 16 heads of 128 x 128: local pass and output pass 193 us each -> 66 and 113 us
-// (161 with one token's sums at a time and the gates read from global memory in the epilogue).
+// 2,048 tokens, 16 heads of 128 x 128: local pass and output pass 133 and 217 us -> 66 and 113 us
+// (161 with one token's sums at a time and the gates read from global memory in the epilogue).  Other states, 16 heads (us, the
+// kernel above and this one): one pass over 64 tokens; local and output pass over 2,048:
+//   64 x 32    29, 30;  42, 17;  53, 40        128 x 32    28, 40;  59, 25;  68, 73
+//   64 x 64    30, 24;  50, 25;  63, 41        128 x 64    34, 34;  87, 37;  108, 72
+//   64 x 128   37, 27;  86, 45;  117, 71       128 x 128   50, 41;  133, 66; 217, 113
+// so 32 columns (blocks of 64 threads) stay with the kernel above, but for the local pass and, at 64 rows, the
+// output pass.
 typedef unsigned long long gla_pair;
 __device__ __forceinline__ gla_pair gla_mul2(gla_pair a, gla_pair b) {
     gla_pair r;
@@ -657,8 +663,9 @@ __global__ void __launch_bounds__(256, 2) gla_scan_tiled_kernel(
     }
 }
 
-// A block is then alone on its SM while there are no more of them than SMs: two walk side by side at half the pace, and the
-// hardware doubles them up where blocks of the kernel in front still sit on the others.
+// A block is alone on its SM while there are no more of them than SMs: two walk side by side at half the pace, and the
+// hardware doubles them up where blocks of the kernel in front still sit on the others.  128 x 128, 128 blocks: one pass over eight
+// requests of 64 tokens 65 -> 42 us, the output pass over 512 tokens 56 -> 36.
 #define GLA_ALONE_BLOCKS 148
 #define GLA_ALONE_SMEM (116 * 1024)
 static bool gla_tiled_takes(int D, int V, int mode) {

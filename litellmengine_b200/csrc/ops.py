@@ -2019,9 +2019,9 @@ F32_TENSOR_ROWS = 2048              # rows at a time: the split of x takes six b
 
 
 def linear_f32_tcgen05(x: torch.Tensor, weight: torch.Tensor) -> torch.Tensor:
-    """x [M, K] @ weight[N, K]^T, all float32, on the tensor cores: both operands as exact sums of three bfloat16 values, six
-    products of them accumulated in float32 (see csrc/gemm_f32_tcgen05.cu; its error is below that of a float32 product added
-    in order).  K must be a multiple of 8 and both operands 16-byte aligned."""
+    """x [M, K] @ weight[N, K]^T, all float32, on the tensor cores: both operands as sums of three bfloat16 values, six products
+    of them accumulated in float32; what is left out of a product is at most 2^-24 of it, and the sums are as near to 64 bits
+    as float32 multiply-adds come (csrc/gemm_f32_tcgen05.cu has the figures).  K must be a multiple of 8 and both operands 16-byte aligned."""
     _dev(x, weight)
     if x.dtype != torch.float32 or weight.dtype != torch.float32:
         raise KernelError("the float32 product takes float32 operands")
@@ -2057,7 +2057,8 @@ def linear(x: torch.Tensor, weight: torch.Tensor, out_dtype: Optional[torch.dtyp
     product `linear_pair`; by default only the gate/up product does, through `linear_silu_mul`) (the reference uses cuBLAS for all its products,
     src/layers/linear.cu:169-215).  bfloat16 operands accumulate in float32; a float32 weight
     keeps its product in true float32 (no TF32), whatever x is: up to 16 rows in the engine's own streaming kernel, more rows of large matrices
-    on the tensor cores as exact sums of bfloat16 values."""
+    on the tensor cores as sums of three bfloat16 values each, as near as float32 sums.  bfloat16 weights may be read before the
+    kernel in front of the product in the stream has finished (they are nobody's output); float32 ones are not."""
     _dev(x, weight)
     rows = x.shape[0]
     if (x.dtype == torch.bfloat16 and weight.dtype == torch.bfloat16 and x.shape[1] % 8 == 0 and weight.data_ptr() % 16 == 0
