@@ -342,10 +342,10 @@ __global__ void __launch_bounds__(64 + 128 * HEADS, 1) paged_prefill_attention_t
 // window's first tile are walked first; kept keys inside the window's tiles are a matter of the mask), one more term
 // exp(sinks[head]) in the softmax's denominator, a sigmoid gate per head (column gate_off + head of a float32 row per
 // token), a factor, and a result that is a column range of a wider buffer.  Measured, 32 heads over 8, window 1,024, four
-// kept keys, learned sinks, 2,500 tokens: 216 us on mma.sync (attention_prefill.cu), 84 us here.  In this mode the reference
+// kept keys, learned sinks, 2,500 tokens: 216 us on mma.sync (attention_prefill.cu), 87 us here.  In this mode the reference
 // is the running maximum itself, so that the largest weight so far is exactly one in bfloat16, as on mma.sync, and the
-// weights are summed as rounded.  With a reference that trails and a sum of unrounded weights it is 74 us, and the error against
-// 64 bits 3, 13 and 20 % above that of mma.sync at spreads of the scores of 1, 2 and 4 (now 0.2 % below, level, 0.1 % below).
+// weights are summed as rounded.  With a reference that trails and a sum of unrounded weights it takes 10 us less, and the error against
+// 64 bits is 3, 13 and 20 % above that of mma.sync at spreads of the scores of 1, 2 and 4 (now 0.2 % below, level, 0.1 % below).
 struct T5Ext {
     int keep_first;
     const float* sinks;
@@ -689,6 +689,21 @@ __global__ void __launch_bounds__(T5O_THREADS, 1) paged_prefill_attention_tcgen0
             weights(rb, 32);
             t5_wait_st();
             t5_fence_before();
+            if constexpr (EXT) {
+                // Keys of the tile that no row of the block sees (behind its last one, below the window, behind the kept ones) have weights
+                // of zero, but what lies there may be anything (a request that had the page before, a held page's copy), and zero times a
+                // value that is not finite is NaN: their values are set to zero before the products, a row of 128 bytes a thread.
+                const int k0 = tile_key(j), key = k0 + (tid & 127), lo_first = first_visible(pos_first, window);
+                if (g == 0 && (k0 + T5O_BN - 1 > pos_last || (k0 < lo_first && k0 + T5O_BN > keep))) {
+                    if (!t5_wait(&v_full[j % STAGES], (j / STAGES) & 1, &abort_flag, status, row_base)) { ok = false; continue; }
+                    if (key > pos_last || (key < lo_first && key >= keep)) {
+                        uint4* v = reinterpret_cast<uint4*>(v_s + (j % STAGES) * T5O_TILE + ((tid - 64) >> 7) * T5O_HALF + (tid & 127) * 64);
+#pragma unroll
+                        for (int c = 0; c < 8; ++c) v[(c + lane) & 7] = make_uint4(0u, 0u, 0u, 0u);      // a quarter-warp: all banks
+                    }
+                    asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+                }
+            }
             t5_arrive(&p_full[g]);
         }
         // the row sum is the two halves' sums

@@ -95,3 +95,42 @@ def test_as_near_as_the_mma_sync_kernel(spread):
     ref = torch.einsum("hts,hsd->thd", p, v).reshape(T, nq * d)
     mine, other = (float((x.to(F64) - ref).norm() / ref.norm()) for x in (a, b))
     assert mine < 1.01 * other, (mine, other)
+
+
+@pytest.mark.parametrize("window,keep", [(None, 0), (100, 5), (300, 130), (-200, 0)])
+def test_what_lies_beside_the_keys_stays_out(window, keep):
+    """Values that no row of a block of 128 sees are not finite: behind a request's end in its last page (somebody else's, from
+    before), behind a block's last row, and below its window."""
+    from litellmengine_b200.csrc import ops
+    g = torch.Generator(device=DEV).manual_seed(keep)
+    nq, nkv, d, page, scale = 4, 2, 128, 16, 128 ** -0.5
+    reqs = [(2, 2), (130, 130), (333, 70), (700, 257), (1001, 30)]
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)
+    width = max(-(-n // page) for n, _ in reqs)
+    table = torch.randperm(len(reqs) * width, generator=g, device=DEV).to(torch.int32).view(len(reqs), width).contiguous()
+    span = abs(window) if window else 0
+    lowest = lambda p: max(0, p - window + 1) if window and window > 0 else p // span * span if window else 0
+    T, starts = sum(t for _, t in reqs), [sum(t for _, t in reqs[:b]) for b in range(len(reqs))]
+    q = torch.randn(T, nq * d, generator=g, device=DEV).to(torch.bfloat16)
+    out, status = torch.zeros(T, nq * d, device=DEV, dtype=torch.bfloat16), i32([0, 0])
+    for b, (n, t) in enumerate(reqs):
+        for r in range(0, t, 128):             # a block at a time, over a cache that holds only what this one sees
+            first, last = n - t + r, n - t + min(t, r + 128) - 1
+            cache = torch.full((table.numel(), 2, nkv, page, d), float("nan"), device=DEV, dtype=torch.bfloat16)
+            j = torch.tensor([x for x in range(last + 1) if x >= lowest(first) or x < keep], device=DEV)
+            k, v = (torch.randn(len(j), nkv, d, generator=g, device=DEV).to(torch.bfloat16) for _ in range(2))
+            for x, kv in ((0, k), (1, v)):
+                cache[table[b, j // page].long(), x, :, j % page] = kv
+            ops.paged_attention_prefill_tcgen05_ext(q, out, 0, cache, i32([(b, r)]), 1, i32(list(range(len(reqs)))), i32(starts),
+                                                    i32([t for _, t in reqs]), i32([n for n, _ in reqs]), table, nq, nkv, d, page, window,
+                                                    scale, status, keep_first=keep)
+            rows = slice(starts[b] + r, starts[b] + r + last - first + 1)
+            i = torch.arange(first, last + 1, device=DEV)[:, None]
+            near = (i - j < window) if window and window > 0 else (j >= i - i % span) if window else torch.ones_like(i - j, dtype=torch.bool)
+            kk, vv = (x.to(F64).repeat_interleave(nq // nkv, 1) for x in (k, v))
+            s = torch.einsum("thd,shd->hts", q[rows].view(-1, nq, d).to(F64), kk) * scale
+            p = torch.softmax(s.masked_fill(~((j <= i) & (near | (j < keep))), float("-inf")), -1)
+            ref = torch.einsum("hts,shd->thd", p, vv)
+            bound = 2 ** -8 * (ref.abs() + torch.einsum("hts,shd->thd", p, vv.abs())) + 1e-3
+            assert bool(((out[rows].view(-1, nq, d).to(F64) - ref).abs() <= bound).all()), (n, t, r)
+    assert status.tolist() == [0, 0]
