@@ -701,7 +701,7 @@ __global__ void __launch_bounds__(WARPS * 32) delta_scan_kernel(
                 for (int t = 0; t < CH; ++t) {
                     const float um = C == 1 ? u[t][0] : C == 2 ? ((m & 1) ? u[t][C - 1] : u[t][0])
                                             : (m & 2) ? ((m & 1) ? u[t][C - 1] : u[t][C >= 4 ? 2 : 0]) : ((m & 1) ? u[t][C >= 2 ? 1 : 0] : u[t][0]);
-                    out += bi[t] * um;
+                    if (t <= i) out += bi[t] * um;              // a later token's u may be NaN, and zero times it too
                 }
                 if (i < left && m < cols_here)
                     o[(static_cast<size_t>(row0 + done + ch * CH + i) * s.H + h) * s.V + c0 + cb + m] = out;

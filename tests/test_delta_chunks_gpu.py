@@ -114,3 +114,26 @@ def test_decays_and_gates_of_the_low_rank_products(T, H, D, V, ra, rg):
     # inputs' split it is 2^-17 of the sum, above 5e-6 of a gate or a decay.
     assert rms(0.5 * outs[0] / outs[1] / gate - 1) < 1e-6
     assert rms(got / decay[:, :, None, :] - 1) < 1e-6
+
+
+@pytest.mark.parametrize("D,V,H", [(128, 128, 2), (64, 20, 2), (128, 128, 16)])
+def test_a_value_that_is_not_finite_reaches_only_later_tokens(D, V, H):
+    from litellmengine_b200.csrc import ops
+    g = torch.Generator(device=DEV).manual_seed(D)
+    T, bad, taps, ra, rg, C = 37, 14, 1, 4, 5, 2 * H * D + H * V
+    rnd = lambda *s: torch.randn(*s, generator=g, device=DEV)
+    proj, conv = rnd(T, C + H + ra + rg), rnd(C, taps)
+    wa, wg, dt, al, nw = rnd(ra, H * D) * 0.3, rnd(rg, H * V) * 0.3, rnd(H * D), rnd(H) * 0.5, torch.ones(V, device=DEV)
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)
+    b = types.SimpleNamespace(positions=i32(list(range(T))), token_entry=i32([0] * T), entry_slot=i32([0]), entry_q_start=i32([0]),
+                              entry_q_len=i32([T]), num_entries=1, max_q_len=T)
+    outs = []
+    for spoil in (False, True):
+        x = proj.clone()
+        if spoil:
+            x[bad, 2 * H * D:C] = float("nan")
+        state = torch.zeros(1, (H * V * ops.delta_padded(D) + taps * C + 3) // 4 * 4, device=DEV)
+        out = torch.zeros(T, H * V, device=DEV)
+        ops.delta_rule(x, (0, C, C + H, C + H + ra), (ra, rg), conv, wa, wg, dt, al, nw, 1e-5, 1.0, out, 0, state, b, H, H, D, V, single=False)
+        outs.append(out)
+    assert torch.equal(outs[0][:bad], outs[1][:bad]) and not bool(torch.isfinite(outs[1][bad:]).any())
