@@ -45,13 +45,61 @@ __device__ __forceinline__ void lp_st8(unsigned taddr, const unsigned (&r)[24], 
                  "r"(r[at + 6]), "r"(r[at + 7]) : "memory");
 }
 
+// A row's attention again, without the tensor cores, over the keys it sees and no others (half of its columns, gated): what a
+// row takes whose sums are not finite.  Weights of hidden keys are zero, and zero times a value that is not finite is NaN; a
+// token of a portion must not spoil the rows before it, nor one behind their window those after it.  q: the row's head; k: the
+// head's [k | v] of the first of `keys` keys; r: their rotated parts.
+__device__ __noinline__ void lp_row_again(const bf16* __restrict__ q, const bf16* __restrict__ k, size_t k_stride, const bf16* __restrict__ r,
+                                          size_t r_stride, int keys, int half, float scale_log2e, float gate, bf16* __restrict__ out) {
+    float m = -CUDART_INF_F, l = 0.0f, acc[64];
+#pragma unroll
+    for (int c = 0; c < 64; ++c) acc[c] = 0.0f;
+#pragma unroll 1
+    for (int j = 0; j < keys; ++j, k += k_stride, r += r_stride) {
+        float s = 0.0f;
+#pragma unroll 1
+        for (int c = 0; c < LP_DK; c += 8) {
+            float a[8], b[8];
+            load8(q + c, a);
+            load8(c < 128 ? k + c : r + c - 128, b);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) s = fmaf(a[i], b[i], s);
+        }
+        s *= scale_log2e;
+        if (s != s) {                                             // a key that the row sees is NaN: so is the row
+            l = s;
+            break;
+        }
+        const float top = fmaxf(m, s), base = top == -CUDART_INF_F ? 0.0f : top;
+        const float alpha = t5_ex2(m - base), p = t5_ex2(s - base);
+        l = fmaf(l, alpha, p);
+        m = top;
+#pragma unroll
+        for (int c = 0; c < 64; c += 8) {
+            float v[8];
+            load8(k + 128 + half * 64 + c, v);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) acc[c + i] = fmaf(p, v[i], acc[c + i] * alpha);
+        }
+    }
+    const float inv = l == 0.0f ? 0.0f : gate / l;
+#pragma unroll
+    for (int c = 0; c < 64; c += 8) {
+        float v[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) v[i] = acc[c + i] * inv;
+        store8(out + c, v);
+    }
+}
+
 // grid (H, work items).  tiles: int32 [n][2] = (segment, first query row inside the portion), 256 rows each, longest walk
 // first; segs: int32 [segments][4] = (entry, first position gathered, first gathered row, rows).
 __global__ void __launch_bounds__(LP_THREADS, 1) latent_prefill_tcgen05_kernel(
     const __grid_constant__ CUtensorMap q_map, const __grid_constant__ CUtensorMap kv_map, const __grid_constant__ CUtensorMap r_map,
     bf16* __restrict__ out, const int32_t* __restrict__ tiles, const int32_t* __restrict__ segs,
     const int32_t* __restrict__ entry_q_start, const int32_t* __restrict__ entry_q_len, const int32_t* __restrict__ entry_kv_len,
-    int H, int R, int window, float scale_log2e, const float* __restrict__ gate, long long gate_stride, int32_t* __restrict__ status) {
+    int H, int R, int window, float scale_log2e, const float* __restrict__ gate, long long gate_stride, int32_t* __restrict__ status,
+    const bf16* __restrict__ q, const bf16* __restrict__ kv, const bf16* __restrict__ gathered) {
     pdl_begin();
     extern __shared__ unsigned char smem_dyn[];
     unsigned char* smem_al = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_dyn) + 1023) & ~uintptr_t(1023));
@@ -292,12 +340,15 @@ __global__ void __launch_bounds__(LP_THREADS, 1) latent_prefill_tcgen05_kernel(
             float inv = (l > 0.0f) ? 1.0f / l : 0.0f;
             if (gate && row < rows_here)                          // a sigmoid gate per token and head, on the result as it leaves
                 inv /= 1.0f + expf(-gate[static_cast<size_t>(row_base + g * LP_BM + row) * gate_stride + h]);
+            bool finite = l <= 3.402823466e38f;                   // not infinite, not NaN
             bf16* orow = out + (static_cast<size_t>(row_base + g * LP_BM + row) * H + h) * LP_DV + half * 64;
 #pragma unroll 1
             for (int c = 0; c < 64; c += 32) {
                 unsigned o[32];
                 t5_ld32(my_o + c, o);
                 t5_wait_ld();
+#pragma unroll
+                for (int i = 0; i < 32; ++i) finite = finite && fabsf(__uint_as_float(o[i])) <= 3.402823466e38f;
                 if (row < rows_here) {
 #pragma unroll
                     for (int i = 0; i < 32; i += 8) {
@@ -309,6 +360,12 @@ __global__ void __launch_bounds__(LP_THREADS, 1) latent_prefill_tcgen05_kernel(
                         *reinterpret_cast<uint4*>(orow + c + i) = w;
                     }
                 }
+            }
+            if (row < rows_here && !finite) {
+                const size_t token = static_cast<size_t>(row_base + g * LP_BM + row), at = static_cast<size_t>(kv_row0 + max(lo, 0));
+                lp_row_again(q + (token * H + h) * LP_DK, kv + (at * H + h) * 256, static_cast<size_t>(H) * 256,
+                             gathered + at * (R + 64) + R, R + 64, pos - max(lo, 0) + 1, half, scale_log2e,
+                             gate ? 1.0f / (1.0f + expf(-gate[token * gate_stride + h])) : 1.0f, orow);
             }
         }
     }
@@ -436,6 +493,7 @@ extern "C" int llm_latent_prefill(const void* q, const void* kv, const void* gat
     if (e != cudaSuccess) return static_cast<int>(e);
     launch_pdl(latent_prefill_tcgen05_kernel, dim3(H, n_tiles), dim3(LP_THREADS), smem, reinterpret_cast<cudaStream_t>(stream), q_map,
                kv_map, r_map, static_cast<bf16*>(out), tiles, segs, entry_q_start, entry_q_len, entry_kv_len, H, R, window,
-               scale * 1.4426950408889634f, gate, gate_stride, status);
+               scale * 1.4426950408889634f, gate, gate_stride, status, static_cast<const bf16*>(q), static_cast<const bf16*>(kv),
+               static_cast<const bf16*>(gathered));
     return launch_status();
 }

@@ -168,3 +168,45 @@ def test_out_of_memory_in_the_expanded_path_takes_the_other(monkeypatch):
         raise torch.cuda.OutOfMemoryError("no room for keys and values")
     monkeypatch.setattr(ops(), "latent_q_pack", full)
     assert torch.equal(mixer.forward(xs, ctx), rows)
+
+
+@pytest.mark.parametrize("window,gated", [(None, False), (100, True)])
+def test_a_row_that_is_not_finite_reaches_only_who_sees_it(window, gated):
+    """Cached rows with infinities and NaN in a portion: the queries before them, and those that have them behind their window, stay
+    as they would be without."""
+    o = ops()
+    g = torch.Generator(device=DEV).manual_seed(7)
+    H, R, n, t, past = 2, 128, 700, 600, 100
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)
+    first = max(0, past - window + 1) if window else 0
+    count, K = -(-(n - first) // o.LATENT_TILE_KEYS) * o.LATENT_TILE_KEYS, o.LATENT_TILE_ROWS
+    rows = torch.zeros(count, R + 64, device=DEV, dtype=torch.bfloat16)
+    rows[:n - first] = torch.randn(n - first, R + 64, generator=g, device=DEV).to(torch.bfloat16)
+    w = (torch.randn(H * 256, R, generator=g, device=DEV) * R ** -0.5).to(torch.bfloat16)
+    kv = torch.mm(rows[:, :R], w.t())
+    bad = {190: float("nan"), 420: float("inf"), 640: float("nan")}
+    for p, x in bad.items():
+        kv.view(count, H, 256)[p - first, :, 128:] = x                     # values only: the scores stay finite
+    kv.view(count, H, 256)[640 - first] = float("nan")
+    q = torch.randn(t, H * 192, generator=g, device=DEV).to(torch.bfloat16)
+    gate = torch.randn(t, H, generator=g, device=DEV) if gated else None
+    out, status, scale = torch.zeros(t, H * 128, device=DEV, dtype=torch.bfloat16), i32([0, 0]), 192 ** -0.5
+    tiles = i32([(0, r) for r in range(0, t, K)])
+    o.latent_prefill(q, kv, rows, out, tiles, len(tiles), i32([[0, first, 0, count]]), i32([0]), i32([t]), i32([n]), H, R, window, scale, status,
+                     gate=gate)
+    assert status.tolist() == [0, 0]
+    j = torch.arange(first, n, device=DEV)
+    i = torch.arange(past, n, device=DEV)[:, None]
+    see = (j <= i) & ((i - j < window) if window else True)
+    spoiled = torch.stack([see[:, p - first] for p in bad], 1).any(1)
+    kh = kv[:n - first].view(-1, H, 256).to(F64)
+    k = torch.cat([kh[..., :128], rows[:n - first, None, R:].to(F64).expand(-1, H, 64)], -1).nan_to_num(0.0)
+    s = torch.einsum("thd,shd->hts", q.view(t, H, 192).to(F64), k) * scale
+    p = torch.softmax(s.masked_fill(~see, float("-inf")), -1)
+    v = kh[..., 128:].nan_to_num(0.0, 0.0, 0.0)
+    ref, bound = torch.einsum("hts,shd->thd", p, v), 2 ** -8 * torch.einsum("hts,shd->thd", p, v.abs())
+    if gated:
+        ref, bound = (x * torch.sigmoid(gate.to(F64))[:, :, None] for x in (ref, bound))
+    got = out.view(t, H, 128).to(F64)
+    assert not bool(torch.isfinite(got[spoiled]).any())
+    assert bool(((got - ref).abs() <= bound + 2 ** -8 * ref.abs() + 1e-3)[~spoiled].all()) and int((~spoiled).sum()) > 60
