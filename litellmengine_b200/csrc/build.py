@@ -52,7 +52,7 @@ FAMILIES: Dict[str, List[str]] = {
     "host_core": ["host_core.cpp"],            # the host side's bookkeeping: plain C++, no device code
 }
 HOST_FAMILIES = {"host_core"}
-HEADERS = ["common.cuh", "mma_tiles.cuh", "tcgen05_attention.cuh", "attention_decode_noalloc.h", "attention_decode_tma.cuh"]
+HEADERS = ["common.cuh", "mma_tiles.cuh", "split_mma.cuh", "tcgen05_attention.cuh", "attention_decode_noalloc.h", "attention_decode_tma.cuh"]
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-lineinfo", "-std=c++17",

@@ -22,11 +22,14 @@ class ScanWork(StepPrelude):
     the request's state.  A longer portion is cut into chunks of `CHUNK` tokens that run side by side:
     every chunk first computes its own contribution from a zero state, a chain kernel then walks each
     entry's chunks in order to find the state that enters each, and a second pass over the chunks
-    produces the outputs.  Items are int32 (entry, first row, tokens, scratch index); chains (entry,
+    produces the outputs.  The line lies where the three passes take less time than the one, for every kind of
+    recurrence (one entry, 16 heads of 128 x 128, one pass and three in us: decays per channel, 96 tokens 37 and 37,
+    128 49 and 37, 200 83 and 37; one decay per head, 100 79 and 86, 128 96 and 86, 200 148 and 86; with a
+    normaliser 91 and 101, 111 and 101, 170 and 101).  Items are int32 (entry, first row, tokens, scratch index); chains (entry,
     first scratch index, chunks)."""
     name = "scan_work"
     CHUNK = 64
-    CHUNKED_FROM = 256
+    CHUNKED_FROM = 128
 
     @dataclass
     class Views:
@@ -36,6 +39,12 @@ class ScanWork(StepPrelude):
         num_short: int
         num_chunks: int
         num_chains: int
+        longest_short: int = -1      # tokens of the longest entry that runs in one pass, once somebody has asked
+
+        def longest(self, batch) -> int:
+            if self.longest_short < 0:
+                self.longest_short = max((n for n in (len(e.tokens) for e in batch.entries) if n < ScanWork.CHUNKED_FROM), default=0)
+            return self.longest_short
 
     def sections(self, max_tokens: int, max_entries: int):
         return {"short": 4 * max_entries, "chunks": 4 * (max_tokens // self.CHUNK + max_entries),
@@ -160,10 +169,10 @@ class GatedLinearAttention(BranchMixer):
                   b.entry_q_start, b.entry_q_len)
         work = b.preludes.get(ScanWork.name)
         if work is None:                                     # no work lists: every entry in one pass
-            ops.gla_scan(*common, None, b.num_entries, ops.GLA_FULL, None, None, H, D, V)
+            ops.gla_scan(*common, None, b.num_entries, ops.GLA_FULL, None, None, H, D, V, longest=b.max_q_len)
             return
         if work.num_short:
-            ops.gla_scan(*common, work.short, work.num_short, ops.GLA_FULL, None, None, H, D, V)
+            ops.gla_scan(*common, work.short, work.num_short, ops.GLA_FULL, None, None, H, D, V, longest=work.longest(b))
         if work.num_chunks:
             scratch_s = torch.empty((work.num_chunks, H, D, V), dtype=torch.float32, device=proj.device)
             scratch_a = torch.empty((work.num_chunks, H, D), dtype=torch.float32, device=proj.device)
