@@ -404,40 +404,71 @@ __global__ void latent_gather_kernel(const bf16* __restrict__ rows_cache, long l
 }
 
 // One block a token: q float32 [T, H * (D + P)] -> bfloat16 of the same layout, the first `dims` entries of every head's
-// P-part rotated (pairs as in latent_attention.cu).  The angles of a token are made once for all heads.
-__global__ void latent_q_pack_kernel(const float* __restrict__ q, bf16* __restrict__ out, const int32_t* __restrict__ positions,
+// P-part rotated (pairs as in latent_attention.cu).  The angles of a token are made once for all heads.  2,000 tokens of 32 heads of
+// 128 + 64: 20 -> 16 us with four heads of a thread on their way before the angles are made.
+#define LQ_HELD 4
+__global__ void __launch_bounds__(1024) latent_q_pack_kernel(const float* __restrict__ q, bf16* __restrict__ out, const int32_t* __restrict__ positions,
                                      const float* __restrict__ inv_freq, int H, int D, int P, int dims, int rot_pairs, float rot_mag) {
     pdl_begin();
     extern __shared__ float2 turn[];                              // (cos, sin) of the token's angles, times the magnitude
     const int t = blockIdx.x, half = dims / 2, W = D + P;
-    const float pos = static_cast<float>(positions[t]);
-    for (int f = threadIdx.x; f < half; f += blockDim.x) {
-        float sn, cs;
-        sincosf(pos * inv_freq[f], &sn, &cs);
-        turn[f] = make_float2(cs * rot_mag, sn * rot_mag);
-    }
-    __syncthreads();
     const float* src = q + static_cast<size_t>(t) * H * W;
     bf16* dst = out + static_cast<size_t>(t) * H * W;
-    for (int i = threadIdx.x; i < H * (W / 8); i += blockDim.x) {
-        const int h = i / (W / 8), c = (i - h * (W / 8)) * 8;
-        const float* hd = src + h * W;
-        float v[8];
-        load8(hd + c, v);
-        if (c >= D) {
+    // a thread keeps its place in the head and goes from head to head, LQ_HELD heads on their way at once
+    const int per = blockDim.x / (W / 8), c = static_cast<int>(threadIdx.x % (W / 8)) * 8, k0 = c - D, h0 = threadIdx.x / (W / 8);
+    const bool whole = k0 >= 0 && k0 + 8 <= dims && (rot_pairs || half % 8 == 0);      // all eight turn, with neighbours or with eight others
+    const bool first = k0 < half;
+    const int f0 = rot_pairs ? k0 >> 1 : first ? k0 : k0 - half;
+    for (int hb = h0; hb < H || hb == h0; hb += LQ_HELD * per) {
+        float v[LQ_HELD][8];
 #pragma unroll
-            for (int u = 0; u < 8; ++u) {
-                const int k = c - D + u;
-                if (k < dims) {
-                    const bool first = rot_pairs ? (k & 1) == 0 : k < half;
-                    const int f = rot_pairs ? k >> 1 : (first ? k : k - half);
-                    const float other = hd[D + (rot_pairs ? k ^ 1 : (first ? k + half : k - half))];
-                    const float2 cs = turn[f];
-                    v[u] = first ? v[u] * cs.x - other * cs.y : v[u] * cs.x + other * cs.y;
+        for (int j = 0; j < LQ_HELD; ++j)
+            if (hb + j * per < H) load8(src + (hb + j * per) * W + c, v[j]);
+        if (hb == h0) {
+            const float pos = static_cast<float>(positions[t]);
+            for (int f = threadIdx.x; f < half; f += blockDim.x) {
+                float sn, cs;
+                sincosf(pos * inv_freq[f], &sn, &cs);
+                turn[f] = make_float2(cs * rot_mag, sn * rot_mag);
+            }
+            __syncthreads();
+        }
+#pragma unroll
+        for (int j = 0; j < LQ_HELD; ++j) {
+            const int h = hb + j * per;
+            if (h >= H) break;
+            const float* hd = src + h * W;
+            if (whole && rot_pairs) {
+#pragma unroll
+                for (int u = 0; u < 8; u += 2) {
+                    const float2 cs = turn[f0 + (u >> 1)];
+                    const float x = v[j][u], y = v[j][u + 1];
+                    v[j][u] = x * cs.x - y * cs.y;
+                    v[j][u + 1] = y * cs.x + x * cs.y;
+                }
+            } else if (whole) {
+                float other[8];
+                load8(hd + c + (first ? half : -half), other);
+#pragma unroll
+                for (int u = 0; u < 8; ++u) {
+                    const float2 cs = turn[f0 + u];
+                    v[j][u] = first ? v[j][u] * cs.x - other[u] * cs.y : v[j][u] * cs.x + other[u] * cs.y;
+                }
+            } else if (k0 >= 0) {
+#pragma unroll
+                for (int u = 0; u < 8; ++u) {
+                    const int k = k0 + u;
+                    if (k < dims) {
+                        const bool low = rot_pairs ? (k & 1) == 0 : k < half;
+                        const int f = rot_pairs ? k >> 1 : (low ? k : k - half);
+                        const float other = hd[D + (rot_pairs ? k ^ 1 : (low ? k + half : k - half))];
+                        const float2 cs = turn[f];
+                        v[j][u] = low ? v[j][u] * cs.x - other * cs.y : v[j][u] * cs.x + other * cs.y;
+                    }
                 }
             }
+            store8(dst + h * W + c, v[j]);
         }
-        store8(dst + h * W + c, v);
     }
 }
 
@@ -465,7 +496,9 @@ extern "C" int llm_latent_q_pack(const float* q, void* out, const int32_t* posit
     if (num_tokens <= 0) return LLM_OK;
     if (H <= 0 || D <= 0 || P < 0 || D % 8 || P % 8 || dims < 0 || dims > P || dims % 2 || (dims > 0 && !inv_freq)) return LLM_REFUSED_SIZE;
     if (!aligned16(q) || !aligned16(out)) return LLM_REFUSED_ALIGN;
-    launch_pdl(latent_q_pack_kernel, dim3(num_tokens), dim3(256), sizeof(float2) * (dims / 2), reinterpret_cast<cudaStream_t>(stream),
+    const int eights = (D + P) / 8;                               // threads: as many whole heads as 256 of them hold
+    if (eights > 1024) return LLM_REFUSED_SIZE;
+    launch_pdl(latent_q_pack_kernel, dim3(num_tokens), dim3(eights > 256 ? eights : 256 / eights * eights), sizeof(float2) * (dims / 2), reinterpret_cast<cudaStream_t>(stream),
                q, static_cast<bf16*>(out), positions, inv_freq, H, D, P, dims, rot_pairs, rot_mag);
     return launch_status();
 }
