@@ -42,7 +42,8 @@
 // p - 1 .. p - taps + 1 and writes row p mod taps, which is none of those, so in a decode step blocks that share a
 // key head may read the ring while one of them writes it.
 #include "common.cuh"
-#include "mma_tiles.cuh"
+#include "split_mma.cuh"
+#include "tcgen05_attention.cuh"
 
 #define DR_TB 16            // tokens staged at a time
 #define DR_CHUNK 8          // tokens that go through the state together
@@ -544,6 +545,29 @@ template <int C> __device__ __forceinline__ void dr_row(float (&v)[C], const flo
     }
 }
 
+// The convolutions' inputs of a portion's last tokens go into the request's ring (the kernels before the scan have read it): by each
+// block of a scan its columns' values, and the head's queries and keys by one.
+__device__ __forceinline__ void dr_keep_inputs(const DeltaShape& s, const float* __restrict__ proj, float* slot, const int32_t* __restrict__ positions,
+                                               long long row0, int count, int h, int c0, int cols, bool first) {
+    const int channels = 2 * s.G * s.D + s.H * s.V, keep = min(count, s.taps - 1), kvh = h / (s.H / s.G);
+    float* ring = slot + s.ring_off;
+    const bool with_qk = first && h % (s.H / s.G) == 0;
+    for (int i = 0; i < keep; ++i) {
+        const long long t = row0 + count - keep + i;
+        float* dst = ring + static_cast<long long>(positions[t] % s.taps) * channels;
+        const float* src = proj + t * s.stride + s.q_off;
+        if (with_qk)
+            for (int d = threadIdx.x; d < s.D; d += blockDim.x) {
+                dst[kvh * s.D + d] = src[kvh * s.D + d];
+                dst[(s.G + kvh) * s.D + d] = src[(s.G + kvh) * s.D + d];
+            }
+        for (int x = threadIdx.x; x < cols && c0 + x < s.V; x += blockDim.x) {
+            const int ch = 2 * s.G * s.D + h * s.V + c0 + x;
+            dst[ch] = src[ch];
+        }
+    }
+}
+
 // grid: entries (longest portion first) x H x column tiles, the tiles fastest: WARPS warps a block, each 32 / L groups of C columns.
 template <int DP, int C, int WARPS, int L>
 __global__ void __launch_bounds__(WARPS * 32) delta_scan_kernel(
@@ -738,27 +762,484 @@ __global__ void __launch_bounds__(WARPS * 32) delta_scan_kernel(
 #pragma unroll
             for (int j = 0; j < R / 4; ++j)
                 *reinterpret_cast<float4*>(col_state + m * DP + 4 * L * j) = make_float4(S[m][4 * j], S[m][4 * j + 1], S[m][4 * j + 2], S[m][4 * j + 3]);
-    // the convolutions' inputs of the portion's last tokens (the kernels before this one have read the ring)
-    const int channels = 2 * s.G * s.D + s.H * s.V, keep = min(count, s.taps - 1), kvh = h / (s.H / s.G);
-    float* ring = slot + s.ring_off;
-    const bool with_qk = tile == 0 && h % (s.H / s.G) == 0;
-    for (int i = 0; i < keep; ++i) {
-        const long long t = row0 + count - keep + i;
-        float* dst = ring + static_cast<long long>(positions[t] % s.taps) * channels;
-        const float* src = proj + t * s.stride + s.q_off;
-        if (with_qk)
-            for (int d = tid; d < s.D; d += THREADS) {
-                dst[kvh * s.D + d] = src[kvh * s.D + d];
-                dst[(s.G + kvh) * s.D + d] = src[(s.G + kvh) * s.D + d];
-            }
-        for (int x = tid; x < COLS && c0 + x < s.V; x += THREADS) {
-            const int ch = 2 * s.G * s.D + h * s.V + c0 + x;
-            dst[ch] = src[ch];
-        }
-    }
+    dr_keep_inputs(s, proj, slot, positions, row0, count, h, c0, COLS, tile == 0);
 }
 
 // A warp per (token, head): o / rms(o) * w * gate * scale.
+// ---- states of 128 rows on the tensor cores -------------------------------------------------------------------------
+// The same recurrence, sixteen tokens at a time, as products: with X = V - (p k) S (tokens by columns),
+//
+//     U = T X       O = (p q) S + B U       S <- p_15 S + (s k)^T U              T = (1 + diag(beta) A)^-1 diag(beta)
+//
+// All factors are products of decays, none is divided by one, whatever the decays are: A and B are made of dot products whose
+// decays from j to i are cut in the middle of the smallest of the batch's halves, quarters, eighths and pairs that holds both,
+// what lies before the cut with k_j, what lies behind with k_i or q_i.  Products of float32 values are sums of six bfloat16 products
+// (split_mma.cuh); the state stays in float32 accumulators, transposed, and takes a batch's contribution with rounded
+// additions.
+//
+//   delta_batch_kernel   a block per (sixteen tokens, head): an image of what all columns of the head share, just as the scan
+//                        wants it in shared memory: planes of p k, p q, s k, of T and B, then p_15 and the mark
+//   delta_scan_mma_kernel  a block per (entry, head, 32 columns), eight warps: 16 columns by 32 rows of the state each.  The
+//                        shares of X and O over the rows go through shared memory; every warp then makes the U of its columns itself.
+//
+// A batch that holds something not finite or very large is marked with its first such token.  The scan makes what is before it as
+// always, with nothing in the place of what follows (a weight of zero times an infinity is NaN), and then walks through the batch
+// token by token for the outputs from the mark on and the state.
+// What bounds it: a batch's chain, 3,700 clocks: 48 small products a warp over the state (1,000), shares and X (700), U (300), the state
+// (600), the outputs of two warps (600) and the waits in between; the tensor pipe would take 1,450.  Portions of 284, 567 and 849
+// tokens, 16 heads of 128 x 128 (us): the scan 160 -> 107, what it shares 24 -> 46 (dot products and the writing of 76 MB).
+// Error against 64 bits (2-norm; outputs and states): 1.61e-7 and 1.56e-7, the kernels of eight tokens 1.60e-7 and 1.57e-7.
+#define DX_T 16
+#define DX_PITCH 136                 // of a row of a plane: eight rows of 16 bytes fall into all banks
+#define DX_PLANE (DX_T * DX_PITCH)
+#define DX_NP 24                     // of a row of T or B
+#define DX_NPLANE (DX_T * DX_NP)
+#define DX_IMAGE (2 * (9 * DX_PLANE + 6 * DX_NPLANE) + 4 * 128 + 16)       // bytes
+#define DX_MOST 1.0737418e9f         // 2^30
+#define DX_LP 132                    // of a row of a level's vectors
+#define DX_ROWS (4 * 4 * 24 * DX_LP) // bytes of the four levels' vectors
+#define DX_BATCH_SMEM (DX_ROWS + 4 * (512 + 32))
+#define DX_STATUS 11
+
+// Where a batch's image is: batches start at every sixteenth row of an entry.
+__device__ __forceinline__ long long dx_place(long long row, int entry) { return row / DX_T + entry; }
+
+__global__ void __launch_bounds__(128) delta_batch_kernel(
+    const DeltaShape s, const float* __restrict__ qn, const float* __restrict__ kn, const float* __restrict__ vn, const float* __restrict__ beta,
+    const float* __restrict__ decay, unsigned char* __restrict__ images, const int32_t* __restrict__ entry_q_start,
+    const int32_t* __restrict__ entry_q_len, int num_entries) {
+    pdl_wait();                      // no early invitation: see delta_chunk_kernel
+    constexpr int D = 128;
+    const int h = blockIdx.y, tid = threadIdx.x, kvh = h / (s.H / s.G);
+    int entry = -1, first = 0, nt = 0;                                      // the entry that has a batch in this place, if any
+    for (int e0 = 0; e0 < num_entries && entry < 0; e0 += 32) {
+        const int e = e0 + (tid & 31);
+        int m = -1, left = 0;
+        if (e < num_entries) {
+            m = static_cast<int>(blockIdx.x) - static_cast<int>(dx_place(entry_q_start[e], e));
+            left = entry_q_len[e] - DX_T * m;
+        }
+        const unsigned found = __ballot_sync(0xffffffffu, m >= 0 && left > 0);
+        if (found) {
+            const int at = __ffs(found) - 1;
+            entry = e0 + at;
+            first = __shfl_sync(0xffffffffu, m, at) * DX_T;
+            nt = min(DX_T, __shfl_sync(0xffffffffu, left, at));
+        }
+    }
+    if (entry < 0) return;
+    const long long t = entry_q_start[entry] + first;
+    extern __shared__ __align__(16) unsigned char dx_smem[];
+    bf16* planes = reinterpret_cast<bf16*>(dx_smem);                        // [p k, p q, s k][3][16][136]
+    bf16* small = planes + 9 * DX_PLANE;                                    // [T, B][3][16][24]
+    float* total = reinterpret_cast<float*>(small + 6 * DX_NPLANE);         // [128], then the mark
+    float* rows = reinterpret_cast<float*>(dx_smem);                        // before the planes: [4 levels][24][132], k_i, q_i, then k_j
+    float* nums = reinterpret_cast<float*>(dx_smem + DX_ROWS);              // A [16][16], then B [16][16]
+    float* shares = nums + 512;                                             // [4 warps][8 tokens]: q_i k_i
+    __shared__ unsigned marks[4];
+    // a thread: channels c and c + 1 of tokens 8 hf .. 8 hf + 7 (and the decays of all)
+    const int c = 2 * (tid & 63), hf = tid >> 6, lane = tid & 31;
+    {
+        float2 k[8], q[8], g[DX_T];
+        const float2 zero = make_float2(0.0f, 0.0f), one = make_float2(1.0f, 1.0f);
+        const float* gp = decay + (static_cast<size_t>(t) * s.H + h) * D + c;
+        const size_t at = (static_cast<size_t>(t + 8 * hf) * s.G + kvh) * D + c;
+#pragma unroll
+        for (int i = 0; i < DX_T; ++i) g[i] = i < nt ? *reinterpret_cast<const float2*>(gp + static_cast<size_t>(i) * s.H * D) : one;      // a missing token
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            k[i] = 8 * hf + i < nt ? *reinterpret_cast<const float2*>(kn + at + static_cast<size_t>(i) * s.G * D) : zero;
+            q[i] = 8 * hf + i < nt ? *reinterpret_cast<const float2*>(qn + at + static_cast<size_t>(i) * s.G * D) : zero;
+        }
+        unsigned bad = 0;                                                   // tokens that are not finite or very large
+        for (int x = 4 * lane; x < s.V; x += 128)                           // a warp four tokens' values
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const int tok = 4 * (tid >> 5) + i;
+                if (tok < nt) {
+                    const float4 v = *reinterpret_cast<const float4*>(vn + (static_cast<size_t>(t + tok) * s.H + h) * s.VP + x);
+                    if (!(fabsf(v.x) <= DX_MOST && fabsf(v.y) <= DX_MOST && fabsf(v.z) <= DX_MOST && fabsf(v.w) <= DX_MOST)) bad |= 1u << tok;
+                }
+            }
+        if (tid < nt && !(fabsf(beta[static_cast<size_t>(t + tid) * s.H + h]) <= 1.0f)) bad |= 1u << tid;
+#pragma unroll
+        for (int i = 0; i < DX_T; ++i)
+            if (!(g[i].x >= 0.0f && g[i].x <= 1.0f && g[i].y >= 0.0f && g[i].y <= 1.0f)) bad |= 1u << i;
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+            if (!(fabsf(k[i].x) <= 2.0f && fabsf(k[i].y) <= 2.0f && fabsf(q[i].x) <= 2.0f && fabsf(q[i].y) <= 2.0f)) bad |= 1u << (8 * hf + i);
+        bad = __reduce_or_sync(0xffffffffu, bad);
+        if (lane == 0) marks[tid >> 5] = bad;
+        for (int i = tid; i < 512; i += 128) nums[i] = 0.0f;
+        // halves of 16, 8, 4 and 2 tokens: `half` tokens either side of a cut
+        auto row = [&](int level, int r) -> float2& { return *reinterpret_cast<float2*>(rows + (24 * level + r) * DX_LP + c); };
+        auto times = [](float2 a, float2 b) { return make_float2(a.x * b.x, a.y * b.y); };
+        if (hf) {
+            float2 f = one;
+#pragma unroll
+            for (int m = 0; m < 8; ++m) {
+                f = times(f, g[8 + m]);
+                row(0, m) = times(f, k[m]);
+                row(0, 8 + m) = times(f, q[m]);
+            }
+        } else {
+            float2 b = one;
+#pragma unroll
+            for (int m = 7; m >= 0; --m) {
+                row(0, 16 + m) = times(b, k[m]);
+                b = times(b, g[m]);
+            }
+        }
+#pragma unroll
+        for (int level = 1; level < 4; ++level) {
+            const int half = 8 >> level;
+#pragma unroll
+            for (int cut = half; cut < 8; cut += 2 * half) {                // of this thread's eight tokens
+                const int base = 4 * hf + (cut - half) / 2;
+                float2 f = one, b = one;
+#pragma unroll
+                for (int m = 0; m < half; ++m) {
+                    f = times(f, hf ? g[8 + cut + m] : g[cut + m]);
+                    row(level, base + m) = times(f, k[cut + m]);
+                    row(level, 8 + base + m) = times(f, q[cut + m]);
+                    row(level, 16 + base + half - 1 - m) = times(b, k[cut - 1 - m]);
+                    b = times(b, hf ? g[8 + cut - 1 - m] : g[cut - 1 - m]);
+                }
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const float x = warp_sum(q[i].x * k[i].x + q[i].y * k[i].y);
+            if (lane == 0) shares[(tid >> 5) * 8 + i] = x;
+        }
+        __syncthreads();
+        // A's and B's dot products of a pair of tokens share its k_j: 64, 32, 16 and 8 pairs a level
+        if (tid < 120) {
+            const int level = tid < 64 ? 0 : tid < 96 ? 1 : tid < 112 ? 2 : 3, half = 8 >> level, n = tid - (128 - (128 >> level));
+            const int i = n / half, j = n % half, base = i / half * half;       // i: row of all eight
+            const float* ka = rows + (24 * level + i) * DX_LP;
+            const float* qa = ka + 8 * DX_LP;
+            const float* b = rows + (24 * level + 16 + base + j) * DX_LP;
+            float2 x0 = zero, x1 = zero, y0 = zero, y1 = zero;
+#pragma unroll 8
+            for (int d = 0; d < D; d += 4) {
+                const float4 u = *reinterpret_cast<const float4*>(ka + d), w = *reinterpret_cast<const float4*>(qa + d), v = *reinterpret_cast<const float4*>(b + d);
+                x0.x = fmaf(u.x, v.x, x0.x); x0.y = fmaf(u.y, v.y, x0.y); x1.x = fmaf(u.z, v.z, x1.x); x1.y = fmaf(u.w, v.w, x1.y);
+                y0.x = fmaf(w.x, v.x, y0.x); y0.y = fmaf(w.y, v.y, y0.y); y1.x = fmaf(w.z, v.z, y1.x); y1.y = fmaf(w.w, v.w, y1.y);
+            }
+            const int to = 16 * (2 * base + half + i % half) + 2 * base + j;
+            nums[to] = (x0.x + x0.y) + (x1.x + x1.y);
+            nums[256 + to] = (y0.x + y0.y) + (y1.x + y1.y);
+        }
+        if (tid < DX_T) nums[256 + 17 * tid] = shares[2 * (tid >> 3) * 8 + (tid & 7)] + shares[(2 * (tid >> 3) + 1) * 8 + (tid & 7)];
+        __syncthreads();                                                    // the planes take the rows' place
+        auto put = [&](int which, int i, float2 v) {
+#pragma unroll
+            for (int p = 0; p < 3; ++p) *reinterpret_cast<unsigned*>(planes + (which * 3 + p) * DX_PLANE + i * DX_PITCH + c) = split_piece(v.x, v.y);
+        };
+        float2 p = one, e = one;
+        if (hf) {
+#pragma unroll
+            for (int i = 0; i < 8; ++i) p = times(p, g[i]);
+        } else {
+#pragma unroll
+            for (int i = 15; i >= 8; --i) e = times(e, g[i]);
+        }
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            p = times(p, hf ? g[8 + i] : g[i]);
+            put(0, 8 * hf + i, times(p, k[i]));
+            put(1, 8 * hf + i, times(p, q[i]));
+        }
+        if (hf) *reinterpret_cast<float2*>(total + c) = p;
+#pragma unroll
+        for (int i = 7; i >= 0; --i) {
+            put(2, 8 * hf + i, times(e, k[i]));
+            e = times(e, hf ? g[8 + i] : g[i]);
+        }
+        const unsigned any = marks[0] | marks[1] | marks[2] | marks[3];
+        if (tid < 4) reinterpret_cast<int*>(total + D)[tid] = any ? __ffs(any) - 1 : DX_T;
+    }
+    auto put_small = [&](int which, int i, int j, float v) {
+        float rest = 0.0f;
+#pragma unroll
+        for (int p = 0; p < 3; ++p) reinterpret_cast<unsigned short*>(small)[(which * 3 + p) * DX_NPLANE + i * DX_NP + j] = static_cast<unsigned short>(split_piece(v, rest));
+    };
+    if (tid < DX_T) {                                // column `tid` of T: rows in order
+        float x[DX_T];
+#pragma unroll
+        for (int i = 0; i < DX_T; ++i) {
+            const float be = i < nt ? beta[static_cast<size_t>(t + i) * s.H + h] : 0.0f;
+            float v = i == tid ? 1.0f : 0.0f, w = 0.0f;
+#pragma unroll
+            for (int m = 0; m < i; ++m) (m & 1 ? w : v) -= nums[16 * i + m] * x[m];
+            x[i] = i < tid ? 0.0f : be * (v + w);
+            put_small(0, i, tid, x[i]);
+        }
+    } else if (tid >= 32) {
+        for (int idx = tid - 32; idx < 256; idx += 96) put_small(1, idx >> 4, idx & 15, nums[256 + idx]);
+    }
+    __syncthreads();
+    uint4* to = reinterpret_cast<uint4*>(images + (static_cast<size_t>(blockIdx.x) * s.H + h) * DX_IMAGE);
+    for (int i = tid; i < DX_IMAGE / 16; i += 128) to[i] = reinterpret_cast<const uint4*>(dx_smem)[i];
+}
+
+// grid: entries (longest portion first) x H x column tiles of 32, the tiles fastest.
+#define DX_COLS 32
+#define DX_SMEM (2 * DX_IMAGE + 8 * 4 * 32 * 16)
+__global__ void __launch_bounds__(256, 2) delta_scan_mma_kernel(
+    const DeltaShape s, const float* __restrict__ proj, const unsigned char* __restrict__ images, const float* __restrict__ qn,
+    const float* __restrict__ kn, const float* __restrict__ vn, const float* __restrict__ beta, const float* __restrict__ decay,
+    float* __restrict__ o, float* __restrict__ state, const int32_t* __restrict__ positions, const int32_t* __restrict__ entry_slot,
+    const int32_t* __restrict__ entry_q_start, const int32_t* __restrict__ entry_q_len, int num_entries, int tiles, int32_t* __restrict__ status) {
+    pdl_begin();
+    constexpr int D = 128;
+    extern __shared__ __align__(16) unsigned char dx_smem[];
+    float4* shares = reinterpret_cast<float4*>(dx_smem + 2 * DX_IMAGE);      // [8 warps][X 2, O 2][32 lanes]
+    __shared__ __align__(8) unsigned long long full[2];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, lg = lane >> 2, lt = lane & 3;
+    const int tile = blockIdx.x % tiles, c0 = tile * DX_COLS, h = blockIdx.x / tiles % s.H, kvh = h / (s.H / s.G);
+    int entry = blockIdx.x / (tiles * s.H);
+    if (num_entries <= 32) {                                    // longest portions first: the entry with `entry` ones before it
+        const int mine = lane < num_entries ? entry_q_len[lane] : -1;
+        int before = 0;
+        for (int e = 0; e < num_entries; ++e) {
+            const int len = __shfl_sync(0xffffffffu, mine, e);
+            before += len > mine || (len == mine && e < lane);
+        }
+        entry = __ffs(__ballot_sync(0xffffffffu, before == entry && lane < num_entries)) - 1;
+    }
+    const long long row0 = entry_q_start[entry];
+    const int count = entry_q_len[entry];
+    float* slot = state + entry_slot[entry] * s.slot_stride;
+    // a warp: columns c0 + 16 (warp / 4) .. + 15, rows 32 (warp % 4) .. + 31; tile n, element i: column v0 + 8 (i >> 1), row d0 + 8 n + (i & 1)
+    const int group = warp >> 2, v0 = c0 + 16 * group + lg, dw = 32 * (warp & 3), d0 = dw + 2 * lt;
+    float* my_state = slot + (static_cast<long long>(h) * s.V + v0) * D + d0;
+    float S[4][4];
+    bool bad_state = false;
+    auto look = [&]() {
+        bad_state = false;
+#pragma unroll
+        for (int n = 0; n < 4; ++n)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) bad_state |= !(fabsf(S[n][i]) < 1.1529215e18f);      // 2^60
+    };
+#pragma unroll
+    for (int n = 0; n < 4; ++n) {
+        const float2 lo = *reinterpret_cast<const float2*>(my_state + 8 * n), hi = *reinterpret_cast<const float2*>(my_state + 8 * D + 8 * n);
+        S[n][0] = lo.x; S[n][1] = lo.y; S[n][2] = hi.x; S[n][3] = hi.y;
+    }
+    look();
+    if (tid == 0) {
+        t5_mbar_init(&full[0], 1);
+        t5_mbar_init(&full[1], 1);
+        asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+    }
+    bool bad = __syncthreads_or(bad_state);
+    const unsigned char* image = images + (static_cast<size_t>(dx_place(row0, entry)) * s.H + h) * DX_IMAGE;
+    const size_t image_step = static_cast<size_t>(s.H) * DX_IMAGE;
+    auto stage = [&](int b) {                                   // one copy for the whole image: by sixteen bytes a thread it took 1,800 clocks to issue
+        if (tid == 0) {
+            t5_expect_tx(&full[b], DX_IMAGE);
+            asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n" ::
+                             "r"(t5_smem(dx_smem + b * DX_IMAGE)), "l"(image), "r"(DX_IMAGE), "r"(t5_smem(&full[b])) : "memory");
+        }
+        image += image_step;
+    };
+    auto landed = [&](int b, unsigned parity) {
+        for (int i = 0; i < T5_WAIT_LIMIT; ++i)
+            if (t5_try_wait(&full[b], parity)) return true;
+        return false;
+    };
+    // values of (column v0 + 8 (i >> 1), token 8 u + 2 lt + (i & 1))
+    const float* my_v = vn + (static_cast<size_t>(row0) * s.H + h) * s.VP + v0;
+    const int v_step = s.H * s.VP;
+    const float* next_v = my_v + static_cast<size_t>(2 * lt) * v_step;
+    float v[2][4];
+    auto fetch = [&](int done) {
+#pragma unroll
+        for (int u = 0; u < 2; ++u)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) v[u][i] = done + 8 * u + 2 * lt + (i & 1) < count ? next_v[(8 * u + (i & 1)) * v_step + 8 * (i >> 1)] : 0.0f;
+        next_v += static_cast<size_t>(DX_T) * v_step;
+    };
+    const int frow = (lane >> 4) * 8 + (lane & 7), fcol = ((lane >> 3) & 1) * 8;
+    const int grow = fcol + (lane & 7), gcol = (lane >> 4) * 8;
+    constexpr int A[6] = {2, 0, 1, 1, 0, 0}, B[6] = {0, 2, 1, 0, 1, 0};          // planes of the six products, the smallest first
+    stage(0);
+    fetch(0);
+    for (int done = 0, b = 0; done < count; done += DX_T, b ^= 1) {
+        const int nb = min(DX_T, count - done);
+        if (__syncthreads_or(!landed(b, (done / (2 * DX_T)) & 1))) {         // (never: the copy did not land in time)
+            if (tid == 0 && atomicCAS(status, 0, DX_STATUS) == 0) status[1] = blockIdx.x;
+            return;
+        }
+        if (done + DX_T < count) stage(b ^ 1);
+        const bf16* planes = reinterpret_cast<const bf16*>(dx_smem + b * DX_IMAGE);
+        const bf16* small = planes + 9 * DX_PLANE;
+        const float* total = reinterpret_cast<const float*>(small + 6 * DX_NPLANE);
+        float* oo = o + (static_cast<size_t>(row0 + done) * s.H + h) * s.V + v0;
+        const size_t o_step = static_cast<size_t>(s.H) * s.V;
+        const int good = bad ? 0 : *reinterpret_cast<const int*>(total + D);      // tokens in front of the mark
+        // shares of (p k) S and (p q) S over this warp's rows
+        float rm[2][4], rs[2][4], xm[2][4], xs[2][4];
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+            unsigned a[3][4], yk[3][4], yq[3][4];
+#pragma unroll
+            for (int p = 0; p < 3; ++p) {
+                ldmatrix_x4(yk[p], planes + p * DX_PLANE + frow * DX_PITCH + dw + 16 * j + fcol);
+                ldmatrix_x4(yq[p], planes + (3 + p) * DX_PLANE + frow * DX_PITCH + dw + 16 * j + fcol);
+            }
+            split_tiles(S[2 * j], S[2 * j + 1], a);
+#pragma unroll
+            for (int i = 0; i < 6; ++i)              // four sums side by side
+#pragma unroll
+                for (int w = 0; w < 4; ++w) {
+                    const int u = w & 1;
+                    float (&c)[4] = w < 2 ? (i < 5 ? rs[u] : rm[u]) : (i < 5 ? xs[u] : xm[u]);
+                    const unsigned b0 = w < 2 ? yk[B[i]][2 * u] : yq[B[i]][2 * u], b1 = w < 2 ? yk[B[i]][2 * u + 1] : yq[B[i]][2 * u + 1];
+                    if (j == 0 && (i == 0 || i == 5)) mma_bf16_first(c, a[A[i]], b0, b1);
+                    else mma_bf16(c, a[A[i]], b0, b1);
+                }
+        }
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+            shares[(warp * 4 + u) * 32 + lane] = make_float4(rm[u][0] + rs[u][0], rm[u][1] + rs[u][1], rm[u][2] + rs[u][2], rm[u][3] + rs[u][3]);
+            shares[(warp * 4 + 2 + u) * 32 + lane] = make_float4(xm[u][0] + xs[u][0], xm[u][1] + xs[u][1], xm[u][2] + xs[u][2], xm[u][3] + xs[u][3]);
+        }
+        __syncthreads();
+        auto over_rows = [&](int which) {            // the four warps' shares, in the same order whoever adds them
+            float4 x[4];
+#pragma unroll
+            for (int w = 0; w < 4; ++w) x[w] = shares[((4 * group + w) * 4 + which) * 32 + lane];
+            return make_float4((x[0].x + x[1].x) + (x[2].x + x[3].x), (x[0].y + x[1].y) + (x[2].y + x[3].y),
+                               (x[0].z + x[1].z) + (x[2].z + x[3].z), (x[0].w + x[1].w) + (x[2].w + x[3].w));
+        };
+        auto before_mark = [&](float (&c)[2][4]) {
+            if (good < DX_T)
+#pragma unroll
+                for (int u = 0; u < 2; ++u)
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) c[u][i] = 8 * u + 2 * lt + (i & 1) < good ? c[u][i] : 0.0f;
+        };
+        float x[2][4];
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+            const float4 r = over_rows(u);
+            x[u][0] = v[u][0] - r.x; x[u][1] = v[u][1] - r.y; x[u][2] = v[u][2] - r.z; x[u][3] = v[u][3] - r.w;
+        }
+        before_mark(x);
+        if (done + DX_T < count) fetch(done + DX_T);
+        unsigned a[3][4], y[3][4];
+        float um[2][4], us[2][4];
+        split_tiles(x[0], x[1], a);
+#pragma unroll
+        for (int p = 0; p < 3; ++p) ldmatrix_x4(y[p], small + p * DX_NPLANE + frow * DX_NP + fcol);
+        split_mma<true>(um, us, a, y);
+#pragma unroll
+        for (int u = 0; u < 2; ++u)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) um[u][i] += us[u][i];
+        before_mark(um);
+        split_tiles(um[0], um[1], a);
+        if (good == DX_T) {
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+                float c[2][4], cs[2][4];
+#pragma unroll
+                for (int p = 0; p < 3; ++p) ldmatrix_x4_trans(y[p], planes + (6 + p) * DX_PLANE + grow * DX_PITCH + dw + 16 * j + gcol);
+                split_mma<true>(c, cs, a, y);
+#pragma unroll
+                for (int u = 0; u < 2; ++u) {
+                    const float2 f = *reinterpret_cast<const float2*>(total + dw + 16 * j + 8 * u + 2 * lt);
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) S[2 * j + u][i] = fmaf(S[2 * j + u][i], i & 1 ? f.y : f.x, cs[u][i]) + c[u][i];
+                }
+            }
+        }
+        if ((warp & 3) >= 2) {                       // two warps of four make the outputs of their columns, eight tokens each
+            const int u = warp & 1;
+            float om[4], os[4];
+#pragma unroll
+            for (int p = 0; p < 3; ++p) ldmatrix_x4(y[p], small + (3 + p) * DX_NPLANE + frow * DX_NP + fcol);
+#pragma unroll
+            for (int i = 0; i < 6; ++i) {
+                const unsigned b0 = u ? y[B[i]][2] : y[B[i]][0], b1 = u ? y[B[i]][3] : y[B[i]][1];
+                if (i == 0) mma_bf16_first(os, a[A[i]], b0, b1);
+                else if (i < 5) mma_bf16(os, a[A[i]], b0, b1);
+                else mma_bf16_first(om, a[A[i]], b0, b1);
+            }
+            const float4 r = over_rows(2 + u);
+            const float out[4] = {r.x + (om[0] + os[0]), r.y + (om[1] + os[1]), r.z + (om[2] + os[2]), r.w + (om[3] + os[3])};
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const int t = 8 * u + 2 * lt + (i & 1);
+                if (t < min(nb, good)) oo[t * o_step + 8 * (i >> 1)] = out[i];
+            }
+        }
+        if (good < DX_T) {                           // token by token
+            __syncthreads();                         // the shares have been read
+            float* sums = reinterpret_cast<float*>(shares);                   // [2][4 row quarters][32 columns]
+            for (int t = 0; t < nb; ++t) {
+                const size_t row = row0 + done + t;
+                const float be = beta[row * s.H + h];
+                float2 kk[4], qq[4];
+                float r0 = 0.0f, r1 = 0.0f;
+#pragma unroll
+                for (int n = 0; n < 4; ++n) {
+                    const float2 g = *reinterpret_cast<const float2*>(decay + (row * s.H + h) * D + d0 + 8 * n);
+                    kk[n] = *reinterpret_cast<const float2*>(kn + (row * s.G + kvh) * D + d0 + 8 * n);
+                    qq[n] = *reinterpret_cast<const float2*>(qn + (row * s.G + kvh) * D + d0 + 8 * n);
+                    S[n][0] *= g.x; S[n][1] *= g.y; S[n][2] *= g.x; S[n][3] *= g.y;
+                    r0 += S[n][0] * kk[n].x + S[n][1] * kk[n].y;
+                    r1 += S[n][2] * kk[n].x + S[n][3] * kk[n].y;
+                }
+                auto all_rows = [&](float& x0, float& x1, float* to) {        // sums over the state's rows, in every warp
+#pragma unroll
+                    for (int off = 1; off <= 2; off <<= 1) {
+                        x0 += __shfl_xor_sync(0xffffffffu, x0, off);
+                        x1 += __shfl_xor_sync(0xffffffffu, x1, off);
+                    }
+                    if (lt == 0) {
+                        to[(warp & 3) * DX_COLS + v0 - c0] = x0;
+                        to[(warp & 3) * DX_COLS + v0 - c0 + 8] = x1;
+                    }
+                    __syncthreads();
+                    x0 = x1 = 0.0f;
+#pragma unroll
+                    for (int w = 0; w < 4; ++w) {
+                        x0 += to[w * DX_COLS + v0 - c0];
+                        x1 += to[w * DX_COLS + v0 - c0 + 8];
+                    }
+                };
+                all_rows(r0, r1, sums);
+                const float u0 = be * (my_v[static_cast<size_t>(done + t) * v_step] - r0), u1 = be * (my_v[static_cast<size_t>(done + t) * v_step + 8] - r1);
+                float x0 = 0.0f, x1 = 0.0f;
+#pragma unroll
+                for (int n = 0; n < 4; ++n) {
+                    S[n][0] += kk[n].x * u0; S[n][1] += kk[n].y * u0; S[n][2] += kk[n].x * u1; S[n][3] += kk[n].y * u1;
+                    x0 += S[n][0] * qq[n].x + S[n][1] * qq[n].y;
+                    x1 += S[n][2] * qq[n].x + S[n][3] * qq[n].y;
+                }
+                all_rows(x0, x1, sums + 4 * DX_COLS);
+                if (lt == 0 && (warp & 3) == 0 && t >= good) {
+                    oo[t * o_step] = x0;
+                    oo[t * o_step + 8] = x1;
+                }
+            }
+            look();
+            bad = __syncthreads_or(bad_state);
+        }
+    }
+#pragma unroll
+    for (int n = 0; n < 4; ++n) {
+        *reinterpret_cast<float2*>(my_state + 8 * n) = make_float2(S[n][0], S[n][1]);
+        *reinterpret_cast<float2*>(my_state + 8 * D + 8 * n) = make_float2(S[n][2], S[n][3]);
+    }
+    dr_keep_inputs(s, proj, slot, positions, row0, count, h, c0, DX_COLS, tile == 0);
+}
+
 template <typename TO>
 __global__ void delta_output_kernel(const float* __restrict__ o, const float* __restrict__ gate, const float* __restrict__ norm_w,
                                     float eps, float out_scale, TO* __restrict__ out, long long out_stride, int out_off, int H,
@@ -980,9 +1461,24 @@ static int delta_shape(DeltaShape& s, int H, int G, int D, int V, int taps, int 
     return LLM_OK;
 }
 
+#define DR_SMS 148
+#define DR_ALONE_SMEM (116 * 1024)
+
+// Whether llm_delta_scan takes the tensor-core kernels: it is then given room for llm_delta_image_bytes() a batch of sixteen tokens and
+// head (T / 16 + entries + 1 places) instead of pk, pq, total and num.  Their fixed part is larger, and few columns spread thinner over
+// the SMs than with a warp to one to four of them.  Whole calls (us, eight tokens a chunk and this; entries x longest portion, heads):
+// 1 x 300, 16: 93, 90; 1 x 1,000, 16: 229, 209; 1 x 2,500, 16: 535, 473; 3 x 849, 16: 265, 238, 8: 224, 185, 4: 182, 155; 3 x 300, 16:
+// 114, 114, 8: 101, 90, 4: 92, 86; but 1 x 1,000, 8: 169, 176; 1 x 2,500, 8: 382, 398; 1 x 100, 16: 60, 64; 4 x 200, 16: 123, 128; 32 x 64,
+// 16: 259, 276.  So: portions of 256 tokens and more, 1,500 columns and more, two blocks an SM at most.
+extern "C" int llm_delta_image_bytes() { return DX_IMAGE; }
+extern "C" int llm_delta_batched(int H, int D, int V, int num_entries, int max_len) {
+    const long long columns = static_cast<long long>(num_entries) * H * V;
+    return D == 128 && V > 0 && V % DX_COLS == 0 && H > 0 && H <= 65535 && max_len >= 256 && columns >= 1500 && columns <= 2 * DR_SMS * DX_COLS;
+}
+
 // Everything of a step that is not all single tokens.  Scratch (float32): qn, kn [T, G, DP], vn [T, H, VP], beta [T, H],
 // decay [T, H, DP] (whose places from D on must be finite), gate and o [T, H, V], pk and pq [T, H, DP], and for P =
-// T / 8 + entries + 1 chunks total [P, H, DP] and num [P, H, 128].
+// T / 8 + entries + 1 chunks total [P, H, DP] and num [P, H, 128]; or, in place of the last four, images (see llm_delta_batched).
 // `conv_w` [C, taps]: the rows of q, k and v one after another.  max_len: tokens of the longest entry, 0: not known.
 extern "C" int llm_delta_scan(
     const float* proj, long long stride, int q_off, int b_off, int a_off, int ra, int g_off, int rg, const float* conv_w, int taps,
@@ -990,7 +1486,8 @@ extern "C" int llm_delta_scan(
     float out_scale, void* out, int out_dtype, long long out_stride, int out_off, float* state, long long slot_stride,
     const int32_t* positions, const int32_t* token_entry, const int32_t* entry_slot, const int32_t* entry_q_start,
     const int32_t* entry_q_len, int num_tokens, int num_entries, int max_len, int H, int G, int D, int V, float* qn, float* kn,
-    float* vn, float* beta, float* decay, float* gate, float* o, float* pk, float* pq, float* total, float* num, uintptr_t stream) {
+    float* vn, float* beta, float* decay, float* gate, float* o, float* pk, float* pq, float* total, float* num, void* images, int32_t* status,
+    uintptr_t stream) {
     if (num_tokens <= 0 || num_entries <= 0) return LLM_OK;
     DeltaShape s;
     const int rc = delta_shape(s, H, G, D, V, taps, q_off, b_off, a_off, ra, g_off, rg, stride, slot_stride);
@@ -1036,6 +1533,23 @@ extern "C" int llm_delta_scan(
     else if (w_dtype == LLM_DT_F32) LOWRANK(float);
     else LOWRANK(bf16);
 #undef LOWRANK
+    const long long walks = static_cast<long long>(num_tokens) * H;
+    if (images) {
+        if (!llm_delta_batched(H, D, V, num_entries, max_len) || !aligned16(images)) return LLM_REFUSED_SIZE;
+        static_assert(DX_IMAGE <= DX_ROWS && DX_IMAGE % 16 == 0, "the image takes the vectors' place");
+        constexpr int most = DX_SMEM > DR_ALONE_SMEM ? DX_SMEM : DR_ALONE_SMEM;
+        cudaError_t e = cudaFuncSetAttribute(delta_batch_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, DX_BATCH_SMEM);
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(delta_scan_mma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+        if (e != cudaSuccess) return static_cast<int>(e);
+        launch_pdl(delta_batch_kernel, dim3(num_tokens / DX_T + num_entries, H), dim3(128), DX_BATCH_SMEM, st, s, qn, kn, vn, beta, decay,
+                   static_cast<unsigned char*>(images), entry_q_start, entry_q_len, num_entries);
+        const int tiles = V / DX_COLS;
+        const long long blocks = static_cast<long long>(num_entries) * H * tiles;
+        const bool alone = blocks <= DR_SMS || (blocks <= 2 * DR_SMS && walks * tiles <= static_cast<long long>(DR_SMS) * max_len);
+        launch_pdl(delta_scan_mma_kernel, dim3(static_cast<unsigned>(blocks)), dim3(256), alone ? most : DX_SMEM, st, s, proj,
+                   static_cast<const unsigned char*>(images), qn, kn, vn, beta, decay, o, state, positions, entry_slot, entry_q_start,
+                   entry_q_len, num_entries, tiles, status);
+    } else {
     const dim3 cgrid(num_tokens, (H + DC_WARPS - 1) / DC_WARPS);
 #define CHUNKS_OF(DP)                                                                                                 \
     launch_pdl((delta_chunk_kernel<DP>), cgrid, dim3(DC_WARPS * 32), 0, st, s, qn, kn, decay, pk, pq, total, num,      \
@@ -1054,8 +1568,6 @@ extern "C" int llm_delta_scan(
 // of 284, 567 and 849 tokens, 192 blocks): as the hardware deals them 241, longest first 188, and alone 160; eight of 55 to 445
 // tokens, 256 blocks: longest first 106, and alone 89; 512 blocks: side by side 179, alone 208.  Equal portions of 256 tokens, the
 // whole layer's kernels: 156 blocks side by side 128, alone 148; 192: 138, 157; 256: 151, 172; 288: 154, 176.
-#define DR_SMS 148
-#define DR_ALONE_SMEM (116 * 1024)
 #define SCAN(DP, C, WARPS, L)                                                                                         \
     do {                                                                                                              \
         auto kern = delta_scan_kernel<DP, C, WARPS, L>;                                                               \
@@ -1076,7 +1588,7 @@ extern "C" int llm_delta_scan(
     // few columns: fewer a warp, so that more schedulers have one; many: more a warp, which costs fewer instructions a column.
     // Measured at 128 rows (us; one, two, four columns on 32 lanes, four on 16): 512 columns (1,000 tokens) 106 111 133 177,
     // 1,024: 141 112 134 181, 2,048: 213 159 136 182, 4,096 (1,500 tokens of 4 requests): 203 154 131 113.
-    const long long columns = static_cast<long long>(num_entries) * H * V, walks = static_cast<long long>(num_tokens) * H;
+    const long long columns = static_cast<long long>(num_entries) * H * V;
     const int plan = columns <= 640 ? 0 : columns <= 1300 ? 1 : columns <= 3000 ? 2 : 3;
     switch (s.DP) {
         case 32: SCAN(32, 2, 2, 8); break;
@@ -1093,6 +1605,7 @@ extern "C" int llm_delta_scan(
             break;
     }
 #undef SCAN
+    }
     const long long items = static_cast<long long>(num_tokens) * H;
     const long long oblocks = (items + 3) / 4;
     if (oblocks > 0x7fffffffLL) return LLM_REFUSED_SIZE;

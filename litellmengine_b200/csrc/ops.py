@@ -1187,21 +1187,28 @@ def delta_rule(proj: torch.Tensor, offs, ranks, conv_w: torch.Tensor, w_decay: t
         _check(f(*args, _ptr(batch.entry_slot), _ptr(batch.entry_q_start), batch.num_entries, H, G, D, V, _stream()), "delta_step")
         return
     DP, VP = delta_padded(D), (V + 3) // 4 * 4
-    chunks = T // 8 + batch.num_entries + 1                 # places for what the eight tokens of a chunk share
-    sizes = (T * H * DP,) + 2 * (T * G * DP,) + (T * H * VP, T * H, T * H * V, T * H * V) + 2 * (T * H * DP,) + (chunks * H * DP, chunks * H * 128)
+    # a graph that is being captured serves other divisions of its tokens too
+    longest = 0 if getattr(batch, "any_division", False) else getattr(batch, "max_q_len", 0)
+    batched = _fn("delta_rule", "llm_delta_batched", [c_int] * 5)(H, D, V, batch.num_entries, longest)
+    if batched:                                             # images of what sixteen tokens share
+        shared = ((T // 16 + batch.num_entries + 1) * H * (_fn("delta_rule", "llm_delta_image_bytes", [])() // 4),)
+    else:                                                   # places for what the eight tokens of a chunk share
+        chunks = T // 8 + batch.num_entries + 1
+        shared = 2 * (T * H * DP,) + (chunks * H * DP, chunks * H * 128)
+    sizes = (T * H * DP,) + 2 * (T * G * DP,) + (T * H * VP, T * H, T * H * V, T * H * V) + shared
     starts = [0]
     for n in sizes:
         starts.append(starts[-1] + (n + 3) // 4 * 4)
     room = torch.empty(starts[-1], dtype=torch.float32, device=dev)
     if D != DP:
         room[:sizes[0]].zero_()                             # decays behind a head's key width must be finite
-    decay, qn, kn, vn, beta, gate, o, pk, pq, total, num = (room.data_ptr() + 4 * n for n in starts[:-1])
+    decay, qn, kn, vn, beta, gate, o, *shared = (room.data_ptr() + 4 * n for n in starts[:-1])
+    shared = [None] * 4 + shared if batched else shared + [None]
     f = _fn("delta_rule", "llm_delta_scan",
-            head + [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int] + [c_void_p] * 12)
-    # a graph that is being captured serves other divisions of its tokens too
-    longest = 0 if getattr(batch, "any_division", False) else getattr(batch, "max_q_len", 0)
+            head + [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int] + [c_void_p] * 14)
     _check(f(*args, _ptr(batch.token_entry), _ptr(batch.entry_slot), _ptr(batch.entry_q_start), _ptr(batch.entry_q_len), T,
-             batch.num_entries, longest, H, G, D, V, qn, kn, vn, beta, decay, gate, o, pk, pq, total, num, _stream()), "delta_scan")
+             batch.num_entries, longest, H, G, D, V, qn, kn, vn, beta, decay, gate, o, *shared,
+             _ptr(stream_status(dev)), _stream()), "delta_scan")
     global launch_count
     launch_count += 4                          # five kernels in one call
 

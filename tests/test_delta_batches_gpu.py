@@ -1,0 +1,78 @@
+"""The delta rule in batches of sixteen tokens on the tensor cores against the token-by-token recurrence in 64 bits: portions that end
+anywhere in a batch, blocks of 32 columns, heads that share keys, decays down to nothing, values that are not finite."""
+import types
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+F64 = torch.float64
+TAPS, RA, RG, EPS = 3, 4, 5, 1e-5
+
+
+def setup(H, G, V, lens, dt_std, seed):
+    D, T, C = 128, sum(lens), 2 * G * 128 + H * V
+    g = torch.Generator(device=DEV).manual_seed(seed)
+    rnd = lambda *s: torch.randn(*s, generator=g, device=DEV)
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)
+    w = dict(proj=rnd(T, C + H + RA + RG), conv=rnd(C, TAPS) * 0.5, wa=rnd(RA, H * D) * 0.3, wg=rnd(RG, H * V) * 0.3, dt=rnd(H * D) * dt_std,
+             al=rnd(H) * 0.5, nw=1 + 0.1 * rnd(V), state=rnd(len(lens), (H * V * D + TAPS * C + 3) // 4 * 4))
+    w["state"][:, H * V * D:] = 0                             # no tokens in front of these
+    starts = [sum(lens[:i]) for i in range(len(lens))]
+    batch = types.SimpleNamespace(positions=i32([p for n in lens for p in range(n)]), token_entry=i32([e for e, n in enumerate(lens) for _ in range(n)]),
+                                  entry_slot=i32(list(range(len(lens)))), entry_q_start=i32(starts), entry_q_len=i32(lens), num_entries=len(lens),
+                                  max_q_len=4096)             # long enough for the batches' kernels to be taken
+    return w, batch, starts
+
+
+def run(w, batch, H, G, V):
+    from litellmengine_b200.csrc import ops
+    C = 2 * G * 128 + H * V
+    assert ops._fn("delta_rule", "llm_delta_batched", [ops.c_int] * 5)(H, 128, V, batch.num_entries, batch.max_q_len)
+    state, out = w["state"].clone(), torch.zeros(w["proj"].shape[0], H * V, device=DEV)
+    ops.delta_rule(w["proj"], (0, C, C + H, C + H + RA), (RA, RG), w["conv"], w["wa"], w["wg"], w["dt"], w["al"], w["nw"], EPS, 1.0, out, 0, state,
+                   batch, H, G, 128, V, single=False)
+    assert ops.stream_status(DEV).tolist() == [0, 0]
+    return out, state
+
+
+@pytest.mark.parametrize("H,G,V,lens", [(12, 12, 128, [1, 2, 15]), (12, 6, 128, [16, 17]), (16, 16, 128, [33, 31]), (2, 2, 32, [1 + i for i in range(32)]),
+                                        (24, 24, 64, [40]), (5, 5, 96, [16, 47, 3, 65])])
+@pytest.mark.parametrize("dt_std", [1.0, 8.0])
+def test_portions_end_anywhere(H, G, V, lens, dt_std):
+    D = 128
+    w, batch, starts = setup(H, G, V, lens, dt_std, H * 100 + V)
+    out, state = run(w, batch, H, G, V)
+    C, x = 2 * G * D + H * V, w["proj"].to(F64)
+    unit = lambda t: t * torch.rsqrt(t.pow(2).sum(-1, keepdim=True) + 1e-6)
+    for e, n in enumerate(lens):
+        u = x[starts[e]:starts[e] + n]
+        mixed = torch.nn.functional.silu(sum(torch.nn.functional.pad(u[:, :C], (0, 0, TAPS - 1 - j, 0))[:n] * w["conv"][:, j].to(F64) for j in range(TAPS)))
+        q, k = (unit(mixed[:, i * G * D:(i + 1) * G * D].view(n, G, D)).repeat_interleave(H // G, dim=1) for i in range(2))
+        v, beta, q = mixed[:, 2 * G * D:].view(n, H, V), torch.sigmoid(u[:, C:C + H]), q * D ** -0.5
+        decay = torch.exp(-torch.exp(w["al"].to(F64))[None, :, None] * torch.nn.functional.softplus(u[:, C + H:C + H + RA] @ w["wa"].to(F64) + w["dt"].to(F64)).view(n, H, D))
+        S = w["state"][e, :H * V * D].view(H, V, D).transpose(1, 2).to(F64)
+        ref = torch.empty(n, H, V, dtype=F64, device=DEV)
+        for t in range(n):
+            S = decay[t][:, :, None] * S
+            S = S + k[t][:, :, None] * (beta[t][:, None] * (v[t] - torch.einsum("hdv,hd->hv", S, k[t])))[:, None, :]
+            ref[t] = torch.einsum("hdv,hd->hv", S, q[t])
+        ref = ref * torch.rsqrt(ref.pow(2).mean(-1, keepdim=True) + EPS) * w["nw"].to(F64) * torch.sigmoid(u[:, C + H + RA:] @ w["wg"].to(F64)).view(n, H, V)
+        # a few dozen 32-bit roundings a token; the norm divides by o's size, which can be small
+        assert float(((out[starts[e]:starts[e] + n].view(n, H, V).to(F64) - ref).abs() / (1 + ref.abs())).max()) < 1e-4, n
+        got = state[e, :H * V * D].view(H, V, D).transpose(1, 2).to(F64)
+        assert float((got - S).abs().max()) < 2e-5 * max(1.0, float(S.abs().max())), n
+
+
+@pytest.mark.parametrize("at", [0, 14, 16, 36])
+@pytest.mark.parametrize("piece", ["value", "key"])
+def test_what_is_not_finite_reaches_only_its_own_and_later_tokens(at, piece):
+    H = G = 12
+    w, batch, _ = setup(H, G, 128, [37, 20], 1.0, 7)
+    clean, _ = run(w, batch, H, G, 128)
+    w["proj"][at, (2 if piece == "value" else 1) * G * 128 + 3] = float("nan")      # the first head's; values stand behind q and k
+    out, state = run(w, batch, H, G, 128)
+    assert torch.equal(out[:at], clean[:at]) and torch.equal(out[37:], clean[37:])
+    assert torch.equal(out[:, 128:], clean[:, 128:]) and not bool(torch.isfinite(out[at:37, 3]).any())
+    assert bool(torch.isfinite(state[1, :H * 128 * 128]).all())
