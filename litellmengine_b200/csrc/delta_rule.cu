@@ -6,7 +6,8 @@
 // with q and k unit vectors per head (q times D^-1/2), q, k and v behind a short causal convolution over time and
 // silu, beta = sigmoid of one projection per head, g = exp(-exp(A_h) softplus(z)) with z a low-rank projection plus
 // a bias, and afterwards per head o / rms(o) * w * sigmoid(a low-rank gate).  The state, the decays, the step sizes,
-// the unit norms and every product of the recurrence are 32-bit CUDA-core arithmetic.
+// the unit norms and every product of the recurrence are 32-bit arithmetic: multiply-adds, or, for long portions of heads of 128,
+// sums of bfloat16 products on the tensor cores that are as near (delta_scan_mma_kernel).
 //
 // The columns of S do not touch one another: column v needs k, q, g of the head and its own v_t.  So blocks take any
 // number of columns of any head, and a long prompt of one request spreads over as many SMs as it has columns without
@@ -31,6 +32,7 @@
 //   delta_chunk_kernel     a warp per (eight tokens, head): p k, p q, s k, p_7, A and B
 //   delta_scan_kernel      one block per (entry, head, columns): the recurrence over the entry's tokens, staged sixteen
 //                          at a time with cp.async into two buffers; o in 32-bit; keeps the convolutions' last inputs
+//                          (delta_batch_kernel and delta_scan_mma_kernel take the places of these two for long portions)
 //   delta_output_kernel    a warp per (token, head): norm, weight, gate, scale, store in the compute dtype
 //   delta_step_kernel      all of it for entries of ONE token (decode steps): one block per (entry, head) copies the head's
 //                          state and its slice of the low-rank weights into shared memory before it waits for the kernel
