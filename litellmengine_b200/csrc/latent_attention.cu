@@ -20,15 +20,8 @@
 #include <math_constants.h>
 
 #define LA_THREADS 256
-#define LA_HELD 4             // times four values of the latents that a thread of latent_prepare holds
-
-__device__ __forceinline__ void la_store4(float* p, float4 v) { *reinterpret_cast<float4*>(p) = v; }
-__device__ __forceinline__ void la_store4(bf16* p, float4 v) {
-    uint2 raw;
-    *reinterpret_cast<__nv_bfloat162*>(&raw.x) = __floats2bfloat162_rn(v.x, v.y);
-    *reinterpret_cast<__nv_bfloat162*>(&raw.y) = __floats2bfloat162_rn(v.z, v.w);
-    *reinterpret_cast<uint2*>(p) = raw;
-}
+#define LA_HELD_Q 8           // values of the query's latent and of the cached one that a thread of latent_prepare holds
+#define LA_HELD_KV 4
 
 // entry i (< dims) of a rotated part x at position pos
 __device__ __forceinline__ float la_rotated(const float* x, int i, int dims, float pos, const float* inv_freq,
@@ -49,7 +42,7 @@ __global__ void latent_prepare_kernel(
     TQ* __restrict__ cq_out, TC* __restrict__ keys, long long key_page_stride,
     const int32_t* __restrict__ positions, const int32_t* __restrict__ token_entry,
     const int32_t* __restrict__ entry_slot, const int32_t* __restrict__ block_table, int table_stride,
-    int page_size, int num_pages, int32_t* __restrict__ status, int rot_pairs, float rot_mag, int vec) {
+    int page_size, int num_pages, int32_t* __restrict__ status, int rot_pairs, float rot_mag, int held) {
     pdl_begin();
     __shared__ float scratch[33];
     const int t = blockIdx.x;
@@ -74,39 +67,31 @@ __global__ void latent_prepare_kernel(
         }
     }
     float ss = 0.0f, ss_kv = 0.0f;
-    if (vec) {                                                // both latents wait in registers, four values at a time
-        float4 v[LA_HELD];
-        const int nq = Q >> 2, n = nq + (keys ? R >> 2 : 0);
+    if (held) {          // both latents and their weights wait in registers; summed in the order of the loops below, value for value
+        float v[LA_HELD_Q], u[LA_HELD_KV], w[LA_HELD_Q], x[LA_HELD_KV];
+        auto each = [&](auto& all, int n, auto&& what) {          // the thread's values of n
 #pragma unroll
-        for (int j = 0; j < LA_HELD; ++j) {
-            const int i = threadIdx.x + j * LA_THREADS;
-            if (i < n) v[j] = *reinterpret_cast<const float4*>(i < nq ? dq + 4 * i : dkv + 4 * (i - nq));
-        }
-#pragma unroll
-        for (int j = 0; j < LA_HELD; ++j) {
-            const int i = threadIdx.x + j * LA_THREADS;
-            if (i < n) (i < nq ? ss : ss_kv) += v[j].x * v[j].x + v[j].y * v[j].y + v[j].z * v[j].z + v[j].w * v[j].w;
-        }
+            for (int j = 0; j < static_cast<int>(sizeof(all) / sizeof(all[0])); ++j)
+                if (const int i = threadIdx.x + j * LA_THREADS; i < n) what(all[j], i, j);
+        };
+        const int n_kv = keys ? R : 0;
+        each(v, Q, [&](float& a, int i, int) { a = dq[i]; });
+        each(u, n_kv, [&](float& a, int i, int) { a = dkv[i]; });
+        each(w, Q, [&](float& a, int i, int) { a = wq[i]; });
+        each(x, n_kv, [&](float& a, int i, int) { a = wkv[i]; });
+        each(v, Q, [&](float& a, int, int) { ss += a * a; });
+        each(u, n_kv, [&](float& a, int, int) { ss_kv += a * a; });
         ss = warp_sum(ss);
         ss_kv = warp_sum(ss_kv);
-        if ((threadIdx.x & 31) == 0) { scratch[threadIdx.x >> 5] = ss; scratch[16 + (threadIdx.x >> 5)] = ss_kv; }
+        if ((threadIdx.x & 31) == 0) { scratch[threadIdx.x >> 5] = ss; scratch[8 + (threadIdx.x >> 5)] = ss_kv; }
         __syncthreads();
-        float sums[2] = {0.0f, 0.0f};
-#pragma unroll
-        for (int w = 0; w < LA_THREADS / 32; ++w) { sums[0] += scratch[w]; sums[1] += scratch[16 + w]; }
-        const float inv_q = 1.0f / sqrtf(sums[0] / static_cast<float>(Q) + eps), inv_kv = 1.0f / sqrtf(sums[1] / static_cast<float>(R) + eps);
-#pragma unroll
-        for (int j = 0; j < LA_HELD; ++j) {
-            const int i = threadIdx.x + j * LA_THREADS;
-            if (i >= n) break;
-            const bool q = i < nq;
-            const float inv = q ? inv_q : inv_kv;
-            const float4 w = *reinterpret_cast<const float4*>(q ? wq + 4 * i : wkv + 4 * (i - nq));
-            const float4 y = make_float4(v[j].x * inv * w.x, v[j].y * inv * w.y, v[j].z * inv * w.z, v[j].w * inv * w.w);
-            if (q) la_store4(cq + 4 * i, y);
-            else if (dst) la_store4(dst + 4 * (i - nq), y);
-        }
+        auto all_warps = [&](const float* s) { return ((s[0] + s[4]) + (s[2] + s[6])) + ((s[1] + s[5]) + (s[3] + s[7])); };      // as warp_sum does
+        static_assert(LA_THREADS == 256, "eight warps");
+        const float inv_q = 1.0f / sqrtf(all_warps(scratch) / static_cast<float>(Q) + eps);
+        each(v, Q, [&](float& a, int i, int j) { cq[i] = from_f32<TQ>(a * inv_q * w[j]); });
         if (!dst) return;
+        const float inv = 1.0f / sqrtf(all_warps(scratch + 8) / static_cast<float>(R) + eps);
+        each(u, R, [&](float& a, int i, int j) { dst[i] = from_f32<TC>(a * inv * x[j]); });
     } else {
         for (int i = threadIdx.x; i < Q; i += blockDim.x) { const float a = dq[i]; ss += a * a; }
         if (keys)
@@ -133,15 +118,14 @@ extern "C" int llm_latent_prepare(
     if (keys && (!block_table || page_size <= 0 || !wkv || (dims > 0 && !inv_freq))) return LLM_REFUSED_SIZE;
     cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
     if (!keys) cache_dtype = q_dtype;
-    // 2,000 tokens, latents of 1,536 and 512: 17 -> 12 us (one value a load, each read twice, and one sum over the block after the other)
-    const int vec = Q % 4 == 0 && R % 4 == 0 && P % 4 == 0 && (Q + (keys ? R : 0)) / 4 <= LA_HELD * LA_THREADS && proj_stride % 4 == 0 &&
-                    dq_off % 4 == 0 && (!keys || (dkv_off % 4 == 0 && key_page_stride % 4 == 0 && aligned16(keys) && aligned16(wkv))) &&
-                    aligned16(proj) && aligned16(wq) && aligned16(cq_out);
+    // 2,000 tokens, latents of 1,536 and 512, the layer in us: 262 with one value a load, each read twice, and one sum over the block after
+    // the other; 258 with both latents held.  The sums keep their order: what is cached must not depend on the form.
+    const int held = Q <= LA_HELD_Q * LA_THREADS && R <= LA_HELD_KV * LA_THREADS;
 #define LAUNCH(TQ, TC)                                                                                              \
     launch_pdl((latent_prepare_kernel<TQ, TC>), dim3(num_tokens), dim3(LA_THREADS), 0, s, proj, proj_stride, dq_off,  \
                dkv_off, Q, R, P, dims, wq, wkv, eps, inv_freq, static_cast<TQ*>(cq_out), static_cast<TC*>(keys),     \
                key_page_stride, positions, token_entry, entry_slot, block_table, table_stride, page_size, num_pages, \
-               status, rot_pairs, rot_mag, vec)
+               status, rot_pairs, rot_mag, held)
     if (q_dtype == LLM_DT_F32 && cache_dtype == LLM_DT_F32) LAUNCH(float, float);
     else if (q_dtype == LLM_DT_BF16 && cache_dtype == LLM_DT_BF16) LAUNCH(bf16, bf16);
     else if (q_dtype == LLM_DT_F32 && cache_dtype == LLM_DT_BF16) LAUNCH(float, bf16);
