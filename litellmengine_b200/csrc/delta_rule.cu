@@ -790,7 +790,9 @@ __global__ void __launch_bounds__(WARPS * 32) delta_scan_kernel(
 // What bounds it: a batch's chain, 3,700 clocks: 48 small products a warp over the state (1,000), shares and X (700), U (300), the state
 // (600), the outputs of two warps (600) and the waits in between; the tensor pipe would take 1,450.  Portions of 284, 567 and 849
 // tokens, 16 heads of 128 x 128 (us): the scan 160 -> 107, what it shares 24 -> 46 (dot products and the writing of 76 MB).
-// Error against 64 bits (2-norm; outputs and states): 1.61e-7 and 1.56e-7, the kernels of eight tokens 1.60e-7 and 1.57e-7.
+// Error against 64 bits (2-norm, outputs and states) from the same unit norms, decays and step sizes: 7.7e-8 and 6.0e-8, the kernels of
+// eight tokens 8.6e-8 and 7.9e-8.  With sums as the tensor cores cut them (split_mma_whole) and dot products in four chains it was
+// 10.4e-8 and 8.6e-8, and the layer 320 us instead of 326.
 #define DX_T 16
 #define DX_PITCH 136                 // of a row of a plane: eight rows of 16 bytes fall into all banks
 #define DX_PLANE (DX_T * DX_PITCH)
@@ -922,16 +924,24 @@ __global__ void __launch_bounds__(128) delta_batch_kernel(
             const float* ka = rows + (24 * level + i) * DX_LP;
             const float* qa = ka + 8 * DX_LP;
             const float* b = rows + (24 * level + 16 + base + j) * DX_LP;
-            float2 x0 = zero, x1 = zero, y0 = zero, y1 = zero;
-#pragma unroll 8
-            for (int d = 0; d < D; d += 4) {
-                const float4 u = *reinterpret_cast<const float4*>(ka + d), w = *reinterpret_cast<const float4*>(qa + d), v = *reinterpret_cast<const float4*>(b + d);
-                x0.x = fmaf(u.x, v.x, x0.x); x0.y = fmaf(u.y, v.y, x0.y); x1.x = fmaf(u.z, v.z, x1.x); x1.y = fmaf(u.w, v.w, x1.y);
-                y0.x = fmaf(w.x, v.x, y0.x); y0.y = fmaf(w.y, v.y, y0.y); y1.x = fmaf(w.z, v.z, y1.x); y1.y = fmaf(w.w, v.w, y1.y);
-            }
+            float x[16], z[16];                      // sixteen chains of eight: four of 32 had twice the error
+#pragma unroll
+            for (int n = 0; n < 16; ++n) x[n] = z[n] = 0.0f;
+#pragma unroll 2
+            for (int d = 0; d < D; d += 16)
+#pragma unroll
+                for (int n = 0; n < 16; n += 4) {
+                    const float4 u = *reinterpret_cast<const float4*>(ka + d + n), w = *reinterpret_cast<const float4*>(qa + d + n), v = *reinterpret_cast<const float4*>(b + d + n);
+                    x[n] = fmaf(u.x, v.x, x[n]); x[n + 1] = fmaf(u.y, v.y, x[n + 1]); x[n + 2] = fmaf(u.z, v.z, x[n + 2]); x[n + 3] = fmaf(u.w, v.w, x[n + 3]);
+                    z[n] = fmaf(w.x, v.x, z[n]); z[n + 1] = fmaf(w.y, v.y, z[n + 1]); z[n + 2] = fmaf(w.z, v.z, z[n + 2]); z[n + 3] = fmaf(w.w, v.w, z[n + 3]);
+                }
+#pragma unroll
+            for (int n = 8; n > 0; n >>= 1)
+#pragma unroll
+                for (int m = 0; m < n; ++m) { x[m] += x[m + n]; z[m] += z[m + n]; }
             const int to = 16 * (2 * base + half + i % half) + 2 * base + j;
-            nums[to] = (x0.x + x0.y) + (x1.x + x1.y);
-            nums[256 + to] = (y0.x + y0.y) + (y1.x + y1.y);
+            nums[to] = x[0];
+            nums[256 + to] = z[0];
         }
         if (tid < DX_T) nums[256 + 17 * tid] = shares[2 * (tid >> 3) * 8 + (tid & 7)] + shares[(2 * (tid >> 3) + 1) * 8 + (tid & 7)];
         __syncthreads();                                                    // the planes take the rows' place
@@ -1138,7 +1148,7 @@ __global__ void __launch_bounds__(256, 2) delta_scan_mma_kernel(
         split_tiles(x[0], x[1], a);
 #pragma unroll
         for (int p = 0; p < 3; ++p) ldmatrix_x4(y[p], small + p * DX_NPLANE + frow * DX_NP + fcol);
-        split_mma<true>(um, us, a, y);
+        split_mma_whole(um, us, a, y);
 #pragma unroll
         for (int u = 0; u < 2; ++u)
 #pragma unroll
@@ -1151,7 +1161,7 @@ __global__ void __launch_bounds__(256, 2) delta_scan_mma_kernel(
                 float c[2][4], cs[2][4];
 #pragma unroll
                 for (int p = 0; p < 3; ++p) ldmatrix_x4_trans(y[p], planes + (6 + p) * DX_PLANE + grow * DX_PITCH + dw + 16 * j + gcol);
-                split_mma<true>(c, cs, a, y);
+                split_mma_whole(c, cs, a, y);
 #pragma unroll
                 for (int u = 0; u < 2; ++u) {
                     const float2 f = *reinterpret_cast<const float2*>(total + dw + 16 * j + 8 * u + 2 * lt);
@@ -1165,13 +1175,9 @@ __global__ void __launch_bounds__(256, 2) delta_scan_mma_kernel(
             float om[4], os[4];
 #pragma unroll
             for (int p = 0; p < 3; ++p) ldmatrix_x4(y[p], small + (3 + p) * DX_NPLANE + frow * DX_NP + fcol);
-#pragma unroll
-            for (int i = 0; i < 6; ++i) {
-                const unsigned b0 = u ? y[B[i]][2] : y[B[i]][0], b1 = u ? y[B[i]][3] : y[B[i]][1];
-                if (i == 0) mma_bf16_first(os, a[A[i]], b0, b1);
-                else if (i < 5) mma_bf16(os, a[A[i]], b0, b1);
-                else mma_bf16_first(om, a[A[i]], b0, b1);
-            }
+            const unsigned b0[3] = {u ? y[0][2] : y[0][0], u ? y[1][2] : y[1][0], u ? y[2][2] : y[2][0]};
+            const unsigned b1[3] = {u ? y[0][3] : y[0][1], u ? y[1][3] : y[1][1], u ? y[2][3] : y[2][1]};
+            split_mma_whole(om, os, a, b0, b1);
             const float4 r = over_rows(2 + u);
             const float out[4] = {r.x + (om[0] + os[0]), r.y + (om[1] + os[1]), r.z + (om[2] + os[2]), r.w + (om[3] + os[3])};
 #pragma unroll
