@@ -695,7 +695,8 @@ static bool gla_tiled_takes(int D, int V, int mode) {
 // register-tiled kernel above before); of the output pass's time the tensor pipe is busy for 30 %, the loads of rows and state come
 // from memory half of the time, two blocks an SM hide some of each other's waits.  Tried: 16 tokens a batch with the state kept in
 // accumulators 92; 64 tokens a batch, one block of 16 warps an SM 87.  Error against 64 bits (2-norm, 2,048 tokens, decays
-// sigmoid(z)^(1/8)): states 6.0e-8, outputs 1.05e-7; the kernel above 7.0e-8 and 1.29e-7.
+// sigmoid(z)^(1/tau), tau 1, 2, 8, 64): states 4.0, 3.2, 4.0 and 6.1e-8, the kernel above 4.0, 4.7, 7.4 and 17.3; outputs 14.7, 10.1, 10.6
+// and 12.4e-8, and 14.4, 13.0, 13.1 and 20.2.  With all sums of the states as the tensor cores cut them the states were 5.7, 5.5, 6.0 and 7.2.
 #define GM_D 128
 #define GM_PITCH 136                 // of a row of a plane: eight rows of 16 bytes fall into all banks
 #define GM_WP 40                     // of a row of weights
@@ -987,7 +988,7 @@ __global__ void __launch_bounds__(256, 2) gla_scan_mma_kernel(
                     for (int b = 0; b < 2; ++b) {
 #pragma unroll
                         for (int p = 0; p < 3; ++p) ldmatrix_x4(y[p], pq + p * PLANE + (16 * b + frow) * GM_PITCH + 16 * j + fcol);
-                        split_mma<false>(o[b], om[b], x, y);
+                        split_mma(o[b], om[b], x, y);
                     }
                 }
                 __syncthreads();
@@ -1016,7 +1017,7 @@ __global__ void __launch_bounds__(256, 2) gla_scan_mma_kernel(
                     for (int b = sb; b < 2; ++b) {
 #pragma unroll
                         for (int p = 0; p < 3; ++p) ldmatrix_x4(y[p], pp + (p * T + 16 * b + frow) * GM_WP + 16 * sb + fcol);
-                        split_mma<false>(o[b], om[b], x, y);
+                        split_mma(o[b], om[b], x, y);
                     }
                 }
                 // the queries' planes were last read in front of a barrier
@@ -1037,14 +1038,14 @@ __global__ void __launch_bounds__(256, 2) gla_scan_mma_kernel(
                 if (!none) fetch(0);
 #pragma unroll
                 for (int j = 0; j < D / 16; ++j) {
-                    float c[2][4], cm[2][4];
+                    float c[2][4] = {}, cm[2][4] = {}, n[2][4];      // n: the last sixteen tokens, which strong decays leave little but
 #pragma unroll
                     for (int sb = 0; sb < T / 16; ++sb) {
                         unsigned y[3][4];
 #pragma unroll
                         for (int p = 0; p < 3; ++p) ldmatrix_x4_trans(y[p], pk + p * PLANE + (16 * sb + grow) * GM_PITCH + 16 * j + gcol);
-                        if (sb == 0) split_mma<true>(c, cm, x[sb], y);
-                        else split_mma<false>(c, cm, x[sb], y);
+                        if (sb + 1 < T / 16) split_mma(c, cm, x[sb], y);
+                        else split_mma_whole<false>(n, cm, x[sb], y);
                     }
                     float old[2][4];
 #pragma unroll
@@ -1058,7 +1059,7 @@ __global__ void __launch_bounds__(256, 2) gla_scan_mma_kernel(
                         const float2 f = *reinterpret_cast<const float2*>(bend + row);
 #pragma unroll
                         for (int i = 0; i < 4; ++i)
-                            s_out[static_cast<size_t>(row + (i & 1)) * V + v0 + 8 * (i >> 1)] = fmaf(old[u][i], i & 1 ? f.y : f.x, cm[u][i]) + c[u][i];
+                            s_out[static_cast<size_t>(row + (i & 1)) * V + v0 + 8 * (i >> 1)] = (fmaf(old[u][i], i & 1 ? f.y : f.x, cm[u][i]) + c[u][i]) + n[u][i];
                     }
                 }
             }

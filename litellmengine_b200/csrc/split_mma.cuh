@@ -27,22 +27,15 @@ __device__ __forceinline__ void mma_bf16_first(float (&c)[4], const unsigned (&a
                  : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(0.0f));
 }
 // Two tiles of 8 columns side by side, a [16 x 16] by b [16 x 16]: the five smaller of the six products, smallest first, onto `small`,
-// the largest onto `main`; FRESH starts both from zero.
-template <bool FRESH>
+// the largest onto `main`.
 __device__ __forceinline__ void split_mma(float (&main)[2][4], float (&small)[2][4], const unsigned (&a)[3][4], const unsigned (&b)[3][4]) {
     constexpr int A[5] = {2, 0, 1, 1, 0}, B[5] = {0, 2, 1, 0, 1};
 #pragma unroll
     for (int i = 0; i < 5; ++i)
 #pragma unroll
-        for (int u = 0; u < 2; ++u) {
-            if (FRESH && i == 0) mma_bf16_first(small[u], a[A[i]], b[B[i]][2 * u], b[B[i]][2 * u + 1]);
-            else mma_bf16(small[u], a[A[i]], b[B[i]][2 * u], b[B[i]][2 * u + 1]);
-        }
+        for (int u = 0; u < 2; ++u) mma_bf16(small[u], a[A[i]], b[B[i]][2 * u], b[B[i]][2 * u + 1]);
 #pragma unroll
-    for (int u = 0; u < 2; ++u) {
-        if (FRESH) mma_bf16_first(main[u], a[0], b[0][2 * u], b[0][2 * u + 1]);
-        else mma_bf16(main[u], a[0], b[0][2 * u], b[0][2 * u + 1]);
-    }
+    for (int u = 0; u < 2; ++u) mma_bf16(main[u], a[0], b[0][2 * u], b[0][2 * u + 1]);
 }
 // The same from zero, and nearer.  The tensor cores cut a sum to 24 bits where an addition rounds, which is twice the error (5.8e-8 of a
 // sum of sixteen, 2-norm); but they have what they cut: the largest product once more, less what came out of it, goes to `small`.
