@@ -714,8 +714,9 @@ __device__ __forceinline__ float gm_inverse(float f) {
     asm("rcp.approx.ftz.f32 %0, %1;\n" : "=f"(r) : "f"(f));
     return fmaf(r, fmaf(-f, r, 1.0f), r);
 }
-// g sigmoid(g); the exponential stops at e^80, where the result is below 1e-32
-__device__ __forceinline__ float gm_silu(float g) { return g * gm_inverse(1.0f + expf(fminf(-g, 80.0f))); }
+// g sigmoid(g) by CUDA's division within 2 ulp, which gives 0 for divisors from 2^126 on: silu is below 1e-36 there, and stays NaN for
+// minus infinity.  (The correctly rounded division: 2 us more of 94.)
+__device__ __forceinline__ float gm_silu(float g) { return __fdividef(g, 1.0f + expf(-g)); }
 __device__ __forceinline__ float4 gm_mul(float4 a, float4 b) { return make_float4(a.x * b.x, a.y * b.y, a.z * b.z, a.w * b.w); }
 __device__ __forceinline__ float4 gm_fma(float4 a, float4 b, float4 c) {
     return make_float4(fmaf(a.x, b.x, c.x), fmaf(a.y, b.y, c.y), fmaf(a.z, b.z, c.z), fmaf(a.w, b.w, c.w));

@@ -108,3 +108,25 @@ def test_no_further_from_64_bits_than_the_register_tiled_kernel(tau, lens, chunk
         out, got = run(proj, alpha, state, lens, H, chunk, longest)
         err.append((float((out - ref).norm() / ref.norm()), float((got - end).norm() / end.norm())))
     assert err[0][0] <= err[1][0] and err[0][1] <= err[1][1], err
+
+
+@pytest.mark.parametrize("chunk", [None, 64])
+def test_gates_of_any_size(chunk):
+    """silu from the lowest to the largest number, infinities and NaN; every other column has an ordinary one."""
+    lens, H = [70], 2
+    x = inputs(lens, H, 0.9, torch.Generator(device=DEV).manual_seed(11))
+    top = 3.4028234663852886e38
+    odd = [-top, -1e35, -1e30, -1e10, -1e4, -1000.0, -200.0, -100.0, -89.0, -88.0, -87.0, -80.0, -20.0, -1e-30, 0.0, 1e-30, 20.0, 88.0, 1e4, 1e30,
+           top, float("inf"), float("-inf"), float("nan")]
+    gates = x[0][:, 3 * H * D:4 * H * D]
+    gates[:, 0:2 * len(odd):2] = torch.tensor(odd, device=DEV)
+    ref, _ = plain(*x, lens, H)
+    # in 64 bits too, silu of minus infinity is minus infinity times zero
+    out = run(*x, lens, H, chunk)[0].to(F64)
+    want = torch.where(ref.abs() > top, ref.sign() * float("inf"), ref)
+    assert torch.equal(torch.isnan(out), torch.isnan(want)) and torch.equal(torch.isinf(out), torch.isinf(want))
+    fine = torch.isfinite(want)
+    # a head's outputs have a root mean square of 1 in front of the gate and are a few dozen 2^-24 of that off, the small ones among them
+    # too; below 1e-36 silu is zero in 32 bits, since exp(-g) is infinite
+    size = torch.nn.functional.silu(gates.view(sum(lens), H, D).to(F64)).abs()
+    assert float(((out - want).abs()[fine] / (1e-30 + size[fine])).max()) < 1e-5
