@@ -708,12 +708,6 @@ static bool gla_tiled_takes(int D, int V, int mode) {
 #define GM_TOKENS(outputs) ((outputs) ? 32 : 64)
 #define GM_SMEM(outputs) ((outputs) ? 2 * (9 * 32 * GM_PITCH + 3 * 32 * GM_WP) + 4 * (32 * GM_D + GM_D) : 2 * 6 * 64 * GM_PITCH + 4 * GM_D)
 
-// 1 / f to the last place, for f between 2^-60 and 2^30
-__device__ __forceinline__ float gm_inverse(float f) {
-    float r;
-    asm("rcp.approx.ftz.f32 %0, %1;\n" : "=f"(r) : "f"(f));
-    return fmaf(r, fmaf(-f, r, 1.0f), r);
-}
 // g sigmoid(g) by CUDA's division within 2 ulp, which gives 0 for divisors from 2^126 on: silu is below 1e-36 there, and stays NaN for
 // minus infinity.  (The correctly rounded division: 2 us more of 94.)
 __device__ __forceinline__ float gm_silu(float g) { return __fdividef(g, 1.0f + expf(-g)); }
@@ -721,7 +715,10 @@ __device__ __forceinline__ float4 gm_mul(float4 a, float4 b) { return make_float
 __device__ __forceinline__ float4 gm_fma(float4 a, float4 b, float4 c) {
     return make_float4(fmaf(a.x, b.x, c.x), fmaf(a.y, b.y, c.y), fmaf(a.z, b.z, c.z), fmaf(a.w, b.w, c.w));
 }
-__device__ __forceinline__ float4 gm_inverse(float4 f) { return make_float4(gm_inverse(f.x), gm_inverse(f.y), gm_inverse(f.z), gm_inverse(f.w)); }
+// 1 / f by CUDA's division within 2 ulp; who needs it nearer has gm_rest1
+__device__ __forceinline__ float4 gm_inverse(float4 f) {
+    return make_float4(__fdividef(1.0f, f.x), __fdividef(1.0f, f.y), __fdividef(1.0f, f.z), __fdividef(1.0f, f.w));
+}
 // a b - p, exactly, where p is a b rounded
 __device__ __forceinline__ float4 gm_rest(float4 a, float4 b, float4 p) {
     return make_float4(fmaf(a.x, b.x, -p.x), fmaf(a.y, b.y, -p.y), fmaf(a.z, b.z, -p.z), fmaf(a.w, b.w, -p.w));
@@ -857,7 +854,7 @@ __global__ void __launch_bounds__(256, 2) gla_scan_mma_kernel(
                     if (OUTPUTS) {
                         const float4 r = gm_inverse(behind[n].hi), qh = gm_mul(q[i], r);
                         bad |= !gm_fits(q[i]);
-                        // 1 / (hi + lo) = r (1 + (1 - r hi) - r lo), as near as matters
+                        // 1 / (hi + lo) = r (1 + (1 - r hi) - r lo), as near as matters: r's own error too is in the bracket
                         split_store4(pq + at, PLANE, qh, gm_fma(qh, gm_rest1(r, behind[n]), gm_rest(q[i], r, qh)));
                     }
                     behind[n] = gm_times(behind[n], a[n][i]);
