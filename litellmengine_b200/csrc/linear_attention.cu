@@ -883,7 +883,139 @@ __global__ void __launch_bounds__(256, 2) gla_scan_mma_kernel(
             }
         }
         const float* o0 = os;
-        if (__syncthreads_or(bad)) {                 // token by token, the state in registers
+        bool walk = __syncthreads_or(bad);
+        if (!walk) {
+            float ahead[2][4];                   // the state's next sixteen rows
+            auto fetch = [&](int j) {
+#pragma unroll
+                for (int u = 0; u < 2; ++u)
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) ahead[u][i] = s_in[static_cast<size_t>(16 * j + 8 * u + 2 * lt + (i & 1)) * V + v0 + 8 * (i >> 1)];
+            };
+            if (OUTPUTS) {
+                fetch(0);
+                // the weights q' . k' of the three pairs of token blocks, 8 keys a tile, a quarter of the channels a unit
+                for (int unit = warp; unit < 24; unit += 8) {
+                    const int tile = unit >> 2, i = tile < 2 ? 0 : 1, s0 = 8 * (tile - 2 * i), d = 32 * (unit & 3);
+                    float w[4] = {}, ws[2][4] = {};
+                    unsigned y[3][4];                // 8 keys, 32 channels
+#pragma unroll
+                    for (int p = 0; p < 3; ++p) ldmatrix_x4(y[p], pk + p * PLANE + (s0 + (lane & 7)) * GM_PITCH + d + 8 * (lane >> 3));
+#pragma unroll
+                    for (int j = 0; j < 2; ++j) {
+                        unsigned x[3][4];
+#pragma unroll
+                        for (int p = 0; p < 3; ++p) ldmatrix_x4(x[p], pq + p * PLANE + (16 * i + grow) * GM_PITCH + d + 16 * j + gcol);
+                        constexpr int A[5] = {2, 0, 1, 1, 0}, B[5] = {0, 2, 1, 0, 1};
+#pragma unroll
+                        for (int m = 0; m < 5; ++m) mma_bf16(ws[j], x[A[m]], y[B[m]][2 * j], y[B[m]][2 * j + 1]);
+                        mma_bf16(w, x[0], y[0][2 * j], y[0][2 * j + 1]);
+                    }
+                    float* to = part + unit * 128 + lg * 8 + 2 * lt;
+                    *reinterpret_cast<float2*>(to) = make_float2(w[0] + (ws[0][0] + ws[1][0]), w[1] + (ws[0][1] + ws[1][1]));
+                    *reinterpret_cast<float2*>(to + 64) = make_float2(w[2] + (ws[0][2] + ws[1][2]), w[3] + (ws[0][3] + ws[1][3]));
+                }
+                float o[2][2][4] = {}, om[2][2][4] = {};
+#pragma unroll
+                for (int j = 0; j < D / 16; ++j) {
+                    float s[2][4];
+#pragma unroll
+                    for (int u = 0; u < 2; ++u) {
+                        const float2 f = *reinterpret_cast<const float2*>(bend + 16 * j + 8 * u + 2 * lt);
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) s[u][i] = ahead[u][i] * (i & 1 ? f.y : f.x);
+                    }
+                    if (j + 1 < D / 16) fetch(j + 1);
+                    unsigned x[3][4], y[3][4];
+                    split_tiles(s[0], s[1], x);
+#pragma unroll
+                    for (int b = 0; b < 2; ++b) {
+#pragma unroll
+                        for (int p = 0; p < 3; ++p) ldmatrix_x4(y[p], pq + p * PLANE + (16 * b + frow) * GM_PITCH + 16 * j + fcol);
+                        split_mma(o[b], om[b], x, y);
+                    }
+                }
+                // A state that is infinite, NaN or beyond bfloat16's range has pieces that are NaN, and these are in the smaller products:
+                // multiply-adds say what becomes of which column.
+                float sum = 0.0f;
+#pragma unroll
+                for (int i = 0; i < 4; ++i) sum += (om[0][0][i] + om[0][1][i]) + (om[1][0][i] + om[1][1][i]);
+                walk = __syncthreads_or(!(fabsf(sum) <= 3.4028235e38f));
+                if (!walk) {
+                    for (int idx = tid; idx < 6 * 64; idx += 256) {          // the shares; what lies ahead of a token weighs nothing
+                        const int tile = idx >> 6, i = tile < 2 ? 0 : 1, at = 2 * (idx & 63);
+                        const int t = 16 * i + (at >> 3), s = 8 * (tile - 2 * i) + (at & 7);
+                        float2 x[4];
+#pragma unroll
+                        for (int u = 0; u < 4; ++u) x[u] = *reinterpret_cast<const float2*>(part + (4 * tile + u) * 128 + at);
+                        float w0 = s <= t ? (x[0].x + x[1].x) + (x[2].x + x[3].x) : 0.0f, w1 = s + 1 <= t ? (x[0].y + x[1].y) + (x[2].y + x[3].y) : 0.0f;
+#pragma unroll
+                        for (int p = 0; p < 3; ++p) *reinterpret_cast<unsigned*>(pp + (p * T + t) * GM_WP + s) = split_piece(w0, w1);
+                    }
+                    __syncthreads();
+                    for (int idx = tid; idx < T * (V / 4); idx += 256) {
+                        const int t = idx / (V / 4), c = (idx % (V / 4)) << 2;
+                        cp_async16(gates + t * V + c, proj + (base + min(t, nb - 1)) * stride + g_off + h * V + c, t < nb);
+                    }
+                    cp_async_commit();
+#pragma unroll
+                    for (int sb = 0; sb < 2; ++sb) {
+                        unsigned x[3][4], y[3][4];
+#pragma unroll
+                        for (int p = 0; p < 3; ++p) ldmatrix_x4_trans(x[p], pv + p * PLANE + (16 * sb + frow) * GM_PITCH + 16 * warp + fcol);
+#pragma unroll
+                        for (int b = sb; b < 2; ++b) {
+#pragma unroll
+                            for (int p = 0; p < 3; ++p) ldmatrix_x4(y[p], pp + (p * T + 16 * b + frow) * GM_WP + 16 * sb + fcol);
+                            split_mma(o[b], om[b], x, y);
+                        }
+                    }
+                    // the queries' planes were last read in front of a barrier
+#pragma unroll
+                    for (int b = 0; b < 2; ++b)
+#pragma unroll
+                        for (int u = 0; u < 2; ++u)
+#pragma unroll
+                            for (int i = 0; i < 4; ++i)
+                                os[(16 * b + 8 * u + 2 * lt + (i & 1)) * GM_OP + v0 + 8 * (i >> 1)] = o[b][u][i] + om[b][u][i];
+                }
+            }
+            if (!walk && (MODE != GLA_OUT || more)) {
+                unsigned x[T / 16][3][4];
+#pragma unroll
+                for (int sb = 0; sb < T / 16; ++sb)
+#pragma unroll
+                    for (int p = 0; p < 3; ++p) ldmatrix_x4_trans(x[sb][p], pv + p * PLANE + (16 * sb + frow) * GM_PITCH + 16 * warp + fcol);
+                if (!none) fetch(0);
+#pragma unroll
+                for (int j = 0; j < D / 16; ++j) {
+                    float c[2][4] = {}, cm[2][4] = {}, n[2][4];      // n: the last sixteen tokens, which strong decays leave little but
+#pragma unroll
+                    for (int sb = 0; sb < T / 16; ++sb) {
+                        unsigned y[3][4];
+#pragma unroll
+                        for (int p = 0; p < 3; ++p) ldmatrix_x4_trans(y[p], pk + p * PLANE + (16 * sb + grow) * GM_PITCH + 16 * j + gcol);
+                        if (sb + 1 < T / 16) split_mma(c, cm, x[sb], y);
+                        else split_mma_whole<false>(n, cm, x[sb], y);
+                    }
+                    float old[2][4];
+#pragma unroll
+                    for (int u = 0; u < 2; ++u)
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) old[u][i] = none ? 0.0f : ahead[u][i];
+                    if (!none && j + 1 < D / 16) fetch(j + 1);
+#pragma unroll
+                    for (int u = 0; u < 2; ++u) {
+                        const int row = 16 * j + 8 * u + 2 * lt;
+                        const float2 f = *reinterpret_cast<const float2*>(bend + row);
+#pragma unroll
+                        for (int i = 0; i < 4; ++i)
+                            s_out[static_cast<size_t>(row + (i & 1)) * V + v0 + 8 * (i >> 1)] = (fmaf(old[u][i], i & 1 ? f.y : f.x, cm[u][i]) + c[u][i]) + n[u][i];
+                    }
+                }
+            }
+        }
+        if (walk) {                                  // token by token, the state in registers
             for (int idx = tid; idx < nb * (D / 4); idx += 256) {
                 const int t = idx / (D / 4), c = (idx % (D / 4)) << 2;
                 const float* pr = proj + (base + t) * stride + h * D + c;
@@ -938,129 +1070,6 @@ __global__ void __launch_bounds__(256, 2) gla_scan_mma_kernel(
                     for (int i = 0; i < 4; ++i) s_out[static_cast<size_t>(d0 + 8 * n + (i & 1)) * V + v0 + 8 * (i >> 1)] = S[n][i];
             __syncthreads();
             o0 = walk_o;
-        } else {
-            float ahead[2][4];                   // the state's next sixteen rows
-            auto fetch = [&](int j) {
-#pragma unroll
-                for (int u = 0; u < 2; ++u)
-#pragma unroll
-                        for (int i = 0; i < 4; ++i) ahead[u][i] = s_in[static_cast<size_t>(16 * j + 8 * u + 2 * lt + (i & 1)) * V + v0 + 8 * (i >> 1)];
-            };
-            if (OUTPUTS) {
-                fetch(0);
-                // the weights q' . k' of the three pairs of token blocks, 8 keys a tile, a quarter of the channels a unit
-                for (int unit = warp; unit < 24; unit += 8) {
-                    const int tile = unit >> 2, i = tile < 2 ? 0 : 1, s0 = 8 * (tile - 2 * i), d = 32 * (unit & 3);
-                    float w[4] = {}, ws[2][4] = {};
-                    unsigned y[3][4];                // 8 keys, 32 channels
-#pragma unroll
-                    for (int p = 0; p < 3; ++p) ldmatrix_x4(y[p], pk + p * PLANE + (s0 + (lane & 7)) * GM_PITCH + d + 8 * (lane >> 3));
-#pragma unroll
-                    for (int j = 0; j < 2; ++j) {
-                        unsigned x[3][4];
-#pragma unroll
-                        for (int p = 0; p < 3; ++p) ldmatrix_x4(x[p], pq + p * PLANE + (16 * i + grow) * GM_PITCH + d + 16 * j + gcol);
-                        constexpr int A[5] = {2, 0, 1, 1, 0}, B[5] = {0, 2, 1, 0, 1};
-#pragma unroll
-                        for (int m = 0; m < 5; ++m) mma_bf16(ws[j], x[A[m]], y[B[m]][2 * j], y[B[m]][2 * j + 1]);
-                        mma_bf16(w, x[0], y[0][2 * j], y[0][2 * j + 1]);
-                    }
-                    float* to = part + unit * 128 + lg * 8 + 2 * lt;
-                    *reinterpret_cast<float2*>(to) = make_float2(w[0] + (ws[0][0] + ws[1][0]), w[1] + (ws[0][1] + ws[1][1]));
-                    *reinterpret_cast<float2*>(to + 64) = make_float2(w[2] + (ws[0][2] + ws[1][2]), w[3] + (ws[0][3] + ws[1][3]));
-                }
-                float o[2][2][4] = {}, om[2][2][4] = {};
-#pragma unroll
-                for (int j = 0; j < D / 16; ++j) {
-                    float s[2][4];
-#pragma unroll
-                    for (int u = 0; u < 2; ++u) {
-                        const float2 f = *reinterpret_cast<const float2*>(bend + 16 * j + 8 * u + 2 * lt);
-#pragma unroll
-                        for (int i = 0; i < 4; ++i) s[u][i] = ahead[u][i] * (i & 1 ? f.y : f.x);
-                    }
-                    if (j + 1 < D / 16) fetch(j + 1);
-                    unsigned x[3][4], y[3][4];
-                    split_tiles(s[0], s[1], x);
-#pragma unroll
-                    for (int b = 0; b < 2; ++b) {
-#pragma unroll
-                        for (int p = 0; p < 3; ++p) ldmatrix_x4(y[p], pq + p * PLANE + (16 * b + frow) * GM_PITCH + 16 * j + fcol);
-                        split_mma(o[b], om[b], x, y);
-                    }
-                }
-                __syncthreads();
-                for (int idx = tid; idx < 6 * 64; idx += 256) {          // the shares; what lies ahead of a token weighs nothing
-                    const int tile = idx >> 6, i = tile < 2 ? 0 : 1, at = 2 * (idx & 63);
-                    const int t = 16 * i + (at >> 3), s = 8 * (tile - 2 * i) + (at & 7);
-                    float2 x[4];
-#pragma unroll
-                    for (int u = 0; u < 4; ++u) x[u] = *reinterpret_cast<const float2*>(part + (4 * tile + u) * 128 + at);
-                    float w0 = s <= t ? (x[0].x + x[1].x) + (x[2].x + x[3].x) : 0.0f, w1 = s + 1 <= t ? (x[0].y + x[1].y) + (x[2].y + x[3].y) : 0.0f;
-#pragma unroll
-                    for (int p = 0; p < 3; ++p) *reinterpret_cast<unsigned*>(pp + (p * T + t) * GM_WP + s) = split_piece(w0, w1);
-                }
-                __syncthreads();
-                for (int idx = tid; idx < T * (V / 4); idx += 256) {
-                    const int t = idx / (V / 4), c = (idx % (V / 4)) << 2;
-                    cp_async16(gates + t * V + c, proj + (base + min(t, nb - 1)) * stride + g_off + h * V + c, t < nb);
-                }
-                cp_async_commit();
-#pragma unroll
-                for (int sb = 0; sb < 2; ++sb) {
-                    unsigned x[3][4], y[3][4];
-#pragma unroll
-                    for (int p = 0; p < 3; ++p) ldmatrix_x4_trans(x[p], pv + p * PLANE + (16 * sb + frow) * GM_PITCH + 16 * warp + fcol);
-#pragma unroll
-                    for (int b = sb; b < 2; ++b) {
-#pragma unroll
-                        for (int p = 0; p < 3; ++p) ldmatrix_x4(y[p], pp + (p * T + 16 * b + frow) * GM_WP + 16 * sb + fcol);
-                        split_mma(o[b], om[b], x, y);
-                    }
-                }
-                // the queries' planes were last read in front of a barrier
-#pragma unroll
-                for (int b = 0; b < 2; ++b)
-#pragma unroll
-                    for (int u = 0; u < 2; ++u)
-#pragma unroll
-                        for (int i = 0; i < 4; ++i)
-                            os[(16 * b + 8 * u + 2 * lt + (i & 1)) * GM_OP + v0 + 8 * (i >> 1)] = o[b][u][i] + om[b][u][i];
-            }
-            if (MODE != GLA_OUT || more) {
-                unsigned x[T / 16][3][4];
-#pragma unroll
-                for (int sb = 0; sb < T / 16; ++sb)
-#pragma unroll
-                    for (int p = 0; p < 3; ++p) ldmatrix_x4_trans(x[sb][p], pv + p * PLANE + (16 * sb + frow) * GM_PITCH + 16 * warp + fcol);
-                if (!none) fetch(0);
-#pragma unroll
-                for (int j = 0; j < D / 16; ++j) {
-                    float c[2][4] = {}, cm[2][4] = {}, n[2][4];      // n: the last sixteen tokens, which strong decays leave little but
-#pragma unroll
-                    for (int sb = 0; sb < T / 16; ++sb) {
-                        unsigned y[3][4];
-#pragma unroll
-                        for (int p = 0; p < 3; ++p) ldmatrix_x4_trans(y[p], pk + p * PLANE + (16 * sb + grow) * GM_PITCH + 16 * j + gcol);
-                        if (sb + 1 < T / 16) split_mma(c, cm, x[sb], y);
-                        else split_mma_whole<false>(n, cm, x[sb], y);
-                    }
-                    float old[2][4];
-#pragma unroll
-                    for (int u = 0; u < 2; ++u)
-#pragma unroll
-                        for (int i = 0; i < 4; ++i) old[u][i] = none ? 0.0f : ahead[u][i];
-                    if (!none && j + 1 < D / 16) fetch(j + 1);
-#pragma unroll
-                    for (int u = 0; u < 2; ++u) {
-                        const int row = 16 * j + 8 * u + 2 * lt;
-                        const float2 f = *reinterpret_cast<const float2*>(bend + row);
-#pragma unroll
-                        for (int i = 0; i < 4; ++i)
-                            s_out[static_cast<size_t>(row + (i & 1)) * V + v0 + 8 * (i >> 1)] = (fmaf(old[u][i], i & 1 ? f.y : f.x, cm[u][i]) + c[u][i]) + n[u][i];
-                    }
-                }
-            }
         }
         if (OUTPUTS) {                               // a warp per token: norm over V, weight, gate, scale
             const float4 nw = *reinterpret_cast<const float4*>(norm_w + 4 * lane);

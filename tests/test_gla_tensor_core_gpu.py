@@ -130,3 +130,18 @@ def test_gates_of_any_size(chunk):
     # too; below 1e-36 silu is zero in 32 bits, since exp(-g) is infinite
     size = torch.nn.functional.silu(gates.view(sum(lens), H, D).to(F64)).abs()
     assert float(((out - want).abs()[fine] / (1e-30 + size[fine])).max()) < 1e-5
+
+
+@pytest.mark.parametrize("chunk", [None, 64])
+@pytest.mark.parametrize("what", [float("inf"), float("-inf"), float("nan"), 3.4e38])
+def test_a_state_that_is_not_finite_or_does_not_split(chunk, what):
+    """Infinite, or too large for three bfloat16 values: the same numbers, zeros and NaN as the register-tiled kernel gives."""
+    lens, H = [40, 20], 2
+    x = inputs(lens, H, 0.9, torch.Generator(device=DEV).manual_seed(17))
+    x[2][0, 1, 5, 7] = what
+    out, state = run(*x, lens, H, chunk)
+    want, end = run(*x, lens, H, chunk, longest=1)
+    assert torch.equal(torch.isnan(out), torch.isnan(want)) and torch.equal(torch.isfinite(state), torch.isfinite(end))
+    assert not bool(torch.isnan(out[:, 0]).any()) and not bool(torch.isnan(out[40:]).any())        # the other head, the other entry
+    near = lambda a, b: float(((a - b).abs() / (1e-3 + b.abs()))[torch.isfinite(b)].max()) < 1e-3
+    assert near(out, want) and near(state, end)
