@@ -1247,15 +1247,20 @@ extern "C" int llm_recur_scan(
 // Items that bring fewer than eight tokens each stay with the register-tiled kernel: a batch costs the tensor-core kernel the same
 // for one token as for 32.  One pass over items of 128 x 128, 16 heads (us, tiled and tensor cores): 32 items of 3 tokens 28
 // and 40, of 16 47 and 41, of 64 130 and 91; one item of 16 tokens 16 and 13, of 64 41 and 25, of 128 74 and 49; 8 of 100 61 and 49.
+// `tau`: decays are sigmoid(z)^(1/tau), 0 if not known.  Below 2 every batch of 32 tokens has a channel that decays to less than 2^-60
+// for a z around zero, so that the passes with outputs would prepare their batches and then walk: they stay with the register-tiled
+// kernel.  2,048 tokens of 16 heads, output pass (us, tiled and tensor cores): tau 1 121 and 176, tau 2 121 and 94 (176 when z is
+// around -2); 8 items of 100 in one pass 70 and 92, 70 and 61.  The local pass takes any decays: 72 and 43.
 #define GM_FROM 8
+#define GM_TAU 2.0f
 extern "C" int llm_gla_scan(
     const float* proj, long long stride, int q_off, int k_off, int v_off, int g_off, const float* la,
     const float* norm_w, float eps, float q_scale, float out_scale, void* out, int out_dtype, long long out_stride,
     int out_off, float* state, const int32_t* entry_slot, const int32_t* entry_q_start, const int32_t* entry_q_len,
-    const int32_t* items, int num_items, int mode, float* scratch_s, float* scratch_a, int H, int D, int V, int longest,
+    const int32_t* items, int num_items, int mode, float* scratch_s, float* scratch_a, int H, int D, int V, int longest, float tau,
     uintptr_t stream) {
     static const bool rows_forced = getenv("LLM_GLA_ROWS") != nullptr;
-    const bool taken = D == GM_D && V == GM_D && (longest <= 0 || longest >= GM_FROM) && !rows_forced && stride % 4 == 0 && q_off % 4 == 0 &&
+    const bool taken = D == GM_D && V == GM_D && (longest <= 0 || longest >= GM_FROM) && (mode == GLA_LOCAL || tau <= 0.0f || tau >= GM_TAU) && !rows_forced && stride % 4 == 0 && q_off % 4 == 0 &&
                        k_off % 4 == 0 && v_off % 4 == 0 && g_off % 4 == 0 && aligned16(proj) && aligned16(la) && norm_w && aligned16(norm_w);
     if (num_items <= 0 || !taken || H <= 0 || H > 65535 || mode < 0 || mode > 2 || (mode != GLA_FULL && (!items || !scratch_s || !scratch_a)) ||
         (mode != GLA_FULL && !aligned16(scratch_a)) || (out_dtype != LLM_DT_F32 && out_dtype != LLM_DT_BF16))

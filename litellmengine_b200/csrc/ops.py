@@ -977,13 +977,14 @@ def gla_decay(proj: torch.Tensor, a_off: int, rank: int, w2t: torch.Tensor, b2: 
 def gla_scan(proj: torch.Tensor, offs, alpha: torch.Tensor, norm_w: torch.Tensor, eps: float, q_scale: float,
              out_scale: float, out: torch.Tensor, out_off: int, state: torch.Tensor, entry_slot, entry_q_start,
              entry_q_len, items: Optional[torch.Tensor], num_items: int, mode: int,
-             scratch_s: Optional[torch.Tensor], scratch_a: Optional[torch.Tensor], H: int, D: int, V: int, longest: int = 0) -> None:
+             scratch_s: Optional[torch.Tensor], scratch_a: Optional[torch.Tensor], H: int, D: int, V: int, longest: int = 0,
+             tau: float = 0.0) -> None:
     """The recurrence S <- diag(alpha) S + k v^T, o = S^T q over the tokens of each work item, per head, with
     the per-head RMS norm of o (weight `norm_w` [V]), the silu output gate and `out_scale` applied before
     the store into columns out_off .. out_off + H*V of `out`.  `offs` = (q, k, v, g) column offsets in the
     float32 projection; `alpha` float32 [T, H*D] from `gla_decay`; `state` float32 [slots, H, D, V]; see
-    csrc/linear_attention.cu for the modes.  `longest`: tokens of the longest work item, 0 if not known (which
-    kernel is the faster one depends on it, no result does)."""
+    csrc/linear_attention.cu for the modes.  `longest`: tokens of the longest work item, `tau`: what `gla_decay`
+    was given, 0 if not known: which kernel is the faster one depends on them, and with it the roundings of 32-bit sums."""
     la = alpha
     _dev(la, norm_w, state, entry_slot, entry_q_start, entry_q_len, items, scratch_s, scratch_a)
     if (proj.dtype != torch.float32 or proj.stride(1) != 1 or la.dtype != torch.float32 or state.dtype != torch.float32
@@ -994,11 +995,11 @@ def gla_scan(proj: torch.Tensor, offs, alpha: torch.Tensor, norm_w: torch.Tensor
     f = _fn("linear_attention", "llm_gla_scan",
             [c_void_p, c_longlong, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_float, c_float, c_float, c_void_p,
              c_int, c_longlong, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_void_p,
-             c_void_p, c_int, c_int, c_int, c_int, c_void_p])
+             c_void_p, c_int, c_int, c_int, c_int, c_float, c_void_p])
     _check(f(_ptr(proj), proj.stride(0), q_off, k_off, v_off, g_off, _ptr(la), _ptr(norm_w), float(eps),
              float(q_scale), float(out_scale), _ptr(out), _dt(out), out.stride(0), out_off, _ptr(state),
              _ptr(entry_slot), _ptr(entry_q_start), _ptr(entry_q_len), _ptr(items), num_items, mode,
-             _ptr(scratch_s), _ptr(scratch_a), H, D, V, int(longest), _stream()), "gla_scan")
+             _ptr(scratch_s), _ptr(scratch_a), H, D, V, int(longest), float(tau), _stream()), "gla_scan")
 
 
 def gla_step(proj: torch.Tensor, offs, alpha: torch.Tensor, norm_w: torch.Tensor, eps: float, q_scale: float,

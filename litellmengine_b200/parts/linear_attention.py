@@ -169,16 +169,16 @@ class GatedLinearAttention(BranchMixer):
                   b.entry_q_start, b.entry_q_len)
         work = b.preludes.get(ScanWork.name)
         if work is None:                                     # no work lists: every entry in one pass
-            ops.gla_scan(*common, None, b.num_entries, ops.GLA_FULL, None, None, H, D, V, longest=b.max_q_len)
+            ops.gla_scan(*common, None, b.num_entries, ops.GLA_FULL, None, None, H, D, V, longest=b.max_q_len, tau=self.tau)
             return
         if work.num_short:
-            ops.gla_scan(*common, work.short, work.num_short, ops.GLA_FULL, None, None, H, D, V, longest=work.longest(b))
+            ops.gla_scan(*common, work.short, work.num_short, ops.GLA_FULL, None, None, H, D, V, longest=work.longest(b), tau=self.tau)
         if work.num_chunks:
             scratch_s = torch.empty((work.num_chunks, H, D, V), dtype=torch.float32, device=proj.device)
             scratch_a = torch.empty((work.num_chunks, H, D), dtype=torch.float32, device=proj.device)
-            ops.gla_scan(*common, work.chunks, work.num_chunks, ops.GLA_LOCAL, scratch_s, scratch_a, H, D, V)
+            ops.gla_scan(*common, work.chunks, work.num_chunks, ops.GLA_LOCAL, scratch_s, scratch_a, H, D, V, tau=self.tau)
             ops.gla_chain(ctx.state, scratch_s, scratch_a, work.chains, work.num_chains, b.entry_slot, H, D, V)
-            ops.gla_scan(*common, work.chunks, work.num_chunks, ops.GLA_OUT, scratch_s, scratch_a, H, D, V)
+            ops.gla_scan(*common, work.chunks, work.num_chunks, ops.GLA_OUT, scratch_s, scratch_a, H, D, V, tau=self.tau)
 
 
 class _HeadDecayRecurrence(BranchMixer):

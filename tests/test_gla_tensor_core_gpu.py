@@ -39,7 +39,7 @@ def plain(proj, alpha, state, lens, H):
     return out * torch.rsqrt(out.pow(2).mean(-1, keepdim=True) + 1e-5) * torch.nn.functional.silu(gate), end
 
 
-def run(proj, alpha, state, lens, H, chunk, longest=0):
+def run(proj, alpha, state, lens, H, chunk, longest=0, tau=0.0):
     """One pass over whole entries (chunk None) or over pieces of `chunk` tokens; float32 outputs and the states after."""
     T, B, o = sum(lens), len(lens), ops()
     starts = [sum(lens[:i]) for i in range(B)]
@@ -47,7 +47,7 @@ def run(proj, alpha, state, lens, H, chunk, longest=0):
     a = (proj, (0, H * D, 2 * H * D, 3 * H * D), alpha, torch.ones(D, device=DEV), 1e-5, D ** -0.5, 1.0, out, 4, state,
          i32(list(range(B))), i32(starts), i32(lens))
     if chunk is None:
-        o.gla_scan(*a, None, B, o.GLA_FULL, None, None, H, D, D, longest=longest)
+        o.gla_scan(*a, None, B, o.GLA_FULL, None, None, H, D, D, longest=longest, tau=tau)
     else:
         items, chains = [], []
         for e, n in enumerate(lens):
@@ -56,9 +56,9 @@ def run(proj, alpha, state, lens, H, chunk, longest=0):
         n = len(items)
         ss, sa = torch.empty(n, H, D, D, device=DEV), torch.empty(n, H, D, device=DEV)
         rows = i32(items + [(-1, 0, 0, 0)])
-        o.gla_scan(*a, rows, n + 1, o.GLA_LOCAL, ss, sa, H, D, D, longest=longest)
+        o.gla_scan(*a, rows, n + 1, o.GLA_LOCAL, ss, sa, H, D, D, longest=longest, tau=tau)
         o.gla_chain(state, ss, sa, i32(chains), B, i32(list(range(B))), H, D, D)
-        o.gla_scan(*a, rows, n + 1, o.GLA_OUT, ss, sa, H, D, D, longest=longest)
+        o.gla_scan(*a, rows, n + 1, o.GLA_OUT, ss, sa, H, D, D, longest=longest, tau=tau)
     assert bool((out[:, :4] == 7).all())
     return out[:, 4:].view(T, H, D), state
 
@@ -145,3 +145,21 @@ def test_a_state_that_is_not_finite_or_does_not_split(chunk, what):
     assert not bool(torch.isnan(out[:, 0]).any()) and not bool(torch.isnan(out[40:]).any())        # the other head, the other entry
     near = lambda a, b: float(((a - b).abs() / (1e-3 + b.abs()))[torch.isfinite(b)].max()) < 1e-3
     assert near(out, want) and near(state, end)
+
+
+@pytest.mark.parametrize("chunk", [None, 64])
+def test_strong_decays_stay_with_the_register_tiled_kernel(chunk):
+    """Below tau = 2 the passes with outputs are the register-tiled kernel's, from 2 on (or unknown) the tensor cores'."""
+    lens, H = [100, 64], 3
+    x = inputs(lens, H, 0.5, torch.Generator(device=DEV).manual_seed(23))
+    tensor, tiled = run(*x, lens, H, chunk), run(*x, lens, H, chunk, longest=1)
+    assert not torch.equal(tensor[0], tiled[0])
+    same = lambda a, b: all(torch.equal(i, j) for i, j in zip(a, b))
+    assert same(run(*x, lens, H, chunk, tau=2.0), tensor) and same(run(*x, lens, H, chunk, tau=64.0), tensor)
+    for tau in (0.1, 1.0, 1.99):
+        got = run(*x, lens, H, chunk, tau=tau)
+        if chunk is None:
+            assert same(got, tiled)
+        else:                                                 # the local pass takes any decays
+            assert torch.equal(got[1], tensor[1]) and not torch.equal(got[0], tensor[0])
+            assert float((got[0] - tiled[0]).abs().max()) < 1e-4
