@@ -22,14 +22,25 @@ class ScanWork(StepPrelude):
     the request's state.  A longer portion is cut into chunks of `CHUNK` tokens that run side by side:
     every chunk first computes its own contribution from a zero state, a chain kernel then walks each
     entry's chunks in order to find the state that enters each, and a second pass over the chunks
-    produces the outputs.  The line lies where the three passes take less time than the one, for every kind of
-    recurrence (one entry, 16 heads of 128 x 128, one pass and three in us: decays per channel, 96 tokens 37 and 37,
-    128 49 and 37, 200 83 and 37; one decay per head, 100 79 and 86, 128 96 and 86, 200 148 and 86; with a
-    normaliser 91 and 101, 111 and 101, 170 and 101).  Items are int32 (entry, first row, tokens, scratch index); chains (entry,
-    first scratch index, chunks)."""
+    produces the outputs.  Items are int32 (entry, first row, tokens, scratch index); chains (entry,
+    first scratch index, chunks).
+
+    Portions shorter than `ALWAYS_FROM` are cut only while their chunks' blocks, one a head, find an SM each, or from
+    `LONG` tokens on average two to an SM: with more of them one pass fills the SMs, and three do the tokens twice.
+    `heads` of the first mixer that asks.  One pass and three (us), 16 heads of 128 x 128, entries x tokens: decays
+    per channel 1 x 130 70 and 46, 3 x 130 72 and 52, 4 x 130 72 and 73, 4 x 250 113 and 76, 6 x 250 113 and 116, 16 x
+    130 117 and 212; one decay per head 1 x 130 119 and 99, 3 x 130 121 and 105, 4 x 130 121 and 123, 4 x 190 166 and
+    193, 4 x 250 213 and 194, 6 x 250 217 and 282; with a normaliser 139 and 117, 139 and 132, 141 and 158, 191 and
+    238, 248 and 241, 250 and 353.  Of 100 tokens one pass is level (37 and 37 per channel) or ahead (79 and 86)."""
     name = "scan_work"
     CHUNK = 64
     CHUNKED_FROM = 128
+    ALWAYS_FROM = 256
+    LONG = 192
+    SMS = 148
+
+    def __init__(self, heads: int = 1):
+        self.heads = heads
 
     @dataclass
     class Views:
@@ -42,8 +53,8 @@ class ScanWork(StepPrelude):
         longest_short: int = -1      # tokens of the longest entry that runs in one pass, once somebody has asked
 
         def longest(self, batch) -> int:
-            if self.longest_short < 0:
-                self.longest_short = max((n for n in (len(e.tokens) for e in batch.entries) if n < ScanWork.CHUNKED_FROM), default=0)
+            if self.longest_short < 0:              # those in one pass are the shortest ones
+                self.longest_short = sorted(len(e.tokens) for e in batch.entries)[self.num_short - 1] if self.num_short else 0
             return self.longest_short
 
     def sections(self, max_tokens: int, max_entries: int):
@@ -52,8 +63,13 @@ class ScanWork(StepPrelude):
 
     def fill(self, facts, out):
         short, chunks, chains = [], [], []
-        for i, (q0, n) in enumerate(zip(facts.q_start.tolist(), facts.q_len.tolist())):
-            if n < self.CHUNKED_FROM:
+        lens = facts.q_len.tolist()
+        between = [n for n in lens if self.CHUNKED_FROM <= n < self.ALWAYS_FROM]
+        blocks = sum(-(-n // self.CHUNK) for n in between) * self.heads
+        cut = blocks <= self.SMS * (2 if sum(between) >= self.LONG * len(between) else 1)
+        chunked_from = self.CHUNKED_FROM if cut else self.ALWAYS_FROM
+        for i, (q0, n) in enumerate(zip(facts.q_start.tolist(), lens)):
+            if n < chunked_from:
                 short.append((i, q0, n, 0))
                 continue
             first = len(chunks)
@@ -145,7 +161,7 @@ class GatedLinearAttention(BranchMixer):
         return StateNeed((self.H, self.D, self.V), "float32")
 
     def step_prelude(self):
-        return ScanWork()
+        return ScanWork(self.H)
 
     graph_variant_group = ("scan_work",)
 
@@ -215,7 +231,7 @@ class _HeadDecayRecurrence(BranchMixer):
         return StateNeed((self.H, self.head_floats), "float32")
 
     def step_prelude(self):
-        return ScanWork()
+        return ScanWork(self.H)
 
     def graph_variant(self, batch, padded: bool):
         work = batch.preludes.get(ScanWork.name)
