@@ -882,6 +882,7 @@ def latent_attention(q: torch.Tensor, rows_cache: torch.Tensor, positions, token
 
 # ---- gated linear attention ------------------------------------------------------------------
 GLA_FULL, GLA_LOCAL, GLA_OUT = 0, 1, 2
+GLA_TENSOR_FROM = 8         # tokens of the longest item from which `gla_scan` may take the tensor cores (csrc/linear_attention.cu)
 
 
 def latent_prefill_supported(D: int, V: int, R: int, P: int) -> bool:

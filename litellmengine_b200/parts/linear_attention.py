@@ -57,6 +57,11 @@ class ScanWork(StepPrelude):
                 self.longest_short = sorted(len(e.tokens) for e in batch.entries)[self.num_short - 1] if self.num_short else 0
             return self.longest_short
 
+        def variant(self, batch):
+            """What a captured graph of the step depends on: the lists' lengths, and on which side of the tensor-core
+            kernel's line the items in one pass are (`ops.gla_scan`), so that a replay launches what the step would."""
+            return self.num_short, self.num_chunks, self.num_chains, self.longest(batch) >= ops.GLA_TENSOR_FROM
+
     def sections(self, max_tokens: int, max_entries: int):
         return {"short": 4 * max_entries, "chunks": 4 * (max_tokens // self.CHUNK + max_entries),
                 "chains": 3 * max_entries}
@@ -167,7 +172,7 @@ class GatedLinearAttention(BranchMixer):
 
     def graph_variant(self, batch, padded: bool):
         work = batch.preludes.get(ScanWork.name)
-        return (work.num_short, work.num_chunks, work.num_chains) if work is not None else 0
+        return work.variant(batch) if work is not None else 0
 
     def mix(self, proj, col0, ctx: StageContext, out, out_col0, out_scale):
         b, (H, D, V) = ctx.batch, (self.H, self.D, self.V)
@@ -235,7 +240,7 @@ class _HeadDecayRecurrence(BranchMixer):
 
     def graph_variant(self, batch, padded: bool):
         work = batch.preludes.get(ScanWork.name)
-        return (work.num_short, work.num_chunks, work.num_chains) if work is not None else 0
+        return work.variant(batch) if work is not None else 0
 
     def _load_in_out(self, t, keys) -> None:
         n = self.names
