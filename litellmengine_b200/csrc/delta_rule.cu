@@ -1479,9 +1479,10 @@ static int delta_shape(DeltaShape& s, int H, int G, int D, int V, int taps, int 
 // 114, 114, 8: 101, 90, 4: 92, 86; but 1 x 1,000, 8: 169, 176; 1 x 2,500, 8: 382, 398; 1 x 100, 16: 60, 64; 4 x 200, 16: 123, 128; 32 x 64,
 // 16: 259, 276.  So: portions of 256 tokens and more, 1,500 columns and more, two blocks an SM at most.
 extern "C" int llm_delta_image_bytes() { return DX_IMAGE; }
+static bool dx_takes(int H, int D, int V) { return D == 128 && V > 0 && V % DX_COLS == 0 && H > 0 && H <= 65535; }
 extern "C" int llm_delta_batched(int H, int D, int V, int num_entries, int max_len) {
     const long long columns = static_cast<long long>(num_entries) * H * V;
-    return D == 128 && V > 0 && V % DX_COLS == 0 && H > 0 && H <= 65535 && max_len >= 256 && columns >= 1500 && columns <= 2 * DR_SMS * DX_COLS;
+    return dx_takes(H, D, V) && max_len >= 256 && columns >= 1500 && columns <= 2 * DR_SMS * DX_COLS;
 }
 
 // Everything of a step that is not all single tokens.  Scratch (float32): qn, kn [T, G, DP], vn [T, H, VP], beta [T, H],
@@ -1543,7 +1544,7 @@ extern "C" int llm_delta_scan(
 #undef LOWRANK
     const long long walks = static_cast<long long>(num_tokens) * H;
     if (images) {
-        if (!llm_delta_batched(H, D, V, num_entries, max_len) || !aligned16(images)) return LLM_REFUSED_SIZE;
+        if (!dx_takes(H, D, V) || !aligned16(images)) return LLM_REFUSED_SIZE;
         static_assert(DX_IMAGE <= DX_ROWS && DX_IMAGE % 16 == 0, "the image takes the vectors' place");
         constexpr int most = DX_SMEM > DR_ALONE_SMEM ? DX_SMEM : DR_ALONE_SMEM;
         cudaError_t e = cudaFuncSetAttribute(delta_batch_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, DX_BATCH_SMEM);

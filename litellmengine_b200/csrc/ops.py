@@ -1157,6 +1157,12 @@ def delta_supported(d: int, v: int) -> bool:
     return bool(_fn("delta_rule", "llm_delta_supported", [c_int, c_int])(d, v))
 
 
+def delta_batched(batch, H: int, D: int, V: int) -> bool:
+    """Whether `delta_rule` takes its tensor-core kernels for this step (csrc/delta_rule.cu has the rule).  They are right
+    for any division of a step's tokens, so a captured graph may hold them: the answer is part of its key."""
+    return bool(_fn("delta_rule", "llm_delta_batched", [c_int] * 5)(H, D, V, batch.num_entries, getattr(batch, "max_q_len", 0)))
+
+
 def delta_rule(proj: torch.Tensor, offs, ranks, conv_w: torch.Tensor, w_decay: torch.Tensor, w_gate: torch.Tensor,
                dt_bias: torch.Tensor, a_log: torch.Tensor, norm_w: torch.Tensor, eps: float, out_scale: float, out: torch.Tensor,
                out_off: int, state: torch.Tensor, batch, H: int, G: int, D: int, V: int, single: bool = False) -> None:
@@ -1191,7 +1197,7 @@ def delta_rule(proj: torch.Tensor, offs, ranks, conv_w: torch.Tensor, w_decay: t
     DP, VP = delta_padded(D), (V + 3) // 4 * 4
     # a graph that is being captured serves other divisions of its tokens too
     longest = 0 if getattr(batch, "any_division", False) else getattr(batch, "max_q_len", 0)
-    batched = _fn("delta_rule", "llm_delta_batched", [c_int] * 5)(H, D, V, batch.num_entries, longest)
+    batched = delta_batched(batch, H, D, V)
     if batched:                                             # images of what sixteen tokens share
         shared = ((T // 16 + batch.num_entries + 1) * H * (_fn("delta_rule", "llm_delta_image_bytes", [])() // 4),)
     else:                                                   # places for what the eight tokens of a chunk share

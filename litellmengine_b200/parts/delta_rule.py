@@ -29,8 +29,8 @@ class DeltaRuleMixer(BranchMixer):
     g1] per token in float32, and nothing of the recurrence is rounded after it.  A request's slot holds the states and
     the convolutions' last inputs in one row of floats (the kernels' layout, see csrc/delta_rule.cu)."""
 
-    graph_safe = True            # kernels on the current stream only; their grids follow the step's entries
-    any_division_safe = False
+    graph_safe = True            # kernels on the current stream only; their grids follow the step's entries,
+    any_division_safe = False    # and which kernels they are is part of a graph's key (see graph_variant)
 
     PADDED = (32, 64, 128, 256)  # what the kernels are instantiated for
 
@@ -96,6 +96,13 @@ class DeltaRuleMixer(BranchMixer):
     def cache_need(self):
         floats = self.H * self.V * self.padded + self.taps * self.channels
         return StateNeed(((floats + 3) // 4 * 4,), "float32")
+
+    @property
+    def graph_variant_group(self):
+        return ("delta_rule", self.H, self.D, self.V)
+
+    def graph_variant(self, batch, padded: bool):
+        return batch.max_q_len > 1 and ops.delta_batched(batch, self.H, self.D, self.V)
 
     def mix(self, proj, col0, ctx: StageContext, out, out_col0, out_scale):
         if ctx.state is None:

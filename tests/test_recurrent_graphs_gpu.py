@@ -36,6 +36,8 @@ def states_after(runner, slots, lens):
 @pytest.mark.parametrize("kind,heads,lens,other", [
     ("gla", 2, [1, 1, 1, 25], [7, 7, 7, 7]),                   # one pass, items on both sides of the tensor-core kernel's line
     ("gla", 2, [7, 7, 7, 7], [1, 1, 1, 25]),
+    ("channel_delta", 12, [300, 1], [150, 151]),               # portions on both sides of the tensor-core kernels' line
+    ("channel_delta", 12, [150, 151], [300, 1]),
 ])
 def test_replayed_steps_launch_what_the_step_would(kind, heads, lens, other):
     runner = runner_of(kind, heads)
