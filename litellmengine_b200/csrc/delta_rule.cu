@@ -548,10 +548,12 @@ template <int C> __device__ __forceinline__ void dr_row(float (&v)[C], const flo
 }
 
 // The convolutions' inputs of a portion's last tokens go into the request's ring (the kernels before the scan have read it): by each
-// block of a scan its columns' values, and the head's queries and keys by one.
+// block of a scan its columns' values, and the head's queries and keys by one.  THREADS: of the block, 0: as it was launched.
+template <int THREADS>
 __device__ __forceinline__ void dr_keep_inputs(const DeltaShape& s, const float* __restrict__ proj, float* slot, const int32_t* __restrict__ positions,
                                                long long row0, int count, int h, int c0, int cols, bool first) {
     const int channels = 2 * s.G * s.D + s.H * s.V, keep = min(count, s.taps - 1), kvh = h / (s.H / s.G);
+    const auto threads = [] { if constexpr (THREADS > 0) return THREADS; else return blockDim.x; }();
     float* ring = slot + s.ring_off;
     const bool with_qk = first && h % (s.H / s.G) == 0;
     for (int i = 0; i < keep; ++i) {
@@ -559,11 +561,11 @@ __device__ __forceinline__ void dr_keep_inputs(const DeltaShape& s, const float*
         float* dst = ring + static_cast<long long>(positions[t] % s.taps) * channels;
         const float* src = proj + t * s.stride + s.q_off;
         if (with_qk)
-            for (int d = threadIdx.x; d < s.D; d += blockDim.x) {
+            for (int d = threadIdx.x; d < s.D; d += threads) {
                 dst[kvh * s.D + d] = src[kvh * s.D + d];
                 dst[(s.G + kvh) * s.D + d] = src[(s.G + kvh) * s.D + d];
             }
-        for (int x = threadIdx.x; x < cols && c0 + x < s.V; x += blockDim.x) {
+        for (int x = threadIdx.x; x < cols && c0 + x < s.V; x += threads) {
             const int ch = 2 * s.G * s.D + h * s.V + c0 + x;
             dst[ch] = src[ch];
         }
@@ -764,7 +766,9 @@ __global__ void __launch_bounds__(WARPS * 32) delta_scan_kernel(
 #pragma unroll
             for (int j = 0; j < R / 4; ++j)
                 *reinterpret_cast<float4*>(col_state + m * DP + 4 * L * j) = make_float4(S[m][4 * j], S[m][4 * j + 1], S[m][4 * j + 2], S[m][4 * j + 3]);
-    dr_keep_inputs(s, proj, slot, positions, row0, count, h, c0, COLS, tile == 0);
+    // The block's size as a constant moves the registers of the walk above (us, launch's size and constant): one column a warp 172 and
+    // 181 (1,000 tokens, 4 heads); two 190 and 184 (8 heads); four 643 and 636 (2,500 tokens beside 16 single ones, 16 heads).
+    dr_keep_inputs<C == 1 ? 0 : THREADS>(s, proj, slot, positions, row0, count, h, c0, COLS, tile == 0);
 }
 
 // A warp per (token, head): o / rms(o) * w * gate * scale.
@@ -1245,7 +1249,7 @@ __global__ void __launch_bounds__(256, 2) delta_scan_mma_kernel(
         *reinterpret_cast<float2*>(my_state + 8 * n) = make_float2(S[n][0], S[n][1]);
         *reinterpret_cast<float2*>(my_state + 8 * D + 8 * n) = make_float2(S[n][2], S[n][3]);
     }
-    dr_keep_inputs(s, proj, slot, positions, row0, count, h, c0, DX_COLS, tile == 0);
+    dr_keep_inputs<256>(s, proj, slot, positions, row0, count, h, c0, DX_COLS, tile == 0);
 }
 
 template <typename TO>
