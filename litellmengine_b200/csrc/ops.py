@@ -1910,8 +1910,8 @@ _stream_status: Dict[str, torch.Tensor] = {}
 
 
 def stream_status(device) -> torch.Tensor:
-    """The status word of the engine's matrix products (code 8: a bounded wait of the weight-streaming
-    product ran out; 9: of the paired or the float32 tcgen05 product)."""
+    """The status word of the engine's matrix products and of the delta rule (code 8: a bounded wait of the weight-streaming
+    product ran out; 9: of the paired or the float32 tcgen05 product; 11: of the delta rule's tensor-core scan)."""
     key = str(device)
     t = _stream_status.get(key)
     if t is None:

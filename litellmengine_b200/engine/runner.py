@@ -23,7 +23,8 @@ STATUS_TEXT = {1: "a token id outside the vocabulary reached the embedding kerne
                5: "a wait on a copy barrier in the decode attention kernel ran out",
                6: "a wait on a barrier in the tcgen05 prompt attention kernel ran out",
                8: "a wait on a copy barrier in the weight-streaming product ran out",
-               9: "a wait on a barrier in a tcgen05 product (the paired one or the float32 one) ran out"}
+               9: "a wait on a barrier in a tcgen05 product (the paired one or the float32 one) ran out",
+               11: "a wait on a copy barrier in the delta rule's tensor-core scan ran out"}
 
 
 class ModelRunner:

@@ -1,6 +1,8 @@
 """The engine against the plain implementation, in float32 and in bfloat16, for every way of
 cutting the work: whole, a tail decoded token by token, portions of changing size, and mixed
 batches of up to four live requests over so few pages that they are used again."""
+import re
+
 import numpy as np
 import pytest
 import torch
@@ -158,11 +160,11 @@ def test_a_status_code_in_either_word_is_raised_and_cleared():
     from litellmengine_b200.engine.runner import STATUS_TEXT
     cfg, page, w, _ = setup("A", "float32")
     runner = rh.make_runner(cfg, w, "float32", page, max_total_tokens=16, max_requests=2)
-    assert set(STATUS_TEXT) == {1, 2, 3, 4, 5, 6, 8, 9}
+    assert set(STATUS_TEXT) == {1, 2, 3, 4, 5, 6, 8, 9, 11}
     for word, code in ((runner.buffers.status, 4), (ops.stream_status(runner.device), 8),
-                       (ops.stream_status(runner.device), 9), (runner.buffers.status, 6)):
+                       (ops.stream_status(runner.device), 9), (runner.buffers.status, 6), (ops.stream_status(runner.device), 11)):
         word.copy_(torch.tensor([code, 123], dtype=torch.int32))
-        with pytest.raises(RuntimeError, match=f"device status {code}: .*index 123"):
+        with pytest.raises(RuntimeError, match=f"device status {code}: {re.escape(STATUS_TEXT[code])} .*index 123"):
             runner.check_status()
         runner.check_status()                                   # cleared by the raise
 
