@@ -414,16 +414,19 @@ __global__ void __launch_bounds__(1024) latent_q_pack_kernel(const float* __rest
     const int t = blockIdx.x, half = dims / 2, W = D + P;
     const float* src = q + static_cast<size_t>(t) * H * W;
     bf16* dst = out + static_cast<size_t>(t) * H * W;
-    // a thread keeps its place in the head and goes from head to head, LQ_HELD heads on their way at once
-    const int per = blockDim.x / (W / 8), c = static_cast<int>(threadIdx.x % (W / 8)) * 8, k0 = c - D, h0 = threadIdx.x / (W / 8);
+    // a thread keeps its place in the head and goes from head to head, LQ_HELD heads on their way at once; a head of more eights than a
+    // block has threads is a row of blocks
+    const int eights = W / 8, blk = blockDim.x, wide = eights > blk, per = wide ? 1 : blk / eights;
+    const int c = static_cast<int>(wide ? blockIdx.y * blk + threadIdx.x : threadIdx.x % eights) * 8, k0 = c - D, h0 = wide ? 0 : threadIdx.x / eights;
+    const int heads = c < W ? H : 0;
     const bool whole = k0 >= 0 && k0 + 8 <= dims && (rot_pairs || half % 8 == 0);      // all eight turn, with neighbours or with eight others
     const bool first = k0 < half;
     const int f0 = rot_pairs ? k0 >> 1 : first ? k0 : k0 - half;
-    for (int hb = h0; hb < H || hb == h0; hb += LQ_HELD * per) {
+    for (int hb = h0; hb < heads || hb == h0; hb += LQ_HELD * per) {
         float v[LQ_HELD][8];
 #pragma unroll
         for (int j = 0; j < LQ_HELD; ++j)
-            if (hb + j * per < H) load8(src + (hb + j * per) * W + c, v[j]);
+            if (hb + j * per < heads) load8(src + (hb + j * per) * W + c, v[j]);
         if (hb == h0) {
             const float pos = static_cast<float>(positions[t]);
             for (int f = threadIdx.x; f < half; f += blockDim.x) {
@@ -436,7 +439,7 @@ __global__ void __launch_bounds__(1024) latent_q_pack_kernel(const float* __rest
 #pragma unroll
         for (int j = 0; j < LQ_HELD; ++j) {
             const int h = hb + j * per;
-            if (h >= H) break;
+            if (h >= heads) break;
             const float* hd = src + h * W;
             if (whole && rot_pairs) {
 #pragma unroll
@@ -496,9 +499,10 @@ extern "C" int llm_latent_q_pack(const float* q, void* out, const int32_t* posit
     if (num_tokens <= 0) return LLM_OK;
     if (H <= 0 || D <= 0 || P < 0 || D % 8 || P % 8 || dims < 0 || dims > P || dims % 2 || (dims > 0 && !inv_freq)) return LLM_REFUSED_SIZE;
     if (!aligned16(q) || !aligned16(out)) return LLM_REFUSED_ALIGN;
-    const int eights = (D + P) / 8;                               // threads: as many whole heads as 256 of them hold
-    if (eights > 1024) return LLM_REFUSED_SIZE;
-    launch_pdl(latent_q_pack_kernel, dim3(num_tokens), dim3(eights > 256 ? eights : 256 / eights * eights), sizeof(float2) * (dims / 2), reinterpret_cast<cudaStream_t>(stream),
+    const int eights = (D + P) / 8;                               // threads: as many whole heads as 256 of them hold, or one, or a part of it
+    const int threads = eights > 1024 ? 1024 : eights > 256 ? eights : 256 / eights * eights, parts = (eights + 1023) / 1024;
+    if (parts > 65535) return LLM_REFUSED_SIZE;
+    launch_pdl(latent_q_pack_kernel, dim3(num_tokens, parts), dim3(threads), sizeof(float2) * (dims / 2), reinterpret_cast<cudaStream_t>(stream),
                q, static_cast<bf16*>(out), positions, inv_freq, H, D, P, dims, rot_pairs, rot_mag);
     return launch_status();
 }

@@ -78,6 +78,31 @@ def test_kernels(H, R, window):
         assert bool(((got - ref).abs() <= bound).all()), (n, t, float(((got - ref).abs() / bound).max()))
 
 
+
+@pytest.mark.parametrize("H,D,P,dims", [(50, 128, 64, 64), (41, 128, 64, 20), (3, 128, 64, 36), (2, 64, 32, 0), (90, 8, 8, 6), (1, 2048, 64, 64), (2, 8184, 8, 8),
+                                        (3, 8192, 64, 48), (1, 24640, 64, 64)])
+@pytest.mark.parametrize("pairs", [False, True])
+def test_queries_are_packed_whatever_the_heads(H, D, P, dims, pairs):
+    """More heads than a block takes at once, angles that cover parts of a group of eight, heads wider than a block."""
+    o, T = ops(), 5
+    g = torch.Generator(device=DEV).manual_seed(H + D)
+    q = torch.randn(T, H * (D + P), generator=g, device=DEV)
+    pos = torch.tensor([0, 1, 7, 500, 40000], dtype=torch.int32, device=DEV)
+    inv = torch.rand(max(1, dims // 2), generator=g, device=DEV)
+    got = o.latent_q_pack(q, pos, inv, H, D, P, dims, rot_pairs=pairs, rot_mag=1.25).view(T, H, D + P)
+    x = q.view(T, H, D + P).to(F64).clone()
+    angle = (pos.float()[:, None] * inv[:dims // 2]).to(F64)          # the product is a 32-bit one
+    c, s = 1.25 * torch.cos(angle)[:, None], 1.25 * torch.sin(angle)[:, None]
+    part = x[..., D:D + dims]
+    u, v = (slice(0, dims, 2), slice(1, dims, 2)) if pairs else (slice(0, dims // 2), slice(dims // 2, dims))
+    a, b = part[..., u].clone(), part[..., v].clone()
+    part[..., u], part[..., v] = a * c - b * s, b * c + a * s
+    assert torch.equal(got[..., :D], q.view(T, H, D + P)[..., :D].to(torch.bfloat16))
+    assert torch.equal(got[..., D + dims:], q.view(T, H, D + P)[..., D + dims:].to(torch.bfloat16))
+    # one rounding to bfloat16 of a number that is a few 2^-24 off
+    assert bool(((got.to(F64) - x).abs() <= 2.0 ** -8 * x.abs() + 1e-5).all())
+
+
 @pytest.mark.parametrize("window", [None, 200])
 def test_long_step_of_every_kind_of_entry(window):
     """Portions with and without earlier tokens beside single tokens, in one step, over both paths."""
