@@ -1478,15 +1478,21 @@ static int delta_shape(DeltaShape& s, int H, int G, int D, int V, int taps, int 
 
 // Whether llm_delta_scan takes the tensor-core kernels: it is then given room for llm_delta_image_bytes() a batch of sixteen tokens and
 // head (T / 16 + entries + 1 places) instead of pk, pq, total and num.  Their fixed part is larger, and few columns spread thinner over
-// the SMs than with a warp to one to four of them.  Whole calls (us, eight tokens a chunk and this; entries x longest portion, heads):
-// 1 x 300, 16: 93, 90; 1 x 1,000, 16: 229, 209; 1 x 2,500, 16: 535, 473; 3 x 849, 16: 265, 238, 8: 224, 185, 4: 182, 155; 3 x 300, 16:
-// 114, 114, 8: 101, 90, 4: 92, 86; but 1 x 1,000, 8: 169, 176; 1 x 2,500, 8: 382, 398; 1 x 100, 16: 60, 64; 4 x 200, 16: 123, 128; 32 x 64,
-// 16: 259, 276.  So: portions of 256 tokens and more, 1,500 columns and more, two blocks an SM at most.
+// the SMs than with a warp to one to four of them; single tokens of other requests count, since the kernels of eight tokens give each
+// warp more columns for them.  Whole calls (us, eight tokens a chunk and this; portions + single tokens, heads of 128 columns):
+//   1,536 and 2,048 columns: 300, 16: 108, 114; 1,000, 16: 219, 219; 2,500, 16: 481, 500; 300 + 1, 8: 119, 125; but 1,000 + 1, 8: 201, 200;
+//   2,500 + 1, 8: 428, 424; 2,500 + 1, 6: 410, 398; 2,500 + 3, 4: 420, 393; 2,500 + 8, 2: 404, 383
+//   more: 300 + 1, 16: 123, 117; 1,000 + 1, 16: 266, 225; 1,000 + 2, 8: 250, 198; 1,000, 24: 287, 254; 2,500, 32: 726, 652; 300 + 300, 16:
+//   129, 123; 284 + 567, 16: 182, 165; 260 + 5, 4: 127, 117
+//   portions below 256: 100, 16: 60, 64; 4 x 200, 16: 123, 128; 32 x 64, 16: 259, 276
+// So: 256 tokens and more; more than 2,048 columns, or 1,500 where several requests share a step with a portion of 1,000 tokens; two
+// blocks an SM at most.
 extern "C" int llm_delta_image_bytes() { return DX_IMAGE; }
 static bool dx_takes(int H, int D, int V) { return D == 128 && V > 0 && V % DX_COLS == 0 && H > 0 && H <= 65535; }
 extern "C" int llm_delta_batched(int H, int D, int V, int num_entries, int max_len) {
     const long long columns = static_cast<long long>(num_entries) * H * V;
-    return dx_takes(H, D, V) && max_len >= 256 && columns >= 1500 && columns <= 2 * DR_SMS * DX_COLS;
+    const bool enough = columns > 2048 || (columns >= 1500 && num_entries > 1 && max_len >= 1000);
+    return dx_takes(H, D, V) && max_len >= 256 && enough && columns <= 2 * DR_SMS * DX_COLS;
 }
 
 // Everything of a step that is not all single tokens.  Scratch (float32): qn, kn [T, G, DP], vn [T, H, VP], beta [T, H],

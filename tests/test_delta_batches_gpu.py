@@ -22,17 +22,19 @@ def setup(H, G, V, lens, dt_std, seed):
     starts = [sum(lens[:i]) for i in range(len(lens))]
     batch = types.SimpleNamespace(positions=i32([p for n in lens for p in range(n)]), token_entry=i32([e for e, n in enumerate(lens) for _ in range(n)]),
                                   entry_slot=i32(list(range(len(lens)))), entry_q_start=i32(starts), entry_q_len=i32(lens), num_entries=len(lens),
-                                  max_q_len=4096)             # long enough for the batches' kernels to be taken
+                                  max_q_len=max(lens))
     return w, batch, starts
 
 
-def run(w, batch, H, G, V):
+def run(w, batch, H, G, V, batched=True):
+    """With the kernels of sixteen tokens a batch, or of eight, whatever the sizes would have chosen."""
     from litellmengine_b200.csrc import ops
     C = 2 * G * 128 + H * V
-    assert ops._fn("delta_rule", "llm_delta_batched", [ops.c_int] * 5)(H, 128, V, batch.num_entries, batch.max_q_len)
     state, out = w["state"].clone(), torch.zeros(w["proj"].shape[0], H * V, device=DEV)
-    ops.delta_rule(w["proj"], (0, C, C + H, C + H + RA), (RA, RG), w["conv"], w["wa"], w["wg"], w["dt"], w["al"], w["nw"], EPS, 1.0, out, 0, state,
-                   batch, H, G, 128, V, single=False)
+    with pytest.MonkeyPatch.context() as m:
+        m.setattr(ops, "delta_batched", lambda *a: batched)
+        ops.delta_rule(w["proj"], (0, C, C + H, C + H + RA), (RA, RG), w["conv"], w["wa"], w["wg"], w["dt"], w["al"], w["nw"], EPS, 1.0, out, 0,
+                       state, batch, H, G, 128, V, single=False)
     assert ops.stream_status(DEV).tolist() == [0, 0]
     return out, state
 
@@ -98,13 +100,41 @@ def test_no_further_from_64_bits_than_the_kernels_of_eight_tokens():
             S = torch.baddbmm(S, k[t][:, :, None], (beta[t][:, None] * (v[t] - (k[t][:, None, :] @ S)[:, 0]))[:, None, :])
             ref[t] = (q[t][:, None, :] @ S)[:, 0]
         ref = ref * torch.rsqrt(ref.pow(2).mean(-1, keepdim=True) + EPS) * w["nw"].to(F64) * torch.sigmoid(x[:, C + H + RA:] @ w["wg"].to(F64)).view(n, H, V)
-        for form, longest in (("batches", n), ("eight", 0)):
-            batch.max_q_len = longest
-            state, out = w["state"].clone(), torch.zeros(n, H * V, device=DEV)
-            from litellmengine_b200.csrc import ops
-            ops.delta_rule(w["proj"], (0, C, C + H, C + H + RA), (RA, RG), w["conv"], w["wa"], w["wg"], w["dt"], w["al"], w["nw"], EPS, 1.0, out, 0, state,
-                           batch, H, H, D, V, single=False)
+        for form in err:
+            out, state = run(w, batch, H, H, V, form == "batches")
             got = state[0, :H * V * D].view(H, V, D).transpose(1, 2).to(F64)
             err[form][0] += float((out.view(n, H, V) - ref).norm() / ref.norm())
             err[form][1] += float((got - S).norm() / S.norm())
     assert err["batches"][0] <= err["eight"][0] and err["batches"][1] <= err["eight"][1], err
+
+
+@pytest.mark.parametrize("H,V,entries,longest,want", [
+    (16, 128, 3, 255, False), (16, 128, 3, 256, True), (16, 128, 1, 8000, False), (17, 128, 1, 256, True),       # 2,048 and 2,176 columns
+    (6, 128, 2, 999, False), (6, 128, 2, 1000, True), (12, 128, 1, 1000, False), (11, 128, 1, 1000, False),        # 1,536: one request, two
+    (37, 128, 2, 256, True), (38, 128, 2, 256, False), (16, 48, 6, 300, False), (16, 96, 6, 300, True), (16, 128, 0, 300, False)])
+def test_which_kernels_a_step_takes(H, V, entries, longest, want):
+    from litellmengine_b200.csrc import ops
+    assert ops.delta_batched(types.SimpleNamespace(num_entries=entries, max_q_len=longest), H, 128, V) == want
+    assert not ops.delta_batched(types.SimpleNamespace(num_entries=entries, max_q_len=longest), H, 64, V)
+
+
+def test_a_portion_beside_single_tokens_and_states_that_are_not_finite():
+    """Against the kernels of eight tokens, which take every column by itself: a portion beside decoding requests, decays of zero and one,
+    and states that hold infinities, NaN and numbers beyond 2^60 in single places."""
+    H, V, lens = 4, 64, [70, 1, 1, 33, 1]
+    w, batch, starts = setup(H, H, V, lens, 1.0, 3)
+    C = 2 * H * 128 + H * V
+    w["dt"][:128:3], w["dt"][1:128:3] = -200.0, 3e4            # decays of one and of zero
+    S = w["state"][:, :H * V * 128].view(len(lens), H, V, 128)
+    S[0, 1, 5, 9], S[0, 2, 40, 100], S[1, 0, 3, 3], S[3, 3, 63, 127], S[3, 0, 0, 0] = float("inf"), float("nan"), 1e30, float("-inf"), 3e38
+    out, state = run(w, batch, H, H, V)
+    ref, end = run(w, batch, H, H, V, False)
+    assert torch.equal(torch.isfinite(state), torch.isfinite(end))
+    ok = torch.isfinite(end)
+    assert float(((state - end).abs() / (1e-2 + end.abs()))[ok].max()) < 1e-3
+    # outputs: what an infinity gives depends on the order of a sum, so those heads are left out
+    for e, (a, n) in enumerate(zip(starts, lens)):
+        for h in range(H):
+            if (e, h) not in ((0, 1), (0, 2), (3, 0), (3, 3)):
+                x, y = (t[a:a + n, h * V:(h + 1) * V] for t in (out, ref))
+                assert float(((x - y).abs() / (1e-2 + y.abs())).max()) < 1e-3, (e, h)
