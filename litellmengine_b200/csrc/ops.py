@@ -1198,16 +1198,23 @@ def delta_rule(proj: torch.Tensor, offs, ranks, conv_w: torch.Tensor, w_decay: t
     # a graph that is being captured serves other divisions of its tokens too
     longest = 0 if getattr(batch, "any_division", False) else getattr(batch, "max_q_len", 0)
     batched = delta_batched(batch, H, D, V)
-    if batched:                                             # images of what sixteen tokens share
-        shared = ((T // 16 + batch.num_entries + 1) * H * (_fn("delta_rule", "llm_delta_image_bytes", [])() // 4),)
-    else:                                                   # places for what the eight tokens of a chunk share
-        chunks = T // 8 + batch.num_entries + 1
-        shared = 2 * (T * H * DP,) + (chunks * H * DP, chunks * H * 128)
-    sizes = (T * H * DP,) + 2 * (T * G * DP,) + (T * H * VP, T * H, T * H * V, T * H * V) + shared
-    starts = [0]
-    for n in sizes:
-        starts.append(starts[-1] + (n + 3) // 4 * 4)
-    room = torch.empty(starts[-1], dtype=torch.float32, device=dev)
+    while True:
+        if batched:                                         # images of what sixteen tokens share
+            shared = ((T // 16 + batch.num_entries + 1) * H * (_fn("delta_rule", "llm_delta_image_bytes", [])() // 4),)
+        else:                                               # places for what the eight tokens of a chunk share
+            chunks = T // 8 + batch.num_entries + 1
+            shared = 2 * (T * H * DP,) + (chunks * H * DP, chunks * H * 128)
+        sizes = (T * H * DP,) + 2 * (T * G * DP,) + (T * H * VP, T * H, T * H * V, T * H * V) + shared
+        starts = [0]
+        for n in sizes:
+            starts.append(starts[-1] + (n + 3) // 4 * 4)
+        try:
+            room = torch.empty(starts[-1], dtype=torch.float32, device=dev)
+            break
+        except torch.cuda.OutOfMemoryError:
+            if not batched:
+                raise
+            batched = False                                 # images take 2.4 times the places' room
     if D != DP:
         room[:sizes[0]].zero_()                             # decays behind a head's key width must be finite
     decay, qn, kn, vn, beta, gate, o, *shared = (room.data_ptr() + 4 * n for n in starts[:-1])

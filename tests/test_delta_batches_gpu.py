@@ -138,3 +138,20 @@ def test_a_portion_beside_single_tokens_and_states_that_are_not_finite():
             if (e, h) not in ((0, 1), (0, 2), (3, 0), (3, 3)):
                 x, y = (t[a:a + n, h * V:(h + 1) * V] for t in (out, ref))
                 assert float(((x - y).abs() / (1e-2 + y.abs())).max()) < 1e-3, (e, h)
+
+
+def test_without_room_for_the_images_a_step_takes_the_kernels_of_eight_tokens():
+    H, V = 12, 128
+    w, batch, _ = setup(H, H, V, [300, 20], 1.0, 9)
+    want = run(w, batch, H, H, V, False)
+    real, refused = torch.empty, []
+
+    def scarce(*a, **kw):
+        if not refused and isinstance(a[0], int):
+            refused.append(a[0])
+            raise torch.cuda.OutOfMemoryError("no room for the images")
+        return real(*a, **kw)
+    with pytest.MonkeyPatch.context() as m:
+        m.setattr(torch, "empty", scarce)
+        got = run(w, batch, H, H, V)
+    assert refused and all(torch.equal(a, b) for a, b in zip(got, want))
