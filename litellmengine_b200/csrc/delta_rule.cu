@@ -771,7 +771,6 @@ __global__ void __launch_bounds__(WARPS * 32) delta_scan_kernel(
     dr_keep_inputs<C == 1 ? 0 : THREADS>(s, proj, slot, positions, row0, count, h, c0, COLS, tile == 0);
 }
 
-// A warp per (token, head): o / rms(o) * w * gate * scale.
 // ---- states of 128 rows on the tensor cores -------------------------------------------------------------------------
 // The same recurrence, sixteen tokens at a time, as products: with X = V - (p k) S (tokens by columns),
 //
@@ -791,9 +790,10 @@ __global__ void __launch_bounds__(WARPS * 32) delta_scan_kernel(
 // A batch that holds something not finite or very large is marked with its first such token.  The scan makes what is before it as
 // always, with nothing in the place of what follows (a weight of zero times an infinity is NaN), and then walks through the batch
 // token by token for the outputs from the mark on and the state.
-// What bounds it: a batch's chain, 3,700 clocks: 48 small products a warp over the state (1,000), shares and X (700), U (300), the state
-// (600), the outputs of two warps (600) and the waits in between; the tensor pipe would take 1,450.  Portions of 284, 567 and 849
-// tokens, 16 heads of 128 x 128 (us): the scan 160 -> 107, what it shares 24 -> 46 (dot products and the writing of 76 MB).
+// What bounds it: a batch's chain, 2.2 us, of which 3,700 clocks are 48 small products a warp over the state (1,000), shares and X (700),
+// U (300), the state (600), the outputs of two warps (600) and the waits in between, and 200 what is added for the sums' last bits
+// (split_mma_whole); the tensor pipe is busy for 40 % of the time.  Portions of 284,
+// 567 and 849 tokens, 16 heads of 128 x 128 (us): the scan 160 -> 118, what it shares 24 -> 44 (dot products and the writing of 76 MB).
 // Error against 64 bits (2-norm, outputs and states) from the same unit norms, decays and step sizes: 7.7e-8 and 6.0e-8, the kernels of
 // eight tokens 8.6e-8 and 7.9e-8.  With sums as the tensor cores cut them (split_mma_whole) and dot products in four chains it was
 // 10.4e-8 and 8.6e-8, and the layer 320 us instead of 326.
@@ -1252,6 +1252,7 @@ __global__ void __launch_bounds__(256, 2) delta_scan_mma_kernel(
     dr_keep_inputs<256>(s, proj, slot, positions, row0, count, h, c0, DX_COLS, tile == 0);
 }
 
+// A warp per (token, head): o / rms(o) * w * gate * scale.
 template <typename TO>
 __global__ void delta_output_kernel(const float* __restrict__ o, const float* __restrict__ gate, const float* __restrict__ norm_w,
                                     float eps, float out_scale, TO* __restrict__ out, long long out_stride, int out_off, int H,

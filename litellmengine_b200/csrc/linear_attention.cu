@@ -691,12 +691,13 @@ static bool gla_tiled_takes(int D, int V, int mode) {
 // from memory as they are needed, transposed, as left operands.
 // A batch whose decays multiply to less than 2^-60 in some channel (q' would leave float32's range in the end), or that holds values
 // beyond 2^30, infinities or NaN (a masked weight of zero times one of them is NaN), walks token by token as the kernels above do.
-// What bounds it: latency.  2,048 tokens of 16 heads, 512 items of 64 tokens: local pass 66 -> 34 us, output pass 113 -> 82 (the
-// register-tiled kernel above before); of the output pass's time the tensor pipe is busy for 30 %, the loads of rows and state come
-// from memory half of the time, two blocks an SM hide some of each other's waits.  Tried: 16 tokens a batch with the state kept in
-// accumulators 92; 64 tokens a batch, one block of 16 warps an SM 87.  Error against 64 bits (2-norm, 2,048 tokens, decays
-// sigmoid(z)^(1/tau), tau 1, 2, 8, 64): states 4.0, 3.2, 4.0 and 6.1e-8, the kernel above 4.0, 4.7, 7.4 and 17.3; outputs 14.7, 10.1, 10.6
-// and 12.4e-8, and 14.4, 13.0, 13.1 and 20.2.  With all sums of the states as the tensor cores cut them the states were 5.7, 5.5, 6.0 and 7.2.
+// What bounds it: latency.  2,048 tokens of 16 heads, 512 items of 64 tokens, everything cold: local pass 72 -> 43 us, output pass
+// 121 -> 94 (the register-tiled kernel above before); of the output pass's time the tensor pipe is busy for 29 %, two blocks an SM hide
+// some of each other's waits for rows, state and shared memory, and at 128 registers a thread spills 184 bytes (88 in the local pass).
+// Tried: 16 tokens a batch with the state kept in accumulators 92 for 82 back to back; 64 tokens a batch, one block of 16 warps an SM 87.
+// Error against 64 bits (2-norm, 2,048 tokens, decays
+// sigmoid(z)^(1/tau), tau 2, 8, 64): states 3.2, 4.0 and 6.1e-8, the kernel above 4.7, 7.4 and 17.3; outputs 10.2, 10.6 and 12.4e-8,
+// and 13.0, 13.1 and 20.2.  With all sums of the states as the tensor cores cut them the states were 5.5, 6.0 and 7.2.
 #define GM_D 128
 #define GM_PITCH 136                 // of a row of a plane: eight rows of 16 bytes fall into all banks
 #define GM_WP 40                     // of a row of weights
