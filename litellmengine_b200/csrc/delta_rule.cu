@@ -1027,6 +1027,7 @@ __global__ void __launch_bounds__(256, 2) delta_scan_mma_kernel(
     }
     const long long row0 = entry_q_start[entry];
     const int count = entry_q_len[entry];
+    if (count <= 0) return;                                     // no copy may be on its way when the block ends
     float* slot = state + entry_slot[entry] * s.slot_stride;
     // a warp: columns c0 + 16 (warp / 4) .. + 15, rows 32 (warp % 4) .. + 31; tile n, element i: column v0 + 8 (i >> 1), row d0 + 8 n + (i & 1)
     const int group = warp >> 2, v0 = c0 + 16 * group + lg, dw = 32 * (warp & 3), d0 = dw + 2 * lt;

@@ -155,3 +155,19 @@ def test_without_room_for_the_images_a_step_takes_the_kernels_of_eight_tokens():
         m.setattr(torch, "empty", scarce)
         got = run(w, batch, H, H, V)
     assert refused and all(torch.equal(a, b) for a, b in zip(got, want))
+
+
+def test_entries_without_tokens():
+    """They keep their states and touch nobody's rows."""
+    H, V, lens = 5, 32, [0, 40, 0, 17, 0]
+    w, batch, _ = setup(H, H, V, lens, 1.0, 2)
+    out, state = run(w, batch, H, H, V)
+    full = [1, 3]
+    short, _, _ = setup(H, H, V, [40, 17], 1.0, 2)
+    short["state"] = w["state"][full].contiguous()
+    _, other, _ = setup(H, H, V, [40, 17], 1.0, 2)
+    for k in ("proj", "conv", "wa", "wg", "dt", "al", "nw"):
+        short[k] = w[k]
+    want, end = run(short, other, H, H, V)
+    assert torch.equal(out, want) and torch.equal(state[full], end)
+    assert torch.equal(state[[0, 2, 4]], w["state"][[0, 2, 4]])
