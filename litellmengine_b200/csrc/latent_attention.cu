@@ -67,8 +67,8 @@ __global__ void latent_prepare_kernel(
         }
     }
     float ss = 0.0f, ss_kv = 0.0f;
-    if (held) {          // both latents and their weights wait in registers; summed in the order of the loops below, value for value
-        float v[LA_HELD_Q], u[LA_HELD_KV], w[LA_HELD_Q], x[LA_HELD_KV];
+    if (held) {          // both latents wait in registers; summed in the order of the loops below, value for value
+        float v[LA_HELD_Q], u[LA_HELD_KV];
         auto each = [&](auto& all, int n, auto&& what) {          // the thread's values of n
 #pragma unroll
             for (int j = 0; j < static_cast<int>(sizeof(all) / sizeof(all[0])); ++j)
@@ -77,8 +77,6 @@ __global__ void latent_prepare_kernel(
         const int n_kv = keys ? R : 0;
         each(v, Q, [&](float& a, int i, int) { a = dq[i]; });
         each(u, n_kv, [&](float& a, int i, int) { a = dkv[i]; });
-        each(w, Q, [&](float& a, int i, int) { a = wq[i]; });
-        each(x, n_kv, [&](float& a, int i, int) { a = wkv[i]; });
         each(v, Q, [&](float& a, int, int) { ss += a * a; });
         each(u, n_kv, [&](float& a, int, int) { ss_kv += a * a; });
         ss = warp_sum(ss);
@@ -88,10 +86,10 @@ __global__ void latent_prepare_kernel(
         auto all_warps = [&](const float* s) { return ((s[0] + s[4]) + (s[2] + s[6])) + ((s[1] + s[5]) + (s[3] + s[7])); };      // as warp_sum does
         static_assert(LA_THREADS == 256, "eight warps");
         const float inv_q = 1.0f / sqrtf(all_warps(scratch) / static_cast<float>(Q) + eps);
-        each(v, Q, [&](float& a, int i, int j) { cq[i] = from_f32<TQ>(a * inv_q * w[j]); });
+        each(v, Q, [&](float& a, int i, int) { cq[i] = from_f32<TQ>(a * inv_q * wq[i]); });
         if (!dst) return;
         const float inv = 1.0f / sqrtf(all_warps(scratch + 8) / static_cast<float>(R) + eps);
-        each(u, R, [&](float& a, int i, int j) { dst[i] = from_f32<TC>(a * inv * x[j]); });
+        each(u, R, [&](float& a, int i, int) { dst[i] = from_f32<TC>(a * inv * wkv[i]); });
     } else {
         for (int i = threadIdx.x; i < Q; i += blockDim.x) { const float a = dq[i]; ss += a * a; }
         if (keys)
@@ -118,8 +116,9 @@ extern "C" int llm_latent_prepare(
     if (keys && (!block_table || page_size <= 0 || !wkv || (dims > 0 && !inv_freq))) return LLM_REFUSED_SIZE;
     cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
     if (!keys) cache_dtype = q_dtype;
-    // 2,000 tokens, latents of 1,536 and 512, the layer in us: 262 with one value a load, each read twice, and one sum over the block after
-    // the other; 258 with both latents held.  The sums keep their order: what is cached must not depend on the form.
+    // 2,000 tokens, latents of 1,536 and 512, cold (us): 26.6 with one value a load, each read twice, and one sum over the block after the
+    // other; 18.5 with both latents held, 20.5 with their weights too (56 registers instead of 38).  The sums keep their order: what is
+    // cached must not depend on the form.
     const int held = Q <= LA_HELD_Q * LA_THREADS && R <= LA_HELD_KV * LA_THREADS;
 #define LAUNCH(TQ, TC)                                                                                              \
     launch_pdl((latent_prepare_kernel<TQ, TC>), dim3(num_tokens), dim3(LA_THREADS), 0, s, proj, proj_stride, dq_off,  \
