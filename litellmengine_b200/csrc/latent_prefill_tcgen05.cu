@@ -407,6 +407,7 @@ __global__ void latent_gather_kernel(const bf16* __restrict__ rows_cache, long l
 // P-part rotated (pairs as in latent_attention.cu).  The angles of a token are made once for all heads.  2,000 tokens of 32 heads of
 // 128 + 64: 20 -> 16 us with four heads of a thread on their way before the angles are made.
 #define LQ_HELD 4
+template <bool WIDE>          // heads of more eights than a block has threads: a row of blocks
 __global__ void __launch_bounds__(1024) latent_q_pack_kernel(const float* __restrict__ q, bf16* __restrict__ out, const int32_t* __restrict__ positions,
                                      const float* __restrict__ inv_freq, int H, int D, int P, int dims, int rot_pairs, float rot_mag) {
     pdl_begin();
@@ -414,11 +415,10 @@ __global__ void __launch_bounds__(1024) latent_q_pack_kernel(const float* __rest
     const int t = blockIdx.x, half = dims / 2, W = D + P;
     const float* src = q + static_cast<size_t>(t) * H * W;
     bf16* dst = out + static_cast<size_t>(t) * H * W;
-    // a thread keeps its place in the head and goes from head to head, LQ_HELD heads on their way at once; a head of more eights than a
-    // block has threads is a row of blocks
-    const int eights = W / 8, blk = blockDim.x, wide = eights > blk, per = wide ? 1 : blk / eights;
-    const int c = static_cast<int>(wide ? blockIdx.y * blk + threadIdx.x : threadIdx.x % eights) * 8, k0 = c - D, h0 = wide ? 0 : threadIdx.x / eights;
-    const int heads = c < W ? H : 0;
+    // a thread keeps its place in the head and goes from head to head, LQ_HELD heads on their way at once
+    const int per = WIDE ? 1 : blockDim.x / (W / 8), c = static_cast<int>(WIDE ? blockIdx.y * blockDim.x + threadIdx.x : threadIdx.x % (W / 8)) * 8;
+    const int k0 = c - D, h0 = WIDE ? 0 : threadIdx.x / (W / 8);
+    const int heads = WIDE && c >= W ? 0 : H;
     const bool whole = k0 >= 0 && k0 + 8 <= dims && (rot_pairs || half % 8 == 0);      // all eight turn, with neighbours or with eight others
     const bool first = k0 < half;
     const int f0 = rot_pairs ? k0 >> 1 : first ? k0 : k0 - half;
@@ -502,8 +502,9 @@ extern "C" int llm_latent_q_pack(const float* q, void* out, const int32_t* posit
     const int eights = (D + P) / 8;                               // threads: as many whole heads as 256 of them hold, or one, or a part of it
     const int threads = eights > 1024 ? 1024 : eights > 256 ? eights : 256 / eights * eights, parts = (eights + 1023) / 1024;
     if (parts > 65535) return LLM_REFUSED_SIZE;
-    launch_pdl(latent_q_pack_kernel, dim3(num_tokens, parts), dim3(threads), sizeof(float2) * (dims / 2), reinterpret_cast<cudaStream_t>(stream),
-               q, static_cast<bf16*>(out), positions, inv_freq, H, D, P, dims, rot_pairs, rot_mag);
+    launch_pdl(parts > 1 ? latent_q_pack_kernel<true> : latent_q_pack_kernel<false>, dim3(num_tokens, parts), dim3(threads),
+               sizeof(float2) * (dims / 2), reinterpret_cast<cudaStream_t>(stream), q, static_cast<bf16*>(out), positions, inv_freq, H, D, P,
+               dims, rot_pairs, rot_mag);
     return launch_status();
 }
 
