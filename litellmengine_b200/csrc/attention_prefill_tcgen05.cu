@@ -310,39 +310,44 @@ __global__ void __launch_bounds__(64 + 128 * HEADS, 1) paged_prefill_attention_t
 // tile (the kernel above stays for groups of odd size): 128 keys a tile, S = Q K^T of head 0 while
 // the softmax threads of head 1 work and the other way round, so the tensor pipe has a product of
 // one head to run while the other head's weights are being made.  Per head TMEM holds S (128
-// columns of float32) and O (128 columns); P (bfloat16) lies over S, 32 columns at column 0 and 32
-// at column 64, each over the columns of the thread that makes it.
+// columns of float32) and O (128 columns); P (bfloat16) lies over S, 64 columns from column 0 on, each over columns
+// that its thread has read.
 // The weights are P = exp2(S*scale*log2e - m) with a reference m per row that trails the running
 // maximum: m moves up only when the maximum has passed it by more than 8 (a factor 256, far
 // inside what bfloat16 and the float32 sums hold), and only then O and the row sum l are
 // multiplied by exp2(m_old - m_new) (the running-maximum form of src/ops/attention.cu:204-249 with
 // the correction made rare).  The result sum(P V) / sum(P) does not depend on which m was used.
+// After a portion's first tile the weights of 64 keys are made at the reference that is there, beside these keys' maximum, and
+// made again in the rare case that it has to move: neither waits for the other.
 // Roles: warp 0 looks up pages and asks the copy engine for keys and values (rings of two tiles
-// each); one lane of warp 1 issues every product; then eight softmax warps per head, two threads
-// to a query row with 64 columns of S each.  What limited earlier forms, in the order found by
-// reading the SM clock inside the kernel: the order of CTAs (long tiles must start
-// first), one thread requesting the copies box by box (140 clocks a request), one thread per row in
-// the softmax; what is left is the chain S -> weights -> P V of one head, about 4,000 clocks a
-// tile against 2,050 of tensor work for both heads.
+// each); warp 1 issues every product; warps 2 and 3 have no work (tensor memory gives a warp the 32 lanes of its index mod 4); then
+// four softmax warps per head, a thread a query row.
+// What bounds it, read from the SM clock inside the kernel: a tile takes 3,900 clocks, of which the tensor pipe works 2,048
+// and the exponentials of both heads (8 clocks a warp and value) 2,048.  A head's chain is 2,100 to 2,500 clocks from S to the
+// last weight, as the other head's exponentials get in its way, and 1,300 from there to the next S: half of P V (the other half runs
+// under the second half's weights), Q K^T, and the commit's way.  Against the form before (two threads a row that exchanged their
+// maxima before the weights, one lane alone in the issuing loop), us: 967 + 1,933 tokens behind 700 and 613 118 -> 95, 2,500 tokens
+// 98 -> 76, 8,192 tokens 605 -> 510, 300 + 600 tokens 31 -> 20; windowed with sinks, 2,500 tokens, 88 -> 73.  A step of that: rows behind a
+// portion's last used to send the whole of its last tile, the longest, through the masked form (98 -> 81).  Two threads a row in this
+// form, with a vote of two warps in the place of the exchange: 2.2 us a tile against 2.05; a share of the exponentials as
+// polynomials on the multiply-add pipe: 15.0 clocks a value and warp against 12.0 (an exponential keeps its warp from issuing for its 8 clocks).
 #define T5O_BN 128
 #define T5O_HALF (T5O_BN * 64)                // elements of one 64-column half of a 128-key tile
 #define T5O_TILE (2 * T5O_HALF)
 #define T5O_STAGES 2
 #define T5O_JUMP 8.0f
-#define T5O_THREADS (64 + 2 * 256)             // producer warp, issuing warp, then 8 softmax warps per head
+#define T5O_THREADS (128 + 2 * 128)            // producer warp, issuing warp, two without work, then 4 softmax warps per head
 
 // BIAS: the scores carry more than the scale.  `head_bias` is float32 [nq][3] = (t, r1, r2) per query head and the
 // weight of key j for the query at position i is exp(S * scale * t - r1 * ln(1 + r2 * (i - j))).  The bias depends on
-// the head and on i - j only, and a tile of 128 rows by 128 keys meets 255 distances: the 256 softmax threads of a
-// head work out one each (a logarithm a thread a tile instead of 64) into a table in shared memory for the NEXT tile,
-// before the barrier that they all pass once a tile.  Three tables take turns: a thread that is late with tile j
-// may still read table j after that barrier (when it has to fetch its scores a second time) while an early one
-// already writes the table of tile j + 2.
+// the head and on i - j only, and a tile of 128 rows by 128 keys meets 255 distances: the 128 softmax threads of a
+// head work out two each (two logarithms a thread a tile instead of 128) into a table in shared memory for the NEXT tile,
+// behind the barrier that they all pass once a tile in this mode.  Two tables take turns.
 // EXT: a window that keeps the sequence's first `keep_first` keys (the tiles that hold them and lie wholly below the
 // window's first tile are walked first; kept keys inside the window's tiles are a matter of the mask), one more term
 // exp(sinks[head]) in the softmax's denominator, a sigmoid gate per head (column gate_off + head of a float32 row per
 // token), a factor, and a result that is a column range of a wider buffer.  Measured, 32 heads over 8, window 1,024, four
-// kept keys, learned sinks, 2,500 tokens: 216 us on mma.sync (attention_prefill.cu), 87 us here.  In this mode the reference
+// kept keys, learned sinks, 2,500 tokens: 216 us on mma.sync (attention_prefill.cu), 73 us here.  In this mode the reference
 // is the running maximum itself, so that the largest weight so far is exactly one in bfloat16, as on mma.sync, and the
 // weights are summed as rounded.  With a reference that trails and a sum of unrounded weights it takes 10 us less, and the error against
 // 64 bits is 3, 13 and 20 % above that of mma.sync at spreads of the scores of 1, 2 and 4 (now 0.2 % below, level, 0.1 % below).
@@ -376,12 +381,10 @@ __global__ void __launch_bounds__(T5O_THREADS, 1) paged_prefill_attention_tcgen0
     // keys and values have rings of their own: a key tile is free once both heads' S are made, a
     // value tile only after both heads' P V, half a tile's work later
     __shared__ __align__(8) unsigned long long q_full, k_full[STAGES], k_empty[STAGES], v_full[STAGES], v_empty[STAGES],
-        s_full[2], p_full[2], pv_done[2];
+        s_full[2], p_full[2][2], pv_half[2], pv_done[2];
     __shared__ unsigned tmem_base_s;
     __shared__ int abort_flag;
-    __shared__ float x_max[2][2][2][128];                         // [tile parity][head][column half][row]: the halves' maxima
-    __shared__ float x_sum[2][2][128];                            // [head][column half][row]: the halves' row sums, at the end
-    __shared__ float bias_tbl[BIAS ? 3 : 1][2][BIAS ? 256 : 1];   // [tile mod 3][head][i - j - (first row - first key of the tile) + 127]
+    __shared__ float bias_tbl[BIAS ? 2 : 1][2][BIAS ? 256 : 1];   // [tile parity][head][i - j - (first row - first key of the tile) + 127]
 
     const int tile = blockIdx.y;
     const int h0 = blockIdx.x * 2;                                // first of this CTA's two query heads
@@ -393,7 +396,7 @@ __global__ void __launch_bounds__(T5O_THREADS, 1) paged_prefill_attention_tcgen0
     const int row_base = entry_q_start[e] + q0;
     const int rows_here = min(T5_BM, q_len - q0);
     const int32_t* table = block_table + static_cast<size_t>(entry_slot[e]) * table_stride;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
     const int pos_first = past + q0, pos_last = past + q0 + rows_here - 1;
     const int k_lo = first_visible(pos_first, window) / T5O_BN * T5O_BN;
     const int keep = EXT && window > 0 ? ext.keep_first : 0;
@@ -410,7 +413,8 @@ __global__ void __launch_bounds__(T5O_THREADS, 1) paged_prefill_attention_tcgen0
         }
         for (int g = 0; g < 2; ++g) {
             t5_mbar_init(&s_full[g], 1);                 // the head's S of a tile is in TMEM
-            t5_mbar_init(&p_full[g], 256);               // every softmax thread of the head has put its part of P over S
+            for (int hf = 0; hf < 2; ++hf) t5_mbar_init(&p_full[g][hf], 4);      // every softmax warp of the head has put its rows of half of P over S
+            t5_mbar_init(&pv_half[g], 1);                // the head's O holds P V of the tile's first 64 keys
             t5_mbar_init(&pv_done[g], 1);                // the head's O holds the tile's P V
         }
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
@@ -422,7 +426,7 @@ __global__ void __launch_bounds__(T5O_THREADS, 1) paged_prefill_attention_tcgen0
     t5_fence_before();
     __syncthreads();
     t5_fence_after();
-    const unsigned tmem = tmem_base_s;
+    const unsigned tmem = __shfl_sync(0xffffffffu, tmem_base_s, 0);
     auto s_col = [](int g) { return static_cast<unsigned>(g * 128); };
     auto o_col = [](int g) { return static_cast<unsigned>(256 + g * 128); };
 
@@ -490,83 +494,65 @@ __global__ void __launch_bounds__(T5O_THREADS, 1) paged_prefill_attention_tcgen0
         }
     } else if (warp == 1) {
         // ---- MMA issuer: S0(j), O1 += P1 V(j-1), S1(j), O0 += P0 V(j), ... ----
-        if (lane == 0) {
-            constexpr unsigned IDESC_QK = t5_idesc(T5_BM, T5O_BN, 0);
-            constexpr unsigned IDESC_PV = t5_idesc(T5_BM, T5_D, 1);
-            // One thread issues every product, and what it computes per instruction is what limits the
-            // rate of issue: every operand descriptor is made once, here, and the loop over tiles is
-            // unrolled by the two stages so that each product names its descriptors by constant index.
-            unsigned long long qd[2][8], kd[2][8], vd[2][8];
-            {
-                const unsigned long long qd0 = t5_desc(q_s, 16, 1024), kd0 = t5_desc(k_s, 16, 1024);
-                const unsigned long long vd0 = t5_desc(v_s, T5O_HALF * sizeof(bf16), 1024);
-                constexpr unsigned long long STAGE_STEP = (T5O_TILE * sizeof(bf16)) >> 4;
+        // All lanes walk the loop, one of them issues.  Descriptors are made of what all lanes hold alike; a tile further on in
+        // shared memory is the same descriptor plus its byte offset / 16 in the address field.
+        constexpr unsigned IDESC_QK = t5_idesc(T5_BM, T5O_BN, 0);
+        constexpr unsigned IDESC_PV = t5_idesc(T5_BM, T5_D, 1);
+        const unsigned lead = t5_elect();
+        const unsigned long long qd0 = t5_desc(q_s, 16, 1024), kd0 = t5_desc(k_s, 16, 1024);
+        const unsigned long long vd0 = t5_desc(v_s, T5O_HALF * sizeof(bf16), 1024);
+        constexpr unsigned long long STAGE_STEP = (T5O_TILE * sizeof(bf16)) >> 4, VSTEP = (16 * 64 * sizeof(bf16)) >> 4;   // 16 keys further, both 64-column halves
+        auto qk = [&](int g, int st) {
 #pragma unroll
-                for (int a = 0; a < 2; ++a)
-#pragma unroll
-                    for (int k = 0; k < 8; ++k) {
-                        qd[a][k] = qd0 + (((a * 2 + (k >> 2)) * T5_QHALF + (k & 3) * 16) * sizeof(bf16) >> 4);
-                        kd[a][k] = kd0 + a * STAGE_STEP + (((k >> 2) * T5O_HALF + (k & 3) * 16) * sizeof(bf16) >> 4);
-                        vd[a][k] = vd0 + a * STAGE_STEP + ((k * 16 * 64) * sizeof(bf16) >> 4);   // 16 keys further, both 64-column halves
-                    }
+            for (int k = 0; k < 8; ++k) {
+                const unsigned long long qo = (((k >> 2) * T5_QHALF + (k & 3) * 16) * sizeof(bf16)) >> 4;
+                const unsigned long long ko = (((k >> 2) * T5O_HALF + (k & 3) * 16) * sizeof(bf16)) >> 4;
+                t5_mma_ss_lead(lead, tmem + s_col(g), qd0 + g * ((2 * T5_QHALF * sizeof(bf16)) >> 4) + qo, kd0 + st * STAGE_STEP + ko, IDESC_QK, k > 0);
             }
-            auto qk = [&](int g, int st) {                        // g, st: constants where this is inlined
+            t5_commit_lead(lead, &s_full[g]);
+        };
+        auto pv = [&](int g, int j, int st) -> bool {
 #pragma unroll
-                for (int k = 0; k < 8; ++k) t5_mma_ss(tmem + s_col(g), qd[g][k], kd[st][k], IDESC_QK, k > 0);
-                t5_commit(&s_full[g]);
-            };
-            auto pv = [&](int g, int st, bool first) {
+            for (int hf = 0; hf < 2; ++hf) {
+                if (!t5_wait_warp(&p_full[g][hf], j & 1, &abort_flag, status, row_base)) return false;
+                t5_fence_after();
 #pragma unroll
-                for (int k = 0; k < 8; ++k)
-                    t5_mma_ts(tmem + o_col(g), tmem + s_col(g) + (k >> 2) * 64 + (k & 3) * 8, vd[st][k], IDESC_PV,
-                              (!first || k > 0) ? 1u : 0u);      // P of keys 64..127 lies over S column 64
-                t5_commit(&pv_done[g]);
-            };
-            bool ok = t5_wait(&q_full, 0, &abort_flag, status, row_base);
-            auto one_tile = [&](int j, int st) -> bool {          // st = j % 2, a constant where this is inlined
-                if (!t5_wait(&k_full[st], (j >> 1) & 1, &abort_flag, status, row_base)) return false;
-                t5_fence_after();
-                qk(0, st);
-                if (j > 0) {
-                    if (!t5_wait(&p_full[1], (j - 1) & 1, &abort_flag, status, row_base)) return false;
-                    t5_fence_after();
-                    pv(1, 1 - st, j == 1);
-                    t5_commit(&v_empty[1 - st]);                       // the last reader of the values of tile j-1
-                }
-                qk(1, st);
-                t5_commit(&k_empty[st]);                               // the last reader of the keys of tile j
-                if (!t5_wait(&p_full[0], j & 1, &abort_flag, status, row_base)) return false;
-                if (!t5_wait(&v_full[st], (j >> 1) & 1, &abort_flag, status, row_base)) return false;
-                t5_fence_after();
-                pv(0, st, j == 0);
-                return true;
-            };
-            static_assert(T5O_STAGES == 2, "the issue loop is unrolled by the number of stages");
-            for (int j = 0; ok && j < n_tiles; j += 2) {
-                ok = one_tile(j, 0);
-                if (ok && j + 1 < n_tiles) ok = one_tile(j + 1, 1);
+                for (int k = 4 * hf; k < 4 * hf + 4; ++k)
+                    t5_mma_ts_lead(lead, tmem + o_col(g), tmem + s_col(g) + k * 8, vd0 + st * STAGE_STEP + k * VSTEP, IDESC_PV, (j > 0 || k > 0) ? 1u : 0u);
+                t5_commit_lead(lead, hf ? &pv_done[g] : &pv_half[g]);
             }
-            if (ok && t5_wait(&p_full[1], (n_tiles - 1) & 1, &abort_flag, status, row_base)) {
-                t5_fence_after();
-                if ((n_tiles - 1) & 1) { pv(1, 1, n_tiles == 1); t5_commit(&v_empty[1]); }
-                else { pv(1, 0, n_tiles == 1); t5_commit(&v_empty[0]); }
+            return true;
+        };
+        bool ok = t5_wait_warp(&q_full, 0, &abort_flag, status, row_base);
+#pragma unroll 1
+        for (int j = 0; ok && j < n_tiles; ++j) {
+            const int st = j & 1;
+            ok = t5_wait_warp(&k_full[st], (j >> 1) & 1, &abort_flag, status, row_base);
+            if (!ok) break;
+            t5_fence_after();
+            qk(0, st);
+            if (j > 0) {
+                ok = pv(1, j - 1, 1 - st);
+                if (!ok) break;
+                t5_commit_lead(lead, &v_empty[1 - st]);                // the last reader of the values of tile j-1
             }
+            qk(1, st);
+            t5_commit_lead(lead, &k_empty[st]);                        // the last reader of the keys of tile j
+            ok = t5_wait_warp(&v_full[st], (j >> 1) & 1, &abort_flag, status, row_base) && pv(0, j, st);
         }
-    } else {
-        // ---- softmax: two threads share a query row of a head (one TMEM lane), 64 columns of S each ----
-        // A warp reaches the 32 TMEM lanes of its quarter (warp index mod 4) only, so the two threads
-        // of a row sit in two warps of the same quarter.  Each keeps its 64 values of S in registers,
-        // the two exchange their maxima through shared memory, and each writes its 32 columns of P
-        // over the first half of ITS OWN columns of S (so neither ever touches the other's columns).
-        const int wl = warp - 2;
-        const int g = wl >> 3;                                    // warps 2..9: head h0, warps 10..17: head h0 + 1
-        const int half = (wl >> 2) & 1;                           // columns 64*half .. 64*half+63 of every tile
-        const int quarter = warp & 3;
+        static_assert(T5O_STAGES == 2, "a tile's stage is its parity");
+        if (ok && pv(1, n_tiles - 1, (n_tiles - 1) & 1)) t5_commit_lead(lead, &v_empty[(n_tiles - 1) & 1]);
+    } else if (warp >= 4) {
+        // ---- softmax: a thread owns one query row of one head = one TMEM lane, all 128 columns of a tile ----
+        const int g = (warp - 4) >> 2;                            // warps 4..7: head h0, warps 8..11: head h0 + 1
+        const int quarter = warp & 3;                             // the TMEM lanes this warp may touch
         const int row = quarter * 32 + lane;
         const unsigned lane_addr = static_cast<unsigned>(quarter * 32) << 16;
-        const unsigned my_s = tmem + lane_addr + s_col(g) + half * 64;
-        const unsigned my_o = tmem + lane_addr + o_col(g) + half * 64;
-        const int pos = (row < rows_here) ? past + q0 + row : -1;
+        const unsigned my_s = tmem + lane_addr + s_col(g);
+        const unsigned my_o = tmem + lane_addr + o_col(g);
+        // Rows behind the portion's last are other tokens' or zeros: they are worked like the rest (nothing of a row reaches another
+        // one) and not stored.
+        const int pos = past + q0 + row;
         const int lo = first_visible(pos, window), lo_last = first_visible(pos_last, window);
         float m = -CUDART_INF_F, l = 0.0f;                        // m: the reference maximum, in units of log2
         bool ok = true;
@@ -577,164 +563,194 @@ __global__ void __launch_bounds__(T5O_THREADS, 1) paged_prefill_attention_tcgen0
             sc *= hb[0]; r1 = hb[1]; r2 = hb[2];
         }
         const float eff = BIAS ? 1.0f : scale_log2e;
-        const int in_head = (wl & 7) * 32 + lane;                 // 0..255 among the head's softmax threads
-        auto fill_table = [&](int jt, int which) {                // the distances of tile jt: first row - first key - 127 + in_head
-            const int dist = pos_first - (k_lo + jt * T5O_BN) - 127 + in_head;
-            bias_tbl[which][g][in_head] = dist > 0 ? r1 * __log2f(fmaf(r2, static_cast<float>(dist), 1.0f)) : 0.0f;
+        auto fill_table = [&](int jt, int which) {                // the distances of tile jt: first row - first key - 127 + (0 .. 255)
+#pragma unroll
+            for (int i = row; i < 256; i += 128) {
+                const int dist = pos_first - (k_lo + jt * T5O_BN) - 127 + i;
+                bias_tbl[which][g][i] = dist > 0 ? r1 * __log2f(fmaf(r2, static_cast<float>(dist), 1.0f)) : 0.0f;
+            }
         };
-        int tb_cur = 0;
-        if constexpr (BIAS) {
-            fill_table(0, 0);
-            asm volatile("bar.sync %0, 256;\n" ::"r"(1 + g) : "memory");
-        }
+        if constexpr (BIAS) fill_table(0, 0);
         for (int j = 0; j < n_tiles; ++j) {
-            const int kt = tile_key(j) + half * 64;               // this thread's first key of the tile
-            const int tb_next = tb_cur == 2 ? 0 : tb_cur + 1;
+            const int kt = tile_key(j);
             if constexpr (BIAS) {
-                if (j + 1 < n_tiles) fill_table(j + 1, tb_next);
+                asm volatile("bar.sync %0, 128;\n" ::"r"(1 + g) : "memory");      // the table of this tile is there
+                if (j + 1 < n_tiles) fill_table(j + 1, (j + 1) & 1);
             }
-            // S of (row, column c + i of this thread's 64) -> S * scale * t - bias(i - j), in place
-            auto biased = [&](unsigned (&r)[32], int c) {
-                const float* tb = &bias_tbl[tb_cur][g][row - (half * 64 + c) + 127];
-#pragma unroll
-                for (int i = 0; i < 32; ++i) r[i] = __float_as_uint(fmaf(__uint_as_float(r[i]), sc, -tb[-i]));
-            };
-            // After a wait has run out (ok false) a thread still passes every barrier below, the same
-            // number of times as the others, and touches nothing else.
-            if (ok && !t5_wait(&s_full[g], j & 1, &abort_flag, status, row_base)) ok = false;
-            t5_fence_after();
-            const bool full_tile = (kt + 63 <= pos_first) && (kt >= lo_last || (EXT && kt + 63 < keep)) && (rows_here == T5_BM);
-            auto seen = [&](int key) { return key <= pos && (key >= lo || (EXT && key < keep)); };
-            unsigned ra[32], rb[32];
-            float mx = -CUDART_INF_F;
-            if (ok) {
-                t5_ld32(my_s, ra);
-                t5_ld32(my_s + 32, rb);
-                t5_wait_ld();
-                if constexpr (BIAS) { biased(ra, 0); biased(rb, 32); }
-                if (full_tile) {
-#pragma unroll
-                    for (int i = 0; i < 32; ++i) mx = fmaxf(mx, fmaxf(__uint_as_float(ra[i]), __uint_as_float(rb[i])));
-                } else {
-#pragma unroll
-                    for (int i = 0; i < 32; ++i) {
-                        if (seen(kt + i)) mx = fmaxf(mx, __uint_as_float(ra[i]));
-                        if (seen(kt + 32 + i)) mx = fmaxf(mx, __uint_as_float(rb[i]));
-                    }
-                }
-                x_max[j & 1][g][half][row] = mx;
-            }
-            asm volatile("bar.sync %0, 256;\n" ::"r"(1 + g) : "memory");      // the 8 softmax warps of this head
-            const int tb_mine = tb_cur;
-            tb_cur = tb_next;
-            if (!ok) continue;
-            mx = fmaxf(mx, x_max[j & 1][g][half ^ 1][row]) * eff;             // scale > 0; -inf stays -inf
-            // move the reference up only when the maximum has run away from it (both threads of a row
-            // see the same numbers and decide alike)
-            const bool adopt = (m == -CUDART_INF_F) && (mx > m);  // nothing accumulated under the old reference
-            const bool jump = (m != -CUDART_INF_F) && (mx > m + (EXT ? 0.0f : T5O_JUMP));
-            if (__any_sync(0xffffffffu, jump)) {
-                // O still receives the previous tile's product: wait for it, then scale this thread's half of its row
-                if (!t5_wait(&pv_done[g], (j - 1) & 1, &abort_flag, status, row_base)) { ok = false; continue; }
-                t5_fence_after();
-                const float alpha = jump ? t5_ex2(m - mx) : 1.0f;
-                l *= alpha;
-#pragma unroll 1
-                for (int c = 0; c < 64; c += 32) {                // through ra, which is read again below
-                    t5_ld32(my_o + c, ra);
-                    t5_wait_ld();
-#pragma unroll
-                    for (int i = 0; i < 32; ++i) ra[i] = __float_as_uint(__uint_as_float(ra[i]) * alpha);
-                    t5_st32(my_o + c, ra);
-                }
-                t5_wait_st();
-                t5_ld32(my_s, ra);
-                t5_wait_ld();
+            const bool full_tile = (kt + T5O_BN - 1 <= pos_first) && (kt >= lo_last || (EXT && kt + T5O_BN - 1 < keep));
+            // columns 32 c .. 32 c + 31 of the scores: S -> S * scale * t - bias(i - j), and what the row does not see to -inf
+            auto settle = [&](unsigned (&r)[32], int c) {
                 if constexpr (BIAS) {
-                    const float* tb = &bias_tbl[tb_mine][g][row - half * 64 + 127];
+                    const float* tb = &bias_tbl[j & 1][g][row - c * 32 + 127];
 #pragma unroll
-                    for (int i = 0; i < 32; ++i) ra[i] = __float_as_uint(fmaf(__uint_as_float(ra[i]), sc, -tb[-i]));
+                    for (int i = 0; i < 32; ++i) r[i] = __float_as_uint(fmaf(__uint_as_float(r[i]), sc, -tb[-i]));
                 }
-            }
-            if (adopt || jump) m = mx;
-            const float msub = (m == -CUDART_INF_F) ? 0.0f : m;
-            // the weights, rounded to bfloat16: 32 columns of P over the first half of this thread's 64 of S; EXT sums them as rounded
-            auto sum_of = [](float p0, float p1, unsigned packed) {
-                return EXT ? __uint_as_float(packed << 16) + __uint_as_float(packed & 0xffff0000u) : p0 + p1;
+                if (!full_tile) {
+                    auto first = [&](int n) { return n <= 0 ? 0u : n >= 32 ? ~0u : (1u << n) - 1u; };
+                    const int k0 = kt + 32 * c;
+                    const unsigned seen = first(pos + 1 - k0) & (~first(lo - k0) | (EXT ? first(keep - k0) : 0u));
+#pragma unroll
+                    for (int i = 0; i < 32; ++i) r[i] = seen & (1u << i) ? r[i] : 0xff800000u;
+                }
             };
-            auto weights = [&](const unsigned (&r)[32], int c) {
-                unsigned pk[16];
-                if (full_tile) {
+            auto max_of = [](const unsigned (&r)[32], float mx) {
+                float a = __uint_as_float(r[0]), b = __uint_as_float(r[1]);
 #pragma unroll
-                    for (int i = 0; i < 32; i += 2) {
-                        const float x0 = fmaf(__uint_as_float(r[i]), eff, -msub);
-                        const float x1 = fmaf(__uint_as_float(r[i + 1]), eff, -msub);
-                        const float p0 = t5_ex2(x0), p1 = t5_ex2(x1);     // (a cubic on the FMA pipe for a share of them: measured slower)
-                        pk[i >> 1] = t5_pack(p0, p1);
-                        l += sum_of(p0, p1, pk[i >> 1]);
-                    }
-                } else {
-#pragma unroll
-                    for (int i = 0; i < 32; i += 2) {
-                        const int key = kt + c + i;
-                        const float p0 = seen(key) ? t5_ex2(fmaf(__uint_as_float(r[i]), eff, -msub)) : 0.0f;
-                        const float p1 = seen(key + 1) ? t5_ex2(fmaf(__uint_as_float(r[i + 1]), eff, -msub)) : 0.0f;
-                        pk[i >> 1] = t5_pack(p0, p1);
-                        l += sum_of(p0, p1, pk[i >> 1]);
-                    }
-                }
-                t5_st16(my_s + (c >> 1), pk);
+                for (int i = 2; i < 32; i += 2) { a = fmaxf(a, __uint_as_float(r[i])); b = fmaxf(b, __uint_as_float(r[i + 1])); }
+                return fmaxf(mx, fmaxf(a, b));
             };
-            weights(ra, 0);
-            weights(rb, 32);
-            t5_wait_st();
-            t5_fence_before();
-            if constexpr (EXT) {
-                // Keys of the tile that no row of the block sees (behind its last one, below the window, behind the kept ones) have weights
-                // of zero, but what lies there may be anything (a request that had the page before, a held page's copy), and zero times a
-                // value that is not finite is NaN: their values are set to zero before the products, a row of 128 bytes a thread.
-                const int k0 = tile_key(j), key = k0 + (tid & 127), lo_first = first_visible(pos_first, window);
-                if (g == 0 && (k0 + T5O_BN - 1 > pos_last || (k0 < lo_first && k0 + T5O_BN > keep))) {
-                    if (!t5_wait(&v_full[j % STAGES], (j / STAGES) & 1, &abort_flag, status, row_base)) { ok = false; continue; }
-                    if (key > pos_last || (key < lo_first && key >= keep)) {
-                        uint4* v = reinterpret_cast<uint4*>(v_s + (j % STAGES) * T5O_TILE + ((tid - 64) >> 7) * T5O_HALF + (tid & 127) * 64);
+            // the weights of 32 columns, rounded to bfloat16, and their sum (EXT: of the rounded ones)
+            auto weights = [&](const unsigned (&r)[32], unsigned (&pk)[16], float ref, float sum) {
+                const unsigned long long e2 = t5_two(eff, eff), m2 = t5_two(-ref, -ref);
+                float s0 = 0.0f, s1 = 0.0f;
 #pragma unroll
-                        for (int c = 0; c < 8; ++c) v[(c + lane) & 7] = make_uint4(0u, 0u, 0u, 0u);      // a quarter-warp: all banks
+                for (int i = 0; i < 32; i += 2) {
+                    float x0, x1;
+                    t5_untwo(t5_fma2(t5_two(__uint_as_float(r[i]), __uint_as_float(r[i + 1])), e2, m2), x0, x1);
+                    const float p0 = t5_ex2(x0), p1 = t5_ex2(x1);
+                    pk[i >> 1] = t5_pack(p0, p1);
+                    if (EXT) {
+                        s0 += __uint_as_float(pk[i >> 1] << 16);
+                        s1 += __uint_as_float(pk[i >> 1] & 0xffff0000u);
+                    } else {
+                        s0 += p0;
+                        s1 += p1;
                     }
-                    asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
                 }
+                return sum + (s0 + s1);
+            };
+            // After a wait has run out (ok false, for whole warps) a thread still passes every barrier above and touches nothing else.
+            if (ok) ok = __all_sync(0xffffffffu, t5_wait(&s_full[g], j & 1, &abort_flag, status, row_base));
+            if (!ok) continue;
+            t5_fence_after();
+            unsigned r[2][32];
+            // the row's O and l on to another reference, once the products that are under way have joined O
+            auto move_to = [&](float mx, bool jump, unsigned long long* done, int parity) {
+                if (__any_sync(0xffffffffu, jump)) {
+                    ok = __all_sync(0xffffffffu, t5_wait(done, parity, &abort_flag, status, row_base));
+                    if (!ok) return;
+                    t5_fence_after();
+                    const float alpha = jump ? t5_ex2(m - mx) : 1.0f;
+                    l *= alpha;
+                    t5_ld32(my_o, r[0]);
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) {
+                        t5_wait_ld();
+                        if (c < 3) t5_ld32(my_o + 32 * (c + 1), r[(c + 1) & 1]);
+#pragma unroll
+                        for (int i = 0; i < 32; ++i) r[c & 1][i] = __float_as_uint(__uint_as_float(r[c & 1][i]) * alpha);
+                        t5_st32(my_o + 32 * c, r[c & 1]);
+                    }
+                }
+            };
+            const bool first_max = EXT || j == 0;                     // the tile's maximum before its weights
+            if (first_max) {                                          // (EXT: the reference is the running maximum itself)
+                float mx = -CUDART_INF_F;
+                t5_ld32(my_s, r[0]);
+#pragma unroll
+                for (int c = 0; c < 4; ++c) {
+                    t5_wait_ld();
+                    if (c < 3) t5_ld32(my_s + 32 * (c + 1), r[(c + 1) & 1]);
+                    settle(r[c & 1], c);
+                    mx = max_of(r[c & 1], mx);
+                }
+                mx *= eff;                                            // scale > 0; -inf stays -inf
+                move_to(mx, m != -CUDART_INF_F && mx > m, &pv_done[g], (j - 1) & 1);
+                if (!ok) continue;
+                m = fmaxf(m, mx);
             }
-            t5_arrive(&p_full[g]);
+            // The tile in two halves of 64 keys: the products over the first run while the weights of the second are made.
+#pragma unroll 1
+            for (int hf = 0; hf < 2; ++hf) {
+                const unsigned s_at = my_s + 64 * hf, p_at = my_s + 32 * hf;
+                unsigned pk[2][16];
+                float ref = m == -CUDART_INF_F ? 0.0f : m;
+                float sum = 0.0f, mx = -CUDART_INF_F;
+                // The weights at the reference that the keys before have left, beside these keys' maximum: the reference hardly ever
+                // moves, and then neither has waited for the other.
+                t5_ld32(s_at, r[0]);
+#pragma unroll
+                for (int c = 0; c < 2; ++c) {
+                    t5_wait_ld();
+                    if (c < 1) t5_ld32(s_at + 32, r[1]);
+                    settle(r[c], 2 * hf + c);
+                    if (!first_max) mx = max_of(r[c], mx);
+                    sum = weights(r[c], pk[c], ref, sum);
+                }
+                if (!first_max) {
+                    mx *= eff;                                        // scale > 0; -inf stays -inf
+                    // move the reference up only when the maximum has run away from it
+                    const bool adopt = (m == -CUDART_INF_F) && (mx > m);      // nothing accumulated under the old reference
+                    const bool jump = (m != -CUDART_INF_F) && (mx > m + T5O_JUMP);
+                    if (__any_sync(0xffffffffu, adopt || jump)) {
+                        move_to(mx, jump, hf ? &pv_half[g] : &pv_done[g], (hf ? j : j - 1) & 1);
+                        if (!ok) break;
+                        if (adopt || jump) m = mx;
+                        ref = m == -CUDART_INF_F ? 0.0f : m;
+                        sum = 0.0f;
+                        t5_ld32(s_at, r[0]);
+#pragma unroll
+                        for (int c = 0; c < 2; ++c) {
+                            t5_wait_ld();
+                            if (c < 1) t5_ld32(s_at + 32, r[1]);
+                            settle(r[c], 2 * hf + c);
+                            sum = weights(r[c], pk[c], ref, sum);
+                        }
+                    }
+                }
+                l += sum;
+                t5_st16(p_at, pk[0]);                                 // over columns of S that have been read
+                t5_st16(p_at + 16, pk[1]);
+                t5_wait_st();
+                t5_fence_before();
+                if constexpr (EXT) {
+                    // Keys of the tile that no row of the block sees (behind its last one, below the window, behind the kept ones) have
+                    // weights of zero, but what lies there may be anything (a request that had the page before, a held page's copy), and
+                    // zero times a value that is not finite is NaN: their values are set to zero before the products, a row of 256 bytes a
+                    // thread.
+                    const int key = kt + row, lo_first = first_visible(pos_first, window);
+                    if (hf == 0 && g == 0 && (kt + T5O_BN - 1 > pos_last || (kt < lo_first && kt + T5O_BN > keep))) {
+                        ok = __all_sync(0xffffffffu, t5_wait(&v_full[j % STAGES], (j / STAGES) & 1, &abort_flag, status, row_base));
+                        if (!ok) break;
+                        if (key > pos_last || (key < lo_first && key >= keep)) {
+                            uint4* v = reinterpret_cast<uint4*>(v_s + (j % STAGES) * T5O_TILE + row * 64);
+#pragma unroll
+                            for (int c = 0; c < 16; ++c) v[(c >> 3) * (T5O_HALF / 8) + ((c + lane) & 7)] = make_uint4(0u, 0u, 0u, 0u);      // a quarter-warp: all banks
+                        }
+                        asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+                    }
+                }
+                __syncwarp();
+                if (lane == 0) t5_arrive(&p_full[g][hf]);
+            }
         }
-        // the row sum is the two halves' sums
-        x_sum[g][half][row] = l;
-        asm volatile("bar.sync %0, 256;\n" ::"r"(1 + g) : "memory");
-        l += x_sum[g][half ^ 1][row];
-        if (ok && t5_wait(&pv_done[g], (n_tiles - 1) & 1, &abort_flag, status, row_base)) {
+        if (ok && __all_sync(0xffffffffu, t5_wait(&pv_done[g], (n_tiles - 1) & 1, &abort_flag, status, row_base))) {
             t5_fence_after();
             if (EXT && ext.sinks) l += t5_ex2(fmaf(ext.sinks[h0 + g], 1.4426950408889634f, -m));   // a term without a value
             float inv = (l > 0.0f) ? 1.0f / l : 0.0f;
-            bf16* orow = out + (static_cast<size_t>(row_base + row) * nq + h0 + g) * T5_D + half * 64;
+            bf16* orow = out + (static_cast<size_t>(row_base + row) * nq + h0 + g) * T5_D;
             if constexpr (EXT) {
-                orow = out + static_cast<size_t>(row_base + row) * ext.out_stride + ext.out_off + (h0 + g) * T5_D + half * 64;
+                orow = out + static_cast<size_t>(row_base + row) * ext.out_stride + ext.out_off + (h0 + g) * T5_D;
                 inv *= ext.out_scale;
                 if (ext.gate && row < rows_here)
                     inv /= 1.0f + expf(-ext.gate[static_cast<size_t>(row_base + row) * ext.gate_stride + ext.gate_off + h0 + g]);
             }
-#pragma unroll 1
-            for (int c = 0; c < 64; c += 32) {
-                unsigned r[32];
-                t5_ld32(my_o + c, r);
+            unsigned r[2][32];
+            t5_ld32(my_o, r[0]);
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
                 t5_wait_ld();
+                if (c < 3) t5_ld32(my_o + 32 * (c + 1), r[(c + 1) & 1]);
                 if (row < rows_here) {
+                    const unsigned (&v)[32] = r[c & 1];
 #pragma unroll
                     for (int i = 0; i < 32; i += 8) {
                         uint4 w;
-                        w.x = t5_pack(__uint_as_float(r[i]) * inv, __uint_as_float(r[i + 1]) * inv);
-                        w.y = t5_pack(__uint_as_float(r[i + 2]) * inv, __uint_as_float(r[i + 3]) * inv);
-                        w.z = t5_pack(__uint_as_float(r[i + 4]) * inv, __uint_as_float(r[i + 5]) * inv);
-                        w.w = t5_pack(__uint_as_float(r[i + 6]) * inv, __uint_as_float(r[i + 7]) * inv);
-                        *reinterpret_cast<uint4*>(orow + c + i) = w;
+                        w.x = t5_pack(__uint_as_float(v[i]) * inv, __uint_as_float(v[i + 1]) * inv);
+                        w.y = t5_pack(__uint_as_float(v[i + 2]) * inv, __uint_as_float(v[i + 3]) * inv);
+                        w.z = t5_pack(__uint_as_float(v[i + 4]) * inv, __uint_as_float(v[i + 5]) * inv);
+                        w.w = t5_pack(__uint_as_float(v[i + 6]) * inv, __uint_as_float(v[i + 7]) * inv);
+                        *reinterpret_cast<uint4*>(orow + c * 32 + i) = w;
                     }
                 }
             }

@@ -34,6 +34,11 @@ __device__ __forceinline__ bool t5_wait(unsigned long long* bar, unsigned parity
     if (atomicCAS(status, 0, 6) == 0) status[1] = where;
     return false;
 }
+// the same by a whole warp: one answer for all lanes
+__device__ __forceinline__ bool t5_wait_warp(unsigned long long* bar, unsigned parity, volatile int* abort_flag, int32_t* status,
+                                             int where) {
+    return __all_sync(0xffffffffu, t5_wait(bar, parity, abort_flag, status, where));
+}
 __device__ __forceinline__ void t5_tma_2d(void* dst, const CUtensorMap* map, int x, int y, unsigned long long* bar) {
     asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];\n" ::
                      "r"(t5_smem(dst)), "l"(map), "r"(x), "r"(y), "r"(t5_smem(bar)) : "memory");
@@ -58,6 +63,32 @@ __device__ __forceinline__ void t5_mma_ts(unsigned d_tmem, unsigned a_tmem, unsi
     asm volatile("{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
                  " tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}\n" ::
                      "r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
+}
+// The same for a warp that goes through its loop with all lanes together, `lead` (t5_elect) set in one of them: operands that
+// all lanes hold alike stay in the registers that these instructions read, and a wait in front of a product costs 15 to 80
+// clocks of the tensor pipe's time.  With the loop inside a branch for one lane it costs 250 (four products of 64 clocks behind
+// each wait: 68 clocks a product against 127).
+__device__ __forceinline__ unsigned t5_elect() {
+    unsigned r;
+    asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}\n" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ void t5_mma_ss_lead(unsigned lead, unsigned d_tmem, unsigned long long a_desc, unsigned long long b_desc,
+                                               unsigned idesc, unsigned accumulate) {
+    asm volatile("{\n .reg .pred p, q;\n setp.ne.b32 p, %4, 0;\n setp.ne.b32 q, %5, 0;\n"
+                 " @q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::
+                     "r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(lead) : "memory");
+}
+__device__ __forceinline__ void t5_mma_ts_lead(unsigned lead, unsigned d_tmem, unsigned a_tmem, unsigned long long b_desc, unsigned idesc,
+                                               unsigned accumulate) {
+    asm volatile("{\n .reg .pred p, q;\n setp.ne.b32 p, %4, 0;\n setp.ne.b32 q, %5, 0;\n"
+                 " @q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}\n" ::
+                     "r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(lead) : "memory");
+}
+__device__ __forceinline__ void t5_commit_lead(unsigned lead, unsigned long long* bar) {
+    asm volatile("{\n .reg .pred q;\n setp.ne.b32 q, %1, 0;\n"
+                 " @q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n}\n" ::
+                     "r"(t5_smem(bar)), "r"(lead) : "memory");
 }
 // 32 consecutive 32-bit columns of this thread's TMEM lane
 __device__ __forceinline__ void t5_ld32(unsigned taddr, unsigned (&r)[32]) {
@@ -105,6 +136,20 @@ __device__ __forceinline__ float t5_ex2(float x) {
     float y;
     asm("ex2.approx.ftz.f32 %0, %1;\n" : "=f"(y) : "f"(x));
     return y;
+}
+// two float32 values in one register pair, for the instructions that work on both
+__device__ __forceinline__ unsigned long long t5_two(float lo, float hi) {
+    unsigned long long v;
+    asm("mov.b64 %0, {%1, %2};\n" : "=l"(v) : "f"(lo), "f"(hi));
+    return v;
+}
+__device__ __forceinline__ void t5_untwo(unsigned long long v, float& lo, float& hi) {
+    asm("mov.b64 {%0, %1}, %2;\n" : "=f"(lo), "=f"(hi) : "l"(v));
+}
+__device__ __forceinline__ unsigned long long t5_fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
+    unsigned long long d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;\n" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
 }
 __device__ __forceinline__ unsigned t5_pack(float lo, float hi) {
     const __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
