@@ -23,19 +23,20 @@
 // warps 10 to 17 drain.  Planes are double-buffered (96 KB of weights' planes, 96 KB of x at NT 128).
 // The weights' planes go to tensor memory, from where the tensor cores take their left operand: kept in shared memory, their
 // stores and the operand reads of 24 products a block (8 KB each) filled the shared-memory path (500 tokens of 4096 x 12288:
-// 323 us, 291 in tensor memory).  What bounds it is the chain of small products: 24 of 128 x NT x 16 a block take 2,500 to 2,900
-// clocks, the tensor pipe is busy for 43 % of the time (q/k/v and output product of a prompt of 500 tokens, width 4,096).
+// 323 us, 291 in tensor memory).  The issuing warp walks the blocks with all its lanes: in a branch for one lane each of the three
+// waits in front of a block kept the tensor pipe idle for 250 clocks of the 2,500 to 2,900 that a block took (its 24 products are
+// 1,536): 500 tokens of 4096 x 12288 296 -> 251, of 6144 x 4096 181 -> 152, 17 tokens of 24576 x 4096 146 -> 114.
 // The loop that makes sums again which are not finite stays rolled: unrolled into each of a drain thread's sums it cost
 // finite ones up to 20 % (500 tokens of 6144 x 4096: 209 us, now 167).
 // Tiles that fill the SMs badly are cut along K (`splits`), the parts added in order by a second kernel.
 //
 // Measured (us; the library's float32 product in brackets):
 //   N x K              17 rows        64 rows        128 rows       500 rows       2,048 rows
-//   6144 x 4096        41 (106)       42 (129)       49 (170)       167 (542)      577 (1,773)
-//   4096 x 4096        33 (105)       34 (106)       38 (126)       101 (311)      390 (1,132)
-//   24576 x 4096       143 (199)      148 (283)      169 (551)      576 (1,779)    2,028 (6,686)
-//   4096 x 12288       77 (250)       81 (321)       87 (373)       283 (925)      1,063 (3,353)
-//   2048 x 2048        23 (54)        23 (53)        25 (52)        37 (87)        109 (308)
+//   6144 x 4096        36 (106)       40 (129)       46 (170)       148 (542)      507 (1,773)
+//   4096 x 4096        30 (105)       32 (106)       40 (126)       95 (311)       343 (1,132)
+//   24576 x 4096       112 (199)      122 (283)      148 (551)      503 (1,779)    1,830 (6,686)
+//   4096 x 12288       71 (250)       77 (321)       91 (373)       282 (925)      990 (3,353)
+//   2048 x 2048        22 (54)        24 (53)        30 (52)        44 (87)        120 (308)
 // Matrices of fewer than 2^21 values stay with the library: of 1024 x 1024, 17 rows take 23 us against 18 (and 64 to 2,048 rows 23
 // to 34 against 29 to 86: for many rows the line could lie lower).
 #include "tcgen05_attention.cuh"
@@ -122,7 +123,7 @@ __global__ void __launch_bounds__(LT_THREADS, 1) linear_f32_tcgen05_kernel(
     const int m0 = blockIdx.x * NT, n0 = blockIdx.y * LT_ROWS;
     const int kb0 = blockIdx.z * blocks_per_split, kb_all = (K + LT_K - 1) / LT_K;
     const int kbs = min(blocks_per_split, kb_all - kb0);          // at least one: the host sees to that
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
     if (tid == 0) {
         abort_flag = 0;
         for (int s = 0; s < WB; ++s) { t5_mbar_init(&w_full[s], 1); t5_mbar_init(&w_empty[s], LT_SPLITTERS); }
@@ -141,7 +142,7 @@ __global__ void __launch_bounds__(LT_THREADS, 1) linear_f32_tcgen05_kernel(
     t5_fence_before();
     __syncthreads();
     t5_fence_after();
-    const unsigned tmem = tmem_base_s;
+    const unsigned tmem = __shfl_sync(0xffffffffu, tmem_base_s, 0);
 
     if (warp == 0) {
         if (lane == 0) {
@@ -183,37 +184,29 @@ __global__ void __launch_bounds__(LT_THREADS, 1) linear_f32_tcgen05_kernel(
         }
     } else if (warp == 1) {
         pdl_wait();                                               // before any bounded wait: the kernel in front may take its time
-        if (lane == 0) {
-            constexpr unsigned IDESC = t5_idesc(LT_ROWS, NT, 0);
-            const unsigned long long xd = t5_desc(x_s, 16, 1024);
-            constexpr unsigned long long X_STEP = X_PLANE * sizeof(bf16) >> 4;
-            // the smallest terms first: l h, h l, m m, m h, h m, h h
-            constexpr int WP[6] = {2, 0, 1, 1, 0, 0}, XP[6] = {0, 2, 1, 0, 1, 0};
-            auto block = [&](int kb, int st) -> bool {            // st = kb % 2, a constant where this is inlined
-                if (kb >= 2 && !lt_wait(&acc_empty[st], ((kb >> 1) - 1) & 1, &abort_flag, status)) return false;
-                const int xs = kb % XS;
-                if (!lt_wait(&x_full[xs], (kb / XS) & 1, &abort_flag, status)) return false;
-                const int ps = kb % PS;
-                if (!lt_wait(&p_full[ps], (kb / PS) & 1, &abort_flag, status)) return false;
-                t5_fence_after();
-                const unsigned long long xb = xd + xs * 3 * X_STEP;
-                const unsigned pl = tmem + PLANE_COL + ps * 96;
+        constexpr unsigned IDESC = t5_idesc(LT_ROWS, NT, 0);
+        const unsigned lead = t5_elect();                         // all lanes walk the blocks, one issues
+        const unsigned long long xd = t5_desc(x_s, 16, 1024);
+        constexpr unsigned long long X_STEP = X_PLANE * sizeof(bf16) >> 4;
+        // the smallest terms first: l h, h l, m m, m h, h m, h h
+        constexpr int WP[6] = {2, 0, 1, 1, 0, 0}, XP[6] = {0, 2, 1, 0, 1, 0};
+#pragma unroll 1
+        for (int kb = 0; kb < kbs; ++kb) {
+            const int st = kb & 1, xs = kb % XS, ps = kb % PS;
+            if (kb >= 2 && !lt_wait_warp(&acc_empty[st], ((kb >> 1) - 1) & 1, &abort_flag, status)) break;
+            if (!lt_wait_warp(&x_full[xs], (kb / XS) & 1, &abort_flag, status)) break;
+            if (!lt_wait_warp(&p_full[ps], (kb / PS) & 1, &abort_flag, status)) break;
+            t5_fence_after();
+            const unsigned long long xb = xd + xs * 3 * X_STEP;
+            const unsigned pl = tmem + PLANE_COL + ps * 96;
 #pragma unroll
-                for (int t = 0; t < 6; ++t)
+            for (int t = 0; t < 6; ++t)
 #pragma unroll
-                    for (int k = 0; k < 4; ++k)
-                        t5_mma_ts(tmem + st * NT, pl + WP[t] * 32 + k * 8, xb + XP[t] * X_STEP + 2 * k, IDESC,
-                                  t > 0 || k > 0);
-                t5_commit(&p_empty[ps]);
-                t5_commit(&x_empty[xs]);
-                t5_commit(&acc_full[st]);
-                return true;
-            };
-            bool ok = true;
-            for (int kb = 0; ok && kb < kbs; kb += 2) {
-                ok = block(kb, 0);
-                if (ok && kb + 1 < kbs) ok = block(kb + 1, 1);
-            }
+                for (int k = 0; k < 4; ++k)
+                    t5_mma_ts_lead(lead, tmem + st * NT, pl + WP[t] * 32 + k * 8, xb + XP[t] * X_STEP + 2 * k, IDESC, t > 0 || k > 0);
+            t5_commit_lead(lead, &p_empty[ps]);
+            t5_commit_lead(lead, &x_empty[xs]);
+            t5_commit_lead(lead, &acc_full[st]);
         }
     } else if (warp < 10) {
         // ---- split the weights: two threads a row, each 16 k-values of every box ----
@@ -300,12 +293,19 @@ __global__ void __launch_bounds__(LT_THREADS, 1) linear_f32_tcgen05_kernel(
     }
 }
 
-__global__ void linear_f32_sum_kernel(const float* __restrict__ parts, float* __restrict__ y, long long n, int splits) {
+// Four neighbours a thread, one where the length is no multiple of four (the parts then start anywhere).  The same sums in the
+// same order; three parts of 500 x 6,144: 17 us with one value a thread, now 11.
+template <typename V>
+__global__ void linear_f32_sum_kernel(const V* __restrict__ parts, V* __restrict__ y, long long n, int splits) {
     pdl_begin();
     const long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    float v = parts[i];
-    for (int s = 1; s < splits; ++s) v += parts[s * n + i];
+    V v = parts[i];
+    for (int s = 1; s < splits; ++s) {
+        const V p = parts[s * n + i];
+        if constexpr (sizeof(V) == 16) { v.x += p.x; v.y += p.y; v.z += p.z; v.w += p.w; }
+        else v += p;
+    }
     y[i] = v;
 }
 
@@ -325,9 +325,10 @@ static bool lt_encode_f32(CUtensorMap* map, const void* base, long long cols, lo
 static int lt_tile(int M) { return M <= 32 ? 32 : M <= 64 ? 64 : 128; }
 
 // Into how many parts K is cut: the least of waves of 148 CTAs x (blocks of 64 x BLK + 4 us) + the parts' way through memory,
-// with a block's time (1.5 us at 128 tokens, 1.0 below).  In 1, 2, 3, 4, 6, 8 parts (us): 500 tokens of 6144 x 4096 195, 169, 167,
-// 200, 203, 238 (takes 3), of 4096 x 4096 101, 115, 124, 134, 148, 155 (1), of 4096 x 12288 278, 297, 307, 315, 328, 313 (1); 17
-// tokens of 4096 x 12288 259, 137, 96, 77, 101, 83 (4), of 24576 x 4096 182, 149, 142, 163, 161, 177 (3).
+// with a block's time (1.5 us at 128 tokens, 1.0 below: a fifth more than it takes, and fewer parts of equal time
+// would sum longer runs).  In 1, 2, 3, 4, 6, 8 parts (us): 500 tokens of 6144 x 4096 171, 148, 146, 171, 175, - (takes 3), of 4096 x
+// 4096 95, 103, 110, 120, 134, 142 (1), of 4096 x 12288 249, 259, 267, 275, 288, 280 (1); 17 tokens of 4096 x 12288 214, 116, 83,
+// 67, 83, 69 (4), of 24576 x 4096 150, 124, 116, 128, 128, 136 (3).
 extern "C" int llm_linear_f32_tcgen05_splits(int M, int N, int K) {
     if (M <= 0 || N <= 0 || K <= 0) return 1;
     const int nt = lt_tile(M);
@@ -372,8 +373,12 @@ extern "C" int llm_linear_f32_tcgen05(const float* x, const float* w, float* y, 
     if (nt == 32) GO(32, 8, 5, 4) else if (nt == 64) GO(64, 6, 5, 4) else GO(128, 4, 3, 2)
 #undef GO
     if (splits > 1) {
-        const long long n = static_cast<long long>(M) * N;
-        launch_pdl(linear_f32_sum_kernel, dim3(static_cast<unsigned>((n + 255) / 256)), dim3(256), 0, s, static_cast<const float*>(parts), y, n, splits);
+        const long long n = static_cast<long long>(M) * N, n4 = n / 4;
+        if (n % 4 == 0 && aligned16(parts) && aligned16(y))
+            launch_pdl((linear_f32_sum_kernel<float4>), dim3(static_cast<unsigned>((n4 + 255) / 256)), dim3(256), 0, s,
+                       reinterpret_cast<const float4*>(parts), reinterpret_cast<float4*>(y), n4, splits);
+        else
+            launch_pdl((linear_f32_sum_kernel<float>), dim3(static_cast<unsigned>((n + 255) / 256)), dim3(256), 0, s, static_cast<const float*>(parts), y, n, splits);
     }
     return launch_status();
 }
