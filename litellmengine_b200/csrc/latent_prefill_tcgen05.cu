@@ -11,10 +11,12 @@
 //   latent_q_pack    the queries [qn | rotated qr] per head in bfloat16
 //   attention        below
 // Measured, 32 heads over rows of 512 + 64, a prompt of 2,000 tokens: attention over the cached rows 1,275 us; here rows 5,
-// map 18, queries 12, attention 81 us (0.54 PFLOP/s of what it cannot do without, 43 GFLOP).  The layer 1,480 -> 273 us.
+// map 18, queries 12, attention 62 us (0.69 PFLOP/s of what it cannot do without, 43 GFLOP; with two threads a row that exchanged
+// their maxima before the weights, and products issued in a branch for one lane, 85).  The layer 1,480 -> 237 us.
 //
 // Attention.  The structure of the one-pass kernel in attention_prefill_tcgen05.cu (a reference maximum that trails the
-// running one, two rows of work in turns on the tensor pipe, P over S in TMEM, two softmax threads a row), with two changes.
+// running one, two rows of work in turns on the tensor pipe, P over S in TMEM, a softmax thread a row, weights of half a tile made
+// beside their maximum), with two changes.
 // Every head has keys of its own, so the two pieces of work that share a key/value tile are two tiles of 128 QUERY rows of
 // one head.  And a tile is 96 keys: queries are 2 x 128 x 192 (96 KB), a tile of 128 keys with its values 80 KB, and two of
 // those would not fit beside them; two of 96 keys (60 KB each) do, and a product of N 96 is as efficient as one of 128.
@@ -30,7 +32,7 @@
 #define LP_DV 128
 #define LP_STAGES 2
 #define LP_JUMP 8.0f
-#define LP_THREADS (64 + 2 * 256)
+#define LP_THREADS (128 + 2 * 128)            // producer, issuer, two without work, four softmax warps a query tile
 
 __device__ __forceinline__ void lp_ld16(unsigned taddr, unsigned (&r)[48], int at) {
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];\n"
@@ -107,11 +109,9 @@ __global__ void __launch_bounds__(LP_THREADS, 1) latent_prefill_tcgen05_kernel(
     bf16* k_s = q_s + 2 * 3 * LP_QB;                              // [stages][3][96][64]
     bf16* v_s = k_s + LP_STAGES * 3 * LP_KB;                      // [stages][2][96][64]
     __shared__ __align__(8) unsigned long long q_full, k_full[LP_STAGES], k_empty[LP_STAGES], v_full[LP_STAGES], v_empty[LP_STAGES],
-        s_full[2], p_full[2], pv_done[2];
+        s_full[2], p_full[2][2], pv_half[2], pv_done[2];
     __shared__ unsigned tmem_base_s;
     __shared__ int abort_flag;
-    __shared__ float x_max[2][2][2][128];                         // [tile parity][query tile][column half][row]
-    __shared__ float x_sum[2][2][128];
 
     const int h = blockIdx.x;
     const int seg = tiles[2 * blockIdx.y], q0 = tiles[2 * blockIdx.y + 1];
@@ -120,7 +120,7 @@ __global__ void __launch_bounds__(LP_THREADS, 1) latent_prefill_tcgen05_kernel(
     const int past = entry_kv_len[e] - q_len - first_pos;         // positions are counted from the first gathered row
     const int row_base = entry_q_start[e] + q0;
     const int rows_all = min(2 * LP_BM, q_len - q0);
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
     auto rows_of = [&](int g) { return max(0, min(LP_BM, rows_all - g * LP_BM)); };
     const int k_lo = first_visible(past + q0, window) / LP_BN * LP_BN;      // the earliest key of the earliest row
     auto tiles_of = [&](int g) {                                  // key tiles that query tile g walks, all from k_lo
@@ -138,7 +138,8 @@ __global__ void __launch_bounds__(LP_THREADS, 1) latent_prefill_tcgen05_kernel(
         }
         for (int g = 0; g < 2; ++g) {
             t5_mbar_init(&s_full[g], 1);
-            t5_mbar_init(&p_full[g], 256);
+            for (int hf = 0; hf < 2; ++hf) t5_mbar_init(&p_full[g][hf], 4);      // a softmax warp each
+            t5_mbar_init(&pv_half[g], 1);
             t5_mbar_init(&pv_done[g], 1);
         }
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
@@ -150,7 +151,7 @@ __global__ void __launch_bounds__(LP_THREADS, 1) latent_prefill_tcgen05_kernel(
     t5_fence_before();
     __syncthreads();
     t5_fence_after();
-    const unsigned tmem = tmem_base_s;
+    const unsigned tmem = __shfl_sync(0xffffffffu, tmem_base_s, 0);
     auto s_col = [](int g) { return static_cast<unsigned>(g * 128); };           // 96 columns used
     auto o_col = [](int g) { return static_cast<unsigned>(256 + g * 128); };
 
@@ -192,158 +193,171 @@ __global__ void __launch_bounds__(LP_THREADS, 1) latent_prefill_tcgen05_kernel(
         }
     } else if (warp == 1) {
         // ---- MMA issuer: S0(j), O1 += P1 V(j-1), S1(j), O0 += P0 V(j); a query tile takes part while it has keys ----
-        if (lane == 0) {
-            constexpr unsigned IDESC_QK = t5_idesc(LP_BM, LP_BN, 0);
-            constexpr unsigned IDESC_PV = t5_idesc(LP_BM, LP_DV, 1);
-            const unsigned long long qd0 = t5_desc(q_s, 16, 1024), kd0 = t5_desc(k_s, 16, 1024);
-            const unsigned long long vd0 = t5_desc(v_s, LP_KB * sizeof(bf16), 1024);
-            constexpr unsigned long long K_STEP = (3 * LP_KB * sizeof(bf16)) >> 4, V_STEP = (2 * LP_KB * sizeof(bf16)) >> 4;
-            auto qk = [&](int g, int st) {                        // g, st: constants where this is inlined
+        // All lanes walk the loop, one of them issues.
+        constexpr unsigned IDESC_QK = t5_idesc(LP_BM, LP_BN, 0);
+        constexpr unsigned IDESC_PV = t5_idesc(LP_BM, LP_DV, 1);
+        const unsigned lead = t5_elect();
+        const unsigned long long qd0 = t5_desc(q_s, 16, 1024), kd0 = t5_desc(k_s, 16, 1024);
+        const unsigned long long vd0 = t5_desc(v_s, LP_KB * sizeof(bf16), 1024);
+        constexpr unsigned long long K_STEP = (3 * LP_KB * sizeof(bf16)) >> 4, V_STEP = (2 * LP_KB * sizeof(bf16)) >> 4;
+        auto qk = [&](int g, int st) {
 #pragma unroll
-                for (int k = 0; k < 12; ++k)
-                    t5_mma_ss(tmem + s_col(g), qd0 + (((g * 3 + (k >> 2)) * LP_QB + (k & 3) * 16) * sizeof(bf16) >> 4),
-                              kd0 + st * K_STEP + (((k >> 2) * LP_KB + (k & 3) * 16) * sizeof(bf16) >> 4), IDESC_QK, k > 0);
-                t5_commit(&s_full[g]);
-            };
-            auto pv = [&](int g, int st, bool first) {
+            for (int k = 0; k < 12; ++k)
+                t5_mma_ss_lead(lead, tmem + s_col(g), qd0 + g * ((3 * LP_QB * sizeof(bf16)) >> 4) + (((k >> 2) * LP_QB + (k & 3) * 16) * sizeof(bf16) >> 4),
+                               kd0 + st * K_STEP + (((k >> 2) * LP_KB + (k & 3) * 16) * sizeof(bf16) >> 4), IDESC_QK, k > 0);
+            t5_commit_lead(lead, &s_full[g]);
+        };
+        auto pv = [&](int g, int j, int st) -> bool {             // in two halves, each as soon as its weights are there
 #pragma unroll
-                for (int k = 0; k < 6; ++k)                       // P of keys 48 .. 95 lies over S column 48
-                    t5_mma_ts(tmem + o_col(g), tmem + s_col(g) + (k / 3) * 48 + (k % 3) * 8, vd0 + st * V_STEP + ((k * 16 * 64) * sizeof(bf16) >> 4),
-                              IDESC_PV, (!first || k > 0) ? 1u : 0u);
-                t5_commit(&pv_done[g]);
-            };
-            bool ok = t5_wait(&q_full, 0, &abort_flag, status, row_base);
-            auto one_tile = [&](int j, int st) -> bool {          // st = j % 2, a constant where this is inlined
-                if (!t5_wait(&k_full[st], (j >> 1) & 1, &abort_flag, status, row_base)) return false;
+            for (int hf = 0; hf < 2; ++hf) {
+                if (!t5_wait_warp(&p_full[g][hf], j & 1, &abort_flag, status, row_base)) return false;
                 t5_fence_after();
-                if (j < n0) qk(0, st);
-                if (j > 0) {
-                    if (j - 1 < n1) {
-                        if (!t5_wait(&p_full[1], (j - 1) & 1, &abort_flag, status, row_base)) return false;
-                        t5_fence_after();
-                        pv(1, 1 - st, j == 1);
-                    }
-                    t5_commit(&v_empty[1 - st]);                  // the last reader of the values of tile j - 1
-                }
-                if (j < n1) qk(1, st);
-                t5_commit(&k_empty[st]);
-                if (!t5_wait(&v_full[st], (j >> 1) & 1, &abort_flag, status, row_base)) return false;
-                if (j < n0) {
-                    if (!t5_wait(&p_full[0], j & 1, &abort_flag, status, row_base)) return false;
-                    t5_fence_after();
-                    pv(0, st, j == 0);
-                }
-                return true;
-            };
-            static_assert(LP_STAGES == 2, "the issue loop is unrolled by the number of stages");
-            for (int j = 0; ok && j < n_tiles; j += 2) {
-                ok = one_tile(j, 0);
-                if (ok && j + 1 < n_tiles) ok = one_tile(j + 1, 1);
+#pragma unroll
+                for (int k = 3 * hf; k < 3 * hf + 3; ++k)
+                    t5_mma_ts_lead(lead, tmem + o_col(g), tmem + s_col(g) + k * 8, vd0 + st * V_STEP + ((k * 16 * 64) * sizeof(bf16) >> 4),
+                                   IDESC_PV, (j > 0 || k > 0) ? 1u : 0u);
+                t5_commit_lead(lead, hf ? &pv_done[g] : &pv_half[g]);
             }
-            if (ok && n1 == n_tiles && t5_wait(&p_full[1], (n1 - 1) & 1, &abort_flag, status, row_base)) {
-                t5_fence_after();
-                if ((n1 - 1) & 1) pv(1, 1, n1 == 1); else pv(1, 0, n1 == 1);
+            return true;
+        };
+        bool ok = t5_wait_warp(&q_full, 0, &abort_flag, status, row_base);
+#pragma unroll 1
+        for (int j = 0; ok && j < n_tiles; ++j) {
+            const int st = j & 1;
+            ok = t5_wait_warp(&k_full[st], (j >> 1) & 1, &abort_flag, status, row_base);
+            if (!ok) break;
+            t5_fence_after();
+            if (j < n0) qk(0, st);
+            if (j > 0) {
+                if (j - 1 < n1) {
+                    ok = pv(1, j - 1, 1 - st);
+                    if (!ok) break;
+                }
+                t5_commit_lead(lead, &v_empty[1 - st]);           // the last reader of the values of tile j - 1
             }
+            if (j < n1) qk(1, st);
+            t5_commit_lead(lead, &k_empty[st]);
+            ok = t5_wait_warp(&v_full[st], (j >> 1) & 1, &abort_flag, status, row_base);
+            if (ok && j < n0) ok = pv(0, j, st);
         }
-    } else {
-        // ---- softmax: two threads share a query row, 48 columns of S each ----
-        const int wl = warp - 2;
-        const int g = wl >> 3;                                    // warps 2..9: the first query tile, 10..17: the second
-        const int half = (wl >> 2) & 1;                           // columns 48 * half .. + 47 of every tile
+        static_assert(LP_STAGES == 2, "a tile's stage is its parity");
+        if (ok && n1 == n_tiles) pv(1, n1 - 1, (n1 - 1) & 1);
+    } else if (warp >= 4) {
+        // ---- softmax: a thread owns one query row = one TMEM lane, all 96 columns of a tile ----
+        const int g = (warp - 4) >> 2;                            // warps 4..7: the first query tile, 8..11: the second
         const int quarter = warp & 3;
         const int row = quarter * 32 + lane;
         const unsigned lane_addr = static_cast<unsigned>(quarter * 32) << 16;
-        const unsigned my_s = tmem + lane_addr + s_col(g) + half * 48;
-        const unsigned my_o = tmem + lane_addr + o_col(g) + half * 64;
+        const unsigned my_s = tmem + lane_addr + s_col(g);
+        const unsigned my_o = tmem + lane_addr + o_col(g);
         const int rows_here = rows_of(g), mine = g ? n1 : n0;
-        const int pos_first = past + q0 + g * LP_BM;
-        const int pos = row < rows_here ? pos_first + row : -1;
+        // rows behind the portion's last are other tokens' or zeros: they are worked like the rest and not stored
+        const int pos_first = past + q0 + g * LP_BM, pos = pos_first + row;
         const int lo = first_visible(pos, window), lo_last = first_visible(pos_first + rows_here - 1, window);
         float m = -CUDART_INF_F, l = 0.0f;                        // m: the reference maximum, in units of log2
         bool ok = true;
         for (int j = 0; j < mine; ++j) {
-            const int kt = k_lo + j * LP_BN + half * 48;          // this thread's first key of the tile
-            // After a wait has run out (ok false) a thread still passes every barrier below, as often as the others.
-            if (ok && !t5_wait(&s_full[g], j & 1, &abort_flag, status, row_base)) ok = false;
+            const int kt = k_lo + j * LP_BN;
+            // after a wait has run out (ok false, for whole warps) a thread touches nothing else
+            if (ok) ok = __all_sync(0xffffffffu, t5_wait(&s_full[g], j & 1, &abort_flag, status, row_base));
+            if (!ok) break;
             t5_fence_after();
-            const bool full_tile = (kt + 47 <= pos_first) && (kt >= lo_last) && (rows_here == LP_BM);
+            const bool full_tile = (kt + LP_BN - 1 <= pos_first) && (kt >= lo_last);
             unsigned r[48];
-            float mx = -CUDART_INF_F;
-            auto fetch = [&] {
-                lp_ld16(my_s, r, 0);
-                lp_ld16(my_s + 16, r, 16);
-                lp_ld16(my_s + 32, r, 32);
+            auto fetch = [&](int hf) {                            // 48 scores of the row, what it does not see at -inf
+                lp_ld16(my_s + 48 * hf, r, 0);
+                lp_ld16(my_s + 48 * hf + 16, r, 16);
+                lp_ld16(my_s + 48 * hf + 32, r, 32);
                 t5_wait_ld();
-            };
-            if (ok) {
-                fetch();
-                if (full_tile) {
-#pragma unroll
-                    for (int i = 0; i < 48; ++i) mx = fmaxf(mx, __uint_as_float(r[i]));
-                } else {
-#pragma unroll
-                    for (int i = 0; i < 48; ++i)
-                        if (kt + i <= pos && kt + i >= lo) mx = fmaxf(mx, __uint_as_float(r[i]));
-                }
-                x_max[j & 1][g][half][row] = mx;
-            }
-            asm volatile("bar.sync %0, 256;\n" ::"r"(1 + g) : "memory");      // the 8 softmax warps of this query tile
-            if (!ok) continue;
-            mx = fmaxf(mx, x_max[j & 1][g][half ^ 1][row]) * scale_log2e;     // scale > 0; -inf stays -inf
-            const bool adopt = (m == -CUDART_INF_F) && (mx > m);
-            const bool jump = (m != -CUDART_INF_F) && (mx > m + LP_JUMP);
-            if (__any_sync(0xffffffffu, jump)) {
-                // O still receives the previous tile's product: wait for it, then scale this thread's half of its row
-                if (!t5_wait(&pv_done[g], (j - 1) & 1, &abort_flag, status, row_base)) { ok = false; continue; }
-                t5_fence_after();
-                const float alpha = jump ? t5_ex2(m - mx) : 1.0f;
-                l *= alpha;
-#pragma unroll 1
-                for (int c = 0; c < 64; c += 32) {
-                    unsigned o[32];
-                    t5_ld32(my_o + c, o);
-                    t5_wait_ld();
-#pragma unroll
-                    for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
-                    t5_st32(my_o + c, o);
-                }
-                t5_wait_st();
-                fetch();
-            }
-            if (adopt || jump) m = mx;
-            const float msub = (m == -CUDART_INF_F) ? 0.0f : m;
-            unsigned pk[24];                                      // the weights, rounded to bfloat16, over the first half of this thread's S
-#pragma unroll
-            for (int i = 0; i < 48; i += 2) {
-                float p0 = t5_ex2(fmaf(__uint_as_float(r[i]), scale_log2e, -msub));
-                float p1 = t5_ex2(fmaf(__uint_as_float(r[i + 1]), scale_log2e, -msub));
                 if (!full_tile) {
-                    const int key = kt + i;
-                    p0 = (key <= pos && key >= lo) ? p0 : 0.0f;
-                    p1 = (key + 1 <= pos && key + 1 >= lo) ? p1 : 0.0f;
+                    const int k0 = kt + 48 * hf;
+                    auto first = [&](int n) { return n <= 0 ? 0ull : n >= 48 ? (1ull << 48) - 1ull : (1ull << n) - 1ull; };
+                    const unsigned long long seen = first(pos + 1 - k0) & ~first(lo - k0);
+#pragma unroll
+                    for (int i = 0; i < 48; ++i) r[i] = seen & (1ull << i) ? r[i] : 0xff800000u;
                 }
-                l += p0 + p1;
-                pk[i >> 1] = t5_pack(p0, p1);
+            };
+            auto max_of = [&] {
+                float a = __uint_as_float(r[0]), b = __uint_as_float(r[1]);
+#pragma unroll
+                for (int i = 2; i < 48; i += 2) { a = fmaxf(a, __uint_as_float(r[i])); b = fmaxf(b, __uint_as_float(r[i + 1])); }
+                return fmaxf(a, b);
+            };
+            auto weights = [&](unsigned (&pk)[24]) {              // rounded to bfloat16, and their sum
+                const float ref = m == -CUDART_INF_F ? 0.0f : m;
+                const unsigned long long e2 = t5_two(scale_log2e, scale_log2e), m2 = t5_two(-ref, -ref);
+                float s0 = 0.0f, s1 = 0.0f;
+#pragma unroll
+                for (int i = 0; i < 48; i += 2) {
+                    float x0, x1;
+                    t5_untwo(t5_fma2(t5_two(__uint_as_float(r[i]), __uint_as_float(r[i + 1])), e2, m2), x0, x1);
+                    const float p0 = t5_ex2(x0), p1 = t5_ex2(x1);
+                    pk[i >> 1] = t5_pack(p0, p1);
+                    s0 += p0;
+                    s1 += p1;
+                }
+                return s0 + s1;
+            };
+            // The row's reference moves up to mx when that has run away from it; O and l move too, once the products under way
+            // have joined O.
+            auto move_to = [&](float mx, unsigned long long* done, int parity) {
+                const bool adopt = (m == -CUDART_INF_F) && (mx > m), jump = (m != -CUDART_INF_F) && (mx > m + LP_JUMP);
+                if (__any_sync(0xffffffffu, jump)) {
+                    ok = __all_sync(0xffffffffu, t5_wait(done, parity, &abort_flag, status, row_base));
+                    if (!ok) return;
+                    t5_fence_after();
+                    const float alpha = jump ? t5_ex2(m - mx) : 1.0f;
+                    l *= alpha;
+#pragma unroll 1
+                    for (int c = 0; c < LP_DV; c += 32) {
+                        unsigned o[32];
+                        t5_ld32(my_o + c, o);
+                        t5_wait_ld();
+#pragma unroll
+                        for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
+                        t5_st32(my_o + c, o);
+                    }
+                }
+                if (adopt || jump) m = mx;
+            };
+            if (j == 0) {                                         // the first tile's maximum before its weights
+                fetch(0);
+                const float mx = max_of();
+                fetch(1);
+                move_to(fmaxf(mx, max_of()) * scale_log2e, nullptr, 0);       // scale > 0; -inf stays -inf; nothing to wait for
             }
-            lp_st8(my_s, pk, 0);
-            lp_st8(my_s + 8, pk, 8);
-            lp_st8(my_s + 16, pk, 16);
-            t5_wait_st();
-            t5_fence_before();
-            t5_arrive(&p_full[g]);
+#pragma unroll 1
+            for (int hf = 0; hf < 2; ++hf) {
+                unsigned pk[24];
+                fetch(hf);
+                // after that the weights are made at the reference that is there, beside their maximum, and again if it has to move
+                const float mx = j == 0 ? m : max_of() * scale_log2e;
+                float sum = weights(pk);
+                if (__any_sync(0xffffffffu, mx > (m == -CUDART_INF_F ? m : m + LP_JUMP))) {
+                    move_to(mx, hf ? &pv_half[g] : &pv_done[g], (hf ? j : j - 1) & 1);
+                    if (!ok) break;
+                    fetch(hf);
+                    sum = weights(pk);
+                }
+                l += sum;
+                lp_st8(my_s + 24 * hf, pk, 0);                    // over columns of S that have been read
+                lp_st8(my_s + 24 * hf + 8, pk, 8);
+                lp_st8(my_s + 24 * hf + 16, pk, 16);
+                t5_wait_st();
+                t5_fence_before();
+                __syncwarp();
+                if (lane == 0) t5_arrive(&p_full[g][hf]);
+            }
         }
-        x_sum[g][half][row] = l;                                  // the row sum is the two halves' sums
-        asm volatile("bar.sync %0, 256;\n" ::"r"(1 + g) : "memory");
-        l += x_sum[g][half ^ 1][row];
-        if (ok && mine > 0 && t5_wait(&pv_done[g], (mine - 1) & 1, &abort_flag, status, row_base)) {
+        if (ok && mine > 0 && __all_sync(0xffffffffu, t5_wait(&pv_done[g], (mine - 1) & 1, &abort_flag, status, row_base))) {
             t5_fence_after();
             float inv = (l > 0.0f) ? 1.0f / l : 0.0f;
             if (gate && row < rows_here)                          // a sigmoid gate per token and head, on the result as it leaves
                 inv /= 1.0f + expf(-gate[static_cast<size_t>(row_base + g * LP_BM + row) * gate_stride + h]);
             bool finite = l <= 3.402823466e38f;                   // not infinite, not NaN
-            bf16* orow = out + (static_cast<size_t>(row_base + g * LP_BM + row) * H + h) * LP_DV + half * 64;
+            bf16* orow = out + (static_cast<size_t>(row_base + g * LP_BM + row) * H + h) * LP_DV;
 #pragma unroll 1
-            for (int c = 0; c < 64; c += 32) {
+            for (int c = 0; c < LP_DV; c += 32) {
                 unsigned o[32];
                 t5_ld32(my_o + c, o);
                 t5_wait_ld();
@@ -363,9 +377,11 @@ __global__ void __launch_bounds__(LP_THREADS, 1) latent_prefill_tcgen05_kernel(
             }
             if (row < rows_here && !finite) {
                 const size_t token = static_cast<size_t>(row_base + g * LP_BM + row), at = static_cast<size_t>(kv_row0 + max(lo, 0));
-                lp_row_again(q + (token * H + h) * LP_DK, kv + (at * H + h) * 256, static_cast<size_t>(H) * 256,
-                             gathered + at * (R + 64) + R, R + 64, pos - max(lo, 0) + 1, half, scale_log2e,
-                             gate ? 1.0f / (1.0f + expf(-gate[token * gate_stride + h])) : 1.0f, orow);
+                const float share = gate ? 1.0f / (1.0f + expf(-gate[token * gate_stride + h])) : 1.0f;
+#pragma unroll 1
+                for (int half = 0; half < 2; ++half)
+                    lp_row_again(q + (token * H + h) * LP_DK, kv + (at * H + h) * 256, static_cast<size_t>(H) * 256,
+                                 gathered + at * (R + 64) + R, R + 64, pos - max(lo, 0) + 1, half, scale_log2e, share, orow + half * 64);
             }
         }
     }
