@@ -95,15 +95,22 @@ __device__ __forceinline__ void gp_tma_2d(void* dst, const CUtensorMap* map, int
 __device__ __forceinline__ void gp_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory"); }
 __device__ __forceinline__ void gp_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory"); }
 // Arrives, once the pair's products issued so far have run, on the barrier at this address in every CTA of `mask`.
-__device__ __forceinline__ void gp_commit_pair(unsigned long long* bar, unsigned short mask) {
-    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n" ::
-                     "r"(gp_smem(bar)), "h"(mask) : "memory");
+// `lead` is set in the one lane that does it.
+__device__ __forceinline__ void gp_commit_pair(unsigned lead, unsigned long long* bar, unsigned short mask) {
+    asm volatile("{\n .reg .pred q;\n setp.ne.b32 q, %2, 0;\n"
+                 " @q tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n}\n" ::
+                     "r"(gp_smem(bar)), "h"(mask), "r"(lead) : "memory");
 }
-__device__ __forceinline__ void gp_mma_pair(unsigned d_tmem, unsigned long long a_desc, unsigned long long b_desc, unsigned idesc,
-                                            unsigned accumulate) {
-    asm volatile("{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-                 " tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::
-                     "r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
+__device__ __forceinline__ void gp_mma_pair(unsigned lead, unsigned d_tmem, unsigned long long a_desc, unsigned long long b_desc,
+                                            unsigned idesc, unsigned accumulate) {
+    asm volatile("{\n .reg .pred p, q;\n setp.ne.b32 p, %4, 0;\n setp.ne.b32 q, %5, 0;\n"
+                 " @q tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::
+                     "r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(lead) : "memory");
+}
+__device__ __forceinline__ unsigned gp_elect() {
+    unsigned r;
+    asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}\n" : "=r"(r));
+    return r;
 }
 __device__ __forceinline__ void gp_ld32(unsigned taddr, unsigned (&r)[32]) {
     asm volatile(
@@ -168,6 +175,11 @@ __device__ __forceinline__ bool gp_unit(const GpPlan& p, int i, int cluster, int
     return true;
 }
 
+// The rows of x that a CTA fetches for its 128 tokens from `row` on: at the end of x the last 128 there are, some of which
+// another CTA writes.  A box that reaches beyond x costs a third more time per stage than one inside it (256 tokens of 24,576 x
+// 4,096 55 us, 255 tokens 74; 512 and 500: 83 and 115).
+__device__ __forceinline__ int gp_first_row(int row, int T) { return T >= GP_BM ? min(row, T - GP_BM) : row; }
+
 // MODE 0: y[T, N] = x . w^T.  MODE 1: w is [gate; up] of 2 * inter rows, y[T, inter] = silu(gate) * up.
 // MODE 2: y[T, N] (float32) += x . w^T: the product joins the residual stream where it lies.
 // MODE 3: MODE 1 with the tanh form of gelu in place of silu (an instantiation of its own).
@@ -189,8 +201,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GP_THREADS, 1) linea
     __shared__ unsigned tmem_base_s;
     __shared__ int abort_flag;
 
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const unsigned rank = gp_cta_rank();
+    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
+    const unsigned rank = __shfl_sync(0xffffffffu, gp_cta_rank(), 0);
     const int cluster = blockIdx.x >> 1, clusters = gridDim.x >> 1;
     const int nk = (K + GP_BK - 1) / GP_BK;
 
@@ -208,7 +220,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GP_THREADS, 1) linea
     __syncthreads();
     gp_cluster_sync();                                            // the other CTA's barriers exist before anyone signals them
     gp_fence_after();
-    const unsigned tmem = tmem_base_s;
+    const unsigned tmem = __shfl_sync(0xffffffffu, tmem_base_s, 0);
     pdl_wait();                                                   // x is the output of the kernel before this one
 
     if (warp == 0) {
@@ -220,7 +232,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GP_THREADS, 1) linea
             GpUnit u;
             for (int i = 0; ok && gp_unit(plan, i, cluster, clusters, &u); ++i) {
                 const int half = (GP_BN / 2) / u.cut;             // rows of w this CTA brings per stage
-                const int row_x = u.mt * (2 * GP_BM) + static_cast<int>(rank) * GP_BM;
+                const int row_x = gp_first_row(u.mt * (2 * GP_BM) + static_cast<int>(rank) * GP_BM, T);
                 const int row_w = GP_GATED(MODE) ? (rank == 0 ? 0 : inter) + u.nt * (GP_BN / 2) + u.part * half
                                             : u.nt * GP_BN + u.part * (2 * half) + static_cast<int>(rank) * half;
                 const CUtensorMap* wm = u.cut == 1 ? &w_map : &w_map2;
@@ -237,8 +249,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GP_THREADS, 1) linea
                 for (int n = 0; n < 2000; ++n) __nanosleep(100);
         }
     } else if (warp == 1) {
-        // ---- product issuer (first CTA of the pair) ----
-        if (lane == 0 && rank == 0) {
+        // ---- product issuer (first CTA of the pair): all lanes walk the stages, one issues.  In a branch for one lane a wait
+        // keeps the tensor pipe idle for about 250 clocks (the operands have to be moved to where the instruction reads them) ----
+        if (rank == 0) {
+            const unsigned lead = gp_elect();
             const unsigned long long ad0 = gp_desc(a_s), bd0 = gp_desc(b_s);
             int it = 0;
             bool ok = true;
@@ -246,20 +260,22 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GP_THREADS, 1) linea
             for (int i = 0; ok && gp_unit(plan, i, cluster, clusters, &u); ++i) {
                 const int buf = i & 1;
                 const unsigned idesc = gp_idesc(2 * GP_BM, GP_BN / u.cut);
-                if (i >= 2 && !gp_wait<true>(&acc_empty[buf], ((i >> 1) - 1) & 1, &abort_flag, status)) break;
+                if (i >= 2) ok = __all_sync(0xffffffffu, gp_wait<true>(&acc_empty[buf], ((i >> 1) - 1) & 1, &abort_flag, status));
                 gp_fence_after();
-                for (int kb = 0; kb < nk; ++kb, ++it) {
+#pragma unroll 1
+                for (int kb = 0; ok && kb < nk; ++kb, ++it) {
                     const int s = it % GP_STAGES;
-                    if (!gp_wait<false>(&full[s], (it / GP_STAGES) & 1, &abort_flag, status)) { ok = false; break; }
+                    ok = __all_sync(0xffffffffu, gp_wait<false>(&full[s], (it / GP_STAGES) & 1, &abort_flag, status));
+                    if (!ok) break;
                     gp_fence_after();
                     const unsigned long long ad = ad0 + static_cast<unsigned long long>(s) * (TILE_ELEMS * sizeof(bf16) >> 4);
                     const unsigned long long bd = bd0 + static_cast<unsigned long long>(s) * (TILE_ELEMS * sizeof(bf16) >> 4);
 #pragma unroll
                     for (int k = 0; k < GP_BK / 16; ++k)          // 16 k-values = 32 bytes further along the swizzled row
-                        gp_mma_pair(tmem + buf * GP_BN, ad + 2 * k, bd + 2 * k, idesc, (kb | k) ? 1u : 0u);
-                    gp_commit_pair(&empty[s], 3);                 // the stage is free in both CTAs when these have run
+                        gp_mma_pair(lead, tmem + buf * GP_BN, ad + 2 * k, bd + 2 * k, idesc, (kb | k) ? 1u : 0u);
+                    gp_commit_pair(lead, &empty[s], 3);           // the stage is free in both CTAs when these have run
                 }
-                if (ok) gp_commit_pair(&acc_full[buf], 3);
+                if (ok) gp_commit_pair(lead, &acc_full[buf], 3);
             }
         }
     } else {
@@ -276,7 +292,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GP_THREADS, 1) linea
             const int buf = i & 1;
             if (!gp_wait<false>(&acc_full[buf], (i >> 1) & 1, &abort_flag, status)) break;
             gp_fence_after();
-            const int tok0 = u.mt * (2 * GP_BM) + static_cast<int>(rank) * GP_BM + quarter * 32;       // the warp's first token
+            const int mine = u.mt * (2 * GP_BM) + static_cast<int>(rank) * GP_BM;      // the first token this CTA writes
+            const int tok0 = gp_first_row(mine, T) + quarter * 32;                     // the warp's first token
             const unsigned acc = tmem + lane_addr + buf * GP_BN;
             const int cols = GP_BN / u.cut;                       // accumulator columns of this unit
             const int out_cols = GP_GATED(MODE) ? cols / 2 : cols;     // columns it writes
@@ -289,7 +306,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GP_THREADS, 1) linea
 #pragma unroll
                     for (int k = 0; k < 8; ++k) {
                         const int tok = tok0 + k * 4 + (lane >> 3), col = f0 + c + (lane & 7) * 4;
-                        old[k] = (tok < T && col < out_n)
+                        old[k] = (tok >= mine && tok < T && col < out_n)
                                      ? *reinterpret_cast<const float4*>(y + static_cast<size_t>(tok) * out_n + col)
                                      : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
                     }
@@ -322,7 +339,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GP_THREADS, 1) linea
                     const int rl = k * 4 + (lane >> 3), q = lane & 7;
                     float4 val = turn[rl * 8 + (q ^ (rl & 7))];
                     const int tok = tok0 + rl, col = f0 + c + q * 4;
-                    if (tok < T && col < out_n) {                 // out_n is a multiple of 8
+                    if (tok >= mine && tok < T && col < out_n) {  // out_n is a multiple of 8
                         TO* dst = y + static_cast<size_t>(tok) * out_n + col;
                         if constexpr (sizeof(TO) == 4) {
                             if (MODE == 2) { val.x += old[k].x; val.y += old[k].y; val.z += old[k].z; val.w += old[k].w; }
