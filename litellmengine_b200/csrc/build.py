@@ -46,6 +46,7 @@ FAMILIES: Dict[str, List[str]] = {
     "attention_wide": ["attention_wide.cu"],
     "sampling": ["sampling.cu"],
     "gemm_skinny": ["gemm_skinny.cu"],
+    "gemm_small": ["gemm_small.cu"],
     "gemm_pair_tcgen05": ["gemm_pair_tcgen05.cu"],
     "gemm_f32": ["gemm_f32.cu"],
     "gemm_f32_tcgen05": ["gemm_f32_tcgen05.cu"],

@@ -1913,6 +1913,79 @@ def linear_skinny(x: torch.Tensor, weight: torch.Tensor, out_dtype: torch.dtype,
     return out
 
 
+# ---- small products: all of their weights on the SMs at once ------------------------------------------
+class PendingRows:
+    """The rows a product will read that nobody has made yet: rmsnorm(h + delta) * weight in `dtype`, with h the float32 residual
+    stream and `delta` what has not joined it (None, a float32 tensor or a `PartialSum`).  The product that takes them makes
+    them and writes the sum to `stream`, the stream from then on (h itself without a delta)."""
+
+    def __init__(self, h: torch.Tensor, delta, weight: torch.Tensor, eps: float, dtype: torch.dtype):
+        self.h, self.delta, self.weight, self.eps, self.dtype = h, delta, weight, float(eps), dtype
+        self.stream = h if delta is None else torch.empty_like(h)
+
+    @property
+    def shape(self):
+        return self.h.shape
+
+
+_small_products: Dict[tuple, bool] = {}
+
+
+def small_product(rows: int, weight: torch.Tensor, normed: bool = False, gated: bool = False) -> bool:
+    """Whether `linear_small` takes a product of `rows` rows with this bfloat16 weight (gated: [gate; up])."""
+    if not (1 <= rows <= SKINNY_MAX_ROWS and weight.is_cuda and weight.dtype == torch.bfloat16 and weight.is_contiguous()
+            and weight.data_ptr() % 16 == 0):
+        return False
+    n, k = weight.shape
+    if normed and rows > 8:
+        return False
+    key = (rows <= 8, n, k, normed, gated)
+    got = _small_products.get(key)
+    if got is None:
+        f = _fn("gemm_small", "llm_linear_small_supported", [c_int, c_int, c_int, c_int, c_int])
+        got = _small_products[key] = bool((not gated or n % 2 == 0) and f(rows, n // 2 if gated else n, k, int(normed), int(gated)))
+    return got
+
+
+def pending_rows(h: torch.Tensor, delta, norm, weight: Optional[torch.Tensor], dtype: torch.dtype, gated: bool) -> Optional[PendingRows]:
+    """`norm`'s output for the product with `weight` that follows, left to that product if it can make it; None if it cannot."""
+    d = delta.parts if isinstance(delta, PartialSum) else delta
+    if (weight is None or dtype != torch.bfloat16 or not getattr(norm, "products_apply_it", False) or h.dim() != 2
+            or h.dtype != torch.float32 or not h.is_contiguous() or h.data_ptr() % 16 != 0 or h.shape[1] != weight.shape[1]
+            or norm.weight.dtype != torch.float32 or norm.weight.numel() != h.shape[1] or norm.weight.data_ptr() % 16 != 0
+            or not small_product(h.shape[0], weight, normed=True, gated=gated)):
+        return None
+    if d is not None and (not isinstance(d, torch.Tensor) or d.dtype != torch.float32 or not d.is_contiguous() or d.data_ptr() % 16 != 0
+                          or d.shape[-2:] != h.shape or (isinstance(delta, PartialSum) and delta.rounds_to is not None)):
+        return None
+    return PendingRows(h, delta, norm.weight, norm.eps, dtype)
+
+
+def linear_small(x, weight: torch.Tensor, out_dtype: torch.dtype, activation: Optional[str] = None, limit: float = 0.0) -> torch.Tensor:
+    """x [M <= 16, K] (bfloat16, or `PendingRows`) @ weight^T for weights that the SMs hold all at once, no partial sums.  With
+    `activation`, weight is [gate; up] and the result act(gate) * up in bfloat16, both rounded to bfloat16 first."""
+    made = isinstance(x, PendingRows)
+    M, K = x.shape
+    gated = activation is not None
+    n = weight.shape[0] // (2 if gated else 1)
+    if weight.shape[1] != K or (not made and x.dtype != torch.bfloat16) or weight.dtype != torch.bfloat16:
+        raise KernelError("the small product takes bfloat16 operands that agree on K")
+    h, pending, parts, stride = (x.h, x.delta, 1, 0) if made else (None, None, 1, 0)
+    if isinstance(pending, PartialSum):
+        parts, stride, pending = pending.parts.shape[0], pending.parts.stride(0), pending.parts
+    _dev(weight, *((h, pending, x.weight, x.stream) if made else (x,)))
+    tiled = _tiled.get(weight.data_ptr())
+    out = torch.empty((M, n), dtype=torch.bfloat16 if gated else out_dtype, device=weight.device)
+    f = _fn("gemm_small", "llm_linear_small",
+            [c_void_p, c_void_p, c_void_p, c_int, c_longlong, c_void_p, c_float, c_void_p, c_void_p, c_int, c_void_p, c_int, c_int, c_int,
+             c_float, c_int, c_int, c_int, c_void_p, c_void_p])
+    _check(f(None if made else _ptr(x), _ptr(h), _ptr(pending), parts, stride, _ptr(x.weight) if made else None, x.eps if made else 0.0,
+             _ptr(x.stream) if made and pending is not None else None, _ptr(tiled if tiled is not None else weight), int(tiled is not None),
+             _ptr(out), _dt(out), int(gated), ACTIVATIONS[activation] if gated else 0, float(limit), M, n, K,
+             _ptr(stream_status(weight.device)), _stream()), "linear_small")
+    return out
+
+
 _stream_status: Dict[str, torch.Tensor] = {}
 
 
@@ -2013,6 +2086,9 @@ def linear_silu_mul(x: torch.Tensor, w_gate_up: torch.Tensor, out_dtype: torch.d
                     limit: float = 0.0):
     """act(x @ gate^T) * (x @ up^T) for w_gate_up = [gate; up]: one kernel where the paired product
     takes it, else the product (which may stay a sum of k-splits) followed by the activation kernel."""
+    if out_dtype == torch.bfloat16 and (isinstance(x, PendingRows) or (x.dtype == torch.bfloat16 and x.is_contiguous() and x.data_ptr() % 16 == 0
+                                                                       and small_product(x.shape[0], w_gate_up, gated=True))):
+        return linear_small(x, w_gate_up, out_dtype, activation=activation, limit=limit)
     if out_dtype == torch.bfloat16 and _pair_takes(x, w_gate_up, w_gate_up.shape[0] // 2, "silu"):
         return linear_pair_silu_mul(x, w_gate_up, activation=activation, limit=limit)
     return silu_and_mul(linear(x, w_gate_up, out_dtype=out_dtype, partials_ok=True), activation=activation, limit=limit)
@@ -2070,9 +2146,9 @@ def linear_f32_tcgen05(x: torch.Tensor, weight: torch.Tensor) -> torch.Tensor:
 
 def linear(x: torch.Tensor, weight: torch.Tensor, out_dtype: Optional[torch.dtype] = None,
            partials_ok: bool = False):
-    """x [T, K] @ weight[N, K]^T.  Up to 16 bfloat16 rows (decode steps; up to 32 for the small products
-    of small models) go through the engine's
-    own weight-streaming kernel: alone it is level with the library for N = 4096..24576 and
+    """x [T, K] @ weight[N, K]^T.  Up to 16 bfloat16 rows with weights that the SMs hold all at once go to `linear_small` (which also
+    takes `PendingRows`); else up to 16 bfloat16 rows (decode steps; up to 32 for the small products of small models) go through the
+    engine's own weight-streaming kernel: alone it is level with the library for N = 4096..24576 and
     faster for K = 12288 (32 us against 36) and N = 151936 (203 against 218), and in a step it
     starts fetching weights while the kernel before it drains (a whole decode step of the
     Qwen3-8B shape at batch 8: 4.35 ms against 4.77 with the library products).  Everything else
@@ -2082,8 +2158,13 @@ def linear(x: torch.Tensor, weight: torch.Tensor, out_dtype: Optional[torch.dtyp
     keeps its product in true float32 (no TF32), whatever x is: up to 16 rows in the engine's own streaming kernel, more rows of large matrices
     on the tensor cores as sums of three bfloat16 values each, as near as float32 sums.  bfloat16 weights may be read before the
     kernel in front of the product in the stream has finished (they are nobody's output); float32 ones are not."""
+    if isinstance(x, PendingRows):
+        return linear_small(x, weight, out_dtype or x.dtype)
     _dev(x, weight)
     rows = x.shape[0]
+    if (x.dtype == torch.bfloat16 and x.is_contiguous() and x.data_ptr() % 16 == 0 and (out_dtype or x.dtype) in (torch.float32, torch.bfloat16)
+            and small_product(rows, weight)):
+        return linear_small(x, weight, out_dtype or x.dtype)
     if (x.dtype == torch.bfloat16 and weight.dtype == torch.bfloat16 and x.shape[1] % 8 == 0 and weight.data_ptr() % 16 == 0
             and rows >= 1 and (rows <= SKINNY_MAX_ROWS
                                or (rows <= SKINNY_SMALL_MAX_ROWS and skinny_small(weight.shape[0], weight.shape[1])))):

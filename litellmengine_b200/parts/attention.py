@@ -150,6 +150,11 @@ class AttentionMixer:
         n_dec = work.padded_rows.shape[0] if padded else work.num_decode
         return decode_key_splits(self.device, n_dec, self.nkv, decode_reach(batch, self.span)) if n_dec else 0
 
+    def first_product(self):
+        """The weight of the one product that reads the layer's input (which may come as `ops.PendingRows`), and whether it is
+        a gate/up pair."""
+        return self.w_qkv, False
+
     def forward(self, x: torch.Tensor, ctx: StageContext) -> torch.Tensor:
         b = ctx.batch
         qkv = ops.linear(x, self.w_qkv, out_dtype=torch.float32, partials_ok=True)   # normalised, rotated in 32-bit

@@ -202,6 +202,18 @@ class Block:
         return self.arrangement(self, h, delta, ctx)
 
 
+def _normed(norm, part, h: torch.Tensor, delta, dtype: torch.dtype):
+    """(h + delta, the part's input norm(h + delta)): by the norm's kernel, in place, or left to the part's first product."""
+    from ..csrc import ops
+    first = getattr(part, "first_product", None)
+    if first is not None and h.is_cuda:
+        weight, gated = first()
+        rows = ops.pending_rows(h, delta, norm, weight, dtype, gated)
+        if rows is not None:
+            return rows.stream, rows
+    return h, norm.forward(h, dtype, delta=delta, write_sum=delta is not None)
+
+
 @register_arrangement("pre_norm")
 def pre_norm(block: Block, h: torch.Tensor, delta: Optional[torch.Tensor], ctx: StageContext):
     """h += mixer(norm1(h)); h += ffn(norm2(h))  (src/model/qwen3.cpp:948-968).
@@ -214,13 +226,13 @@ def pre_norm(block: Block, h: torch.Tensor, delta: Optional[torch.Tensor], ctx: 
     from ..csrc import ops
     if not getattr(block.mixer_norm, "accepts_partials", False):
         delta = ops.as_tensor(delta)
-    x = block.mixer_norm.forward(h, block.dtype, delta=delta, write_sum=delta is not None)
+    h, x = _normed(block.mixer_norm, block.mixer, h, delta, block.dtype)
     ctx.partials_ok = getattr(block.feed_forward_norm, "accepts_partials", False)
     ctx.residual = h                                            # a part may add its result here itself and return None
     a = block.mixer.forward(x, ctx)
     if block.feed_forward is None:                              # a layer that is its mixer only: its output is what is pending
         return h, a
-    y = block.feed_forward_norm.forward(h, block.dtype, delta=a, write_sum=a is not None)
+    h, y = _normed(block.feed_forward_norm, block.feed_forward, h, a, block.dtype)
     extra = {}
     if getattr(block.feed_forward, "supports_partials", False):
         extra["partials_ok"] = True                             # the next norm (or `pre_norm` above) adds the splits

@@ -55,6 +55,9 @@ class SwiGLU:
     supports_partials = True   # forward(x, partials_ok=True) may return an ops.PartialSum
     supports_residual = True   # forward(x, residual=h) may add its result to h itself and return None
 
+    def first_product(self):
+        return self.w_gate_up, True                 # its input may come as ops.PendingRows
+
     def forward(self, x: torch.Tensor, partials_ok: bool = False, residual: Optional[torch.Tensor] = None):
         act = ops.linear_silu_mul(x, self.w_gate_up, self.dtype, self.activation, self.limit)
         if residual is not None and ops.linear_into(act, self.w_down, residual):

@@ -20,6 +20,7 @@ class RMSNorm:
 
     accepts_partials = True    # `delta` may be an ops.PartialSum: the kernel adds the k-splits as it reads
     accepts_join = True        # and a PendingNormed with a `join`
+    products_apply_it = True   # a small product may make this norm's output itself (ops.PendingRows)
     center = False             # what a kernel that applies this norm itself needs to know beside weight and eps
 
     def __init__(self, spec: NormSpec, size: int):
