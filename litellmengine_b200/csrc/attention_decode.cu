@@ -295,7 +295,8 @@ static int launch_decode(const bf16* q, const bf16* cache, const int32_t* rows, 
                          const int32_t* token_entry, const int32_t* entry_slot, const int32_t* block_table,
                          int table_stride, float* part_acc, float* part_ml, bf16* out, int n_rows, int nq, int nkv,
                          int page_size, int window, float scale, int num_pages, int num_splits, int32_t* status,
-                         const float* dist_bias, int dist_len, int keep_first, const float* sinks, cudaStream_t s) {
+                         const float* dist_bias, int dist_len, int keep_first, const float* sinks, cudaStream_t s,
+                         const AdMade* mk = nullptr) {
     const size_t smem = static_cast<size_t>(16 + 2 * AD_STAGES * AD_BN) * D * sizeof(bf16);
     const bool ext = dist_bias || (keep_first > 0 && window > 0) || sinks;      // the instantiation that knows them
     auto kern = ext ? paged_decode_attention_kernel<D, AD_STAGES, true> : paged_decode_attention_kernel<D, AD_STAGES, false>;
@@ -309,18 +310,22 @@ static int launch_decode(const bf16* q, const bf16* cache, const int32_t* rows, 
     if (map != nullptr) {
 #define TMA_GO(TS)                                                                                                   \
     {                                                                                                                \
-        const size_t tsmem = static_cast<size_t>(2 * TS * AD_BN + 16) * D * sizeof(bf16) + 1024;                     \
-        auto tk = ext ? paged_decode_attention_tma_kernel<D, TS, true> : paged_decode_attention_tma_kernel<D, TS, false>; \
+        const size_t tsmem = static_cast<size_t>(2 * TS * AD_BN + 16) * D * sizeof(bf16) + 1024 +                    \
+                             (mk && mk->cluster ? static_cast<size_t>(nq / nkv) * (D + 2) * sizeof(float) : 0);      \
+        auto tk = ext ? paged_decode_attention_tma_kernel<D, TS, true, false> : paged_decode_attention_tma_kernel<D, TS, false, false>; \
+        if (mk) tk = paged_decode_attention_tma_kernel<D, TS, false, true>;                                           \
         const cudaError_t te = cudaFuncSetAttribute(tk, cudaFuncAttributeMaxDynamicSharedMemorySize,                 \
                                                     static_cast<int>(tsmem));                                        \
         if (te != cudaSuccess) return static_cast<int>(te);                                                          \
-        launch_pdl(tk, dim3(grid), dim3(AD_THREADS + 32), tsmem, s, *map, q, rows, positions, token_entry, entry_slot, block_table,      \
+        launch_pdl_cluster(tk, dim3(grid), dim3(AD_THREADS + 32), tsmem, s, mk && mk->cluster ? num_splits : 1, *map, q, rows, positions, token_entry, entry_slot, block_table,      \
                                                 table_stride, part_acc, part_ml, out, nq, nkv, page_size, window,    \
                                                 scale * 1.4426950408889634f, num_pages, num_splits, status,          \
-                                                dist_bias, dist_len, keep_first, sinks);               \
+                                                dist_bias, dist_len, keep_first, sinks, mk ? *mk : AdMade{});         \
     }
         TMA_GO(3)                                                   // three tiles in shared memory: one read, two in flight
 #undef TMA_GO
+    } else if (mk) {
+        return LLM_REFUSED_SIZE;                                    // only the kernel whose tiles the copy engine brings makes its rows
     } else {
         launch_pdl(kern, dim3(grid), dim3(AD_THREADS), smem, s, q, cache, rows, positions, token_entry, entry_slot, block_table, table_stride,
                                             part_acc, part_ml, out, nq, nkv, page_size, window,
@@ -328,7 +333,7 @@ static int launch_decode(const bf16* q, const bf16* cache, const int32_t* rows, 
                                             keep_first, sinks);
     }
     int rc = launch_status();
-    if (rc != LLM_OK || num_splits == 1) return rc;
+    if (rc != LLM_OK || num_splits == 1 || (mk && mk->cluster)) return rc;
     dim3 cgrid(n_rows, nq);
     launch_pdl((paged_decode_combine_kernel<D>), cgrid, dim3(D <= 64 ? 64 : 128), 0, s, part_acc, part_ml, rows, out, nq, num_splits,
                sinks);
@@ -380,6 +385,50 @@ extern "C" int llm_paged_attention_decode_ex(
                                  num_splits, status, dist_bias, dist_len, keep_first, sinks, s)
     if (d == 64) GO(64, 3);
     GO(128, 3);
+#undef GO
+}
+
+// Whether `llm_paged_attention_decode_made` takes these: the kernel that makes its queries, keys and values itself.
+extern "C" int llm_paged_decode_made_supported(int d, int group, int page_size) {
+    return llm_paged_decode_supported(d, group) && decode_tma_page_ok(page_size);
+}
+
+// Whether its splits merge in a cluster (2 to 8 of them) instead of by scratch and a second kernel: while seven eighths of the two CTAs
+// an SM hold them all.  A decode step of 8 layers of width 1,024 at a context of 320, merge kernel and cluster (us): 3 requests (96
+// CTAs) 240, 231; 5 (160) 250, 239; 8 (256) 275, 269; 16 (256) 312, 306; but 9 (288) 294, 331 and 12 (288) 304, 344: clusters then wait
+// for room side by side.
+extern "C" int llm_paged_decode_made_cluster(int n_rows, int nkv, int num_splits) {
+    static int sms = 0;
+    int dev = 0;
+    if (!sms && (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)) return 0;
+    return num_splits >= 2 && num_splits <= 8 && 8LL * n_rows * nkv * num_splits <= 14LL * sms ? 1 : 0;
+}
+
+// The attention of a step of single tokens (rows 0 .. n_rows - 1, every key of each) from its projection: qkv float32
+// [parts][n_rows][(nq + 2 nkv) * d] (part_stride apart); norm weights, inv_freq and angles as llm_qk_norm_rope_kv_write takes
+// them (each may be null; a rotation turns whole heads).  Writes the step's keys and values into their pages and out like
+// llm_paged_attention_decode.
+extern "C" int llm_paged_attention_decode_made(
+    const float* qkv, int parts, long long part_stride, const float* q_norm_w, const float* k_norm_w, float eps, const float* inv_freq,
+    const float* angles, void* out, void* cache, int n_rows, const int32_t* positions, const int32_t* token_entry,
+    const int32_t* entry_slot, const int32_t* block_table, int table_stride, int nq, int nkv, int d, int page_size, float scale,
+    int num_pages, int num_splits, float* scratch, int32_t* status, uintptr_t stream) {
+    if (n_rows <= 0) return LLM_OK;
+    if (nq <= 0 || nkv <= 0 || nq % nkv != 0 || num_splits < 1 || num_splits > 65535 || nkv > 65535 || n_rows > 65535 || parts < 1 ||
+        !llm_paged_decode_made_supported(d, nq / nkv, page_size))
+        return LLM_REFUSED_SIZE;
+    if (!aligned16(cache) || !aligned16(qkv) || part_stride % 4 || (angles && !aligned16(angles)) || (num_splits > 1 && !llm_paged_decode_made_cluster(n_rows, nkv, num_splits) && (!scratch || !aligned16(scratch))))
+        return LLM_REFUSED_ALIGN;
+    const AdMade mk = {qkv, q_norm_w, k_norm_w, inv_freq, reinterpret_cast<const float4*>(angles), static_cast<bf16*>(cache), part_stride, parts, eps,
+                       llm_paged_decode_made_cluster(n_rows, nkv, num_splits)};
+    float* part_ml = scratch ? scratch + static_cast<size_t>(n_rows) * nq * num_splits * d : nullptr;
+    cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
+#define GO(DD)                                                                                                                          \
+    return launch_decode<DD, 3>(nullptr, static_cast<const bf16*>(cache), nullptr, positions, token_entry, entry_slot, block_table,      \
+                                table_stride, scratch, part_ml, static_cast<bf16*>(out), n_rows, nq, nkv, page_size, 0, scale,          \
+                                num_pages, num_splits, status, nullptr, 0, 0, nullptr, s, &mk)
+    if (d == 64) GO(64);
+    GO(128);
 #undef GO
 }
 

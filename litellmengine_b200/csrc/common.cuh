@@ -155,6 +155,30 @@ static inline void launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, s
     (void)cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(std::forward<Args>(args))...);
 }
 
+// The same with `cluster` blocks along x a thread-block cluster (1: none).
+template <typename... KArgs, typename... Args>
+static inline void launch_pdl_cluster(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, int cluster,
+                                      Args&&... args) {
+    if (cluster <= 1) {
+        launch_pdl(kernel, grid, block, smem, stream, std::forward<Args>(args)...);
+        return;
+    }
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = cluster;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = pdl_enabled() ? 2 : 1;
+    (void)cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(std::forward<Args>(args))...);
+}
+
 static inline int launch_status() {
     const cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? LLM_OK : static_cast<int>(e);

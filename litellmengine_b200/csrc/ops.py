@@ -1510,6 +1510,54 @@ def paged_attention_decode(q: torch.Tensor, out: torch.Tensor, cache: torch.Tens
     return out
 
 
+def decode_makes_its_rows(qkv, cache: torch.Tensor, d: int, group: int, page_size: int) -> bool:
+    """Whether `paged_attention_decode_made` takes this projection and cache."""
+    t = qkv.parts if isinstance(qkv, PartialSum) else qkv
+    return (t.dtype == torch.float32 and t.is_contiguous() and t.data_ptr() % 16 == 0 and cache.dtype == torch.bfloat16
+            and not (isinstance(qkv, PartialSum) and qkv.rounds_to is not None) and d in (64, 128)
+            and bool(_fn("attention_decode", "llm_paged_decode_made_supported", [c_int, c_int, c_int])(d, group, page_size)))
+
+
+def paged_attention_decode_made(qkv, cache: torch.Tensor, positions, token_entry, entry_slot, block_table: torch.Tensor, q_norm_w, k_norm_w,
+                                eps: float, inv_freq, angles: Optional[torch.Tensor], nq: int, nkv: int, d: int, page_size: int,
+                                scale: float, num_splits: int, status: torch.Tensor) -> torch.Tensor:
+    """`qk_norm_rope_kv_write` and `paged_attention_decode` of a step of single tokens (every row, every key) in one kernel: qkv
+    float32 [T, (nq + 2 nkv) * d] or a `PartialSum` of it, a rotation over whole heads or none.  Returns bfloat16 [T, nq * d]."""
+    parts, part_stride = 1, 0
+    if isinstance(qkv, PartialSum):
+        parts, part_stride = qkv.parts.shape[0], qkv.parts.stride(0)
+        qkv = qkv.parts[0]
+    _dev(qkv, cache, positions, token_entry, entry_slot, block_table, q_norm_w, k_norm_w, inv_freq, angles, status)
+    for t, n in ((positions, "positions"), (token_entry, "token_entry"), (entry_slot, "entry_slot"), (block_table, "block_table")):
+        _i32(t, n)
+    T = qkv.shape[0]
+    if qkv.shape[1] != (nq + 2 * nkv) * d or tuple(cache.shape[1:]) != (2, nkv, page_size, d) or cache.dtype != torch.bfloat16:
+        raise KernelError("qkv must be [T, (heads + 2 kv_heads) * head_dim] and cache bfloat16 [pages, 2, kv_heads, page_size, head_dim]")
+    for w in (q_norm_w, k_norm_w):
+        if w is not None and (w.dtype != torch.float32 or w.numel() != d):
+            raise KernelError("q/k norm weight must be float32 [head_dim]")
+    if inv_freq is not None and (inv_freq.dtype != torch.float32 or inv_freq.numel() * 2 != d):
+        raise KernelError("inv_freq must be float32 [head_dim / 2]")
+    if angles is not None and (inv_freq is None or angles.dtype != torch.float32 or not angles.is_contiguous()
+                               or tuple(angles.shape) != (T, d // 2, 2)):
+        raise KernelError("angles must be float32 [T, head_dim / 2, 2] from rope_angles")
+    out = torch.empty((T, nq * d), dtype=torch.bfloat16, device=qkv.device)
+    merged = num_splits == 1 or bool(_fn("attention_decode", "llm_paged_decode_made_cluster", [c_int, c_int, c_int])(T, nkv, num_splits))
+    need = 0 if merged else _fn("attention_decode", "llm_paged_decode_scratch_floats", [c_int, c_int, c_int, c_int],
+                                restype=c_longlong)(T, nq, d, num_splits)
+    scratch = decode_scratch(qkv.device, int(need))
+    f = _fn("attention_decode", "llm_paged_attention_decode_made",
+            [c_void_p, c_int, c_longlong, c_void_p, c_void_p, c_float, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p,
+             c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_float, c_int, c_int, c_void_p, c_void_p, c_void_p])
+    _check(f(_ptr(qkv), parts, part_stride, _ptr(q_norm_w), _ptr(k_norm_w), float(eps), _ptr(inv_freq), _ptr(angles), _ptr(out), _ptr(cache), T,
+             _ptr(positions), _ptr(token_entry), _ptr(entry_slot), _ptr(block_table), block_table.shape[1], nq, nkv, d, page_size,
+             float(scale), cache.shape[0], num_splits, _ptr(scratch), _ptr(status), _stream()), "paged_attention_decode_made")
+    if not merged:
+        global launch_count
+        launch_count += 1                         # the merge kernel
+    return out
+
+
 def wide_attention_supported(dk: int, dv: int, group: int) -> bool:
     """Whether the tensor-core kernels for keys and values of any widths take this shape (`wide_attention_*`)."""
     if dk % 8 or dv % 8:     # do not compile them just to hear "no"

@@ -168,6 +168,16 @@ class AttentionMixer:
         if hasattr(self.position, "rotation"):
             # a rotation (or nothing): norms, rotation and cache write in one kernel
             rot = self.position.rotation(b)
+            work = b.preludes.get(AttentionWork.name)
+            if (has_kv and self.dtype == torch.bfloat16 and self.span is None and work is not None and not getattr(b, "any_division", False)
+                    and work.num_decode == b.num_tokens and not work.num_prefill_tiles and (rot is None or rot.rotary_dim == self.d)
+                    and ops.decode_makes_its_rows(qkv, cache, self.d, self.nq // self.nkv, ctx.page_size)):
+                # a step of single tokens: norms, rotation and cache write inside the attention kernel too
+                splits = decode_key_splits(self.device, b.num_tokens, self.nkv, decode_reach(b, None))
+                a = ops.paged_attention_decode_made(
+                    qkv, cache, b.positions, b.token_entry, b.entry_slot, table, qw, kw, eps, rot.inv_freq if rot is not None else None,
+                    rot.angles if rot is not None else None, self.nq, self.nkv, self.d, ctx.page_size, self.scale, splits, ctx.status)
+                return self._out(a, ctx)
             q = ops.qk_norm_rope_kv_write(
                 qkv, cache, b.positions, b.token_entry, b.entry_slot, table, qw, kw, eps,
                 rot.inv_freq if rot is not None else None, rot.rotary_dim if rot is not None else 0,
@@ -183,7 +193,9 @@ class AttentionMixer:
                              k32.reshape(T, self.nkv * self.d).contiguous() if k32 is not None else None, qkv, cache,
                              b.positions, b.token_entry, b.entry_slot, table, self.nq, self.nkv, self.d,
                              ctx.page_size, has_kv, ctx.status, self.dtype)
-        a = attention_over_pages(q, ctx, self.nq, self.nkv, self.d, self.span, self.scale)
+        return self._out(attention_over_pages(q, ctx, self.nq, self.nkv, self.d, self.span, self.scale), ctx)
+
+    def _out(self, a: torch.Tensor, ctx: StageContext):
         # joins the float32 residual; may stay a sum of k-splits if the layer's norm adds them itself
         residual = getattr(ctx, "residual", None)
         if residual is not None and ops.linear_into(a, self.w_o, residual):
