@@ -784,16 +784,18 @@ __global__ void __launch_bounds__(WARPS * 32) delta_scan_kernel(
 //
 //   delta_batch_kernel   a block per (sixteen tokens, head): an image of what all columns of the head share, just as the scan
 //                        wants it in shared memory: planes of p k, p q, s k, of T and B, then p_15 and the mark
-//   delta_scan_mma_kernel  a block per (entry, head, 32 columns), eight warps: 16 columns by 32 rows of the state each.  The
+//   delta_scan_mma_kernel  a block per (entry, head, 16 columns), four warps: 32 rows of the state each.  The
 //                        shares of X and O over the rows go through shared memory; every warp then makes the U of its columns itself.
 //
 // A batch that holds something not finite or very large is marked with its first such token.  The scan makes what is before it as
 // always, with nothing in the place of what follows (a weight of zero times an infinity is NaN), and then walks through the batch
 // token by token for the outputs from the mark on and the state.
-// What bounds it: a batch's chain, 2.2 us, of which 3,700 clocks are 48 small products a warp over the state (1,000), shares and X (700),
-// U (300), the state (600), the outputs of two warps (600) and the waits in between, and 200 what is added for the sums' last bits
-// (split_mma_whole); the tensor pipe is busy for 40 % of the time.  Portions of 284,
-// 567 and 849 tokens, 16 heads of 128 x 128 (us): the scan 160 -> 118, what it shares 24 -> 44 (dot products and the writing of 76 MB).
+// What bounds it: a batch's chain, 1.5 us alone on an SM: 48 small products a warp over the state, shares and X, U, the state, the
+// outputs of two warps and the waits in between.  With 32 columns and eight warps a block, two warps a scheduler, it was 2.2 us
+// (3,700 clocks, 1,000 of them the products over the state, 600 the update, the tensor pipe busy for 40 %); blocks of 16 columns fetch
+// the images twice as often and two of them share an SM without waiting for one another.  Portions of 284,
+// 567 and 849 tokens, 16 heads of 128 x 128: the layer 335 -> 319 us; one portion of 1,000 and one of 1,000 tokens 419 -> 383; the
+// kernels of eight tokens before (us): the scan 160, what it shares 24 (here 44: dot products and the writing of 76 MB).
 // Error against 64 bits (2-norm, outputs and states) from the same unit norms, decays and step sizes: 7.7e-8 and 6.0e-8, the kernels of
 // eight tokens 8.6e-8 and 7.9e-8.  With sums as the tensor cores cut them (split_mma_whole) and dot products in four chains it was
 // 10.4e-8 and 8.6e-8, and the layer 320 us instead of 326.
@@ -1001,9 +1003,9 @@ __global__ void __launch_bounds__(128) delta_batch_kernel(
 }
 
 // grid: entries (longest portion first) x H x column tiles of 32, the tiles fastest.
-#define DX_COLS 32
-#define DX_SMEM (2 * DX_IMAGE + 8 * 4 * 32 * 16)
-__global__ void __launch_bounds__(256, 2) delta_scan_mma_kernel(
+#define DX_COLS 16
+#define DX_SMEM (2 * DX_IMAGE + 4 * 4 * 32 * 16)
+__global__ void __launch_bounds__(128, 2) delta_scan_mma_kernel(
     const DeltaShape s, const float* __restrict__ proj, const unsigned char* __restrict__ images, const float* __restrict__ qn,
     const float* __restrict__ kn, const float* __restrict__ vn, const float* __restrict__ beta, const float* __restrict__ decay,
     float* __restrict__ o, float* __restrict__ state, const int32_t* __restrict__ positions, const int32_t* __restrict__ entry_slot,
@@ -1011,7 +1013,7 @@ __global__ void __launch_bounds__(256, 2) delta_scan_mma_kernel(
     pdl_begin();
     constexpr int D = 128;
     extern __shared__ __align__(16) unsigned char dx_smem[];
-    float4* shares = reinterpret_cast<float4*>(dx_smem + 2 * DX_IMAGE);      // [8 warps][X 2, O 2][32 lanes]
+    float4* shares = reinterpret_cast<float4*>(dx_smem + 2 * DX_IMAGE);      // [4 warps][X 2, O 2][32 lanes]
     __shared__ __align__(8) unsigned long long full[2];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, lg = lane >> 2, lt = lane & 3;
     const int tile = blockIdx.x % tiles, c0 = tile * DX_COLS, h = blockIdx.x / tiles % s.H, kvh = h / (s.H / s.G);
@@ -1029,8 +1031,8 @@ __global__ void __launch_bounds__(256, 2) delta_scan_mma_kernel(
     const int count = entry_q_len[entry];
     if (count <= 0) return;                                     // no copy may be on its way when the block ends
     float* slot = state + entry_slot[entry] * s.slot_stride;
-    // a warp: columns c0 + 16 (warp / 4) .. + 15, rows 32 (warp % 4) .. + 31; tile n, element i: column v0 + 8 (i >> 1), row d0 + 8 n + (i & 1)
-    const int group = warp >> 2, v0 = c0 + 16 * group + lg, dw = 32 * (warp & 3), d0 = dw + 2 * lt;
+    // a warp: all columns, rows 32 warp .. + 31; tile n, element i: column v0 + 8 (i >> 1), row d0 + 8 n + (i & 1)
+    const int v0 = c0 + lg, dw = 32 * warp, d0 = dw + 2 * lt;
     float* my_state = slot + (static_cast<long long>(h) * s.V + v0) * D + d0;
     float S[4][4];
     bool bad_state = false;
@@ -1129,7 +1131,7 @@ __global__ void __launch_bounds__(256, 2) delta_scan_mma_kernel(
         auto over_rows = [&](int which) {            // the four warps' shares, in the same order whoever adds them
             float4 x[4];
 #pragma unroll
-            for (int w = 0; w < 4; ++w) x[w] = shares[((4 * group + w) * 4 + which) * 32 + lane];
+            for (int w = 0; w < 4; ++w) x[w] = shares[(w * 4 + which) * 32 + lane];
             return make_float4((x[0].x + x[1].x) + (x[2].x + x[3].x), (x[0].y + x[1].y) + (x[2].y + x[3].y),
                                (x[0].z + x[1].z) + (x[2].z + x[3].z), (x[0].w + x[1].w) + (x[2].w + x[3].w));
         };
@@ -1175,7 +1177,7 @@ __global__ void __launch_bounds__(256, 2) delta_scan_mma_kernel(
                 }
             }
         }
-        if ((warp & 3) >= 2) {                       // two warps of four make the outputs of their columns, eight tokens each
+        if (warp >= 2) {                             // two warps of the four make the outputs, eight tokens each
             const int u = warp & 1;
             float om[4], os[4];
 #pragma unroll
@@ -1193,7 +1195,7 @@ __global__ void __launch_bounds__(256, 2) delta_scan_mma_kernel(
         }
         if (good < DX_T) {                           // token by token
             __syncthreads();                         // the shares have been read
-            float* sums = reinterpret_cast<float*>(shares);                   // [2][4 row quarters][32 columns]
+            float* sums = reinterpret_cast<float*>(shares);                   // [2][4 row quarters][16 columns]
             for (int t = 0; t < nb; ++t) {
                 const size_t row = row0 + done + t;
                 const float be = beta[row * s.H + h];
@@ -1215,8 +1217,8 @@ __global__ void __launch_bounds__(256, 2) delta_scan_mma_kernel(
                         x1 += __shfl_xor_sync(0xffffffffu, x1, off);
                     }
                     if (lt == 0) {
-                        to[(warp & 3) * DX_COLS + v0 - c0] = x0;
-                        to[(warp & 3) * DX_COLS + v0 - c0 + 8] = x1;
+                        to[warp * DX_COLS + v0 - c0] = x0;
+                        to[warp * DX_COLS + v0 - c0 + 8] = x1;
                     }
                     __syncthreads();
                     x0 = x1 = 0.0f;
@@ -1236,7 +1238,7 @@ __global__ void __launch_bounds__(256, 2) delta_scan_mma_kernel(
                     x1 += S[n][2] * qq[n].x + S[n][3] * qq[n].y;
                 }
                 all_rows(x0, x1, sums + 4 * DX_COLS);
-                if (lt == 0 && (warp & 3) == 0 && t >= good) {
+                if (lt == 0 && warp == 0 && t >= good) {
                     oo[t * o_step] = x0;
                     oo[t * o_step + 8] = x1;
                 }
@@ -1250,7 +1252,7 @@ __global__ void __launch_bounds__(256, 2) delta_scan_mma_kernel(
         *reinterpret_cast<float2*>(my_state + 8 * n) = make_float2(S[n][0], S[n][1]);
         *reinterpret_cast<float2*>(my_state + 8 * D + 8 * n) = make_float2(S[n][2], S[n][3]);
     }
-    dr_keep_inputs<256>(s, proj, slot, positions, row0, count, h, c0, DX_COLS, tile == 0);
+    dr_keep_inputs<128>(s, proj, slot, positions, row0, count, h, c0, DX_COLS, tile == 0);
 }
 
 // A warp per (token, head): o / rms(o) * w * gate * scale.
@@ -1487,14 +1489,16 @@ static int delta_shape(DeltaShape& s, int H, int G, int D, int V, int taps, int 
 //   more: 300 + 1, 16: 123, 117; 1,000 + 1, 16: 266, 225; 1,000 + 2, 8: 250, 198; 1,000, 24: 287, 254; 2,500, 32: 726, 652; 300 + 300, 16:
 //   129, 123; 284 + 567, 16: 182, 165; 260 + 5, 4: 127, 117
 //   portions below 256: 100, 16: 60, 64; 4 x 200, 16: 123, 128; 32 x 64, 16: 259, 276
+// (with blocks of 32 columns; with 16 the layer of one request takes 1,000, 16: 263, 231; 2,500, 16: 605, 524; 2,000, 8: 344, 297; 2,000,
+// 4: 306, 275, and below 256 tokens both are level: the line could lie lower, and one request come here too)
 // So: 256 tokens and more; more than 2,048 columns, or 1,500 where several requests share a step with a portion of 1,000 tokens; two
 // blocks an SM at most.
 extern "C" int llm_delta_image_bytes() { return DX_IMAGE; }
-static bool dx_takes(int H, int D, int V) { return D == 128 && V > 0 && V % DX_COLS == 0 && H > 0 && H <= 65535; }
+static bool dx_takes(int H, int D, int V) { return D == 128 && V > 0 && V % 32 == 0 && H > 0 && H <= 65535; }
 extern "C" int llm_delta_batched(int H, int D, int V, int num_entries, int max_len) {
     const long long columns = static_cast<long long>(num_entries) * H * V;
     const bool enough = columns > 2048 || (columns >= 1500 && num_entries > 1 && max_len >= 1000);
-    return dx_takes(H, D, V) && max_len >= 256 && enough && columns <= 2 * DR_SMS * DX_COLS;
+    return dx_takes(H, D, V) && max_len >= 256 && enough && columns <= 2 * DR_SMS * 32;
 }
 
 // Everything of a step that is not all single tokens.  Scratch (float32): qn, kn [T, G, DP], vn [T, H, VP], beta [T, H],
@@ -1558,16 +1562,17 @@ extern "C" int llm_delta_scan(
     if (images) {
         if (!dx_takes(H, D, V) || !aligned16(images)) return LLM_REFUSED_SIZE;
         static_assert(DX_IMAGE <= DX_ROWS && DX_IMAGE % 16 == 0, "the image takes the vectors' place");
-        constexpr int most = DX_SMEM > DR_ALONE_SMEM ? DX_SMEM : DR_ALONE_SMEM;
         cudaError_t e = cudaFuncSetAttribute(delta_batch_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, DX_BATCH_SMEM);
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(delta_scan_mma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
         if (e != cudaSuccess) return static_cast<int>(e);
         launch_pdl(delta_batch_kernel, dim3(num_tokens / DX_T + num_entries, H), dim3(128), DX_BATCH_SMEM, st, s, qn, kn, vn, beta, decay,
                    static_cast<unsigned char*>(images), entry_q_start, entry_q_len, num_entries);
+        constexpr int most = DX_SMEM > DR_ALONE_SMEM ? DX_SMEM : DR_ALONE_SMEM;
+        e = cudaFuncSetAttribute(delta_scan_mma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+        if (e != cudaSuccess) return static_cast<int>(e);
         const int tiles = V / DX_COLS;
         const long long blocks = static_cast<long long>(num_entries) * H * tiles;
         const bool alone = blocks <= DR_SMS || (blocks <= 2 * DR_SMS && walks * tiles <= static_cast<long long>(DR_SMS) * max_len);
-        launch_pdl(delta_scan_mma_kernel, dim3(static_cast<unsigned>(blocks)), dim3(256), alone ? most : DX_SMEM, st, s, proj,
+        launch_pdl(delta_scan_mma_kernel, dim3(static_cast<unsigned>(blocks)), dim3(128), alone ? most : DX_SMEM, st, s, proj,
                    static_cast<const unsigned char*>(images), qn, kn, vn, beta, decay, o, state, positions, entry_slot, entry_q_start,
                    entry_q_len, num_entries, tiles, status);
     } else {
