@@ -184,13 +184,32 @@ __device__ __forceinline__ int gp_first_row(int row, int T) { return T >= GP_BM 
 // MODE 2: y[T, N] (float32) += x . w^T: the product joins the residual stream where it lies.
 // MODE 3: MODE 1 with the tanh form of gelu in place of silu (an instantiation of its own).
 // MODE 4: the clamped form with `limit` (`clamped_swish`, alpha 1.702, up value plus one).
+// MODE 5 and 6: the rows of w are heads of 128 (queries, keys, values) and the result is attention's: see GpHeads.
 // w_map, w_map2: the same weights read in boxes of 128 and 64 rows (for whole tiles and for halves).
-#define GP_GATED(MODE) ((MODE) == 1 || (MODE) >= 3)
+#define GP_GATED(MODE) ((MODE) == 1 || (MODE) == 3 || (MODE) == 4)
+
+// MODE 5: what rope_cache.cu (and, without biases and temperatures, attention_prepare.cu) does behind a q/k/v product, in the
+// product's epilogue, where a thread has a token's sums: RMS norm of every query and key head, the rotation of its pairs (i, i + 64)
+// (MODE 6: of the first 64 entries' pairs (i, i + 32)), queries in bfloat16 to q_out [T, nq * 128], keys and values to
+// their pages ([pages][2][nkv][page_size][128]).  That kernel reads the float32 product again (71 MB for 2,900 tokens of the 8B layer)
+// and takes 23 to 30 us of the layer's 330; here its work runs under the next tile's products.  A thread holds its token's 64 angles
+// for a unit (asked for before it waits) and a quarter of a head at a time; a warp's head goes through shared memory, so that
+// sixteen lanes write one token's 256 bytes.
+struct GpHeads {
+    const int32_t *positions, *token_entry, *entry_slot, *block_table;
+    const float *q_norm_w, *k_norm_w;     // [128] each, null: no norm
+    const float4* angles;                 // [T][64] (MODE 6: [T][32]) pairs (sin, cos), null: no rotation
+    bf16 *q_out, *cache;
+    int table_stride, nq, nkv, page_size, num_pages;
+    float eps;
+};
+#define GP_HEADS(MODE) ((MODE) == 5 || (MODE) == 6)
+#define GP_TURN(MODE) (GP_HEADS(MODE) ? 8192 : 4096)      // bytes of a warp's block of shared memory for turning its results
 template <int MODE, typename TO>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GP_THREADS, 1) linear_pair_tcgen05_kernel(
     const __grid_constant__ CUtensorMap x_map, const __grid_constant__ CUtensorMap w_map,
     const __grid_constant__ CUtensorMap w_map2, TO* __restrict__ y,
-    int T, int N, int K, int inter, GpPlan plan, int32_t* __restrict__ status, float limit) {
+    int T, int N, int K, int inter, GpPlan plan, int32_t* __restrict__ status, float limit, const GpHeads hd) {
     pdl_invite();
     constexpr int TILE_ELEMS = GP_BM * GP_BK;
     extern __shared__ unsigned char smem_dyn[];
@@ -285,11 +304,114 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GP_THREADS, 1) linea
         const int quarter = warp & 3;                             // the TMEM lanes this warp may touch
         const unsigned lane_addr = static_cast<unsigned>(quarter * 32) << 16;
         const unsigned acc_empty_first = gp_map_to(gp_smem(&acc_empty[0]), 0);
-        float4* turn = reinterpret_cast<float4*>(b_s + GP_STAGES * TILE_ELEMS) + (warp - 2) * (32 * 8);    // [32 rows][8 chunks]
+        float4* turn = reinterpret_cast<float4*>(b_s + GP_STAGES * TILE_ELEMS) + (warp - 2) * (GP_TURN(MODE) / 16);    // [32 rows][8 chunks]
         const int out_n = GP_GATED(MODE) ? inter : N;
         GpUnit u;
         for (int i = 0; gp_unit(plan, i, cluster, clusters, &u); ++i) {
             const int buf = i & 1;
+            if constexpr (GP_HEADS(MODE)) {
+                constexpr int PAIRS = MODE == 5 ? 64 : 32;        // pairs of a head that turn
+                const int mine = u.mt * (2 * GP_BM) + static_cast<int>(rank) * GP_BM;
+                const int tok = gp_first_row(mine, T) + quarter * 32 + lane, cols = GP_BN / u.cut;
+                const bool there = tok >= mine && tok < T;
+                const int head0 = (u.nt * GP_BN + u.part * cols) / 128, heads = min(cols / 128, hd.nq + 2 * hd.nkv - head0);
+                float ang[2 * PAIRS];                             // (sin, cos) of the token's angles
+                if (hd.angles && there && head0 < hd.nq + hd.nkv) {
+#pragma unroll
+                    for (int k = 0; k < PAIRS / 2; ++k) {
+                        const float4 a = hd.angles[static_cast<size_t>(tok) * (PAIRS / 2) + k];
+                        ang[4 * k] = a.x; ang[4 * k + 1] = a.y; ang[4 * k + 2] = a.z; ang[4 * k + 3] = a.w;
+                    }
+                }
+                long long row = -1;                               // the token's place in its page, in elements of the cache
+                if (there && head0 + heads > hd.nq) {
+                    const int pos = hd.positions[tok], slot = hd.entry_slot[hd.token_entry[tok]], logical = pos / hd.page_size;
+                    const int page = pos >= 0 && logical < hd.table_stride ? hd.block_table[static_cast<size_t>(slot) * hd.table_stride + logical] : -1;
+                    if (page < 0 || page >= hd.num_pages) {
+                        if (atomicCAS(status, 0, 3) == 0) status[1] = tok;
+                    } else {
+                        row = (static_cast<long long>(page) * 2 * hd.nkv * hd.page_size + pos % hd.page_size) * 128;
+                    }
+                }
+                if (!__all_sync(0xffffffffu, gp_wait<false>(&acc_full[buf], (i >> 1) & 1, &abort_flag, status))) break;
+                gp_fence_after();
+#pragma unroll 1
+                for (int hh = 0; hh < heads; ++hh) {
+                    const unsigned acc = tmem + lane_addr + buf * GP_BN + hh * 128;
+                    const int head = head0 + hh;
+                    const bool is_q = head < hd.nq, is_v = head >= hd.nq + hd.nkv;
+                    const float* nw = is_v ? nullptr : is_q ? hd.q_norm_w : hd.k_norm_w;
+                    float inv = 1.0f;
+                    if (nw) {
+                        float ss = 0.0f;
+#pragma unroll 1
+                        for (int c = 0; c < 128; c += 32) {
+                            unsigned r[32];
+                            gp_ld32(acc + c, r);
+                            gp_ld_wait();
+#pragma unroll
+                            for (int e = 0; e < 32; ++e) ss += __uint_as_float(r[e]) * __uint_as_float(r[e]);
+                        }
+                        inv = 1.0f / sqrtf(ss / 128.0f + hd.eps);
+                    }
+                    uint4* out = reinterpret_cast<uint4*>(turn);  // [32 rows][16 chunks], XOR-swizzled by the row
+#pragma unroll
+                    for (int j = 0; j < 2; ++j) {                 // columns ca .. + 31 and cb .. + 31, pairs in MODE 5, and with j 0 in MODE 6
+                        constexpr int CA = MODE == 5 ? 32 : 64, CB = MODE == 5 ? 64 : 32;
+                        const int ca = CA * j, cb = ca + CB;
+                        unsigned lo[32], hi[32];
+                        gp_ld32(acc + ca, lo);
+                        gp_ld32(acc + cb, hi);
+                        gp_ld_wait();
+#pragma unroll
+                        for (int e = 0; e < 32; ++e) {
+                            float a = __uint_as_float(lo[e]), b = __uint_as_float(hi[e]);
+                            if (nw) {
+                                a = a * inv * __ldg(nw + ca + e);
+                                b = b * inv * __ldg(nw + cb + e);
+                            }
+                            if ((MODE == 5 || j == 0) && hd.angles && !is_v) {
+                                const int at = MODE == 5 ? 2 * (ca + e) : 2 * e;
+                                const float sn = ang[at], cs = ang[at + 1], x = a;
+                                a = x * cs - b * sn;
+                                b = b * cs + x * sn;
+                            }
+                            lo[e] = __float_as_uint(a);
+                            hi[e] = __float_as_uint(b);
+                        }
+#pragma unroll
+                        for (int k = 0; k < 4; ++k) {
+                            auto pack = [](unsigned x, unsigned y) {
+                                const __nv_bfloat162 p = __floats2bfloat162_rn(__uint_as_float(x), __uint_as_float(y));
+                                return *reinterpret_cast<const unsigned*>(&p);
+                            };
+                            out[lane * 16 + ((ca / 8 + k) ^ (lane & 7))] = make_uint4(pack(lo[8 * k], lo[8 * k + 1]), pack(lo[8 * k + 2], lo[8 * k + 3]),
+                                                                                     pack(lo[8 * k + 4], lo[8 * k + 5]), pack(lo[8 * k + 6], lo[8 * k + 7]));
+                            out[lane * 16 + ((cb / 8 + k) ^ (lane & 7))] = make_uint4(pack(hi[8 * k], hi[8 * k + 1]), pack(hi[8 * k + 2], hi[8 * k + 3]),
+                                                                                     pack(hi[8 * k + 4], hi[8 * k + 5]), pack(hi[8 * k + 6], hi[8 * k + 7]));
+                        }
+                    }
+                    __syncwarp();
+                    // where the token's head goes; -1: nowhere
+                    const long long to = !there ? -1
+                                         : is_q ? (static_cast<long long>(tok) * hd.nq + head) * 128
+                                         : row < 0 ? -1
+                                                   : row + static_cast<long long>(is_v ? hd.nkv + head - hd.nq - hd.nkv : head - hd.nq) * hd.page_size * 128;
+                    bf16* base = is_q ? hd.q_out : hd.cache;
+#pragma unroll
+                    for (int k = 0; k < 16; ++k) {
+                        const int rl = 2 * k + (lane >> 4), q = lane & 15;
+                        const long long at = __shfl_sync(0xffffffffu, to, rl);
+                        const uint4 val = out[rl * 16 + (q ^ (rl & 7))];
+                        if (at >= 0) *reinterpret_cast<uint4*>(base + at + q * 8) = val;
+                    }
+                    __syncwarp();
+                }
+                gp_fence_before();
+                __syncwarp();
+                if (lane == 0) gp_arrive_cluster(acc_empty_first + buf * 8);
+                continue;
+            }
             if (!gp_wait<false>(&acc_full[buf], (i >> 1) & 1, &abort_flag, status)) break;
             gp_fence_after();
             const int mine = u.mt * (2 * GP_BM) + static_cast<int>(rank) * GP_BM;      // the first token this CTA writes
@@ -446,7 +568,7 @@ extern "C" int llm_linear_pair_efficiency(int T, int N, int K, int gate_up) {
 
 template <int MODE, typename TO>
 static int gp_launch(const bf16* x, const bf16* w, void* y, int T, int N, int K, int inter, long long w_rows, int32_t* status,
-                     cudaStream_t s, float limit = 0.0f) {
+                     cudaStream_t s, float limit = 0.0f, const GpHeads& hd = {}) {
     CUtensorMap x_map, w_map, w_map2;
     if (!gp_encode(&x_map, x, T, K, GP_BM) || !gp_encode(&w_map, w, w_rows, K, GP_BN / 2) ||
         !gp_encode(&w_map2, w, w_rows, K, GP_BN / 4))
@@ -457,12 +579,12 @@ static int gp_launch(const bf16* x, const bf16* w, void* y, int T, int N, int K,
     GpPlan plan;
     int clusters;
     gp_make_plan(tiles_m, tiles_n, &plan, &clusters);
-    const size_t smem = static_cast<size_t>(GP_STAGES) * GP_STAGE_BYTES + 4 * 32 * 32 * sizeof(float) + 1024;   // stages, the epilogue's four blocks, alignment
+    const size_t smem = static_cast<size_t>(GP_STAGES) * GP_STAGE_BYTES + 4 * GP_TURN(MODE) + 1024;   // stages, the epilogue's four blocks, alignment
     auto kern = linear_pair_tcgen05_kernel<MODE, TO>;
     const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
     if (e != cudaSuccess) return static_cast<int>(e);
     launch_pdl(kern, dim3(2 * clusters), dim3(GP_THREADS), smem, s, x_map, w_map, w_map2, static_cast<TO*>(y), T, N, K,
-               inter, plan, status, limit);
+               inter, plan, status, limit, hd);
     return launch_status();
 }
 
@@ -500,4 +622,22 @@ extern "C" int llm_linear_pair_silu_mul(const void* x, const void* w, void* y, i
                                   status, reinterpret_cast<cudaStream_t>(stream));
     return gp_launch<1, bf16>(static_cast<const bf16*>(x), static_cast<const bf16*>(w), y, T, inter, K, inter, 2LL * inter, status,
                               reinterpret_cast<cudaStream_t>(stream));
+}
+
+// A q/k/v product whose heads of 128 leave it as attention reads them: x bfloat16 [T, K], w bfloat16 [(nq + 2 nkv) * 128, K]; norm
+// weights float32 [128] or null; angles float32 [T, pairs, 2] (sin, cos) of 64 pairs (i, i + 64) or 32 pairs (i, i + 32), or null; q_out bfloat16 [T, nq * 128], cache bfloat16
+// [num_pages, 2, nkv, page_size, 128].  A token whose page is outside the cache sets status 3, its key and value are left out.
+extern "C" int llm_linear_pair_heads(const void* x, const void* w, int T, int K, const float* q_norm_w, const float* k_norm_w, float eps,
+                                     const float* angles, int pairs, void* q_out, void* cache, const int32_t* positions,
+                                     const int32_t* token_entry, const int32_t* entry_slot, const int32_t* block_table, int table_stride, int nq, int nkv,
+                                     int page_size, int num_pages, int32_t* status, uintptr_t stream) {
+    if (nq <= 0 || nkv <= 0 || page_size <= 0 || (angles && pairs != 64 && pairs != 32) || nq > 65535 || nkv > 65535 || !llm_linear_pair_supported(T, (nq + 2 * nkv) * 128, K)) return LLM_REFUSED_SIZE;
+    if (!aligned16(x) || !aligned16(w) || !aligned16(q_out) || !aligned16(cache) || !aligned16(angles) || status == nullptr) return LLM_REFUSED_ALIGN;
+    if (!gp_ready()) return LLM_REFUSED_SIZE;
+    const GpHeads hd = {positions, token_entry, entry_slot, block_table, q_norm_w, k_norm_w, reinterpret_cast<const float4*>(angles),
+                        static_cast<bf16*>(q_out), static_cast<bf16*>(cache), table_stride, nq, nkv, page_size, num_pages, eps};
+    const int N = (nq + 2 * nkv) * 128;
+    auto go = angles && pairs == 32 ? gp_launch<6, bf16> : gp_launch<5, bf16>;
+    return go(static_cast<const bf16*>(x), static_cast<const bf16*>(w), nullptr, T, N, K, 0, N, status,
+              reinterpret_cast<cudaStream_t>(stream), 0.0f, hd);
 }

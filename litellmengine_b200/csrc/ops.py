@@ -2094,6 +2094,36 @@ def linear_pair_silu_mul(x: torch.Tensor, w_gate_up: torch.Tensor, out: Optional
     return out
 
 
+def linear_pair_heads(x: torch.Tensor, weight: torch.Tensor, cache: torch.Tensor, positions, token_entry, entry_slot, block_table: torch.Tensor,
+                      q_norm_w, k_norm_w, eps: float, angles: Optional[torch.Tensor], nq: int, nkv: int, page_size: int,
+                      status: torch.Tensor) -> torch.Tensor:
+    """`qk_norm_rope_kv_write` of x [T, K] @ weight^T for heads of 128, in the epilogue of the paired product: keys and values go to
+    their pages, the queries come back as bfloat16 [T, nq * 128].  angles: the step's table from `rope_angles`, of 64 pairs (i, i + 64)
+    or 32 pairs (i, i + 32); None: no rotation.
+    `status`: int32 [2] (3: a page outside the cache; 9: a wait that ran out)."""
+    _dev(x, weight, cache, positions, token_entry, entry_slot, block_table, q_norm_w, k_norm_w, angles, status)
+    for t, n in ((positions, "positions"), (token_entry, "token_entry"), (entry_slot, "entry_slot"), (block_table, "block_table")):
+        _i32(t, n)
+    if x.dtype != torch.bfloat16 or weight.dtype != torch.bfloat16 or cache.dtype != torch.bfloat16:
+        raise KernelError("the paired product takes bfloat16 operands")
+    T, K = x.shape
+    if tuple(weight.shape) != ((nq + 2 * nkv) * 128, K) or tuple(cache.shape[1:]) != (2, nkv, page_size, 128):
+        raise KernelError("weight must be [(heads + 2 kv_heads) * 128, K] and cache [pages, 2, kv_heads, page_size, 128]")
+    for w in (q_norm_w, k_norm_w):
+        if w is not None and (w.dtype != torch.float32 or w.numel() != 128):
+            raise KernelError("q/k norm weight must be float32 [128]")
+    if angles is not None and (angles.dtype != torch.float32 or not angles.is_contiguous() or tuple(angles.shape) not in ((T, 64, 2), (T, 32, 2))):
+        raise KernelError("angles must be float32 [T, 64 or 32, 2] from rope_angles")
+    q = torch.empty((T, nq * 128), dtype=torch.bfloat16, device=x.device)
+    f = _fn("gemm_pair_tcgen05", "llm_linear_pair_heads",
+            [c_void_p, c_void_p, c_int, c_int, c_void_p, c_void_p, c_float, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
+             c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p])
+    _check(f(_ptr(x), _ptr(weight), T, K, _ptr(q_norm_w), _ptr(k_norm_w), float(eps), _ptr(angles),
+             angles.shape[1] if angles is not None else 0, _ptr(q), _ptr(cache), _ptr(positions), _ptr(token_entry), _ptr(entry_slot), _ptr(block_table), block_table.shape[1], nq, nkv, page_size, cache.shape[0],
+             _ptr(status), _stream()), "linear_pair_heads")
+    return q
+
+
 _PAIR_POLICY = os.environ.get("LLM_PAIR", "auto")       # auto | all | off: which prompt-portion products take the paired kernel
 PAIR_MIN_ROWS = 129                                      # fewer rows leave the second CTA of a pair idle
 # Thousandths of the clusters' time that a product's tiles must fill for the paired kernel to be taken
@@ -2103,7 +2133,19 @@ PAIR_MIN_ROWS = 129                                      # fewer rows leave the 
 # the library kernel by kernel, but a prefill is power-bound and the clocks settle lower with it: taking
 # the other products too gave 57.6 and 127.1 ms at 4,096 and 8,192 tokens, and adding into the residual
 # 28.9 ms at 2,048.
-_PAIR_NEEDS = {"plain": None, "silu": 850, "into": None}
+_PAIR_NEEDS = {"plain": None, "silu": 850, "into": None, "heads": 750}
+# The q/k/v product with norms, rotation and the cache write in its epilogue saves a kernel that reads the float32 product again.
+# Against the library product and that kernel, cold (us), 6,144 x 4,096: 500 tokens (tiles that fill 0.63 of the time) 40 against 38;
+# 640 (0.81) 41, 42; 900 (0.76) 52, 52; 1,024 (0.86) 52, 54; 2,045 (0.86) 97, 114; 2,900 (0.92) 146, 166; of 4,096 x 1,024: 512
+# (0.86) 18.5, 17.4; 1,024 (0.86) 22.5, 25.6; 8,192 86, 126.
+PAIR_HEADS_MIN_ROWS = 600
+
+
+def heads_product(x: torch.Tensor, weight: torch.Tensor, cache: Optional[torch.Tensor], d: int) -> bool:
+    """Whether `linear_pair_heads` is the faster way for this q/k/v product."""
+    return (d == 128 and isinstance(x, torch.Tensor) and x.shape[0] >= PAIR_HEADS_MIN_ROWS and cache is not None and cache.dtype == torch.bfloat16
+            and cache.is_contiguous() and x.data_ptr() % 16 == 0 and weight.data_ptr() % 16 == 0
+            and _pair_takes(x, weight, weight.shape[0], "heads"))
 
 
 def _pair_takes(x: torch.Tensor, weight: torch.Tensor, n: int, kind: str) -> bool:

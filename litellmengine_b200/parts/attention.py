@@ -157,7 +157,6 @@ class AttentionMixer:
 
     def forward(self, x: torch.Tensor, ctx: StageContext) -> torch.Tensor:
         b = ctx.batch
-        qkv = ops.linear(x, self.w_qkv, out_dtype=torch.float32, partials_ok=True)   # normalised, rotated in 32-bit
         has_kv = self.spec.has_kv and ctx.writes_cache
         if self.spec.has_kv and not ctx.writes_cache:
             raise RuntimeError("a mixer with its own keys and values was given a borrowed cache")
@@ -165,7 +164,16 @@ class AttentionMixer:
         qw = self.q_norm.weight if self.q_norm is not None else None
         kw = self.k_norm.weight if self.k_norm is not None else None
         cache, table = (ctx.cache, ctx.block_table) if has_kv else (None, None)
-        if hasattr(self.position, "rotation"):
+        rotates = hasattr(self.position, "rotation")
+        if rotates and has_kv and self.dtype == torch.bfloat16 and ops.heads_product(x, self.w_qkv, cache, self.d):
+            rot = self.position.rotation(b)
+            if rot is None or (rot.rotary_dim == self.d and rot.angles is not None):
+                # prompt portions: norms, rotation and cache write in the product's epilogue
+                q = ops.linear_pair_heads(x, self.w_qkv, cache, b.positions, b.token_entry, b.entry_slot, table, qw, kw, eps,
+                                          rot.angles if rot is not None else None, self.nq, self.nkv, ctx.page_size, ctx.status)
+                return self._out(attention_over_pages(q, ctx, self.nq, self.nkv, self.d, self.span, self.scale), ctx)
+        qkv = ops.linear(x, self.w_qkv, out_dtype=torch.float32, partials_ok=True)   # normalised, rotated in 32-bit
+        if rotates:
             # a rotation (or nothing): norms, rotation and cache write in one kernel
             rot = self.position.rotation(b)
             work = b.preludes.get(AttentionWork.name)
@@ -410,6 +418,28 @@ class GatedAttentionMixer(BranchMixer):
         n_tiles = 0 if work is None else (work.padded_tiles.shape[0] if padded else work.num_prefill_tiles)
         return decode_key_splits(self.device, n_dec, self.nkv, decode_reach(batch, self.span)) if n_dec and (self._wide or not n_tiles) else 0
 
+    def forward(self, x: torch.Tensor, ctx: StageContext):
+        s, b = self.spec, ctx.batch
+        # prompt portions of a layer whose product is heads and nothing else: norm, rotation and cache write in the product's epilogue
+        turns = self.rotation is None or (not self.rotation[3] and self.rotation[2] == 1.0 and self.rotation[1] in (64, 128))
+        if (turns and ctx.writes_cache and self.dtype == torch.bfloat16 and self.dv == self.d and not s.output_gate and self.biases is None
+                and s.query_temperature is None and (s.qk_norm is None or s.qk_norm_scope == "head")
+                and ops.heads_product(x, self.w_in, ctx.cache, self.d)):
+            angles = None
+            if self.rotation is not None:
+                tables, key = getattr(b, "tables", None), ("half_angles", s.position)
+                angles = tables.get(key) if tables is not None else None
+                if angles is None:
+                    angles = ops.rope_angles(b.positions, self.rotation[0])
+                    if tables is not None:
+                        tables[key] = angles
+            q = ops.linear_pair_heads(x, self.w_in, ctx.cache, b.positions, b.token_entry, b.entry_slot, ctx.block_table, self.q_norm_w, self.k_norm_w,
+                                      s.qk_norm.eps if s.qk_norm is not None else 0.0, angles, self.nq, self.nkv, ctx.page_size, ctx.status)
+            out = torch.empty((x.shape[0], self.out_width), dtype=self.dtype, device=x.device)
+            self._attend(q, None, 0, ctx, out, 0, 1.0)
+            return ops.linear(out, self.w_o, out_dtype=torch.float32, partials_ok=getattr(ctx, "partials_ok", False))
+        return super().forward(x, ctx)
+
     def mix(self, proj, col0, ctx, out, out_col0, out_scale):
         b, s = ctx.batch, self.spec
         if not ctx.writes_cache:
@@ -420,6 +450,11 @@ class GatedAttentionMixer(BranchMixer):
             s.query_temperature, ctx.cache_keys, ctx.cache_values, b.positions, b.token_entry, b.entry_slot,
             ctx.block_table, self.nq, self.nkv, self.d, self.dv, ctx.page_size, ctx.status, self.dtype,
             rotation=self.rotation)
+        self._attend(q, proj, col0, ctx, out, out_col0, out_scale)
+
+    def _attend(self, q, proj, col0, ctx, out, out_col0, out_scale):
+        """Attention of the prepared queries over the pages; `proj`: where the output gate's columns are, for layers with one."""
+        b, s = ctx.batch, self.spec
         if self._tuned and ctx.cache is not None and b.preludes.get(AttentionWork.name) is not None:
             # without a gate, a scale or a column offset the kernels write where the output product reads
             direct = (not s.output_gate and out_col0 == 0 and out_scale == 1.0 and out.is_contiguous()
