@@ -185,6 +185,7 @@ __device__ __forceinline__ int gp_first_row(int row, int T) { return T >= GP_BM 
 // MODE 3: MODE 1 with the tanh form of gelu in place of silu (an instantiation of its own).
 // MODE 4: the clamped form with `limit` (`clamped_swish`, alpha 1.702, up value plus one).
 // MODE 5 and 6: the rows of w are heads of 128 (queries, keys, values) and the result is attention's: see GpHeads.
+// MODE 7: MODE 0 for latent attention's queries: heads of 128 entries and 64 whose neighbouring pairs turn (angles [T][32] in GpHeads).
 // w_map, w_map2: the same weights read in boxes of 128 and 64 rows (for whole tiles and for halves).
 #define GP_GATED(MODE) ((MODE) == 1 || (MODE) == 3 || (MODE) == 4)
 
@@ -203,6 +204,7 @@ struct GpHeads {
     int table_stride, nq, nkv, page_size, num_pages;
     float eps;
 };
+#define GP_LATENT 192             // entries of a head in MODE 7
 #define GP_HEADS(MODE) ((MODE) == 5 || (MODE) == 6)
 #define GP_TURN(MODE) (GP_HEADS(MODE) ? 8192 : 4096)      // bytes of a warp's block of shared memory for turning its results
 template <int MODE, typename TO>
@@ -451,6 +453,21 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GP_THREADS, 1) linea
                     gp_ld_wait();
 #pragma unroll
                     for (int e = 0; e < 32; ++e) v[e] = __uint_as_float(r[e]);
+                    if constexpr (MODE == 7) {                    // a third of the chunks: 16 pairs, a line of the step's table a token
+                        const int off = (f0 + c) % GP_LATENT, tok = tok0 + lane;
+                        if (hd.angles && off >= 128 && tok >= mine && tok < T) {
+                            const float4* a = hd.angles + static_cast<size_t>(tok) * 16 + (off - 128) / 4;
+#pragma unroll
+                            for (int k = 0; k < 8; ++k) {
+                                const float4 sc = a[k];
+                                const float x0 = v[4 * k], y0 = v[4 * k + 1], x1 = v[4 * k + 2], y1 = v[4 * k + 3];
+                                v[4 * k] = x0 * sc.y - y0 * sc.x;
+                                v[4 * k + 1] = y0 * sc.y + x0 * sc.x;
+                                v[4 * k + 2] = x1 * sc.w - y1 * sc.z;
+                                v[4 * k + 3] = y1 * sc.w + x1 * sc.z;
+                            }
+                        }
+                    }
                 }
 #pragma unroll
                 for (int j = 0; j < 8; ++j)
@@ -640,4 +657,18 @@ extern "C" int llm_linear_pair_heads(const void* x, const void* w, int T, int K,
     auto go = angles && pairs == 32 ? gp_launch<6, bf16> : gp_launch<5, bf16>;
     return go(static_cast<const bf16*>(x), static_cast<const bf16*>(w), nullptr, T, N, K, 0, N, status,
               reinterpret_cast<cudaStream_t>(stream), 0.0f, hd);
+}
+
+// Latent attention's queries, x bfloat16 [T, K] . w bfloat16 [H * 192, K] -> y bfloat16 [T, H * 192]: the last 64 entries of a head turn in
+// pairs of neighbours by angles float32 [T, 32, 2] (sin, cos), null: not at all.  In float32 until they are stored, as latent_q_pack has them.
+extern "C" int llm_linear_pair_latent_q(const void* x, const void* w, void* y, int T, int H, int K, const float* angles, int32_t* status,
+                                        uintptr_t stream) {
+    if (H <= 0 || H > (1 << 20) || !llm_linear_pair_supported(T, H * GP_LATENT, K)) return LLM_REFUSED_SIZE;
+    if (!aligned16(x) || !aligned16(w) || !aligned16(y) || !aligned16(angles) || status == nullptr) return LLM_REFUSED_ALIGN;
+    if (!gp_ready()) return LLM_REFUSED_SIZE;
+    GpHeads hd = {};
+    hd.angles = reinterpret_cast<const float4*>(angles);
+    const int N = H * GP_LATENT;
+    return gp_launch<7, bf16>(static_cast<const bf16*>(x), static_cast<const bf16*>(w), y, T, N, K, 0, N, status,
+                              reinterpret_cast<cudaStream_t>(stream), 0.0f, hd);
 }

@@ -2125,6 +2125,21 @@ def linear_pair_heads(x: torch.Tensor, weight: torch.Tensor, cache: torch.Tensor
     return q
 
 
+def linear_pair_latent_q(x: torch.Tensor, weight: torch.Tensor, angles: Optional[torch.Tensor], H: int) -> torch.Tensor:
+    """`latent_q_pack` of x [T, K] @ weight^T for heads of 128 + 64 whose 64 turn in neighbouring pairs, in the epilogue of the paired
+    product.  angles: float32 [T, 32, 2] from `rope_angles`, None: no rotation.  Returns bfloat16 [T, H * 192]."""
+    _dev(x, weight, angles)
+    T, K = x.shape
+    if x.dtype != torch.bfloat16 or weight.dtype != torch.bfloat16 or tuple(weight.shape) != (H * 192, K):
+        raise KernelError("the paired product takes bfloat16 operands, a weight of [heads * 192, K]")
+    if angles is not None and (angles.dtype != torch.float32 or tuple(angles.shape) != (T, 32, 2)):
+        raise KernelError("angles must be float32 [T, 32, 2] from rope_angles")
+    out = torch.empty((T, H * 192), dtype=torch.bfloat16, device=x.device)
+    f = _fn("gemm_pair_tcgen05", "llm_linear_pair_latent_q", [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p])
+    _check(f(_ptr(x), _ptr(weight), _ptr(out), T, H, K, _ptr(angles), _ptr(stream_status(x.device)), _stream()), "linear_pair_latent_q")
+    return out
+
+
 _PAIR_POLICY = os.environ.get("LLM_PAIR", "auto")       # auto | all | off: which prompt-portion products take the paired kernel
 PAIR_MIN_ROWS = 129                                      # fewer rows leave the second CTA of a pair idle
 # Thousandths of the clusters' time that a product's tiles must fill for the paired kernel to be taken
@@ -2161,6 +2176,12 @@ def _pair_takes(x: torch.Tensor, weight: torch.Tensor, n: int, kind: str) -> boo
         return False
     need = _PAIR_NEEDS[kind]
     return _PAIR_POLICY == "all" or (need is not None and eff >= need)
+
+
+def latent_q_product(x: torch.Tensor, weight: torch.Tensor) -> bool:
+    """Whether `linear_pair_latent_q` is the faster way for these queries (the rule of the q/k/v product)."""
+    return (x.shape[0] >= PAIR_HEADS_MIN_ROWS and x.data_ptr() % 16 == 0 and weight.data_ptr() % 16 == 0
+            and _pair_takes(x, weight, weight.shape[0], "heads"))
 
 
 def linear_into(x: torch.Tensor, weight: torch.Tensor, residual: torch.Tensor) -> bool:

@@ -230,16 +230,29 @@ class LatentAttentionMixer:
             ops.gate_mul(heads, gates, off, heads, 0, self.spec.output_gate, per_head=self.V if self.gate_per_head else 0)
         return heads
 
+    def _angles(self, b) -> Optional[torch.Tensor]:
+        """The step's table of angles, shared by all layers of the same rotation."""
+        if not self.rot_dims:
+            return None
+        tables, key = getattr(b, "tables", None), ("latent_angles", self.spec.position, self.P)
+        got = tables.get(key) if tables is not None else None
+        if got is None:
+            got = ops.rope_angles(b.positions, self.inv_freq)
+            if tables is not None:
+                tables[key] = got
+        return got
+
     def _portions(self, q: torch.Tensor, proj: torch.Tensor, work: LatentWork.Views, ctx: StageContext) -> torch.Tensor:
         """[T, H * V] whose rows that belong to segments hold their attention over per-head keys and values (a gate per head is
-        applied as the kernel stores)."""
+        applied as the kernel stores).  q: float32, or packed already (bfloat16)."""
         b, s = ctx.batch, self.spec
         H, D, P, R, V, T = self.H, self.D, self.P, self.R, self.V, q.shape[0]
         heads = torch.empty((T, H * V), dtype=self.dtype, device=q.device)
         rows = ops.latent_gather(ctx.cache_keys, work.segs, work.num_segs, work.gathered, work.longest, b.entry_slot, b.entry_kv_len,
                                  ctx.block_table, ctx.page_size, ctx.status)
         kv = torch.mm(rows[:, :R], self._expand[0].t())
-        packed = ops.latent_q_pack(q, b.positions, self.inv_freq, H, D, P, self.rot_dims, rot_pairs=self.rot_pairs, rot_mag=self.rot_mag)
+        packed = q if q.dtype == torch.bfloat16 else ops.latent_q_pack(q, b.positions, self.inv_freq, H, D, P, self.rot_dims,
+                                                                       rot_pairs=self.rot_pairs, rot_mag=self.rot_mag)
         ops.latent_prefill(packed, kv, rows, heads, work.tiles, work.num_tiles, work.segs, b.entry_q_start, b.entry_q_len,
                            b.entry_kv_len, H, R, s.window, self.scale, ctx.status, gate=proj if self.gate_per_head else None,
                            gate_off=self.g_off)
@@ -266,14 +279,22 @@ class LatentAttentionMixer:
         cq = ops.latent_prepare(proj, self.dq_off, self.dkv_off, self.Q, R, P, self.rot_dims, self.wq_norm, self.wkv_norm,
                                 self.eps, self.inv_freq, ctx.cache_keys if s.has_kv else None, b, ctx.block_table,
                                 ctx.page_size, ctx.status, self.dtype, rot_pairs=self.rot_pairs, rot_mag=self.rot_mag)
-        q = ops.as_tensor(ops.linear(cq, self.w_uq, out_dtype=torch.float32))
+        q = None
         work = b.preludes.get(self._work.name) if self._expand is not None and not getattr(b, "any_division", False) else None
         heads = None
         if work is not None and work.num_tiles and 2 * work.gathered * H * (D + V) <= self.EXPANDED_BYTES:
             try:
-                heads = self._expanded(q, proj, work, ctx)
+                if (not work.num_rest and (not self.rot_dims or (self.rot_pairs and self.rot_mag == 1.0 and self.rot_dims == P))
+                        and ops.latent_q_product(cq, self.w_uq)):
+                    # every token belongs to a portion: the queries leave their product as the attention kernel reads them
+                    heads = self._portions(ops.linear_pair_latent_q(cq, self.w_uq, self._angles(b), H), proj, work, ctx)
+                else:
+                    q = ops.as_tensor(ops.linear(cq, self.w_uq, out_dtype=torch.float32))
+                    heads = self._expanded(q, proj, work, ctx)
             except torch.cuda.OutOfMemoryError:
                 pass                                  # what it holds grows with the cached rows; the other path's does not
         if heads is None:
+            if q is None:
+                q = ops.as_tensor(ops.linear(cq, self.w_uq, out_dtype=torch.float32))
             heads = self._gated(self._absorbed(q, b.positions, b.token_entry, ctx), proj, self.g_off)
         return ops.linear(heads, self.w_o, out_dtype=torch.float32, partials_ok=getattr(ctx, "partials_ok", False))

@@ -67,3 +67,26 @@ def test_which_products_come_here():
     takes = lambda T, **k: ops.heads_product(bf(T, 4096), k.get("w", w), k.get("cache", cache), k.get("d", 128))
     assert takes(640) and takes(2900) and not takes(500) and not takes(128) and not takes(599)
     assert not takes(2900, d=64) and not takes(2900, cache=cache.float()) and not takes(2900, w=w.float()) and not takes(2900, cache=None)
+
+
+@pytest.mark.parametrize("H,K", [(1, 64), (3, 200), (8, 136), (11, 64)])
+@pytest.mark.parametrize("turned", [False, True])
+def test_latent_queries_like_the_kernel_behind_the_product(H, K, turned):
+    from litellmengine_b200.csrc import ops
+    g = torch.Generator(device=DEV).manual_seed(H + K)
+    w = (torch.randn(H * 192, K, generator=g, device=DEV) * K ** -0.5).to(torch.bfloat16)
+    inv = 10000.0 ** (-torch.arange(32, device=DEV) / 32.0)
+    for T in (1, 128, 129, 255, 257, 700):
+        x = torch.randn(T, K, generator=g, device=DEV).to(torch.bfloat16)
+        pos = torch.randint(0, 40000, (T,), generator=g, device=DEV, dtype=torch.int32)
+        angles = ops.rope_angles(pos, inv) if turned else None
+        want = ops.latent_q_pack(ops.linear_pair(x, w, torch.float32), pos, inv, H, 128, 64, 64 if turned else 0, rot_pairs=True)
+        got = ops.linear_pair_latent_q(x, w, angles, H)
+        if not turned:
+            assert torch.equal(got, want), T
+        else:                                                    # as above: which product of a turned entry is rounded first
+            off = 2.0 ** -21 * float(want.abs().max())
+            assert bool(((got.float() - want.float()).abs() <= 2.0 ** -7 * want.float().abs() + off).all()), T
+            assert float((got != want).float().mean()) < 0.01
+            assert torch.equal(got.view(T, H, 192)[..., :128], want.view(T, H, 192)[..., :128])
+    assert ops.stream_status(torch.device(DEV)).tolist() == [0, 0]
