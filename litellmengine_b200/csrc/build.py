@@ -48,6 +48,7 @@ FAMILIES: Dict[str, List[str]] = {
     "gemm_skinny": ["gemm_skinny.cu"],
     "gemm_small": ["gemm_small.cu"],
     "gemm_pair_tcgen05": ["gemm_pair_tcgen05.cu"],
+    "gemm_mid_tcgen05": ["gemm_mid_tcgen05.cu"],
     "gemm_f32": ["gemm_f32.cu"],
     "gemm_f32_tcgen05": ["gemm_f32_tcgen05.cu"],
     "host_core": ["host_core.cpp"],            # the host side's bookkeeping: plain C++, no device code

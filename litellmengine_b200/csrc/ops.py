@@ -2035,11 +2035,55 @@ def linear_small(x, weight: torch.Tensor, out_dtype: torch.dtype, activation: Op
     return out
 
 
+# Rows that take `linear_mid`.  Up to 32 it was faster than the library product (below them `linear_skinny` is) at every size tried
+# from 1,024 x 3,072 to 151,936 x 2,048 (4,096 x 2,048 at 32 rows: 6.3 us against 6.2) and than `linear_skinny` where that took so many
+# (2,048 x 6,144: 7.7 against 9.6).  With up to 48 rows the parts' sums weigh more: wide products of a short K stay with the library
+# (40 rows, 4,096 x 2,048: 6.7, 6.3; 5,120 x 2,048: 7.3, 6.8) unless they need no parts (52,224 x 2,048: 40.5, 41.8).
+MID_ROWS = range(SKINNY_MAX_ROWS + 1, 49)
+_mid_products: Dict[tuple, bool] = {}
+
+
+def mid_product(x, weight: torch.Tensor, out_dtype: torch.dtype, gated: bool = False) -> bool:
+    """Whether `linear_mid` is the faster way for these operands (gated: weight is [gate; up])."""
+    if not (x.shape[0] in MID_ROWS and x.is_cuda and x.dtype == torch.bfloat16 and weight.dtype == torch.bfloat16
+            and out_dtype in (torch.float32, torch.bfloat16) and x.is_contiguous() and weight.is_contiguous()
+            and x.shape[1] == weight.shape[1] and x.data_ptr() % 16 == 0 and weight.data_ptr() % 16 == 0):
+        return False
+    n, k = weight.shape
+    key = (x.shape[0] <= 32, n, k, gated)
+    got = _mid_products.get(key)
+    if got is None:
+        got = not gated or n % 2 == 0
+        n = n // 2 if gated else n
+        got = got and bool(_fn("gemm_mid_tcgen05", "llm_linear_mid_supported", [c_int] * 4)(x.shape[0], n, k, int(gated)))
+        if got and x.shape[0] > 32 and not gated:
+            got = k >= min(n, 4096) or _fn("gemm_mid_tcgen05", "llm_linear_mid_parts", [c_int] * 3)(n, k, 0) == 1
+        _mid_products[key] = got
+    return got
+
+
+def linear_mid(x: torch.Tensor, weight: torch.Tensor, out_dtype: torch.dtype, activation: Optional[str] = None, limit: float = 0.0) -> torch.Tensor:
+    """x [M <= 48, K] @ weight^T, bfloat16, streaming the weights once through the tensor cores; with `activation`, weight is
+    [gate; up] and the result act(gate) * up in bfloat16, both rounded to bfloat16 first."""
+    _dev(x, weight)
+    M, K = x.shape
+    gated = activation is not None
+    n = weight.shape[0] // (2 if gated else 1)
+    if weight.shape[1] != K or x.dtype != torch.bfloat16 or weight.dtype != torch.bfloat16 or not x.is_contiguous() or not weight.is_contiguous():
+        raise KernelError("the streaming product takes contiguous bfloat16 operands that agree on K")
+    out = torch.empty((M, n), dtype=torch.bfloat16 if gated else out_dtype, device=weight.device)
+    f = _fn("gemm_mid_tcgen05", "llm_linear_mid",
+            [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_float, c_int, c_int, c_int, c_void_p, c_void_p])
+    _check(f(_ptr(x), _ptr(weight), _ptr(out), _dt(out), int(gated), ACTIVATIONS[activation] if gated else 0, float(limit), M, n, K,
+             _ptr(stream_status(weight.device)), _stream()), "linear_mid")
+    return out
+
+
 _stream_status: Dict[str, torch.Tensor] = {}
 
 
 def stream_status(device) -> torch.Tensor:
-    """The status word of the engine's matrix products and of the delta rule (code 8: a bounded wait of the weight-streaming
+    """The status word of the engine's matrix products and of the delta rule (code 8: a bounded wait of a weight-streaming
     product ran out; 9: of the paired or the float32 tcgen05 product; 11: of the delta rule's tensor-core scan)."""
     key = str(device)
     t = _stream_status.get(key)
@@ -2201,6 +2245,8 @@ def linear_silu_mul(x: torch.Tensor, w_gate_up: torch.Tensor, out_dtype: torch.d
     if out_dtype == torch.bfloat16 and (isinstance(x, PendingRows) or (x.dtype == torch.bfloat16 and x.is_contiguous() and x.data_ptr() % 16 == 0
                                                                        and small_product(x.shape[0], w_gate_up, gated=True))):
         return linear_small(x, w_gate_up, out_dtype, activation=activation, limit=limit)
+    if out_dtype == torch.bfloat16 and mid_product(x, w_gate_up, out_dtype, gated=True):
+        return linear_mid(x, w_gate_up, out_dtype, activation=activation, limit=limit)
     if out_dtype == torch.bfloat16 and _pair_takes(x, w_gate_up, w_gate_up.shape[0] // 2, "silu"):
         return linear_pair_silu_mul(x, w_gate_up, activation=activation, limit=limit)
     return silu_and_mul(linear(x, w_gate_up, out_dtype=out_dtype, partials_ok=True), activation=activation, limit=limit)
@@ -2259,11 +2305,12 @@ def linear_f32_tcgen05(x: torch.Tensor, weight: torch.Tensor) -> torch.Tensor:
 def linear(x: torch.Tensor, weight: torch.Tensor, out_dtype: Optional[torch.dtype] = None,
            partials_ok: bool = False):
     """x [T, K] @ weight[N, K]^T.  Up to 16 bfloat16 rows with weights that the SMs hold all at once go to `linear_small` (which also
-    takes `PendingRows`); else up to 16 bfloat16 rows (decode steps; up to 32 for the small products of small models) go through the
+    takes `PendingRows`); else up to 16 bfloat16 rows (decode steps; up to 32 for small products that `linear_mid` does not take) go through the
     engine's own weight-streaming kernel: alone it is level with the library for N = 4096..24576 and
     faster for K = 12288 (32 us against 36) and N = 151936 (203 against 218), and in a step it
     starts fetching weights while the kernel before it drains (a whole decode step of the
-    Qwen3-8B shape at batch 8: 4.35 ms against 4.77 with the library products).  Everything else
+    Qwen3-8B shape at batch 8: 4.35 ms against 4.77 with the library products).  17 to 48 bfloat16 rows: `linear_mid`, by the rule of
+    `mid_product`.  Everything else
     goes through the library matrix product (under `LLM_PAIR=all`, prompt portions take the paired tcgen05
     product `linear_pair`; by default only the gate/up product does, through `linear_silu_mul`) (the reference uses cuBLAS for all its products,
     src/layers/linear.cu:169-215).  bfloat16 operands accumulate in float32; a float32 weight
@@ -2277,6 +2324,8 @@ def linear(x: torch.Tensor, weight: torch.Tensor, out_dtype: Optional[torch.dtyp
     if (x.dtype == torch.bfloat16 and x.is_contiguous() and x.data_ptr() % 16 == 0 and (out_dtype or x.dtype) in (torch.float32, torch.bfloat16)
             and small_product(rows, weight)):
         return linear_small(x, weight, out_dtype or x.dtype)
+    if mid_product(x, weight, out_dtype or x.dtype):
+        return linear_mid(x, weight, out_dtype or x.dtype)
     if (x.dtype == torch.bfloat16 and weight.dtype == torch.bfloat16 and x.shape[1] % 8 == 0 and weight.data_ptr() % 16 == 0
             and rows >= 1 and (rows <= SKINNY_MAX_ROWS
                                or (rows <= SKINNY_SMALL_MAX_ROWS and skinny_small(weight.shape[0], weight.shape[1])))):
