@@ -100,38 +100,70 @@ __global__ void gla_decay_kernel(const float* __restrict__ proj, long long strid
         }
 }
 
+typedef unsigned long long gla_pair;
+__device__ __forceinline__ gla_pair gla_mul2(gla_pair a, gla_pair b) {
+    gla_pair r;
+    asm("mul.rn.f32x2 %0, %1, %2;\n" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ gla_pair gla_fma2(gla_pair a, gla_pair b, gla_pair c) {
+    gla_pair r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;\n" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ gla_pair gla_both(float lo, float hi) {
+    gla_pair r;
+    asm("mov.b64 %0, {%1, %2};\n" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ float2 gla_split(gla_pair a) {
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;\n" : "=f"(r.x), "=f"(r.y) : "l"(a));
+    return r;
+}
+
 // The same where channels come in fours: a thread makes 4 channels x 8 tokens, so that a weight load and two loads of four
 // inputs (kept token-minor in shared memory) feed 32 multiply-adds; one thread a channel needed a shared load for every
 // multiply-add.  The sums run over the rank in the same order.  2,048 tokens x 2,048 channels of rank 64: 71 -> 36 us,
-// 29 with one form of ln(sigmoid(z)) for either sign (the two sides of a branch were both walked).
-__global__ void __launch_bounds__(128) gla_decay_tiled_kernel(const float* __restrict__ proj, long long stride, int a_off, int rank,
+// 29 with one form of ln(sigmoid(z)) for either sign (the two sides of a branch were both walked), 21 with the inputs laid out so that
+// storing them token-minor meets every bank once (32 lanes had met one), without a division per input, and two tokens an instruction;
+// 700 tokens 24 -> 11.  Issue bounds it, and half of what is issued are the exponentials and logarithms of a 2,048 x 2,048 result.
+// Six to eight blocks an SM (fewer registers, weights four at a time) 22 to 26.
+__global__ void __launch_bounds__(128, 5) gla_decay_tiled_kernel(const float* __restrict__ proj, long long stride, int a_off, int rank,
                                                               const float* __restrict__ w2t, const float* __restrict__ b2,
                                                               float inv_tau, float* __restrict__ la, int channels, int num_tokens) {
     pdl_begin();
-    extern __shared__ __align__(16) float a[];      // [rank][GLA_DECAY_TOKENS]
+    extern __shared__ __align__(16) float a[];      // [rank][GLA_DECAY_TOKENS], a row's eights of tokens exchanged by its index
     const int t0 = blockIdx.x * GLA_DECAY_TOKENS;
     const int nt = min(GLA_DECAY_TOKENS, num_tokens - t0);
-    for (int idx = threadIdx.x; idx < GLA_DECAY_TOKENS * rank; idx += blockDim.x) {
-        const int t = idx / rank, j = idx - t * rank;
-        a[j * GLA_DECAY_TOKENS + t] = t < nt ? proj[static_cast<size_t>(t0 + t) * stride + a_off + j] : 0.0f;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, tg = warp * 8;
+    {   // a warp brings eight tokens, four inputs of each at a time: every bank once
+        const int t = tg + (lane >> 2);
+        const float* row = proj + static_cast<size_t>(t0 + min(t, nt - 1)) * stride + a_off;
+#pragma unroll 8
+        for (int j = lane & 3; j < rank; j += 4)
+            a[j * GLA_DECAY_TOKENS + ((warp ^ (j & 3)) << 3) + (lane >> 2)] = t < nt ? row[j] : 0.0f;
     }
     __syncthreads();
-    const int c = blockIdx.y * GLA_DECAY_CHANNELS + (threadIdx.x & 31) * 4, tg = (threadIdx.x >> 5) * 8;
+    const int c = blockIdx.y * GLA_DECAY_CHANNELS + lane * 4;
     if (c >= channels) return;
-    float z[8][4];
+    gla_pair z[4][4];                               // [tokens in twos][channel]
     const float4 bias = b2 ? *reinterpret_cast<const float4*>(b2 + c) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
 #pragma unroll
-    for (int t = 0; t < 8; ++t) { z[t][0] = bias.x; z[t][1] = bias.y; z[t][2] = bias.z; z[t][3] = bias.w; }
+    for (int t = 0; t < 4; ++t) {
+        z[t][0] = gla_both(bias.x, bias.x);
+        z[t][1] = gla_both(bias.y, bias.y);
+        z[t][2] = gla_both(bias.z, bias.z);
+        z[t][3] = gla_both(bias.w, bias.w);
+    }
     auto add = [&](const float4 w, int j) {
-        float x[8];
-        load8(a + j * GLA_DECAY_TOKENS + tg, x);
+        const ulonglong2* at = reinterpret_cast<const ulonglong2*>(a + j * GLA_DECAY_TOKENS + ((warp ^ (j & 3)) << 3));
+        const ulonglong2 lo = at[0], hi = at[1];
+        const gla_pair x[4] = {lo.x, lo.y, hi.x, hi.y}, w2[4] = {gla_both(w.x, w.x), gla_both(w.y, w.y), gla_both(w.z, w.z), gla_both(w.w, w.w)};
 #pragma unroll
-        for (int t = 0; t < 8; ++t) {
-            z[t][0] += w.x * x[t];
-            z[t][1] += w.y * x[t];
-            z[t][2] += w.z * x[t];
-            z[t][3] += w.w * x[t];
-        }
+        for (int t = 0; t < 4; ++t)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) z[t][i] = gla_fma2(w2[i], x[t], z[t][i]);
     };
     int j = 0;
     for (; j + 8 <= rank; j += 8) {
@@ -142,14 +174,15 @@ __global__ void __launch_bounds__(128) gla_decay_tiled_kernel(const float* __res
         for (int u = 0; u < 8; ++u) add(w[u], j + u);
     }
     for (; j < rank; ++j) add(*reinterpret_cast<const float4*>(w2t + static_cast<size_t>(j) * channels + c), j);
+    auto decay = [&](float v) { return expf((fminf(v, 0.0f) - log1pf(expf(-fabsf(v)))) * inv_tau); };
 #pragma unroll
     for (int t = 0; t < 8; ++t)
         if (tg + t < nt) {
             float r[4];
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
-                const float ls = fminf(z[t][i], 0.0f) - log1pf(expf(-fabsf(z[t][i])));
-                r[i] = expf(ls * inv_tau);
+                const float2 two = gla_split(z[t / 2][i]);
+                r[i] = decay(t & 1 ? two.y : two.x);
             }
             *reinterpret_cast<float4*>(la + static_cast<size_t>(t0 + tg + t) * channels + c) = make_float4(r[0], r[1], r[2], r[3]);
         }
@@ -459,27 +492,6 @@ __global__ void __launch_bounds__(MAX_THREADS) gla_scan_kernel(
 //   64 x 128   37, 27;  86, 45;  117, 71       128 x 128   50, 41;  133, 66; 217, 113
 // so 32 columns (blocks of 64 threads) stay with the kernel above, but for the local pass and, at 64 rows, the
 // output pass.
-typedef unsigned long long gla_pair;
-__device__ __forceinline__ gla_pair gla_mul2(gla_pair a, gla_pair b) {
-    gla_pair r;
-    asm("mul.rn.f32x2 %0, %1, %2;\n" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-__device__ __forceinline__ gla_pair gla_fma2(gla_pair a, gla_pair b, gla_pair c) {
-    gla_pair r;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;\n" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-    return r;
-}
-__device__ __forceinline__ gla_pair gla_both(float lo, float hi) {
-    gla_pair r;
-    asm("mov.b64 %0, {%1, %2};\n" : "=l"(r) : "f"(lo), "f"(hi));
-    return r;
-}
-__device__ __forceinline__ float2 gla_split(gla_pair a) {
-    float2 r;
-    asm("mov.b64 {%0, %1}, %2;\n" : "=f"(r.x), "=f"(r.y) : "l"(a));
-    return r;
-}
 
 template <int RR, int MODE, typename TO>
 __global__ void __launch_bounds__(256, 2) gla_scan_tiled_kernel(
