@@ -26,7 +26,7 @@
 // which is the recurrence with its sums regrouped: every factor is a product of decays, none is divided by one.  The
 // vectors p k, p q, s k and the numbers A, B are the same for all columns of a head.
 //
-//   delta_prepare_kernel   a warp per (four tokens, head of q, k or v): convolution, silu, unit norm of q and k; beta
+//   delta_prepare_kernel   (or ..._fours_kernel) a warp per (four tokens, head of q, k or v): convolution, silu, unit norm of q and k; beta
 //   delta_lowrank_kernel   the second halves of both low-rank projections: decays and gates (delta_lowrank_mma_kernel: bfloat16
 //                          weights and ranks above 32, on the tensor cores)
 //   delta_chunk_kernel     a warp per (eight tokens, head): p k, p q, s k, p_7, A and B
@@ -170,6 +170,92 @@ __global__ void delta_prepare_kernel(const DeltaShape s, const float* __restrict
                 const int c = c0 + lane + 32 * i;
                 if (j < nt && c < padded) dst[j * dst_stride + c] = y[j][i];      // behind a head's end: zeros
             }
+    }
+    if (is_v && lane < nt) beta[static_cast<size_t>(t0 + lane) * s.H + head] = dr_sigmoid(proj[(t0 + lane) * s.stride + s.b_off + head]);
+}
+
+// The same for heads of up to 128 channels, up to four taps and rows that can be read sixteen bytes at a time.  A lane takes four
+// neighbouring channels, and all it reads (seven rows, the taps) is on its way before the first use: the kernel above waits for
+// its loads four times in a row, and a block at a portion's start reads the ring or zeros one value after another.  Here rows come from
+// wherever they are: a block whose tokens belong to several portions passes once for each.
+// Latency bounds it (a warp has seven rows to wait for; three blocks of 80 registers an SM).  1,700 tokens of three portions, 16 heads of
+// 128, everything cold: 43 -> 33 us.  Two blocks of 96 registers 38; four 38; rows fetched before the portion is known 37 (spills).
+__global__ void __launch_bounds__(DP_WARPS * 32, 3) delta_prepare_fours_kernel(
+    const DeltaShape s, const float* __restrict__ proj, const float* __restrict__ conv_w, const float* __restrict__ state,
+    const int32_t* __restrict__ positions, const int32_t* __restrict__ token_entry, const int32_t* __restrict__ entry_slot,
+    const int32_t* __restrict__ entry_q_start, float* __restrict__ qn, float* __restrict__ kn, float* __restrict__ vn,
+    float* __restrict__ beta, int num_tokens) {
+    pdl_begin();
+    const int t0 = blockIdx.x * DP_TOKENS, nt = min(DP_TOKENS, num_tokens - t0);
+    const int item = blockIdx.y * DP_WARPS + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (item >= 2 * s.G + s.H) return;
+    const bool is_v = item >= 2 * s.G, is_q = item < s.G;
+    const int head = is_v ? item - 2 * s.G : is_q ? item : item - s.G;
+    const int width = is_v ? s.V : s.D, padded = is_v ? s.VP : s.DP;
+    const int ch0 = is_v ? 2 * s.G * s.D + head * s.V : item * s.D;        // the head's first channel in q | k | v
+    const int C = 2 * s.G * s.D + s.H * s.V;
+    float* dst = (is_v ? vn : is_q ? qn : kn) + (static_cast<size_t>(t0) * (is_v ? s.H : s.G) + head) * padded;
+    const int dst_stride = (is_v ? s.H : s.G) * padded;
+    int last;
+    for (int first = 0; first < nt; first = last) {                         // the block's tokens of one portion
+        const int e = token_entry[t0 + first], begin = entry_q_start[e];
+        for (last = first + 1; last < nt && token_entry[t0 + last] == e;) ++last;
+        const bool within = begin <= t0 - 3 && nt == DP_TOKENS;             // every row is one of this step
+        const int pos0 = within ? 0 : positions[t0 + first] - first - 3;    // the position of row 0, if it is the portion's
+        const float* ring = within ? nullptr : state + entry_slot[e] * s.slot_stride + s.ring_off;
+        for (int c0 = 0; c0 < padded; c0 += 128) {
+            const int c = c0 + 4 * lane, cc = ch0 + min(c, width - 4);      // lanes behind the head's end read its last channels
+            const float4 zero = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            float4 x[DP_TOKENS + 3], w[4];
+#pragma unroll
+            for (int j = 0; j < DP_TOKENS + 3; ++j) {
+                const int t = t0 - 3 + j;
+                if (within || (t >= begin && t < t0 + nt))
+                    x[j] = *reinterpret_cast<const float4*>(proj + t * s.stride + s.q_off + cc);
+                else if (j >= 4 - s.taps && t < begin && pos0 + j >= 0)
+                    x[j] = *reinterpret_cast<const float4*>(ring + static_cast<long long>((pos0 + j) % s.taps) * C + cc);
+                else
+                    x[j] = zero;
+            }
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const float* tap = conv_w + static_cast<size_t>(cc + i) * s.taps;
+                if (s.taps == 4) w[i] = *reinterpret_cast<const float4*>(tap);
+                else w[i] = make_float4(0.0f, s.taps > 2 ? tap[s.taps - 3] : 0.0f, s.taps > 1 ? tap[s.taps - 2] : 0.0f, tap[s.taps - 1]);
+            }
+            float y[DP_TOKENS][4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                auto part = [&](int j) { return i == 0 ? x[j].x : i == 1 ? x[j].y : i == 2 ? x[j].z : x[j].w; };
+#pragma unroll
+                for (int j = 0; j < DP_TOKENS; ++j) {
+                    float acc = 0.0f;               // only taps there are: none times a row that is not finite
+                    if (s.taps > 3) acc = w[i].x * part(j);
+                    if (s.taps > 2) acc = fmaf(w[i].y, part(j + 1), acc);
+                    if (s.taps > 1) acc = fmaf(w[i].z, part(j + 2), acc);
+                    y[j][i] = c < width ? dr_silu(fmaf(w[i].w, part(j + 3), acc)) : 0.0f;
+                }
+            }
+            if (!is_v) {                            // unit vectors; q also times D^-1/2 (the whole head is here)
+                float n[DP_TOKENS];
+#pragma unroll
+                for (int j = 0; j < DP_TOKENS; ++j) n[j] = y[j][0] * y[j][0] + y[j][1] * y[j][1] + y[j][2] * y[j][2] + y[j][3] * y[j][3];
+#pragma unroll
+                for (int m = 16; m > 0; m >>= 1)
+#pragma unroll
+                    for (int j = 0; j < DP_TOKENS; ++j) n[j] += __shfl_xor_sync(0xffffffffu, n[j], m);
+#pragma unroll
+                for (int j = 0; j < DP_TOKENS; ++j) {
+                    const float inv = 1.0f / sqrtf((n[j] + 1e-6f) * (is_q ? static_cast<float>(s.D) : 1.0f));
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) y[j][i] *= inv;
+                }
+            }
+#pragma unroll
+            for (int j = 0; j < DP_TOKENS; ++j)
+                if (j >= first && j < last && c < padded)                   // behind a head's end: zeros
+                    *reinterpret_cast<float4*>(dst + j * dst_stride + c) = make_float4(y[j][0], y[j][1], y[j][2], y[j][3]);
+        }
     }
     if (is_v && lane < nt) beta[static_cast<size_t>(t0 + lane) * s.H + head] = dr_sigmoid(proj[(t0 + lane) * s.stride + s.b_off + head]);
 }
@@ -1524,6 +1610,12 @@ extern "C" int llm_delta_scan(
     if (out_dtype != LLM_DT_F32 && out_dtype != LLM_DT_BF16) return LLM_REFUSED_DTYPE;
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
     const dim3 pgrid((num_tokens + DP_TOKENS - 1) / DP_TOKENS, (2 * G + H + DP_WARPS - 1) / DP_WARPS);
+    const bool fours = s.DP == 128 && taps <= 4 && D % 4 == 0 && V % 4 == 0 && stride % 4 == 0 && q_off % 4 == 0 && slot_stride % 4 == 0 &&
+                       s.ring_off % 4 == 0 && aligned16(proj) && aligned16(conv_w);
+    if (fours) {
+        launch_pdl(delta_prepare_fours_kernel, pgrid, dim3(DP_WARPS * 32), 0, st, s, proj, conv_w, state, positions, token_entry, entry_slot,
+                   entry_q_start, qn, kn, vn, beta, num_tokens);
+    } else {
 #define PREPARE(PER)                                                                                                  \
     launch_pdl((delta_prepare_kernel<PER>), pgrid, dim3(DP_WARPS * 32), 0, st, s, proj, conv_w, state, positions,      \
                token_entry, entry_slot, entry_q_start, qn, kn, vn, beta, num_tokens)
@@ -1534,6 +1626,7 @@ extern "C" int llm_delta_scan(
         default: PREPARE(8); break;
     }
 #undef PREPARE
+    }
     const int da = (H * D + DL_CHANNELS - 1) / DL_CHANNELS, ga = (H * V + DL_CHANNELS - 1) / DL_CHANNELS;
     const dim3 lgrid((num_tokens + DL_TOKENS - 1) / DL_TOKENS, da + ga);
     const size_t lsmem = static_cast<size_t>(DL_PITCH) * (ra > rg ? ra : rg) * sizeof(float);
