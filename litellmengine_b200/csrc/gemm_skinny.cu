@@ -306,7 +306,9 @@ static void skinny_plan(int N, int K, int bk, int* ctas, int* slices, int* per_t
 // library's kernels (6.9 against 5.4 us on 4,096 x 1,024), but inside a step it starts fetching weights
 // while the kernel before it drains and hands its k-splits to the kernel after it (a decode step of the
 // 0.6B shape at batch 32: 1.27 ms against 1.48).  On large products the 32-token tile loses (45.6 against
-// 35.7 us on 24,576 x 4,096) and the library stays.
+// 35.7 us on 24,576 x 4,096) and the library stays.  Contiguous rows of 64 values and more take gemm_mid_tcgen05.cu from 17 rows on
+// (2,048 x 6,144: 7.4 us against 9.6; 5,120 x 2,048: 6.5, 9.7; a step of 8 layers of width 1,024 for 20, 32 requests 429 -> 367,
+// 448 -> 389).
 extern "C" int llm_linear_skinny_small(int N, int K) {
     if (!skinny_device()) return 0;
     int ctas, slices, per_tile;
