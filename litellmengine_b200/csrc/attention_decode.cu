@@ -394,14 +394,16 @@ extern "C" int llm_paged_decode_made_supported(int d, int group, int page_size) 
 }
 
 // Whether its splits merge in a cluster (2 to 8 of them) instead of by scratch and a second kernel: while seven eighths of the two CTAs
-// an SM hold them all.  A decode step of 8 layers of width 1,024 at a context of 320, merge kernel and cluster (us): 3 requests (96
+// an SM hold them all, two thirds where a cluster has more than four (they leave more gaps).  A decode step of 8 layers of width 1,024 at a context of 320, merge kernel and cluster (us): 3 requests (96
 // CTAs) 240, 231; 5 (160) 250, 239; 8 (256) 275, 269; 16 (256) 312, 306; but 9 (288) 294, 331 and 12 (288) 304, 344: clusters then wait
-// for room side by side.
+// for room side by side.  An attention layer of width 4,096: 3 requests at 1,000 in 8 splits (192) 26.6, 26.1; 4 (256) 27.6, 29.3, at 4,096
+// 34.1, 37.3, at 16,000 61.6, 71.8; 8 in 4 splits (256) at 4,096 42.5, 41.7.
 extern "C" int llm_paged_decode_made_cluster(int n_rows, int nkv, int num_splits) {
     static int sms = 0;
     int dev = 0;
     if (!sms && (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)) return 0;
-    return num_splits >= 2 && num_splits <= 8 && 8LL * n_rows * nkv * num_splits <= 14LL * sms ? 1 : 0;
+    const long long ctas = static_cast<long long>(n_rows) * nkv * num_splits;
+    return num_splits >= 2 && num_splits <= 8 && (num_splits <= 4 ? 8 * ctas <= 14LL * sms : 3 * ctas <= 4LL * sms) ? 1 : 0;
 }
 
 // The attention of a step of single tokens (rows 0 .. n_rows - 1, every key of each) from its projection: qkv float32

@@ -1511,8 +1511,14 @@ def paged_attention_decode(q: torch.Tensor, out: torch.Tensor, cache: torch.Tens
     return out
 
 
-def decode_makes_its_rows(qkv, cache: torch.Tensor, d: int, group: int, page_size: int) -> bool:
-    """Whether `paged_attention_decode_made` takes this projection and cache."""
+def decode_makes_its_rows(qkv, cache: torch.Tensor, d: int, group: int, page_size: int, num_splits: int = 1) -> bool:
+    """Whether `paged_attention_decode_made` takes this projection and cache and is the faster way.  Every split of a row adds up its
+    group's partial sums again: with more than four the kernels of their own are as fast (an attention layer of width 4,096,
+    us, made and not: 2 requests at 500 in 6 splits 25.3, 24.8; 5 at 1,000 in 7 28.8, 28.0; 4 at 4,096 in 8 34.1, 34.5; but 8 at 4,096 in
+    4 41.7, 43.2; 16 in 2 63.1, 67.4).  From a product that leaves whole sums it is faster with any number (width 1,024: 1 request at
+    1,000 11.9, 14.1; 6 in 6 splits 16.2, 18.0)."""
+    if isinstance(qkv, PartialSum) and num_splits > 4:
+        return False
     t = qkv.parts if isinstance(qkv, PartialSum) else qkv
     return (t.dtype == torch.float32 and t.is_contiguous() and t.data_ptr() % 16 == 0 and cache.dtype == torch.bfloat16
             and not (isinstance(qkv, PartialSum) and qkv.rounds_to is not None) and d in (64, 128)

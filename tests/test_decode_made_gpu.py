@@ -45,3 +45,6 @@ def test_what_is_not_taken():
     assert not ops.decode_makes_its_rows(qkv, cache, 128, 1, 128) and not ops.decode_makes_its_rows(qkv, cache, 128, 17, 16)
     assert not ops.decode_makes_its_rows(qkv, cache.float(), 128, 1, 16) and not ops.decode_makes_its_rows(qkv, cache, 256, 1, 16)
     assert not ops.decode_makes_its_rows(ops.PartialSum(qkv[None], torch.bfloat16), cache, 128, 1, 16)
+    sums = ops.PartialSum(qkv[None])
+    assert ops.decode_makes_its_rows(sums, cache, 128, 1, 16, 4) and not ops.decode_makes_its_rows(sums, cache, 128, 1, 16, 5)
+    assert ops.decode_makes_its_rows(qkv, cache, 128, 1, 16, 16)
