@@ -306,8 +306,9 @@ static int launch_decode(const bf16* q, const bf16* cache, const int32_t* rows, 
     }
     dim3 grid(num_splits, nkv, n_rows);
     // pages of 8 to 64 tokens are boxes the copy engine fetches; other page sizes go through cp.async
-    const CUtensorMap* map = decode_tma_page_ok(page_size) ? kv_tensor_map(cache, num_pages, nkv, page_size, D) : nullptr;
-    if (map != nullptr) {
+    CUtensorMap map;
+    const bool mapped = decode_tma_page_ok(page_size) && kv_tensor_map(&map, cache, num_pages, nkv, page_size, D);
+    if (mapped) {
 #define TMA_GO(TS)                                                                                                   \
     {                                                                                                                \
         const size_t tsmem = static_cast<size_t>(2 * TS * AD_BN + 16) * D * sizeof(bf16) + 1024 +                    \
@@ -317,7 +318,7 @@ static int launch_decode(const bf16* q, const bf16* cache, const int32_t* rows, 
         const cudaError_t te = cudaFuncSetAttribute(tk, cudaFuncAttributeMaxDynamicSharedMemorySize,                 \
                                                     static_cast<int>(tsmem));                                        \
         if (te != cudaSuccess) return static_cast<int>(te);                                                          \
-        launch_pdl_cluster(tk, dim3(grid), dim3(AD_THREADS + 32), tsmem, s, mk && mk->cluster ? num_splits : 1, *map, q, rows, positions, token_entry, entry_slot, block_table,      \
+        launch_pdl_cluster(tk, dim3(grid), dim3(AD_THREADS + 32), tsmem, s, mk && mk->cluster ? num_splits : 1, map, q, rows, positions, token_entry, entry_slot, block_table,      \
                                                 table_stride, part_acc, part_ml, out, nq, nkv, page_size, window,    \
                                                 scale * 1.4426950408889634f, num_pages, num_splits, status,          \
                                                 dist_bias, dist_len, keep_first, sinks, mk ? *mk : AdMade{});         \
@@ -325,7 +326,7 @@ static int launch_decode(const bf16* q, const bf16* cache, const int32_t* rows, 
         TMA_GO(3)                                                   // three tiles in shared memory: one read, two in flight
 #undef TMA_GO
     } else if (mk) {
-        return LLM_REFUSED_SIZE;                                    // only the kernel whose tiles the copy engine brings makes its rows
+        return LLM_REFUSED_SIZE;                                    // only the kernel whose tiles the copy engine brings makes its rows: the caller has asked
     } else {
         launch_pdl(kern, dim3(grid), dim3(AD_THREADS), smem, s, q, cache, rows, positions, token_entry, entry_slot, block_table, table_stride,
                                             part_acc, part_ml, out, nq, nkv, page_size, window,
@@ -389,8 +390,9 @@ extern "C" int llm_paged_attention_decode_ex(
 }
 
 // Whether `llm_paged_attention_decode_made` takes these: the kernel that makes its queries, keys and values itself.
-extern "C" int llm_paged_decode_made_supported(int d, int group, int page_size) {
-    return llm_paged_decode_supported(d, group) && decode_tma_page_ok(page_size);
+extern "C" int llm_paged_decode_made_supported(const void* cache, int num_pages, int nkv, int d, int group, int page_size) {
+    CUtensorMap map;
+    return llm_paged_decode_supported(d, group) && decode_tma_page_ok(page_size) && kv_tensor_map(&map, cache, num_pages, nkv, page_size, d);
 }
 
 // Whether its splits merge in a cluster (2 to 8 of them) instead of by scratch and a second kernel: while seven eighths of the two CTAs
@@ -417,7 +419,7 @@ extern "C" int llm_paged_attention_decode_made(
     int num_pages, int num_splits, float* scratch, int32_t* status, uintptr_t stream) {
     if (n_rows <= 0) return LLM_OK;
     if (nq <= 0 || nkv <= 0 || nq % nkv != 0 || num_splits < 1 || num_splits > 65535 || nkv > 65535 || n_rows > 65535 || parts < 1 ||
-        !llm_paged_decode_made_supported(d, nq / nkv, page_size))
+        !llm_paged_decode_supported(d, nq / nkv) || !decode_tma_page_ok(page_size))
         return LLM_REFUSED_SIZE;
     if (!aligned16(cache) || !aligned16(qkv) || part_stride % 4 || (angles && !aligned16(angles)) || (num_splits > 1 && !llm_paged_decode_made_cluster(n_rows, nkv, num_splits) && (!scratch || !aligned16(scratch))))
         return LLM_REFUSED_ALIGN;

@@ -499,26 +499,17 @@ __global__ void __launch_bounds__(AD_THREADS + 32) paged_decode_attention_tma_ke
     }
 }
 
-// ---- host side: the tensor map of a stage's cache, made once per (pointer, shape) ----
+// ---- host side ----
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
                                   const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
                                   CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-struct KvMapEntry {
-    const void* ptr;
-    long long rows;
-    int d, page;
-    CUtensorMap map;
-};
-#define KV_MAP_CACHE 512
-static KvMapEntry g_kv_maps[KV_MAP_CACHE];
-static int g_kv_map_count = 0;
 static EncodeTiledFn g_encode_tiled = nullptr;
 static int g_encode_state = 0;       // 0 unknown, 1 available, -1 not available
 
 // The cache of one stage as a 2-D tensor [pages*2*kv_heads*page_size rows, d columns] with boxes of
-// [page_size rows, 64 columns], 128-byte swizzle.  Null if the driver entry point is missing or refuses.
-static const CUtensorMap* kv_tensor_map(const void* cache, int num_pages, int nkv, int page_size, int d) {
+// [page_size rows, 64 columns], 128-byte swizzle.  False if the driver entry point is missing or refuses.  Made for every launch, as
+// the other kernels' maps are: a table of maps by address would fill up in a process that makes many caches.
+static bool kv_tensor_map(CUtensorMap* map, const void* cache, int num_pages, int nkv, int page_size, int d) {
     if (g_encode_state == 0) {
         void* fn = nullptr;
         cudaDriverEntryPointQueryResult qres;
@@ -531,27 +522,15 @@ static const CUtensorMap* kv_tensor_map(const void* cache, int num_pages, int nk
             g_encode_state = -1;
         }
     }
-    if (g_encode_state < 0) return nullptr;
     const long long rows = static_cast<long long>(num_pages) * 2 * nkv * page_size;
-    for (int i = 0; i < g_kv_map_count; ++i)
-        if (g_kv_maps[i].ptr == cache && g_kv_maps[i].rows == rows && g_kv_maps[i].d == d && g_kv_maps[i].page == page_size)
-            return &g_kv_maps[i].map;
-    if (g_kv_map_count >= KV_MAP_CACHE || rows >= (1LL << 31)) return nullptr;
-    KvMapEntry& e = g_kv_maps[g_kv_map_count];
+    if (g_encode_state < 0 || rows >= (1LL << 31)) return false;
     const cuuint64_t dims[2] = {static_cast<cuuint64_t>(d), static_cast<cuuint64_t>(rows)};
     const cuuint64_t strides[1] = {static_cast<cuuint64_t>(d) * sizeof(bf16)};
     const cuuint32_t box[2] = {64u, static_cast<cuuint32_t>(page_size)};
     const cuuint32_t estr[2] = {1u, 1u};
-    const CUresult rc = g_encode_tiled(&e.map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(cache), dims, strides,
-                                       box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-                                       CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (rc != CUDA_SUCCESS) return nullptr;
-    e.ptr = cache;
-    e.rows = rows;
-    e.d = d;
-    e.page = page_size;
-    ++g_kv_map_count;
-    return &e.map;
+    return g_encode_tiled(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(cache), dims, strides, box, estr,
+                          CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                          CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
 static bool decode_tma_page_ok(int page_size) { return page_size == 8 || page_size == 16 || page_size == 32 || page_size == 64; }

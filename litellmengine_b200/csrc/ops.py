@@ -1522,7 +1522,8 @@ def decode_makes_its_rows(qkv, cache: torch.Tensor, d: int, group: int, page_siz
     t = qkv.parts if isinstance(qkv, PartialSum) else qkv
     return (t.dtype == torch.float32 and t.is_contiguous() and t.data_ptr() % 16 == 0 and cache.dtype == torch.bfloat16
             and not (isinstance(qkv, PartialSum) and qkv.rounds_to is not None) and d in (64, 128)
-            and bool(_fn("attention_decode", "llm_paged_decode_made_supported", [c_int, c_int, c_int])(d, group, page_size)))
+            and bool(_fn("attention_decode", "llm_paged_decode_made_supported", [c_void_p, c_int, c_int, c_int, c_int, c_int])(
+                _ptr(cache), cache.shape[0], cache.shape[2], d, group, page_size)))
 
 
 def paged_attention_decode_made(qkv, cache: torch.Tensor, positions, token_entry, entry_slot, block_table: torch.Tensor, q_norm_w, k_norm_w,

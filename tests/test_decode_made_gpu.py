@@ -48,3 +48,25 @@ def test_what_is_not_taken():
     sums = ops.PartialSum(qkv[None])
     assert ops.decode_makes_its_rows(sums, cache, 128, 1, 16, 4) and not ops.decode_makes_its_rows(sums, cache, 128, 1, 16, 5)
     assert ops.decode_makes_its_rows(qkv, cache, 128, 1, 16, 16)
+
+
+def test_many_caches():
+    """A process that makes caches at ever new addresses: what is taken once is taken again."""
+    from litellmengine_b200.csrc import ops
+    nq, nkv, page, d = 4, 2, 8, 64
+    g = torch.Generator(device=DEV).manual_seed(1)
+    caches = torch.randn(700, 1, 2, nkv, page, d, generator=g, device=DEV).to(torch.bfloat16)
+    two = caches.clone()
+    qkv = torch.randn(1, (nq + 2 * nkv) * d, generator=g, device=DEV)
+    pos, zero = torch.tensor([5], dtype=torch.int32, device=DEV), torch.zeros(1, dtype=torch.int32, device=DEV)
+    table, status = torch.zeros(1, 1, dtype=torch.int32, device=DEV), torch.zeros(2, dtype=torch.int32, device=DEV)
+    got = []
+    for c in caches:
+        assert ops.decode_makes_its_rows(qkv, c, d, nq // nkv, page)
+        got.append(ops.paged_attention_decode_made(qkv, c, pos, zero, zero, table, None, None, 1e-6, None, None, nq, nkv, d, page, d ** -0.5, 1, status))
+    for c, a in zip(two, got):
+        q = ops.qk_norm_rope_kv_write(qkv, c, pos, zero, zero, table, None, None, 1e-6, None, 0, nq, nkv, d, page, True, status,
+                                      q_dtype=torch.bfloat16)
+        want = ops.paged_attention_decode(q, torch.empty_like(q), c, None, 1, pos, zero, zero, table, nq, nkv, d, page, None, d ** -0.5, 1, status)
+        assert torch.equal(a, want)
+    assert status.tolist() == [0, 0] and torch.equal(caches, two)
