@@ -19,16 +19,16 @@
 // registers and half the shared memory a CTA, so that the next kernel's CTAs find room while this one's still run (with 8 eights of a row
 // held where 4 do, 267 us for 5 requests instead of 247).
 // Products run on mma.sync m16n8k16 with the weights as the 16-row operand and the tokens as the 8 columns; sums are float32.
-// The wait for the weights is bounded: when it runs out the kernel records status code 8 and goes on (its result is then flagged).
+// The wait for the weights is bounded: a thread whose tries run out records status code 8 and goes on (the result is then flagged), but
+// does not end before the copies have landed, for which it waits, bounded again: the block's memory may be another one's next.
 #include "common.cuh"
 #include <cuda.h>
-#include <unordered_map>
 
 #define GM_ROWS 16          // output features of a CTA
 #define GM_THREADS 256
 #define GM_WARPS 8
 #define GM_SUB 64           // k-values of a piece of weights: 16 rows of 128 bytes, chunks of 16 bytes XOR-swizzled by the row
-#define GM_WAIT_LIMIT 2000000
+#define GM_DRAIN_LIMIT 8000000
 #define GM_HELD 8           // eights of a row that a lane of a norming warp holds at most: rows of up to 2,048
 
 __device__ __forceinline__ unsigned gm_smem(const void* p) { return static_cast<unsigned>(__cvta_generic_to_shared(p)); }
@@ -78,7 +78,7 @@ __host__ __device__ constexpr int gm_first_bytes(int mt, int slabs, int subs) {
 // HELD: eights of a row that a lane of a norming warp holds (4 or 8; 0: the rows are there).
 template <int MT, int HELD, bool GATED, typename TO, bool BOXES>
 __global__ void __launch_bounds__(GM_THREADS, HELD == 8 ? 2 : 3) linear_small_kernel(const GmRows in, const bf16* __restrict__ w_tiled, TO* __restrict__ y,
-                                                                  int M, int N, int K, int act, float limit, int32_t* __restrict__ status,
+                                                                  int M, int N, int K, int act, float limit, int waits, int32_t* __restrict__ status,
                                                                   const __grid_constant__ CUtensorMap w_map) {
     constexpr int SLABS = GM_SLABS(GATED, HELD), PIECE = GM_ROWS * GM_SUB, SUMS = GM_ROWS * MT;
     extern __shared__ __align__(1024) unsigned char smem_raw[];          // the swizzle's pattern repeats every 1024 bytes
@@ -191,15 +191,8 @@ __global__ void __launch_bounds__(GM_THREADS, HELD == 8 ? 2 : 3) linear_small_ke
         asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;\n" ::: "memory");
     }
     __syncthreads();                                                     // the rows are there, and the barrier exists for everyone
-    {
-        int n = 0;
-        while (!gm_try_wait(&full, 0)) {
-            if (++n > GM_WAIT_LIMIT) {
-                if (atomicCAS(status, 0, 8) == 0) status[1] = blockIdx.x;
-                break;
-            }
-        }
-    }
+    bool landed = false;
+    for (int n = 0; n < waits && !landed; ++n) landed = gm_try_wait(&full, 0);
     float acc[SLABS][MT / 8][4], acc2[SLABS][MT / 8][4];                 // over the even and the odd steps of 16 k-values
 #pragma unroll
     for (int z = 0; z < SLABS; ++z)
@@ -248,6 +241,10 @@ __global__ void __launch_bounds__(GM_THREADS, HELD == 8 ? 2 : 3) linear_small_ke
         float out = sum_of(o);
         if constexpr (GATED) out = gm_gated(to_f32(from_f32<bf16>(out)), to_f32(from_f32<bf16>(sum_of(SUMS + o))), act, limit);
         y[static_cast<size_t>(tok) * N + f] = from_f32<TO>(out);
+    }
+    if (!landed) {
+        if (atomicCAS(status, 0, 8) == 0) status[1] = blockIdx.x;
+        for (int n = 0; n < GM_DRAIN_LIMIT && !gm_try_wait(&full, 0); ++n) {}
     }
 }
 
@@ -307,7 +304,7 @@ static bool gm_weight_map(CUtensorMap* map, const void* w, long long rows, int K
 }
 
 template <int MT, int HELD, bool GATED, typename TO, bool BOXES>
-static int gm_launch(const GmRows& in, const void* w, void* y, int M, int N, int K, int act, float limit, int32_t* status, cudaStream_t s) {
+static int gm_launch(const GmRows& in, const void* w, void* y, int M, int N, int K, int act, float limit, int waits, int32_t* status, cudaStream_t s) {
     CUtensorMap map = {};
     if (BOXES && !gm_weight_map(&map, w, static_cast<long long>(N) * (GATED ? 2 : 1), K)) return LLM_REFUSED_ALIGN;
     const size_t smem = static_cast<size_t>(gm_bytes(MT, K, HELD > 0, GATED));
@@ -315,26 +312,27 @@ static int gm_launch(const GmRows& in, const void* w, void* y, int M, int N, int
     const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
     if (e != cudaSuccess) return static_cast<int>(e);
     launch_pdl(kern, dim3(gm_ctas(N, HELD > 0, GATED)), dim3(GM_THREADS), smem, s, in, static_cast<const bf16*>(w), static_cast<TO*>(y), M, N, K,
-               act, limit, status, map);
+               act, limit, waits, status, map);
     return launch_status();
 }
 
 template <int HELD, bool GATED, typename TO>
-static int gm_pick(const GmRows& in, const void* w, int tiled, void* y, int M, int N, int K, int act, float limit, int32_t* status, cudaStream_t s) {
+static int gm_pick(const GmRows& in, const void* w, int tiled, void* y, int M, int N, int K, int act, float limit, int waits, int32_t* status, cudaStream_t s) {
     if (HELD > 0 || M <= 8)
-        return tiled ? gm_launch<8, HELD, GATED, TO, false>(in, w, y, M, N, K, act, limit, status, s)
-                     : gm_launch<8, HELD, GATED, TO, true>(in, w, y, M, N, K, act, limit, status, s);
-    return tiled ? gm_launch<16, 0, GATED, TO, false>(in, w, y, M, N, K, act, limit, status, s)
-                 : gm_launch<16, 0, GATED, TO, true>(in, w, y, M, N, K, act, limit, status, s);
+        return tiled ? gm_launch<8, HELD, GATED, TO, false>(in, w, y, M, N, K, act, limit, waits, status, s)
+                     : gm_launch<8, HELD, GATED, TO, true>(in, w, y, M, N, K, act, limit, waits, status, s);
+    return tiled ? gm_launch<16, 0, GATED, TO, false>(in, w, y, M, N, K, act, limit, waits, status, s)
+                 : gm_launch<16, 0, GATED, TO, true>(in, w, y, M, N, K, act, limit, waits, status, s);
 }
 
 // x: bfloat16 [M, K], or null: then the rows are rmsnorm(h + pending) * g with h, pending float32 [M, K] (pending: null, or
 // pending_parts of them pending_stride apart) and h_out (null, or another buffer than h) = h + pending.  w: bfloat16 [N, K] (gated:
 // [2 N, K] = [gate; up]) as it is, or (`tiled`) in the stored blocks of gemm_skinny.cu.  y: [M, N] float32 or bfloat16; gated:
-// bfloat16, act 0 silu, 1 the tanh form of gelu, 2 the clamped form with `limit`.
+// bfloat16, act 0 silu, 1 the tanh form of gelu, 2 the clamped form with `limit`.  waits: tries of the wait for the weights (each suspends
+// for a while) before a block gives up.
 extern "C" int llm_linear_small(const void* x, const float* h, const float* pending, int pending_parts, long long pending_stride, const float* g,
                                 float eps, float* h_out, const void* w, int tiled, void* y, int out_dtype, int gated, int act, float limit,
-                                int M, int N, int K, int32_t* status, uintptr_t stream) {
+                                int M, int N, int K, int waits, int32_t* status, uintptr_t stream) {
     const int normed = x == nullptr;
     if (!llm_linear_small_supported(M, N, K, normed, gated) || (normed && (!h || !g || (pending && pending_parts < 1) || h_out == h)))
         return LLM_REFUSED_SIZE;
@@ -349,9 +347,9 @@ extern "C" int llm_linear_small(const void* x, const float* h, const float* pend
     in.g = g; in.eps = eps; in.h_out = h_out;
     cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
 #define GO(GATED, TO)                                                                                     \
-    return !normed    ? gm_pick<0, GATED, TO>(in, w, tiled, y, M, N, K, act, limit, status, s)            \
-           : K <= 1024 ? gm_pick<4, GATED, TO>(in, w, tiled, y, M, N, K, act, limit, status, s)           \
-                       : gm_pick<8, GATED, TO>(in, w, tiled, y, M, N, K, act, limit, status, s)
+    return !normed    ? gm_pick<0, GATED, TO>(in, w, tiled, y, M, N, K, act, limit, waits, status, s)            \
+           : K <= 1024 ? gm_pick<4, GATED, TO>(in, w, tiled, y, M, N, K, act, limit, waits, status, s)           \
+                       : gm_pick<8, GATED, TO>(in, w, tiled, y, M, N, K, act, limit, waits, status, s)
     if (gated) GO(true, bf16);
     if (out_dtype == LLM_DT_F32) GO(false, float);
     GO(false, bf16);

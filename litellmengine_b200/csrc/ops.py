@@ -2017,7 +2017,11 @@ def pending_rows(h: torch.Tensor, delta, norm, weight: Optional[torch.Tensor], d
     return PendingRows(h, delta, norm.weight, norm.eps, dtype)
 
 
-def linear_small(x, weight: torch.Tensor, out_dtype: torch.dtype, activation: Optional[str] = None, limit: float = 0.0) -> torch.Tensor:
+STREAM_WAITS = 2_000_000      # tries of a wait for weights before a streaming product gives up and sets `stream_status`
+
+
+def linear_small(x, weight: torch.Tensor, out_dtype: torch.dtype, activation: Optional[str] = None, limit: float = 0.0,
+                 waits: int = STREAM_WAITS) -> torch.Tensor:
     """x [M <= 16, K] (bfloat16, or `PendingRows`) @ weight^T for weights that the SMs hold all at once, no partial sums.  With
     `activation`, weight is [gate; up] and the result act(gate) * up in bfloat16, both rounded to bfloat16 first."""
     made = isinstance(x, PendingRows)
@@ -2034,10 +2038,10 @@ def linear_small(x, weight: torch.Tensor, out_dtype: torch.dtype, activation: Op
     out = torch.empty((M, n), dtype=torch.bfloat16 if gated else out_dtype, device=weight.device)
     f = _fn("gemm_small", "llm_linear_small",
             [c_void_p, c_void_p, c_void_p, c_int, c_longlong, c_void_p, c_float, c_void_p, c_void_p, c_int, c_void_p, c_int, c_int, c_int,
-             c_float, c_int, c_int, c_int, c_void_p, c_void_p])
+             c_float, c_int, c_int, c_int, c_int, c_void_p, c_void_p])
     _check(f(None if made else _ptr(x), _ptr(h), _ptr(pending), parts, stride, _ptr(x.weight) if made else None, x.eps if made else 0.0,
              _ptr(x.stream) if made and pending is not None else None, _ptr(tiled if tiled is not None else weight), int(tiled is not None),
-             _ptr(out), _dt(out), int(gated), ACTIVATIONS[activation] if gated else 0, float(limit), M, n, K,
+             _ptr(out), _dt(out), int(gated), ACTIVATIONS[activation] if gated else 0, float(limit), M, n, K, int(waits),
              _ptr(stream_status(weight.device)), _stream()), "linear_small")
     return out
 

@@ -82,3 +82,29 @@ def test_what_is_not_taken():
     assert o.pending_rows(h, h.to(torch.bfloat16), Norm, w, torch.bfloat16, False) is None
     assert o.pending_rows(h.t().contiguous().t(), None, Norm, w, torch.bfloat16, False) is None
     assert o.pending_rows(h, None, object(), w, torch.bfloat16, False) is None
+
+
+@pytest.mark.parametrize("form", ["rows", "tiled", "normed", "gated"])
+def test_a_wait_that_runs_out(form):
+    """A block that has no tries left for its weights records the status, lets its copies land and ends; the next products are right."""
+    o = ops()
+    g = torch.Generator(device=DEV).manual_seed(5)
+    w = (torch.randn(2048, 1024, generator=g, device=DEV) / 32).to(torch.bfloat16)
+    x, h = torch.randn(5, 1024, generator=g, device=DEV).to(torch.bfloat16), torch.randn(5, 1024, generator=g, device=DEV)
+    if form == "tiled":
+        o._tiled[w.data_ptr()] = o.tile_weight(w)
+    rows = o.PendingRows(h, None, torch.ones(1024, device=DEV), 1e-6, torch.bfloat16) if form == "normed" else x
+    out = dict(out_dtype=torch.bfloat16, activation="silu") if form == "gated" else dict(out_dtype=torch.float32)
+    status = o.stream_status(torch.device(DEV))
+    try:
+        want = o.linear_small(rows, w, **out)
+        assert status.tolist() == [0, 0]
+        o.linear_small(rows, w, waits=0, **out)
+        assert status.tolist()[0] == 8
+        status.zero_()
+        for _ in range(3):
+            assert torch.equal(o.linear_small(rows, w, **out), want)
+        assert status.tolist() == [0, 0]
+    finally:
+        status.zero_()
+        o._tiled.pop(w.data_ptr(), None)
