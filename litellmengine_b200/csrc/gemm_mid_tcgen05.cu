@@ -11,6 +11,8 @@
 //   * The issuing warp walks its stages with all lanes (a wait inside a branch for one lane keeps the tensor pipe idle for 250 clocks).
 //   * Weights come as boxes of the matrix as it is: the stored blocks of gemm_skinny.cu instead were -1.0 to +5 us of 5 to 52.
 // Roles: warp 0 feeds the copy engine, warp 1 issues, warps 2 to 5 take the sums (a thread a feature); all six add the parts.
+// Waits are bounded: one that runs out, in whichever warp, sets status code 8 (the result is then flagged), and the feeding thread waits
+// for its last copies before the CTA ends.
 //
 // Against the library product (gated: and the activation kernel), cold weights, us at 17 / 40 rows; [floor by bytes]:
 //   1,024 x 3,072   3.8, 7.1 / 4.4, 6.6  [1.0]      5,120 x 13,824  25.4, 31.1 / 26.6, 32.5  [21.6]
@@ -27,10 +29,9 @@
 #define GD_THREADS 192
 #define GD_MAX_TOKENS 48
 #define GD_STATUS 8
-#define GD_WAIT_LIMIT 2000000
 
-__device__ __forceinline__ bool gd_wait(unsigned long long* bar, unsigned parity, volatile int* abort_flag, int32_t* status) {
-    for (int i = 0; i < GD_WAIT_LIMIT; ++i) {
+__device__ __forceinline__ bool gd_wait(unsigned long long* bar, unsigned parity, int waits, volatile int* abort_flag, int32_t* status) {
+    for (int i = 0; i < waits; ++i) {
         if (t5_try_wait(bar, parity)) return true;
         if (*abort_flag) return false;
     }
@@ -47,7 +48,7 @@ __device__ __forceinline__ float gd_gated(float g, float u, int act, float limit
 template <int NT, int STAGES, bool GATED, typename TO>
 __global__ void __launch_bounds__(GD_THREADS, 2) linear_mid_kernel(
     const __grid_constant__ CUtensorMap w_map, const __grid_constant__ CUtensorMap x_map, TO* __restrict__ y,
-    int M, int N, int K, int act, float limit, int32_t* __restrict__ status) {
+    int M, int N, int K, int act, float limit, int waits, int32_t* __restrict__ status) {
     constexpr int X_PIECE = NT * GD_K;
     constexpr unsigned W_BYTES = 2 * GD_PIECE * sizeof(bf16), X_BYTES = X_PIECE * sizeof(bf16);
     extern __shared__ unsigned char smem_dyn[];
@@ -78,6 +79,7 @@ __global__ void __launch_bounds__(GD_THREADS, 2) linear_mid_kernel(
     pdl_invite();                                                 // not before: this CTA's tensor memory is taken
     const unsigned tmem = __shfl_sync(0xffffffffu, tmem_base_s, 0);
 
+    int issued = 0;                                               // stages that were asked for, in the thread that asks
     if (warp == 0) {
         if (lane == 0) {
             auto weights = [&](int kb) {                          // both pieces of a stage; the stage is free
@@ -91,16 +93,13 @@ __global__ void __launch_bounds__(GD_THREADS, 2) linear_mid_kernel(
             for (int kb = 0; kb < first; ++kb) weights(kb);       // nobody's output
             pdl_wait();
             for (int kb = 0; kb < first; ++kb) tokens(kb);
-            int issued = first;
+            issued = first;
             for (int kb = STAGES; kb < kbs; ++kb) {
-                if (!gd_wait(&empty[kb % STAGES], (kb / STAGES - 1) & 1, &abort_flag, status)) break;
+                if (!gd_wait(&empty[kb % STAGES], (kb / STAGES - 1) & 1, waits, &abort_flag, status)) break;
                 weights(kb);
                 tokens(kb);
                 issued = kb + 1;
             }
-            if (abort_flag)                                       // let what is in flight land before the CTA goes away
-                for (int kb = max(0, issued - STAGES); kb < issued; ++kb)
-                    for (int i = 0; i < T5_WAIT_LIMIT && !t5_try_wait(&full[kb % STAGES], (kb / STAGES) & 1); ++i) {}
         }
         __syncwarp();
     } else if (warp == 1) {
@@ -112,7 +111,7 @@ __global__ void __launch_bounds__(GD_THREADS, 2) linear_mid_kernel(
 #pragma unroll 1
         for (int kb = 0; kb < kbs; ++kb) {
             const int st = kb % STAGES;
-            ok = __all_sync(0xffffffffu, gd_wait(&full[st], (kb / STAGES) & 1, &abort_flag, status));
+            ok = __all_sync(0xffffffffu, gd_wait(&full[st], (kb / STAGES) & 1, waits, &abort_flag, status));
             if (!ok) break;
 #pragma unroll
             for (int k = 0; k < GD_K / 16; ++k)
@@ -123,7 +122,7 @@ __global__ void __launch_bounds__(GD_THREADS, 2) linear_mid_kernel(
     } else {
         pdl_wait();
         const int quarter = warp & 3, row = quarter * 32 + lane;
-        const bool ok = __all_sync(0xffffffffu, gd_wait(&acc_full, 0, &abort_flag, status));
+        const bool ok = __all_sync(0xffffffffu, gd_wait(&acc_full, 0, waits, &abort_flag, status));
         t5_fence_after();
         unsigned r[NT / 16][16];
 #pragma unroll
@@ -179,6 +178,10 @@ __global__ void __launch_bounds__(GD_THREADS, 2) linear_mid_kernel(
             }
         }
     }
+    if (tid == 0 && abort_flag)                                   // whoever gave up: what is in flight lands before the CTA goes away
+        for (int kb = max(0, issued - STAGES); kb < issued; ++kb)
+            for (int i = 0; i < T5_WAIT_LIMIT && !t5_try_wait(&full[kb % STAGES], (kb / STAGES) & 1); ++i) {}
+    __syncwarp();
     asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;\n" ::: "memory");      // nobody leaves while its sums are read
     if (warp == 1) {
         t5_fence_after();
@@ -213,7 +216,7 @@ extern "C" int llm_linear_mid_parts(int N, int K, int gated) {
 }
 
 template <int NT, int STAGES, bool GATED, typename TO>
-static int gd_launch(const void* x, const void* w, void* y, int M, int N, int K, int act, float limit, int parts, int32_t* status, cudaStream_t s) {
+static int gd_launch(const void* x, const void* w, void* y, int M, int N, int K, int act, float limit, int parts, int waits, int32_t* status, cudaStream_t s) {
     CUtensorMap w_map, x_map;
     if (!t5_encode_2d(&x_map, x, K, M, GD_K, NT)) return LLM_REFUSED_SIZE;
     if (!t5_encode_2d(&w_map, w, K, static_cast<long long>(N) * (GATED ? 2 : 1), GD_K, 64)) return LLM_REFUSED_SIZE;
@@ -224,15 +227,15 @@ static int gd_launch(const void* x, const void* w, void* y, int M, int N, int K,
     const int tiles = GATED ? N / 64 : (N + GD_ROWS - 1) / GD_ROWS;
     if (tiles > 65535) return LLM_REFUSED_SIZE;
     launch_pdl_cluster(kern, dim3(parts, tiles), dim3(GD_THREADS), smem, s, parts, w_map, x_map, static_cast<TO*>(y), M, N, K,
-                       act, limit, status);
+                       act, limit, waits, status);
     return launch_status();
 }
 
 // x: bfloat16 [M, K]; w: bfloat16 [N, K] (gated: [2 N, K] = [gate; up]);
 // y: [M, N] float32 or bfloat16; gated: bfloat16, act 0 silu, 1 the tanh form of gelu, 2 the clamped form with `limit`, gate and up
-// rounded to bfloat16 first.
+// rounded to bfloat16 first.  waits: tries of a wait (each suspends for a while) before it gives up.
 extern "C" int llm_linear_mid(const void* x, const void* w, void* y, int out_dtype, int gated, int act, float limit, int M, int N, int K,
-                              int32_t* status, uintptr_t stream) {
+                              int waits, int32_t* status, uintptr_t stream) {
     if (!llm_linear_mid_supported(M, N, K, gated)) return LLM_REFUSED_SIZE;
     if (gated && (act < 0 || act > 2 || (act == 2 && !(limit > 0.0f)))) return LLM_REFUSED_SIZE;
     if ((out_dtype != LLM_DT_F32 && out_dtype != LLM_DT_BF16) || (gated && out_dtype != LLM_DT_BF16)) return LLM_REFUSED_DTYPE;
@@ -240,8 +243,8 @@ extern "C" int llm_linear_mid(const void* x, const void* w, void* y, int out_dty
     const int parts = llm_linear_mid_parts(N, K, gated);
     cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
 #define GO_M(GATED, TO)                                                                                \
-    return M <= 32 ? gd_launch<32, 5, GATED, TO>(x, w, y, M, N, K, act, limit, parts, status, s)      \
-                   : gd_launch<48, 5, GATED, TO>(x, w, y, M, N, K, act, limit, parts, status, s)
+    return M <= 32 ? gd_launch<32, 5, GATED, TO>(x, w, y, M, N, K, act, limit, parts, waits, status, s)      \
+                   : gd_launch<48, 5, GATED, TO>(x, w, y, M, N, K, act, limit, parts, waits, status, s)
     if (gated) GO_M(true, bf16);
     if (out_dtype == LLM_DT_F32) GO_M(false, float);
     GO_M(false, bf16);

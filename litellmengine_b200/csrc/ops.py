@@ -2073,7 +2073,8 @@ def mid_product(x, weight: torch.Tensor, out_dtype: torch.dtype, gated: bool = F
     return got
 
 
-def linear_mid(x: torch.Tensor, weight: torch.Tensor, out_dtype: torch.dtype, activation: Optional[str] = None, limit: float = 0.0) -> torch.Tensor:
+def linear_mid(x: torch.Tensor, weight: torch.Tensor, out_dtype: torch.dtype, activation: Optional[str] = None, limit: float = 0.0,
+               waits: int = STREAM_WAITS) -> torch.Tensor:
     """x [M <= 48, K] @ weight^T, bfloat16, streaming the weights once through the tensor cores; with `activation`, weight is
     [gate; up] and the result act(gate) * up in bfloat16, both rounded to bfloat16 first."""
     _dev(x, weight)
@@ -2084,8 +2085,8 @@ def linear_mid(x: torch.Tensor, weight: torch.Tensor, out_dtype: torch.dtype, ac
         raise KernelError("the streaming product takes contiguous bfloat16 operands that agree on K")
     out = torch.empty((M, n), dtype=torch.bfloat16 if gated else out_dtype, device=weight.device)
     f = _fn("gemm_mid_tcgen05", "llm_linear_mid",
-            [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_float, c_int, c_int, c_int, c_void_p, c_void_p])
-    _check(f(_ptr(x), _ptr(weight), _ptr(out), _dt(out), int(gated), ACTIVATIONS[activation] if gated else 0, float(limit), M, n, K,
+            [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_float, c_int, c_int, c_int, c_int, c_void_p, c_void_p])
+    _check(f(_ptr(x), _ptr(weight), _ptr(out), _dt(out), int(gated), ACTIVATIONS[activation] if gated else 0, float(limit), M, n, K, int(waits),
              _ptr(stream_status(weight.device)), _stream()), "linear_mid")
     return out
 

@@ -56,3 +56,25 @@ def test_sizes_it_leaves():
     w = torch.randn(2 * 72, 256, device=DEV).to(torch.bfloat16)   # features that do not fill their tiles
     assert not o.mid_product(x[:, :256].contiguous(), w, torch.bfloat16, gated=True)
     assert o.linear_silu_mul(x[:, :256].contiguous(), w, torch.bfloat16).shape == (20, 72)
+
+
+@pytest.mark.parametrize("N,K,gated", [(4096, 4096, False), (1024, 256, False), (24576, 1024, False), (512, 2048, True)])
+def test_a_wait_that_runs_out(N, K, gated):
+    """Waits without tries: the status is set, the copies land before the blocks end, and the next products are right."""
+    o = ops()
+    g = torch.Generator(device=DEV).manual_seed(9)
+    w = (torch.randn(2 * N if gated else N, K, generator=g, device=DEV) * K ** -0.5).to(torch.bfloat16)
+    x = torch.randn(40, K, generator=g, device=DEV).to(torch.bfloat16)
+    out = dict(out_dtype=torch.bfloat16, activation="silu") if gated else dict(out_dtype=torch.float32)
+    status = o.stream_status(torch.device(DEV))
+    try:
+        want = o.linear_mid(x, w, **out)
+        assert status.tolist() == [0, 0]
+        o.linear_mid(x, w, waits=0, **out)
+        assert status.tolist()[0] == 8
+        status.zero_()
+        for _ in range(3):
+            assert torch.equal(o.linear_mid(x, w, **out), want)
+        assert status.tolist() == [0, 0]
+    finally:
+        status.zero_()
