@@ -8,7 +8,7 @@ import torch
 from ..config.specs import BlockSpec
 from ..weights.loader import ParamSpec
 from .context import StageContext
-from .registry import lookup, register_arrangement
+from .registry import lookup, register_arrangement, speaks_for_forward
 
 
 class StreamConnection:
@@ -205,9 +205,8 @@ class Block:
 def _normed(norm, part, h: torch.Tensor, delta, dtype: torch.dtype):
     """(h + delta, the part's input norm(h + delta)): by the norm's kernel, in place, or left to the part's first product."""
     from ..csrc import ops
-    first = getattr(part, "first_product", None)
-    if first is not None and h.is_cuda:
-        weight, gated = first()
+    if h.is_cuda and speaks_for_forward(norm, "products_apply_it") and speaks_for_forward(part, "first_product"):
+        weight, gated = part.first_product()
         rows = ops.pending_rows(h, delta, norm, weight, dtype, gated)
         if rows is not None:
             return rows.stream, rows

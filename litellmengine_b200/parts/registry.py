@@ -32,6 +32,12 @@ a consumer that says it adds them itself: a norm with `accepts_partials = True` 
 may then be one), a feed-forward with `supports_partials = True` (it is then called with
 `partials_ok=True`), a mixer through `ctx.partials_ok`.  Parts that say nothing never see one.
 
+In small decode steps a norm may be left to the product behind it: a norm that says `products_apply_it = True` (its forward is
+RMS normalisation by `weight` and `eps`, nothing else) in front of a mixer or feed-forward that has `first_product()`, the weight
+of the one product that reads its input and whether that is a gate/up pair.  The part's forward then gets an `ops.PendingRows`, which it
+hands to that product.  Both are read with `speaks_for_forward`: a class that derives from such a part and has a forward of its own
+says so again or is called as any other.
+
 A mixer or feed-forward whose forward only launches kernels on the current stream (no host
 reads, no loops over host data) may set the class attribute `graph_safe = True`; steps of a
 model whose parts all do are replayed as CUDA graphs, one per (tokens, entries) of a step.  A
@@ -72,6 +78,19 @@ def register_feed_forward(kind: str):
 
 def register_arrangement(kind: str):
     return _register("arrangement", kind)
+
+
+def speaks_for_forward(part, name: str) -> bool:
+    """Whether attribute `name` of the part was stated about the forward that it has: by the class that defines `forward`, or by
+    one that derives from that."""
+    if "forward" in getattr(part, "__dict__", {}):
+        return name in part.__dict__
+    for cls in type(part).__mro__:
+        if name in cls.__dict__:
+            return True
+        if "forward" in cls.__dict__:
+            return False
+    return False
 
 
 def unregister(family: str, kind: str) -> None:

@@ -76,3 +76,46 @@ def test_small_products_take_the_streaming_kernel_up_to_32_rows():
     y = ops.linear(x, w, out_dtype=torch.float32)
     assert ops.launch_count > before                              # the engine's own kernel ran, not the library's
     assert float((y - x.float() @ w.float().t()).abs().max()) < 1e-4
+
+
+def test_rows_are_left_to_a_product_only_by_parts_that_say_so_of_their_own_forward(monkeypatch):
+    """`products_apply_it` and `first_product` speak for the forward of the class that states them: a part that derives from
+    such a one and has a forward of its own is called, and is given a tensor."""
+    from litellmengine_b200.config.specs import NormSpec
+    from litellmengine_b200.parts import block
+    from litellmengine_b200.parts.attention import AttentionMixer
+    from litellmengine_b200.parts.feed_forward import SwiGLU
+    from litellmengine_b200.parts.norms import RMSNorm
+
+    class Own(RMSNorm):
+        def forward(self, *a, **k):
+            return "own"
+
+    class Again(Own):
+        products_apply_it = True
+
+    class Kept(RMSNorm):
+        def load(self, tensors):
+            self.weight = 1.0 + tensors[self.name]
+
+    class Mixer(AttentionMixer):
+        def forward(self, x, ctx):
+            return x.shape
+
+    rows = types.SimpleNamespace(stream="stream")
+    monkeypatch.setattr(ops, "pending_rows", lambda *a: rows)
+    monkeypatch.setattr(RMSNorm, "forward", lambda self, *a, **k: "normed")
+    h = types.SimpleNamespace(is_cuda=True)
+    spec = NormSpec("rmsnorm", 1e-6)
+    new = lambda cls: cls.__new__(cls)
+    mixer, ff = new(AttentionMixer), new(SwiGLU)
+    mixer.w_qkv = ff.w_gate_up = None
+    normed = lambda norm, part: block._normed(norm, part, h, None, torch.bfloat16)
+    assert normed(RMSNorm(spec, 8), mixer) == normed(Kept(spec, 8), ff) == normed(Again(spec, 8), ff) == ("stream", rows)
+    assert normed(Own(spec, 8), mixer) == (h, "own")
+    other = new(Mixer)
+    other.w_qkv = None
+    assert normed(RMSNorm(spec, 8), other) == (h, "normed")
+    patched = RMSNorm(spec, 8)
+    patched.forward = lambda *a, **k: "patched"
+    assert normed(patched, mixer) == (h, "patched")
