@@ -421,8 +421,10 @@ class GatedAttentionMixer(BranchMixer):
     def forward(self, x: torch.Tensor, ctx: StageContext):
         s, b = self.spec, ctx.batch
         # prompt portions of a layer whose product is heads and nothing else: norm, rotation and cache write in the product's epilogue
+        # (a class that derives from this one and mixes in its own way does so here too)
         turns = self.rotation is None or (not self.rotation[3] and self.rotation[2] == 1.0 and self.rotation[1] in (64, 128))
-        if (turns and ctx.writes_cache and self.dtype == torch.bfloat16 and self.dv == self.d and not s.output_gate and self.biases is None
+        own = type(self).mix is GatedAttentionMixer.mix
+        if (own and turns and ctx.writes_cache and self.dtype == torch.bfloat16 and self.dv == self.d and not s.output_gate and self.biases is None
                 and s.query_temperature is None and (s.qk_norm is None or s.qk_norm_scope == "head")
                 and ops.heads_product(x, self.w_in, ctx.cache, self.d)):
             angles = None

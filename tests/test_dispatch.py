@@ -119,3 +119,26 @@ def test_rows_are_left_to_a_product_only_by_parts_that_say_so_of_their_own_forwa
     patched = RMSNorm(spec, 8)
     patched.forward = lambda *a, **k: "patched"
     assert normed(patched, mixer) == (h, "patched")
+
+
+def test_a_mixer_that_mixes_in_its_own_way_is_asked_to(monkeypatch):
+    """The q/k/v product that prepares attention itself stands for `GatedAttentionMixer.mix` only."""
+    from litellmengine_b200.config.specs import MixerSpec
+    from litellmengine_b200.parts.attention import GatedAttentionMixer
+
+    class Own(GatedAttentionMixer):
+        def mix(self, proj, col0, ctx, out, out_col0, out_scale):
+            out.fill_(3.0)
+
+    spec = MixerSpec("gated_attention", num_heads=1, num_kv_heads=1, head_dim=128, position=PositionSpec(kind="none"))
+    monkeypatch.setattr(ops, "heads_product", lambda *a: True)
+    monkeypatch.setattr(ops, "linear", lambda x, w, **k: x.float() @ w.float().t())
+    x, ctx = torch.ones(4, 8, dtype=torch.bfloat16), types.SimpleNamespace(batch=types.SimpleNamespace(tables={}, positions=None, token_entry=None,
+              entry_slot=None), writes_cache=True, cache=torch.zeros(1), block_table=None, page_size=16, status=None)
+    asked = []
+    monkeypatch.setattr(ops, "linear_pair_heads", lambda *a: asked.append(a) or torch.zeros(4, 128))
+    monkeypatch.setattr(GatedAttentionMixer, "_attend", lambda self, q, proj, col0, ctx, out, at, scale: out.fill_(5.0))
+    for cls, value, times in ((GatedAttentionMixer, 5.0, 1), (Own, 3.0, 1)):
+        m = cls(spec, 8, torch.bfloat16, "cpu")
+        m.w_in, m.w_o = torch.ones(384, 8), torch.ones(1, 128)
+        assert torch.equal(m.forward(x, ctx), torch.full((4, 1), 128 * value)) and len(asked) == times
