@@ -13,6 +13,7 @@ from ..config.specs import MixerSpec
 from ..csrc import ops
 from ..weights.loader import ParamSpec
 from .context import StageContext, StepPrelude
+from .position import step_angles
 from .registry import lookup, register_mixer
 
 
@@ -286,7 +287,8 @@ class GatedAttentionMixer(BranchMixer):
         # a rotation after the norm, inside the kernel that prepares q, k and v
         self.rotation = None
         if spec.position.kind != "none":
-            self.rotation = lookup("position", spec.position.kind)(spec.position, self.d, device).kernel_args()
+            position = lookup("position", spec.position.kind)(spec.position, self.d, device)
+            self.rotation, self.table_key = position.kernel_args(), getattr(position, "table_key", None)
         self.keep_first = int(getattr(spec, "keep_first", 0)) if spec.window is not None else 0
         self.learned_sink = bool(getattr(spec, "learned_sink", False))
         self.sink = None                        # float32 [heads] on the device: a score per head, none of them scaled
@@ -427,14 +429,7 @@ class GatedAttentionMixer(BranchMixer):
         if (own and turns and ctx.writes_cache and self.dtype == torch.bfloat16 and self.dv == self.d and not s.output_gate and self.biases is None
                 and s.query_temperature is None and (s.qk_norm is None or s.qk_norm_scope == "head")
                 and ops.heads_product(x, self.w_in, ctx.cache, self.d)):
-            angles = None
-            if self.rotation is not None:
-                tables, key = getattr(b, "tables", None), ("half_angles", s.position)
-                angles = tables.get(key) if tables is not None else None
-                if angles is None:
-                    angles = ops.rope_angles(b.positions, self.rotation[0])
-                    if tables is not None:
-                        tables[key] = angles
+            angles = step_angles(b, self.rotation[0], self.table_key) if self.rotation is not None else None
             q = ops.linear_pair_heads(x, self.w_in, ctx.cache, b.positions, b.token_entry, b.entry_slot, ctx.block_table, self.q_norm_w, self.k_norm_w,
                                       s.qk_norm.eps if s.qk_norm is not None else 0.0, angles, self.nq, self.nkv, ctx.page_size, ctx.status)
             out = torch.empty((x.shape[0], self.out_width), dtype=self.dtype, device=x.device)

@@ -13,6 +13,7 @@ from ..config.specs import MixerSpec
 from ..csrc import ops
 from ..weights.loader import ParamSpec
 from .context import StageContext, StepPrelude
+from .position import step_angles
 from .registry import lookup, register_mixer
 
 
@@ -133,15 +134,16 @@ class LatentAttentionMixer:
         self.spec, self.hidden, self.dtype, self.device = spec, hidden_size, compute_dtype, torch.device(device)
         self.scale = spec.scale if spec.scale is not None else 1.0 / math.sqrt(float(self.D + self.P))
         self.names = dict(self._DEFAULT_NAMES, **dict(spec.tensor_names))
-        self.rot_dims, self.inv_freq, self.rot_pairs, self.rot_mag = 0, None, False, 1.0
+        self.rot_dims, self.inv_freq, self.rot_pairs, self.rot_mag, pos = 0, None, False, 1.0, None
         if spec.position.kind == "rope" and self.P:
             pos = lookup("position", "rope")(spec.position, self.P, device)       # the rotation's frequencies, float32
             self.rot_dims, self.inv_freq = pos.rotary_dim, pos.inv_freq
         elif spec.position.kind == "rope_pairs" and self.P:                       # neighbouring pairs, stretched frequencies
-            self.inv_freq, self.rot_dims, self.rot_mag, self.rot_pairs = lookup("position", "rope_pairs")(
-                spec.position, self.P, device).kernel_args()
+            pos = lookup("position", "rope_pairs")(spec.position, self.P, device)
+            self.inv_freq, self.rot_dims, self.rot_mag, self.rot_pairs = pos.kernel_args()
         elif spec.position.kind != "none":
             raise ValueError("latent attention rotates by 'rope', by 'rope_pairs' or not at all")
+        self.table_key = getattr(pos, "table_key", None)
         if spec.output_gate_scope not in ("channel", "head"):
             raise ValueError(f"output_gate_scope {spec.output_gate_scope!r}: 'channel' or 'head'")
         self.gate_per_head = bool(spec.output_gate) and spec.output_gate_scope == "head"
@@ -232,15 +234,7 @@ class LatentAttentionMixer:
 
     def _angles(self, b) -> Optional[torch.Tensor]:
         """The step's table of angles, shared by all layers of the same rotation."""
-        if not self.rot_dims:
-            return None
-        tables, key = getattr(b, "tables", None), ("latent_angles", self.spec.position, self.P)
-        got = tables.get(key) if tables is not None else None
-        if got is None:
-            got = ops.rope_angles(b.positions, self.inv_freq)
-            if tables is not None:
-                tables[key] = got
-        return got
+        return step_angles(b, self.inv_freq, self.table_key) if self.rot_dims else None
 
     def _portions(self, q: torch.Tensor, proj: torch.Tensor, work: LatentWork.Views, ctx: StageContext) -> torch.Tensor:
         """[T, H * V] whose rows that belong to segments hold their attention over per-head keys and values (a gate per head is

@@ -30,6 +30,19 @@ class Rotation:
     angles: Optional[torch.Tensor] = None
 
 
+def step_angles(batch, inv_freq: torch.Tensor, key: tuple) -> torch.Tensor:
+    """float32 [T, len(inv_freq), 2]: sines and cosines of position * inv_freq for the step's tokens, made once for all layers of one
+    `key` (a position part's `table_key`)."""
+    from ..csrc import ops
+    tables = getattr(batch, "tables", None) if key is not None else None      # a part without a key shares nothing
+    got = tables.get(key) if tables is not None else None
+    if got is None:
+        got = ops.rope_angles(batch.positions, inv_freq)
+        if tables is not None:
+            tables[key] = got
+    return got
+
+
 @register_position("none")
 class NoPosition:
     def __init__(self, spec: PositionSpec, head_dim: int, device):
@@ -86,7 +99,7 @@ class RotaryPosition:
         theta32 = torch.tensor(spec.theta, dtype=torch.float32)
         inv = torch.pow(theta32.double(), expo.double()).to(torch.float32)
         self.inv_freq = inv.to(device).contiguous()
-        self._key = ("rope", float(spec.theta), rd)
+        self.table_key = ("rope", float(spec.theta), rd)
         self._table_ok = rd == head_dim and head_dim in (64, 128)      # what the kernel that reads the table takes
 
     def rotation(self, batch) -> Rotation:
@@ -101,9 +114,7 @@ class RotaryPosition:
         if (tables is None or not self._table_ok or batch.num_tokens < ops.ROPE_TABLE_MIN_TOKENS
                 or not self.inv_freq.is_cuda):
             return None
-        if self._key not in tables:
-            tables[self._key] = ops.rope_angles(batch.positions, self.inv_freq)
-        return tables[self._key]
+        return step_angles(batch, self.inv_freq, self.table_key)
 
 
 @register_position("rope_pairs")
@@ -150,6 +161,7 @@ class PairRotation:
                     s = (turns - low) / (high - low) if high > low else 1.0
                     freq[i] = (1.0 - s) * f / factor + s * f
         self.rotary_dim = rd
+        self.table_key = (type(self), repr(spec), head_dim)        # (a spec's numbers may be in lists, which have no hash)
         self.magnitude = float(p.get("magnitude", 1.0))
         self.freq = torch.tensor(freq, dtype=torch.float64).to(torch.float32).to(device).contiguous()
 

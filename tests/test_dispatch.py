@@ -142,3 +142,22 @@ def test_a_mixer_that_mixes_in_its_own_way_is_asked_to(monkeypatch):
         m = cls(spec, 8, torch.bfloat16, "cpu")
         m.w_in, m.w_o = torch.ones(384, 8), torch.ones(1, 128)
         assert torch.equal(m.forward(x, ctx), torch.full((4, 1), 128 * value)) and len(asked) == times
+
+
+def test_tables_of_angles_go_by_the_spec(monkeypatch):
+    """Layers of equal specs share a step's table, others do not, and a spec may hold its numbers in a list."""
+    from litellmengine_b200.config.specs import MixerSpec
+    from litellmengine_b200.parts.latent_attention import LatentAttentionMixer
+    made = []
+    monkeypatch.setattr(ops, "rope_angles", lambda positions, inv_freq: made.append(inv_freq) or len(made))
+
+    def mixer(numbers, theta=10000.0):
+        position = PositionSpec(kind="rope_pairs", theta=theta, rotary_dim=64, params=(("wavelengths", numbers),))
+        return LatentAttentionMixer(MixerSpec("latent_attention", num_heads=2, head_dim=128, value_dim=128, position=position,
+                                              params=(("q_rank", 16), ("kv_rank", 512), ("rot_dim", 64))), 32, torch.bfloat16, "cpu")
+
+    step = types.SimpleNamespace(tables={}, positions=None)
+    first = mixer([8.0, 1.0, 4.0, 8192.0])
+    assert first._angles(step) == 1 and first._angles(step) == 1 and mixer([8.0, 1.0, 4.0, 8192.0])._angles(step) == 1
+    assert mixer([4.0, 1.0, 4.0, 8192.0])._angles(step) == 2 and mixer([8.0, 1.0, 4.0, 8192.0], 5000.0)._angles(step) == 3
+    assert first._angles(types.SimpleNamespace(positions=None)) == 4 and len(made) == 4           # a batch that keeps no tables
