@@ -2003,6 +2003,19 @@ def small_product(rows: int, weight: torch.Tensor, normed: bool = False, gated: 
     return got
 
 
+PENDING_WIDTH = 1024      # widest stream whose rows a block leaves to the product
+
+
+def rows_worth_leaving(h: torch.Tensor, delta) -> bool:
+    """Whether a block leaves its rows to the product behind the norm where that can make them.  Every CTA of the product reads all that the
+    rows are made of.  With k-splits pending the norm's kernel, which adds them once, is faster; with rows of more than 1,024 values a CTA's
+    weights and rows leave the next kernel's no room beside them.  Decode steps of 8 layers at a context of 320, rows made by the product and by
+    the norm's kernel, us, at 1 / 8 requests: width 1,024 with 12 splits of 48 heads' output product pending 277, 252 / 313, 282, with 10 of a
+    feed-forward of 4,736 238, 225 / 279, 267; width 1,536, 13 splits 366, 321 / 392, 345; without splits width 2,048 248, 237 / 280, 256,
+    1,536 262, 244 / 273, 264, 1,280 232, 229 / 266, 257, 1,024 206, 218 / 249, 248, 512 155, 171 / 184, 190."""
+    return h.shape[-1] <= PENDING_WIDTH and not isinstance(delta, PartialSum)
+
+
 def pending_rows(h: torch.Tensor, delta, norm, weight: Optional[torch.Tensor], dtype: torch.dtype, gated: bool) -> Optional[PendingRows]:
     """`norm`'s output for the product with `weight` that follows, left to that product if it can make it; None if it cannot."""
     d = delta.parts if isinstance(delta, PartialSum) else delta

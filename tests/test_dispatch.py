@@ -105,7 +105,7 @@ def test_rows_are_left_to_a_product_only_by_parts_that_say_so_of_their_own_forwa
     rows = types.SimpleNamespace(stream="stream")
     monkeypatch.setattr(ops, "pending_rows", lambda *a: rows)
     monkeypatch.setattr(RMSNorm, "forward", lambda self, *a, **k: "normed")
-    h = types.SimpleNamespace(is_cuda=True)
+    h = types.SimpleNamespace(is_cuda=True, shape=(4, 8))
     spec = NormSpec("rmsnorm", 1e-6)
     new = lambda cls: cls.__new__(cls)
     mixer, ff = new(AttentionMixer), new(SwiGLU)
@@ -161,3 +161,20 @@ def test_tables_of_angles_go_by_the_spec(monkeypatch):
     assert first._angles(step) == 1 and first._angles(step) == 1 and mixer([8.0, 1.0, 4.0, 8192.0])._angles(step) == 1
     assert mixer([4.0, 1.0, 4.0, 8192.0])._angles(step) == 2 and mixer([8.0, 1.0, 4.0, 8192.0], 5000.0)._angles(step) == 3
     assert first._angles(types.SimpleNamespace(positions=None)) == 4 and len(made) == 4           # a batch that keeps no tables
+
+
+def test_rows_of_wide_streams_and_pending_splits_are_the_norm_kernels(monkeypatch):
+    """Each block of a product that makes its rows reads all they are made of: that pays for whole sums of up to 1,024 values only."""
+    from litellmengine_b200.config.specs import NormSpec
+    from litellmengine_b200.parts import block
+    from litellmengine_b200.parts.attention import AttentionMixer
+    from litellmengine_b200.parts.norms import RMSNorm
+    rows = types.SimpleNamespace(stream="stream")
+    monkeypatch.setattr(ops, "pending_rows", lambda *a: rows)
+    monkeypatch.setattr(RMSNorm, "forward", lambda self, *a, **k: "normed")
+    norm, part = RMSNorm(NormSpec("rmsnorm", 1e-6), 8), AttentionMixer.__new__(AttentionMixer)
+    part.w_qkv = None
+    for width, delta, left in ((1024, None, True), (512, torch.zeros(4, 512), True), (1032, None, False),
+                               (1024, ops.PartialSum(torch.zeros(2, 4, 1024)), False)):
+        h = types.SimpleNamespace(is_cuda=True, shape=(4, width))
+        assert block._normed(norm, part, h, delta, torch.bfloat16) == (("stream", rows) if left else (h, "normed"))
