@@ -2219,15 +2219,30 @@ PAIR_MIN_ROWS = 129                                      # fewer rows leave the 
 # the other products too gave 57.6 and 127.1 ms at 4,096 and 8,192 tokens, and adding into the residual
 # 28.9 ms at 2,048.
 _PAIR_NEEDS = {"plain": None, "silu": 850, "into": None, "heads": 750}
-# The q/k/v product with norms, rotation and the cache write in its epilogue saves a kernel that reads the float32 product again.
-# Against the library product and that kernel, cold (us), 6,144 x 4,096: 500 tokens (tiles that fill 0.63 of the time) 40 against 38;
-# 640 (0.81) 41, 42; 900 (0.76) 52, 52; 1,024 (0.86) 52, 54; 2,045 (0.86) 97, 114; 2,900 (0.92) 146, 166; of 4,096 x 1,024: 512
-# (0.86) 18.5, 17.4; 1,024 (0.86) 22.5, 25.6; 8,192 86, 126.
+# The q/k/v product with norms, rotation and the cache write in its epilogue, and the latent queries': by the product alone, cold.
 PAIR_HEADS_MIN_ROWS = 600
 
 
+def heads_pay(rows: int, weight: torch.Tensor) -> bool:
+    """Whether a layer whose q/k/v product `heads_product` takes is faster with it.  It saves a kernel that reads the float32 product again,
+    rows * N values of it; it loses what the clusters idle at the end of its tiles, which grows with K.  So there is a least number of
+    values, and a least share of the clusters' time that the tiles fill: 1 / (1.05 + 694 / K), 0.75 for a K of up to 2,500.  Whole
+    layers, us with it and with the library product and the other kernel (share): 6,144 x 4,096 600 tokens (0.76) 75, 69; 768 (0.97) 82, 82;
+    1,024 (0.86) 102, 100; 1,280 (0.81) 127, 127; 1,536 (0.97) 135, 140; 1,600 (0.81) 154, 149; 2,048 (0.86) 179, 191; 2,900 (0.92) 276, 301;
+    6,144 x 2,560 1,024 (0.86) 80.4, 79.5; 1,280 (0.81) 94, 97; 2,048 137, 148; 4,096 x 2,048 768 (0.65) 52.6, 51.3; 900 (0.76) 57.3, 57.7;
+    1,024 (0.86) 58.5, 60.2; 1,700 (0.72) 87, 85; 2,048 97, 101; 4,096 x 1,024 900 (0.76) 48.6, 49.6; 2,048 83, 85; 2,048 x 1,024 1,024 (0.86)
+    47.0, 46.5; 1,800 (0.76) 58, 61; 7,168 x 5,120 1,100 (0.81) 185, 182; 1,536 (0.91) 261, 277; 10,240 x 5,120 1,100 (0.77) 202, 200; 1,280 (0.90) 230, 260."""
+    n, k = weight.shape
+    if _PAIR_POLICY == "all":
+        return True
+    if rows * n < (3_500_000 if k <= 2048 else 7_800_000):
+        return False
+    filled = _fn("gemm_pair_tcgen05", "llm_linear_pair_efficiency", [c_int, c_int, c_int, c_int])(rows, n, k, 0)
+    return filled >= max(750.0, 1000.0 / (1.05 + 694.0 / k))
+
+
 def heads_product(x: torch.Tensor, weight: torch.Tensor, cache: Optional[torch.Tensor], d: int) -> bool:
-    """Whether `linear_pair_heads` is the faster way for this q/k/v product."""
+    """Whether `linear_pair_heads` takes this q/k/v product, and its tiles fill the clusters well enough to ask `heads_pay`."""
     return (d == 128 and isinstance(x, torch.Tensor) and x.shape[0] >= PAIR_HEADS_MIN_ROWS and cache is not None and cache.dtype == torch.bfloat16
             and cache.is_contiguous() and x.data_ptr() % 16 == 0 and weight.data_ptr() % 16 == 0
             and _pair_takes(x, weight, weight.shape[0], "heads"))
@@ -2248,7 +2263,9 @@ def _pair_takes(x: torch.Tensor, weight: torch.Tensor, n: int, kind: str) -> boo
 
 
 def latent_q_product(x: torch.Tensor, weight: torch.Tensor) -> bool:
-    """Whether `linear_pair_latent_q` is the faster way for these queries (the rule of the q/k/v product)."""
+    """Whether `linear_pair_latent_q` is the faster way for these queries.  Whole layers, us with it and without: 32 heads, K 1,536, 1,280
+    tokens (tiles that fill 0.81 of the time) 141, 146; 1,800 (0.76) 188, 197; 2,500 (0.90) 263, 277; 4,000 486, 517; 16 heads, K 768, 1,280
+    (0.81) 89, 89; 2,000 (0.84) 116, 118; 4,000 202, 214; 8 heads, K 384, 1,500 (0.95) 75, 75; 4,000 (0.84) 152, 154."""
     return (x.shape[0] >= PAIR_HEADS_MIN_ROWS and x.data_ptr() % 16 == 0 and weight.data_ptr() % 16 == 0
             and _pair_takes(x, weight, weight.shape[0], "heads"))
 

@@ -166,7 +166,7 @@ class AttentionMixer:
         kw = self.k_norm.weight if self.k_norm is not None else None
         cache, table = (ctx.cache, ctx.block_table) if has_kv else (None, None)
         rotates = hasattr(self.position, "rotation")
-        if rotates and has_kv and self.dtype == torch.bfloat16 and ops.heads_product(x, self.w_qkv, cache, self.d):
+        if rotates and has_kv and self.dtype == torch.bfloat16 and ops.heads_product(x, self.w_qkv, cache, self.d) and ops.heads_pay(x.shape[0], self.w_qkv):
             rot = self.position.rotation(b)
             if rot is None or (rot.rotary_dim == self.d and rot.angles is not None):
                 # prompt portions: norms, rotation and cache write in the product's epilogue
@@ -428,7 +428,7 @@ class GatedAttentionMixer(BranchMixer):
         own = type(self).mix is GatedAttentionMixer.mix
         if (own and turns and ctx.writes_cache and self.dtype == torch.bfloat16 and self.dv == self.d and not s.output_gate and self.biases is None
                 and s.query_temperature is None and (s.qk_norm is None or s.qk_norm_scope == "head")
-                and ops.heads_product(x, self.w_in, ctx.cache, self.d)):
+                and ops.heads_product(x, self.w_in, ctx.cache, self.d) and ops.heads_pay(x.shape[0], self.w_in)):
             angles = step_angles(b, self.rotation[0], self.table_key) if self.rotation is not None else None
             q = ops.linear_pair_heads(x, self.w_in, ctx.cache, b.positions, b.token_entry, b.entry_slot, ctx.block_table, self.q_norm_w, self.k_norm_w,
                                       s.qk_norm.eps if s.qk_norm is not None else 0.0, angles, self.nq, self.nkv, ctx.page_size, ctx.status)

@@ -93,6 +93,21 @@ def test_prompts_through_the_heads_product(monkeypatch, config):
     near(one, two, 2e-3)
 
 
+def test_prompts_that_the_heads_product_would_slow_down(monkeypatch):
+    """1,024 tokens of 2,048 x 256: fewer values than the saved kernel is worth."""
+    from litellmengine_b200.csrc import ops
+    calls, real = [], ops.linear_pair_heads
+    monkeypatch.setattr(ops, "linear_pair_heads", lambda *a, **k: calls.append(1) or real(*a, **k))
+    for config in (qwen(), windowed(64, None)):
+        layer(config, [800, 224])
+    assert not calls
+    w = lambda n, k: torch.empty(n, k, device=DEV, dtype=torch.bfloat16)
+    big = w(6144, 4096)
+    assert [t for t in (640, 768, 1024, 1200, 1536, 1600, 2048, 2900) if ops.heads_pay(t, big)] == [1536, 2048, 2900]
+    assert [t for t in (768, 1024, 1100, 1280, 2048) if ops.heads_pay(t, w(4096, 2048))] == [1024, 2048]
+    assert [t for t in (1024, 1800) if ops.heads_pay(t, w(2048, 1024))] == [1800]
+
+
 @pytest.mark.parametrize("rot", [True, False])
 def test_prompts_whose_latent_queries_are_packed(monkeypatch, rot):
     one, two = both_ways(monkeypatch, "latent_q_product", False, "linear_pair_latent_q", lambda: layer(latent(rot), [900, 380]))
