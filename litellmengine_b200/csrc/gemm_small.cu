@@ -7,7 +7,8 @@
 //     are no partial sums.  gemm_skinny.cu gives a CTA 64 features by 512 k-values, which moves large weights faster, but its 4
 //     to 6 sums an output are read again by the next kernel.
 //   * Its weights (16 x K, pieces of 2 KB) are asked for before the wait for the kernel in front.  The rule that sends a product
-//     here is that every CTA is on an SM at once: then all of the weights are on their way while that kernel still runs.
+//     here (llm_linear_small_supported) is that every CTA is on an SM at once: then all of the weights are on their way while that
+//     kernel still runs.
 //   * The rows may be made on the way (`normed`): rmsnorm of the residual stream plus what is pending, a warp a row, every CTA for
 //     itself (2 x M x K floats from L2).  Row r of the sum is written to another buffer by CTA r: the stream itself is still
 //     being read by the rest of the grid.
@@ -15,9 +16,9 @@
 // The norm's and the activation's numbers are those of norm.cu and activation.cu, added in their order.
 // A decode step of 8 layers of width 1,024 at a context of 320, us, before (streaming product, norm and activation kernels) and now: 1
 // request 268, 233; 5 287, 252; 8 303, 278; 9 334, 311; 16 347, 330.  Rows made by every CTA pay up to 8 of them: with more
-// the stream is read too often (16 requests 354; and with 16 features a CTA instead of 32, 374).  What it takes to get there: at most 128
-// registers and half the shared memory a CTA, so that the next kernel's CTAs find room while this one's still run (with 8 eights of a row
-// held where 4 do, 267 us for 5 requests instead of 247).
+// the stream is read too often (16 requests 354; and with 16 features a CTA instead of 32, 374).  It is better where the next kernel's
+// CTAs find room while this one's still run: with 8 eights of a row held where 4 do, 267 us for 5 requests instead of 247; rows of more
+// than 1,024 values, whose CTAs take 110 to 170 KB, are not left to a product by a block (`rows_worth_leaving` in ops.py).
 // Products run on mma.sync m16n8k16 with the weights as the 16-row operand and the tokens as the 8 columns; sums are float32.
 // The wait for the weights is bounded: a thread whose tries run out records status code 8 and goes on (the result is then flagged), but
 // does not end before the copies have landed, for which it waits, bounded again: the block's memory may be another one's next.
@@ -265,14 +266,37 @@ static int gm_ctas(int N, bool normed, bool gated) {
     return (N + each - 1) / each;
 }
 
+// CTAs of a form that an SM holds by their registers: four for up to eight rows that are there, three otherwise, two for wide made rows.
+template <int MT, int HELD, bool GATED>
+static int gm_resident() {
+    static int n = 0;
+    if (n == 0 && cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, linear_small_kernel<MT, HELD, GATED, bf16, true>, GM_THREADS, 0) != cudaSuccess) {
+        (void)cudaGetLastError();
+        n = 0;
+    }
+    return n;
+}
+static int gm_resident_of(int M, int K, int normed, int gated) {
+    if (normed && K <= 1024) return gated ? gm_resident<8, 4, true>() : gm_resident<8, 4, false>();
+    if (normed) return gated ? gm_resident<8, 8, true>() : gm_resident<8, 8, false>();
+    if (M <= 8) return gated ? gm_resident<8, 0, true>() : gm_resident<8, 0, false>();
+    return gated ? gm_resident<16, 0, true>() : gm_resident<16, 0, false>();
+}
+
 // Whether a product of M rows, N features (gated: the activation's, with 2 N rows of weights) over K values comes here: all CTAs on the
-// SMs at once, 220 KB each.  normed: at most eight rows, which a warp's registers hold.
+// SMs at once, by their registers and in 220 KB of shared memory an SM.  normed: at most eight rows, which a warp's registers hold.
+// A second wave of CTAs asks for its weights when the first one is done.  Chains of products, us, this kernel and the streaming product, 8
+// rows: K 512, N 11,840 (five CTAs an SM where four fit) 4.8, 3.2; K 256, N 18,944 (eight) 4.4, 3.1; 16 rows, K 256, N 9,472 (four where
+// three fit) 4.2, 3.1; gated, K 256, N 9,472 4.4, 4.3.  With a K of up to 512 the streaming product leaves whole sums as well, and is
+// faster from 385 on with many features: 8 rows, K 512, N 4,096 2.70, 2.56; 6,144 2.90, 2.64; 9,472 3.16, 2.65; K 448, N 9,472 3.07, 2.66; K
+// 384, N 8,192 2.81, 2.90; K 576, N 9,472 3.49, 3.67 and then a kernel that adds the slices.
 extern "C" int llm_linear_small_supported(int M, int N, int K, int normed, int gated) {
     if (M < 1 || M > (normed ? 8 : 16) || N < 1 || K < 64 || K % 8 || (normed && K > 256 * GM_HELD) || (gated && N % GM_ROWS) || N > (1 << 20) || K > (1 << 16)) return 0;
+    if (!normed && !gated && K > 384 && K <= 512 && N > 4096) return 0;
     if (!gm_device()) return 0;
     const long long each = gm_bytes(M <= 8 ? 8 : 16, K, normed, gated) + 1024, ctas = gm_ctas(N, normed, gated);
     const long long per_sm = (ctas + g_gm_sms - 1) / g_gm_sms;
-    return per_sm <= 8 && per_sm * each <= 220 * 1024 ? 1 : 0;
+    return per_sm <= gm_resident_of(M, K, normed, gated) && per_sm * each <= 220 * 1024 ? 1 : 0;
 }
 
 typedef CUresult (*GmEncodeFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,

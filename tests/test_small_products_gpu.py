@@ -108,3 +108,16 @@ def test_a_wait_that_runs_out(form):
     finally:
         status.zero_()
         o._tiled.pop(w.data_ptr(), None)
+
+
+def test_all_blocks_of_a_product_fit_at_once():
+    """By registers as well as by shared memory: 148 SMs hold four blocks of 16 features for up to eight rows, three otherwise."""
+    o = ops()
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    takes = lambda rows, n, k, **f: o.small_product(rows, torch.empty(n, k, device=DEV, dtype=torch.bfloat16), **f)
+    assert takes(8, 64 * sms, 256) and not takes(8, 64 * sms + 16, 256) and takes(16, 48 * sms, 256) and not takes(16, 48 * sms + 16, 256)
+    assert takes(8, 2 * 48 * sms, 256, gated=True) and not takes(8, 2 * (48 * sms + 16), 256, gated=True)
+    assert takes(8, 96 * sms, 256, normed=True) and not takes(8, 96 * sms + 32, 256, normed=True)
+    assert takes(8, 64 * sms, 1024) and not takes(8, 64 * sms + 16, 1024)
+    # where the streaming product leaves whole sums too, and has many features to do it with
+    assert takes(8, 4096, 512) and not takes(8, 4112, 512) and not takes(8, 4112, 392) and takes(8, 4112, 384) and takes(8, 4112, 520)
