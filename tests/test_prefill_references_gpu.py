@@ -96,3 +96,51 @@ def test_latent_maxima_that_move(loud, times, window):
         bound = 2.0 ** -8 * (carried + want.abs()) * 1.02 + 2 * cut * carried + 1e-6
         got = out[starts[b]:starts[b] + t].to(F64)
         assert bool(((got - want).abs() <= bound).all()), (n, t, float(((got - want).abs() / bound).max()))
+
+
+@pytest.mark.parametrize("loud,times", [([], 1.0), ([127, 128, 200, 383], 12.0), ([64, 129, 450], 60.0), (list(range(0, 600, 37)), 400.0)])
+@pytest.mark.parametrize("window", [None, 70])
+def test_biased_maxima_that_move(loud, times, window):
+    """The same with a temperature per head and a logarithmic bias of the distance, whose two tables take turns tile by tile."""
+    from litellmengine_b200.csrc import ops
+    g = torch.Generator(device=DEV).manual_seed(15 + len(loud))
+    reqs = [(2, 2), (65, 65), (128, 128), (257, 129), (600, 255), (640, 1 + 128), (513, 513)]      # (cached and new, new)
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)
+    width = max(-(-n // PAGE) for n, _ in reqs)
+    table = torch.randperm(len(reqs) * width, generator=g, device=DEV).to(torch.int32).view(len(reqs), width).contiguous()
+    cache = torch.zeros(len(reqs) * width, 2, NKV, PAGE, D, device=DEV, dtype=torch.bfloat16)
+    kv = []
+    for b, (n, _) in enumerate(reqs):
+        x = torch.randn(2, n, NKV, D, generator=g, device=DEV)
+        for k in loud:
+            if k < n:
+                x[0, k] *= times
+        x = x.to(torch.bfloat16)
+        j = torch.arange(n, device=DEV)
+        for s in (0, 1):
+            cache[table[b, j // PAGE].long(), s, :, j % PAGE] = x[s]
+        kv.append(x)
+    T, starts = sum(t for _, t in reqs), [sum(t for _, t in reqs[:b]) for b in range(len(reqs))]
+    q = torch.randn(T, NQ * D, generator=g, device=DEV).to(torch.bfloat16)
+    three = torch.tensor([[1.0, 0.0, 0.0], [0.7, 1.5, 0.3], [1.3, 0.4, 5.0], [0.2, 3.0, 1.0]], device=DEV)      # temperature, r1, r2
+    out = torch.full((T, NQ * D), float("nan"), device=DEV, dtype=torch.bfloat16)
+    tiles = [(b, r) for b, (_, t) in enumerate(reqs) for r in range(0, t, 128)] + [(-1, -1)]
+    status = i32([0, 0])
+    ops.paged_attention_prefill_tcgen05_biased(q, out, cache, i32(tiles), len(tiles), i32(list(range(len(reqs)))), i32(starts),
+                                               i32([t for _, t in reqs]), i32([n for n, _ in reqs]), table, NQ, NKV, D, PAGE, window, D ** -0.5,
+                                               status, three)
+    assert status.tolist() == [0, 0]
+    temp, r1, r2 = (c.to(F64)[:, None, None] for c in three.unbind(1))
+    for b, (n, t) in enumerate(reqs):
+        k, v = (x.to(F64).repeat_interleave(NQ // NKV, 1) for x in kv[b])
+        i, j = torch.arange(n - t, n, device=DEV)[:, None], torch.arange(n, device=DEV)[None, :]
+        off = r1 * torch.log1p(r2 * (i - j).clamp(min=0))
+        s = torch.einsum("thd,shd->hts", q[starts[b]:starts[b] + t].view(t, NQ, D).to(F64), k) * D ** -0.5 * temp
+        see = (j <= i) & ((i - j < window) if window else torch.ones_like(i - j, dtype=torch.bool))
+        p = torch.softmax((s - off).masked_fill(~see, float("-inf")), -1)
+        want, carried = (torch.einsum("hts,shd->thd", p, x).reshape(t, -1) for x in (v, v.abs()))
+        # the bound of the first test; the bias is a float32 product of r1 and a logarithm that is within 2^-21 of its size or of 1
+        cut = float(s.abs().max()) * 128 * 2.0 ** -23 + (1 + float(off.max())) * 4 * 2.0 ** -21
+        bound = 2.0 ** -8 * (carried + want.abs()) * 1.02 + 2 * cut * carried + 1e-6
+        got = out[starts[b]:starts[b] + t].to(F64)
+        assert bool(((got - want).abs() <= bound).all()), (n, t, float(((got - want).abs() / bound).max()))
