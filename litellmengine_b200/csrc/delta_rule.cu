@@ -1088,7 +1088,7 @@ __global__ void __launch_bounds__(128) delta_batch_kernel(
     for (int i = tid; i < DX_IMAGE / 16; i += 128) to[i] = reinterpret_cast<const uint4*>(dx_smem)[i];
 }
 
-// grid: entries (longest portion first) x H x column tiles of 32, the tiles fastest.
+// grid: entries (longest portion first) x H x column tiles of DX_COLS, the tiles fastest.
 #define DX_COLS 16
 #define DX_SMEM (2 * DX_IMAGE + 4 * 4 * 32 * 16)
 __global__ void __launch_bounds__(128, 2) delta_scan_mma_kernel(
@@ -1577,14 +1577,19 @@ static int delta_shape(DeltaShape& s, int H, int G, int D, int V, int taps, int 
 //   portions below 256: 100, 16: 60, 64; 4 x 200, 16: 123, 128; 32 x 64, 16: 259, 276
 // (with blocks of 32 columns; with 16 the layer of one request takes 1,000, 16: 263, 231; 2,500, 16: 605, 524; 2,000, 8: 344, 297; 2,000,
 // 4: 306, 275, and below 256 tokens both are level: the line could lie lower, and one request come here too)
-// So: 256 tokens and more; more than 2,048 columns, or 1,500 where several requests share a step with a portion of 1,000 tokens; two
-// blocks an SM at most.
+// So: 256 tokens and more; more than 2,048 columns, or 1,500 where several requests share a step with a portion of 1,000 tokens; up to
+// 9,472 columns, the two blocks of 32 columns an SM for which the line was measured first.  With blocks of 16 columns that are four, two of
+// which an SM holds (97 KB each); a second wave of equal portions does not double the walk, because a block alone on its SM has half the
+// columns and nothing in its way.  Layers, us, eight tokens a chunk, blocks of 32 columns and these: portions of 16 heads: 2 x 1,000 392, 378, 354; 3 x
+// 1,000 591, 577, 572; 4 x 1,000 (8,192 columns) 681, 679, 672; 4 x 500 354, 361, 358; 4 x 260 205, 213, 209; 400, 800, 1,200 and 1,600
+// 765, 707, 664; 3 x 300 and 2,000 650, 581, 546; 8 heads: 6 x 1,000 532, 517, 513; 8 x 1,000 605, 606, 598; 9 x 900 578, 584, 577; 8 from 200
+// to 900 400, 377, 337.  (Equal short portions near the end of the range would be 1 to 2 % faster with eight tokens a chunk.)
 extern "C" int llm_delta_image_bytes() { return DX_IMAGE; }
 static bool dx_takes(int H, int D, int V) { return D == 128 && V > 0 && V % 32 == 0 && H > 0 && H <= 65535; }
 extern "C" int llm_delta_batched(int H, int D, int V, int num_entries, int max_len) {
     const long long columns = static_cast<long long>(num_entries) * H * V;
     const bool enough = columns > 2048 || (columns >= 1500 && num_entries > 1 && max_len >= 1000);
-    return dx_takes(H, D, V) && max_len >= 256 && enough && columns <= 2 * DR_SMS * 32;
+    return dx_takes(H, D, V) && max_len >= 256 && enough && columns <= 64 * DR_SMS;
 }
 
 // Everything of a step that is not all single tokens.  Scratch (float32): qn, kn [T, G, DP], vn [T, H, VP], beta [T, H],

@@ -8,11 +8,13 @@
 //   latent_gather    the rows of every portion, from their pages, to consecutive rows of one tensor, each request's padded
 //                    with zero rows to whole tiles (so that a tile never shows another request's rows)
 //   (a product)      [k | v] of all rows and heads
-//   latent_q_pack    the queries [qn | rotated qr] per head in bfloat16
+//   queries          [qn | rotated qr] per head in bfloat16: in the epilogue of their product (linear_pair_latent_q in
+//                    gemm_pair_tcgen05.cu) where that takes them, else by latent_q_pack (12 us of 2,000 tokens and 32 heads)
 //   attention        below
 // Measured, 32 heads over rows of 512 + 64, a prompt of 2,000 tokens: attention over the cached rows 1,275 us; here rows 5,
-// map 18, queries 12, attention 62 us (0.69 PFLOP/s of what it cannot do without, 43 GFLOP; with two threads a row that exchanged
-// their maxima before the weights, and products issued in a branch for one lane, 85).  The layer 1,480 -> 237 us.
+// map 18, attention 62 us (0.69 PFLOP/s of what it cannot do without, 43 GFLOP; with two threads a row that exchanged
+// their maxima before the weights, and products issued in a branch for one lane, 85).  The layer 1,480 -> 237 us, and 224 with packed
+// queries (and a step's table of angles, which all layers share: 2 us to make, not in the layer's figure).
 //
 // Attention.  The structure of the one-pass kernel in attention_prefill_tcgen05.cu (a reference maximum that trails the
 // running one, two rows of work in turns on the tensor pipe, P over S in TMEM, a softmax thread a row, weights of half a tile made
@@ -196,7 +198,7 @@ __global__ void __launch_bounds__(LP_THREADS, 1) latent_prefill_tcgen05_kernel(
         // All lanes walk the loop, one of them issues.
         constexpr unsigned IDESC_QK = t5_idesc(LP_BM, LP_BN, 0);
         constexpr unsigned IDESC_PV = t5_idesc(LP_BM, LP_DV, 1);
-        const unsigned lead = t5_elect();
+        const unsigned lead = elect_one();
         const unsigned long long qd0 = t5_desc(q_s, 16, 1024), kd0 = t5_desc(k_s, 16, 1024);
         const unsigned long long vd0 = t5_desc(v_s, LP_KB * sizeof(bf16), 1024);
         constexpr unsigned long long K_STEP = (3 * LP_KB * sizeof(bf16)) >> 4, V_STEP = (2 * LP_KB * sizeof(bf16)) >> 4;

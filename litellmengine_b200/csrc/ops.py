@@ -2059,8 +2059,8 @@ def linear_small(x, weight: torch.Tensor, out_dtype: torch.dtype, activation: Op
     return out
 
 
-# Rows that take `linear_mid`.  Up to 32 it was faster than the library product (below them `linear_skinny` is) at every size tried
-# from 1,024 x 3,072 to 151,936 x 2,048 (4,096 x 2,048 at 32 rows: 6.3 us against 6.2) and than `linear_skinny` where that took so many
+# Rows that take `linear_mid`.  Up to 32 it was level with the library product (below them `linear_skinny` is faster) or faster at every size tried
+# from 1,024 x 3,072 to 151,936 x 2,048 (the worst, 4,096 x 2,048 at 32 rows: 6.3 us against 6.2), and faster than `linear_skinny` where that took so many
 # (2,048 x 6,144: 7.7 against 9.6).  With up to 48 rows the parts' sums weigh more: wide products of a short K stay with the library
 # (40 rows, 4,096 x 2,048: 6.7, 6.3; 5,120 x 2,048: 7.3, 6.8) unless they need no parts (52,224 x 2,048: 40.5, 41.8).
 MID_ROWS = range(SKINNY_MAX_ROWS + 1, 49)
