@@ -7,15 +7,6 @@
 #include "common.cuh"
 #include <algorithm>
 
-__device__ __forceinline__ float silu(float g) { return g / (1.0f + expf(-g)); }
-__device__ __forceinline__ float gelu_tanh(float g) {
-    return 0.5f * g * (1.0f + tanhf(0.7978845608028654f * (g + 0.044715f * g * g * g)));
-}
-__device__ __forceinline__ float gated(float g, float u, int kind, float limit) {
-    if (kind == 2) return clamped_swish(g, u, limit, CLAMPED_SWISH_ALPHA, 1.0f);
-    return (kind == 1 ? gelu_tanh(g) : silu(g)) * u;
-}
-
 // grid (blocks along the row, tokens): a thread takes 8 consecutive features of one token.
 template <typename T>
 __global__ void silu_and_mul_kernel(const T* __restrict__ gu, T* __restrict__ out, int inter, int act, float limit) {

@@ -498,7 +498,7 @@ __global__ void __launch_bounds__(T5O_THREADS, 1) paged_prefill_attention_tcgen0
         // shared memory is the same descriptor plus its byte offset / 16 in the address field.
         constexpr unsigned IDESC_QK = t5_idesc(T5_BM, T5O_BN, 0);
         constexpr unsigned IDESC_PV = t5_idesc(T5_BM, T5_D, 1);
-        const unsigned lead = t5_elect();
+        const unsigned lead = elect_one();
         const unsigned long long qd0 = t5_desc(q_s, 16, 1024), kd0 = t5_desc(k_s, 16, 1024);
         const unsigned long long vd0 = t5_desc(v_s, T5O_HALF * sizeof(bf16), 1024);
         constexpr unsigned long long STAGE_STEP = (T5O_TILE * sizeof(bf16)) >> 4, VSTEP = (16 * 64 * sizeof(bf16)) >> 4;   // 16 keys further, both 64-column halves

@@ -96,6 +96,23 @@ __device__ __forceinline__ float clamped_swish(float g, float u, float limit, fl
 }
 #define CLAMPED_SWISH_ALPHA 1.702f
 
+// A gated feed-forward's middle by its kind: 0 silu(g) * u, 1 the tanh form of gelu, 2 the clamped form with `limit`.
+__device__ __forceinline__ float silu(float g) { return g / (1.0f + expf(-g)); }
+__device__ __forceinline__ float gelu_tanh(float g) {
+    return 0.5f * g * (1.0f + tanhf(0.7978845608028654f * (g + 0.044715f * g * g * g)));
+}
+__device__ __forceinline__ float gated(float g, float u, int kind, float limit) {
+    if (kind == 2) return clamped_swish(g, u, limit, CLAMPED_SWISH_ALPHA, 1.0f);
+    return (kind == 1 ? gelu_tanh(g) : silu(g)) * u;
+}
+
+// 1 in one lane of the warp, whose lanes are all here.
+__device__ __forceinline__ unsigned elect_one() {
+    unsigned r;
+    asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}\n" : "=r"(r));
+    return r;
+}
+
 // The first key that the query at `pos` sees.  span > 0: a sliding window, the last `span` keys, its own included.
 // span < 0: chunks of -span positions counted from the sequence's start, each query its own chunk's keys.  0: every key.
 __device__ __forceinline__ int first_visible(int pos, int span) {

@@ -19,24 +19,25 @@
 // A CTA makes 128 weight rows x NT tokens (the MMA's M side is the weights, so that 17 tokens cost a tile of 32).  Roles: warp
 // 0 feeds the copy engine: 128 x 64 weights as float32, and NT x 64 of the three planes of x, which a small kernel has
 // split; warps 2 to 9 split the weights in shared memory, half a row a thread (11 instructions for two values; storing the split
-// weights instead would double their memory and their bytes); one lane of warp 1 issues 6 x 4 products a block of 64;
+// weights instead would double their memory and their bytes); warp 1 issues 6 x 4 products a block of 64;
 // warps 10 to 17 drain.  Planes are double-buffered (96 KB of weights' planes, 96 KB of x at NT 128).
 // The weights' planes go to tensor memory, from where the tensor cores take their left operand: kept in shared memory, their
 // stores and the operand reads of 24 products a block (8 KB each) filled the shared-memory path (500 tokens of 4096 x 12288:
 // 323 us, 291 in tensor memory).  The issuing warp walks the blocks with all its lanes: in a branch for one lane each of the three
 // waits in front of a block kept the tensor pipe idle for 250 clocks of the 2,500 to 2,900 that a block took (its 24 products are
-// 1,536): 500 tokens of 4096 x 12288 296 -> 251, of 6144 x 4096 181 -> 152, 17 tokens of 24576 x 4096 146 -> 114.
+// 1,536); the table has both.
 // The loop that makes sums again which are not finite stays rolled: unrolled into each of a drain thread's sums it cost
 // finite ones up to 20 % (500 tokens of 6144 x 4096: 209 us, now 167).
 // Tiles that fill the SMs badly are cut along K (`splits`), the parts added in order by a second kernel.
 //
-// Measured (us; the library's float32 product in brackets):
-//   N x K              17 rows        64 rows        128 rows       500 rows       2,048 rows
-//   6144 x 4096        36 (106)       40 (129)       46 (170)       148 (542)      507 (1,773)
-//   4096 x 4096        30 (105)       32 (106)       40 (126)       95 (311)       343 (1,132)
-//   24576 x 4096       112 (199)      122 (283)      148 (551)      503 (1,779)    1,830 (6,686)
-//   4096 x 12288       71 (250)       77 (321)       91 (373)       282 (925)      990 (3,353)
-//   2048 x 2048        22 (54)        24 (53)        30 (52)        44 (87)        120 (308)
+// Measured (us; products issued in a branch for one lane, in turns on one GPU; the library's float32 product in brackets), everything cold:
+//   N x K              17 rows            64 rows            128 rows           500 rows           2,048 rows
+//   6144 x 4096        36; 46 (106)       40; 48 (129)       46; 56 (170)       148; 180 (542)     513; 597 (1,773)
+//   4096 x 4096        30; 38 (105)       32; 38 (106)       40; 46 (126)       95; 112 (311)      347; 409 (1,132)
+//   24576 x 4096       112; 148 (199)     123; 155 (283)     150; 182 (551)     509; 591 (1,779)   1,850; 2,100 (6,686)
+//   4096 x 12288       63; 80 (250)       69; 83 (321)       81; 97 (373)       251; 296 (925)     985; 1,100 (3,353)
+//   2048 x 2048        22; 28 (54)        24; 28 (53)        30; 34 (52)        44; 51 (87)        118; 136 (308)
+// (4096 x 12288 from 500 rows on depends on the clocks: behind a second of such products 292 to 304 and 1,050, and 337 and 1,210 before.)
 // Matrices of fewer than 2^21 values stay with the library: of 1024 x 1024, 17 rows take 23 us against 18 (and 64 to 2,048 rows 23
 // to 34 against 29 to 86: for many rows the line could lie lower).
 #include "tcgen05_attention.cuh"
@@ -185,7 +186,7 @@ __global__ void __launch_bounds__(LT_THREADS, 1) linear_f32_tcgen05_kernel(
     } else if (warp == 1) {
         pdl_wait();                                               // before any bounded wait: the kernel in front may take its time
         constexpr unsigned IDESC = t5_idesc(LT_ROWS, NT, 0);
-        const unsigned lead = t5_elect();                         // all lanes walk the blocks, one issues
+        const unsigned lead = elect_one();                         // all lanes walk the blocks, one issues
         const unsigned long long xd = t5_desc(x_s, 16, 1024);
         constexpr unsigned long long X_STEP = X_PLANE * sizeof(bf16) >> 4;
         // the smallest terms first: l h, h l, m m, m h, h m, h h
@@ -326,9 +327,9 @@ static int lt_tile(int M) { return M <= 32 ? 32 : M <= 64 ? 64 : 128; }
 
 // Into how many parts K is cut: the least of waves of 148 CTAs x (blocks of 64 x BLK + 4 us) + the parts' way through memory,
 // with a block's time (1.5 us at 128 tokens, 1.0 below: a fifth more than it takes, and fewer parts of equal time
-// would sum longer runs).  In 1, 2, 3, 4, 6, 8 parts (us): 500 tokens of 6144 x 4096 171, 148, 146, 171, 175, - (takes 3), of 4096 x
-// 4096 95, 103, 110, 120, 134, 142 (1), of 4096 x 12288 249, 259, 267, 275, 288, 280 (1); 17 tokens of 4096 x 12288 214, 116, 83,
-// 67, 83, 69 (4), of 24576 x 4096 150, 124, 116, 128, 128, 136 (3).
+// would sum longer runs).  In 1, 2, 3, 4, 6, 8 parts (us, cold): 500 tokens of 6144 x 4096 169, 151, 146, 173, 183, 206 (takes 3), of 4096 x
+// 4096 93, 103, 110, 120, 134, 144 (1), of 4096 x 12288 247, 261, then at lower clocks 319, 328, 336, 328 (1); 17 tokens of 4096 x 12288 239,
+// 128, 85, 65, 83, 71 (4), of 24576 x 4096 149, 120, 114, 126, 124, 130 (3).
 extern "C" int llm_linear_f32_tcgen05_splits(int M, int N, int K) {
     if (M <= 0 || N <= 0 || K <= 0) return 1;
     const int nt = lt_tile(M);

@@ -39,10 +39,6 @@ __device__ __forceinline__ bool gd_wait(unsigned long long* bar, unsigned parity
     if (atomicCAS(status, 0, GD_STATUS) == 0) status[1] = blockIdx.y;
     return false;
 }
-__device__ __forceinline__ float gd_gated(float g, float u, int act, float limit) {
-    if (act == 2) return clamped_swish(g, u, limit, CLAMPED_SWISH_ALPHA, 1.0f);
-    return (act == 1 ? 0.5f * g * (1.0f + tanhf(0.7978845608028654f * (g + 0.044715f * g * g * g))) : g / (1.0f + expf(-g))) * u;
-}
 
 // grid (parts of K, tiles), a cluster the parts of a tile.  N: features of the result.
 template <int NT, int STAGES, bool GATED, typename TO>
@@ -105,7 +101,7 @@ __global__ void __launch_bounds__(GD_THREADS, 2) linear_mid_kernel(
     } else if (warp == 1) {
         pdl_wait();
         constexpr unsigned IDESC = t5_idesc(GD_ROWS, NT, 0);
-        const unsigned lead = t5_elect();
+        const unsigned lead = elect_one();
         const unsigned long long wd = t5_desc(w_s, 16, 1024), xd = t5_desc(x_s, 16, 1024);
         bool ok = true;
 #pragma unroll 1
@@ -154,7 +150,7 @@ __global__ void __launch_bounds__(GD_THREADS, 2) linear_mid_kernel(
                 if (p < parts) v.x += f[p].x, v.y += f[p].y, v.z += f[p].z, v.w += f[p].w;
             return v;
         };
-                if constexpr (GATED) {
+        if constexpr (GATED) {
             const int f = 4 * (tid & 15);
 #pragma unroll 2
             for (int tok = part + (tid >> 4) * parts; tok < M; tok += GD_THREADS / 16 * parts) {
@@ -163,7 +159,7 @@ __global__ void __launch_bounds__(GD_THREADS, 2) linear_mid_kernel(
                 __align__(8) bf16 out[4];
 #pragma unroll
                 for (int i = 0; i < 4; ++i)
-                    out[i] = from_f32<bf16>(gd_gated(to_f32(from_f32<bf16>(gs[i])), to_f32(from_f32<bf16>(us[i])), act, limit));
+                    out[i] = from_f32<bf16>(gated(to_f32(from_f32<bf16>(gs[i])), to_f32(from_f32<bf16>(us[i])), act, limit));
                 *reinterpret_cast<uint2*>(y + static_cast<size_t>(tok) * N + tile * 64 + f) = *reinterpret_cast<const uint2*>(out);
             }
         } else {

@@ -107,11 +107,6 @@ __device__ __forceinline__ void gp_mma_pair(unsigned lead, unsigned d_tmem, unsi
                  " @q tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::
                      "r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(lead) : "memory");
 }
-__device__ __forceinline__ unsigned gp_elect() {
-    unsigned r;
-    asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}\n" : "=r"(r));
-    return r;
-}
 __device__ __forceinline__ void gp_ld32(unsigned taddr, unsigned (&r)[32]) {
     asm volatile(
         "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
@@ -140,10 +135,6 @@ __host__ __device__ constexpr unsigned gp_idesc(int m, int n) {
 __device__ __forceinline__ void gp_cluster_sync() {
     asm volatile("barrier.cluster.arrive.release.aligned;\n" ::: "memory");
     asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory");
-}
-__device__ __forceinline__ float gp_silu(float g) { return g / (1.0f + expf(-g)); }
-__device__ __forceinline__ float gp_gelu_tanh(float g) {
-    return 0.5f * g * (1.0f + tanhf(0.7978845608028654f * (g + 0.044715f * g * g * g)));
 }
 
 // The work of one cluster, in order: whole tiles c, c + C, ... below `whole` (a multiple of C), then the
@@ -273,7 +264,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GP_THREADS, 1) linea
         // ---- product issuer (first CTA of the pair): all lanes walk the stages, one issues.  In a branch for one lane a wait
         // keeps the tensor pipe idle for about 250 clocks (the operands have to be moved to where the instruction reads them) ----
         if (rank == 0) {
-            const unsigned lead = gp_elect();
+            const unsigned lead = elect_one();
             const unsigned long long ad0 = gp_desc(a_s), bd0 = gp_desc(b_s);
             int it = 0;
             bool ok = true;
@@ -445,7 +436,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GP_THREADS, 1) linea
                         const float gate = __bfloat162float(__float2bfloat16_rn(__uint_as_float(g[e])));
                         const float upv = __bfloat162float(__float2bfloat16_rn(__uint_as_float(up[e])));
                         if (MODE == 4) v[e] = clamped_swish(gate, upv, limit, CLAMPED_SWISH_ALPHA, 1.0f);
-                        else v[e] = (MODE == 3 ? gp_gelu_tanh(gate) : gp_silu(gate)) * upv;
+                        else v[e] = (MODE == 3 ? gelu_tanh(gate) : silu(gate)) * upv;
                     }
                 } else {
                     unsigned r[32];

@@ -51,10 +51,6 @@ __device__ __forceinline__ void gm_mma(float (&c)[4], const unsigned (&a)[4], un
 // 16-byte chunk `chunk` (of 8) of row `row` in a [rows][64] piece
 __device__ __forceinline__ bf16* gm_at(bf16* base, int row, int chunk) { return base + row * GM_SUB + ((chunk ^ (row & 7)) << 3); }
 
-__device__ __forceinline__ float gm_gated(float g, float u, int act, float limit) {
-    if (act == 2) return clamped_swish(g, u, limit, CLAMPED_SWISH_ALPHA, 1.0f);
-    return (act == 1 ? 0.5f * g * (1.0f + tanhf(0.7978845608028654f * (g + 0.044715f * g * g * g))) : g / (1.0f + expf(-g))) * u;
-}
 
 // Where the rows come from: x (bfloat16 [M, K]), or h, pending and the norm's weight g.
 struct GmRows {
@@ -240,7 +236,7 @@ __global__ void __launch_bounds__(GM_THREADS, HELD == 8 ? 2 : 3) linear_small_ke
             return v;
         };
         float out = sum_of(o);
-        if constexpr (GATED) out = gm_gated(to_f32(from_f32<bf16>(out)), to_f32(from_f32<bf16>(sum_of(SUMS + o))), act, limit);
+        if constexpr (GATED) out = gated(to_f32(from_f32<bf16>(out)), to_f32(from_f32<bf16>(sum_of(SUMS + o))), act, limit);
         y[static_cast<size_t>(tok) * N + f] = from_f32<TO>(out);
     }
     if (!landed) {

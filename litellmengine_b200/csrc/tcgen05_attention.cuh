@@ -64,15 +64,10 @@ __device__ __forceinline__ void t5_mma_ts(unsigned d_tmem, unsigned a_tmem, unsi
                  " tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}\n" ::
                      "r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
 }
-// The same for a warp that goes through its loop with all lanes together, `lead` (t5_elect) set in one of them: operands that
+// The same for a warp that goes through its loop with all lanes together, `lead` (elect_one) set in one of them: operands that
 // all lanes hold alike stay in the registers that these instructions read, and a wait in front of a product costs 15 to 80
 // clocks of the tensor pipe's time.  With the loop inside a branch for one lane it costs 250 (four products of 64 clocks behind
 // each wait: 68 clocks a product against 127).
-__device__ __forceinline__ unsigned t5_elect() {
-    unsigned r;
-    asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}\n" : "=r"(r));
-    return r;
-}
 __device__ __forceinline__ void t5_mma_ss_lead(unsigned lead, unsigned d_tmem, unsigned long long a_desc, unsigned long long b_desc,
                                                unsigned idesc, unsigned accumulate) {
     asm volatile("{\n .reg .pred p, q;\n setp.ne.b32 p, %4, 0;\n setp.ne.b32 q, %5, 0;\n"
