@@ -2226,9 +2226,10 @@ PAIR_HEADS_MIN_ROWS = 600
 def heads_pay(rows: int, weight: torch.Tensor) -> bool:
     """Whether a layer whose q/k/v product `heads_product` takes is faster with it.  It saves a kernel that reads the float32 product again,
     rows * N values of it; it loses what the clusters idle at the end of its tiles, which grows with K.  So there is a least number of
-    values, and a least share of the clusters' time that the tiles fill: 1 / (1.05 + 694 / K), 0.75 for a K of up to 2,500.  Whole
-    layers, us with it and with the library product and the other kernel (share): 6,144 x 4,096 600 tokens (0.76) 75, 69; 768 (0.97) 82, 82;
-    1,024 (0.86) 102, 100; 1,280 (0.81) 127, 127; 1,536 (0.97) 135, 140; 1,600 (0.81) 154, 149; 2,048 (0.86) 179, 191; 2,900 (0.92) 276, 301;
+    values, and a least share of the clusters' time that the tiles fill: 1 / (1.05 + 694 / K), at least 0.75 and, from 11 million values on, at
+    most 0.79.  Whole layers, us with it and with the library product and the other kernel (share): 6,144 x 4,096 600 tokens (0.76) 75, 69; 768 (0.97) 82, 82;
+    1,024 (0.86) 102, 100; 1,280 (0.81) 127, 127; 1,536 (0.97) 135, 140; 1,600 (0.81) 154, 149; 1,820 (0.77) 169, 166; 1,880
+    (0.79) 167, 171; 2,048 (0.86) 179, 191; 2,900 (0.92) 276, 301;
     6,144 x 2,560 1,024 (0.86) 80.4, 79.5; 1,280 (0.81) 94, 97; 2,048 137, 148; 4,096 x 2,048 768 (0.65) 52.6, 51.3; 900 (0.76) 57.3, 57.7;
     1,024 (0.86) 58.5, 60.2; 1,700 (0.72) 87, 85; 2,048 97, 101; 4,096 x 1,024 900 (0.76) 48.6, 49.6; 2,048 83, 85; 2,048 x 1,024 1,024 (0.86)
     47.0, 46.5; 1,800 (0.76) 58, 61; 7,168 x 5,120 1,100 (0.81) 185, 182; 1,536 (0.91) 261, 277; 10,240 x 5,120 1,100 (0.77) 202, 200; 1,280 (0.90) 230, 260."""
@@ -2238,7 +2239,8 @@ def heads_pay(rows: int, weight: torch.Tensor) -> bool:
     if rows * n < (3_500_000 if k <= 2048 else 7_800_000):
         return False
     filled = _fn("gemm_pair_tcgen05", "llm_linear_pair_efficiency", [c_int, c_int, c_int, c_int])(rows, n, k, 0)
-    return filled >= max(750.0, 1000.0 / (1.05 + 694.0 / k))
+    need = 1000.0 / (1.05 + 694.0 / k)
+    return filled >= max(750.0, min(need, 790.0) if rows * n >= 11_000_000 else need)
 
 
 def heads_product(x: torch.Tensor, weight: torch.Tensor, cache: Optional[torch.Tensor], d: int) -> bool:
