@@ -179,7 +179,8 @@ __global__ void delta_prepare_kernel(const DeltaShape s, const float* __restrict
 // its loads four times in a row, and a block at a portion's start reads the ring or zeros one value after another.  Here rows come from
 // wherever they are: a block whose tokens belong to several portions passes once for each.
 // Latency bounds it (a warp has seven rows to wait for; three blocks of 80 registers an SM).  1,700 tokens of three portions, 16 heads of
-// 128, everything cold: 43 -> 33 us.  Two blocks of 96 registers 38; four 38; rows fetched before the portion is known 37 (spills).
+// 128, everything cold: 43 -> 33 us; layers with eight tokens a chunk: 2 x 1,000 tokens 402 -> 392, 4 x 500 363 -> 354, 4 x 260 215 -> 205, 8 heads
+// 2 x 1,000 248 -> 235, 8 x 1,000 621 -> 605, 9 x 900 594 -> 578.  Two blocks of 96 registers 38; four 38; rows fetched before the portion is known 37 (spills).
 __global__ void __launch_bounds__(DP_WARPS * 32, 3) delta_prepare_fours_kernel(
     const DeltaShape s, const float* __restrict__ proj, const float* __restrict__ conv_w, const float* __restrict__ state,
     const int32_t* __restrict__ positions, const int32_t* __restrict__ token_entry, const int32_t* __restrict__ entry_slot,
