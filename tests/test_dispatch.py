@@ -132,6 +132,7 @@ def test_a_mixer_that_mixes_in_its_own_way_is_asked_to(monkeypatch):
 
     spec = MixerSpec("gated_attention", num_heads=1, num_kv_heads=1, head_dim=128, position=PositionSpec(kind="none"))
     monkeypatch.setattr(ops, "heads_product", lambda *a: True)
+    monkeypatch.setattr(ops, "heads_pay", lambda *a: True)
     monkeypatch.setattr(ops, "linear", lambda x, w, **k: x.float() @ w.float().t())
     x, ctx = torch.ones(4, 8, dtype=torch.bfloat16), types.SimpleNamespace(batch=types.SimpleNamespace(tables={}, positions=None, token_entry=None,
               entry_slot=None), writes_cache=True, cache=torch.zeros(1), block_table=None, page_size=16, status=None)
