@@ -2059,29 +2059,39 @@ def linear_small(x, weight: torch.Tensor, out_dtype: torch.dtype, activation: Op
     return out
 
 
-# Rows that take `linear_mid`.  Up to 32 it was level with the library product (below them `linear_skinny` is faster) or faster at every size tried
-# from 1,024 x 3,072 to 151,936 x 2,048 (the worst, 4,096 x 2,048 at 32 rows: 6.3 us against 6.2), and faster than `linear_skinny` where that took so many
-# (2,048 x 6,144: 7.7 against 9.6).  With up to 48 rows the parts' sums weigh more: wide products of a short K stay with the library
-# (40 rows, 4,096 x 2,048: 6.7, 6.3; 5,120 x 2,048: 7.3, 6.8) unless they need no parts (52,224 x 2,048: 40.5, 41.8).
+# Rows that may take `linear_mid` (fewer: `linear_skinny` is faster), measured inside layers of width 1,024 to 5,120 with it and without, the
+# layers' other products as they are.  Up to 32 rows: small products (else `linear_skinny`'s) make a layer 2 to 3 us shorter on average, others
+# (else the library's) 2 in attention, 4 in MLPs and 8 in the delta rule (the worst of 243: 1.8 of 65 longer).  Inputs
+# of the other branch mixers that are not small make a layer up to 5.4 us of 45 longer (8,192 x 4,096; 6,144 x 3,072: 1.6 to 2.5 of 34 to 39), and
+# so do their outputs behind a library product (4,096 x 4,096 to 6,144: up to 2.4 of 45, 5,120 x 5,120 3 shorter): both stay with the library.
+# With up to 48 rows the parts' sums weigh more.  Plain: a K below min(N, 4,096) stays with the library unless it needs no parts, one below 1,024
+# always (1,536 x 384: a layer of 38 us 1.2 longer), and the delta rule's outputs (4,096 x 4,096: 0.4 to 1.0 of 97 to 112 longer).  Gated: two parts of a
+# K of 1,025 to 2,048 (7,168 x 1,536: 1.6 to 1.8 of 20 longer; of 1,024 0.2 to 0.4 shorter, of 2,560 level) and eight parts of more than 2,048
+# (2,048 x 2,560: 0.7 to 0.9 of 14 longer; of 2,048 1.4 shorter).
 MID_ROWS = range(SKINNY_MAX_ROWS + 1, 49)
 _mid_products: Dict[tuple, bool] = {}
 
 
-def mid_product(x, weight: torch.Tensor, out_dtype: torch.dtype, gated: bool = False) -> bool:
-    """Whether `linear_mid` is the faster way for these operands (gated: weight is [gate; up])."""
+def mid_product(x, weight: torch.Tensor, out_dtype: torch.dtype, gated: bool = False, large_rows: int = MID_ROWS[-1]) -> bool:
+    """Whether `linear_mid` is the faster way for these operands (gated: weight is [gate; up]); beyond `large_rows` rows only for
+    products that `linear_skinny` would take."""
     if not (x.shape[0] in MID_ROWS and x.is_cuda and x.dtype == torch.bfloat16 and weight.dtype == torch.bfloat16
             and out_dtype in (torch.float32, torch.bfloat16) and x.is_contiguous() and weight.is_contiguous()
             and x.shape[1] == weight.shape[1] and x.data_ptr() % 16 == 0 and weight.data_ptr() % 16 == 0):
         return False
-    n, k = weight.shape
-    key = (x.shape[0] <= 32, n, k, gated)
+    (n, k), rows = weight.shape, x.shape[0]
+    if rows > large_rows and not (rows <= SKINNY_SMALL_MAX_ROWS and skinny_small(n, k)):
+        return False
+    key = (rows <= 32, n, k, gated)
     got = _mid_products.get(key)
     if got is None:
         got = not gated or n % 2 == 0
         n = n // 2 if gated else n
-        got = got and bool(_fn("gemm_mid_tcgen05", "llm_linear_mid_supported", [c_int] * 4)(x.shape[0], n, k, int(gated)))
-        if got and x.shape[0] > 32 and not gated:
-            got = k >= min(n, 4096) or _fn("gemm_mid_tcgen05", "llm_linear_mid_parts", [c_int] * 3)(n, k, 0) == 1
+        got = got and bool(_fn("gemm_mid_tcgen05", "llm_linear_mid_supported", [c_int] * 4)(rows, n, k, int(gated)))
+        if got and rows > 32:
+            parts = _fn("gemm_mid_tcgen05", "llm_linear_mid_parts", [c_int] * 3)(n, k, int(gated))
+            got = (not (1024 < k <= 2048 if parts == 2 else k > 2048 and parts == 8) if gated
+                   else k >= 1024 and (k >= min(n, 4096) or parts == 1))
         _mid_products[key] = got
     return got
 
@@ -2347,14 +2357,14 @@ def linear_f32_tcgen05(x: torch.Tensor, weight: torch.Tensor) -> torch.Tensor:
 
 
 def linear(x: torch.Tensor, weight: torch.Tensor, out_dtype: Optional[torch.dtype] = None,
-           partials_ok: bool = False):
+           partials_ok: bool = False, large_mid_rows: int = MID_ROWS[-1]):
     """x [T, K] @ weight[N, K]^T.  Up to 16 bfloat16 rows with weights that the SMs hold all at once go to `linear_small` (which also
     takes `PendingRows`); else up to 16 bfloat16 rows (decode steps; up to 32 for small products that `linear_mid` does not take) go through the
     engine's own weight-streaming kernel: alone it is level with the library for N = 4096..24576 and
     faster for K = 12288 (32 us against 36) and N = 151936 (203 against 218), and in a step it
     starts fetching weights while the kernel before it drains (a whole decode step of the
     Qwen3-8B shape at batch 8: 4.35 ms against 4.77 with the library products).  17 to 48 bfloat16 rows: `linear_mid`, by the rule of
-    `mid_product`.  Everything else
+    `mid_product` (`large_mid_rows`: up to how many the caller's products gain from it that are not small).  Everything else
     goes through the library matrix product (under `LLM_PAIR=all`, prompt portions take the paired tcgen05
     product `linear_pair`; by default only the gate/up product does, through `linear_silu_mul`) (the reference uses cuBLAS for all its products,
     src/layers/linear.cu:169-215).  bfloat16 operands accumulate in float32; a float32 weight
@@ -2368,7 +2378,7 @@ def linear(x: torch.Tensor, weight: torch.Tensor, out_dtype: Optional[torch.dtyp
     if (x.dtype == torch.bfloat16 and x.is_contiguous() and x.data_ptr() % 16 == 0 and (out_dtype or x.dtype) in (torch.float32, torch.bfloat16)
             and small_product(rows, weight)):
         return linear_small(x, weight, out_dtype or x.dtype)
-    if mid_product(x, weight, out_dtype or x.dtype):
+    if mid_product(x, weight, out_dtype or x.dtype, large_rows=large_mid_rows):
         return linear_mid(x, weight, out_dtype or x.dtype)
     if (x.dtype == torch.bfloat16 and weight.dtype == torch.bfloat16 and x.shape[1] % 8 == 0 and weight.data_ptr() % 16 == 0
             and rows >= 1 and (rows <= SKINNY_MAX_ROWS

@@ -224,16 +224,18 @@ class BranchMixer:
     out_width = 0
     w_in: Optional[torch.Tensor] = None
     w_o: Optional[torch.Tensor] = None
+    large_in_rows, large_out_rows = 0, 0       # rows up to which `ops.linear_mid` gains in products that are not small (see `ops.MID_ROWS`)
 
     def mix(self, proj: torch.Tensor, col0: int, ctx: StageContext, out: torch.Tensor, out_col0: int,
             out_scale: float) -> None:
         raise NotImplementedError
 
     def forward(self, x: torch.Tensor, ctx: StageContext):
-        proj = ops.linear(x, self.w_in, out_dtype=torch.float32)
+        proj = ops.linear(x, self.w_in, out_dtype=torch.float32, large_mid_rows=self.large_in_rows)
         out = torch.empty((x.shape[0], self.out_width), dtype=self.dtype, device=x.device)
         self.mix(proj, 0, ctx, out, 0, 1.0)
-        return ops.linear(out, self.w_o, out_dtype=torch.float32, partials_ok=getattr(ctx, "partials_ok", False))
+        return ops.linear(out, self.w_o, out_dtype=torch.float32, partials_ok=getattr(ctx, "partials_ok", False),
+                          large_mid_rows=self.large_out_rows)
 
     def fused_by_parent(self) -> None:
         """A parent holds the fused matrices now; the branch keeps no copies."""

@@ -32,6 +32,7 @@ class DeltaRuleMixer(BranchMixer):
     graph_safe = True            # kernels on the current stream only; their grids follow the step's entries,
     any_division_safe = False    # and which kernels they are is part of a graph's key (see graph_variant)
 
+    large_in_rows, large_out_rows = 48, 32
     PADDED = (32, 64, 128, 256)  # what the kernels are instantiated for
 
     _DEFAULT_NAMES = {"q": "q_proj.weight", "k": "k_proj.weight", "v": "v_proj.weight", "o": "o_proj.weight",

@@ -145,6 +145,26 @@ def test_a_mixer_that_mixes_in_its_own_way_is_asked_to(monkeypatch):
         assert torch.equal(m.forward(x, ctx), torch.full((4, 1), 128 * value)) and len(asked) == times
 
 
+def test_branch_mixers_say_where_middling_products_gain(monkeypatch):
+    from litellmengine_b200.parts.attention import BranchMixer, GatedAttentionMixer
+    from litellmengine_b200.parts.delta_rule import DeltaRuleMixer
+    from litellmengine_b200.parts.linear_attention import GatedLinearAttention, RetentionMixer
+    from litellmengine_b200.parts.parallel import ParallelMixer
+    asked = []
+    monkeypatch.setattr(ops, "linear", lambda x, w, large_mid_rows, **k: asked.append(large_mid_rows) or torch.zeros(x.shape[0], w.shape[0]))
+    for cls, rows in ((GatedAttentionMixer, [0, 0]), (GatedLinearAttention, [0, 0]), (RetentionMixer, [0, 0]), (DeltaRuleMixer, [48, 32])):
+        m = cls.__new__(cls)
+        m.w_in, m.w_o, m.out_width, m.dtype = torch.ones(6, 8), torch.ones(8, 4), 4, torch.bfloat16
+        m.mix = lambda *a: None
+        BranchMixer.forward(m, torch.ones(20, 8), types.SimpleNamespace())
+        assert asked == rows, cls
+        asked.clear()
+    m = ParallelMixer.__new__(ParallelMixer)
+    m.w_in, m.w_o, m.dtype, m.branches, m.scales, m.in_cols, m.out_cols = torch.ones(6, 8), torch.ones(8, 4), torch.bfloat16, [], [], [], []
+    m.forward(torch.ones(20, 8), types.SimpleNamespace())
+    assert asked == [0, 0]
+
+
 def test_tables_of_angles_go_by_the_spec(monkeypatch):
     """Layers of equal specs share a step's table, others do not, and a spec may hold its numbers in a list."""
     from litellmengine_b200.config.specs import MixerSpec
