@@ -2357,9 +2357,9 @@ def linear_f32_tcgen05(x: torch.Tensor, weight: torch.Tensor) -> torch.Tensor:
 
 
 def linear(x: torch.Tensor, weight: torch.Tensor, out_dtype: Optional[torch.dtype] = None,
-           partials_ok: bool = False, large_mid_rows: int = MID_ROWS[-1]):
+           partials_ok: bool = False, large_mid_rows: int = MID_ROWS[-1], small: bool = True):
     """x [T, K] @ weight[N, K]^T.  Up to 16 bfloat16 rows with weights that the SMs hold all at once go to `linear_small` (which also
-    takes `PendingRows`); else up to 16 bfloat16 rows (decode steps; up to 32 for small products that `linear_mid` does not take) go through the
+    takes `PendingRows`) unless `small` says that the caller loses by it; else up to 16 bfloat16 rows (decode steps; up to 32 for small products that `linear_mid` does not take) go through the
     engine's own weight-streaming kernel: alone it is level with the library for N = 4096..24576 and
     faster for K = 12288 (32 us against 36) and N = 151936 (203 against 218), and in a step it
     starts fetching weights while the kernel before it drains (a whole decode step of the
@@ -2375,7 +2375,7 @@ def linear(x: torch.Tensor, weight: torch.Tensor, out_dtype: Optional[torch.dtyp
         return linear_small(x, weight, out_dtype or x.dtype)
     _dev(x, weight)
     rows = x.shape[0]
-    if (x.dtype == torch.bfloat16 and x.is_contiguous() and x.data_ptr() % 16 == 0 and (out_dtype or x.dtype) in (torch.float32, torch.bfloat16)
+    if (small and x.dtype == torch.bfloat16 and x.is_contiguous() and x.data_ptr() % 16 == 0 and (out_dtype or x.dtype) in (torch.float32, torch.bfloat16)
             and small_product(rows, weight)):
         return linear_small(x, weight, out_dtype or x.dtype)
     if mid_product(x, weight, out_dtype or x.dtype, large_rows=large_mid_rows):

@@ -33,6 +33,14 @@ class DeltaRuleMixer(BranchMixer):
     any_division_safe = False    # and which kernels they are is part of a graph's key (see graph_variant)
 
     large_in_rows, large_out_rows = 48, 32
+
+    @staticmethod
+    def small_gains(rows: int, k: int) -> bool:
+        """As `BranchMixer.small_gains`; this layer's kernels leave the product's less room.  Up to 8 rows K 512 to 1,536 mostly 0.5 to 4 us of
+        13 to 20 shorter, 1,792 1 to 3.6 longer, 2,048 up to 2 longer with up to 4 rows; 9 to 16 rows K 640 to 1,152 1 to 5 shorter, 512 with
+        N 1,668 1 to 2.8 longer, 1,280 and 1,536 0.1 to 2, 2,560 2 to 5."""
+        return k <= 1536 if rows <= 8 else k <= 1152 and not 384 < k <= 512
+
     PADDED = (32, 64, 128, 256)  # what the kernels are instantiated for
 
     _DEFAULT_NAMES = {"q": "q_proj.weight", "k": "k_proj.weight", "v": "v_proj.weight", "o": "o_proj.weight",

@@ -151,7 +151,7 @@ def test_branch_mixers_say_where_middling_products_gain(monkeypatch):
     from litellmengine_b200.parts.linear_attention import GatedLinearAttention, RetentionMixer
     from litellmengine_b200.parts.parallel import ParallelMixer
     asked = []
-    monkeypatch.setattr(ops, "linear", lambda x, w, large_mid_rows, **k: asked.append(large_mid_rows) or torch.zeros(x.shape[0], w.shape[0]))
+    monkeypatch.setattr(ops, "linear", lambda x, w, large_mid_rows, small=True, **k: asked.append(large_mid_rows) or torch.zeros(x.shape[0], w.shape[0]))
     for cls, rows in ((GatedAttentionMixer, [0, 0]), (GatedLinearAttention, [0, 0]), (RetentionMixer, [0, 0]), (DeltaRuleMixer, [48, 32])):
         m = cls.__new__(cls)
         m.w_in, m.w_o, m.out_width, m.dtype = torch.ones(6, 8), torch.ones(8, 4), 4, torch.bfloat16
@@ -163,6 +163,24 @@ def test_branch_mixers_say_where_middling_products_gain(monkeypatch):
     m.w_in, m.w_o, m.dtype, m.branches, m.scales, m.in_cols, m.out_cols = torch.ones(6, 8), torch.ones(8, 4), torch.bfloat16, [], [], [], []
     m.forward(torch.ones(20, 8), types.SimpleNamespace())
     assert asked == [0, 0]
+
+
+@pytest.mark.parametrize("rows,k,delta,other", [(1, 1536, True, True), (8, 1544, False, True), (1, 2048, False, True), (8, 4096, False, True),
+                                                (9, 384, True, True), (9, 512, False, True), (16, 520, True, True), (16, 1152, True, True),
+                                                (9, 1160, False, True), (16, 2040, False, True), (9, 2048, False, False), (16, 4096, False, False)])
+def test_branch_mixers_say_where_small_products_gain(monkeypatch, rows, k, delta, other):
+    from litellmengine_b200.parts.delta_rule import DeltaRuleMixer
+    from litellmengine_b200.parts.linear_attention import GatedLinearAttention
+    from litellmengine_b200.parts.parallel import ParallelMixer
+    asked = []
+    monkeypatch.setattr(ops, "linear", lambda x, w, small=True, **k: asked.append(small) or torch.zeros(x.shape[0], w.shape[0]))
+    for cls, want in ((GatedLinearAttention, other), (DeltaRuleMixer, delta), (ParallelMixer, other)):
+        m = cls.__new__(cls)
+        m.w_in, m.w_o, m.out_width, m.dtype = torch.ones(6, 8), torch.ones(8, 4), 4, torch.bfloat16
+        m.branches, m.scales, m.in_cols, m.out_cols, m.mix = [], [], [], [], lambda *a: None
+        m.forward(torch.ones(rows, k), types.SimpleNamespace())
+        assert asked == [want, True], cls
+        asked.clear()
 
 
 def test_tables_of_angles_go_by_the_spec(monkeypatch):
