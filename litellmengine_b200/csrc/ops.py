@@ -1526,6 +1526,15 @@ def decode_makes_its_rows(qkv, cache: torch.Tensor, d: int, group: int, page_siz
                 _ptr(cache), cache.shape[0], cache.shape[2], d, group, page_size)))
 
 
+def rows_worth_making(qkv, group: int) -> bool:
+    """Whether a step's rows are made in the attention kernel where that can make them.  With k-splits pending a row's CTAs, one to a key head
+    and split, add them up, each for its heads; the kernel of its own does that once.  Steps of 4 layers, time
+    with and without, at contexts of 60 to 4,000: groups of 4, width 2,560 and 4,096, up to 4 splits, 1 to 8 rows 0.97 to 1.02, up to 6 and
+    up to 300 1.00 to 1.02, 9 to 16 rows 0.97 to 1.00; groups of 2, width 2,048, 9 rows 0.98 to 1.02, 12 0.98 to 1.01, 16 0.97 to 1.00.
+    Without pending splits 0.94 to 1.01 (1 to 40 rows, width 1,024 to 4,096)."""
+    return not isinstance(qkv, PartialSum) or (qkv.parts.shape[1] > 8 and qkv.parts.shape[1] * group >= 32)
+
+
 def paged_attention_decode_made(qkv, cache: torch.Tensor, positions, token_entry, entry_slot, block_table: torch.Tensor, q_norm_w, k_norm_w,
                                 eps: float, inv_freq, angles: Optional[torch.Tensor], nq: int, nkv: int, d: int, page_size: int,
                                 scale: float, num_splits: int, status: torch.Tensor) -> torch.Tensor:

@@ -180,6 +180,7 @@ class AttentionMixer:
             work = b.preludes.get(AttentionWork.name)
             if (has_kv and self.dtype == torch.bfloat16 and self.span is None and work is not None and not getattr(b, "any_division", False)
                     and work.num_decode == b.num_tokens and not work.num_prefill_tiles and (rot is None or rot.rotary_dim == self.d)
+                    and ops.rows_worth_making(qkv, self.nq // self.nkv)
                     and ops.decode_makes_its_rows(qkv, cache, self.d, self.nq // self.nkv, ctx.page_size,
                                                   splits := decode_key_splits(self.device, b.num_tokens, self.nkv, decode_reach(b, None)))):
                 # a step of single tokens: norms, rotation and cache write inside the attention kernel too

@@ -183,6 +183,13 @@ def test_branch_mixers_say_where_small_products_gain(monkeypatch, rows, k, delta
         asked.clear()
 
 
+@pytest.mark.parametrize("rows,group,pending,worth", [(1, 4, False, True), (16, 1, False, True), (8, 4, True, False), (8, 16, True, False),
+                                                      (9, 4, True, True), (9, 3, True, False), (15, 2, True, False), (16, 2, True, True)])
+def test_rows_are_made_in_the_attention_kernel_where_that_pays(rows, group, pending, worth):
+    qkv = torch.zeros(rows, 384)
+    assert ops.rows_worth_making(ops.PartialSum(torch.stack([qkv, qkv])) if pending else qkv, group) == worth
+
+
 def test_tables_of_angles_go_by_the_spec(monkeypatch):
     """Layers of equal specs share a step's table, others do not, and a spec may hold its numbers in a list."""
     from litellmengine_b200.config.specs import MixerSpec
