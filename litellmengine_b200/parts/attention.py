@@ -227,19 +227,16 @@ class BranchMixer:
     w_o: Optional[torch.Tensor] = None
     large_in_rows, large_out_rows = 0, 0       # rows up to which `ops.linear_mid` gains in products that are not small (see `ops.MID_ROWS`)
 
-    @staticmethod
-    def small_gains(rows: int, k: int) -> bool:
-        """Whether an input product of `rows` rows over k values gains from `ops.linear_small` where that takes it.  Layers, us, with it and with
-        the streaming product, gated linear attention: 9 to 16 rows, K 2,048, N 2,112 2 to 5 of 25 longer; K below that 0 to 5 shorter, as up to
-        8 rows with any."""
-        return rows <= 8 or k < 2048
+    def small_gains(self, rows: int) -> bool:
+        """Whether an input product of `rows` rows gains from `ops.linear_small` where that takes it."""
+        return True
 
     def mix(self, proj: torch.Tensor, col0: int, ctx: StageContext, out: torch.Tensor, out_col0: int,
             out_scale: float) -> None:
         raise NotImplementedError
 
     def forward(self, x: torch.Tensor, ctx: StageContext):
-        proj = ops.linear(x, self.w_in, out_dtype=torch.float32, large_mid_rows=self.large_in_rows, small=self.small_gains(*x.shape))
+        proj = ops.linear(x, self.w_in, out_dtype=torch.float32, large_mid_rows=self.large_in_rows, small=self.small_gains(x.shape[0]))
         out = torch.empty((x.shape[0], self.out_width), dtype=self.dtype, device=x.device)
         self.mix(proj, 0, ctx, out, 0, 1.0)
         return ops.linear(out, self.w_o, out_dtype=torch.float32, partials_ok=getattr(ctx, "partials_ok", False),

@@ -34,12 +34,13 @@ class DeltaRuleMixer(BranchMixer):
 
     large_in_rows, large_out_rows = 48, 32
 
-    @staticmethod
-    def small_gains(rows: int, k: int) -> bool:
-        """As `BranchMixer.small_gains`; this layer's kernels leave the product's less room.  Up to 8 rows K 512 to 1,536 mostly 0.5 to 4 us of
-        13 to 20 shorter, 1,792 1 to 3.6 longer, 2,048 up to 2 longer with up to 4 rows; 9 to 16 rows K 640 to 1,152 1 to 5 shorter, 512 with
-        N 1,668 1 to 2.8 longer, 1,280 and 1,536 0.1 to 2, 2,560 2 to 5."""
-        return k <= 1536 if rows <= 8 else k <= 1152 and not 384 < k <= 512
+    def small_gains(self, rows: int) -> bool:
+        """As `BranchMixer.small_gains`.  Decode steps of 4 layers with feed-forwards, us, with it and with the streaming product, input K and N: 1,024,
+        3,208, 1 / 8 / 16 requests 112, 129 / 121, 138 / 154, 170; 1,536, 2,438 153, 154 / 150, 172 / 193, 204; 2,048, 3,208 176, 182 / 194, 196.  Not with
+        9 to 16 rows of up to 512 values, whose sums the streaming product leaves whole as well (512, 1,668, 12 / 16 requests 136, 127 / 137, 130), and not
+        with wide rows and an odd N (1,792, 2,823, 8 requests 194, 174; a layer alone 2 to 3.6 of 20 longer; 2,560, 2,053 up to 5)."""
+        n, k = self.w_in.shape
+        return not (rows > 8 and 384 < k <= 512) and not (n % 2 and k > 1280)
 
     PADDED = (32, 64, 128, 256)  # what the kernels are instantiated for
 

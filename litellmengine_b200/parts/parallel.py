@@ -80,8 +80,7 @@ class ParallelMixer:
         return tuple(b.graph_variant(batch, padded) for b in self.branches if hasattr(b, "graph_variant"))
 
     def forward(self, x: torch.Tensor, ctx: StageContext):
-        proj = ops.linear(x, self.w_in, out_dtype=torch.float32, large_mid_rows=BranchMixer.large_in_rows,
-                          small=BranchMixer.small_gains(*x.shape))
+        proj = ops.linear(x, self.w_in, out_dtype=torch.float32, large_mid_rows=BranchMixer.large_in_rows)
         out = torch.empty((x.shape[0], self.w_o.shape[1]), dtype=self.dtype, device=x.device)
         for b, scale, c_in, c_out in zip(self.branches, self.scales, self.in_cols, self.out_cols):
             b.mix(proj, c_in, ctx, out, c_out, scale)

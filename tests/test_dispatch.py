@@ -165,19 +165,16 @@ def test_branch_mixers_say_where_middling_products_gain(monkeypatch):
     assert asked == [0, 0]
 
 
-@pytest.mark.parametrize("rows,k,delta,other", [(1, 1536, True, True), (8, 1544, False, True), (1, 2048, False, True), (8, 4096, False, True),
-                                                (9, 384, True, True), (9, 512, False, True), (16, 520, True, True), (16, 1152, True, True),
-                                                (9, 1160, False, True), (16, 2040, False, True), (9, 2048, False, False), (16, 4096, False, False)])
-def test_branch_mixers_say_where_small_products_gain(monkeypatch, rows, k, delta, other):
+@pytest.mark.parametrize("rows,n,k,small", [(1, 3208, 2048, True), (16, 3208, 2048, True), (8, 1668, 512, True), (9, 1668, 512, False), (16, 1024, 392, False),
+                                            (16, 1024, 384, True), (9, 1024, 520, True), (1, 2053, 1280, True), (1, 2053, 1288, False), (16, 2054, 1288, True)])
+def test_the_delta_rule_says_where_small_products_gain(monkeypatch, rows, n, k, small):
     from litellmengine_b200.parts.delta_rule import DeltaRuleMixer
     from litellmengine_b200.parts.linear_attention import GatedLinearAttention
-    from litellmengine_b200.parts.parallel import ParallelMixer
     asked = []
     monkeypatch.setattr(ops, "linear", lambda x, w, small=True, **k: asked.append(small) or torch.zeros(x.shape[0], w.shape[0]))
-    for cls, want in ((GatedLinearAttention, other), (DeltaRuleMixer, delta), (ParallelMixer, other)):
+    for cls, want in ((GatedLinearAttention, True), (DeltaRuleMixer, small)):
         m = cls.__new__(cls)
-        m.w_in, m.w_o, m.out_width, m.dtype = torch.ones(6, 8), torch.ones(8, 4), 4, torch.bfloat16
-        m.branches, m.scales, m.in_cols, m.out_cols, m.mix = [], [], [], [], lambda *a: None
+        m.w_in, m.w_o, m.out_width, m.dtype, m.mix = torch.ones(n, k), torch.ones(8, 4), 4, torch.bfloat16, lambda *a: None
         m.forward(torch.ones(rows, k), types.SimpleNamespace())
         assert asked == [want, True], cls
         asked.clear()
