@@ -2070,13 +2070,12 @@ def linear_small(x, weight: torch.Tensor, out_dtype: torch.dtype, activation: Op
 
 # Rows that may take `linear_mid` (fewer: `linear_skinny` is faster), measured inside layers of width 1,024 to 5,120 with it and without, the
 # layers' other products as they are.  Up to 32 rows: small products (else `linear_skinny`'s) make a layer 2 to 3 us shorter on average, others
-# (else the library's) 2 in attention, 4 in MLPs and 8 in the delta rule (the worst of 243: 1.8 of 65 longer).  Inputs
-# of the other branch mixers that are not small make a layer up to 5.4 us of 45 longer (8,192 x 4,096; 6,144 x 3,072: 1.6 to 2.5 of 34 to 39), and
-# so do their outputs behind a library product (4,096 x 4,096 to 6,144: up to 2.4 of 45, 5,120 x 5,120 3 shorter): both stay with the library.
+# (else the library's) 2 in attention, 4 in MLPs and 8 in the delta rule (the worst of 243: 1.8 of 65 longer).  Branch
+# mixers say for their products that are not small up to how many rows (see `BranchMixer.large_rows`).
 # With up to 48 rows the parts' sums weigh more.  Plain: a K below min(N, 4,096) stays with the library unless it needs no parts, one below 1,024
-# always (1,536 x 384: a layer of 38 us 1.2 longer), and the delta rule's outputs (4,096 x 4,096: 0.4 to 1.0 of 97 to 112 longer).  Gated: two parts of a
-# K of 1,025 to 2,048 (7,168 x 1,536: 1.6 to 1.8 of 20 longer; of 1,024 0.2 to 0.4 shorter, of 2,560 level) and eight parts of more than 2,048
-# (2,048 x 2,560: 0.7 to 0.9 of 14 longer; of 2,048 1.4 shorter).
+# always (1,536 x 384: a layer of 38 us 1.2 longer).  Gated ones all
+# come here: the few that are slower alone (7,168 x 1,536 1.6 to 1.8 of 20, 2,048 x 2,560 0.7 to 0.9 of 14) are faster in steps, where the
+# weights are fetched while a norm runs (4 layers of width 2,048 at 40 requests, with and without: 6,144 259, 278; 8,192 278, 291).
 MID_ROWS = range(SKINNY_MAX_ROWS + 1, 49)
 _mid_products: Dict[tuple, bool] = {}
 
@@ -2097,10 +2096,8 @@ def mid_product(x, weight: torch.Tensor, out_dtype: torch.dtype, gated: bool = F
         got = not gated or n % 2 == 0
         n = n // 2 if gated else n
         got = got and bool(_fn("gemm_mid_tcgen05", "llm_linear_mid_supported", [c_int] * 4)(rows, n, k, int(gated)))
-        if got and rows > 32:
-            parts = _fn("gemm_mid_tcgen05", "llm_linear_mid_parts", [c_int] * 3)(n, k, int(gated))
-            got = (not (1024 < k <= 2048 if parts == 2 else k > 2048 and parts == 8) if gated
-                   else k >= 1024 and (k >= min(n, 4096) or parts == 1))
+        if got and rows > 32 and not gated:
+            got = k >= 1024 and (k >= min(n, 4096) or _fn("gemm_mid_tcgen05", "llm_linear_mid_parts", [c_int] * 3)(n, k, 0) == 1)
         _mid_products[key] = got
     return got
 

@@ -225,7 +225,13 @@ class BranchMixer:
     out_width = 0
     w_in: Optional[torch.Tensor] = None
     w_o: Optional[torch.Tensor] = None
-    large_in_rows, large_out_rows = 0, 0       # rows up to which `ops.linear_mid` gains in products that are not small (see `ops.MID_ROWS`)
+
+    def large_rows(self, between: bool):
+        """Rows up to which the input and the output product gain from `ops.linear_mid` where they are not small; `between`: in a layer with
+        norms' kernels in front and behind, while which the weights are fetched already.  Alone gated linear attention's and gated attention's lose (8,192 x
+        4,096 5.4 us of 45; 6,144 x 3,072 1.6 to 2.5 of 34 to 39; output 4,096 x 4,096 up to 4 of 38); gated linear attention's in steps too (width
+        4,096, 40 requests 235 us, 244)."""
+        return 0, 0
 
     def small_gains(self, rows: int) -> bool:
         """Whether an input product of `rows` rows gains from `ops.linear_small` where that takes it."""
@@ -236,11 +242,12 @@ class BranchMixer:
         raise NotImplementedError
 
     def forward(self, x: torch.Tensor, ctx: StageContext):
-        proj = ops.linear(x, self.w_in, out_dtype=torch.float32, large_mid_rows=self.large_in_rows, small=self.small_gains(x.shape[0]))
+        partials_ok = getattr(ctx, "partials_ok", False)
+        rows_in, rows_out = self.large_rows(partials_ok or getattr(ctx, "residual", None) is not None)
+        proj = ops.linear(x, self.w_in, out_dtype=torch.float32, large_mid_rows=rows_in, small=self.small_gains(x.shape[0]))
         out = torch.empty((x.shape[0], self.out_width), dtype=self.dtype, device=x.device)
         self.mix(proj, 0, ctx, out, 0, 1.0)
-        return ops.linear(out, self.w_o, out_dtype=torch.float32, partials_ok=getattr(ctx, "partials_ok", False),
-                          large_mid_rows=self.large_out_rows)
+        return ops.linear(out, self.w_o, out_dtype=torch.float32, partials_ok=partials_ok, large_mid_rows=rows_out)
 
     def fused_by_parent(self) -> None:
         """A parent holds the fused matrices now; the branch keeps no copies."""
@@ -426,6 +433,11 @@ class GatedAttentionMixer(BranchMixer):
         n_dec = 0 if work is None else (work.padded_rows.shape[0] if padded else work.num_decode)
         n_tiles = 0 if work is None else (work.padded_tiles.shape[0] if padded else work.num_prefill_tiles)
         return decode_key_splits(self.device, n_dec, self.nkv, decode_reach(batch, self.span)) if n_dec and (self._wide or not n_tiles) else 0
+
+    def large_rows(self, between: bool):
+        """As `BranchMixer.large_rows`.  Decode steps of 4 layers, us, without and with both: width 4,096, 17 / 24 / 32 requests 430, 400 / 441, 417 / 456,
+        435, 48 474, 476; 5,120 552, 532 / 555, 543 / 573, 572; outputs of up to 3,072 values, 40 / 48 requests 356, 344 / 367, 357."""
+        return (32, 48 if self.w_o.shape[1] < 4096 else 32) if between else (0, 0)
 
     def forward(self, x: torch.Tensor, ctx: StageContext):
         s, b = self.spec, ctx.batch

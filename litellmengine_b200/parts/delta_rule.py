@@ -32,7 +32,12 @@ class DeltaRuleMixer(BranchMixer):
     graph_safe = True            # kernels on the current stream only; their grids follow the step's entries,
     any_division_safe = False    # and which kernels they are is part of a graph's key (see graph_variant)
 
-    large_in_rows, large_out_rows = 48, 32
+
+    def large_rows(self, between: bool):
+        """As `BranchMixer.large_rows`.  Decode steps of 4 layers, us, without and with it, width 4,096, 17 / 24 / 32 / 40 / 48 requests 427, 415 / 452,
+        441 / 527, 516 / 553, 538 / 563, 551.  A layer alone, up to 32 rows: decode 1 to 4 of 37 to 59 shorter, prompts 0.5 shorter to 2 of 50 longer; more:
+        decode 1 to 2 shorter, prompts 2 to 4 of 54 longer, but where the library reads odd rows (7,828 x 5,120) 36 to 40 of 78 to 120 shorter."""
+        return 48 if between or self.w_in.shape[0] % 8 else 32, 32
 
     def small_gains(self, rows: int) -> bool:
         """As `BranchMixer.small_gains`.  Decode steps of 4 layers with feed-forwards, us, with it and with the streaming product, input K and N: 1,024,

@@ -9,7 +9,6 @@ import torch
 from ..config.specs import MixerSpec
 from ..csrc import ops
 from ..weights.loader import ParamSpec
-from .attention import BranchMixer
 from .context import StageContext
 from .registry import lookup, register_mixer
 
@@ -80,9 +79,8 @@ class ParallelMixer:
         return tuple(b.graph_variant(batch, padded) for b in self.branches if hasattr(b, "graph_variant"))
 
     def forward(self, x: torch.Tensor, ctx: StageContext):
-        proj = ops.linear(x, self.w_in, out_dtype=torch.float32, large_mid_rows=BranchMixer.large_in_rows)
+        proj = ops.linear(x, self.w_in, out_dtype=torch.float32, large_mid_rows=0)
         out = torch.empty((x.shape[0], self.w_o.shape[1]), dtype=self.dtype, device=x.device)
         for b, scale, c_in, c_out in zip(self.branches, self.scales, self.in_cols, self.out_cols):
             b.mix(proj, c_in, ctx, out, c_out, scale)
-        return ops.linear(out, self.w_o, out_dtype=torch.float32, partials_ok=getattr(ctx, "partials_ok", False),
-                          large_mid_rows=BranchMixer.large_out_rows)
+        return ops.linear(out, self.w_o, out_dtype=torch.float32, partials_ok=getattr(ctx, "partials_ok", False), large_mid_rows=0)

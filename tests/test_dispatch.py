@@ -152,13 +152,17 @@ def test_branch_mixers_say_where_middling_products_gain(monkeypatch):
     from litellmengine_b200.parts.parallel import ParallelMixer
     asked = []
     monkeypatch.setattr(ops, "linear", lambda x, w, large_mid_rows, small=True, **k: asked.append(large_mid_rows) or torch.zeros(x.shape[0], w.shape[0]))
-    for cls, rows in ((GatedAttentionMixer, [0, 0]), (GatedLinearAttention, [0, 0]), (RetentionMixer, [0, 0]), (DeltaRuleMixer, [48, 32])):
+    alone = types.SimpleNamespace(partials_ok=False, residual=None)
+    between = (types.SimpleNamespace(partials_ok=True, residual=None), types.SimpleNamespace(partials_ok=False, residual=torch.zeros(1)))
+    for cls, n, k, rows, inside in ((GatedAttentionMixer, 8, 4096, [0, 0], [32, 32]), (GatedAttentionMixer, 8, 4088, [0, 0], [32, 48]),
+                                    (GatedLinearAttention, 8, 8, [0, 0], [0, 0]), (RetentionMixer, 8, 8, [0, 0], [0, 0]),
+                                    (DeltaRuleMixer, 8, 8, [32, 32], [48, 32]), (DeltaRuleMixer, 12, 8, [48, 32], [48, 32])):
         m = cls.__new__(cls)
-        m.w_in, m.w_o, m.out_width, m.dtype = torch.ones(6, 8), torch.ones(8, 4), 4, torch.bfloat16
-        m.mix = lambda *a: None
-        BranchMixer.forward(m, torch.ones(20, 8), types.SimpleNamespace())
-        assert asked == rows, cls
-        asked.clear()
+        m.w_in, m.w_o, m.out_width, m.dtype, m.mix = torch.ones(n, 8), torch.ones(8, k), k, torch.bfloat16, lambda *a: None
+        for ctx, want in ((alone, rows), (types.SimpleNamespace(), rows), (between[0], inside), (between[1], inside)):
+            BranchMixer.forward(m, torch.ones(20, 8), ctx)
+            assert asked == want, cls
+            asked.clear()
     m = ParallelMixer.__new__(ParallelMixer)
     m.w_in, m.w_o, m.dtype, m.branches, m.scales, m.in_cols, m.out_cols = torch.ones(6, 8), torch.ones(8, 4), torch.bfloat16, [], [], [], []
     m.forward(torch.ones(20, 8), types.SimpleNamespace())
