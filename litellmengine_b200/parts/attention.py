@@ -233,9 +233,7 @@ class BranchMixer:
         4,096, 40 requests 235 us, 244)."""
         return 0, 0
 
-    def small_gains(self, rows: int) -> bool:
-        """Whether an input product of `rows` rows gains from `ops.linear_small` where that takes it."""
-        return True
+    small_gains = None        # small_gains(rows): whether the input product gains from `ops.linear_small` where that takes it (None: always)
 
     def mix(self, proj: torch.Tensor, col0: int, ctx: StageContext, out: torch.Tensor, out_col0: int,
             out_scale: float) -> None:
@@ -243,9 +241,10 @@ class BranchMixer:
 
     def forward(self, x: torch.Tensor, ctx: StageContext):
         partials_ok = getattr(ctx, "partials_ok", False)
-        rows_in, rows_out = self.large_rows(partials_ok or getattr(ctx, "residual", None) is not None)
-        proj = ops.linear(x, self.w_in, out_dtype=torch.float32, large_mid_rows=rows_in, small=self.small_gains(x.shape[0]))
-        out = torch.empty((x.shape[0], self.out_width), dtype=self.dtype, device=x.device)
+        rows = x.shape[0]
+        rows_in, rows_out = self.large_rows(partials_ok or getattr(ctx, "residual", None) is not None) if rows in ops.MID_ROWS else (0, 0)
+        proj = ops.linear(x, self.w_in, out_dtype=torch.float32, large_mid_rows=rows_in, small=self.small_gains is None or self.small_gains(rows))
+        out = torch.empty((rows, self.out_width), dtype=self.dtype, device=x.device)
         self.mix(proj, 0, ctx, out, 0, 1.0)
         return ops.linear(out, self.w_o, out_dtype=torch.float32, partials_ok=partials_ok, large_mid_rows=rows_out)
 

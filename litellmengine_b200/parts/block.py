@@ -205,7 +205,8 @@ class Block:
 def _normed(norm, part, h: torch.Tensor, delta, dtype: torch.dtype):
     """(h + delta, the part's input norm(h + delta)): by the norm's kernel, in place, or left to the part's first product."""
     from ..csrc import ops
-    if h.is_cuda and ops.rows_worth_leaving(h, delta) and speaks_for_forward(norm, "products_apply_it") and speaks_for_forward(part, "first_product"):
+    if (getattr(part, "first_product", None) is not None and h.is_cuda and ops.rows_worth_leaving(h, delta)
+            and speaks_for_forward(norm, "products_apply_it") and speaks_for_forward(part, "first_product")):
         weight, gated = part.first_product()
         rows = ops.pending_rows(h, delta, norm, weight, dtype, gated)
         if rows is not None:

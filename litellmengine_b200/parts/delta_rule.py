@@ -40,7 +40,7 @@ class DeltaRuleMixer(BranchMixer):
         return 48 if between or self.w_in.shape[0] % 8 else 32, 32
 
     def small_gains(self, rows: int) -> bool:
-        """As `BranchMixer.small_gains`.  Decode steps of 4 layers with feed-forwards, us, with it and with the streaming product, input K and N: 1,024,
+        """See `BranchMixer.small_gains`.  Decode steps of 4 layers with feed-forwards, us, with it and with the streaming product, input K and N: 1,024,
         3,208, 1 / 8 / 16 requests 112, 129 / 121, 138 / 154, 170; 1,536, 2,438 153, 154 / 150, 172 / 193, 204; 2,048, 3,208 176, 182 / 194, 196.  Not with
         9 to 16 rows of up to 512 values, whose sums the streaming product leaves whole as well (512, 1,668, 12 / 16 requests 136, 127 / 137, 130), and not
         with wide rows and an odd N (1,792, 2,823, 8 requests 194, 174; a layer alone 2 to 3.6 of 20 longer; 2,560, 2,053 up to 5)."""
