@@ -1531,8 +1531,12 @@ def rows_worth_making(qkv, group: int) -> bool:
     and split, add them up, each for its heads; the kernel of its own does that once.  Steps of 4 layers, time
     with and without, at contexts of 60 to 4,000: groups of 4, width 2,560 and 4,096, up to 4 splits, 1 to 8 rows 0.97 to 1.02, up to 6 and
     up to 300 1.00 to 1.02, 9 to 16 rows 0.97 to 1.00; groups of 2, width 2,048, 9 rows 0.98 to 1.02, 12 0.98 to 1.01, 16 0.97 to 1.00.
-    Without pending splits 0.94 to 1.01 (1 to 40 rows, width 1,024 to 4,096)."""
-    return not isinstance(qkv, PartialSum) or (qkv.parts.shape[1] > 8 and qkv.parts.shape[1] * group >= 32)
+    Without pending splits 0.94 to 1.01 (1 to 40 rows, width 1,024 to 4,096).  That is a captured step; where the host launches each kernel the one
+    launch less counts more (a layer of width 4,096, 1 to 8 requests, 61 us and 79).  The numbers are the same bits either way."""
+    if not isinstance(qkv, PartialSum):
+        return True
+    rows = qkv.parts.shape[1]
+    return (rows > 8 and rows * group >= 32) or not torch.cuda.is_current_stream_capturing()
 
 
 def paged_attention_decode_made(qkv, cache: torch.Tensor, positions, token_entry, entry_slot, block_table: torch.Tensor, q_norm_w, k_norm_w,

@@ -180,9 +180,9 @@ class AttentionMixer:
             work = b.preludes.get(AttentionWork.name)
             if (has_kv and self.dtype == torch.bfloat16 and self.span is None and work is not None and not getattr(b, "any_division", False)
                     and work.num_decode == b.num_tokens and not work.num_prefill_tiles and (rot is None or rot.rotary_dim == self.d)
-                    and ops.rows_worth_making(qkv, self.nq // self.nkv)
                     and ops.decode_makes_its_rows(qkv, cache, self.d, self.nq // self.nkv, ctx.page_size,
-                                                  splits := decode_key_splits(self.device, b.num_tokens, self.nkv, decode_reach(b, None)))):
+                                                  splits := decode_key_splits(self.device, b.num_tokens, self.nkv, decode_reach(b, None)))
+                    and ops.rows_worth_making(qkv, self.nq // self.nkv)):
                 # a step of single tokens: norms, rotation and cache write inside the attention kernel too
                 a = ops.paged_attention_decode_made(
                     qkv, cache, b.positions, b.token_entry, b.entry_slot, table, qw, kw, eps, rot.inv_freq if rot is not None else None,
@@ -233,17 +233,17 @@ class BranchMixer:
         4,096, 40 requests 235 us, 244)."""
         return 0, 0
 
-    small_gains = None        # small_gains(rows): whether the input product gains from `ops.linear_small` where that takes it (None: always)
+    small_rows = 16           # rows up to which the input product gains from `ops.linear_small` where that takes it
 
     def mix(self, proj: torch.Tensor, col0: int, ctx: StageContext, out: torch.Tensor, out_col0: int,
             out_scale: float) -> None:
         raise NotImplementedError
 
     def forward(self, x: torch.Tensor, ctx: StageContext):
-        partials_ok = getattr(ctx, "partials_ok", False)
-        rows = x.shape[0]
-        rows_in, rows_out = self.large_rows(partials_ok or getattr(ctx, "residual", None) is not None) if rows in ops.MID_ROWS else (0, 0)
-        proj = ops.linear(x, self.w_in, out_dtype=torch.float32, large_mid_rows=rows_in, small=self.small_gains is None or self.small_gains(rows))
+        rows, partials_ok, rows_in, rows_out = x.shape[0], getattr(ctx, "partials_ok", False), 0, 0
+        if rows in ops.MID_ROWS:
+            rows_in, rows_out = self.large_rows(partials_ok or getattr(ctx, "residual", None) is not None)
+        proj = ops.linear(x, self.w_in, out_dtype=torch.float32, large_mid_rows=rows_in, small=rows <= self.small_rows)
         out = torch.empty((rows, self.out_width), dtype=self.dtype, device=x.device)
         self.mix(proj, 0, ctx, out, 0, 1.0)
         return ops.linear(out, self.w_o, out_dtype=torch.float32, partials_ok=partials_ok, large_mid_rows=rows_out)

@@ -39,14 +39,6 @@ class DeltaRuleMixer(BranchMixer):
         decode 1 to 2 shorter, prompts 2 to 4 of 54 longer, but where the library reads odd rows (7,828 x 5,120) 36 to 40 of 78 to 120 shorter."""
         return 48 if between or self.w_in.shape[0] % 8 else 32, 32
 
-    def small_gains(self, rows: int) -> bool:
-        """See `BranchMixer.small_gains`.  Decode steps of 4 layers with feed-forwards, us, with it and with the streaming product, input K and N: 1,024,
-        3,208, 1 / 8 / 16 requests 112, 129 / 121, 138 / 154, 170; 1,536, 2,438 153, 154 / 150, 172 / 193, 204; 2,048, 3,208 176, 182 / 194, 196.  Not with
-        9 to 16 rows of up to 512 values, whose sums the streaming product leaves whole as well (512, 1,668, 12 / 16 requests 136, 127 / 137, 130), and not
-        with wide rows and an odd N (1,792, 2,823, 8 requests 194, 174; a layer alone 2 to 3.6 of 20 longer; 2,560, 2,053 up to 5)."""
-        n, k = self.w_in.shape
-        return not (rows > 8 and 384 < k <= 512) and not (n % 2 and k > 1280)
-
     PADDED = (32, 64, 128, 256)  # what the kernels are instantiated for
 
     _DEFAULT_NAMES = {"q": "q_proj.weight", "k": "k_proj.weight", "v": "v_proj.weight", "o": "o_proj.weight",
@@ -98,6 +90,11 @@ class DeltaRuleMixer(BranchMixer):
         self.g_off = self.a_off + self.ranks[0]
         self.w_in = torch.cat([x.to(dt) for x in rows], dim=0).contiguous()
         self.in_width = self.w_in.shape[0]
+        # Decode steps of 4 layers with feed-forwards, us, with the product that leaves no parts and with the streaming product, input K and N: 1,024,
+        # 3,208, 1 / 8 / 16 requests 112, 129 / 121, 138 / 154, 170; 1,536, 2,438 153, 154 / 150, 172 / 193, 204; 2,048, 3,208 176, 182 / 194, 196.  Not with
+        # 9 to 16 rows of up to 512 values, whose sums the streaming product leaves whole as well (512, 1,668, 12 / 16 requests 136, 127 / 137, 130), and not
+        # with wide rows and an odd N (1,792, 2,823, 8 requests 194, 174; a layer alone 2 to 3.6 of 20 longer; 2,560, 2,053 up to 5).
+        self.small_rows = 0 if self.in_width % 2 and self.hidden > 1280 else 8 if 384 < self.hidden <= 512 else 16
         self.w_o = t[n["o"]].contiguous()
         self.conv_w = torch.cat([t[n[k]].float() for k in ("q_conv", "k_conv", "v_conv")], dim=0).contiguous()
         # the second halves of the low-rank projections are read transposed, [rank, channels], by kernels that add in 32-bit

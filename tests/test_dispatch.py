@@ -169,26 +169,30 @@ def test_branch_mixers_say_where_middling_products_gain(monkeypatch):
     assert asked == [0, 0]
 
 
-@pytest.mark.parametrize("rows,n,k,small", [(1, 3208, 2048, True), (16, 3208, 2048, True), (8, 1668, 512, True), (9, 1668, 512, False), (16, 1024, 392, False),
-                                            (16, 1024, 384, True), (9, 1024, 520, True), (1, 2053, 1280, True), (1, 2053, 1288, False), (16, 2054, 1288, True)])
-def test_the_delta_rule_says_where_small_products_gain(monkeypatch, rows, n, k, small):
+@pytest.mark.parametrize("heads,hidden,rows", [(16, 2048, 16), (8, 512, 8), (8, 392, 8), (8, 384, 16), (8, 520, 16), (5, 1280, 16), (5, 1288, 0), (6, 1288, 16)])
+def test_the_delta_rule_says_where_small_products_gain(monkeypatch, heads, hidden, rows):
+    from litellmengine_b200.config.specs import MixerSpec
     from litellmengine_b200.parts.delta_rule import DeltaRuleMixer
-    from litellmengine_b200.parts.linear_attention import GatedLinearAttention
     asked = []
+    m = DeltaRuleMixer(MixerSpec("channel_delta", num_heads=heads, head_dim=32, params=(("taps", 1), ("decay_rank", 4), ("gate_rank", 4))), hidden,
+                       torch.bfloat16, "cpu")
+    m.load({n: torch.zeros(p.shape) for n, p in m.parameters().items()})
+    assert m.w_in.shape == (m.in_width, hidden) and m.in_width % 2 == heads % 2
     monkeypatch.setattr(ops, "linear", lambda x, w, small=True, **k: asked.append(small) or torch.zeros(x.shape[0], w.shape[0]))
-    for cls, want in ((GatedLinearAttention, True), (DeltaRuleMixer, small)):
-        m = cls.__new__(cls)
-        m.w_in, m.w_o, m.out_width, m.dtype, m.mix = torch.ones(n, k), torch.ones(8, 4), 4, torch.bfloat16, lambda *a: None
-        m.forward(torch.ones(rows, k), types.SimpleNamespace())
-        assert asked == [want, True], cls
-        asked.clear()
+    m.mix = lambda *a: None
+    for n in (1, 8, 9, 16):
+        m.forward(torch.ones(n, hidden), types.SimpleNamespace())
+    assert asked[::2] == [n <= rows for n in (1, 8, 9, 16)] and all(asked[1::2])
 
 
 @pytest.mark.parametrize("rows,group,pending,worth", [(1, 4, False, True), (16, 1, False, True), (8, 4, True, False), (8, 16, True, False),
                                                       (9, 4, True, True), (9, 3, True, False), (15, 2, True, False), (16, 2, True, True)])
-def test_rows_are_made_in_the_attention_kernel_where_that_pays(rows, group, pending, worth):
+def test_rows_are_made_in_the_attention_kernel_where_that_pays(monkeypatch, rows, group, pending, worth):
     qkv = torch.zeros(rows, 384)
-    assert ops.rows_worth_making(ops.PartialSum(torch.stack([qkv, qkv])) if pending else qkv, group) == worth
+    qkv = ops.PartialSum(torch.stack([qkv, qkv])) if pending else qkv
+    for captured in (True, False):
+        monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: captured)
+        assert ops.rows_worth_making(qkv, group) == (worth or not captured)
 
 
 def test_tables_of_angles_go_by_the_spec(monkeypatch):
